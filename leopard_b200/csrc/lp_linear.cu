@@ -282,6 +282,256 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) linear_rows_kernel(LinArgs a)
   }
 }
 
+// ---------------------------------------------------------------------------------------------------------------------------------
+// Up to 64 rows (decoding): a product is bound by reading its weights once, at every number of rows, when the multiply-adds are
+// out of the way.  So the weight tile is the 16-row operand of the warp's matrix instruction and up to MG groups of eight rows of A
+// are its other one: a CTA owns 16 NT output columns, its warps share out K in steps of 32 (a lane reads 16 bytes of each weight row and of its
+// row of A; the same permutation of k on both sides, which a sum does not see), eight weight loads per lane are in flight before the
+// first product, and the warps' sums meet in shared memory, warp by warp in a fixed order.  The gated units take gate row n and up
+// row n + N / 2 as rows g and g + 8 of one tile, so both halves of an output end up in one lane.
+// fp32 rows of A are cut into three bf16 terms that add up to them exactly (8 + 8 + 8 bits): every product is still exact.  The
+// instruction cuts its running sum off instead of rounding it, a bias that grows with the chain: every 16 products start a
+// chain of their own (small terms first) and are added to the sum in fp32.
+// Measured (B200, graph of launches, weights from HBM, M = 8): N = 8192, K = 2048 9.8 us (3.4 TB/s; a warp per column with fp32 FMAs: 67.6),
+// N = 32000, K = 4096 53 us (4.9 TB/s; 350), N = 2048, K = 2048 5.8 us (29.7), fp32 A 10.9 us (66).  Error against 64 bits at K = 2048
+// / 8192: 0.9e-7 / 1.2e-7 of the result (FMA chains of a lane: 0.8e-7 / 1.25e-7; of the tile kernel: 3.9e-7 / 9.6e-7).
+// Pairs (experts): the CTAs of weight group blockIdx.y gather the pairs that chose it and read the group's weights once for all of them.
+constexpr int STREAM_MAX_ROWS = 64, STREAM_MAX_PAIRS = 1024;
+
+struct Bf16Terms { uint4 hi, mid, lo; };
+__device__ __forceinline__ uint32_t pack_upper(float x, float y) { return (__float_as_uint(x) >> 16) | (__float_as_uint(y) & 0xffff0000u); }
+__device__ __forceinline__ uint32_t take_upper(float& x, float& y) {      // what is left of x and y stays behind
+  const uint32_t r = pack_upper(x, y);
+  x -= __uint_as_float(__float_as_uint(x) & 0xffff0000u);
+  y -= __uint_as_float(__float_as_uint(y) & 0xffff0000u);
+  return r;
+}
+__device__ __forceinline__ Bf16Terms split3(const float4& a, const float4& b) {
+  float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  Bf16Terms r;
+  bool odd = false;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) odd |= (__float_as_uint(v[i]) & 0x7f800000u) == 0x7f800000u;
+  if (odd) {      // an infinity leaves nothing behind, a NaN stays one without its lower bits
+    float w[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t u = __float_as_uint(v[i]);
+      const bool whole = (u & 0x7f800000u) == 0x7f800000u;
+      w[i] = !whole ? v[i] - __uint_as_float(u & 0xffff0000u) : 0.f;
+      if (whole && (u & 0x7fffffu)) v[i] = __uint_as_float(u | 0x400000u);
+    }
+    r.hi = make_uint4(pack_upper(v[0], v[1]), pack_upper(v[2], v[3]), pack_upper(v[4], v[5]), pack_upper(v[6], v[7]));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = w[i];
+  } else {
+    r.hi.x = take_upper(v[0], v[1]); r.hi.y = take_upper(v[2], v[3]); r.hi.z = take_upper(v[4], v[5]); r.hi.w = take_upper(v[6], v[7]);
+  }
+  r.mid.x = take_upper(v[0], v[1]); r.mid.y = take_upper(v[2], v[3]); r.mid.z = take_upper(v[4], v[5]); r.mid.w = take_upper(v[6], v[7]);
+  r.lo = make_uint4(pack_upper(v[0], v[1]), pack_upper(v[2], v[3]), pack_upper(v[4], v[5]), pack_upper(v[6], v[7]));
+  return r;
+}
+// the two halves of a step of 32 products, in chains of their own
+__device__ __forceinline__ void mma_step(float* d, float* e, const uint4& w0, const uint4& w1, const uint4& x) {
+  mma_bf16(d, w0.x, w1.x, w0.y, w1.y, x.x, x.y);
+  mma_bf16(e, w0.z, w1.z, w0.w, w1.w, x.z, x.w);
+}
+
+template <typename AT, int NT, int MG>
+__global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) linear_stream_kernel(LinArgs a, int gated, int c_fp32, int n_pairs) {
+  extern __shared__ float dyn_smem[];      // [warps][NT MG 4][32] partial sums
+  __shared__ int pair_of[STREAM_MAX_PAIRS];
+  __shared__ int pair_count[STREAM_MAX_PAIRS / 32];
+  constexpr int U = MG >= 4 ? 1 : 2;      // k steps whose weights are in flight together
+  constexpr int SLOTS = NT * MG * 4;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const bool pairs = a.z_group != nullptr;
+  const int z = blockIdx.z;
+  const int n_out = gated ? a.N / 2 : a.N;
+  const int cols = gated ? 8 * NT : 16 * NT;
+  const int n0 = blockIdx.x * cols;
+  int rows = a.M;
+  if (pairs) {      // the group's pairs, in order: a ballot for every 32 of them, then their places
+    const int spans = (n_pairs + 31) / 32;
+    for (int q = warp; q < spans; q += n_warps) {
+      const unsigned m = __ballot_sync(0xffffffffu, q * 32 + lane < n_pairs && a.z_group[q * 32 + lane] == (int)blockIdx.y);
+      if (lane == 0) pair_count[q] = __popc(m);
+      pair_of[q * 32 + lane] = (m >> lane & 1u) ? __popc(m & ((1u << lane) - 1u)) : -1;
+    }
+    __syncthreads();
+    int at[STREAM_MAX_PAIRS / (4 * 32)];      // the places of this warp's pairs
+    int before = 0, k = 0;
+    for (int q = 0; q < spans; ++q) {
+      if (q % n_warps == warp) {
+        const int r = pair_of[q * 32 + lane];
+        at[k++] = r >= 0 ? before + r : -1;
+      }
+      before += pair_count[q];
+    }
+    __syncthreads();
+    k = 0;
+    for (int q = warp; q < spans; q += n_warps, ++k)
+      if (at[k] >= 0) pair_of[at[k]] = q * 32 + lane;
+    __syncthreads();
+    rows = before;
+    if (rows == 0) return;
+  }
+  const AT* A = reinterpret_cast<const AT*>(a.A) + (pairs ? 0 : (long long)z * a.a_batch) + lin_seg(a, n0);
+  const bf16* W = a.W + (long long)(pairs ? (int)blockIdx.y : z) * a.w_batch;
+  const bf16* w0[NT];
+  const bf16* w1[NT];
+#pragma unroll
+  for (int j = 0; j < NT; ++j) {
+    const int r0 = n0 + j * (gated ? 8 : 16) + g, r1 = gated ? r0 + n_out : r0 + 8;
+    w0[j] = r0 < n_out ? W + (long long)r0 * a.ldw : nullptr;
+    w1[j] = (gated ? r0 : r1) < n_out ? W + (long long)r1 * a.ldw : nullptr;
+  }
+  const uint4 none = make_uint4(0, 0, 0, 0);
+  for (int m0 = 0; m0 < rows; m0 += 8 * MG) {
+    const AT* x[MG];
+#pragma unroll
+    for (int i = 0; i < MG; ++i) {
+      const int m = m0 + 8 * i + g;
+      x[i] = m < rows ? A + (long long)(pairs ? pair_of[m] / a.a_div : m) * a.lda : nullptr;
+    }
+    float acc[NT][MG][4];
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int i = 0; i < MG; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[j][i][c] = 0.f;
+    for (int s = warp; s * 32 < a.K; s += U * n_warps) {
+      uint4 u0[U][NT], u1[U][NT];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = (s + u * n_warps) * 32 + t * 8;
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          u0[u][j] = k < a.K && w0[j] != nullptr ? ldg_once(w0[j] + k) : none;
+          u1[u][j] = k < a.K && w1[j] != nullptr ? ldg_once(w1[j] + k) : none;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = (s + u * n_warps) * 32 + t * 8;
+        if constexpr (sizeof(AT) == 2) {
+          uint4 v[MG];
+#pragma unroll
+          for (int i = 0; i < MG; ++i) v[i] = k < a.K && x[i] != nullptr ? *reinterpret_cast<const uint4*>(x[i] + k) : none;
+#pragma unroll
+          for (int i = 0; i < MG; ++i)
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+              float d[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
+              mma_step(d, e, u0[u][j], u1[u][j], v[i]);
+#pragma unroll
+              for (int c = 0; c < 4; ++c) acc[j][i][c] += d[c] + e[c];
+            }
+        } else {
+#pragma unroll
+          for (int i = 0; i < MG; ++i) {
+            float4 p = make_float4(0.f, 0.f, 0.f, 0.f), q = p;
+            if (k < a.K && x[i] != nullptr) {
+              p = *reinterpret_cast<const float4*>(x[i] + k);
+              q = *reinterpret_cast<const float4*>(x[i] + k + 4);
+            }
+            const Bf16Terms v = split3(p, q);
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {      // the small terms first
+              float d[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
+              mma_step(d, e, u0[u][j], u1[u][j], v.lo);
+              mma_step(d, e, u0[u][j], u1[u][j], v.mid);
+              mma_step(d, e, u0[u][j], u1[u][j], v.hi);
+#pragma unroll
+              for (int c = 0; c < 4; ++c) acc[j][i][c] += d[c] + e[c];
+            }
+          }
+        }
+      }
+    }
+    if (m0 > 0) __syncthreads();      // the sums of the rows before have been read
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int i = 0; i < MG; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) dyn_smem[(warp * SLOTS + (j * MG + i) * 4 + c) * 32 + lane] = acc[j][i][c];
+    __syncthreads();
+    const int here = min(8 * MG, rows - m0);
+    for (int e = threadIdx.x; e < cols * here; e += blockDim.x) {
+      const int nl = e % cols, ml = e / cols, n = n0 + nl;
+      if (n >= n_out) continue;
+      const int j = gated ? nl >> 3 : nl >> 4, r = gated ? nl & 7 : nl & 15;
+      const int at = (((j * MG + (ml >> 3)) * 4 + (r >> 3) * 2 + (ml & 1)) * 32) + (r & 7) * 4 + ((ml & 7) >> 1);
+      float s = 0.f, s2 = 0.f;
+      for (int w = 0; w < n_warps; ++w) {
+        s += dyn_smem[w * SLOTS * 32 + at];
+        if (gated) s2 += dyn_smem[w * SLOTS * 32 + at + 64];
+      }
+      const int m = pairs ? pair_of[m0 + ml] : m0 + ml;
+      if (a.row_scale != nullptr) {
+        s *= a.row_scale[m];
+        s2 *= a.row_scale[m];
+      }
+      if (a.bias != nullptr) {
+        s += a.bias[n];
+        if (gated) s2 += a.bias[n + n_out];
+      }
+      float v = gated ? lin_gate(a.epi, s, s2, a.e0, a.e1) : lin_epi(a.epi, s, a.e0, a.e1);
+      if (a.gate != nullptr) v /= 1.0f + expf(-a.gate[(pairs ? 0 : (long long)z * a.gate_batch) + (long long)m * a.ldg + n]);
+      const long long at_c = (pairs ? 0 : (long long)z * a.c_batch) + (long long)m * a.ldc + n;
+      if (c_fp32) {
+        float* C = reinterpret_cast<float*>(a.C) + at_c;
+        *C = a.c_accum ? fmaf(a.c_scale, v, *C) : v;
+      } else {
+        bf16* C = reinterpret_cast<bf16*>(a.C) + at_c;
+        *C = __float2bfloat16(a.c_accum ? fmaf(a.c_scale, v, __bfloat162float(*C)) : v);
+      }
+    }
+  }
+}
+
+static bool gated_epi(int epi) { return epi == LP_EPI_SILU_GATE || epi == LP_EPI_CLAMP_GLU || epi == LP_EPI_GELU_GATE; }
+
+template <typename AT, int NT, int MG>
+static int launch_stream(const LinArgs& a, int c_fp32, dim3 grid, int warps, int n_pairs, cudaStream_t stream) {
+  const size_t smem = (size_t)warps * NT * MG * 4 * 32 * sizeof(float);
+  if (smem > 40 * 1024) LP_CHECK_CUDA(cudaFuncSetAttribute(linear_stream_kernel<AT, NT, MG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536));
+  linear_stream_kernel<AT, NT, MG><<<grid, warps * 32, smem, stream>>>(a, gated_epi(a.epi), c_fp32, n_pairs);
+  note_launch();
+  LP_CHECK_CUDA(cudaGetLastError());
+  return 0;
+}
+
+// rows of whole 16-byte pieces on both sides: what linear_stream_kernel reads
+static bool stream_ok(const LinArgs& a, int a_fp32, int batch) {
+  const int q = a_fp32 ? 4 : 8;
+  return a.K % 8 == 0 && a.ldw % 8 == 0 && a.lda % q == 0 && (batch == 1 || a.a_batch % q == 0) && a.w_batch % 8 == 0 &&
+         (a.seg_cols == 0 || a.a_seg % q == 0) && (reinterpret_cast<uintptr_t>(a.A) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.W) & 15) == 0;
+}
+
+// n_groups > 0: pairs, of which a group has up to about `rows` (more run in further rounds over its weights); else one problem of `rows` rows per batch entry
+static int dispatch_stream(const LinArgs& a, int a_fp32, int c_fp32, int batch, int rows, int n_groups, int n_pairs, cudaStream_t stream) {
+  const int n_out = gated_epi(a.epi) ? a.N / 2 : a.N, per = gated_epi(a.epi) ? 8 : 16;
+  const int mg = rows <= 8 ? 1 : rows <= 16 ? 2 : rows <= 32 ? 4 : 8;
+  const long long problems = n_groups > 0 ? n_groups : batch;
+  // two tiles a CTA read A half as often (and cut it into terms once): taken once the grid still has two CTAs for every SM and where
+  // segments allow; with more than eight bf16 rows its registers cost more CTAs than it saves (N = 12288, K = 4096, M = 16: 35 us with one tile, 46 with two)
+  const long long wide = problems * ((n_out + 2 * per - 1) / (2 * per));
+  const int nt = (mg == 1 || a_fp32) && wide >= 2 * sm_count() && (a.seg_cols == 0 || a.seg_cols % (2 * per) == 0) ? 2 : 1;
+  const long long ctas = problems * ((n_out + nt * per - 1) / (nt * per));
+  // a short K has no work for more warps; a grid of few CTAs wants more loads in flight in each (N = 2048, K = 8192: 15 us with 16 warps, 11 with 32)
+  int warps = a.K <= 256 ? 4 : !a_fp32 && mg * nt == 1 && ctas <= sm_count() && a.K >= 4096 ? 32 : ctas <= 2 * sm_count() && a.K >= 1024 && mg <= 4 ? 16 : 8;
+  dim3 grid((n_out + nt * per - 1) / (nt * per), n_groups > 0 ? n_groups : 1, n_groups > 0 ? 1 : batch);
+#define LP_STREAM(MG)                                                                                                              \
+  (a_fp32 ? (nt == 2 ? launch_stream<float, 2, MG>(a, c_fp32, grid, warps, n_pairs, stream) : launch_stream<float, 1, MG>(a, c_fp32, grid, warps, n_pairs, stream)) \
+          : (nt == 2 ? launch_stream<bf16, 2, MG>(a, c_fp32, grid, warps, n_pairs, stream) : launch_stream<bf16, 1, MG>(a, c_fp32, grid, warps, n_pairs, stream)))
+  return mg == 1 ? LP_STREAM(1) : mg == 2 ? LP_STREAM(2) : mg == 4 ? LP_STREAM(4) : LP_STREAM(8);
+#undef LP_STREAM
+}
+
 template <typename AT, typename CT, bool GATED>
 static int launch_linear(const LinArgs& a, int batch, int m_tiles, bool allow_rows, cudaStream_t stream) {
   const int n_out = GATED ? a.N / 2 : a.N;
@@ -296,8 +546,6 @@ static int launch_linear(const LinArgs& a, int batch, int m_tiles, bool allow_ro
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
-
-static bool gated_epi(int epi) { return epi == LP_EPI_SILU_GATE || epi == LP_EPI_CLAMP_GLU || epi == LP_EPI_GELU_GATE; }
 
 static int dispatch_linear(const LinArgs& a, int a_fp32, int c_fp32, int batch, int m_tiles, bool allow_rows, cudaStream_t stream) {
   const bool gated = gated_epi(a.epi);
@@ -339,6 +587,8 @@ extern "C" int lp_linear(const lp_linear_desc* d, void* stream_) {
   LP_REQUIRE(d->seg_cols == 0 || (d->seg_cols > 0 && d->n_segs >= 1 && d->seg_cols % (d->M <= ROWS_MAX ? ROWS_WARPS : LIN_BN) == 0),
              "lp_linear: column segments of %d do not fit the CTAs of a product of %d rows", d->seg_cols, d->M);
   LP_REQUIRE(d->seg_cols == 0 || !gated_epi(d->epi), "lp_linear: a gated unit has one operand");
+  if (d->M <= STREAM_MAX_ROWS && stream_ok(a, d->a_fp32, d->batch) && (d->seg_cols == 0 || d->seg_cols % 16 == 0))
+    return dispatch_stream(a, d->a_fp32, d->c_fp32, d->batch, d->M, 0, 0, stream);
   return dispatch_linear(a, d->a_fp32, d->c_fp32, d->batch, (d->M + LIN_BM - 1) / LIN_BM, true, stream);
 }
 
@@ -361,6 +611,9 @@ extern "C" int lp_linear_pairs(const lp_linear_desc* d, const int* pair_group, i
   a.a_rows = nullptr; a.tile_group = nullptr; a.z_group = pair_group; a.a_div = a_div;
   a.bias = d->bias; a.row_scale = d->row_scale; a.gate = d->gate; a.ldg = d->ldg; a.gate_batch = d->gate_batch;
   a.seg_cols = 0; a.n_segs = 0; a.a_seg = 0;
+  // with the number of groups (batch > 1) a group's weights are read once for all of its pairs
+  if (d->batch > 1 && n_pairs <= STREAM_MAX_PAIRS && stream_ok(a, d->a_fp32, 1))
+    return dispatch_stream(a, d->a_fp32, d->c_fp32, 1, 2 * ((n_pairs + d->batch - 1) / d->batch), d->batch, n_pairs, stream);
   return dispatch_linear(a, d->a_fp32, d->c_fp32, n_pairs, 1, true, stream);
 }
 

@@ -31,7 +31,11 @@ from .seqcache import SequenceCache
 
 F32, BF16, I32 = torch.float32, torch.bfloat16, torch.int32
 TENSOR_CORE_MIN_ROWS = 64
-MOE_PAIRS_MAX = 64             # up to this many (token, choice) pairs the experts run as one-row weight-streaming problems
+# up to 64 rows a product is bound by its weights and lp_linear streams them once, epilogue included; its operand traffic grows with
+# rows times columns, the tcgen05 GEMM's latency with K alone: they cross near rows * columns = 170,000 (K = 2048: 32 rows by 8192
+# columns 17.3 us against 13.7, 16 rows 11.5 against 14.4, 64 rows by 2048 columns 18.7 against 13.4, 32 rows 9.9 against 12.7)
+STREAM_ROWS, STREAM_ROWS_ALONE, STREAM_MAX_OUTPUTS = 64, 8, 170_000
+MOE_PAIRS_MAX = 512            # up to this many (token, choice) pairs an expert's weights are streamed once for the pairs that chose it
 PAD_PROJECTION_ROWS = 128      # a projection narrower than a tensor-core tile is padded with zero rows beside ones that are at least this wide
 MAX_DECODE_GRAPHS = 32         # captured decode layouts kept at a time
 PAGE_TABLE_STEP = 16           # decode batches round their page-table width up to a multiple of this
@@ -869,9 +873,15 @@ class SeqLMEngine:
 
     def _on_tensor_cores(self, a, w, M, N, K) -> bool:
         """The tcgen05 GEMM takes a product when it is large enough to fill tiles and meets the 16-byte rules of its TMA loads."""
-        return (self.tensor_core_rows is not None and M >= self.tensor_core_rows and a.dtype == BF16 and N >= 128 and K >= 64
-                and N % 8 == 0 and K % 8 == 0 and a.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and a.stride(1) == 1
-                and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+        return M >= (self.tensor_core_rows or 0) and self._fits_tensor_cores(a, w, N, K)
+
+    def _streams(self, a, w, M, N, K) -> bool:
+        """lp_linear's weight-streaming kernel takes a product of few rows, unless the GEMM can and has the columns to be faster"""
+        return M <= STREAM_ROWS_ALONE or (M <= STREAM_ROWS and (M * N <= STREAM_MAX_OUTPUTS or not self._fits_tensor_cores(a, w, N, K)))
+
+    def _fits_tensor_cores(self, a, w, N, K) -> bool:
+        return (self.tensor_core_rows is not None and a.dtype == BF16 and N >= 128 and K >= 64 and N % 8 == 0 and K % 8 == 0
+                and a.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and a.stride(1) == 1 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
     def linear(self, a: torch.Tensor, w: torch.Tensor, out_dtype, epi=_lib.EPI_NONE, epi_a=0.0, epi_b=0.0, out=None, into=None, bias=None,
                row_scale=None):
@@ -881,7 +891,7 @@ class SeqLMEngine:
         N = w.shape[0]
         n_out = N // 2 if epi in _lib.GATED_EPIS else N
         # a row scale reaches the tensor-core path only through the activation kernel that follows the product
-        tc = self._on_tensor_cores(a, w, M, N, K) and (row_scale is None or (epi != _lib.EPI_NONE and bias is None))
+        tc = not self._streams(a, w, M, N, K) and self._fits_tensor_cores(a, w, N, K) and (row_scale is None or (epi != _lib.EPI_NONE and bias is None))
         if into is not None:
             x, mult = into[0], into[1]
             gate = into[2] if len(into) > 2 else None
@@ -926,7 +936,7 @@ class SeqLMEngine:
         out = self._empty((R, N), F32)
         parts = [(ops[i], w[a:b], out[:, a:b]) for i, (a, b) in enumerate(zip(bounds, bounds[1:]))]
         fits = seg % (_lib.LINEAR_ROWS_COLS if R <= _lib.LINEAR_ROWS_MAX else self.tile_rows) == 0
-        if not fits or any(self._on_tensor_cores(a, wi, R, wi.shape[0], D) for a, wi, _ in parts):
+        if not fits or any(not self._streams(a, wi, R, wi.shape[0], D) and self._fits_tensor_cores(a, wi, wi.shape[0], D) for a, wi, _ in parts):
             for a, wi, o in parts:
                 self.linear(a, wi, F32, out=o)
             return out
@@ -1316,17 +1326,17 @@ class SeqLMEngine:
         self._check(rc, "lp_moe_route")
         n_pairs = T * f.top
         if n_pairs <= MOE_PAIRS_MAX:
-            # few (token, choice) pairs (decoding): no sorting — every pair streams its expert's weights once, pair z = row z
+            # few (token, choice) pairs (decoding): no sorting — an expert's weights are streamed once for its pairs, pair z = row z
             w_gu, w_dn = lw["w_gu"], lw["w_edown"]
             h1 = self._empty((n_pairs, f.expert_ff), self.act)
             d1 = _lib.LinearDesc(A=_lib.ptr(h), lda=h.stride(0), a_batch=0, a_fp32=int(h.dtype == F32), W=_lib.ptr(w_gu), ldw=w_gu.stride(1),
                                  w_batch=w_gu.stride(0), C=_lib.ptr(h1), ldc=h1.stride(0), c_batch=0, c_fp32=int(h1.dtype == F32), M=1,
-                                 N=2 * f.expert_ff, K=D, batch=1, epi=epi, epi_a=epi_a, epi_b=epi_b, row_scale=_lib.ptr(wts) if on_input else None)
+                                 N=2 * f.expert_ff, K=D, batch=f.experts, epi=epi, epi_a=epi_a, epi_b=epi_b, row_scale=_lib.ptr(wts) if on_input else None)
             self._check(L.lp_linear_pairs(C.byref(d1), _lib.ptr(idx), f.top, n_pairs, st), "lp_linear_pairs")
             y = self._empty((n_pairs, D), F32)
             d2 = _lib.LinearDesc(A=_lib.ptr(h1), lda=h1.stride(0), a_batch=0, a_fp32=int(h1.dtype == F32), W=_lib.ptr(w_dn),
                                  ldw=w_dn.stride(1), w_batch=w_dn.stride(0), C=_lib.ptr(y), ldc=y.stride(0), c_batch=0, c_fp32=1, M=1, N=D,
-                                 K=f.expert_ff, batch=1, epi=_lib.EPI_NONE, epi_a=0.0, epi_b=0.0)
+                                 K=f.expert_ff, batch=f.experts, epi=_lib.EPI_NONE, epi_a=0.0, epi_b=0.0)
             self._check(L.lp_linear_pairs(C.byref(d2), _lib.ptr(idx), 1, n_pairs, st), "lp_linear_pairs")
             return self._moe_combine(f, lw, h, y, self._pair_identity(n_pairs), None if on_input else wts, gate)
         tiles = int(L.lp_moe_max_tiles(n_pairs, f.experts, self.tile_rows))

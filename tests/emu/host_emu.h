@@ -59,6 +59,19 @@ inline long long clock64() { return 0; }
 inline void __trap() { std::abort(); }
 template <typename T> inline T __ldcg(const T* p) { return *p; }
 inline float __bfloat162float(__nv_bfloat16 v) { return (float)v; }
+inline unsigned __float_as_uint(float f) { unsigned u; std::memcpy(&u, &f, 4); return u; }
+inline int __popc(unsigned v) { return __builtin_popcount(v); }
+inline unsigned __ballot_sync(unsigned mask, bool pred) {
+  unsigned r = 0;
+  const unsigned t = emu::linear_tid(), w = t >> 5, l = t & 31;
+  float* buf = emu::t_ctx->warp_buf.data() + w * 32;
+  auto& bar = emu::t_ctx->group(w, mask);
+  buf[l] = pred ? 1.f : 0.f;
+  bar.arrive_and_wait();
+  for (int i = 0; i < 32; ++i) r |= (unsigned)((mask >> i & 1) && buf[i] != 0.f) << i;
+  bar.arrive_and_wait();
+  return r;
+}
 inline float __uint_as_float(unsigned u) { float f; std::memcpy(&f, &u, 4); return f; }
 inline __nv_bfloat16 __ushort_as_bfloat16(unsigned short u) { __nv_bfloat16 r; r.bits = u; return r; }
 #define __align__(n) alignas(n)
@@ -87,6 +100,29 @@ inline void pdl_launch_dependents() {}
 inline int sm_count() { return 4; }
 inline float2 fma2(float2 a, float2 b, float2 c) { return {std::fma(a.x, b.x, c.x), std::fma(a.y, b.y, c.y)}; }
 inline float2 mul2(float2 a, float2 b) { return {a.x * b.x, a.y * b.y}; }
+inline uint4 ldg_once(const void* p) { return *reinterpret_cast<const uint4*>(p); }
+// warp-wide 16 x 8 x 16 product: every lane's registers go round the warp, each lane sums its four outputs over k
+inline void mma_bf16(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  uint32_t all[6][32];
+  const uint32_t mine[6] = {a0, a1, a2, a3, b0, b1};
+  const unsigned w = emu::linear_tid() >> 5, l = emu::linear_tid() & 31;
+  float* buf = emu::t_ctx->warp_buf.data() + w * 32;
+  for (int r = 0; r < 6; ++r) {
+    std::memcpy(buf + l, &mine[r], 4);
+    emu::t_ctx->warp_bar[w]->arrive_and_wait();
+    std::memcpy(all[r], buf, 128);
+    emu::t_ctx->warp_bar[w]->arrive_and_wait();
+  }
+  auto half = [](uint32_t v, int hi) { const uint32_t u = hi ? v & 0xffff0000u : v << 16; float f; std::memcpy(&f, &u, 4); return f; };
+  const int g = l >> 2, t = l & 3;
+  for (int c = 0; c < 4; ++c) {
+    const int row = g + (c >> 1) * 8, col = 2 * t + (c & 1);
+    for (int k = 0; k < 16; ++k) {
+      const int from = (k & 7) >> 1, up = k >> 3;
+      d[c] = std::fma(half(all[(row >> 3) + 2 * up][(row & 7) * 4 + from], k & 1), half(all[4 + up][col * 4 + from], k & 1), d[c]);
+    }
+  }
+}
 inline uint32_t smem_u32(const void* p) { return (uint32_t)(uintptr_t)p; }
 struct ProfScope { ProfScope(int, int, int, int, cudaStream_t) {} };
 }  // namespace lp
