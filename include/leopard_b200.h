@@ -623,6 +623,10 @@ int lp_embed_rows_f32(const int* ids, int R, const void* table, long long ldt, i
 /* y = x / sqrt(mean(x^2) + eps) * gain_scalar (* gain_vec[c]); written to `out` (fp32 or bf16) or added to `accum` (fp32) */
 int lp_rmsnorm_f32(const float* x, long long ldx, int M, int D, float gain_scalar, const float* gain_vec, float eps, void* out,
                    long long ldo, int out_fp32, float* accum, long long ld_accum, void* stream);
+/* x <- x + norm(y) with the first gains, then out = norm(x) with the second ones (the end of a sublayer whose output is normed and the
+ * operand of the next), in one pass; both norms as in lp_rmsnorm_f32 */
+int lp_rmsnorm_add_norm_f32(const float* y, long long ldy, int M, int D, float gain_scalar, const float* gain_vec, float eps, float* x,
+                            long long ldx, float next_scalar, const float* next_vec, void* out, long long ldo, int out_fp32, void* stream);
 /* standalone activation for products that ran on lp_gemm_bf16: mode XIELU, RELU2 (N columns) or SILU_GATE, GELU_GATE, CLAMP_GLU
  * (in has 2N columns: gate | up) */
 int lp_glu_f32(const void* in, long long ldi, int in_fp32, void* out, long long ldo, int out_fp32, int M, int N, int mode, float a,

@@ -45,6 +45,14 @@ __global__ void embed_rows_f32_kernel(const int* __restrict__ ids, int R, const 
   if (id < 0 || id >= vocab) id = 0;   // the host validates ids; this only keeps a bad one inside the table
   const bf16* src = table + (long long)id * ldt;
   float* dst = out + (long long)r * ldo;
+  if (D % 4 == 0 && ldt % 4 == 0 && ldo % 4 == 0 && (reinterpret_cast<uintptr_t>(table) & 7) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+    for (int c = threadIdx.x * 4; c < D; c += blockDim.x * 4) {      // four columns a thread
+      const uint2 u = *reinterpret_cast<const uint2*>(src + c);
+      *reinterpret_cast<float4*>(dst + c) = make_float4(__uint_as_float(u.x << 16) * scale, __uint_as_float(u.x & 0xffff0000u) * scale,
+                                                        __uint_as_float(u.y << 16) * scale, __uint_as_float(u.y & 0xffff0000u) * scale);
+    }
+    return;
+  }
   for (int c = threadIdx.x; c < D; c += blockDim.x) dst[c] = __bfloat162float(src[c]) * scale;
 }
 
@@ -80,33 +88,7 @@ template <> __device__ __forceinline__ float ld32<bf16>(const bf16* p) { return 
 __device__ __forceinline__ void st32(float* p, float v) { *p = v; }
 __device__ __forceinline__ void st32(bf16* p, float v) { *p = __float2bfloat16(v); }
 
-// mode LP_EPI_XIELU: out[m, n] = xielu(in[m, n]); LP_EPI_SILU_GATE, LP_EPI_GELU_GATE:
-// out[m, n] = silu | gelu (in[m, n]) * in[m, n + N]; LP_EPI_CLAMP_GLU: the
-// clamped gated unit of lp_linear on (in[m, n], in[m, n + N]) with limit a and slope b.  row_scale multiplies what is read.
-template <typename IT, typename OT>
-__global__ void glu_kernel(const IT* __restrict__ in, long long ldi, OT* __restrict__ out, long long ldo, int M, int N, int mode, float a,
-                           float b, const float* __restrict__ row_scale) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)M * N) return;
-  const int m = (int)(i / N), n = (int)(i % N);
-  const float rs = row_scale != nullptr ? row_scale[m] : 1.0f;
-  const float z = ld32<IT>(in + (long long)m * ldi + n) * rs;
-  float v;
-  if (mode == LP_EPI_SILU_GATE) v = z / (1.0f + expf(-z)) * (ld32<IT>(in + (long long)m * ldi + n + N) * rs);
-  else if (mode == LP_EPI_GELU_GATE) {      // tanh form: 1/2 (1 + tanh t) = sigmoid(2 t) with t = sqrt(2 / pi) (z + 0.044715 z^3)
-    const float t = 0.7978845608028654f * fmaf(0.044715f * z * z, z, z);
-    v = z / (1.0f + expf(-2.0f * t)) * (ld32<IT>(in + (long long)m * ldi + n + N) * rs);
-  }
-  else if (mode == LP_EPI_CLAMP_GLU) {
-    const float g = fminf(z, a), u = fminf(fmaxf(ld32<IT>(in + (long long)m * ldi + n + N) * rs, -a), a);
-    v = g / (1.0f + expf(-b * g)) * (u + 1.0f);
-  }
-  else if (mode == LP_EPI_RELU2) v = fmaxf(z, 0.f) * fmaxf(z, 0.f);
-  else v = z > 0.f ? a * z * z + 0.5f * z : b * (expm1f(z) - z) + 0.5f * z;
-  st32(out + (long long)m * ldo + n, v);
-}
-
-// The three elementwise kernels below work on groups of V consecutive columns per thread: V = 4 (16-byte fp32 accesses, 8-byte bf16
+// The elementwise kernels work on groups of V consecutive columns per thread: V = 4 (16-byte fp32 accesses, 8-byte bf16
 // stores) when the width and every row stride and base allow it, else V = 1.
 template <int V> struct f32vec;
 template <> struct f32vec<1> { float v[1]; };
@@ -124,6 +106,137 @@ template <int V> __device__ __forceinline__ void stv(bf16* p, const f32vec<V>& x
     *p = __float2bfloat16(x.v[0]);
   }
 }
+
+// A CTA per row, the row in registers (VN groups of four columns a thread): it is read once, all its loads in flight together.
+// Optionally a second norm follows: the first one's result is added to `accum` and the sum is normed again with gains of its own into
+// `next` — the end of one sublayer and the start of the next in one pass over the stream.  A row of 4096 (a decode step) took 16.6 us with a
+// warp a row, 2.5 us with a CTA; 4096 rows of 2048 are bound by their bytes (11.6 us, 9.9 us; the pair of norms 15.4 us instead of 2 x 11.6).
+constexpr int NORM_ROW_MAX = 8192;
+struct NormNext { float gain_scalar; const float* gain_vec; float* out_f32; bf16* out_bf16; long long ldo; };
+__device__ __forceinline__ float block_sum(float v, float* red) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane == 0) red[warp] = v;
+  __syncthreads();
+  v = lane < n_warps ? red[lane] : 0.f;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+template <int VN>
+__global__ void __launch_bounds__(1024)
+rmsnorm_row_kernel(const float* __restrict__ x, long long ldx, int D, float gain_scalar, const float* __restrict__ gain_vec, float eps,
+                   float* __restrict__ out_f32, bf16* __restrict__ out_bf16, long long ldo, float* __restrict__ accum, long long lda,
+                   NormNext next) {
+  __shared__ float red[2][32];
+  const long long row = blockIdx.x;
+  f32vec<4> v[VN], y[VN];
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < VN; ++i) {
+    const int c = (threadIdx.x + i * blockDim.x) * 4;
+    if (c < D) {
+      v[i] = ldv<4>(x + row * ldx + c);
+      if (accum != nullptr) y[i] = ldv<4>(accum + row * lda + c);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) ss = fmaf(v[i].v[k], v[i].v[k], ss);
+    }
+  }
+  const float r = 1.0f / sqrtf(block_sum(ss, red[0]) / (float)D + eps);
+  float s2 = 0.f;
+#pragma unroll
+  for (int i = 0; i < VN; ++i) {
+    const int c = (threadIdx.x + i * blockDim.x) * 4;
+    if (c < D) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[i].v[k] = v[i].v[k] * r * gain_scalar;
+      if (gain_vec != nullptr) {
+        const f32vec<4> g = ldv<4>(gain_vec + c);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[i].v[k] *= g.v[k];
+      }
+      if (accum != nullptr) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          y[i].v[k] += v[i].v[k];
+          s2 = fmaf(y[i].v[k], y[i].v[k], s2);
+        }
+        stv<4>(accum + row * lda + c, y[i]);
+      } else if (out_f32 != nullptr) {
+        stv<4>(out_f32 + row * ldo + c, v[i]);
+      } else {
+        stv<4>(out_bf16 + row * ldo + c, v[i]);
+      }
+    }
+  }
+  if (next.out_f32 == nullptr && next.out_bf16 == nullptr) return;      // the same for the whole grid
+  const float q = 1.0f / sqrtf(block_sum(s2, red[1]) / (float)D + eps);
+#pragma unroll
+  for (int i = 0; i < VN; ++i) {
+    const int c = (threadIdx.x + i * blockDim.x) * 4;
+    if (c < D) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) y[i].v[k] = y[i].v[k] * q * next.gain_scalar;
+      if (next.gain_vec != nullptr) {
+        const f32vec<4> g = ldv<4>(next.gain_vec + c);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) y[i].v[k] *= g.v[k];
+      }
+      if (next.out_f32 != nullptr) stv<4>(next.out_f32 + row * next.ldo + c, y[i]);
+      else stv<4>(next.out_bf16 + row * next.ldo + c, y[i]);
+    }
+  }
+}
+
+
+template <int V> __device__ __forceinline__ f32vec<V> ldv(const bf16* p) {
+  f32vec<V> r;
+  if constexpr (V == 4) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    r.v[0] = __uint_as_float(u.x << 16); r.v[1] = __uint_as_float(u.x & 0xffff0000u);
+    r.v[2] = __uint_as_float(u.y << 16); r.v[3] = __uint_as_float(u.y & 0xffff0000u);
+  } else {
+    r.v[0] = __bfloat162float(*p);
+  }
+  return r;
+}
+
+__device__ __forceinline__ float glu_one(int mode, float z, float u, float a, float b) {
+  if (mode == LP_EPI_SILU_GATE) return z / (1.0f + expf(-z)) * u;
+  if (mode == LP_EPI_GELU_GATE) {      // tanh form: 1/2 (1 + tanh t) = sigmoid(2 t) with t = sqrt(2 / pi) (z + 0.044715 z^3)
+    const float t = 0.7978845608028654f * fmaf(0.044715f * z * z, z, z);
+    return z / (1.0f + expf(-2.0f * t)) * u;
+  }
+  if (mode == LP_EPI_CLAMP_GLU) {
+    const float g = fminf(z, a), c = fminf(fmaxf(u, -a), a);
+    return g / (1.0f + expf(-b * g)) * (c + 1.0f);
+  }
+  if (mode == LP_EPI_RELU2) return fmaxf(z, 0.f) * fmaxf(z, 0.f);
+  return z > 0.f ? a * z * z + 0.5f * z : b * (expm1f(z) - z) + 0.5f * z;
+}
+
+// mode LP_EPI_XIELU: out[m, n] = xielu(in[m, n]); LP_EPI_SILU_GATE, LP_EPI_GELU_GATE:
+// out[m, n] = silu | gelu (in[m, n]) * in[m, n + N]; LP_EPI_CLAMP_GLU: the
+// clamped gated unit of lp_linear on (in[m, n], in[m, n + N]) with limit a and slope b.  row_scale multiplies what is read.
+// Bound by its bytes: 4096 x 8192 fp32 -> bf16 130 us with a column a thread (and a 64-bit division each), 41 us = 4.9 TB/s with four (relu2).
+template <typename IT, typename OT, int V>
+__global__ void glu_kernel(const IT* __restrict__ in, long long ldi, OT* __restrict__ out, long long ldo, int M, int N, int mode, float a,
+                           float b, const float* __restrict__ row_scale) {
+  const int n = (int)(blockIdx.x * blockDim.x + threadIdx.x) * V;
+  if (n >= N) return;
+  const bool pair = mode == LP_EPI_SILU_GATE || mode == LP_EPI_GELU_GATE || mode == LP_EPI_CLAMP_GLU;
+  for (int m = blockIdx.y; m < M; m += gridDim.y) {
+    const float rs = row_scale != nullptr ? row_scale[m] : 1.0f;
+    const f32vec<V> z = ldv<V>(in + (long long)m * ldi + n);
+    f32vec<V> u = z, v;
+    if (pair) u = ldv<V>(in + (long long)m * ldi + n + N);
+#pragma unroll
+    for (int i = 0; i < V; ++i) v.v[i] = glu_one(mode, z.v[i] * rs, u.v[i] * rs, a, b);
+    stv<V>(out + (long long)m * ldo + n, v);
+  }
+}
+
 
 // a warp per row; the lanes take groups of V consecutive columns (V = 4: 16-byte reads of the row and of its gate)
 template <typename OT, int V>
@@ -243,11 +356,20 @@ static bool vec4_ok(int N, std::initializer_list<const void*> bases, std::initia
   return true;
 }
 
+// a CTA of 256 threads to so many groups of columns, rows in the grid's second dimension (and in turns beyond its limit)
+static dim3 rows_grid(int groups, int M) { return dim3((unsigned)((groups + 255) / 256), (unsigned)(M < 65535 ? M : 65535)); }
+
+template <int V>
 __global__ void axpy_f32_kernel(float* __restrict__ y, long long ldy, const float* __restrict__ x, long long ldx, float alpha, int M, int N) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)M * N) return;
-  const int m = (int)(i / N), n = (int)(i % N);
-  y[(long long)m * ldy + n] = fmaf(alpha, x[(long long)m * ldx + n], y[(long long)m * ldy + n]);
+  const int n = (int)(blockIdx.x * blockDim.x + threadIdx.x) * V;
+  if (n >= N) return;
+  for (int m = blockIdx.y; m < M; m += gridDim.y) {
+    f32vec<V> acc = ldv<V>(y + (long long)m * ldy + n);
+    const f32vec<V> v = ldv<V>(x + (long long)m * ldx + n);
+#pragma unroll
+    for (int i = 0; i < V; ++i) acc.v[i] = fmaf(alpha, v.v[i], acc.v[i]);
+    stv<V>(y + (long long)m * ldy + n, acc);
+  }
 }
 
 // pair i of a row: (sin, cos) of position * frequency i; an odd width leaves the last sine without its cosine.  The frequency comes as
@@ -869,7 +991,36 @@ extern "C" int lp_embed_rows_f32(const int* ids, int R, const void* table, long 
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LP_REQUIRE(ids != nullptr && table != nullptr && out != nullptr && R >= 0 && D > 0 && vocab > 0, "lp_embed_rows_f32: bad arguments");
   if (R == 0) return 0;
-  embed_rows_f32_kernel<<<R, 128, 0, stream>>>(ids, R, reinterpret_cast<const bf16*>(table), ldt, vocab, scale, out, ldo, D);
+  embed_rows_f32_kernel<<<R, 512, 0, stream>>>(ids, R, reinterpret_cast<const bf16*>(table), ldt, vocab, scale, out, ldo, D);
+  note_launch();
+  LP_CHECK_CUDA(cudaGetLastError());
+  return 0;
+}
+
+static int launch_rmsnorm(const float* x, long long ldx, int M, int D, float gain_scalar, const float* gain_vec, float eps, void* out,
+                          long long ldo, int out_fp32, float* accum, long long ld_accum, const NormNext& next, cudaStream_t stream) {
+  float* of = (out != nullptr && out_fp32) ? reinterpret_cast<float*>(out) : nullptr;
+  bf16* ob = (out != nullptr && !out_fp32) ? reinterpret_cast<bf16*>(out) : nullptr;
+  const bool second = next.out_f32 != nullptr || next.out_bf16 != nullptr;
+  if (D <= NORM_ROW_MAX && vec4_ok(D, {x, gain_vec, out, accum, next.gain_vec, next.out_f32, next.out_bf16},
+                                   {ldx, out != nullptr ? ldo : 0, accum != nullptr ? ld_accum : 0, second ? next.ldo : 0})) {
+    // few rows: one group a thread, as many warps as that takes; many rows: two groups, CTAs of half the size
+    const int groups = D / 4;
+    if (groups <= 1024 && M <= 4 * sm_count())
+      rmsnorm_row_kernel<1><<<M, (groups + 31) / 32 * 32, 0, stream>>>(x, ldx, D, gain_scalar, gain_vec, eps, of, ob, ldo, accum, ld_accum, next);
+    else
+      rmsnorm_row_kernel<2><<<M, (groups + 63) / 64 * 32, 0, stream>>>(x, ldx, D, gain_scalar, gain_vec, eps, of, ob, ldo, accum, ld_accum, next);
+    note_launch();
+    LP_CHECK_CUDA(cudaGetLastError());
+    return 0;
+  }
+  const unsigned grid = (unsigned)((M + NORM32_WARPS - 1) / NORM32_WARPS);
+  rmsnorm_f32_kernel<<<grid, NORM32_WARPS * 32, 0, stream>>>(x, ldx, M, D, gain_scalar, gain_vec, eps, of, ob, ldo, accum, ld_accum);
+  if (second) {
+    rmsnorm_f32_kernel<<<grid, NORM32_WARPS * 32, 0, stream>>>(accum, ld_accum, M, D, next.gain_scalar, next.gain_vec, eps, next.out_f32,
+                                                               next.out_bf16, next.ldo, nullptr, 0);
+    note_launch();
+  }
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
@@ -877,16 +1028,21 @@ extern "C" int lp_embed_rows_f32(const int* ids, int R, const void* table, long 
 
 extern "C" int lp_rmsnorm_f32(const float* x, long long ldx, int M, int D, float gain_scalar, const float* gain_vec, float eps, void* out,
                               long long ldo, int out_fp32, float* accum, long long ld_accum, void* stream_) {
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LP_REQUIRE(x != nullptr && M >= 0 && D > 0, "lp_rmsnorm_f32: bad arguments");
   LP_REQUIRE((out != nullptr) != (accum != nullptr), "lp_rmsnorm_f32: give either `out` or `accum`");
   if (M == 0) return 0;
-  rmsnorm_f32_kernel<<<(M + NORM32_WARPS - 1) / NORM32_WARPS, NORM32_WARPS * 32, 0, stream>>>(
-      x, ldx, M, D, gain_scalar, gain_vec, eps, (out != nullptr && out_fp32) ? reinterpret_cast<float*>(out) : nullptr,
-      (out != nullptr && !out_fp32) ? reinterpret_cast<bf16*>(out) : nullptr, ldo, accum, ld_accum);
-  note_launch();
-  LP_CHECK_CUDA(cudaGetLastError());
-  return 0;
+  return launch_rmsnorm(x, ldx, M, D, gain_scalar, gain_vec, eps, out, ldo, out_fp32, accum, ld_accum, NormNext{0.f, nullptr, nullptr, nullptr, 0},
+                        reinterpret_cast<cudaStream_t>(stream_));
+}
+
+extern "C" int lp_rmsnorm_add_norm_f32(const float* y, long long ldy, int M, int D, float gain_scalar, const float* gain_vec, float eps,
+                                       float* x, long long ldx, float next_scalar, const float* next_vec, void* out, long long ldo,
+                                       int out_fp32, void* stream_) {
+  LP_REQUIRE(y != nullptr && x != nullptr && out != nullptr && y != x && M >= 0 && D > 0, "lp_rmsnorm_add_norm_f32: bad arguments");
+  if (M == 0) return 0;
+  return launch_rmsnorm(y, ldy, M, D, gain_scalar, gain_vec, eps, nullptr, 0, 0, x, ldx,
+                        NormNext{next_scalar, next_vec, out_fp32 ? reinterpret_cast<float*>(out) : nullptr,
+                                 out_fp32 ? nullptr : reinterpret_cast<bf16*>(out), ldo}, reinterpret_cast<cudaStream_t>(stream_));
 }
 
 extern "C" int lp_glu_f32(const void* in, long long ldi, int in_fp32, void* out, long long ldo, int out_fp32, int M, int N, int mode,
@@ -902,15 +1058,19 @@ extern "C" int lp_glu_scaled_f32(const void* in, long long ldi, int in_fp32, voi
                  mode == LP_EPI_GELU_GATE,
              "lp_glu_f32: mode %d is not an activation", mode);
   if (M == 0) return 0;
-  const unsigned grid = (unsigned)(((long long)M * N + 255) / 256);
-  if (in_fp32 && out_fp32)
-    glu_kernel<float, float><<<grid, 256, 0, stream>>>(reinterpret_cast<const float*>(in), ldi, reinterpret_cast<float*>(out), ldo, M, N, mode, a, b, row_scale);
-  else if (in_fp32)
-    glu_kernel<float, bf16><<<grid, 256, 0, stream>>>(reinterpret_cast<const float*>(in), ldi, reinterpret_cast<bf16*>(out), ldo, M, N, mode, a, b, row_scale);
-  else if (out_fp32)
-    glu_kernel<bf16, float><<<grid, 256, 0, stream>>>(reinterpret_cast<const bf16*>(in), ldi, reinterpret_cast<float*>(out), ldo, M, N, mode, a, b, row_scale);
-  else
-    glu_kernel<bf16, bf16><<<grid, 256, 0, stream>>>(reinterpret_cast<const bf16*>(in), ldi, reinterpret_cast<bf16*>(out), ldo, M, N, mode, a, b, row_scale);
+  // bf16 rows of four are 8 bytes: their bases need 8-byte alignment, which the 16-byte test covers
+  const bool v4 = vec4_ok(N, {in, out}, {ldi, ldo});
+  const dim3 grid = rows_grid(v4 ? N / 4 : N, M);
+#define LP_GLU(IT, OT)                                                                                                                        \
+  do {                                                                                                                                        \
+    if (v4) glu_kernel<IT, OT, 4><<<grid, 256, 0, stream>>>(reinterpret_cast<const IT*>(in), ldi, reinterpret_cast<OT*>(out), ldo, M, N, mode, a, b, row_scale); \
+    else glu_kernel<IT, OT, 1><<<grid, 256, 0, stream>>>(reinterpret_cast<const IT*>(in), ldi, reinterpret_cast<OT*>(out), ldo, M, N, mode, a, b, row_scale);    \
+  } while (0)
+  if (in_fp32 && out_fp32) LP_GLU(float, float);
+  else if (in_fp32) LP_GLU(float, bf16);
+  else if (out_fp32) LP_GLU(bf16, float);
+  else LP_GLU(bf16, bf16);
+#undef LP_GLU
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
@@ -997,7 +1157,10 @@ extern "C" int lp_axpy_f32(float* y, long long ldy, const float* x, long long ld
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LP_REQUIRE(y != nullptr && x != nullptr && M >= 0 && N > 0, "lp_axpy_f32: bad arguments");
   if (M == 0) return 0;
-  axpy_f32_kernel<<<(unsigned)(((long long)M * N + 255) / 256), 256, 0, stream>>>(y, ldy, x, ldx, alpha, M, N);
+  const bool v4 = vec4_ok(N, {y, x}, {ldy, ldx});
+  const dim3 grid = rows_grid(v4 ? N / 4 : N, M);
+  if (v4) axpy_f32_kernel<4><<<grid, 256, 0, stream>>>(y, ldy, x, ldx, alpha, M, N);
+  else axpy_f32_kernel<1><<<grid, 256, 0, stream>>>(y, ldy, x, ldx, alpha, M, N);
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;

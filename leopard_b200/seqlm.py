@@ -969,6 +969,17 @@ class SeqLMEngine:
         self._check(rc, "lp_rmsnorm_f32")
         return out
 
+    def add_and_norm(self, y: torch.Tensor, gain, x: torch.Tensor, next_gain) -> torch.Tensor:
+        """x <- x + norm(y) and, in the same pass, the operand norm(x) of the sublayer that follows"""
+        M, D = x.shape
+        out = self._empty((M, D), self.act)
+        scalar, vector = (1.0, gain) if isinstance(gain, torch.Tensor) else (gain, None)
+        scalar2, vector2 = (1.0, next_gain) if isinstance(next_gain, torch.Tensor) else (next_gain, None)
+        rc = self.L.lp_rmsnorm_add_norm_f32(_lib.ptr(y), y.stride(0), M, D, scalar, _lib.ptr(vector), self.cfg.eps, _lib.ptr(x), x.stride(0),
+                                            scalar2, _lib.ptr(vector2), _lib.ptr(out), out.stride(0), int(out.dtype == F32), self._stream())
+        self._check(rc, "lp_rmsnorm_add_norm_f32")
+        return out
+
     def dyt(self, x: torch.Tensor, first, second=None):
         """Dynamic Tanh of the same rows with one or two parameter sets (alpha, gain, shift): the operands of a layer's sublayers"""
         M, D = x.shape
@@ -1486,6 +1497,13 @@ class SeqLMEngine:
         if cfg.norm == "post":
             return self._forward_post(b, want, x)
         pre = cfg.norm in ("pre", "pre_plain")
+
+        def reads_norm(lj):      # the mixer of layer lj reads norm(x) in the operand dtype, x as the layer before it left it
+            if lj >= len(cfg.layers) or self.tap is not None or self.w.add_before[lj] is not None:
+                return False
+            nc = cfg.layers[lj]
+            return not (nc.token_shift or nc.input_conv or isinstance(nc.mixer, WKVConfig))
+        h = None      # the next sublayer's operand, when the end of the one before has made it
         for li, (lc, lw) in enumerate(zip(cfg.layers, self.w.layers)):
             if self.w.add_before[li] is not None:
                 rc = self.L.lp_add_row_f32(_lib.ptr(x), x.stride(0), _lib.ptr(self.w.add_before[li]), b.R, D, self._stream())
@@ -1500,23 +1518,33 @@ class SeqLMEngine:
                 self._check(rc, "lp_token_shift_f32")
                 if lc.input_conv:
                     h = self.convolved(h, li, "conv1", b)
-            else:
+            elif h is None:
                 h = self.operand(x, lw["norm1"], li, "conv1", b)
+            h_in, h = h, None
             if pre:        # x <- x + m * mixer(norm(x)): the update is the store of the mixer's output product
-                self._mix(li, lc.mixer, lw, h, b, into=(x, cfg.residual_mult))
+                self._mix(li, lc.mixer, lw, h_in, b, into=(x, cfg.residual_mult))
             else:
-                self.norm(self._mix(li, lc.mixer, lw, h, b), lw["norm1b"], accum=x)
+                y = self._mix(li, lc.mixer, lw, h_in, b)
+                if lc.ff is not None and not lc.input_conv:
+                    h = self.add_and_norm(y, lw["norm1b"], x, lw["norm2"])
+                elif lc.ff is None and reads_norm(li + 1):
+                    h = self.add_and_norm(y, lw["norm1b"], x, self.w.layers[li + 1]["norm1"])
+                else:
+                    self.norm(y, lw["norm1b"], accum=x)
             if lc.ff is not None:
-                h = self.operand(x, lw["norm2"], li, "conv2", b)
+                h_in, h = h if h is not None else self.operand(x, lw["norm2"], li, "conv2", b), None
                 if pre and isinstance(lc.ff, DenseFFConfig):
-                    self._dense(lc.ff, lw, h, into=(x, cfg.residual_mult))
+                    self._dense(lc.ff, lw, h_in, into=(x, cfg.residual_mult))
                 elif pre:
-                    y = self._moe(lc.ff, lw, h)
+                    y = self._moe(lc.ff, lw, h_in)
                     rc = self.L.lp_axpy_f32(_lib.ptr(x), x.stride(0), _lib.ptr(y), y.stride(0), cfg.residual_mult, b.R, D, self._stream())
                     self._check(rc, "lp_axpy_f32")
                 else:
-                    y = self._dense(lc.ff, lw, h) if isinstance(lc.ff, DenseFFConfig) else self._moe(lc.ff, lw, h)
-                    self.norm(y, lw["norm2b"], accum=x)
+                    y = self._dense(lc.ff, lw, h_in) if isinstance(lc.ff, DenseFFConfig) else self._moe(lc.ff, lw, h_in)
+                    if reads_norm(li + 1):
+                        h = self.add_and_norm(y, lw["norm2b"], x, self.w.layers[li + 1]["norm1"])
+                    else:
+                        self.norm(y, lw["norm2b"], accum=x)
             if self.tap is not None:
                 self.tap(li, x)
         if want is None:
