@@ -57,7 +57,7 @@ __device__ __forceinline__ uint4 ldg_once(const void* p) {
 // a rows g, g + 8 at columns 2t, 2t + 1 (a0, a1) and 8 + 2t, 9 + 2t (a2, a3), b column g at the same rows (b0, b1), and holds
 // d[g, 2t], d[g, 2t + 1], d[g + 8, 2t], d[g + 8, 2t + 1].
 __device__ __forceinline__ void mma_bf16(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }

@@ -395,13 +395,15 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
       const int m = m0 + 8 * i + g;
       x[i] = m < rows ? A + (long long)(pairs ? pair_of[m] / a.a_div : m) * a.lda : nullptr;
     }
-    float acc[NT][MG][4];
+    constexpr bool LONG = MG == 8 && sizeof(AT) == 2;      // many rows: chains of eight steps, the additions would cost more than the products
+    float acc[NT][MG][4], run[LONG ? NT : 1][LONG ? MG : 1][4];
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
       for (int i = 0; i < MG; ++i)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[j][i][c] = 0.f;
+        for (int c = 0; c < 4; ++c) acc[j][i][c] = run[LONG ? j : 0][LONG ? i : 0][c] = 0.f;
+    int turn = 0;
     for (int s = warp; s * 32 < a.K; s += U * n_warps) {
       uint4 u0[U][NT], u1[U][NT];
 #pragma unroll
@@ -424,10 +426,14 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
           for (int i = 0; i < MG; ++i)
 #pragma unroll
             for (int j = 0; j < NT; ++j) {
-              float d[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
-              mma_step(d, e, u0[u][j], u1[u][j], v[i]);
+              if constexpr (LONG) {
+                mma_step(run[j][i], run[j][i], u0[u][j], u1[u][j], v[i]);
+              } else {
+                float d[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
+                mma_step(d, e, u0[u][j], u1[u][j], v[i]);
 #pragma unroll
-              for (int c = 0; c < 4; ++c) acc[j][i][c] += d[c] + e[c];
+                for (int c = 0; c < 4; ++c) acc[j][i][c] += d[c] + e[c];
+              }
             }
         } else {
 #pragma unroll
@@ -450,6 +456,27 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
           }
         }
       }
+      if constexpr (LONG) {
+        if ((++turn & 7) == 0) {
+#pragma unroll
+          for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int i = 0; i < MG; ++i)
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                acc[j][i][c] += run[j][i][c];
+                run[j][i][c] = 0.f;
+              }
+        }
+      }
+    }
+    if constexpr (LONG) {
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int i = 0; i < MG; ++i)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[j][i][c] += run[j][i][c];
     }
     if (m0 > 0) __syncthreads();      // the sums of the rows before have been read
 #pragma unroll
@@ -525,11 +552,175 @@ static int dispatch_stream(const LinArgs& a, int a_fp32, int c_fp32, int batch, 
   // a short K has no work for more warps; a grid of few CTAs wants more loads in flight in each (N = 2048, K = 8192: 15 us with 16 warps, 11 with 32)
   int warps = a.K <= 256 ? 4 : !a_fp32 && mg * nt == 1 && ctas <= sm_count() && a.K >= 4096 ? 32 : ctas <= 2 * sm_count() && a.K >= 1024 && mg <= 4 ? 16 : 8;
   dim3 grid((n_out + nt * per - 1) / (nt * per), n_groups > 0 ? n_groups : 1, n_groups > 0 ? 1 : batch);
-#define LP_STREAM(MG)                                                                                                              \
+#define LP_STREAM(MG)                                                                                                               \
   (a_fp32 ? (nt == 2 ? launch_stream<float, 2, MG>(a, c_fp32, grid, warps, n_pairs, stream) : launch_stream<float, 1, MG>(a, c_fp32, grid, warps, n_pairs, stream)) \
-          : (nt == 2 ? launch_stream<bf16, 2, MG>(a, c_fp32, grid, warps, n_pairs, stream) : launch_stream<bf16, 1, MG>(a, c_fp32, grid, warps, n_pairs, stream)))
+          : launch_stream<bf16, 1, MG>(a, c_fp32, grid, warps, n_pairs, stream))
+  if (!a_fp32 && nt == 2) return launch_stream<bf16, 2, 1>(a, c_fp32, grid, warps, n_pairs, stream);      // nt == 2 means mg == 1
   return mg == 1 ? LP_STREAM(1) : mg == 2 ? LP_STREAM(2) : mg == 4 ? LP_STREAM(4) : LP_STREAM(8);
 #undef LP_STREAM
+}
+
+// ---------------------------------------------------------------------------------------------------------------------------------
+// More rows: 64 x 128 output tiles, K in steps of 32 through two shared-memory buffers, two CTAs an SM (one's loads and cuts run beside the
+// other's products: 128-row tiles with one CTA of 16 warps were 15 % slower), a warp to 32 x 32 outputs on the same matrix instruction.  fp32 rows are cut into their three bf16 terms once, on the way
+// into shared memory (a plane each), so the inner loop is loads and products only; the next step's global loads are in flight meanwhile.
+// A lane reads 16 bytes of a row, eight k, the same permutation of k on both sides; rows are 64 bytes apart, so eight lanes read two
+// whole rows: no two of them in the same bank.  Chains as above: each step's products form sums of their own, added in fp32.
+// The gated units interleave gate and up rows in groups of eight, so both halves of an output are neighbours in one lane.
+// Measured (B200, M = 4096, N = 8192, K = 2048): fp32 rows 1.47 ms = 93 TFLOP/s (three products each; 64 x 64 tiles on fp32 FMAs 5.4 ms, 25),
+// bf16 rows 0.72 ms; mma.sync alone reaches 520 TFLOP/s of bf16 products here, 450 with a sum of its own every few.  Error against 64 bits at
+// K = 1024 / 4096: 1.2e-7 / 2.1e-7 (FMA chains over K: 5.7e-7 / 1.1e-6).
+constexpr int MT_BM = LIN_BM, MT_BN = 128, MT_BK = 32, MT_LDC = MT_BN + 4, MT_THREADS = 256;
+
+template <typename AT>
+__global__ void __launch_bounds__(MT_THREADS, 2) linear_mma_kernel(LinArgs a, int gated, int c_fp32) {
+  extern __shared__ float dyn_smem[];
+  constexpr int PLANES = sizeof(AT) == 4 ? 3 : 1;
+  constexpr int BM = MT_BM, A_WORDS = BM * MT_BK / 2, W_WORDS = MT_BN * MT_BK / 2, STAGE = PLANES * A_WORDS + W_WORDS;      // 32-bit words
+  constexpr int THREADS = MT_THREADS, WARPS_N = 4, NI = MT_BN / WARPS_N / 8;
+  constexpr int A_CHUNKS = BM * 4 / THREADS, W_CHUNKS = MT_BN * 4 / THREADS;      // 16-byte (eight k) pieces a thread brings
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int z = blockIdx.z, m0 = blockIdx.y * BM, n_out = gated ? a.N / 2 : a.N;
+  const int cols = gated ? MT_BN / 2 : MT_BN, n0 = blockIdx.x * cols;
+  int group = 0;
+  if (a.tile_group != nullptr) {
+    group = a.tile_group[blockIdx.y];
+    if (group < 0) return;
+  }
+  const AT* A = reinterpret_cast<const AT*>(a.A) + (long long)z * a.a_batch + lin_seg(a, n0);
+  const bf16* W = a.W + (long long)(z + group) * a.w_batch;
+  uint32_t* smem = reinterpret_cast<uint32_t*>(dyn_smem);
+  const AT* a_src[A_CHUNKS];
+  const bf16* w_src[W_CHUNKS];
+#pragma unroll
+  for (int i = 0; i < A_CHUNKS; ++i) {
+    const int m = m0 + (tid + i * THREADS) / 4;
+    const long long r = m >= a.M ? -1 : a.a_rows != nullptr ? a.a_rows[m] : m;
+    a_src[i] = r < 0 ? nullptr : A + r * a.lda;
+  }
+#pragma unroll
+  for (int i = 0; i < W_CHUNKS; ++i) {
+    const int j = (tid + i * THREADS) / 4;
+    const int n = gated ? n0 + (j >> 4) * 8 + (j & 7) : n0 + j;
+    w_src[i] = n >= n_out ? nullptr : W + (long long)(gated && (j & 8) ? n + n_out : n) * a.ldw;
+  }
+  const int kc = (tid & 3) * 8;      // this thread's eight k of a step
+  const uint4 none = make_uint4(0, 0, 0, 0);
+  uint4 ra[A_CHUNKS][sizeof(AT) / 2], rw[W_CHUNKS];
+  auto fetch = [&](int k0) {
+    const bool in = k0 + kc < a.K;
+#pragma unroll
+    for (int i = 0; i < A_CHUNKS; ++i)
+#pragma unroll
+      for (int h = 0; h < (int)sizeof(AT) / 2; ++h)
+        ra[i][h] = in && a_src[i] != nullptr ? *(reinterpret_cast<const uint4*>(a_src[i] + k0 + kc) + h) : none;
+#pragma unroll
+    for (int i = 0; i < W_CHUNKS; ++i) rw[i] = in && w_src[i] != nullptr ? *reinterpret_cast<const uint4*>(w_src[i] + k0 + kc) : none;
+  };
+  auto put = [&](int buf) {
+    uint32_t* st = smem + buf * STAGE;
+#pragma unroll
+    for (int i = 0; i < A_CHUNKS; ++i) {
+      uint4* dst = reinterpret_cast<uint4*>(st + (tid + i * THREADS) * 4);
+      if constexpr (PLANES == 3) {
+        const uint4 p = ra[i][0], q = ra[i][1];
+        const Bf16Terms v = split3(make_float4(__uint_as_float(p.x), __uint_as_float(p.y), __uint_as_float(p.z), __uint_as_float(p.w)),
+                                   make_float4(__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z), __uint_as_float(q.w)));
+        dst[0] = v.hi;
+        dst[A_WORDS / 4] = v.mid;
+        dst[2 * (A_WORDS / 4)] = v.lo;
+      } else {
+        dst[0] = ra[i][0];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < W_CHUNKS; ++i) *reinterpret_cast<uint4*>(st + PLANES * A_WORDS + (tid + i * THREADS) * 4) = rw[i];
+  };
+  const int wm = (warp / WARPS_N) * 32, wn = (warp % WARPS_N) * NI * 8;
+  float acc[2][NI][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < NI; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[i][j][c] = 0.f;
+  fetch(0);
+  put(0);
+  __syncthreads();
+  const int steps = (a.K + MT_BK - 1) / MT_BK;
+  for (int s = 0; s < steps; ++s) {
+    if (s + 1 < steps) fetch((s + 1) * MT_BK);
+    const uint32_t* st = smem + (s & 1) * STAGE;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      uint4 x0[PLANES], x1[PLANES];
+#pragma unroll
+      for (int p = 0; p < PLANES; ++p) {
+        x0[p] = *reinterpret_cast<const uint4*>(st + p * A_WORDS + (wm + 16 * i + g) * 16 + t * 4);
+        x1[p] = *reinterpret_cast<const uint4*>(st + p * A_WORDS + (wm + 16 * i + g + 8) * 16 + t * 4);
+      }
+#pragma unroll
+      for (int j = 0; j < NI; ++j) {
+        const uint4 w = *reinterpret_cast<const uint4*>(st + PLANES * A_WORDS + (wn + 8 * j + g) * 16 + t * 4);
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int p = PLANES - 1; p >= 0; --p) {      // the small terms first
+          mma_bf16(d, x0[p].x, x1[p].x, x0[p].y, x1[p].y, w.x, w.y);
+          mma_bf16(d, x0[p].z, x1[p].z, x0[p].w, x1[p].w, w.z, w.w);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[i][j][c] += d[c];
+      }
+    }
+    if (s + 1 < steps) put((s + 1) & 1);
+    __syncthreads();
+  }
+  // through shared memory, so that one copy of the epilogue's code serves whole rows (the stages are no longer read)
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < NI; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) dyn_smem[(wm + 16 * i + g + 8 * (c >> 1)) * MT_LDC + wn + 8 * j + 2 * t + (c & 1)] = acc[i][j][c];
+  __syncthreads();
+#pragma unroll 1
+  for (int e = tid; e < BM * cols; e += THREADS) {
+    const int ml = e / cols, nl = e % cols, m = m0 + ml, n = n0 + nl;
+    if (m >= a.M || n >= n_out) continue;
+    const int at = ml * MT_LDC + (gated ? (nl >> 3) * 16 + (nl & 7) : nl);
+    float s = dyn_smem[at], s2 = gated ? dyn_smem[at + 8] : 0.f;
+    if (a.row_scale != nullptr) {
+      s *= a.row_scale[m];
+      s2 *= a.row_scale[m];
+    }
+    if (a.bias != nullptr) {
+      s += a.bias[n];
+      if (gated) s2 += a.bias[n + n_out];
+    }
+    float v = gated ? lin_gate(a.epi, s, s2, a.e0, a.e1) : lin_epi(a.epi, s, a.e0, a.e1);
+    if (a.gate != nullptr) v /= 1.0f + expf(-a.gate[(long long)z * a.gate_batch + (long long)m * a.ldg + n]);
+    const long long at_c = (long long)z * a.c_batch + (long long)m * a.ldc + n;
+    if (c_fp32) {
+      float* C = reinterpret_cast<float*>(a.C) + at_c;
+      *C = a.c_accum ? fmaf(a.c_scale, v, *C) : v;
+    } else {
+      bf16* C = reinterpret_cast<bf16*>(a.C) + at_c;
+      *C = __float2bfloat16(a.c_accum ? fmaf(a.c_scale, v, __bfloat162float(*C)) : v);
+    }
+  }
+}
+
+template <typename AT>
+static int launch_mma(const LinArgs& a, int c_fp32, int batch, int m_tiles, cudaStream_t stream) {
+  constexpr size_t stages = 2 * sizeof(uint32_t) * ((sizeof(AT) == 4 ? 3 : 1) * MT_BM * MT_BK / 2 + MT_BN * MT_BK / 2), tile = sizeof(float) * MT_BM * MT_LDC;
+  constexpr size_t smem = stages > tile ? stages : tile;
+  const int cols = gated_epi(a.epi) ? MT_BN / 2 : MT_BN, n_out = gated_epi(a.epi) ? a.N / 2 : a.N;
+  if (smem > 48 * 1024) LP_CHECK_CUDA(cudaFuncSetAttribute(linear_mma_kernel<AT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  dim3 grid((n_out + cols - 1) / cols, m_tiles, batch);
+  linear_mma_kernel<AT><<<grid, MT_THREADS, smem, stream>>>(a, gated_epi(a.epi), c_fp32);
+  note_launch();
+  LP_CHECK_CUDA(cudaGetLastError());
+  return 0;
 }
 
 template <typename AT, typename CT, bool GATED>
@@ -589,6 +780,11 @@ extern "C" int lp_linear(const lp_linear_desc* d, void* stream_) {
   LP_REQUIRE(d->seg_cols == 0 || !gated_epi(d->epi), "lp_linear: a gated unit has one operand");
   if (d->M <= STREAM_MAX_ROWS && stream_ok(a, d->a_fp32, d->batch) && (d->seg_cols == 0 || d->seg_cols % 16 == 0))
     return dispatch_stream(a, d->a_fp32, d->c_fp32, d->batch, d->M, 0, 0, stream);
+  // the tile kernel on the matrix instructions; operands without 16-byte rows stay on fp32 FMAs
+  if (stream_ok(a, d->a_fp32, d->batch) && (d->seg_cols == 0 || d->seg_cols % MT_BN == 0) && d->M > STREAM_MAX_ROWS) {
+    const int m_tiles = (d->M + MT_BM - 1) / MT_BM;
+    return d->a_fp32 ? launch_mma<float>(a, d->c_fp32, d->batch, m_tiles, stream) : launch_mma<bf16>(a, d->c_fp32, d->batch, m_tiles, stream);
+  }
   return dispatch_linear(a, d->a_fp32, d->c_fp32, d->batch, (d->M + LIN_BM - 1) / LIN_BM, true, stream);
 }
 
@@ -634,6 +830,8 @@ extern "C" int lp_linear_grouped(const lp_linear_desc* d, const int* tile_group,
   a.a_rows = a_rows; a.tile_group = tile_group; a.z_group = nullptr; a.a_div = 1;
   a.bias = d->bias; a.row_scale = d->row_scale; a.gate = d->gate; a.ldg = d->ldg; a.gate_batch = d->gate_batch;
   a.seg_cols = 0; a.n_segs = 0; a.a_seg = 0;
+  if (stream_ok(a, d->a_fp32, 1))
+    return d->a_fp32 ? launch_mma<float>(a, d->c_fp32, 1, n_tiles, stream) : launch_mma<bf16>(a, d->c_fp32, 1, n_tiles, stream);
   return dispatch_linear(a, d->a_fp32, d->c_fp32, 1, n_tiles, false, stream);
 }
 

@@ -1,6 +1,6 @@
-"""The weight-streaming product of up to 64 rows (lp_linear) and of grouped pairs (lp_linear_pairs with the number of groups) against a
-float64 product: the edges of its row groups, column tiles and K steps, both operand types, every kind of epilogue; on the kernel sources
-under the CPU emulator and, marked gpu, on the native library.
+"""The weight-streaming product of up to 64 rows (lp_linear), of grouped pairs (lp_linear_pairs with the number of groups) and the tile
+product of more rows (lp_linear, lp_linear_grouped) against a float64 product: the edges of their row groups, column tiles and K steps, both
+operand types, every kind of epilogue; on the kernel sources under the CPU emulator and, marked gpu, on the native library.
 
 Error bounds: products are exact (a bf16 weight times a bf16 value or one of three bf16 terms of an fp32 one), at most about K / 16 fp32 sums
 follow: for K <= 400 below 32 * 2^-24 < 2e-6 of the result's size in the root mean square."""
@@ -40,7 +40,7 @@ def _data(M, N, K, dtype, device, seed=0):
 
 
 @pytest.mark.parametrize("dtype", [BF16, F32])
-@pytest.mark.parametrize("M,N,K", [(1, 1, 8), (8, 17, 40), (9, 33, 256), (16, 16, 264), (33, 48, 400), (64, 40, 72)])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 8), (8, 17, 40), (9, 33, 256), (16, 16, 264), (33, 48, 400), (64, 40, 72), (65, 130, 40), (129, 9, 72)])
 def test_rows_columns_and_steps(backend, dtype, M, N, K):
     a, w, want, ad, wd = _data(M, N, K, dtype, backend[0])
     out = torch.empty(M, N, device=backend[0])
@@ -52,8 +52,9 @@ def test_rows_columns_and_steps(backend, dtype, M, N, K):
 
 
 @pytest.mark.parametrize("dtype", [BF16, F32])
-def test_epilogues(backend, dtype):
-    M, N, K = 11, 36, 64
+@pytest.mark.parametrize("M", [11, 70])
+def test_epilogues(backend, dtype, M):
+    N, K = 36, 64
     a, w, z, ad, wd = _data(M, N, K, dtype, backend[0])
     g = torch.Generator().manual_seed(1)
     bias, scale, gate, x = torch.randn(N, generator=g), torch.rand(M, generator=g), torch.randn(M, N, generator=g), torch.randn(M, N, generator=g)
@@ -70,11 +71,12 @@ def test_epilogues(backend, dtype):
 
 def test_batches_and_segments(backend):
     g = torch.Generator().manual_seed(3)
-    heads, M, N, K = 3, 10, 24, 40
-    a, w = torch.randn(M, heads * 48, generator=g), torch.randn(heads, N, K, generator=g).to(BF16)
-    out = torch.empty(M, heads * N, device=backend[0])
-    _call(backend, a.to(backend[0]), w.to(backend[0]), out, M, batch=heads, a_batch=48, c_batch=N)
-    assert rel_err(out, torch.cat([a[:, 48 * h:48 * h + K].double() @ w[h].double().T for h in range(heads)], 1)) < 2e-6
+    for M in (10, 66):
+        heads, N, K = 3, 24, 40
+        a, w = torch.randn(M, heads * 48, generator=g), torch.randn(heads, N, K, generator=g).to(BF16)
+        out = torch.empty(M, heads * N, device=backend[0])
+        _call(backend, a.to(backend[0]), w.to(backend[0]), out, M, batch=heads, a_batch=48, c_batch=N)
+        assert rel_err(out, torch.cat([a[:, 48 * h:48 * h + K].double() @ w[h].double().T for h in range(heads)], 1)) < 2e-6
     ops, w = torch.randn(2, 5, K, generator=g).to(BF16), torch.randn(40, K, generator=g).to(BF16)
     out = torch.empty(5, 40, device=backend[0])
     od, wd = ops.to(backend[0]), w.to(backend[0])
@@ -111,3 +113,23 @@ def test_unusual_numbers(backend):
     assert torch.isfinite(out[0]).all() and torch.isnan(out[2]).all() and torch.isnan(out[4]).all()
     assert torch.equal(out[1].isinf(), want[1].isinf()) and torch.equal(out[1].sign(), want[1].sign().float())
     assert rel_err(out[3], want[3]) < 2e-6
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
+def test_row_tiles_of_groups(backend, dtype):
+    """tiles of 64 gathered rows, each on its group's weight; padding rows are zeros, a tile without a group is left alone"""
+    g = torch.Generator().manual_seed(9)
+    N, K, T = 136, 40, 30
+    a, w = torch.randn(T, K, generator=g).to(dtype), (torch.randn(3, N, K, generator=g) * K ** -0.5).to(BF16)
+    groups, rows = torch.tensor([2, -1, 0], dtype=torch.int32), torch.randint(-1, T, (192,), generator=g).to(torch.int32)
+    out = torch.full((192, N), 7.0)
+    od = out.clone().to(backend[0])
+    L = _lib_of(backend)
+    ad, wd, gd, rd = a.to(backend[0]), w.to(backend[0]), groups.to(backend[0]), rows.to(backend[0])
+    d = _lib.LinearDesc(A=_lib.ptr(ad), lda=K, a_fp32=int(dtype == F32), W=_lib.ptr(wd), ldw=K, w_batch=N * K, C=_lib.ptr(od), ldc=N, c_fp32=1,
+                        M=192, N=N, K=K, batch=1)
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream) if ad.is_cuda else None
+    assert L.lp_linear_grouped(C.byref(d), _lib.ptr(gd), 3, _lib.ptr(rd), stream) == 0
+    picked = torch.where((rows >= 0)[:, None], a.double()[rows.clamp(min=0).long()], 0.0)
+    want = torch.cat([picked[:64] @ w[2].double().T, out[64:128].double(), picked[128:] @ w[0].double().T])
+    assert rel_err(od, want) < 2e-6
