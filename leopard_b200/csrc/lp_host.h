@@ -61,6 +61,19 @@ __device__ __forceinline__ void mma_bf16(float* d, uint32_t a0, uint32_t a1, uin
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+// fp32 values as three bf16 terms, rounded to nearest each (8 + 8 + 8 bits: what is left is below 2^-26 of the value), packed in pairs
+__device__ __forceinline__ void cut3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  __nv_bfloat162 p = __floats2bfloat162_rn(x, y);
+  hi = *reinterpret_cast<const uint32_t*>(&p);
+  x -= __uint_as_float(hi << 16);
+  y -= __uint_as_float(hi & 0xffff0000u);
+  p = __floats2bfloat162_rn(x, y);
+  mid = *reinterpret_cast<const uint32_t*>(&p);
+  x -= __uint_as_float(mid << 16);
+  y -= __uint_as_float(mid & 0xffff0000u);
+  p = __floats2bfloat162_rn(x, y);
+  lo = *reinterpret_cast<const uint32_t*>(&p);
+}
 #endif
 
 // prefill kernels are launched with the programmatic-dependent-launch attribute when this is on (lp_set_prefill_pdl):

@@ -32,6 +32,7 @@
 //   lp_window_attn_talk_tiles  the same for prompts, a CTA per tile of 4 consecutive rows of a request and all heads.
 //   lp_window_attn_tiles  the same for prompts, a CTA per tile of 2 or 4 consecutive rows of a request: the rows share every key and
 //                         value row the tile reads, each (row, key) pair masked by the row's own rule.
+#include <cuda_pipeline.h>
 #include "lp_host.h"
 #include "../../include/leopard_b200.h"
 
@@ -81,6 +82,32 @@ __device__ __forceinline__ float win_distance_bias(bool linear, float amp, float
 __device__ __forceinline__ float win_out(const WinArgs& a, int r, int c, float v) {
   if (a.gate != nullptr) v /= 1.0f + expf(-a.gate[(long long)r * a.ldg + c]);
   return v * a.out_scale;
+}
+
+// channel cc of one finished head row `o` on its way out: rotated values are turned back by the query's position, then gate and factor
+__device__ __forceinline__ void win_store(const WinArgs& a, const float* o, int cc, int vhalf, int pos, int r, int head, void* out, long long ldo,
+                                          int out_fp32) {
+  float v = o[cc];
+  if (cc < 2 * vhalf) {
+    int pair, partner;
+    bool first;
+    if (a.v_rot_layout == LP_ROT_INTERLEAVED) {
+      pair = cc >> 1;
+      first = (cc & 1) == 0;
+      partner = first ? cc + 1 : cc - 1;
+    } else {
+      first = cc < vhalf;
+      pair = first ? cc : cc - vhalf;
+      partner = first ? cc + vhalf : cc - vhalf;
+    }
+    float sn, cs;
+    sincosf((float)pos * a.v_inv_freq[pair], &sn, &cs);
+    v = first ? o[cc] * cs + o[partner] * sn : o[cc] * cs - o[partner] * sn;
+  }
+  v = win_out(a, r, head * a.vdim + cc, v);
+  const long long at = (long long)r * ldo + (long long)head * a.vdim + cc;
+  if (out_fp32) reinterpret_cast<float*>(out)[at] = v;
+  else reinterpret_cast<bf16*>(out)[at] = __float2bfloat16(v);
 }
 
 // the two members of rotation pair i
@@ -699,28 +726,232 @@ window_attn_tile_kernel(WinArgs a, int n_chunks, const int* __restrict__ chunk_s
   for (int i = tid; i < X * a.vdim; i += blockDim.x) {
     const int x = i / a.vdim, cc = i % a.vdim, rq = x / QH, h = x % QH;
     if (rq >= nrows) continue;
-    const float* o = f_s + x * a.vdim;
-    float v = o[cc];
-    if (cc < 2 * vhalf) {
-      int pair, partner;
-      bool first;
-      if (a.v_rot_layout == LP_ROT_INTERLEAVED) {
-        pair = cc >> 1;
-        first = (cc & 1) == 0;
-        partner = first ? cc + 1 : cc - 1;
+    win_store(a, f_s + x * a.vdim, cc, vhalf, pos0 + rq, r0 + rq, h0 + h, out, ldo, out_fp32);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------------------------
+// Prompts on the matrix instructions, heads of 128: a CTA takes one chunk (up to 32 rows) and QH query heads of a key / value head, a warp
+// 16 (row, head) pairs, and walks the union of what its rows see 32 keys at a time.  Everything stays fp32-exact in kind: queries, keys,
+// softmax weights and values are cut into three bf16 terms (cut3) and the six products of weight above 2^-26 are taken, so a product carries
+// what an fp32 multiplication keeps; the instruction's sums are cut off instead of rounded, so they are short (32 channels of a score, 32
+// keys of an output, small terms first) and added in fp32.  Maxima, exponentials, denominators and rescaling are fp32 as before.
+// Shared memory holds the terms in planes: queries and keys as [32-channel block][row][64 bytes] (a lane reads eight channels, the same
+// permutation on both sides, eight lanes two neighbouring rows: no bank twice), values transposed as [channel][16 words], the words in the order
+// in which a lane's score fragments become its weight fragments.  The next keys' fp32 rows are copied in (cp.async) meanwhile.
+constexpr int WM_D = 128, WM_KT = 32, WM_ROWS = 32, WM_MIN_ROWS = 32;
+template <int QH> constexpr size_t wm_smem_words() { return (size_t)3 * WM_ROWS * QH * WM_D / 2 + 2 * 3 * WM_KT * WM_D / 2 + 2 * WM_KT * WM_D; }
+
+template <int QH, bool DIST>
+__global__ void __launch_bounds__(QH * 64)
+window_attn_mma_kernel(WinArgs a, int n_chunks, const int* __restrict__ chunk_seq, const int* __restrict__ chunk_row0,
+                       const int* __restrict__ chunk_len, const int* __restrict__ row_pos, void* __restrict__ out, long long ldo, int out_fp32) {
+  extern __shared__ float dyn_smem[];
+  constexpr int X = WM_ROWS * QH, THREADS = QH * 64, Q_PLANE = X * WM_D / 2, K_PLANE = WM_KT * WM_D / 2;      // planes in 32-bit words
+  uint32_t* q_p = reinterpret_cast<uint32_t*>(dyn_smem);      // [3][4][X][16]
+  uint32_t* k_p = q_p + 3 * Q_PLANE;                          // [3][4][WM_KT][16]
+  uint32_t* v_p = k_p + 3 * K_PLANE;                          // [3][WM_D][16]
+  float* raw = reinterpret_cast<float*>(v_p + 3 * K_PLANE);   // [WM_KT][keys | values]
+  const int c = n_chunks - 1 - (int)blockIdx.x;               // later chunks see more keys: they start first
+  const int nrows = chunk_len[c], r0 = chunk_row0[c], seq = chunk_seq[c], pos0 = row_pos[r0];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int ratio = a.heads / a.kv_heads, per_g = ratio / QH;
+  const int kvh = blockIdx.y / per_g, h0 = kvh * ratio + (blockIdx.y % per_g) * QH;
+  for (int i = tid; i < X * (WM_D / 8); i += THREADS) {      // eight channels of a pair
+    const int x = i >> 4, e = i & 15, rq = x / QH, h = x % QH;
+    uint32_t w[3][4];
+    const float* src = a.qkv + (long long)(r0 + (rq < nrows ? rq : 0)) * a.ld + a.q_off + (long long)(h0 + h) * WM_D + e * 8;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) cut3(rq < nrows ? src[2 * k] : 0.f, rq < nrows ? src[2 * k + 1] : 0.f, w[0][k], w[1][k], w[2][k]);
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+      *reinterpret_cast<uint4*>(q_p + p * Q_PLANE + ((e >> 2) * X + x) * 16 + (e & 3) * 4) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+  }
+  const WinVisible first = win_visible(a, pos0), last = win_visible(a, pos0 + nrows - 1);
+  WinVisible uni;      // the union, in the index space of win_visible_row
+  uni.n_keep = last.n_keep;
+  uni.n_blocks = last.n_blocks;
+  uni.lo = first.lo;
+  uni.count = uni.n_keep + uni.n_blocks + (pos0 + nrows - 1 - uni.lo + 1);
+  const int k_off = kvh * WM_D, v_off = a.v_base + kvh * WM_D;
+  auto load = [&](int t0) {      // the fp32 rows of the next keys; zeros past the end
+    for (int j = warp; j < WM_KT; j += THREADS / 32) {
+      float* dst = raw + j * 2 * WM_D + 4 * lane;
+      if (t0 + j < uni.count) {
+        const float* row = win_visible_row(a, uni, seq, t0 + j);
+        __pipeline_memcpy_async(dst, row + k_off + 4 * lane, 16);
+        __pipeline_memcpy_async(dst + WM_D, row + v_off + 4 * lane, 16);
       } else {
-        first = cc < vhalf;
-        pair = first ? cc : cc - vhalf;
-        partner = first ? cc + vhalf : cc - vhalf;
+        *reinterpret_cast<float4*>(dst) = *reinterpret_cast<float4*>(dst + WM_D) = make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      float sn, cs;
-      sincosf((float)(pos0 + rq) * a.v_inv_freq[pair], &sn, &cs);
-      v = first ? o[cc] * cs + o[partner] * sn : o[cc] * cs - o[partner] * sn;
     }
-    v = win_out(a, r0 + rq, (h0 + h) * a.vdim + cc, v);
-    const long long at = (long long)(r0 + rq) * ldo + (long long)(h0 + h) * a.vdim + cc;
-    if (out_fp32) reinterpret_cast<float*>(out)[at] = v;
-    else reinterpret_cast<bf16*>(out)[at] = __float2bfloat16(v);
+    __pipeline_commit();
+  };
+  // this lane's two pairs
+  int my_row[2], keep[2], blocks[2], lo[2];
+  float mx[2], den[2], amp[2], rate[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int x = warp * 16 + g + 8 * i, rq = x / QH, h = h0 + x % QH;
+    my_row[i] = rq < nrows ? pos0 + rq : -1;
+    const WinVisible v = win_visible(a, rq < nrows ? pos0 + rq : pos0);
+    keep[i] = v.n_keep;
+    blocks[i] = v.n_blocks;
+    lo[i] = v.lo;
+    mx[i] = a.sink ? 0.f : -INFINITY;
+    den[i] = a.sink ? 1.f : 0.f;
+    amp[i] = DIST ? a.dist_amp[h] : 0.f;
+    rate[i] = DIST && a.dist_rate != nullptr ? a.dist_rate[h] : 0.f;
+  }
+  float o[WM_D / 8][4];
+#pragma unroll
+  for (int n = 0; n < WM_D / 8; ++n)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) o[n][k] = 0.f;
+  load(0);
+  for (int t0 = 0; t0 < uni.count; t0 += WM_KT) {
+    __pipeline_wait_prior(0);
+    __syncthreads();      // the rows are here for everyone, and nobody reads the planes any more
+    for (int i = tid; i < WM_KT * (WM_D / 8); i += THREADS) {
+      const int j = i >> 4, e = i & 15;
+      const float4 u = *reinterpret_cast<const float4*>(raw + j * 2 * WM_D + e * 8), v = *reinterpret_cast<const float4*>(raw + j * 2 * WM_D + e * 8 + 4);
+      uint32_t w[3][4];
+      cut3(u.x, u.y, w[0][0], w[1][0], w[2][0]);
+      cut3(u.z, u.w, w[0][1], w[1][1], w[2][1]);
+      cut3(v.x, v.y, w[0][2], w[1][2], w[2][2]);
+      cut3(v.z, v.w, w[0][3], w[1][3], w[2][3]);
+#pragma unroll
+      for (int p = 0; p < 3; ++p)
+        *reinterpret_cast<uint4*>(k_p + p * K_PLANE + ((e >> 2) * WM_KT + j) * 16 + (e & 3) * 4) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+    }
+    for (int i = tid; i < WM_D * 4; i += THREADS) {      // channel d, the eight keys that lanes t = i / WM_D of a warp take
+      const int d = i % WM_D, kt = i / WM_D;
+      uint32_t w[3][4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {      // keys 16 (k / 2) + 8 (k % 2) + 2 kt and the next
+        const float* src = raw + (16 * (k >> 1) + 8 * (k & 1) + 2 * kt) * 2 * WM_D + WM_D + d;
+        cut3(src[0], src[2 * WM_D], w[0][k], w[1][k], w[2][k]);
+      }
+#pragma unroll
+      for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(v_p + p * K_PLANE + d * 16 + kt * 4) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+    }
+    __syncthreads();
+    if (t0 + WM_KT < uni.count) load(t0 + WM_KT);
+    // scores of 16 pairs and 32 keys
+    float sc[4][4], small[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) sc[j][k] = small[j][k] = 0.f;
+#pragma unroll
+    for (int s = 0; s < WM_D / 32; ++s) {
+      uint4 qa[3], qb[3];
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        const uint32_t* src = q_p + p * Q_PLANE + (s * X + warp * 16 + g) * 16 + t * 4;
+        qa[p] = *reinterpret_cast<const uint4*>(src);
+        qb[p] = *reinterpret_cast<const uint4*>(src + 8 * 16);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint4 kk[3];
+#pragma unroll
+        for (int p = 0; p < 3; ++p) kk[p] = *reinterpret_cast<const uint4*>(k_p + p * K_PLANE + (s * WM_KT + 8 * j + g) * 16 + t * 4);
+        float big[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int p = 2; p >= 0; --p)      // (2, 0) (1, 1) (0, 2) (1, 0) (0, 1), then (0, 0)
+#pragma unroll
+          for (int q = p; q >= 0; --q) {
+            float* d = p == 0 ? big : small[j];
+            mma_bf16(d, qa[q].x, qb[q].x, qa[q].y, qb[q].y, kk[p - q].x, kk[p - q].y);
+            mma_bf16(d, qa[q].z, qb[q].z, qa[q].w, qb[q].w, kk[p - q].z, kk[p - q].w);
+          }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) sc[j][k] += big[k];
+      }
+    }
+    // softmax of this tile; rows g and g + 8 of the warp's pairs
+    float corr[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float top = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const int key = t0 + 8 * j + 2 * t + k;
+          const int seg = key < uni.n_keep ? 0 : (key < uni.n_keep + uni.n_blocks ? 1 : 2);
+          const int idx = seg == 0 ? key : (seg == 1 ? key - uni.n_keep : uni.lo + (key - uni.n_keep - uni.n_blocks));
+          bool seen = my_row[i] >= 0 && key < uni.count;
+          if (seg == 0) seen = seen && idx < keep[i];
+          else if (seg == 1) seen = seen && idx < blocks[i];
+          else seen = seen && idx >= lo[i] && idx <= my_row[i];
+          float v = (sc[j][2 * i + k] + small[j][2 * i + k]) * a.scale;
+          if (a.softcap > 0.f) v = a.softcap * tanhf(v / a.softcap);
+          if (DIST) v -= win_distance_bias(a.dist_rate == nullptr, amp[i], rate[i], my_row[i] - idx, out_fp32);
+          v = seen ? v : -INFINITY;
+          sc[j][2 * i + k] = v;
+          top = fmaxf(top, v);
+        }
+      top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+      top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+      const float mn = fmaxf(mx[i], top), ref = mn == -INFINITY ? 0.f : mn;      // -inf: nothing seen so far
+      corr[i] = expf(mx[i] - ref);
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const float p = expf(sc[j][2 * i + k] - ref);      // exp(-inf) = 0 for what this row does not see
+          sc[j][2 * i + k] = p;
+          sum += p;
+        }
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      den[i] = fmaf(den[i], corr[i], sum);
+      mx[i] = mn;
+    }
+    // weights as the left operand: score fragments of two neighbouring groups of eight keys are one of 16
+    uint32_t w[3][2][4];
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int j = 2 * q + (k >> 1), i = k & 1;
+        cut3(sc[j][2 * i], sc[j][2 * i + 1], w[0][q][k], w[1][q][k], w[2][q][k]);
+      }
+#pragma unroll
+    for (int n = 0; n < WM_D / 8; ++n) {
+      uint4 vv[3];
+#pragma unroll
+      for (int p = 0; p < 3; ++p) vv[p] = *reinterpret_cast<const uint4*>(v_p + p * K_PLANE + (8 * n + g) * 16 + t * 4);
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int p = 2; p >= 0; --p)
+#pragma unroll
+        for (int q = p; q >= 0; --q) {
+          mma_bf16(d, w[q][0][0], w[q][0][1], w[q][0][2], w[q][0][3], vv[p - q].x, vv[p - q].y);
+          mma_bf16(d, w[q][1][0], w[q][1][1], w[q][1][2], w[q][1][3], vv[p - q].z, vv[p - q].w);
+        }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) o[n][k] = fmaf(o[n][k], corr[k >> 1], d[k]);
+    }
+  }
+  __syncthreads();      // the query planes become the output rows
+  float* f_s = dyn_smem;      // [X][WM_D + 4]
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float inv = den[i] > 0.f ? 1.0f / den[i] : 0.f;      // rows past the end of the chunk have seen nothing and are not stored
+#pragma unroll
+    for (int n = 0; n < WM_D / 8; ++n)
+#pragma unroll
+      for (int k = 0; k < 2; ++k) f_s[(warp * 16 + g + 8 * i) * (WM_D + 4) + 8 * n + 2 * t + k] = o[n][2 * i + k] * inv;
+  }
+  __syncthreads();
+  const int vhalf = a.v_inv_freq != nullptr ? a.v_rot_dims >> 1 : 0;
+  for (int i = tid; i < nrows * QH * WM_D; i += THREADS) {
+    const int x = i / WM_D, cc = i % WM_D, rq = x / QH, h = x % QH;
+    win_store(a, f_s + x * (WM_D + 4), cc, vhalf, pos0 + rq, r0 + rq, h0 + h, out, ldo, out_fp32);
   }
 }
 
@@ -1193,6 +1424,18 @@ static int launch_window_attn_tiles(const WinArgs& a, int R, int n_chunks, const
   return 0;
 }
 
+template <int QH, bool DIST>
+static int launch_window_attn_mma(const WinArgs& a, int n_chunks, const int* chunk_seq, const int* chunk_row0, const int* chunk_len, const int* row_pos,
+                                  void* out, long long ldo, int out_fp32, cudaStream_t stream) {
+  constexpr size_t smem = wm_smem_words<QH>() * 4;
+  LP_CHECK_CUDA(cudaFuncSetAttribute(window_attn_mma_kernel<QH, DIST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  window_attn_mma_kernel<QH, DIST><<<dim3(n_chunks, a.heads / QH), QH * 64, smem, stream>>>(a, n_chunks, chunk_seq, chunk_row0, chunk_len, row_pos, out,
+                                                                                            ldo, out_fp32);
+  note_launch();
+  LP_CHECK_CUDA(cudaGetLastError());
+  return 0;
+}
+
 }  // namespace lp
 
 using namespace lp;
@@ -1299,6 +1542,15 @@ extern "C" int lp_window_attn_tiles(const lp_window_attn_desc* d, int R, const i
              d->vdim, WIN_MAX_DIM);
   if (R <= 0 || n_chunks <= 0) return 0;
   const int ratio = d->heads / d->kv_heads;
+  // heads of 128 whose cache rows are whole 16-byte pieces run on the matrix instructions; a handful of rows leaves their tiles empty
+  if (d->dim == WM_D && d->vdim == WM_D && R >= WM_MIN_ROWS && a.roww % 4 == 0 && a.v_base % 4 == 0 && (reinterpret_cast<uintptr_t>(a.cache) & 15) == 0 &&
+      (a.pool == 0 || (reinterpret_cast<uintptr_t>(a.pooled) & 15) == 0)) {
+#define LP_WM(QH)                                                                                                                              \
+  (d->dist_amp != nullptr ? launch_window_attn_mma<QH, true>(a, n_chunks, chunk_seq, chunk_row0, chunk_len, row_pos, out, ldo, out_fp32, stream) \
+                          : launch_window_attn_mma<QH, false>(a, n_chunks, chunk_seq, chunk_row0, chunk_len, row_pos, out, ldo, out_fp32, stream))
+    return ratio % 4 == 0 ? LP_WM(4) : ratio % 2 == 0 ? LP_WM(2) : LP_WM(1);
+#undef LP_WM
+  }
   int rc;
   if (d->dist_amp != nullptr) {
     if (ratio % 4 == 0) rc = launch_window_attn_tiles<4, 2, true>(a, R, n_chunks, chunk_seq, chunk_row0, chunk_len, row_pos, out, ldo, out_fp32, stream);

@@ -123,6 +123,15 @@ inline void mma_bf16(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a
     }
   }
 }
+inline void cut3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  uint32_t* out[3] = {&hi, &mid, &lo};
+  for (int i = 0; i < 3; ++i) {
+    const __nv_bfloat162 p = __floats2bfloat162_rn(x, y);
+    *out[i] = (uint32_t)p.x.bits | ((uint32_t)p.y.bits << 16);
+    x -= (float)p.x;
+    y -= (float)p.y;
+  }
+}
 inline uint32_t smem_u32(const void* p) { return (uint32_t)(uintptr_t)p; }
 struct ProfScope { ProfScope(int, int, int, int, cudaStream_t) {} };
 }  // namespace lp

@@ -1,0 +1,118 @@
+"""Attention of prompts with heads of 128 (lp_window_attn_tiles on the matrix instructions) against float64: ragged chunks and last tiles,
+every number of query heads to a key / value head, windows with kept tokens or pooled blocks, blocks, caps, sinks, distance terms, values turned
+back; and that it is as near to float64 as the one-row kernel (lp_window_attn) is.  On the kernel sources under the CPU emulator and, marked
+gpu, on the native library.
+
+Bound: three-term products keep 2^-24 of each factor, sums are short chains added in fp32; with scores of size 4 an error of 1e-6 in a score is
+1e-6 of a weight, so 4e-6 of the result's root mean square; the one-row kernel's FMA chains measure about 3e-7."""
+import ctypes as C
+
+import pytest
+import torch
+
+from leopard_b200 import _lib
+from seqlm_common import backend, emu_lib, rel_err  # noqa: F401
+
+F32, D, PAGE = torch.float32, 128, 16
+
+FORMS = {
+    "window": dict(window=20),
+    "kept": dict(window=16, keep_first=3, sink=1),
+    "pooled": dict(window=24, pool=8, softcap=6.0),
+    "all": dict(),
+    "blocks": dict(chunk=24),
+    "bias": dict(window=40, dist="log"),
+    "slope": dict(dist="linear"),
+    "turned": dict(window=30, vrot=64),
+}
+
+
+def _run(backend, form, heads, kv_heads, pos0, lens, seed=0):
+    device, lib = backend
+    L = lib if lib is not None else _lib.stream32_lib()
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream) if device == "cuda" else None
+    g = torch.Generator().manual_seed(seed)
+    f, R = FORMS[form], sum(lens)
+    total = [p + n for p, n in zip(pos0, lens)]
+    pages = [-(-t // PAGE) for t in total]
+    q = torch.randn(R, heads * D, generator=g)
+    roww = kv_heads * 2 * D
+    cache = torch.randn(sum(pages), PAGE, roww, generator=g)
+    table = torch.full((len(lens), max(pages)), -1, dtype=torch.int32)
+    at = 0
+    for i, n in enumerate(pages):
+        table[i, :n] = torch.randperm(n, generator=g).to(torch.int32) + at
+        at += n
+    rows = [torch.stack([cache[int(table[i, p // PAGE]), p % PAGE] for p in range(t)]) for i, t in enumerate(total)]
+    pool = f.get("pool", 0)
+    pooled = ptab = None
+    if pool:
+        n_blocks = max(max(t // pool for t in total), 1)
+        pooled = torch.zeros(len(lens), -(-n_blocks // PAGE), PAGE, roww)
+        for i, t in enumerate(total):
+            for b in range(t // pool):
+                pooled[i, b // PAGE, b % PAGE] = rows[i][b * pool:(b + 1) * pool].mean(0)
+        ptab = torch.arange(pooled.shape[0] * pooled.shape[1], dtype=torch.int32).view(len(lens), -1)
+    amp = torch.rand(heads, generator=g) * 0.3 if "dist" in f else None
+    rate = torch.rand(heads, generator=g) if f.get("dist") == "log" else None
+    vfreq = 100.0 ** (-torch.arange(f["vrot"] // 2) * 2.0 / f["vrot"]) if "vrot" in f else None
+    row_pos = torch.cat([torch.arange(p, p + n) for p, n in zip(pos0, lens)]).to(torch.int32)
+    row_seq = torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens)).to(torch.int32)
+    chunks, r0 = [], 0
+    for i, n in enumerate(lens):
+        chunks += [(i, r0 + a, min(32, n - a)) for a in range(0, n, 32)]
+        r0 += n
+    cs, cr, cl = (torch.tensor(x, dtype=torch.int32) for x in zip(*chunks))
+    t = {k: (v.to(device) if v is not None else None) for k, v in dict(q=q, cache=cache, table=table, pooled=pooled, ptab=ptab, amp=amp, rate=rate,
+                                                                        vfreq=vfreq, row_pos=row_pos, row_seq=row_seq, cs=cs, cr=cr, cl=cl).items()}
+    one = torch.ones(1, device=device)
+    d = _lib.WindowAttnDesc(
+        qkv=_lib.ptr(t["q"]), ld=heads * D, q_off=0, k_off=0, v_off=0, heads=heads, kv_heads=kv_heads, dim=D, vdim=D, norm_mode=_lib.QKNORM_NONE,
+        g_off=-1, eps=1e-6, inv_freq=_lib.ptr(one), rot_dims=0, rot_layout=_lib.ROT_HALF, rot_mscale=1.0, v_inv_freq=_lib.ptr(t["vfreq"]),
+        v_rot_dims=f.get("vrot", 0), v_rot_layout=_lib.ROT_HALF, cache=_lib.ptr(t["cache"]), page_size=PAGE, page_table=_lib.ptr(t["table"]),
+        max_pages=table.shape[1], pooled=_lib.ptr(t["pooled"]), pooled_table=_lib.ptr(t["ptab"]), max_pooled_pages=ptab.shape[1] if pool else 0, pool=pool,
+        window=f.get("window", 0), keep_first=f.get("keep_first", 0), scale=D ** -0.5, softcap=f.get("softcap", 0.0), sink=f.get("sink", 0),
+        chunk=f.get("chunk", 0), kv_shared=1, dist_amp=_lib.ptr(t["amp"]), dist_rate=_lib.ptr(t["rate"]), out_scale=1.0)
+    got, row_wise = torch.full((R, heads * D), 9.0, device=device), torch.empty(R, heads * D, device=device)
+    rc = L.lp_window_attn_tiles(C.byref(d), R, _lib.ptr(t["row_seq"]), _lib.ptr(t["row_pos"]), len(chunks), _lib.ptr(t["cs"]), _lib.ptr(t["cr"]),
+                                _lib.ptr(t["cl"]), _lib.ptr(got), heads * D, 1, st)
+    assert rc == 0, L.lp_last_error()
+    assert L.lp_window_attn(C.byref(d), R, _lib.ptr(t["row_seq"]), _lib.ptr(t["row_pos"]), _lib.ptr(row_wise), heads * D, 1, st) == 0
+    want = torch.zeros(R, heads, D, dtype=torch.float64)
+    for r in range(R):
+        i, p = int(row_seq[r]), int(row_pos[r])
+        w, ch = f.get("window", 0), f.get("chunk", 0)
+        lo = max(p - w + 1, 0) if w else 0
+        lo = max(lo, p // ch * ch) if ch else lo
+        seen = [j for j in range(p + 1) if j >= lo or j < f.get("keep_first", 0)]
+        blocks = [b for b in range(total[i]) if pool and w and b * pool + pool - 1 <= p - w]
+        kv = torch.cat([pooled[i].reshape(-1, roww)[blocks] if blocks else torch.zeros(0, roww), rows[i][seen]]).double()
+        dist = torch.tensor([0.0] * len(blocks) + [float(p - j) for j in seen], dtype=torch.float64)
+        k, v = kv[:, :kv_heads * D].view(-1, kv_heads, D), kv[:, kv_heads * D:].view(-1, kv_heads, D)
+        for h in range(heads):
+            s = k[:, h // (heads // kv_heads)] @ q[r, h * D:(h + 1) * D].double() * D ** -0.5
+            if f.get("softcap"):
+                s = f["softcap"] * torch.tanh(s / f["softcap"])
+            if amp is not None:
+                s = s - float(amp[h]) * (torch.log1p(float(rate[h]) * dist) if rate is not None else dist)
+            e = torch.exp(s)
+            want[r, h] = (e / (e.sum() + f.get("sink", 0))) @ v[:, h // (heads // kv_heads)]
+        if vfreq is not None:
+            n = f["vrot"] // 2
+            ang = (float(p) * vfreq.float()).double()
+            x, y = want[r, :, :n].clone(), want[r, :, n:2 * n].clone()
+            want[r, :, :n], want[r, :, n:2 * n] = x * ang.cos() + y * ang.sin(), y * ang.cos() - x * ang.sin()
+    return rel_err(got, want.view(R, -1)), rel_err(row_wise, want.view(R, -1))
+
+
+@pytest.mark.parametrize("form", sorted(FORMS))
+def test_forms(backend, form):
+    """two requests, one from its beginning, one after 37 earlier tokens; last chunks of 1 and 9 rows"""
+    tiles, row_wise = _run(backend, form, 4, 1, [0, 37], [33, 41] if backend[0] == "cuda" else [33, 9])
+    assert tiles < 4e-6 and tiles < 2 * row_wise + 2e-7, (tiles, row_wise)
+
+
+@pytest.mark.parametrize("heads,kv_heads", [(1, 1), (2, 2), (2, 1), (6, 1), (8, 1), (3, 1)])
+def test_head_groups(backend, heads, kv_heads):
+    tiles, row_wise = _run(backend, "kept", heads, kv_heads, [5], [40])
+    assert tiles < 4e-6 and tiles < 2 * row_wise + 2e-7, (tiles, row_wise)
