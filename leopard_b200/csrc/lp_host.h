@@ -61,6 +61,12 @@ __device__ __forceinline__ void mma_bf16(float* d, uint32_t a0, uint32_t a1, uin
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+// the same from zero sums: d = a b
+__device__ __forceinline__ void mma_bf16_first(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
 // fp32 values as three bf16 terms, rounded to nearest each (8 + 8 + 8 bits: what is left is below 2^-26 of the value), packed in pairs
 __device__ __forceinline__ void cut3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   __nv_bfloat162 p = __floats2bfloat162_rn(x, y);

@@ -123,6 +123,10 @@ inline void mma_bf16(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a
     }
   }
 }
+inline void mma_bf16_first(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  d[0] = d[1] = d[2] = d[3] = 0.f;
+  mma_bf16(d, a0, a1, a2, a3, b0, b1);
+}
 inline void cut3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   uint32_t* out[3] = {&hi, &mid, &lo};
   for (int i = 0; i < 3; ++i) {
