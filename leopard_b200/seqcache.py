@@ -130,7 +130,7 @@ class SequenceCache:
 
     def reserve(self, seq: Sequence, n_tokens: int) -> None:
         """Make sure pages exist for positions [seq.length, seq.length + n_tokens) and for the blocks they complete."""
-        if not self.row_widths:
+        if not self.row_widths or (n_tokens == 1 and not self.summary_every and len(seq.pages) * self.page_size > seq.length):
             return
         need = -(-(seq.length + n_tokens) // self.page_size)
         while len(seq.pages) < need:
@@ -150,6 +150,8 @@ class SequenceCache:
         if self.window is None or not self.row_widths:
             return
         first_needed = seq.length - self.window + 1          # the oldest position the NEXT query (at seq.length) sees
+        if n_tokens == 1 and (first_needed <= 0 or first_needed % self.page_size):
+            return                                           # one position further inside a page: nothing new falls out
         kept = -(-self.keep_first // self.page_size)           # pages that hold a token some layer keeps for ever
         for b in range(kept, min(len(seq.pages), max(first_needed, 0) // self.page_size)):
             if seq.pages[b] >= 0:

@@ -685,15 +685,21 @@ class _Batch:
         self.R, self.n, self.lens = R, n, lens
         self.decode = all(ln == 1 for ln in lens)
         self.longest_chunk = min(max(lens), _lib.RETENTION_CHUNK)
-        row0 = np.zeros(n + 1, np.int32)
-        row0[1:] = np.cumsum(lens)
-        pos0 = np.array([s.length for s in seqs], np.int32)
-        slot = np.array([s.slot for s in seqs], np.int32)
-        tokens = np.concatenate([np.asarray(e.tokens, np.int64) for e in entries])
+        pos0 = np.fromiter([s.length for s in seqs], np.int32, n)
+        slot = np.fromiter([s.slot for s in seqs], np.int32, n)
+        if self.decode:      # one row a request: every per-row table is a per-request one
+            row0 = np.arange(n + 1, dtype=np.int32)
+            row_seq, row_pos = row0[:n], pos0
+            tokens = np.fromiter([e.tokens[0] for e in entries], np.int64, n)
+        else:
+            row0 = np.zeros(n + 1, np.int32)
+            row0[1:] = np.cumsum(lens)
+            row_seq = np.repeat(np.arange(n, dtype=np.int32), lens)
+            row_pos = np.concatenate([np.arange(p, p + ln, dtype=np.int32) for p, ln in zip(pos0, lens)])
+            tokens = np.concatenate([np.asarray(e.tokens, np.int64) for e in entries])
         if tokens.min() < 0 or tokens.max() >= eng.cfg.vocab:
             raise ValueError("token id outside the vocabulary")
-        row_seq = np.repeat(np.arange(n, dtype=np.int32), lens)
-        row_pos = np.concatenate([np.arange(p, p + ln, dtype=np.int32) for p, ln in zip(pos0, lens)])
+
         def page_table(lists):
             width = max([len(p) for p in lists] + [1])
             if self.decode:
@@ -710,24 +716,29 @@ class _Batch:
             sum_tables.append(t.reshape(-1))
             self.summary_width.append(width)
             self.summary_new.append(max((s.length + ln) // every - s.length // every for s, ln in zip(seqs, lens)))
-        ch = _lib.RETENTION_CHUNK
-        c_seq, c_row0, c_len, seq_c0 = [], [], [], [0]
-        for i, ln in enumerate(lens):
-            for a in range(0, ln, ch):
-                c_seq.append(i)
-                c_row0.append(int(row0[i]) + a)
-                c_len.append(min(ch, ln - a))
-            seq_c0.append(len(c_seq))
+        if self.decode:      # a chunk a request
+            c_seq, c_row0, c_len, seq_c0 = row_seq, row_seq, np.ones(n, np.int32), row0
+        else:
+            ch = _lib.RETENTION_CHUNK
+            c_seq, c_row0, c_len, seq_c0 = [], [], [], [0]
+            for i, ln in enumerate(lens):
+                for a in range(0, ln, ch):
+                    c_seq.append(i)
+                    c_row0.append(int(row0[i]) + a)
+                    c_len.append(min(ch, ln - a))
+                seq_c0.append(len(c_seq))
         self.n_chunks = len(c_seq)
         self.max_pages = max_pages
-        want = [int(row0[i]) + int(k) for i, e in enumerate(entries) for k in e.want]
-        for i, e in enumerate(entries):
-            if any(k < 0 or k >= lens[i] for k in e.want):
-                raise ValueError(f"request {e.key!r}: a wanted index is outside its tokens")
+        want = []
+        for r0, ln, e in zip(row0.tolist(), lens, entries):
+            for k in e.want:
+                if k < 0 or k >= ln:
+                    raise ValueError(f"request {e.key!r}: a wanted index is outside its tokens")
+                want.append(r0 + int(k))
         self.n_want = len(want)
         parts = [tokens.astype(np.int32), row_seq, row_pos, row0, pos0, slot, table.reshape(-1), np.asarray(c_seq, np.int32),
                  np.asarray(c_row0, np.int32), np.asarray(c_len, np.int32), np.asarray(seq_c0, np.int32)] + sum_tables
-        tables = torch.from_numpy(np.concatenate(parts).astype(np.int32))
+        tables = torch.from_numpy(np.concatenate(parts).astype(np.int32, copy=False))
         want_t = torch.from_numpy(np.asarray(want, np.int32))
         self.layout = (n, max_pages, *self.summary_width) if self.decode else None      # fixes the size of every table of a decode batch
         if eng.device.type == "cuda":
