@@ -8,7 +8,8 @@ is such a list), shift its mixer's input towards the previous token's, run a sho
 sublayers, and add a learned vector to the stream before it runs.  Every mechanism is a separate native entry point with its constants
 as arguments (include/leopard_b200.h, "32-BIT RESIDUAL-STREAM MODELS"), so another design is another list.  The residual stream, norms, routers, rotary angles, attention scores and recurrent state are fp32; matrix
 products take bf16 weights and, in the serving precision, bf16 activations with fp32 accumulation ("bfloat16"), or fp32 activations
-on fp32 FMAs ("float32": a true 32-bit forward, no tensor-core rounding).
+("float32": a true 32-bit forward — an activation is cut into three bf16 terms that add up to it exactly, so every product is exact and the
+sums are fp32).
 
 `SeqLMEngine.step(entries)` is THE step function: a packed batch of requests, each bringing its next tokens (a whole prompt, a
 portion of one, or one token), runs from the cache and state that earlier steps left (leopard_b200/seqcache.py) and returns the
