@@ -1,8 +1,7 @@
 // leopard_b200 — general linear layers for the 32-bit residual-stream models (any M, N, K; fp32 or bf16 activations).
 //
 //   lp_linear          C[M,N] = epi(A[M,K] · W[N,K]^T): A fp32 or bf16, W bf16 (nn.Linear layout), C fp32 or bf16, accumulation in
-//                      fp32 FMAs in index order of K (no tensor-core rounding: with fp32 A this is a true 32-bit product, the bf16
-//                      weight is exact in fp32).  Epilogues: none, xIELU, squared relu, and the gated units silu, gelu (tanh form)
+//                      fp32 (with fp32 A this is a true 32-bit product: the bf16 weight is exact, no operand is rounded).  Epilogues: none, xIELU, squared relu, and the gated units silu, gelu (tanh form)
 //                      and the clamped one (W = [gate rows; up rows], C has N/2 columns).  Before the epilogue every accumulator may be multiplied by a
 //                      number per output row (row_scale: a router weight that multiplies an expert's INPUT is the same as one
 //                      that multiplies its first products) and take a bias per weight row.  With c_accum the result is scaled
@@ -10,7 +9,9 @@
 //                      sigmoid(gate[m, n]) (a gated residual branch closes in the store of its last product).
 //                      seg_cols: groups of output columns that read operands of their own (a mixer whose projections see different
 //                      mixes of the stream) in one launch.  `batch` independent problems with element strides (per-head products of latent attention).
-//                      Two kernels: a 64 x 64 x 16 shared-memory tile kernel (prefill), and a weight-streaming kernel with one warp
+//                      Operands whose rows are whole 16-byte pieces run on the matrix instructions, a weight-streaming kernel for up to 64
+//                      rows and 64 x 128 tiles for more; fp32 rows as three bf16 terms that add up to them exactly.  The others run on
+//                      two fp32-FMA kernels: a 64 x 64 x 16 shared-memory tile kernel, and one with one warp
 //                      per output column for M <= 8 rows (decode: every weight byte is read once, 16-byte loads).
 //   lp_linear_grouped  the same tile kernel over row tiles that each belong to one group (expert): tile t multiplies rows
 //                      [64 t, 64 t + 64) of the padded, group-sorted row space by the weight of group tile_group[t] (< 0: skip);

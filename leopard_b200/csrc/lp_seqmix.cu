@@ -172,7 +172,9 @@ retention_scan_kernel(RetArgs a, const int* __restrict__ seq_chunk0, const int* 
 }
 
 // (3) o_i = decay^(i+1) q_i^T S_start + sum_(j<=i) decay^(i-j) (q_i . k_j) v_j; then o / rms(o) * silu(g).  The chunk's start state is
-// staged in shared memory (stage_s; read from global when a head is too large for that); 4 x 4 outputs per thread.
+// staged in shared memory where that is small (stage_s); a state of 128 x 128 would leave one CTA an SM, and the CTAs waiting for it and for
+// each other's phases took 1.23 ms (4096 tokens, 16 heads): read where it lies (L2, whole lines, eight loads in flight) three CTAs share an
+// SM and it takes 0.46 ms.  4 x 4 outputs per thread.
 __global__ void __launch_bounds__(RET_CHUNK_THREADS)
 retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const int* __restrict__ chunk_row0, const int* __restrict__ chunk_len,
                            const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0, const float* __restrict__ ws, int stage_s) {
@@ -211,31 +213,28 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
       Ss[i] = y < a.vdim ? S[d * a.vdim + y] : 0.f;
     }
   __syncthreads();
-  // in-chunk scores, 4 x 4 per thread (rows i0 .. i0+3, columns tj, tj+8, tj+16, tj+24)
-  for (int tile = tid; tile < (RET_CHUNK / 4) * (RET_CHUNK / 4); tile += blockDim.x) {
-    const int i0 = (tile / (RET_CHUNK / 4)) * 4, tj = tile % (RET_CHUNK / 4);
-    float acc[4][4];
-#pragma unroll
-    for (int p = 0; p < 4; ++p)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[p][q] = 0.f;
+  // in-chunk scores, 2 x 2 per thread (rows i0, i0 + 1, columns tj, tj + 16): every thread has one
+  for (int tile = tid; tile < (RET_CHUNK / 2) * (RET_CHUNK / 2); tile += blockDim.x) {
+    const int i0 = (tile / (RET_CHUNK / 2)) * 2, tj = tile % (RET_CHUNK / 2);
+    float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 8
     for (int d = 0; d < a.dim; ++d) {
-      float q4[4], k4[4];
+      float q2[2], k2[2];
 #pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        q4[p] = qs[(i0 + p) * dimp + d];
-        k4[p] = ks[(tj + p * (RET_CHUNK / 4)) * dimp + d];
+      for (int p = 0; p < 2; ++p) {
+        q2[p] = qs[(i0 + p) * dimp + d];
+        k2[p] = ks[(tj + p * (RET_CHUNK / 2)) * dimp + d];
       }
 #pragma unroll
-      for (int p = 0; p < 4; ++p)
+      for (int p = 0; p < 2; ++p)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) acc[p][q] = fmaf(q4[p], k4[q], acc[p][q]);
+        for (int q = 0; q < 2; ++q) acc[p][q] = fmaf(q2[p], k2[q], acc[p][q]);
     }
 #pragma unroll
-    for (int p = 0; p < 4; ++p)
+    for (int p = 0; p < 2; ++p)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int i = i0 + p, j = tj + q * (RET_CHUNK / 4);
+      for (int q = 0; q < 2; ++q) {
+        const int i = i0 + p, j = tj + q * (RET_CHUNK / 2);
         pp[i * (RET_CHUNK + 1) + j] = (j <= i && i < len) ? acc[p][q] * powf(dec, (float)(i - j)) : 0.f;
       }
   }
@@ -248,6 +247,7 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
     for (int p = 0; p < 4; ++p)
 #pragma unroll
       for (int q = 0; q < 4; ++q) acc[p][q] = 0.f;
+#pragma unroll 8
     for (int d = 0; d < a.dim; ++d) {
       float q4[4], s4[4];
 #pragma unroll
@@ -853,7 +853,7 @@ extern "C" int lp_retention_prefill(const lp_retention_desc* d, int n_seqs, int 
   const size_t smem1 = (size_t)RET_CHUNK * (dimp + vdimp) * sizeof(float);
   size_t smem3 = ((size_t)RET_CHUNK * (2 * dimp + 2 * vdimp) + RET_CHUNK * (RET_CHUNK + 1) + RET_CHUNK) * sizeof(float);
   LP_REQUIRE(smem3 <= 200 * 1024, "lp_retention_prefill: dim=%d vdim=%d do not fit the chunk kernel's shared memory", d->dim, d->vdim);
-  const int stage_s = smem3 + (size_t)d->dim * vdimp * sizeof(float) <= 200 * 1024;      // the chunk's start state next to the operands
+  const int stage_s = smem3 + (size_t)d->dim * vdimp * sizeof(float) <= 64 * 1024;      // three CTAs an SM keep their operands and the chunk's start state
   if (stage_s) smem3 += (size_t)d->dim * vdimp * sizeof(float);
   LP_CHECK_CUDA(ensure_smem(retention_chunk_state_kernel, smem1, g_smem_chunk_state));
   LP_CHECK_CUDA(ensure_smem(retention_chunk_out_kernel, smem3, g_smem_chunk_out));
