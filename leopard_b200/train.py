@@ -517,7 +517,11 @@ class SFTTrainer:
         else:
             micro = [(tokens, labels, loss_mask, images)]
         self.iteration += 1
-        self.flat_grad.zero_()
+        # the decoder's gradients are overwritten by the first micro-batch; the embedding's are added to, and the projector's and the
+        # tower's stay zero in a step without images
+        rest = next((n for n in self.names if not n.startswith("dec.")), None)
+        if rest is not None:
+            self.flat_grad[self.layout[rest][0]:].zero_()
         handles: list = []
         losses = []
         for k, mb in enumerate(micro):
