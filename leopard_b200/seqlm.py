@@ -869,6 +869,9 @@ class SeqLMEngine:
         # its second appearance and replayed from then on; only the index tables change between replays (LEOPARD_DECODE_GRAPH=0: off)
         import os
         self.use_graphs = self.device.type == "cuda" and os.environ.get("LEOPARD_DECODE_GRAPH", "1") != "0"
+        # pair z of unsorted expert products is row z: made once for the most pairs that run so, because captured steps hold its address
+        self._pair_rows = (torch.arange(MOE_PAIRS_MAX, dtype=I32, device=self.device)
+                           if any(isinstance(lc.ff, MoEConfig) for lc in cfg.layers) else None)
         self._static_tables: Dict = {}
         self._graphs: Dict = {}
         self._seen: Dict = {}
@@ -1361,7 +1364,7 @@ class SeqLMEngine:
                                  ldw=w_dn.stride(1), w_batch=w_dn.stride(0), C=_lib.ptr(y), ldc=y.stride(0), c_batch=0, c_fp32=1, M=1, N=D,
                                  K=f.expert_ff, batch=f.experts, epi=_lib.EPI_NONE, epi_a=0.0, epi_b=0.0)
             self._check(L.lp_linear_pairs(C.byref(d2), _lib.ptr(idx), 1, n_pairs, st), "lp_linear_pairs")
-            return self._moe_combine(f, lw, h, y, self._pair_identity(n_pairs), None if on_input else wts, gate)
+            return self._moe_combine(f, lw, h, y, self._pair_rows, None if on_input else wts, gate)
         tiles = int(L.lp_moe_max_tiles(n_pairs, f.experts, self.tile_rows))
         tile_group = self._empty((tiles,), I32)
         sorted_token = self._empty((tiles * self.tile_rows,), I32)
@@ -1404,12 +1407,6 @@ class SeqLMEngine:
                                  N=D, K=f.expert_ff, batch=1, epi=_lib.EPI_NONE, epi_a=0.0, epi_b=0.0)
             self._check(L.lp_linear_grouped(C.byref(d2), _lib.ptr(tile_group), tiles, None, st), "lp_linear_grouped")
         return self._moe_combine(f, lw, h, y, pair_row, None if on_input else wts, gate)
-
-    def _pair_identity(self, n: int) -> torch.Tensor:
-        t = getattr(self, "_arange", None)
-        if t is None or t.numel() < n:
-            t = self._arange = torch.arange(max(n, 256), dtype=I32, device=self.device)
-        return t
 
     def _moe_combine(self, f: MoEConfig, lw, h, y, pair_row, wts, gate) -> torch.Tensor:
         T, D = h.shape
