@@ -80,6 +80,7 @@ __device__ __forceinline__ void cut3(float x, float y, uint32_t& hi, uint32_t& m
   p = __floats2bfloat162_rn(x, y);
   lo = *reinterpret_cast<const uint32_t*>(&p);
 }
+__device__ __forceinline__ bool not_finite(float v) { return !(fabsf(v) <= 3.402823466e38f); }
 #endif
 
 // prefill kernels are launched with the programmatic-dependent-launch attribute when this is on (lp_set_prefill_pdl):

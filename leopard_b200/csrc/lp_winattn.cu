@@ -739,6 +739,9 @@ window_attn_tile_kernel(WinArgs a, int n_chunks, const int* __restrict__ chunk_s
 // Shared memory holds the terms in planes: queries and keys as [32-channel block][row][64 bytes] (a lane reads eight channels, the same
 // permutation on both sides, eight lanes two neighbouring rows: no bank twice), values transposed as [channel][16 words], the words in the order
 // in which a lane's score fragments become its weight fragments.  The next keys' fp32 rows are copied in (cp.async) meanwhile.
+// An infinity, a NaN and a number that rounds to infinity have no terms (their last one is NaN), and a weight of zero times one of them is NaN in
+// every row of the product, seen or not.  So a CTA with an output that is not finite starts again on wm_plain_chunk: fp32 multiply-adds, each
+// pair over the keys it sees, as window_attn_kernel does.
 // Bound by instruction issue at two warps a scheduler (Q, K and V planes fill shared memory): about 2,000 instructions beside the 384 products
 // of a warp's tile, so rows are looked up once a key (a lane each), chains start from zero in the instruction, masks run only on tiles that
 // need them.  Measured (B200, 4096 tokens, 16 heads on 4, window 1024 + pooled blocks, capped): 0.90 ms a layer, without the cap and blocks 0.76;
@@ -746,9 +749,61 @@ window_attn_tile_kernel(WinArgs a, int n_chunks, const int* __restrict__ chunk_s
 constexpr int WM_D = 128, WM_KT = 32, WM_ROWS = 32, WM_MIN_ROWS = 32;
 template <int QH> constexpr size_t wm_smem_words() { return (size_t)3 * WM_ROWS * QH * WM_D / 2 + 2 * 3 * WM_KT * WM_D / 2 + 2 * WM_KT * WM_D; }
 
+// all pairs of a chunk, a warp to one at a time, a lane to a key and to four channels; f_s: shared memory for the rows and the warps' weights
+template <int QH, bool DIST>
+__device__ __noinline__ void wm_plain_chunk(const WinArgs& a, int seq, int r0, int nrows, int pos0, int kvh, int h0, float* f_s, void* out, long long ldo,
+                                            int out_fp32) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k_off = kvh * WM_D, v_off = a.v_base + kvh * WM_D;
+  const int vhalf = a.v_inv_freq != nullptr ? a.v_rot_dims >> 1 : 0;
+  float* p_s = f_s + WM_ROWS * QH * WM_D + warp * 32;
+  for (int x = warp; x < nrows * QH; x += QH * 2) {
+    const int rq = x / QH, h = h0 + x % QH, pos = pos0 + rq;
+    const WinVisible vis = win_visible(a, pos);
+    const float* q = a.qkv + (long long)(r0 + rq) * a.ld + a.q_off + (long long)h * WM_D;
+    float mx = a.sink ? 0.f : -INFINITY, den = a.sink ? 1.f : 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int t0 = 0; t0 < vis.count; t0 += 32) {
+      const int t = t0 + lane;
+      float s = -INFINITY;
+      if (t < vis.count) {
+        const float* key = win_visible_row(a, vis, seq, t) + k_off;
+        s = 0.f;
+        for (int d = 0; d < WM_D; ++d) s = fmaf(q[d], key[d], s);
+        s *= a.scale;
+        if (a.softcap > 0.f) s = a.softcap * tanhf(s / a.softcap);
+        const int idx = t < vis.n_keep ? t : t < vis.n_keep + vis.n_blocks ? t - vis.n_keep : vis.lo + (t - vis.n_keep - vis.n_blocks);
+        if (DIST) s -= win_distance_bias(a.dist_rate == nullptr, a.dist_amp[h], a.dist_rate != nullptr ? a.dist_rate[h] : 0.f, pos - idx, out_fp32);
+      }
+      float top = s;
+#pragma unroll
+      for (int m = 16; m > 0; m >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, m));
+      const float mn = fmaxf(mx, top), ref = mn == -INFINITY ? 0.f : mn, corr = expf(mx - ref), p = t < vis.count ? expf(s - ref) : 0.f;
+      float sum = p;
+#pragma unroll
+      for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+      den = fmaf(den, corr, sum);
+      mx = mn;
+      p_s[lane] = p;
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) o[i] *= corr;
+      for (int j = 0; j < 32 && t0 + j < vis.count; ++j) {
+        const float* v = win_visible_row(a, vis, seq, t0 + j) + v_off;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[i] = fmaf(p_s[j], v[lane + 32 * i], o[i]);
+      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) f_s[x * WM_D + lane + 32 * i] = den == 0.f ? 0.f : o[i] / den;      // 0: every score was -inf
+    __syncwarp();
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) win_store(a, f_s + x * WM_D, lane + 32 * i, vhalf, pos, r0 + rq, h, out, ldo, out_fp32);
+  }
+}
+
 template <int QH, bool DIST>
 __global__ void __launch_bounds__(QH * 64)
-window_attn_mma_kernel(WinArgs a, int n_chunks, const int* __restrict__ chunk_seq, const int* __restrict__ chunk_row0,
+window_attn_mma_kernel(const __grid_constant__ WinArgs a, int n_chunks, const int* __restrict__ chunk_seq, const int* __restrict__ chunk_row0,
                        const int* __restrict__ chunk_len, const int* __restrict__ row_pos, void* __restrict__ out, long long ldo, int out_fp32) {
   extern __shared__ float dyn_smem[];
   constexpr int X = WM_ROWS * QH, THREADS = QH * 64, Q_PLANE = X * WM_D / 2, K_PLANE = WM_KT * WM_D / 2;      // planes in 32-bit words
@@ -980,7 +1035,15 @@ window_attn_mma_kernel(WinArgs a, int n_chunks, const int* __restrict__ chunk_se
         for (int k = 0; k < 4; ++k) o[n0 + n][k] = fmaf(o[n0 + n][k], corr[k >> 1], d[n][k]);
     }
   }
-  __syncthreads();      // the query planes become the output rows
+  bool odd = false;
+#pragma unroll
+  for (int n = 0; n < WM_D / 8; ++n)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) odd |= not_finite(o[n][k]);
+  if (__syncthreads_or(odd)) {      // and the query planes become the output rows
+    wm_plain_chunk<QH, DIST>(a, seq, r0, nrows, pos0, kvh, h0, dyn_smem, out, ldo, out_fp32);
+    return;
+  }
   float* f_s = dyn_smem;      // [X][WM_D + 4]
 #pragma unroll
   for (int i = 0; i < 2; ++i) {

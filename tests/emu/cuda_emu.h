@@ -26,6 +26,7 @@
 #define __device__
 #define __host__
 #define __forceinline__ inline
+#define __noinline__
 #define __launch_bounds__(...)
 #define __shared__ static
 #define __grid_constant__
@@ -255,6 +256,15 @@ inline unsigned linear_tid() { return threadIdx.x + blockDim.x * (threadIdx.y + 
 }  // namespace emu
 
 inline void __syncthreads() { emu::t_ctx->block_bar->arrive_and_wait(); }
+inline int __syncthreads_or(int pred) {
+  const unsigned t = emu::linear_tid();
+  emu::t_ctx->warp_buf[t] = pred ? 1.f : 0.f;
+  __syncthreads();
+  int any = 0;
+  for (unsigned i = 0; i < blockDim.x * blockDim.y * blockDim.z; ++i) any |= emu::t_ctx->warp_buf[i] != 0.f;
+  __syncthreads();
+  return any;
+}
 inline float __shfl_xor_sync(unsigned mask, float v, int lane_mask) {
   const unsigned t = emu::linear_tid(), w = t >> 5, l = t & 31;
   float* buf = emu::t_ctx->warp_buf.data() + w * 32;

@@ -136,6 +136,7 @@ inline void cut3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
     y -= (float)p.y;
   }
 }
+inline bool not_finite(float v) { return !std::isfinite(v); }
 inline uint32_t smem_u32(const void* p) { return (uint32_t)(uintptr_t)p; }
 struct ProfScope { ProfScope(int, int, int, int, cudaStream_t) {} };
 }  // namespace lp

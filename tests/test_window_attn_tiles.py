@@ -6,6 +6,7 @@ gpu, on the native library.
 Bound: three-term products keep 2^-24 of each factor, sums are short chains added in fp32; with scores of size 4 an error of 1e-6 in a score is
 1e-6 of a weight, so 4e-6 of the result's root mean square; the one-row kernel's FMA chains measure about 3e-7."""
 import ctypes as C
+import math
 
 import pytest
 import torch
@@ -27,7 +28,9 @@ FORMS = {
 }
 
 
-def _run(backend, form, heads, kv_heads, pos0, lens, seed=0):
+def _run(backend, form, heads, kv_heads, pos0, lens, seed=0, plant=None):
+    """errors of (tiles, one-row kernel) against float64; with plant(queries, cached row (request, position), pooled) the tiles' outputs
+    and float64's"""
     device, lib = backend
     L = lib if lib is not None else _lib.stream32_lib()
     st = C.c_void_p(torch.cuda.current_stream().cuda_stream) if device == "cuda" else None
@@ -53,6 +56,9 @@ def _run(backend, form, heads, kv_heads, pos0, lens, seed=0):
             for b in range(t // pool):
                 pooled[i, b // PAGE, b % PAGE] = rows[i][b * pool:(b + 1) * pool].mean(0)
         ptab = torch.arange(pooled.shape[0] * pooled.shape[1], dtype=torch.int32).view(len(lens), -1)
+    if plant is not None:
+        plant(q, lambda i, p: cache[int(table[i, p // PAGE]), p % PAGE], pooled)
+        rows = [torch.stack([cache[int(table[i, p // PAGE]), p % PAGE] for p in range(t)]) for i, t in enumerate(total)]
     amp = torch.rand(heads, generator=g) * 0.3 if "dist" in f else None
     rate = torch.rand(heads, generator=g) if f.get("dist") == "log" else None
     vfreq = 100.0 ** (-torch.arange(f["vrot"] // 2) * 2.0 / f["vrot"]) if "vrot" in f else None
@@ -95,13 +101,16 @@ def _run(backend, form, heads, kv_heads, pos0, lens, seed=0):
                 s = f["softcap"] * torch.tanh(s / f["softcap"])
             if amp is not None:
                 s = s - float(amp[h]) * (torch.log1p(float(rate[h]) * dist) if rate is not None else dist)
-            e = torch.exp(s)
-            want[r, h] = (e / (e.sum() + f.get("sink", 0))) @ v[:, h // (heads // kv_heads)]
+            top = max([0.0] + s[s.isfinite()].tolist())
+            e = torch.exp(s - top)
+            want[r, h] = (e / (e.sum() + f.get("sink", 0) * math.exp(-top))) @ v[:, h // (heads // kv_heads)]
         if vfreq is not None:
             n = f["vrot"] // 2
             ang = (float(p) * vfreq.float()).double()
             x, y = want[r, :, :n].clone(), want[r, :, n:2 * n].clone()
             want[r, :, :n], want[r, :, n:2 * n] = x * ang.cos() + y * ang.sin(), y * ang.cos() - x * ang.sin()
+    if plant is not None:
+        return got.cpu(), want.view(R, -1)
     return rel_err(got, want.view(R, -1)), rel_err(row_wise, want.view(R, -1))
 
 
@@ -116,3 +125,36 @@ def test_forms(backend, form):
 def test_head_groups(backend, heads, kv_heads):
     tiles, row_wise = _run(backend, "kept", heads, kv_heads, [5], [40])
     assert tiles < 4e-6 and tiles < 2 * row_wise + 2e-7, (tiles, row_wise)
+
+
+INF, NAN, TOP = float("inf"), float("nan"), torch.finfo(F32).max
+# what is planted: (form, where, number); values and keys of head 0's key / value head, channel 5
+ODD = {
+    "later value": ("all", lambda q, row, pooled, x: row(0, 20)[D + 5:D + 6].fill_(x)),
+    "value that leaves the window": ("window", lambda q, row, pooled, x: row(0, 4)[D + 5:D + 6].fill_(x)),
+    "later key": ("all", lambda q, row, pooled, x: row(0, 20)[5:6].fill_(x)),
+    "later key under a cap": ("pooled", lambda q, row, pooled, x: row(0, 25)[5:6].fill_(x)),
+    "kept value": ("kept", lambda q, row, pooled, x: row(0, 1)[D + 5:D + 6].fill_(x)),
+    "kept key": ("kept", lambda q, row, pooled, x: row(0, 1)[5:6].fill_(x)),
+    "pooled value": ("pooled", lambda q, row, pooled, x: pooled[0, 0, 0, D + 5:D + 6].fill_(x)),
+    "pooled key": ("pooled", lambda q, row, pooled, x: pooled[0, 0, 0, 5:6].fill_(x)),
+    "key with a distance term": ("bias", lambda q, row, pooled, x: row(0, 20)[5:6].fill_(x)),
+    "query": ("window", lambda q, row, pooled, x: q[7, 5:6].fill_(x)),
+    "query under a cap": ("pooled", lambda q, row, pooled, x: q[7, 5:6].fill_(x)),
+}
+
+
+@pytest.mark.parametrize("what", sorted(ODD))
+@pytest.mark.parametrize("x", [NAN, INF, -INF, TOP], ids=["nan", "inf", "-inf", "largest"])
+def test_unusual_numbers_stay_with_the_rows_that_see_them(backend, what, x):
+    """41 rows in chunks of 32 and 9: what a row does not see does not reach it, a key of score -inf has no weight, an infinite value keeps
+    its sign; the largest fp32 number (of a value: a score of it leaves fp32) rounds to infinity in a bf16 term and is none.  Bound as above."""
+    form, plant = ODD[what]
+    if x == TOP and "value" not in what:
+        pytest.skip("leaves fp32")
+    tiles, want = _run(backend, form, 4, 1, [0], [41], plant=lambda q, row, pooled: plant(q, row, pooled, x))
+    fine = want.isfinite()
+    assert fine.any() and torch.equal(tiles.isfinite(), fine) and torch.equal(tiles.isnan(), want.isnan())
+    assert torch.equal(tiles[tiles.isinf()].double(), want[want.isinf()])
+    usual = fine & (want.abs() < 1e30)
+    assert rel_err(tiles[usual], want[usual]) < 4e-6 and rel_err(tiles[fine] * 2.0 ** -64, want[fine] * 2.0 ** -64) < 4e-6
