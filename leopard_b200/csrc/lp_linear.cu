@@ -332,6 +332,38 @@ __device__ __forceinline__ Bf16Terms split3(const float4& a, const float4& b) {
   r.lo = make_uint4(pack_upper(v[0], v[1]), pack_upper(v[2], v[3]), pack_upper(v[4], v[5]), pack_upper(v[6], v[7]));
   return r;
 }
+// An infinite weight times a term that is zero, or of the other sign, is a NaN that the product of the uncut number is not.  So sums of three-term
+// rows that are not finite are looked at once more, a CTA at a time: each that is NaN is taken again in fp32 multiply-adds (a NaN ends the
+// walk: it stays one).  The walks are functions of their own: in the epilogues their registers made the tile kernel spill (5 to 17 % slower).
+template <typename AT>
+__device__ float lin_plain_dot(const AT* x, const bf16* w, int K) {
+  float s = 0.f;
+#pragma unroll 1
+  for (int k = 0; k < K && s == s; ++k) s = fmaf(lin_load(x + k), lin_load(w + k), s);
+  return s;
+}
+// linear_stream_kernel: `here` rows from m0 on, the first warp's share takes the new sum
+template <typename AT, int NT, int MG>
+__device__ __noinline__ void lin_mend_sums(float* sums, const AT* A, long long lda, const int* pair_of, int a_div, const bf16* W, long long ldw, int K,
+                                           int m0, int here, int n0, int n_out, int gated) {
+  const int n_warps = blockDim.x >> 5, cols = gated ? 8 * NT : 16 * NT;
+  for (int e = threadIdx.x; e < cols * here; e += blockDim.x) {
+    const int nl = e % cols, ml = e / cols, n = n0 + nl;
+    if (n >= n_out) continue;
+    const int j = gated ? nl >> 3 : nl >> 4, r = gated ? nl & 7 : nl & 15;
+    const int at = (((j * MG + (ml >> 3)) * 4 + (r >> 3) * 2 + (ml & 1)) * 32) + (r & 7) * 4 + ((ml & 7) >> 1);
+    const AT* x = A + (long long)(pair_of != nullptr ? pair_of[m0 + ml] / a_div : m0 + ml) * lda;
+    for (int half = 0; half < (gated ? 2 : 1); ++half) {
+      float* p = sums + at + 64 * half;
+      float s = 0.f;
+      for (int w = 0; w < n_warps; ++w) s += p[w * NT * MG * 4 * 32];
+      if (s == s) continue;
+      p[0] = lin_plain_dot(x, W + (long long)(n + half * n_out) * ldw, K);
+      for (int w = 1; w < n_warps; ++w) p[w * NT * MG * 4 * 32] = 0.f;
+    }
+  }
+  __syncthreads();
+}
 // the two halves of a step of 32 products, in chains of their own
 __device__ __forceinline__ void mma_step(float* d, float* e, const uint4& w0, const uint4& w1, const uint4& x) {
   mma_bf16(d, w0.x, w1.x, w0.y, w1.y, x.x, x.y);
@@ -480,14 +512,23 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
           for (int c = 0; c < 4; ++c) acc[j][i][c] += run[j][i][c];
     }
     if (m0 > 0) __syncthreads();      // the sums of the rows before have been read
+    bool odd = false;
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
       for (int i = 0; i < MG; ++i)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) dyn_smem[(warp * SLOTS + (j * MG + i) * 4 + c) * 32 + lane] = acc[j][i][c];
-    __syncthreads();
+        for (int c = 0; c < 4; ++c) {
+          dyn_smem[(warp * SLOTS + (j * MG + i) * 4 + c) * 32 + lane] = acc[j][i][c];
+          if constexpr (sizeof(AT) == 4) odd |= not_finite(acc[j][i][c]);
+        }
     const int here = min(8 * MG, rows - m0);
+    if constexpr (sizeof(AT) == 4) {
+      if (__syncthreads_or(odd))
+        lin_mend_sums<AT, NT, MG>(dyn_smem, A, a.lda, pairs ? pair_of : nullptr, a.a_div, W, a.ldw, a.K, m0, here, n0, n_out, gated);
+    } else {
+      __syncthreads();
+    }
     for (int e = threadIdx.x; e < cols * here; e += blockDim.x) {
       const int nl = e % cols, ml = e / cols, n = n0 + nl;
       if (n >= n_out) continue;
@@ -572,6 +613,23 @@ static int dispatch_stream(const LinArgs& a, int a_fp32, int c_fp32, int batch, 
 // bf16 rows 0.72 ms; mma.sync alone reaches 520 TFLOP/s of bf16 products here, 450 with a sum of its own every few.  Error against 64 bits at
 // K = 1024 / 4096: 1.2e-7 / 2.1e-7 (FMA chains over K: 5.7e-7 / 1.1e-6).
 constexpr int MT_BM = LIN_BM, MT_BN = 128, MT_BK = 32, MT_LDC = MT_BN + 4, MT_THREADS = 256;
+
+// the tile's sums in shared memory (a gated unit's halves eight columns apart), rows from m0 and output columns from n0 on
+template <typename AT>
+__device__ __noinline__ void lin_mend_tile(float* tile, const AT* A, long long lda, const int* a_rows, const bf16* W, long long ldw, int K, int m0,
+                                           int M, int n0, int n_out, int gated) {
+  const int cols = gated ? MT_BN / 2 : MT_BN;
+  for (int e = threadIdx.x; e < MT_BM * cols; e += MT_THREADS) {
+    const int ml = e / cols, nl = e % cols, m = m0 + ml, n = n0 + nl;
+    if (m >= M || n >= n_out) continue;
+    const long long r = a_rows != nullptr ? a_rows[m] : m;
+    for (int half = 0; half < (gated ? 2 : 1); ++half) {
+      float* s = tile + ml * MT_LDC + (gated ? (nl >> 3) * 16 + (nl & 7) + 8 * half : nl);
+      if (r >= 0 && *s != *s) *s = lin_plain_dot(A + r * lda, W + (long long)(n + half * n_out) * ldw, K);
+    }
+  }
+  __syncthreads();
+}
 
 template <typename AT>
 __global__ void __launch_bounds__(MT_THREADS, 2) linear_mma_kernel(LinArgs a, int gated, int c_fp32) {
@@ -677,13 +735,21 @@ __global__ void __launch_bounds__(MT_THREADS, 2) linear_mma_kernel(LinArgs a, in
     __syncthreads();
   }
   // through shared memory, so that one copy of the epilogue's code serves whole rows (the stages are no longer read)
+  bool odd = false;
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < NI; ++j)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) dyn_smem[(wm + 16 * i + g + 8 * (c >> 1)) * MT_LDC + wn + 8 * j + 2 * t + (c & 1)] = acc[i][j][c];
-  __syncthreads();
+      for (int c = 0; c < 4; ++c) {
+        dyn_smem[(wm + 16 * i + g + 8 * (c >> 1)) * MT_LDC + wn + 8 * j + 2 * t + (c & 1)] = acc[i][j][c];
+        if constexpr (PLANES == 3) odd |= not_finite(acc[i][j][c]);
+      }
+  if constexpr (PLANES == 3) {
+    if (__syncthreads_or(odd)) lin_mend_tile(dyn_smem, A, a.lda, a.a_rows, W, a.ldw, a.K, m0, a.M, n0, n_out, gated);
+  } else {
+    __syncthreads();
+  }
 #pragma unroll 1
   for (int e = tid; e < BM * cols; e += THREADS) {
     const int ml = e / cols, nl = e % cols, m = m0 + ml, n = n0 + nl;

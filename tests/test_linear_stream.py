@@ -116,6 +116,41 @@ def test_unusual_numbers(backend):
 
 
 @pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("M,kind", [(5, "rows"), (40, "rows"), (70, "rows"), (5, "pairs"), (64, "groups")])
+def test_infinite_weights(backend, dtype, M, kind):
+    """an infinite weight makes its column's outputs infinite, with the sign of the product, in both halves of a gated unit too; NaN where it
+    meets a zero, an infinity of the other sign or a NaN"""
+    N, K, dev = 24, 40, backend[0]
+    a, w, _, _, _ = _data(M, N, K, dtype, dev)
+    a[0, 3], a[1, 5] = 0.0, float("nan")
+    w[2, 3], w[5, 3], w[7, 11], w[7, 12], w[N // 2 + 3, 30] = float("inf"), -float("inf"), float("inf"), -float("inf"), float("inf")
+    want = a.double() @ w.double().T
+    ad, wd = a.to(dev), w.to(dev)
+    out, half = torch.empty(M, N, device=dev), torch.empty(M, N // 2, device=dev)
+
+    def call(o, **kw):
+        if kind == "groups":
+            L = _lib_of(backend)
+            d = _lib.LinearDesc(A=_lib.ptr(ad), lda=K, a_fp32=int(dtype == F32), W=_lib.ptr(wd), ldw=K, w_batch=N * K, C=_lib.ptr(o), ldc=o.stride(0),
+                                c_fp32=1, M=M, N=N, K=K, batch=1, **kw)
+            rows, group = torch.arange(M, dtype=torch.int32, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+            stream = C.c_void_p(torch.cuda.current_stream().cuda_stream) if ad.is_cuda else None
+            assert L.lp_linear_grouped(C.byref(d), _lib.ptr(group), 1, _lib.ptr(rows), stream) == 0
+        elif kind == "pairs":
+            _call(backend, ad, wd[None].expand(2, N, K).contiguous(), o, 1, batch=2, pairs=torch.arange(M, device=dev).to(torch.int32) % 2, **kw)
+        else:
+            _call(backend, ad, wd, o, M, **kw)
+
+    call(out)
+    assert torch.equal(out.cpu().isnan(), want.isnan()) and torch.equal(out.cpu()[want.isinf()].double(), want[want.isinf()])
+    assert rel_err(out.cpu()[want.isfinite()], want[want.isfinite()]) < 2e-6
+    call(half, epi=_lib.EPI_SILU_GATE)
+    g = want[:, : N // 2].float()
+    unit = g / (1 + torch.exp(-g)) * want[:, N // 2:].float()      # in fp32, where exp(-(-inf)) is an infinity too
+    assert torch.equal(half.cpu().isnan(), unit.isnan()) and torch.equal(half.cpu()[unit.isinf()], unit[unit.isinf()])
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
 def test_row_tiles_of_groups(backend, dtype):
     """tiles of 64 gathered rows, each on its group's weight; padding rows are zeros, a tile without a group is left alone"""
     g = torch.Generator().manual_seed(9)
