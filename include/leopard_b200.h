@@ -613,9 +613,11 @@ int lp_linear(const lp_linear_desc* desc, void* stream);
  * tile is skipped); a_rows[row] (optional) = the A row to read for that row of the sorted space (< 0: zeros). */
 int lp_linear_grouped(const lp_linear_desc* desc, const int* tile_group, int n_tiles, const int* a_rows, void* stream);
 int lp_linear_tile_rows(void);
-/* n_pairs one-row problems: problem z = A row z / a_div times the weight of group pair_group[z] -> C row z (weight-streaming kernel).
- * batch > 1: the number of groups — every group's weights are then read once for all of its pairs (pair_group[z] < batch). */
+/* n_pairs one-row problems: problem z = A row z / a_div times the weight of group pair_group[z] -> C row z (weight-streaming kernel;
+ * M and batch of the description are not read) */
 int lp_linear_pairs(const lp_linear_desc* desc, const int* pair_group, int a_div, int n_pairs, void* stream);
+/* the same with the number of groups (0 <= pair_group[z] < n_groups; others are not computed): a group's weights are read once for its pairs */
+int lp_linear_group_pairs(const lp_linear_desc* desc, const int* pair_group, int n_groups, int a_div, int n_pairs, void* stream);
 
 /* out[r, :] = table[ids[r], :] * scale */
 int lp_embed_rows_f32(const int* ids, int R, const void* table, long long ldt, int vocab, float scale, float* out, long long ldo, int D,

@@ -855,9 +855,7 @@ extern "C" int lp_linear(const lp_linear_desc* d, void* stream_) {
   return dispatch_linear(a, d->a_fp32, d->c_fp32, d->batch, (d->M + LIN_BM - 1) / LIN_BM, true, stream);
 }
 
-// n_pairs one-row problems on the weight-streaming kernel: problem z multiplies A row z / a_div by the weight of group pair_group[z]
-// (w_batch elements apart) into C row z — the expert products of a decode step, where every (token, choice) pair has its own weight.
-extern "C" int lp_linear_pairs(const lp_linear_desc* d, const int* pair_group, int a_div, int n_pairs, void* stream_) {
+static int linear_pairs(const lp_linear_desc* d, const int* pair_group, int n_groups, int a_div, int n_pairs, void* stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LP_REQUIRE(d != nullptr && d->A != nullptr && d->W != nullptr && d->C != nullptr && pair_group != nullptr, "lp_linear_pairs: null operand");
   LP_REQUIRE(d->N > 0 && d->K > 0 && a_div >= 1 && n_pairs >= 0 && n_pairs <= 65535, "lp_linear_pairs: bad problem N=%d K=%d pairs=%d", d->N,
@@ -874,10 +872,23 @@ extern "C" int lp_linear_pairs(const lp_linear_desc* d, const int* pair_group, i
   a.a_rows = nullptr; a.tile_group = nullptr; a.z_group = pair_group; a.a_div = a_div;
   a.bias = d->bias; a.row_scale = d->row_scale; a.gate = d->gate; a.ldg = d->ldg; a.gate_batch = d->gate_batch;
   a.seg_cols = 0; a.n_segs = 0; a.a_seg = 0;
-  // with the number of groups (batch > 1) a group's weights are read once for all of its pairs
-  if (d->batch > 1 && n_pairs <= STREAM_MAX_PAIRS && stream_ok(a, d->a_fp32, 1))
-    return dispatch_stream(a, d->a_fp32, d->c_fp32, 1, 2 * ((n_pairs + d->batch - 1) / d->batch), d->batch, n_pairs, stream);
+  // with the number of groups a group's weights are read once for all of its pairs
+  if (n_groups > 0 && n_pairs <= STREAM_MAX_PAIRS && stream_ok(a, d->a_fp32, 1))
+    return dispatch_stream(a, d->a_fp32, d->c_fp32, 1, 2 * ((n_pairs + n_groups - 1) / n_groups), n_groups, n_pairs, stream);
   return dispatch_linear(a, d->a_fp32, d->c_fp32, n_pairs, 1, true, stream);
+}
+
+// n_pairs one-row problems on the weight-streaming kernel: problem z multiplies A row z / a_div by the weight of group pair_group[z]
+// (w_batch elements apart) into C row z — the expert products of a decode step, where every (token, choice) pair has its own weight.
+extern "C" int lp_linear_pairs(const lp_linear_desc* d, const int* pair_group, int a_div, int n_pairs, void* stream) {
+  return linear_pairs(d, pair_group, 0, a_div, n_pairs, stream);
+}
+
+// the same for a caller that knows the number of groups (pair_group[z] < n_groups): a CTA a group and column tile reads the weights once
+// for all of the group's pairs
+extern "C" int lp_linear_group_pairs(const lp_linear_desc* d, const int* pair_group, int n_groups, int a_div, int n_pairs, void* stream) {
+  LP_REQUIRE(n_groups >= 1 && n_groups <= 65535, "lp_linear_group_pairs: %d groups", n_groups);
+  return linear_pairs(d, pair_group, n_groups, a_div, n_pairs, stream);
 }
 
 extern "C" int lp_linear_grouped(const lp_linear_desc* d, const int* tile_group, int n_tiles, const int* a_rows, void* stream_) {

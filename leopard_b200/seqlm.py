@@ -1357,13 +1357,13 @@ class SeqLMEngine:
             h1 = self._empty((n_pairs, f.expert_ff), self.act)
             d1 = _lib.LinearDesc(A=_lib.ptr(h), lda=h.stride(0), a_batch=0, a_fp32=int(h.dtype == F32), W=_lib.ptr(w_gu), ldw=w_gu.stride(1),
                                  w_batch=w_gu.stride(0), C=_lib.ptr(h1), ldc=h1.stride(0), c_batch=0, c_fp32=int(h1.dtype == F32), M=1,
-                                 N=2 * f.expert_ff, K=D, batch=f.experts, epi=epi, epi_a=epi_a, epi_b=epi_b, row_scale=_lib.ptr(wts) if on_input else None)
-            self._check(L.lp_linear_pairs(C.byref(d1), _lib.ptr(idx), f.top, n_pairs, st), "lp_linear_pairs")
+                                 N=2 * f.expert_ff, K=D, batch=1, epi=epi, epi_a=epi_a, epi_b=epi_b, row_scale=_lib.ptr(wts) if on_input else None)
+            self._check(L.lp_linear_group_pairs(C.byref(d1), _lib.ptr(idx), f.experts, f.top, n_pairs, st), "lp_linear_group_pairs")
             y = self._empty((n_pairs, D), F32)
             d2 = _lib.LinearDesc(A=_lib.ptr(h1), lda=h1.stride(0), a_batch=0, a_fp32=int(h1.dtype == F32), W=_lib.ptr(w_dn),
                                  ldw=w_dn.stride(1), w_batch=w_dn.stride(0), C=_lib.ptr(y), ldc=y.stride(0), c_batch=0, c_fp32=1, M=1, N=D,
-                                 K=f.expert_ff, batch=f.experts, epi=_lib.EPI_NONE, epi_a=0.0, epi_b=0.0)
-            self._check(L.lp_linear_pairs(C.byref(d2), _lib.ptr(idx), 1, n_pairs, st), "lp_linear_pairs")
+                                 K=f.expert_ff, batch=1, epi=_lib.EPI_NONE, epi_a=0.0, epi_b=0.0)
+            self._check(L.lp_linear_group_pairs(C.byref(d2), _lib.ptr(idx), f.experts, 1, n_pairs, st), "lp_linear_group_pairs")
             return self._moe_combine(f, lw, h, y, self._pair_rows, None if on_input else wts, gate)
         tiles = int(L.lp_moe_max_tiles(n_pairs, f.experts, self.tile_rows))
         tile_group = self._empty((tiles,), I32)

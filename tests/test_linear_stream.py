@@ -1,4 +1,4 @@
-"""The weight-streaming product of up to 64 rows (lp_linear), of grouped pairs (lp_linear_pairs with the number of groups) and the tile
+"""The weight-streaming product of up to 64 rows (lp_linear), of grouped pairs (lp_linear_group_pairs) and the tile
 product of more rows (lp_linear, lp_linear_grouped) against a float64 product: the edges of their row groups, column tiles and K steps, both
 operand types, every kind of epilogue; on the kernel sources under the CPU emulator and, marked gpu, on the native library.
 
@@ -19,7 +19,7 @@ def _lib_of(backend):
     return backend[1] if backend[1] is not None else _lib.stream32_lib()
 
 
-def _call(backend, a, w, out, M, batch=1, pairs=None, a_div=1, **kw):
+def _call(backend, a, w, out, M, batch=1, pairs=None, groups=None, a_div=1, **kw):
     L = _lib_of(backend)
     stream = C.c_void_p(torch.cuda.current_stream().cuda_stream) if a.is_cuda else None
     d = _lib.LinearDesc(A=_lib.ptr(a), lda=a.stride(-2), a_batch=kw.pop("a_batch", 0), a_fp32=int(a.dtype == F32), W=_lib.ptr(w), ldw=w.stride(-2),
@@ -27,8 +27,10 @@ def _call(backend, a, w, out, M, batch=1, pairs=None, a_div=1, **kw):
                         c_fp32=int(out.dtype == F32), M=M, N=w.shape[-2], K=w.shape[-1], batch=batch, **{k: _lib.ptr(v) if isinstance(v, torch.Tensor) else v for k, v in kw.items()})
     if pairs is None:
         rc = L.lp_linear(C.byref(d), stream)
-    else:
+    elif groups is None:
         rc = L.lp_linear_pairs(C.byref(d), _lib.ptr(pairs), a_div, pairs.numel(), stream)
+    else:
+        rc = L.lp_linear_group_pairs(C.byref(d), _lib.ptr(pairs), groups, a_div, pairs.numel(), stream)
     assert rc == 0, L.lp_last_error()
 
 
@@ -94,8 +96,12 @@ def test_pairs_of_groups(backend, dtype, n_pairs, groups):
     w = (torch.randn(groups + 1, N, K, generator=g) * K ** -0.5).to(BF16)      # nobody chooses the last group
     of = torch.randint(0, groups, (n_pairs,), generator=g).to(torch.int32)
     out = torch.empty(n_pairs, N, device=backend[0])
-    _call(backend, a.to(backend[0]), w.to(backend[0]), out, 1, batch=groups + 1, pairs=of.to(backend[0]), a_div=2)
+    _call(backend, a.to(backend[0]), w.to(backend[0]), out, 1, groups=groups + 1, pairs=of.to(backend[0]), a_div=2)
     want = torch.stack([w[int(e)].double() @ a[z // 2].double() for z, e in enumerate(of)])
+    assert rel_err(out, want) < 2e-6
+    # without the number of groups a description's batch means nothing, whatever it holds
+    out.fill_(9.0)
+    _call(backend, a.to(backend[0]), w.to(backend[0]), out, 1, batch=groups - 1, pairs=of.to(backend[0]), a_div=2)
     assert rel_err(out, want) < 2e-6
 
 
@@ -137,7 +143,7 @@ def test_infinite_weights(backend, dtype, M, kind):
             stream = C.c_void_p(torch.cuda.current_stream().cuda_stream) if ad.is_cuda else None
             assert L.lp_linear_grouped(C.byref(d), _lib.ptr(group), 1, _lib.ptr(rows), stream) == 0
         elif kind == "pairs":
-            _call(backend, ad, wd[None].expand(2, N, K).contiguous(), o, 1, batch=2, pairs=torch.arange(M, device=dev).to(torch.int32) % 2, **kw)
+            _call(backend, ad, wd[None].expand(2, N, K).contiguous(), o, 1, groups=2, pairs=torch.arange(M, device=dev).to(torch.int32) % 2, **kw)
         else:
             _call(backend, ad, wd, o, M, **kw)
 
