@@ -287,15 +287,17 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) linear_rows_kernel(LinArgs a)
 // Up to 64 rows (decoding): a product is bound by reading its weights once, at every number of rows, when the multiply-adds are
 // out of the way.  So the weight tile is the 16-row operand of the warp's matrix instruction and up to MG groups of eight rows of A
 // are its other one: a CTA owns 16 NT output columns, its warps share out K in steps of 32 (a lane reads 16 bytes of each weight row and of its
-// row of A; the same permutation of k on both sides, which a sum does not see), eight weight loads per lane are in flight before the
-// first product, and the warps' sums meet in shared memory, warp by warp in a fixed order.  The gated units take gate row n and up
-// row n + N / 2 as rows g and g + 8 of one tile, so both halves of an output end up in one lane.
+// row of A; the same permutation of k on both sides, which a sum does not see), 4 NT weight loads per lane (2 NT from 17 rows on, where registers
+// are short) are in flight before the first product, and the warps' sums meet in shared memory in a fixed order, what each addition rounds
+// off kept and added at the end.  The gated units take gate row n and up row n + N / 2 as rows g and g + 8 of one tile, so both halves of an
+// output end up in one lane.
 // fp32 rows of A are cut into three bf16 terms that add up to them exactly (8 + 8 + 8 bits): every product is still exact.  The
-// instruction cuts its running sum off instead of rounding it, a bias that grows with the chain: every 16 products start a
-// chain of their own (small terms first) and are added to the sum in fp32.
-// Measured (B200, graph of launches, weights from HBM, M = 8): N = 8192, K = 2048 9.8 us (3.4 TB/s; a warp per column with fp32 FMAs: 67.6),
-// N = 32000, K = 4096 53 us (4.9 TB/s; 350), N = 2048, K = 2048 5.8 us (29.7), fp32 A 10.9 us (66).  Error against 64 bits at K = 2048
-// / 8192: 0.9e-7 / 1.2e-7 of the result (FMA chains of a lane: 0.8e-7 / 1.25e-7; of the tile kernel: 3.9e-7 / 9.6e-7).
+// instruction cuts its running sum off instead of rounding it, a bias that grows with the chain.  So chains are short and added in fp32: 16
+// products of bf16 rows, 3 x 16 of fp32 rows (small terms first), 256 of 33 to 64 bf16 rows, whose additions would cost more than the products.
+// Measured (B200, graph of launches, weights from HBM, M = 8): N = 8192, K = 2048 10.4 us (3.2 TB/s; a warp per column with fp32 FMAs: 67.6),
+// N = 32000, K = 4096 51 us (5.1 TB/s; 350), N = 2048, K = 2048 6.6 us (29.7), fp32 A 6.5 us (66).  Error against 64 bits at N = 2048, K = 2048 /
+// 8192, 1e-7 of the result: bf16 rows 0.58 / 0.70 (without what the sums of the warps round off 0.92 / 1.23; FMA chains of a lane, which this
+// kernel replaced, 0.80 / 1.24), fp32 rows 0.75 / 1.0 (1.6 / 2.9), 64 bf16 rows 2.3 / 2.3 (FMA chains over K 3.9 / 9.5).
 // Pairs (experts): the CTAs of weight group blockIdx.y gather the pairs that chose it and read the group's weights once for all of them.
 constexpr int STREAM_MAX_ROWS = 64, STREAM_MAX_PAIRS = 1024;
 
@@ -331,6 +333,13 @@ __device__ __forceinline__ Bf16Terms split3(const float4& a, const float4& b) {
   r.mid.x = take_upper(v[0], v[1]); r.mid.y = take_upper(v[2], v[3]); r.mid.z = take_upper(v[4], v[5]); r.mid.w = take_upper(v[6], v[7]);
   r.lo = make_uint4(pack_upper(v[0], v[1]), pack_upper(v[2], v[3]), pack_upper(v[4], v[5]), pack_upper(v[6], v[7]));
   return r;
+}
+// s <- s + v, rounded; the exact rest of that sum (Knuth's two-sum)
+__device__ __forceinline__ float add_exactly(float& s, float v) {
+  const float t = s + v, u = t - s;
+  const float rest = (s - (t - u)) + (v - u);
+  s = t;
+  return rest;
 }
 // An infinite weight times a term that is zero, or of the other sign, is a NaN that the product of the uncut number is not.  So sums of three-term
 // rows that are not finite are looked at once more, a CTA at a time: each that is NaN is taken again in fp32 multiply-adds (a NaN ends the
@@ -534,11 +543,13 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
       if (n >= n_out) continue;
       const int j = gated ? nl >> 3 : nl >> 4, r = gated ? nl & 7 : nl & 15;
       const int at = (((j * MG + (ml >> 3)) * 4 + (r >> 3) * 2 + (ml & 1)) * 32) + (r & 7) * 4 + ((ml & 7) >> 1);
-      float s = 0.f, s2 = 0.f;
+      float s = 0.f, s2 = 0.f, lost = 0.f, lost2 = 0.f;      // what the additions round off is added at the end
       for (int w = 0; w < n_warps; ++w) {
-        s += dyn_smem[w * SLOTS * 32 + at];
-        if (gated) s2 += dyn_smem[w * SLOTS * 32 + at + 64];
+        lost += add_exactly(s, dyn_smem[w * SLOTS * 32 + at]);
+        if (gated) lost2 += add_exactly(s2, dyn_smem[w * SLOTS * 32 + at + 64]);
       }
+      if (s + lost == s + lost) s += lost;      // beside an infinity the rest is NaN
+      if (s2 + lost2 == s2 + lost2) s2 += lost2;
       const int m = pairs ? pair_of[m0 + ml] : m0 + ml;
       if (a.row_scale != nullptr) {
         s *= a.row_scale[m];

@@ -105,6 +105,22 @@ def test_pairs_of_groups(backend, dtype, n_pairs, groups):
     assert rel_err(out, want) < 2e-6
 
 
+@pytest.mark.parametrize("M,N,K", [(4, 96, 512), (8, 48, 2048)])
+def test_few_rows_lose_no_more_than_a_lane_of_multiply_adds(backend, M, N, K):
+    """bf16 rows up to eight against float64, beside what fp32 multiply-adds of a warp's lanes and a tree over the lanes lose on the same data"""
+    a, w, want, ad, wd = _data(M, N, K, BF16, backend[0])
+    out = torch.empty(M, N, device=backend[0])
+    _call(backend, ad, wd, out, M)
+    lanes = torch.zeros(M, N, 32)
+    for k in range(0, K, 256):
+        for i in range(8):      # lane l takes k + 8 l .. k + 8 l + 7
+            x, y = a[:, k + i:k + 256:8].double(), w[:, k + i:k + 256:8].double()
+            lanes = (lanes.double() + x[:, None] * y[None]).float()      # one rounding, as a fused multiply-add
+    for half in (16, 8, 4, 2, 1):
+        lanes = lanes[..., :half] + lanes[..., half:2 * half]
+    assert rel_err(out, want) < 1.05 * rel_err(lanes[..., 0], want)
+
+
 def test_unusual_numbers(backend):
     """an infinity or a NaN in a row of A stays in its row, as it does in an fp32 product; the largest number is no infinity"""
     M, N, K = 5, 16, 40
