@@ -886,17 +886,17 @@ class SeqLMEngine:
     def _empty(self, shape, dtype):
         return torch.empty(shape, dtype=dtype, device=self.device)
 
-    def _on_tensor_cores(self, a, w, M, N, K) -> bool:
-        """The tcgen05 GEMM takes a product when it is large enough to fill tiles and meets the 16-byte rules of its TMA loads."""
-        return M >= (self.tensor_core_rows or 0) and self._fits_tensor_cores(a, w, N, K)
-
-    def _streams(self, a, w, M, N, K) -> bool:
-        """lp_linear's weight-streaming kernel takes a product of few rows, unless the GEMM can and has the columns to be faster"""
-        return M <= STREAM_ROWS_ALONE or (M <= STREAM_ROWS and (M * N <= STREAM_MAX_OUTPUTS or not self._fits_tensor_cores(a, w, N, K)))
-
-    def _fits_tensor_cores(self, a, w, N, K) -> bool:
-        return (self.tensor_core_rows is not None and a.dtype == BF16 and N >= 128 and K >= 64 and N % 8 == 0 and K % 8 == 0
-                and a.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and a.stride(1) == 1 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+    def _on_gemm(self, a: torch.Tensor, w: torch.Tensor) -> bool:
+        """Whether the tcgen05 GEMM takes a[M, K] @ w[N, K].T: it has the rows to fill tiles, or (above the few rows that are always streamed)
+        the columns to be faster than lp_linear's weight-streaming kernel, and its TMA loads can start on 16-byte boundaries.  A limit
+        above TENSOR_CORE_MIN_ROWS (tensor_core_rows; None: never) holds for every product."""
+        (M, K), N = a.shape, w.shape[0]
+        if self.tensor_core_rows is None or M < self.tensor_core_rows > TENSOR_CORE_MIN_ROWS:
+            return False
+        if M <= STREAM_ROWS_ALONE or (M <= STREAM_ROWS and M * N <= STREAM_MAX_OUTPUTS):
+            return False
+        return (a.dtype == BF16 and N >= 128 and K >= 64 and N % 8 == 0 and K % 8 == 0 and a.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
+                and a.stride(1) == 1 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
     def linear(self, a: torch.Tensor, w: torch.Tensor, out_dtype, epi=_lib.EPI_NONE, epi_a=0.0, epi_b=0.0, out=None, into=None, bias=None,
                row_scale=None):
@@ -906,7 +906,7 @@ class SeqLMEngine:
         N = w.shape[0]
         n_out = N // 2 if epi in _lib.GATED_EPIS else N
         # a row scale reaches the tensor-core path only through the activation kernel that follows the product
-        tc = not self._streams(a, w, M, N, K) and self._fits_tensor_cores(a, w, N, K) and (row_scale is None or (epi != _lib.EPI_NONE and bias is None))
+        tc = self._on_gemm(a, w) and (row_scale is None or (epi != _lib.EPI_NONE and bias is None))
         if into is not None:
             x, mult = into[0], into[1]
             gate = into[2] if len(into) > 2 else None
@@ -951,7 +951,7 @@ class SeqLMEngine:
         out = self._empty((R, N), F32)
         parts = [(ops[i], w[a:b], out[:, a:b]) for i, (a, b) in enumerate(zip(bounds, bounds[1:]))]
         fits = seg % (_lib.LINEAR_ROWS_COLS if R <= _lib.LINEAR_ROWS_MAX else self.tile_rows) == 0
-        if not fits or any(not self._streams(a, wi, R, wi.shape[0], D) and self._fits_tensor_cores(a, wi, wi.shape[0], D) for a, wi, _ in parts):
+        if not fits or any(self._on_gemm(a, wi) for a, wi, _ in parts):
             for a, wi, o in parts:
                 self.linear(a, wi, F32, out=o)
             return out
