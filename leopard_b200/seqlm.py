@@ -36,7 +36,13 @@ TENSOR_CORE_MIN_ROWS = 64
 # rows times columns, the tcgen05 GEMM's latency with K alone: they cross near rows * columns = 170,000 (K = 2048: 32 rows by 8192
 # columns 17.3 us against 13.7, 16 rows 11.5 against 14.4, 64 rows by 2048 columns 18.7 against 13.4, 32 rows 9.9 against 12.7)
 STREAM_ROWS, STREAM_ROWS_ALONE, STREAM_MAX_OUTPUTS = 64, 8, 170_000
-MOE_PAIRS_MAX = 512            # up to this many (token, choice) pairs an expert's weights are streamed once for the pairs that chose it
+# Up to MOE_PAIRS_MAX (token, choice) pairs an expert's weights are streamed once for the pairs that chose it.  Both products of 16 experts,
+# width 2048, 1024 inside (us, bf16; fp32 rows), against sorted tiles: 128 pairs 66, 108; 85, 182.  256 pairs 93, 108; 138, 182.  512 pairs 161,
+# 108; 282, 182: with this few experts the sorted tiles are ahead from about 300 pairs, with 32 (width 4096) not yet at 512: 554, 683; 876, 1116.
+# Rows that are not whole 16-byte pieces cannot be streamed so: each pair reads its expert's weights, and beyond MOE_PAIRS_ALONE pairs sorting is
+# faster (width 2044, 1020 inside, 16 experts: 64 pairs 481, 488; 128 pairs 936, 488).
+MOE_PAIRS_MAX = 512
+MOE_PAIRS_ALONE = 64
 PAD_PROJECTION_ROWS = 128      # a projection narrower than a tensor-core tile is padded with zero rows beside ones that are at least this wide
 MAX_DECODE_GRAPHS = 32         # captured decode layouts kept at a time
 PAGE_TABLE_STEP = 16           # decode batches round their page-table width up to a multiple of this
@@ -1351,7 +1357,7 @@ class SeqLMEngine:
                                 _lib.ptr(lw["w_sg"]) if gate is not None else None, _lib.ptr(idx), _lib.ptr(wts), _lib.ptr(gate), st)
         self._check(rc, "lp_moe_route")
         n_pairs = T * f.top
-        if n_pairs <= MOE_PAIRS_MAX:
+        if n_pairs <= (MOE_PAIRS_MAX if D % 8 == 0 and f.expert_ff % 8 == 0 else MOE_PAIRS_ALONE):
             # few (token, choice) pairs (decoding): no sorting — an expert's weights are streamed once for its pairs, pair z = row z
             w_gu, w_dn = lw["w_gu"], lw["w_edown"]
             h1 = self._empty((n_pairs, f.expert_ff), self.act)

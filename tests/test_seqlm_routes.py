@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from leopard_b200 import _lib
-from leopard_b200.seqlm import MOE_PAIRS_MAX, STREAM_MAX_OUTPUTS, StepEntry
+from leopard_b200.seqlm import MOE_PAIRS_ALONE, MOE_PAIRS_MAX, STREAM_MAX_OUTPUTS, StepEntry
 from oracle import seqlm as O
 from seqlm_common import TOL, backend, dense, emu_lib, latent_layer, make_engine, model, moe, rel_err, retention_layer  # noqa: F401  (fixtures)
 
@@ -94,16 +94,17 @@ def test_captured_steps_on_both_sides_of_the_crossover(requests, wide):
     assert rel_err(got, torch.stack([want[k][1:] for k in toks])) < TOL["bfloat16"]
 
 
-@pytest.mark.parametrize("ff", [moe(), moe(experts=4, top=1, groups=1, keep=1, ff=8, shared=0)], ids=["moe", "moe-top1"])
+@pytest.mark.parametrize("ff,width,limit", [(moe(), 32, MOE_PAIRS_MAX), (moe(experts=4, top=1, groups=1, keep=1, ff=8, shared=0), 32, MOE_PAIRS_MAX),
+                                            (moe(ff=6), 32, MOE_PAIRS_ALONE), (moe(), 36, MOE_PAIRS_ALONE)], ids=["moe", "moe-top1", "ff6", "width36"])
 @pytest.mark.parametrize("over", [0, 1])
-def test_experts_on_both_sides_of_the_pair_limit(backend, ff, over):
-    """the most pairs that run without sorting, and one token more: tiles of the sorted rows"""
+def test_experts_on_both_sides_of_the_pair_limit(backend, ff, width, limit, over):
+    """the most pairs that run without sorting, and one token more: tiles of the sorted rows; fewer where rows are not whole 16-byte pieces"""
     top = ff["router"]["top"]
-    T = MOE_PAIRS_MAX // top + over
-    cfg = model([retention_layer(mlp=ff)])
+    T = limit // top + over
+    cfg = model([retention_layer(mlp=ff)], width=width)
     w = O.random_weights(cfg, seed=1)
     eng = make_engine(cfg, w, backend)
-    h = torch.randn(T, 32, generator=torch.Generator().manual_seed(T))
+    h = torch.randn(T, width, generator=torch.Generator().manual_seed(T))
     want = O.feed_forward(h.double(), {k: v.double() for k, v in w.items()}, "l0.mlp.", ff)
     eng.L = _Spy(eng.L)
     got = eng._moe(eng.cfg.layers[0].ff, eng.w.layers[0], h.to(backend[0]))
