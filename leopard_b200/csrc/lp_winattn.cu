@@ -746,7 +746,7 @@ window_attn_tile_kernel(WinArgs a, int n_chunks, const int* __restrict__ chunk_s
 // of a warp's tile, so rows are looked up once a key (a lane each), chains start from zero in the instruction, masks run only on tiles that
 // need them.  Measured (B200, 4096 tokens, 16 heads on 4, window 1024 + pooled blocks, capped): 0.90 ms a layer, without the cap and blocks 0.76;
 // fp32 multiply-adds (window_attn_tile_kernel, which keeps other head sizes) 1.90; the first form of this kernel 1.07.
-constexpr int WM_D = 128, WM_KT = 32, WM_ROWS = 32, WM_MIN_ROWS = 32;
+constexpr int WM_D = 128, WM_KT = 32, WM_ROWS = 32;
 template <int QH> constexpr size_t wm_smem_words() { return (size_t)3 * WM_ROWS * QH * WM_D / 2 + 2 * 3 * WM_KT * WM_D / 2 + 2 * WM_KT * WM_D; }
 
 // all pairs of a chunk, a warp to one at a time, a lane to a key and to four channels; f_s: shared memory for the rows and the warps' weights
@@ -1530,6 +1530,19 @@ static int launch_window_attn_tiles(const WinArgs& a, int R, int n_chunks, const
   return 0;
 }
 
+// Prompts on the matrix instructions where their tiles fill and the chip has enough of them; elsewhere window_attn_tile_kernel, whose CTAs hold 2 or
+// 4 rows.  A CTA walks its keys alone, so what counts is the rows (times groups of query heads) an SM gets, and how full the chunks are.  Mostly
+// full ones come from long prompts, whose first chunks see few keys: they need more.  Measured (us, tile kernel against this one, window 1024;
+// rows x query heads on key / value heads): 512 x 8 on 2 79, 116; 1024 x 8 on 2 219, 216; 2048 x 8 on 2 449, 226; 512 x 16 on 4 133, 116; 1024 x 2 on 1
+// 110, 163 (two heads a CTA); 1280 x 4 on 2 182, 168; a head a CTA (two CTAs an SM): 512 x 8 on 8 89, 102; 768 x 8 on 8 154, 151; 1280 x 8 on 8
+// 299, 205.  64 portions after 700 tokens: of 8 rows x 16 on 4 316, 349; of 12 452, 351; of 16 589, 354; of 8 x 8 on 2 156, 178; of 12 290, 179; of 8 x 4
+// on 4 122, 163; of 12 227, 167.
+static bool wm_pays(int R, int n_chunks, int heads, int qh) {
+  const bool full = R >= 24LL * n_chunks;
+  const int rows_an_sm = qh == 1 ? (full ? 36 : 20) : (full ? 14 : 10);
+  return (long long)R * (heads / qh) >= (long long)rows_an_sm * sm_count() && R >= 12LL * n_chunks;
+}
+
 template <int QH, bool DIST>
 static int launch_window_attn_mma(const WinArgs& a, int n_chunks, const int* chunk_seq, const int* chunk_row0, const int* chunk_len, const int* row_pos,
                                   void* out, long long ldo, int out_fp32, cudaStream_t stream) {
@@ -1649,8 +1662,8 @@ extern "C" int lp_window_attn_tiles(const lp_window_attn_desc* d, int R, const i
              d->vdim, WIN_MAX_DIM);
   if (R <= 0 || n_chunks <= 0) return 0;
   const int ratio = d->heads / d->kv_heads;
-  // heads of 128 whose cache rows are whole 16-byte pieces run on the matrix instructions; a handful of rows leaves their tiles empty
-  if (d->dim == WM_D && d->vdim == WM_D && R >= WM_MIN_ROWS && a.roww % 4 == 0 && a.v_base % 4 == 0 && (reinterpret_cast<uintptr_t>(a.cache) & 15) == 0 &&
+  // heads of 128 whose cache rows are whole 16-byte pieces run on the matrix instructions when that pays
+  if (d->dim == WM_D && d->vdim == WM_D && wm_pays(R, n_chunks, d->heads, ratio % 4 == 0 ? 4 : ratio % 2 == 0 ? 2 : 1) && a.roww % 4 == 0 && a.v_base % 4 == 0 && (reinterpret_cast<uintptr_t>(a.cache) & 15) == 0 &&
       (a.pool == 0 || (reinterpret_cast<uintptr_t>(a.pooled) & 15) == 0)) {
 #define LP_WM(QH)                                                                                                                              \
   (d->dist_amp != nullptr ? launch_window_attn_mma<QH, true>(a, n_chunks, chunk_seq, chunk_row0, chunk_len, row_pos, out, ldo, out_fp32, stream) \

@@ -97,7 +97,8 @@ inline void set_error(const char* fmt, ...) {
 inline void note_launch(int = 1) {}
 inline void pdl_wait() {}
 inline void pdl_launch_dependents() {}
-inline int sm_count() { return 4; }
+inline int g_emu_sms = 4;      // emu_set_sm_count: rules that count CTAs per SM
+inline int sm_count() { return g_emu_sms; }
 inline float2 fma2(float2 a, float2 b, float2 c) { return {std::fma(a.x, b.x, c.x), std::fma(a.y, b.y, c.y)}; }
 inline float2 mul2(float2 a, float2 b) { return {a.x * b.x, a.y * b.y}; }
 inline uint4 ldg_once(const void* p) { return *reinterpret_cast<const uint4*>(p); }

@@ -28,10 +28,15 @@ FORMS = {
 }
 
 
-def _run(backend, form, heads, kv_heads, pos0, lens, seed=0, plant=None):
+def _run(backend, form, heads, kv_heads, pos0, lens, seed=0, plant=None, rule=False):
     """errors of (tiles, one-row kernel) against float64; with plant(queries, cached row (request, position), pooled) the tiles' outputs
-    and float64's"""
+    and float64's.  The matrix-instruction kernel takes launches that fill the chip: here the emulator has no SMs to fill, and on a GPU the heads
+    are so many times as many, unless `rule` leaves the sizes and the emulator's four SMs as they are."""
     device, lib = backend
+    if device == "cuda" and not rule:
+        qh = next(q for q in (4, 2, 1) if heads // kv_heads % q == 0)
+        times = -(-(36 if qh == 1 else 14) * torch.cuda.get_device_properties(0).multi_processor_count // (sum(lens) * (heads // qh)))
+        heads, kv_heads = heads * times, kv_heads * times
     L = lib if lib is not None else _lib.stream32_lib()
     st = C.c_void_p(torch.cuda.current_stream().cuda_stream) if device == "cuda" else None
     g = torch.Generator().manual_seed(seed)
@@ -80,8 +85,12 @@ def _run(backend, form, heads, kv_heads, pos0, lens, seed=0, plant=None):
         window=f.get("window", 0), keep_first=f.get("keep_first", 0), scale=D ** -0.5, softcap=f.get("softcap", 0.0), sink=f.get("sink", 0),
         chunk=f.get("chunk", 0), kv_shared=1, dist_amp=_lib.ptr(t["amp"]), dist_rate=_lib.ptr(t["rate"]), out_scale=1.0)
     got, row_wise = torch.full((R, heads * D), 9.0, device=device), torch.empty(R, heads * D, device=device)
+    if lib is not None and not rule:
+        lib.emu_set_sm_count(0)
     rc = L.lp_window_attn_tiles(C.byref(d), R, _lib.ptr(t["row_seq"]), _lib.ptr(t["row_pos"]), len(chunks), _lib.ptr(t["cs"]), _lib.ptr(t["cr"]),
                                 _lib.ptr(t["cl"]), _lib.ptr(got), heads * D, 1, st)
+    if lib is not None:
+        lib.emu_set_sm_count(4)
     assert rc == 0, L.lp_last_error()
     assert L.lp_window_attn(C.byref(d), R, _lib.ptr(t["row_seq"]), _lib.ptr(t["row_pos"]), _lib.ptr(row_wise), heads * D, 1, st) == 0
     want = torch.zeros(R, heads, D, dtype=torch.float64)
@@ -128,15 +137,19 @@ def test_head_groups(backend, heads, kv_heads):
 
 
 INF, NAN, TOP = float("inf"), float("nan"), torch.finfo(F32).max
+def _value(row):
+    return row[len(row) // 2 + 5:len(row) // 2 + 6]
+
+
 # what is planted: (form, where, number); values and keys of head 0's key / value head, channel 5
 ODD = {
-    "later value": ("all", lambda q, row, pooled, x: row(0, 20)[D + 5:D + 6].fill_(x)),
-    "value that leaves the window": ("window", lambda q, row, pooled, x: row(0, 4)[D + 5:D + 6].fill_(x)),
+    "later value": ("all", lambda q, row, pooled, x: _value(row(0, 20)).fill_(x)),
+    "value that leaves the window": ("window", lambda q, row, pooled, x: _value(row(0, 4)).fill_(x)),
     "later key": ("all", lambda q, row, pooled, x: row(0, 20)[5:6].fill_(x)),
     "later key under a cap": ("pooled", lambda q, row, pooled, x: row(0, 25)[5:6].fill_(x)),
-    "kept value": ("kept", lambda q, row, pooled, x: row(0, 1)[D + 5:D + 6].fill_(x)),
+    "kept value": ("kept", lambda q, row, pooled, x: _value(row(0, 1)).fill_(x)),
     "kept key": ("kept", lambda q, row, pooled, x: row(0, 1)[5:6].fill_(x)),
-    "pooled value": ("pooled", lambda q, row, pooled, x: pooled[0, 0, 0, D + 5:D + 6].fill_(x)),
+    "pooled value": ("pooled", lambda q, row, pooled, x: _value(pooled[0, 0, 0]).fill_(x)),
     "pooled key": ("pooled", lambda q, row, pooled, x: pooled[0, 0, 0, 5:6].fill_(x)),
     "key with a distance term": ("bias", lambda q, row, pooled, x: row(0, 20)[5:6].fill_(x)),
     "query": ("window", lambda q, row, pooled, x: q[7, 5:6].fill_(x)),
@@ -158,3 +171,12 @@ def test_unusual_numbers_stay_with_the_rows_that_see_them(backend, what, x):
     assert torch.equal(tiles[tiles.isinf()].double(), want[want.isinf()])
     usual = fine & (want.abs() < 1e30)
     assert rel_err(tiles[usual], want[usual]) < 4e-6 and rel_err(tiles[fine] * 2.0 ** -64, want[fine] * 2.0 ** -64) < 4e-6
+
+
+@pytest.mark.parametrize("heads,kv_heads,lens", [
+    (4, 1, [32, 24]), (4, 1, [32, 23]), (16, 4, [12, 12, 12]), (16, 4, [12, 12, 11]), (2, 2, [72]), (2, 2, [64]), (2, 2, [20, 20]), (2, 2, [20, 19])])
+def test_both_sides_of_the_rule(backend, heads, kv_heads, lens):
+    """on the emulator's four SMs the first of each pair has the rows and the filled chunks for the matrix-instruction kernel, the second just
+    not"""
+    tiles, row_wise = _run(backend, "window", heads, kv_heads, [7] * len(lens), lens, rule=True)
+    assert tiles < 4e-6 and tiles < 2 * row_wise + 2e-7, (tiles, row_wise)
