@@ -1601,10 +1601,13 @@ extern "C" int lp_window_attn(const lp_window_attn_desc* d, int R, const int* ro
              WIN_MAX_DIM);
   if (R <= 0) return 0;
   const int ratio = d->heads / d->kv_heads;
-  // query heads of a key / value head share the reading of its rows, four to a CTA — unless that leaves SMs without one: the rows of a
-  // decode step are in L2, and a CTA's chain over its keys is what takes the time (one row, 32 heads on 8, 500 keys: two launches 67 -> 41 us)
+  // Query heads of a key / value head share the reading of its rows, four to a CTA, where there are CTAs for half of the SMs: the rows of a decode
+  // step are in L2, and with fewer CTAs a CTA's chain over its keys is what takes the time, so each head gets one.  Measured (us, four heads
+  // a CTA against one, 500 / 3000 keys, window 1024): one row of 8 heads on 2 32 / 58, 19 / 34; 32 rows of 8 on 2 57 / 137, 34 / 112; against two,
+  // where there would be 80 CTAs 58 / 173, 61 / 210, 128 CTAs 59 / 207, 81 / 222.  Heads in pairs: one a CTA below a CTA an SM.
   int qh = ratio % 4 == 0 ? 4 : ratio % 2 == 0 ? 2 : 1;
-  while (qh > 1 && (long long)R * (d->heads / qh) < sm_count()) qh >>= 1;
+  const long long ctas = (long long)R * (d->heads / qh);
+  if (qh == 4 ? 2 * ctas < sm_count() : ctas < sm_count()) qh = 1;
 #define LP_WA(QH)                                                                                                   \
   (d->dist_amp != nullptr ? launch_window_attn<QH, true>(a, R, row_seq, row_pos, out, ldo, out_fp32, stream) \
                           : launch_window_attn<QH, false>(a, R, row_seq, row_pos, out, ldo, out_fp32, stream))

@@ -180,3 +180,11 @@ def test_both_sides_of_the_rule(backend, heads, kv_heads, lens):
     not"""
     tiles, row_wise = _run(backend, "window", heads, kv_heads, [7] * len(lens), lens, rule=True)
     assert tiles < 4e-6 and tiles < 2 * row_wise + 2e-7, (tiles, row_wise)
+
+
+@pytest.mark.parametrize("heads,kv_heads,rows", [(4, 1, 1), (8, 1, 1), (16, 2, 1), (2, 1, 3), (2, 1, 4), (6, 1, 1)])
+def test_one_row_steps_with_and_without_shared_rows(backend, heads, kv_heads, rows):
+    """the one-row kernel with a query head a CTA and with two or four: on the emulator's four SMs the first, fourth and last launches have a head
+    a CTA, the others share"""
+    _, row_wise = _run(backend, "kept", heads, kv_heads, [9] * rows, [1] * rows, rule=True)
+    assert row_wise < 4e-6
