@@ -69,3 +69,15 @@ def test_activations_and_update(backend, N, ld):
     xd, yd = x.clone().to(device), y.to(device)
     assert L.lp_axpy_f32(_lib.ptr(xd), ld, _lib.ptr(yd), N, 0.5, M, N, st) == 0
     assert rel_err(xd[:, :N], x[:, :N].double() + 0.5 * y.double()) < 1e-6 and torch.equal(xd[:, N:].cpu(), x[:, N:])
+
+
+@pytest.mark.parametrize("D", [4, 30, 512, 516, 1030, 2052])
+def test_embedding_rows(backend, D):
+    """the numbers of threads that widths take, four columns a thread and one; an id outside the table reads its first row"""
+    device, L, st = _setup(backend)
+    g = torch.Generator().manual_seed(D)
+    table, ids = torch.randn(7, D, generator=g).to(BF16), torch.tensor([3, 0, 6, 9, -1], dtype=torch.int32)
+    out = torch.empty(5, D, device=device)
+    td, idd = table.to(device), ids.to(device)
+    assert L.lp_embed_rows_f32(_lib.ptr(idd), 5, _lib.ptr(td), D, 7, 0.5, _lib.ptr(out), D, D, st) == 0
+    assert torch.equal(out.cpu(), table[[3, 0, 6, 0, 0]].float() * 0.5)
