@@ -125,8 +125,7 @@ int lp_tp_reduce(const lp_tp_desc* tp, const void* stage, long long ld, const vo
 /* GEMM scheduling mode: 0 = one CTA per 128-row tile; 1 = CTA pairs (thread-block cluster of 2, tcgen05
  * cta_group::2, 256-row tiles) for problems with at least one tile per SM pair.  Returns the previous mode.
  * Results are identical up to fp32 summation order (same K order: bit-identical in practice).
- * 2 = 4-CTA clusters: two pairs on column-adjacent tiles share the A tile by TMA multicast (-25 % L2 reads per tile);
- *     opt-in, verified under the CPU emulator only so far. */
+ * Every other value is taken as 1 (2 was a variant in clusters of four, slower and with the same bits). */
 int lp_gemm_set_pair_mode(int enable);
 
 /* Stream-K tail of lp_gemm_bf16 / lp_gemm_bf16_ex (large problems whose last wave of tiles would leave most SMs idle, e.g. the

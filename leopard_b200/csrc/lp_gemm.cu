@@ -824,17 +824,6 @@ extern "C" int lp_gemm_bf16_ex(const lp_gemm_desc* d, void* stream_) {
   if (rc) return rc;
   ProfScope prof(1, M, N, K, stream);
   note_launch();
-  const bool plain = d->norm_mode == LP_NORM_NONE && d->stats_out == nullptr && d->rope_heads == 0;
-  if (plain && pair && g_gemm_pair_mode == 2 && (block_n == 256 || block_n == 192 || block_n == 128) && args.num_n_blk >= 2) {
-    // two pairs per 4-CTA cluster on column-adjacent tiles, A multicast between them (lp_gemm4.cu): work units are
-    // (row block, column-block pair); A is requested in 64-row boxes
-    GemmArgs a4 = args;
-    a4.num_n_blk = (args.num_n_blk + 1) / 2;
-    CUtensorMap tmAh;
-    rc = make_tmap_bf16_2d(&tmAh, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, GEMM_BK, GEMM_BM / 2);
-    if (rc) return rc;
-    return launch_gemm4(tmAh, tmB, tmC, a4, block_n, stream);
-  }
   if (g_sk_enable && g_sk_ws != nullptr && M >= 1024) {
     // stream-K tail: when the last wave would be mostly idle, the last 1 + fraction waves of tiles are cut along K so that every
     // unit gets the same number of k-blocks (gemm_schedule); bit-identical results (the accumulator is handed over, not re-added)
@@ -1033,6 +1022,6 @@ extern "C" int lp_gemm_set_streamk(int enable) {
 
 extern "C" int lp_gemm_set_pair_mode(int enable) {
   const int old = g_gemm_pair_mode;
-  g_gemm_pair_mode = enable == 2 ? 2 : (enable ? 1 : 0);   // 2 = 4-CTA clusters with A multicast (lp_gemm4.cu, opt-in)
+  g_gemm_pair_mode = enable ? 1 : 0;
   return old;
 }

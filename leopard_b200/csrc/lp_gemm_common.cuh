@@ -1,5 +1,5 @@
-// leopard_b200 — pieces shared by the tcgen05 GEMM kernels (lp_gemm.cu: one CTA or a CTA pair per tile; lp_gemm4.cu: two pairs
-// per 4-CTA cluster sharing the A tile by TMA multicast): tile geometry, launch arguments, shared-memory plan, tile
+// leopard_b200 — pieces shared by the tcgen05 GEMM kernels (lp_gemm.cu: one CTA or a CTA pair per tile; lp_gemm_chain.cu: two GEMMs in
+// one launch): tile geometry, launch arguments, shared-memory plan, tile
 // rasterisation and the epilogue (bias / activation / residual / fp32 or swizzled-staging bf16 stores).
 #pragma once
 #include "lp_common.cuh"
@@ -144,12 +144,6 @@ struct GemmSegMaps {
 };
 
 enum { LP_NORM_NONE_ = 0, LP_NORM_RMS_ = 1, LP_NORM_LAYER_ = 2 };
-
-#ifndef LP_EMULATE
-// 4-CTA-cluster variant (lp_gemm4.cu); args.num_n_blk counts column-block pairs, tmAh has 64-row boxes
-int launch_gemm4(const CUtensorMap& tmAh, const CUtensorMap& tmB, const CUtensorMap& tmC, const GemmArgs& args, int block_n,
-                 cudaStream_t stream);
-#endif
 
 // EPI_BUFS: 2 KiB staging tiles per epilogue warp — 1 = output staging only; 3 = ring shared by the TMA-loaded residual tile and
 // the output tile (the TMARES kernels: residual chunk g + 1 lands while chunk g is added in place and chunk g - 1 is stored)

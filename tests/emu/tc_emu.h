@@ -11,8 +11,7 @@
 //              CTAs of a pair (A rows and B rows split between their shared memories, D rows between their TMEMs)
 //   TMEM       128 lanes x 512 columns of 32-bit cells per CTA; 32x32b loads / stores address lane = base lane + lane id
 //   cluster    clusters of 2 or 4 CTAs run concurrently (emu_tc::launch_clusters): %cluster_ctarank, mapa, remote mbarrier
-//              arrive, barrier.cluster, masked multicast commits, cta_group::2 multicast TMA loads (bytes counted on each
-//              destination's pair leader)
+//              arrive, barrier.cluster, masked multicast commits
 //   named barriers  bar.sync / bar.arrive id, n
 // The layouts are the author's reading of the hardware, the same reading the GPU-verified kernels are built on; the emulator
 // checks a kernel's LOGIC (protocol, indexing, masks, operand roles), not the hardware.
@@ -260,16 +259,6 @@ inline void tma_load_tile_to(emu_tc::Cta& dst_cta, uint32_t dst, const CUtensorM
 inline void tma_load_tile(void* smem_dst, const CUtensorMap* m, uint32_t bar_addr, int c0, int c1, int c2) {
   tma_load_tile_to(emu_tc::cta(), smem_u32(smem_dst), m, c0, c1, c2);
   mbar_complete_tx_addr(bar_addr, m->box[0] * m->box[1] * m->elem_bytes);
-}
-// cta_group::2 multicast: the box lands at the same offset in every CTA of the mask; each destination's bytes are counted on
-// the barrier at the given offset in that destination's PAIR LEADER (even rank)
-inline void tma_load_2d_pair_mcast(void* smem_dst, const CUtensorMap* m, uint32_t bar_cluster_addr, int c0, int c1, uint16_t mask) {
-  const uint32_t dst = smem_u32(smem_dst), boff = emu_tc::off_of(bar_cluster_addr);
-  for (uint32_t d = 0; d < 4; ++d)
-    if (mask & (1u << d)) {
-      tma_load_tile_to(emu_tc::g_cta[d], dst, m, c0, c1, 0);
-      mbar_complete_tx_addr(boff | (((d & ~1u) + 1u) << 28), m->box[0] * m->box[1] * m->elem_bytes);
-    }
 }
 inline void tma_load_3d(void* d, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2) { tma_load_tile(d, m, smem_u32(bar), c0, c1, c2); }
 inline void tma_load_2d(void* d, const CUtensorMap* m, uint64_t* bar, int c0, int c1) { tma_load_tile(d, m, smem_u32(bar), c0, c1, 0); }

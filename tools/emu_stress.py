@@ -1,8 +1,8 @@
-"""Randomised runs of the CPU-emulated kernels that have not been on hardware yet: the flash attention backward
-(lp_attn_bwd.cu) and the 4-CTA multicast GEMM (lp_gemm4.cu).  Builds the same emulation libraries as the CPU tests, then draws
+"""Randomised runs of the CPU-emulated attention kernels: the flash attention backward
+(lp_attn_bwd.cu).  Builds the same emulation libraries as the CPU tests, then draws
 shapes until the time budget is spent.  Scheduling noise of the OS threads varies from run to run, which is the point: a protocol
 race shows up as a mismatch or as the emulator's deadlock abort.
-    python tools/emu_stress.py [--seconds 300] [--which attn,gemm4] [--seed 1]
+    python tools/emu_stress.py [--seconds 300] [--which attn,fwd] [--seed 1]
 `--which fwd` adds the forward attention kernels whose scheduling changed last (lp_attn3.cu: next S half loaded before the hand-over,
 alternating pv_done barriers; lp_attn5.cu: persistent CTAs, barrier parities running across items) — 765 random cases in 600 s
 passed before the round closed.
@@ -54,23 +54,6 @@ def build_attn(out):
     return _gxx(out, "attn_bwd_emu.cpp", "libattn.so")
 
 
-def build_gemm(out):
-    _helpers(out, "// UMMA descriptors", fix_tanh=True)
-
-    def part(path, end):
-        src = (ROOT / path).read_text()
-        return src[src.index("namespace lp {"):src.index(end)].replace("extern __shared__ uint8_t smem_raw[];",
-                                                                       "uint8_t* smem_raw = emu_tc::cta().smem;")
-
-    shared = (ROOT / "leopard_b200/csrc/lp_gemm_common.cuh").read_text()
-    shared = shared[shared.index("namespace lp {"):].replace('asm volatile("bar.sync 1, 256;" ::: "memory");', "named_bar(1, 256, true);")
-    k1 = part("leopard_b200/csrc/lp_gemm.cu", "template <int BN, int STAGES, bool CTA2>\nstatic int launch_gemm(")
-    k4 = part("leopard_b200/csrc/lp_gemm4.cu", "#ifndef LP_EMULATE\ntemplate <int BN, int STAGES>\nstatic int launch4(")
-    (out / "gemm_kernel.inc").write_text(shared + "\n" + k1 + "\n}  // namespace lp\n")
-    (out / "gemm4_kernel.inc").write_text(k4 + "\n}  // namespace lp\n")
-    return _gxx(out, "gemm_emu.cpp", "libgemm.so", "-DLP_EMULATE=1")
-
-
 def attn_case(L, n):
     hd, hs = random.choice([(128, 128), (128, 128), (72, 80)])
     causal = False if hd == 72 else random.choice([True, True, False])
@@ -95,30 +78,6 @@ def attn_case(L, n):
                         int(causal), C.c_float(hd ** -0.5), P(got), LL(got.stride(0)), P(lse), P(dl), 3)
     e = float((got.float() - want.float()).abs().max() / (want.float().abs().max() + 1e-12))
     return (e > 2e-2 or bool(torch.isnan(got.float()).any())), f"B{B} T{T} heads {heads}/{kvh} causal={causal} hd={hd}: {e:.4f}"
-
-
-def gemm4_case(L, n):
-    bn = random.choice([128, 128, 192, 256])
-    M, K = random.choice([130, 256, 300, 512, 777]), random.choice([64, 72, 136, 200, 320])
-    N = bn * random.choice([2, 3, 4, 5]) - random.choice([0, 0, 8, 40, bn // 2])
-    act = random.choice([0, 0, 1, 2, 3])
-    if act == 3:
-        N -= N % 64
-    bias, res = random.random() < 0.5, random.random() < 0.5
-    fp32 = act != 3 and random.random() < 0.3
-    res = res and not fp32
-    ctas, gm = random.choice([4, 8, 12]), random.choice([1, 2, 3])
-    g = torch.Generator().manual_seed(n)
-    a = torch.randn((M, K), generator=g).to(BF)
-    w = (torch.randn((N, K), generator=g) * K ** -0.5).to(BF)
-    b = torch.randn(N, generator=g) if bias else None
-    no = N // 2 if act == 3 else N
-    r = torch.randn((M, no), generator=g).to(BF) if res else None
-    want = ref.gemm(a, w, bias=b, residual=r, act=act, out_fp32=fp32)
-    out = torch.full((M, no), float("nan"), dtype=torch.float32 if fp32 else BF)
-    L.emu_gemm4(P(a), LL(K), P(w), LL(K), P(out), LL(no), M, N, K, P(b), P(r), LL(no), 0, act, int(fp32), bn, gm, ctas)
-    e = float((out.float() - want.float()).abs().max() / (want.float().abs().max() + 1e-12))
-    return (e > 8e-3 or bool(torch.isnan(out.float()).any())), f"M{M} N{N} K{K} bn{bn} act{act} bias={bias} res={res} fp32={fp32} ctas={ctas}: {e:.2e}"
 
 
 def build_fwd(out):
@@ -175,7 +134,7 @@ def fwd_case(libs, n):
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--seconds", type=int, default=300)
-    ap.add_argument("--which", default="attn,gemm4")
+    ap.add_argument("--which", default="attn")
     ap.add_argument("--seed", type=int, default=1)
     a = ap.parse_args()
     random.seed(a.seed)
@@ -186,9 +145,6 @@ def main():
         if "attn" in which:
             (out / "a").mkdir()
             jobs.append(("attn", build_attn(out / "a"), attn_case))
-        if "gemm4" in which:
-            (out / "g").mkdir()
-            jobs.append(("gemm4", build_gemm(out / "g"), gemm4_case))
         if "fwd" in which:
             (out / "f").mkdir()
             jobs.append(("fwd", build_fwd(out / "f"), fwd_case))

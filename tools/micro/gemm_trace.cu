@@ -5,7 +5,6 @@
 //   tools/micro/gemm_trace <M> <N> <K> <bias 0|1> <act> <residual 0|1> <cta to trace>
 #define LP_GEMM_TRACE 1
 #include "../../leopard_b200/csrc/lp_host.cu"
-#include "../../leopard_b200/csrc/lp_gemm4.cu"
 #include "../../leopard_b200/csrc/lp_gemm.cu"
 #include <cstdio>
 #include <cstdlib>
