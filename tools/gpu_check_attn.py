@@ -1,4 +1,4 @@
-"""GPU-side check + timing of lp_attention_fwd against torch fp32 SDPA (run under gpurun)."""
+"""GPU-side check + timing of lp_attention_fwd against torch fp32 SDPA."""
 import argparse
 import json
 import sys

@@ -1,4 +1,4 @@
-"""GPU-side check + timing of lp_gemm_bf16 against torch fp32 matmul (run under gpurun).
+"""GPU-side check + timing of lp_gemm_bf16 against torch fp32 matmul.
 
 Usage: python tools/gpu_check_gemm.py [--case NAME] [--list] [--time]
 Each case prints one JSON line; failures print an error-pattern summary to help debug descriptor/layout bugs.

@@ -1,6 +1,6 @@
 """Decode-step kernels in isolation for ncu (eager launches, GEMV mode): one cfg3 prefill, then a few greedy steps.
     ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum --clock-control none \
-        -k regex:'gemv_kernel|decode_' -s 400 -c 200 --csv --log-file gpurun_out/decode_launches.csv \
+        -k regex:'gemv_kernel|decode_' -s 400 -c 200 --csv --log-file decode_launches.csv \
         python tools/gpu_decode_prof.py
 """
 import os

@@ -1,4 +1,4 @@
-"""Greedy decode speed of the native generate() (SURVEY.md §8f-2) on the cfg3 request: ms per generated token for each
+"""Greedy decode speed of the native generate() on the cfg3 request: ms per generated token for each
 decode implementation, against the HBM floor (every decoder weight + the KV cache read once per token).
 
   mode 0 eager : first implementation, M = 1 rows through the tcgen05 GEMM, one launch per op
@@ -7,7 +7,7 @@ decode implementation, against the HBM floor (every decoder weight + the KV cach
   mode 5 graph : block-cooperative GEMV kernels, CUDA-graph replay (default)
   mode 7 graph : + programmatic dependent launch edges
   mode 21      : one persistent cooperative kernel per token (eager / graph)
-Writes one JSON line per variant to stdout (and to gpurun_out/decode_speed.json when that directory exists).
+Writes one JSON line per variant to stdout.
 """
 import json
 import os
@@ -85,6 +85,3 @@ for mode, graph in ((0, "0"), (1, "1"), (5, "0"), (5, "1"), (7, "1"), (21, "0"),
     print(json.dumps(rec), flush=True)
     out.append(rec)
 _lib.lib().lp_decode_set_mode(7)
-od = Path(__file__).resolve().parents[1] / "gpurun_out"
-if od.exists():
-    (od / "decode_speed.json").write_text("\n".join(json.dumps(r) for r in out) + "\n")

@@ -1,4 +1,4 @@
-"""BASELINE.json configs[3] (Leopard-Idefics2, 8 images 980x980 -> 8 x 4900 patches -> 512 image rows + 64 text ids,
+"""The Idefics2 configuration (Leopard-Idefics2, 8 images 980x980 -> 8 x 4900 patches -> 512 image rows + 64 text ids,
 S = 576) on the native path with device-side random weights: timing of one request per step (parity of this path is
 tests/test_gpu_idefics2.py; this is a measurement aid, not the bench line)."""
 import json

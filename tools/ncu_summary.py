@@ -1,6 +1,6 @@
 """Summarise an .ncu-rep (ncu --set full) into a small text table for profiles/ (read here, no GPU needed).
 
-usage: python tools/ncu_summary.py gpurun_out/prof.ncu-rep > profiles/<name>.txt
+usage: python tools/ncu_summary.py prof.ncu-rep > profiles/<name>.txt
 """
 import csv
 import subprocess
