@@ -6,7 +6,7 @@
                                                             (oracle port, host cores, bounded sample; rank 0 only)
 
 Metric  : prefill tokens/sec = merged decoder rows (image rows + text rows) processed / time, whole job.
-Workload: BASELINE.json configs[2] — 4 images 896x1152 -> adaptive allocation -> 28 crops (4 x (6 tiles + global)),
+Workload: 4 images 896x1152 -> adaptive allocation -> 28 crops (4 x (6 tiles + global)),
           64 text ids + 28 placeholders -> S = 4796 merged rows; ONE such request per GPU per step (the config's batch
           of 8 spread over 8 GPUs = weak scaling: per-GPU work fixed as N grows).  Synthetic weights/pixels/ids.
 A step  : ViT over 28 crops -> pixel-shuffle + projector -> embed+merge -> 32-layer decoder -> last-token logits.
@@ -31,7 +31,7 @@ ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
 N_TEXT = 64
-# (width, height) lists — BASELINE.json configs[2] (the metric's configuration) and configs[1]
+# (width, height) lists — cfg3 is the metric's configuration
 WORKLOADS = {
     "cfg3": {"images": [(896, 1152)] * 4,
              "label": "cfg3: LLaVA 4x(896x1152) -> adaptive allocation -> 28 crops, 92 prompt ids -> S=4796 merged rows"},
@@ -136,7 +136,7 @@ def workload_config(name, per_image, S, world):
 
 
 def flops_model(n_crops, S, cfg):
-    """Algorithmic FLOPs of one step (SURVEY.md §8d)."""
+    """Algorithmic FLOPs of one step."""
     T = cfg.vit.tokens
     vit = n_crops * (27 * (30_449_664 * T + 4608 * T * T) + 1_354_752 * T)
     proj = n_crops * 2 * 169 * (4608 * 4096 + 4096 * 4096)
@@ -190,7 +190,7 @@ def run_reference(args):
 
 # ------------------------------------------------------------------------------------------------ extras (rank 0, N = 1)
 def decode_extra(model, ids_h, pix_h, cfg, S, peaks, n_new=65):
-    """Greedy decode after the prefill (SURVEY.md §8f-2): ms per generated token from generate(n_new) - generate(1),
+    """Greedy decode after the prefill: ms per generated token from generate(n_new) - generate(1),
     against the HBM floor (every decoder weight + lm_head + the KV cache read once per token)."""
     import time
     import torch
@@ -219,7 +219,7 @@ def decode_extra(model, ids_h, pix_h, cfg, S, peaks, n_new=65):
 
 
 def frontend_extra(model, ids_h, cfg, S, dev, steps):
-    """GPU image front-end (SURVEY.md §8f-3) on the same request given as raw images: 4 x (896 x 1152) RGB uint8 ->
+    """GPU image front-end on the same request given as raw images: 4 x (896 x 1152) RGB uint8 ->
     28 crops.  Times the front-end alone (pinned uint8 H2D + kernels), the request end to end from raw images, and the
     reference's host path (PIL resize/pad/tile + processor arithmetic, 1 thread) on this box; checks bit-exactness."""
     import time
@@ -504,7 +504,7 @@ def run_ours(args):
                              "tflops": round(2.0 * a * b * c * v[1] / (v[0] * 1e-3) / 1e12, 1)}
                             for (a, b, c), v in sorted(gemm_shapes.items(), key=lambda kv: -kv[1][0])],
             "flops": {kk: float(v) for kk, v in fm.items()},
-            # BASELINE.json's "ViT+decoder % roofline": algorithmic FLOPs of the stage / the stage's time against the measured
+            # "ViT+decoder % roofline": algorithmic FLOPs of the stage / the stage's time against the measured
             # sustained cuBLAS bf16 peak.  `roofline_by_stage` times each stage on its own exactly as the step launches it (no
             # events between kernels; the three add up to the step); `roofline_by_stage_kernel_events` is the earlier basis — the
             # summed per-kernel CUDA-event intervals of one profiled step, which carry the event pair and the lost launch overlap of

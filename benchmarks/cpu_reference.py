@@ -1,5 +1,5 @@
 """CPU arm of the bench: the reference's own (torch-cpu, fp32) implementation of the prefill path = the oracle port
-(oracle/model.py — neither of the reference's two implementations imports in this image, SURVEY.md §8c), timed on the GPU
+(oracle/model.py — neither of the reference's two implementations imports in this image), timed on the GPU
 box's host cores on a BOUNDED SAMPLE of the benchmark workload.
 
 The sample is a proportional slice of the request at FULL DEPTH (27 ViT + 32 decoder layers, real widths): `n_crops` of the

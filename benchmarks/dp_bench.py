@@ -52,7 +52,7 @@ class DpHarness:
         return [float(x) for x in t.tolist()]
 
 
-# a mixed queue for the strong-scaling leg: 8 requests, 1 .. 28 crops (SURVEY.md §8d: "8/4/2/1 samples per GPU as a varlen batch")
+# a mixed queue for the strong-scaling leg: 8 requests, 1 .. 28 crops ("8/4/2/1 samples per GPU as a varlen batch")
 STRONG_QUEUE = [[(896, 1152)] * 4, [(1344, 1344)], [(896, 1152)] * 2, [(364, 364)], [(1344, 1344)] * 2, [(896, 1152)] * 4,
                 [(728, 1092)], [(1092, 1456)] * 3]
 

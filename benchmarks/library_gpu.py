@@ -1,4 +1,4 @@
-"""The "library GPU" competitor of BASELINE.md §3: the SAME prefill computed by stock libraries on the same B200 —
+"""The "library GPU" competitor: the SAME prefill computed by stock libraries on the same B200 —
 cuBLAS through `F.linear`, flash-attn 2 (`flash_attn_func`, what the reference's flash path calls:
 Pai-Megatron-Patch/megatron_patch/model/llava/transformer.py:476-515,869-877) or torch SDPA when the wheel does not
 load, and eager torch element-wise ops — in bf16, on the product's own weight tensors (kernel layout, no copy).

@@ -1,8 +1,8 @@
-"""bench.py --workload cfg4 | cfg5: the two BASELINE.json configurations that are not the headline metric.
+"""bench.py --workload cfg4 | cfg5: the two configurations that are not the headline metric.
 
 cfg4  Leopard-Idefics2, 8 images 980 x 980 -> 8 x 4900 patches -> perceiver -> 512 image rows + 64 text ids (S = 576):
       prefill tokens/s, one request per GPU per step (replicas: the path has no exchange step).
-cfg5  Leopard-LLaVA SFT step (SURVEY.md §8f-1): tokens [1, 4096] = 21 crops x 169 image slots + 547 text ids, loss on the
+cfg5  Leopard-LLaVA SFT step: tokens [1, 4096] = 21 crops x 169 image slots + 547 text ids, loss on the
       last 256 positions, bf16 compute / fp32 main params + Adam, full recompute (the reference's setting), vision tower
       trainable unless --sft-freeze-vit (the launch script passes no freeze flag).  N > 1 = data parallel over NCCL: one
       micro-batch per rank, bucketed gradient all-reduce overlapped with the backward pass

@@ -1,6 +1,5 @@
 """The reference's training loop body (Pai-Megatron-Patch/examples/llava/pretrain_megatron_llava.py + Megatron's `train`) with
 leopard_b200 under it — what a maintainer's script looks like after the switch described in INTEGRATION.md §2.
-NOT YET RUN ON A B200: the step's kernels are verified under CPU emulation only.
 
 Reference                                   here
   :37-50   model_provider                    leopard_b200.megatron.model_provider (+ configure_provider for args / weights)

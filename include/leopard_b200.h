@@ -1,6 +1,6 @@
 /* leopard_b200 — C ABI of the B200-native Leopard multi-image prefill path.
  *
- * This is the drop-in boundary under the reference's Python plugin surface (SURVEY.md §8b): the shims in
+ * This is the drop-in boundary under the reference's Python plugin surface: the shims in
  * leopard_b200/hf.py and leopard_b200/megatron.py keep the reference's class/function names and call ONLY the
  * functions below through ctypes.  The reference has no FFI of its own (it calls torch / transformers /
  * TransformerEngine / flash-attn); each entry point cites the reference call site whose arithmetic it replaces
@@ -53,7 +53,7 @@ int lp_gemm_bf16(const void* A, long long lda, const void* W, long long ldw, voi
                  int block_n, void* stream);
 
 /* Extended GEMM: the same kernel with three epilogue fusions that remove the standalone HBM-bound glue kernels of the layer loops
- * (SURVEY.md §2.3 K2/K5 "LN prologue + GEMM", K9 "RMSNorm fused into the next GEMM", K10/K11 "RoPE in the QKV epilogue";
+ * (LayerNorm and RMSNorm folded into the next GEMM, RoPE in the QKV epilogue;
  * reference: TELayerNormColumnParallelLinear MP/model/llava/clip_encoder.py:51-72, RMSNorm MLM/legacy/model/rms_norm.py:26-31,
  * RoPE MLM/core/models/common/embeddings/rotary_pos_embedding.py:197-239).
  *   norm_mode != NONE (consumer): C = act(norm(A) W^T + b).  The norm's gain is folded into W offline (W' = W diag(gamma), what
@@ -92,7 +92,7 @@ int lp_row_stats(const void* x, long long ldx, int rows, int width, float* stats
  * when the weight structs carry the folded matrices, 0 = standalone norm / RoPE kernels.  Returns the previous setting. */
 int lp_model_set_fused_norm(int enable);
 
-/* Tensor parallel + sequence parallel launches (SURVEY.md §8f-4; reference: ColumnParallelLinear / RowParallelLinear with
+/* Tensor parallel + sequence parallel launches (reference: ColumnParallelLinear / RowParallelLinear with
  * sequence_parallel, MLM/core/tensor_parallel/layers.py:387-454, mappings.py:119-199).  The M rows are tp_size segments of
  * seg_rows rows, segment r owned by rank r.  One kernel does the collective AND the GEMM over NVLink peer memory:
  *   LP_TP_ALLGATHER       C[M, N'] = act(A W^T): A is this rank's [M, lda] gather buffer of which only its own segment is valid
@@ -160,7 +160,7 @@ int lp_gemm_set_epilogue_sleep(int ns);
 /* Launch the hot prefill kernels (GEMM, attention v3, norms, RoPE) with programmatic dependent launch: the next kernel's
  * CTAs are scheduled as SMs free up and run their prologue (barrier init, TMEM allocation, descriptor prefetch) while the
  * previous kernel drains; each kernel executes griddepcontrol.wait before its first dependent global access.  Results
- * are unchanged.  Returns the previous setting (default set by the library, see DESIGN.md). */
+ * are unchanged.  Returns the previous setting (default set by the library). */
 int lp_set_prefill_pdl(int enable);
 
 /* O[b,t,h,:] = softmax(scale * Q K^T (+causal)) V          (tcgen05 flash attention, fp32 softmax, bf16 in/out)
@@ -242,7 +242,7 @@ int lp_rope_inplace(void* x, long long ld, int S, int col0, int n_heads, int hea
  *   Every id == image_id is an image slot that receives rows_per_slot consecutive rows of feats (slots consume feature
  *   rows in order); every other id receives table[clamp(id, 0, vocab-1)].
  *   rows_per_slot = 169, image_id = 128200: HF expand convention (_merge_input_ids_with_image_features as called at
- *     EV/llava_multiimg_siglip_anyres.py:285-287; SURVEY.md App. A.1, B = 1 / no padding) -> S = L + 168 * slots.
+ *     EV/llava_multiimg_siglip_anyres.py:285-287, B = 1 / no padding) -> S = L + 168 * slots.
  *   rows_per_slot = 1, image_id = -200: Megatron scatter convention (MP/model/llava/vlm_model.py:516-533).
  * plan: device int32 scratch [2*L + 2]; on completion plan[2*L] = number of slots, plan[2*L+1] = merged length S
  *   (the host shim reads them back to raise the reference's count-mismatch error). */
@@ -269,7 +269,7 @@ int lp_pixel_shuffle(const void* x, long long ldx, void* out, long long ldo, int
 
 /* ------------------------------------------------------------------------------------------------------------------
  * Model-level entry points (the layer loops).  Weight structs hold DEVICE pointers in the kernel-native layout that
- * leopard_b200/native_weights.py produces from an HF- or Megatron-layout state dict (SURVEY.md App. E):
+ * leopard_b200/native_weights.py produces from an HF- or Megatron-layout state dict:
  *   bf16 matrices in nn.Linear layout [out, in]; biases / norm gains as fp32 vectors (bf16-rounded values).
  * ------------------------------------------------------------------------------------------------------------------ */
 typedef struct lp_vit_dims {
@@ -307,7 +307,7 @@ typedef struct lp_proj_weights {
   const float* b1;
   const void* w2; /* [hidden_dec, hidden_dec] */
   const float* b2;
-  int act;        /* LP_ACT_GELU_ERF (HF eval) or LP_ACT_GELU_TANH (Megatron fused path, SURVEY D8) */
+  int act;        /* LP_ACT_GELU_ERF (HF eval) or LP_ACT_GELU_TANH (Megatron fused path) */
 } lp_proj_weights;
 
 typedef struct lp_dec_dims {
@@ -428,7 +428,7 @@ int lp_decode_set_mode(int mode);
 int lp_decode_set_prefetch(int o_proj_mb, int gateup_mb);
 
 /* ------------------------------------------------------------------------------------------------------------------
- * GPU image front-end (SURVEY.md §8 a3 + a5, "next" row f-3): one RGB uint8 image -> the ViT inputs it contributes.
+ * GPU image front-end: one RGB uint8 image -> the ViT inputs it contributes.
  *   rgb: DEVICE uint8 [H, W, 3] (what np.asarray(PIL.Image.convert('RGB')) holds), 16-byte aligned base.
  *   out_global: [3, 364, 364] — SiglipImageProcessor.preprocess(image) (EV/llava_multiimg_siglip_anyres.py:403-404):
  *     bicubic resize of the whole image to 364 x 364, x * rescale (float64, rounded to float32), (x - mean) / std.
@@ -460,7 +460,7 @@ int lp_image_resize(const void* rgb, int H, int W, int out_w, int out_h, int fil
                     void* workspace, size_t ws_bytes, void* stream);
 
 /* ------------------------------------------------------------------------------------------------------------------
- * SFT step (FIRST IMPLEMENTATION, specification = oracle/train.py): the HBM-bound half of the backward
+ * SFT step (specification: oracle/train.py): the HBM-bound half of the backward
  * pass, the masked LM loss and the optimizer.  In the reference all of this is torch autograd + apex inside Megatron's
  * train_step (Pai-Megatron-Patch/examples/llava/pretrain_megatron_llava.py:101-160,
  * Megatron-LM-240424/megatron/core/optimizer/optimizer.py:300-370, clip_grads.py:103-141).  The dgrad / wgrad
@@ -554,7 +554,7 @@ int lp_profile_enable(int capacity);
 int lp_profile_read(lp_profile_record* out, int capacity);
 
 /* ------------------------------------------------------------------------------------------------------------------
- * PARITY MODE (leopard_b200/parity.py): the fp32-equivalent forward that answers BASELINE.json's "logits within 1e-3 max-abs of
+ * PARITY MODE (leopard_b200/parity.py): the fp32-equivalent forward that gives "logits within 1e-3 max-abs of
  * the reference forward" — the reference's HF evaluation is fp32 end to end (EV/llava_multiimg_siglip_anyres.py:373).  Activations
  * stay fp32; every contraction runs on lp_gemm_bf16 with the fp32 operand split into three bf16 terms laid out along K
  * (lp_parity_split), fp32 accumulation in TMEM, fp32 output; the glue between the GEMMs are these fp32 kernels.

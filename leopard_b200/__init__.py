@@ -2,6 +2,6 @@
 
 Host code is Python/PyTorch (device memory, streams, torch.distributed); all arithmetic on the path runs in the
 hand-written CUDA library `lib/libleopard_b200.so` behind the C ABI in `include/leopard_b200.h`.
-See DESIGN.md for the scope and INTEGRATION.md for how the reference scripts bind to it.
+The reference's scripts bind to it through hf.py, megatron.py and idefics2.py.
 """
 __version__ = "0.1.0"

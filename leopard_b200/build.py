@@ -1,8 +1,7 @@
 """In-tree build of the native library (nvcc, sm_100a only).
 
 `build_native()` compiles every `csrc/*.cu` into `leopard_b200/lib/libleopard_b200.so`.  nvcc cross-compiles
-without a GPU, so this runs in the authoring container; the built `.so` travels to the GPU box with the repo
-snapshot (it is git-ignored, not gpurun-ignored).
+without a GPU; the built `.so` stays in the tree and is git-ignored.
 """
 from __future__ import annotations
 

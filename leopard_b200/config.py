@@ -1,4 +1,4 @@
-"""Model hyper-parameters of the two Leopard variants on the prefill path (SURVEY.md §8 header line).
+"""Model hyper-parameters of the two Leopard variants on the prefill path.
 
 Leopard-LLaVA  = SigLIP-SO400M/14-364 + pixel-shuffle/2-layer MLP projector + Llama-3.1-8B
                  (Pai-Megatron-Patch/examples/llava/train_multiimg_llava_siglip.sh:56,73-93,179-180,220-228;
@@ -70,7 +70,7 @@ class LeopardConfig:
     dec: DecoderConfig = field(default_factory=DecoderConfig)
     image_token_index: int = 128200        # <|reserved_special_token_195|>, EV/llava_multiimg_siglip_anyres.py:426-435
     megatron_image_index: int = -200       # IMAGE_TOKEN_INDEX, MP/model/llava/vlm_model.py:526
-    projector_act: str = "gelu"            # HF: exact erf GELU; Megatron fused path: "gelu_pytorch_tanh" 
+    projector_act: str = "gelu"            # HF: exact erf GELU; Megatron fused path: "gelu_pytorch_tanh"
     shuffle: int = 2                       # pixel_shuffle scale factor
 
     @property
@@ -123,7 +123,7 @@ def leopard_llava() -> LeopardConfig:
 
 
 def leopard_idefics2_decoder() -> DecoderConfig:
-    """Mistral-7B parameterisation of the same decoder kernels (SURVEY D1)."""
+    """Mistral-7B parameterisation of the same decoder kernels."""
     return DecoderConfig(vocab=32003, rope_theta=10000.0, rope_scaling=None)
 
 

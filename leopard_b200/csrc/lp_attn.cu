@@ -2,7 +2,7 @@
 //
 //   O[b, t, h, :] = softmax( scale · Q[b,t,h,:] · K[b,:,h/g,:]^T  (+ causal mask) ) · V[b,:,h/g,:]
 //
-// Replaces, on Leopard's prefill path (SURVEY.md §2.3):
+// Replaces, on Leopard's prefill path:
 //   K3  SigLIP non-causal MHA, 16 heads x 72 (HF SiglipAttention; Megatron TEDotProductAttention,
 //       Pai-Megatron-Patch/megatron_patch/model/llava/clip_encoder.py:58-63)            -> DH = 80 (72 zero-padded)
 //   K12 decoder causal GQA attention, 32 q / 8 kv heads x 128 (flash_attn_varlen_func call at

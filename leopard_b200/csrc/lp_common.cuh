@@ -2,8 +2,8 @@
 //
 // Thin inline-PTX wrappers (mbarrier, TMA, tcgen05/TMEM, UMMA descriptors) used by
 // lp_gemm.cu and lp_attn.cu.  Nothing here comes from the reference: Leopard ships no
-// native code of its own (SURVEY.md §2.2); these replace the cuBLAS / flash-attn /
-// TransformerEngine library calls its hot path makes (SURVEY.md §2.3 K1-K16).
+// native code of its own; these replace the cuBLAS / flash-attn /
+// TransformerEngine library calls its hot path makes.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>

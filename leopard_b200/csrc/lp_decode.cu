@@ -3,7 +3,7 @@
 // The cached-decode branch of myLlavaForConditionalGeneration.forward
 // (evaluations/models/llava_multiimg_siglip_anyres.py:291-320, driven by `generate(..., max_new_tokens=128,
 // use_cache=True)` at :448-452): with B = 1 and no padding the rebuilt mask is all ones and the position is the
-// number of cached rows (SURVEY.md App. A.2).
+// number of cached rows.
 //
 // The step is HBM-bound: every decoder weight (15.0 GB for Llama-3.1-8B incl. lm_head) is read exactly once per token,
 // so the floor is weights / HBM bandwidth (~2.4 ms on a B200) and the design is about keeping the memory system

@@ -7,7 +7,7 @@
 //   lp_rope_table / lp_rope_inplace   rotate-half RoPE on the q/k column slices of the fused QKV buffer
 //                    (megatron/core/models/common/embeddings/rotary_pos_embedding.py:197-239)
 //   lp_embed_merge   token embedding + image-feature merge, HF-expand and Megatron-scatter conventions
-//                    (HF _merge_input_ids_with_image_features, SURVEY.md App. A.1; vlm_model.py:516-533)
+//                    (HF _merge_input_ids_with_image_features; vlm_model.py:516-533)
 //   lp_im2col_patch14  14x14/stride-14 patch extraction feeding the patch-embed GEMM
 //                    (megatron_patch/model/idefics2/idefics_vision_tower.py:57-64,118-122)
 #include "lp_common.cuh"

@@ -3,7 +3,7 @@
 //   C[M,N] = epilogue( A[M,K] · W[N,K]^T )          A, W bf16 row-major (K contiguous), fp32 accumulate in TMEM
 //
 // Replaces every dense contraction on Leopard's prefill path, which the reference delegates to cuBLAS /
-// TransformerEngine through torch (SURVEY.md §2.3):
+// TransformerEngine through torch:
 //   K1  patch-embed GEMM + bias + position embedding   (HF SiglipVisionEmbeddings; Megatron
 //       Pai-Megatron-Patch/megatron_patch/model/idefics2/idefics_vision_tower.py:118-150)
 //   K2/K4/K5 ViT qkv / out-proj / fc1(GELU-tanh) / fc2  (megatron_patch/model/llava/clip_encoder.py:51-72)
@@ -903,7 +903,7 @@ extern "C" int lp_gemm_bf16(const void* A, long long lda, const void* W, long lo
   return lp_gemm_bf16_ex(&d, stream_);
 }
 
-// ---- tensor-parallel launches (SURVEY.md §8f-4): all-gather -> GEMM and GEMM -> reduce-scatter in ONE kernel over NVLink peer memory
+// ---- tensor-parallel launches: all-gather -> GEMM and GEMM -> reduce-scatter in ONE kernel over NVLink peer memory
 extern "C" int lp_gemm_bf16_tp(const lp_gemm_desc* d, const lp_tp_desc* t, void* stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LP_REQUIRE(d && t, "lp_gemm_bf16_tp: null descriptor");

@@ -27,7 +27,7 @@ struct GemmArgs {
   int group_m;
   int prefetch_a;
   unsigned epi_sleep_ns;         // epilogue warps sleep this long between probes of the accumulator-full barrier (0 = spin)
-  // ---- fused row normalisation of the A operand (consumer side; SURVEY.md K2/K5/K9: LayerNorm / RMSNorm folded into the GEMM).
+  // ---- fused row normalisation of the A operand (consumer side: LayerNorm / RMSNorm folded into the GEMM).
   // The gain is folded into W offline (W' = W diag(gamma)), so norm(x) W^T = rs[row] * (x W'^T - mu[row] * colsum[col]) (+ beta W^T
   // + b, passed as `bias`).  mu / rs come from per-row partial (sum, sum of squares) pairs the PRODUCING GEMM's epilogue wrote.
   int norm_mode;                 // LP_NORM_NONE / LP_NORM_RMS / LP_NORM_LAYER
@@ -42,7 +42,7 @@ struct GemmArgs {
   const float* rope_cos;
   const float* rope_sin;
   int rope_heads;
-  // ---- tensor-parallel fusions (lp_gemm_bf16_tp, SURVEY.md §8f-4).  tp_size > 0: the M rows are tp_size segments of seg_rows rows,
+  // ---- tensor-parallel fusions (lp_gemm_bf16_tp).  tp_size > 0: the M rows are tp_size segments of seg_rows rows,
   // segment r owned by rank r (Megatron sequence parallelism); tiles never straddle a segment (seg_m_blk row blocks per segment)
   // and the rank's own segment is scheduled first.
   int tp_size, tp_rank, seg_rows, seg_m_blk;

@@ -128,7 +128,7 @@ static int vit_layers_impl(const lp_vit_dims* d, const lp_vit_weights* w, void* 
   const int qkv_w = 3 * d->heads * d->head_stride;
   int rc;
   if (vit_can_fuse(d, w) && stA.buf && stB.buf) {
-    // LayerNorm folded into the consuming GEMM (SURVEY.md K2 / K5): 4 GEMMs + attention per layer, no norm launches
+    // LayerNorm folded into the consuming GEMM: 4 GEMMs + attention per layer, no norm launches
     if (stA.parts == 0) {
       LP_TRY(lp_row_stats(x, d->hidden, rows, d->hidden, stA.buf, stream));
       stA.parts = 1;
@@ -323,7 +323,7 @@ extern "C" int lp_decoder_prefill(const lp_dec_dims* d, const lp_dec_weights* w,
     __nv_bfloat16* kc = kv_cache ? (__nv_bfloat16*)kv_cache + (size_t)l * 2 * kv_capacity * kv_w : nullptr;
     if (fused) {
       // RMSNorm folded into the QKV GEMM (gain in the weights, rstd in the epilogue) together with rotate-half RoPE on the
-      // q and k heads (SURVEY.md K9-K11)
+      // q and k heads
       lp_gemm_desc g = gemm_desc(x, H, L->qkv_wf, H, qkv, qkv_w, R, qkv_w, H, nullptr, nullptr, 0, 0, LP_ACT_NONE);
       consume_stats(g, LP_NORM_RMS, stA, nullptr, d->eps);
       g.rope_cos = cs; g.rope_sin = sn; g.rope_heads = d->heads + d->kv_heads;

@@ -1,7 +1,7 @@
 // leopard_b200 — PARITY MODE glue: fp32 element-wise kernels for the fp32-equivalent forward (leopard_b200/parity.py).
 //
-// The reference's HF evaluation runs the whole model in fp32 (evaluations/models/llava_multiimg_siglip_anyres.py:373)
-// asks for logits within 1e-3 max-abs of it — below bf16 resolution through 59 layers.  Parity mode keeps every
+// The reference's HF evaluation runs the whole model in fp32 (evaluations/models/llava_multiimg_siglip_anyres.py:373); this
+// mode answers it with logits within 1e-3 max-abs of it — below bf16 resolution through 59 layers.  Parity mode keeps every
 // activation in fp32 and runs every contraction on the SAME tcgen05 GEMM kernel with the fp32 operand split into three bf16
 // terms (x = hi + mid + lo, 8 + 8 + 8 mantissa bits): products of bf16 terms are exact in the fp32 TMEM accumulator, so
 // A W^T = (hi + mid + lo) W^T is computed to fp32 accuracy as ONE bf16 GEMM over a 3x longer contraction (weights are

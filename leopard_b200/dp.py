@@ -1,4 +1,4 @@
-"""Data-parallel sharding of independent prefill requests over the GPUs of one node (SURVEY.md §8e).
+"""Data-parallel sharding of independent prefill requests over the GPUs of one node.
 
 The path has no exchange step: each request (its crops, projector rows and decoder sequence) depends on nothing else,
 and the reference itself runs one process per GPU on contiguous index shards and merges result files
@@ -17,7 +17,7 @@ import torch.distributed as dist
 
 
 def request_cost(n_crops: int, seq_len: int) -> float:
-    """GFLOP model of one request (SURVEY.md §8d/§8e): 625.6 per crop + 13.96 per token + 2.62e-4 * S^2."""
+    """GFLOP model of one request: 625.6 per crop + 13.96 per token + 2.62e-4 * S^2."""
     return 625.6 * n_crops + 13.96 * seq_len + 2.62144e-4 * seq_len * seq_len
 
 

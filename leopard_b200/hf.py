@@ -1,4 +1,4 @@
-"""Drop-in for the HF-eval plugin surface of the reference (first row).
+"""Drop-in for the HF-eval plugin surface of the reference.
 
 Same names and call conventions as evaluations/models/llava_multiimg_siglip_anyres.py:
     pixel_shuffle(x, scale_factor=2)                                   (:165-176)
@@ -168,7 +168,7 @@ class _LanguageModel:
             raise NotImplementedError("cached decode goes through myLlavaForConditionalGeneration.generate")
         eng = self._o.engine
         if inputs_embeds.shape[0] != 1:
-            raise NotImplementedError("the reference path is B = 1 (SURVEY.md App. A.1)")
+            raise NotImplementedError("the reference path is B = 1")
         x = inputs_embeds[0].to(eng.device, torch.bfloat16).contiguous().clone()
         S = x.shape[0]
         pos = torch.arange(S, device=eng.device) if position_ids is None else position_ids.reshape(-1)
@@ -194,8 +194,8 @@ class _NativeParameters(nn.Module):
 
 
 def plan_padded_batch(input_ids: torch.Tensor, attention_mask: Optional[torch.Tensor], image_id: int, rows_per_image: int):
-    """Host plan of HF's `_merge_input_ids_with_image_features` for a padded batch (transformers 4.38-4.4x algorithm, SURVEY.md
-    App. A.1 steps 1-3; the reference's forward calls it at …anyres.py:285-287).  Padding is removed instead of masked: the rows the
+    """Host plan of HF's `_merge_input_ids_with_image_features` for a padded batch (transformers 4.38-4.4x algorithm;
+    the reference's forward calls it at …anyres.py:285-287).  Padding is removed instead of masked: the rows the
     attention mask keeps of batch row b form one packed sequence of S_b = kept ids + (rows_per_image - 1) per image placeholder,
     with positions 0 .. S_b - 1 (= cumsum(mask) - 1 of step 4), and land in the merged [B, max_len] layout at offset off_b:
     left padding -> right-aligned (new_pos += nb_image_pad), right padding -> left-aligned.
@@ -401,7 +401,7 @@ class myLlavaForConditionalGeneration(nn.Module):
 
     def _cached_step(self, input_ids, past):
         """The cached branch of the reference forward (…anyres.py:291-320) for B = 1 without padding: the new token's
-        position is the number of cached rows (SURVEY.md App. A.2); one native decode step over the cache."""
+        position is the number of cached rows; one native decode step over the cache."""
         import ctypes as C
         eng = self.engine
         L = _lib.lib()

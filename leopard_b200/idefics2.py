@@ -1,4 +1,4 @@
-"""Leopard-Idefics2 prefill on the native path (SURVEY.md §8a rows a14, a15) and its plugin surface.
+"""Leopard-Idefics2 prefill on the native path and its plugin surface.
 
 Reference surface (evaluations/models/idefics2_multiimg.py:22-30,88-97): `processor, model = load_model(args)`;
 `model.generate(**{input_ids, attention_mask, pixel_values[B,n,3,H,W], pixel_attention_mask[B,n,H,W]},

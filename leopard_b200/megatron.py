@@ -1,4 +1,4 @@
-"""Drop-in for the Megatron plugin surface of the reference (second row): forward / prefill, and the training
+"""Drop-in for the Megatron plugin surface of the reference: forward / prefill, and the training
 iteration's entry points (mm_collate_fn, loss_func, train_step over leopard_b200.train.SFTTrainer).
 
     model_provider(pre_process=True, post_process=True) -> model         (Pai-Megatron-Patch/examples/llava/
@@ -11,7 +11,7 @@ tiles + [global]; ids -100 (padding) read embedding row 0 (vlm_model.py:226); `i
 "no image" dummy (vlm_model.py:518; dummy = zeros(1, 10), pretrain_megatron_llava.py:188); a feature/slot count
 mismatch raises AssertionError with the reference's message (vlm_model.py:528-529).  The attention mask is ignored
 exactly like the flash-attention path of the reference (causal only).  forward(labels=...) returns the per-token loss
-[b, s] (lp_cross_entropy).  There is no autograd graph: the training iteration (§8f-1, first implementation — DESIGN.md §6b)
+[b, s] (lp_cross_entropy).  There is no autograd graph: the training iteration
 is `train_step`, which hands the batch to SFTTrainer.step (forward, loss_func, backward, reduce, clip, AdamW on native
 kernels).  Checkpoint surface: state_dict_for_save_checkpoint() / load_state_dict() speak the reference's nested Megatron
 layout and export the live (trained) tensors.

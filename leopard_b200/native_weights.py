@@ -1,6 +1,6 @@
 """Checkpoint -> kernel-native device layout (what the lp_*_weights structs of include/leopard_b200.h point at).
 
-Accepts the two layouts the reference produces (SURVEY.md App. E):
+Accepts the two layouts the reference produces:
   * HF (transformers <= 4.4x LLaVA keys, separate q/k/v and gate/up)  — `load_hf`
   * Megatron (`language_model/{embedding,vision_tower,mm_projector,encoder,output_layer}`, fused + interleaved)
     — `megatron_to_hf` first restores HF tensors exactly as the reference converter does
@@ -301,7 +301,7 @@ def random_native(cfg: LeopardConfig, device="cuda", seed: int = 1234) -> Native
 
 
 # ----------------------------------------------------------------------------------------------------------------
-# Megatron checkpoint layout -> HF layout (SURVEY.md App. E)
+# Megatron checkpoint layout -> HF layout
 # ----------------------------------------------------------------------------------------------------------------
 def megatron_to_hf(cfg: LeopardConfig, lm: Dict[str, torch.Tensor]) -> Dict[str, torch.Tensor]:
     """`lm` = flattened `state['model']['language_model']` of a TP=1 Megatron checkpoint with keys such as

@@ -1,7 +1,7 @@
 """Parity mode: the fp32-EQUIVALENT forward of Leopard-LLaVA's prefill on the native kernels.
 
 Why: the reference's HF evaluation runs in fp32 (`torch_dtype=torch.float32`, evaluations/models/
-llava_multiimg_siglip_anyres.py:373) and BASELINE.json states the tolerance as "logits within 1e-3 max-abs of the reference
+llava_multiimg_siglip_anyres.py:373) and the tolerance asked for is "logits within 1e-3 max-abs of the reference
 forward".  The fast path keeps activations in bf16 (what the reference's Megatron training does) and lands at ~6e-2 max-abs after
 59 layers; that is bf16 resolution, not a bug, but it cannot demonstrate the stated tolerance.  This module can.
 
@@ -16,7 +16,7 @@ of csrc/lp_parity.cu.  torch is used for allocation and pure data movement (view
 Cost: 3-6x the tensor work plus per-head attention launches — a verification path (seconds per request), selected explicitly:
     logits = ParityForward(engine).prefill_logits(input_ids, pixel_values)          # fp32 [S, vocab]
     model.set_precision("fp32")   # myLlavaForConditionalGeneration: forward() then answers with these logits
-Measured against the CPU oracle (tests/test_gpu_parity_mode.py): see DESIGN.md §4.
+Measured against the CPU oracle (tests/test_gpu_parity_mode.py).
 """
 from __future__ import annotations
 

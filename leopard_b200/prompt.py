@@ -1,4 +1,4 @@
-"""Host-side prompt construction of the reference's evaluation loop (SURVEY.md §8 a4) — pure string logic.
+"""Host-side prompt construction of the reference's evaluation loop — pure string logic.
 
 `build_eval_prompt` restates evaluations/models/llava_multiimg_siglip_anyres.py:412-442: the Llama-3 chat frame
 (`head` / `tail`, :22-23), the `<image>` bookkeeping and the per-image placeholder text

@@ -1,4 +1,4 @@
-"""Tensor parallel + Megatron sequence parallel decoder (SURVEY.md §8f-4): the reference's real training / inference sharding.
+"""Tensor parallel + Megatron sequence parallel decoder: the reference's real training / inference sharding.
 
 Reference: `--tensor-model-parallel-size 8 --sequence-parallel` (Pai-Megatron-Patch/examples/llava/train_multiimg_llava_siglip.sh:
 57-71,151-153); ColumnParallelLinear / RowParallelLinear with sequence parallelism
@@ -21,7 +21,7 @@ What is here
     `comm="fused"`: the all-gather is done INSIDE the consuming GEMM kernel over NVLink peer memory (lp_gemm_allgather: the
     epilogue warps pull the peers' rows while the first tiles — the rank's own rows — are being multiplied) and the
     reduce-scatter leaves the GEMM's epilogue as TMA stores of partial tiles into the owner rank's memory, tile by tile
-    (lp_gemm_reduce_scatter), followed by a fixed-order reduction on the owner.  See csrc/lp_tp.cu and DESIGN.md §9.
+    (lp_gemm_reduce_scatter), followed by a fixed-order reduction on the owner.  See csrc/lp_tp.cu.
 Every column-parallel output is bit-identical to the same columns of the TP = 1 GEMM (same kernel, same K order); row-parallel
 sums differ from TP = 1 only by the bf16 rounding of the partial sums (as in the reference, whose reduce-scatter sums bf16).
 """

@@ -1,4 +1,4 @@
-"""SFT step on the native kernels — FIRST IMPLEMENTATION, not yet measured on a B200.
+"""SFT step on the native kernels.
 
 What Megatron's `train_step` does for Pai-Megatron-Patch/examples/llava/pretrain_megatron_llava.py, sequenced on the host
 over C-ABI calls (allocation, shapes and ordering only; every contraction, reduction and update is a native kernel):

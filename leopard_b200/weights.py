@@ -1,12 +1,12 @@
 """Synthetic checkpoints in the reference's HF (transformers <= 4.4x LLaVA) key layout, and the key inventory.
 
-No Leopard checkpoint exists offline (SURVEY.md App. D), so parity and performance work uses seeded synthetic
-weights (SURVEY.md §8d): every tensor is drawn from its own generator seeded by (base seed, tensor name), in fp32 on
+No Leopard checkpoint exists offline, so parity and performance work uses seeded synthetic
+weights: every tensor is drawn from its own generator seeded by (base seed, tensor name), in fp32 on
 the CPU, and rounded once to bf16 — the SAME bf16 values feed the CPU oracle and the CUDA path.  Because each tensor is
 independent of every other, the oracle and the loaders can stream layer by layer.
 
 Key layout = target of the reference converter
-(Pai-Megatron-Patch/toolkits/model_checkpoints_convertor/llava/hf2megatron_llava.py:1100-1460; SURVEY.md App. E).
+(Pai-Megatron-Patch/toolkits/model_checkpoints_convertor/llava/hf2megatron_llava.py:1100-1460).
 """
 from __future__ import annotations
 
@@ -177,7 +177,7 @@ class SyntheticCheckpoint:
 
 
 def synth_inputs(cfg: LeopardConfig, n_crops: int, n_text: int, seed: int = 1, placeholder_per_crop: bool = True):
-    """Seeded synthetic inputs in the HF-eval convention (SURVEY.md §8d): pixels U(-1,1) fp32 [N,3,364,364] and a
+    """Seeded synthetic inputs in the HF-eval convention: pixels U(-1,1) fp32 [N,3,364,364] and a
     prompt with ONE placeholder id per crop (EV/llava_multiimg_siglip_anyres.py:426-435) surrounded by text ids."""
     g = torch.Generator(device="cpu").manual_seed(seed)
     pix = torch.rand((n_crops, 3, cfg.vit.image_size, cfg.vit.image_size), generator=g) * 2.0 - 1.0

@@ -1,4 +1,4 @@
-"""CPU ORACLE, Idefics2 rows of the scope table — test infrastructure only.
+"""CPU ORACLE, Idefics2 rows — test infrastructure only.
 
 Plain torch-CPU fp32 restatement of Leopard-Idefics2's prefill: NaViT-style SigLIP tower over variable-resolution
 images (bucketised position ids, padded patches masked), gated-MLP modality projection, perceiver resampler

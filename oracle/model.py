@@ -3,7 +3,7 @@
 Plain torch-CPU fp32 restatement of Leopard-LLaVA's multi-image prefill arithmetic, used ONLY as the checker by
 tests/, __graft_entry__.smoke() and bench.py's cpu_baseline / --impl reference leg.
 
-PARITY PINNING: the reference has no tests or golden vectors for this path (SURVEY.md §4, §8c) and neither of its two
+PARITY PINNING: the reference has no tests or golden vectors for this path and neither of its two
 implementations runs in this image (HF eval needs transformers <= 4.4x APIs; Megatron needs TransformerEngine).  The
 blocks below are therefore pinned against what CAN run here:
   * pixel_shuffle / projector / crop planner: executed from the reference source itself
@@ -11,7 +11,7 @@ blocks below are therefore pinned against what CAN run here:
   * SigLIP tower, Llama decoder layer, RMSNorm, llama3.1 RoPE: the installed transformers-5.5.0 modules the reference
     calls as third-party code, with shared seeded weights (tests/golden/gen_hf_goldens.py -> tests/golden/hf_*.npz);
   * HF `_merge_input_ids_with_image_features` (transformers 4.38-4.4x, absent here): restated from the published
-    algorithm (SURVEY.md App. A.1) — "parity unpinned" for that one function beyond the B=1 reduction the reference uses.
+    algorithm — "parity unpinned" for that one function beyond the B=1 reduction the reference uses.
 
 Every function cites the reference lines it follows (paths relative to the reference checkout).
 Weights come from any object with `f32(name) -> fp32 tensor` using the HF key layout (leopard_b200.weights).
@@ -100,9 +100,9 @@ def projector(ck, cfg, vit_out: torch.Tensor) -> torch.Tensor:
 # ----------------------------------------------------------------------------------------------------------------
 def merge_hf_expand(ck, cfg, input_ids: torch.Tensor, image_features: torch.Tensor):
     """HF `_merge_input_ids_with_image_features` for the only case the reference uses: B = 1, no padding, mask all
-    ones (EV/...anyres.py:285-287,443-446; SURVEY.md App. A.1).  Each placeholder id expands to its crop's 169 rows in
+    ones (EV/...anyres.py:285-287,443-446).  Each placeholder id expands to its crop's 169 rows in
     crop order.  Returns (embeds [1,S,D], position_ids [1,S])."""
-    assert input_ids.shape[0] == 1, "the reference only ever merges B=1 (see SURVEY.md App. A.1)"
+    assert input_ids.shape[0] == 1, "the reference only ever merges B=1"
     ids = input_ids[0]
     table = ck.f32(LM + "embed_tokens.weight")
     n, p, d = image_features.shape
@@ -127,7 +127,7 @@ def merge_hf_expand(ck, cfg, input_ids: torch.Tensor, image_features: torch.Tens
 
 def merge_hf_batched(ck, cfg, input_ids: torch.Tensor, attention_mask: torch.Tensor, image_features: torch.Tensor,
                      pad_token_id: int):
-    """HF `_merge_input_ids_with_image_features` for a padded batch, restated step by step from SURVEY.md App. A.1 (the
+    """HF `_merge_input_ids_with_image_features` for a padded batch, restated step by step (the
     transformers 4.38-4.4x algorithm the reference's forward calls at EV/...anyres.py:285-287; "parity unpinned": the source
     is in neither tree).  input_ids / attention_mask [B, L], image_features [N, P, D].  Returns (final_embedding [B, max_len, D],
     final_attention_mask [B, max_len], position_ids [B, max_len])."""

@@ -13,7 +13,7 @@ Stored per config (fp32 unless noted; the full [S, V] logits would be 1.5-2.5 GB
   row_argmax [R] (int64), row_top5_idx/val [R, 5], row_absmax [R]
   feat_sub [N, 13, 64]            image_features[:, ::13, ::64] (tower + shuffle + projector)
   hidden_sub [R, 64]              final-norm hidden state at rows, every 64th channel
-tests/test_gpu_fullsize.py compares the CUDA path with these on the GPU box (where /root/reference and the minutes of
+tests/test_gpu_fullsize.py compares the CUDA path with these on a GPU machine (where /root/reference and the minutes of
 CPU time are not available)."""
 import sys
 import time

@@ -1,4 +1,4 @@
-"""Pin the oracle's restatement of the THIRD-PARTY blocks the reference calls (SURVEY.md §8c): run the installed
+"""Pin the oracle's restatement of the THIRD-PARTY blocks the reference calls: run the installed
 transformers SiglipVisionModel / LlamaForCausalLM (the modules `self.vision_tower(...)` and `self.language_model(...)`
 resolve to, evaluations/models/llava_multiimg_siglip_anyres.py:268,322-331) on the seeded synthetic checkpoint of
 leopard_b200.weights at FULL width and reduced depth, and store sub-sampled outputs in hf_goldens.npz.

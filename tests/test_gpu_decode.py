@@ -1,4 +1,4 @@
-"""-m gpu: the greedy decode step (SURVEY.md §8f-2; cached branch of myLlavaForConditionalGeneration.forward,
+"""-m gpu: the greedy decode step (cached branch of myLlavaForConditionalGeneration.forward,
 evaluations/models/llava_multiimg_siglip_anyres.py:291-320) against the oracle and against itself.
 
 The GEMV decode kernels must agree with (a) the oracle's full recomputation of the extended sequence, (b) the first

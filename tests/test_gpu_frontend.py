@@ -1,5 +1,5 @@
 """-m gpu: the CUDA image front-end (lp_image_frontend through the C ABI) against the CPU oracle — bit-exact: the
-path is integer / byte arithmetic plus a table lookup (SURVEY.md §8 a3, a5, f-3)."""
+path is integer / byte arithmetic plus a table lookup."""
 import json
 import sys
 from pathlib import Path

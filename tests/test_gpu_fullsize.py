@@ -1,5 +1,5 @@
-"""-m gpu: BASELINE.json's FULL sizes (27 + 32 layers, real widths, cfg2 / cfg3 shapes, 16k-token prompts) checked
-through size-independent properties — the CPU oracle needs ~7-13 minutes per such pass (BASELINE.md §4), so parity at
+"""-m gpu: the benchmark's FULL sizes (27 + 32 layers, real widths, cfg2 / cfg3 shapes, 16k-token prompts) checked
+through size-independent properties — the CPU oracle needs ~7-13 minutes per such pass, so parity at
 these sizes is established two ways: (1) size-independent properties on the benchmark's device-side random weights —
 bit-determinism, causality, crop-permutation equivariance, request-packing invariance (all bitwise, because every output
 element's accumulation order is independent of tiling), finiteness/scale; (2) the committed full-depth oracle fixtures
@@ -103,7 +103,7 @@ def _load_golden(name):
 def test_full_depth_logits_match_the_committed_oracle_fixture(seeded_full_engine, name, n_crops, S):
     """BASELINE configs 2 and 3 (the bench workload) at 27 + 32 layers against the fp32 CPU oracle: image features,
     the final hidden state's logits on every 64th row x every 97th vocabulary column, the whole last row, and the
-    greedy token of every sampled row.  Tolerances are the bf16-path bounds of DESIGN.md §4 (relative to max|oracle|)."""
+    greedy token of every sampled row.  Tolerances are the bf16-path bounds of the stage tests (relative to max|oracle|)."""
     import sys
     from pathlib import Path
     sys.path.insert(0, str(Path(__file__).parent / "golden"))

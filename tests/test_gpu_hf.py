@@ -188,7 +188,7 @@ def test_megatron_provider_matches_oracle(small):
 
 
 def test_padded_batch_forward_and_generate_follow_the_hf_merge(small):
-    """B = 3 left-padded batch with 1 / 2 / 0 images (HF's batched-generation layout, SURVEY.md App. A.1): logits of the merged
+    """B = 3 left-padded batch with 1 / 2 / 0 images (HF's batched-generation layout): logits of the merged
     [B, max_len, V] layout against the oracle's restatement of the HF merge + decoder; every kept row of a batch row equals the
     same prompt run alone (packing / padding invariance, bit for bit); batched generate == per-row generate, padded with
     pad_token_id."""

@@ -84,7 +84,7 @@ def test_prefill_matches_oracle_with_padding_and_dropped_image(small):
 
 
 def test_full_resolution_image_tile_counts(small):
-    """cfg4 geometry: a 980 x 980 image is 70 x 70 = 4900 patches -> 64 rows (SURVEY.md §8d cfg4), 1 image here."""
+    """cfg4 geometry: a 980 x 980 image is 70 x 70 = 4900 patches -> 64 rows, 1 image here."""
     cfg, ck, model = small
     g = torch.Generator().manual_seed(2)
     pv = (torch.rand(1, 1, 3, 980, 980, generator=g) * 2 - 1).to(torch.bfloat16)

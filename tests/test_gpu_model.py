@@ -1,9 +1,9 @@
 """-m gpu: model-level parity of the CUDA path (through the C ABI) against the CPU oracle on identical seeded
 weights and inputs.
 
-Tolerance ladder (SURVEY.md §7 "hard parts", D5): the CUDA path keeps bf16 activations with fp32 accumulation /
+Tolerance ladder: the CUDA path keeps bf16 activations with fp32 accumulation /
 statistics, the oracle is fp32 math on the same bf16-rounded weights.  We bound  max|cuda - oracle| / max|oracle|
-per stage; the measured values are printed (run with -s) and recorded in DESIGN.md.  BASELINE.json's 1e-3 logit
+per stage; the measured values are printed (run with -s).  A 1e-3 logit
 max-abs figure is below bf16 resolution for 32 layers and is NOT claimed.
 """
 import pytest

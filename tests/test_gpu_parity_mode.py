@@ -1,5 +1,5 @@
 """-m gpu: PARITY MODE (leopard_b200/parity.py, csrc/lp_parity.cu) — the fp32-equivalent forward on the tcgen05 GEMM with
-three-term bf16 operand splitting — against the fp32 CPU oracle.  This is the test that carries BASELINE.json's stated tolerance:
+three-term bf16 operand splitting — against the fp32 CPU oracle.  This is the test that carries the stated tolerance:
 "logits within 1e-3 max-abs of the reference forward" (the reference's HF evaluation is fp32,
 evaluations/models/llava_multiimg_siglip_anyres.py:373).  Tolerance asserted here: 1e-3 max-abs on logits of magnitude <= ~5,
 at reduced depth (2 + 2 layers), at full depth for BASELINE config 1 (27 + 32 layers, S = 201), and at full depth on the bench

@@ -140,7 +140,7 @@ def test_bench_workload_bookkeeping():
     assert per_image == [7, 7, 7, 7] and n_crops == 28 and S == 4796 and ids.shape == (1, 92)
     assert pix.shape == (28, 3, 364, 364) and float(pix.min()) >= -1 and float(pix.max()) <= 1
     fm = bench.flops_model(n_crops, S, cfg)
-    assert abs(fm["total"] / 1e12 - 90.5) < 0.3  # SURVEY.md §8d: 90.5 TFLOP per cfg3 request
+    assert abs(fm["total"] / 1e12 - 90.5) < 0.3  # 90.5 TFLOP per cfg3 request
 
 
 def test_from_pretrained_reads_hf_checkpoint_dir(tmp_path):
@@ -228,7 +228,7 @@ def test_megatron_checkpoint_nesting_round_trip():
 
 def test_eval_prompt_builder_matches_reference_executed_goldens():
     """leopard_b200.prompt.build_eval_prompt == the reference's own lines 412-442 (executed by
-    tests/golden/gen_prompt_goldens.py), quirks and failure modes included (SURVEY.md §8 a4)."""
+    tests/golden/gen_prompt_goldens.py), quirks and failure modes included."""
     import json
     from pathlib import Path
     from leopard_b200.prompt import build_eval_prompt, get_instruction, image_placeholder
@@ -414,7 +414,7 @@ def test_checkpoint_export_reads_the_live_trained_tensors():
 
 def test_padded_batch_plan_reproduces_the_hf_merge_layout():
     """plan_padded_batch (leopard_b200/hf.py) against the oracle's step-by-step restatement of HF's
-    `_merge_input_ids_with_image_features` (SURVEY.md App. A.1): same max_len, the kept rows of every batch row land exactly where
+    `_merge_input_ids_with_image_features`: same max_len, the kept rows of every batch row land exactly where
     HF's final_attention_mask is 1, positions 0 .. S_b - 1, image features consumed in batch-row order."""
     import pytest
     from types import SimpleNamespace as NS

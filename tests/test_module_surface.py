@@ -1,4 +1,4 @@
-"""CPU: the plugin classes are real `nn.Module`s over the native weights (VERDICT r1 item 7): parameters share storage with what the
+"""CPU: the plugin classes are real `nn.Module`s over the native weights: parameters share storage with what the
 kernels read, state_dict speaks the reference's HF keys, load_state_dict is in place; the Megatron shim's train_step takes the
 batch from the reference's own forward_step_func."""
 import types

@@ -45,7 +45,7 @@ def test_crop_planner_matches_reference_goldens():
 
 
 def test_baseline_config_crop_counts():
-    # SURVEY.md §8a a1/a2, D3: the allocator gives 17 / 4x7 / 8x5 ViT inputs for configs 2 / 3 / 4, 1 for config 1
+    # the allocator gives 17 / 4x7 / 8x5 ViT inputs for configs 2 / 3 / 4, 1 for config 1
     assert pp.plan_crops([(384, 384)]) == [1]
     assert pp.plan_crops([(1344, 1344)]) == [17]
     assert pp.plan_crops([(896, 1152)] * 4) == [7, 7, 7, 7]

@@ -1,4 +1,4 @@
-"""CPU: tensor-parallel + sequence-parallel decoder (leopard_b200/tp.py, SURVEY.md §8f-4).
+"""CPU: tensor-parallel + sequence-parallel decoder (leopard_b200/tp.py).
   * TP-sharded Megatron checkpoint split / merge follow the converter's per-key rules and are exact inverses;
   * the TP layer loop (world 2, gloo, native ops replaced by their contract restatements) reproduces the TP = 1 oracle."""
 import os

@@ -1,8 +1,7 @@
 """-m gpu: the SFT step's kernels (csrc/lp_train.cu) and the whole step (train.py) against the oracle.
 
-First run on a B200 in round 2 (gpurun_out/r02a_train_tests.log -> profiles/r02_train_tests.log): all green except the
-trainable-tower step on the materialised route (T = 676 is not a multiple of 8: fixed with zero-padded key / value
-operands); the flash-style backward is the default route since then.  Hard passes: no xfail markers.
+The flash-style attention backward is the default route; the materialised one pads keys and values where T (676 in the tower) is
+not a multiple of 8.  Hard passes: no xfail markers.
 Checker: oracle/native_ops.py per kernel (same signatures), oracle/train.py (autograd) for the whole step."""
 import pytest
 import torch
