@@ -32,10 +32,11 @@ from .seqcache import SequenceCache
 
 F32, BF16, I32 = torch.float32, torch.bfloat16, torch.int32
 TENSOR_CORE_MIN_ROWS = 64
-# up to 64 rows a product is bound by its weights and lp_linear streams them once, epilogue included; its operand traffic grows with
-# rows times columns, the tcgen05 GEMM's latency with K alone: they cross near rows * columns = 170,000 (K = 2048: 32 rows by 8192
-# columns 17.3 us against 13.7, 16 rows 11.5 against 14.4, 64 rows by 2048 columns 18.7 against 13.4, 32 rows 9.9 against 12.7)
-STREAM_ROWS, STREAM_ROWS_ALONE, STREAM_MAX_OUTPUTS = 64, 8, 170_000
+# Below 64 rows a product is bound by its weights and lp_linear streams them once, epilogue included.  From rows * columns = 170,000 on the tcgen05
+# GEMM would be faster there too (K = 2048, us: 32 rows by 8192 columns 17.3, GEMM 13.7; 16 rows 11.5, 14.4), but it adds up all of K in one chain
+# whose sums are cut off: 2.1e-6 of the result at K = 2048, 9.1e-6 at 8192, against 2.3e-7 streamed and 3.9e-7, 9.6e-7 of fp32 multiply-adds.  So
+# it has the products of 64 rows and more, as large prompts always had; at 64 rows only those above the crossing.
+STREAM_MAX_OUTPUTS = 170_000
 # Up to MOE_PAIRS_MAX (token, choice) pairs an expert's weights are streamed once for the pairs that chose it.  Both products of 16 experts,
 # width 2048, 1024 inside (us, bf16; fp32 rows), against sorted tiles: 128 pairs 66, 108; 85, 182.  256 pairs 93, 108; 138, 182.  512 pairs 161,
 # 108; 282, 182: with this few experts the sorted tiles are ahead from about 300 pairs, with 32 (width 4096) not yet at 512: 554, 683; 876, 1116.
@@ -893,13 +894,10 @@ class SeqLMEngine:
         return torch.empty(shape, dtype=dtype, device=self.device)
 
     def _on_gemm(self, a: torch.Tensor, w: torch.Tensor) -> bool:
-        """Whether the tcgen05 GEMM takes a[M, K] @ w[N, K].T: it has the rows to fill tiles, or (above the few rows that are always streamed)
-        the columns to be faster than lp_linear's weight-streaming kernel, and its TMA loads can start on 16-byte boundaries.  A limit
-        above TENSOR_CORE_MIN_ROWS (tensor_core_rows; None: never) holds for every product."""
+        """Whether the tcgen05 GEMM takes a[M, K] @ w[N, K].T: it has the rows (tensor_core_rows; None: never) to fill tiles, at the fewest rows the
+        columns to be faster than lp_linear's weight-streaming kernel, and its TMA loads can start on 16-byte boundaries."""
         (M, K), N = a.shape, w.shape[0]
-        if self.tensor_core_rows is None or M < self.tensor_core_rows > TENSOR_CORE_MIN_ROWS:
-            return False
-        if M <= STREAM_ROWS_ALONE or (M <= STREAM_ROWS and M * N <= STREAM_MAX_OUTPUTS):
+        if self.tensor_core_rows is None or M < self.tensor_core_rows or (M <= TENSOR_CORE_MIN_ROWS and M * N <= STREAM_MAX_OUTPUTS):
             return False
         return (a.dtype == BF16 and N >= 128 and K >= 64 and N % 8 == 0 and K % 8 == 0 and a.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
                 and a.stride(1) == 1 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)

@@ -140,7 +140,7 @@ def test_feed_forward_alone(backend, T, ff):
 
 @pytest.mark.gpu
 def test_large_bf16_products_run_on_the_tensor_cores():
-    """in the serving precision a product of more than 64 rows, or with the columns for it of more than 8, goes to the tcgen05 GEMM; same result as
+    """in the serving precision a product of more than 64 rows, or of 64 with the columns for it, goes to the tcgen05 GEMM; same result as
     lp_linear's kernels up to the rounding of the accumulation order, ragged N and K included, with and without an epilogue"""
     cfg = model([retention_layer()])
     w = O.random_weights(cfg, seed=2)
