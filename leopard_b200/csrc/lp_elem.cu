@@ -597,8 +597,10 @@ extern "C" int lp_embed_merge(const long long* ids, int L, long long image_id, i
   note_launch(2);
   merge_plan_kernel<<<1, 1024, 0, stream>>>(ids, L, image_id, rows_per_slot, dst, src, totals);
   LP_CHECK_CUDA(cudaGetLastError());
-  // about 16,000 CTAs: a slot's rows over as many as short prompts leave room for, one a token where there are no image rows
-  const int spread = n_feat_rows <= 0 ? 1 : min(rows_per_slot, max(1, 16384 / L));
+  // A slot's rows over as many CTAs as a grid of about 16,000 leaves room for, eight at least; one a token where there are no image rows.  Measured (us,
+  // width 4096, slots of 169 rows; a CTA a row, one CTA at least, eight): 200 ids with 1 slot 22, 13, 13; 1000 with 28 93, 26, 26; 3559 with 28
+  // 322, 69, 53; 8192 with 40 737, 130, 84; 16,384 with 50 1477, 250, 142.  Four times the grid: 200 ids 22, 1000 41, 16,384 137.
+  const int spread = n_feat_rows <= 0 ? 1 : min(rows_per_slot, max(8, 16384 / L));
   merge_copy_kernel<<<dim3(L, spread), 128, 0, stream>>>(ids, dst, src, reinterpret_cast<const bf16*>(table), ldt, vocab,
                                            reinterpret_cast<const bf16*>(feats), ldf, n_feat_rows,
                                            reinterpret_cast<bf16*>(out), ldo, D, rows_per_slot);

@@ -63,7 +63,7 @@ void emu_embed_merge(const long long* ids, int L, long long image_id, int rows_p
   int* src = plan + L;
   int* totals = plan + 2 * L;
   emu::launch(dim3(1), dim3(1024), [&] { merge_plan_kernel(ids, L, image_id, rows_per_slot, dst, src, totals); });
-  emu::launch(dim3(L, rows_per_slot), dim3(128), [&] {
+  emu::launch(dim3(L, rows_per_slot > 1 ? 2 : 1), dim3(128), [&] {
     merge_copy_kernel(ids, dst, src, B(table), ldt, vocab, B(feats), ldf, n_feat_rows, B(out), ldo, D, rows_per_slot);
   });
 }

@@ -212,6 +212,19 @@ def test_embed_merge_both_conventions(native_lib):
     assert n3 == 0 and torch.equal(out3[:4].cpu(), table[ids[:4]])
 
 
+@pytest.mark.parametrize("L", [95, 97, 2500, 17000])
+def test_embed_merge_slots_of_several_rows_a_cta(native_lib, L):
+    """a CTA a row of a slot, two rows to a few CTAs, and many rows to eight"""
+    g = torch.Generator().manual_seed(L)
+    table, feats = _bf(torch.randn(500, 64, generator=g)), _bf(torch.randn(3 * 169, 64, generator=g))
+    ids = torch.randint(0, 400, (L,), generator=g)
+    ids[[0, 50, L - 1]] = 450
+    out, n_slots, S = ops.embed_merge(ids.cuda(), table.cuda(), feats.cuda(), 450, 169)
+    assert (n_slots, S) == (3, L + 3 * 168)
+    want = torch.cat([feats[:169], table[ids[1:50]], feats[169:338], table[ids[51:L - 1]], feats[338:]])
+    assert torch.equal(out[:S].cpu(), want)
+
+
 def test_bad_arguments_report_errors(native_lib):
     from leopard_b200._lib import NativeError
     a = torch.zeros(8, 60, dtype=torch.bfloat16, device="cuda")
