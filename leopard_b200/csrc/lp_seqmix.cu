@@ -174,7 +174,9 @@ retention_scan_kernel(RetArgs a, const int* __restrict__ seq_chunk0, const int* 
 // (3) o_i = decay^(i+1) q_i^T S_start + sum_(j<=i) decay^(i-j) (q_i . k_j) v_j; then o / rms(o) * silu(g).  The chunk's start state is
 // staged in shared memory where that is small (stage_s); a state of 128 x 128 would leave one CTA an SM, and the CTAs waiting for it and for
 // each other's phases took 1.23 ms (4096 tokens, 16 heads): read where it lies (L2, whole lines, eight loads in flight) three CTAs share an
-// SM and it takes 0.46 ms.  4 x 4 outputs per thread.
+// SM and it takes 0.46 ms.  4 x 4 outputs per thread.  The line is what leaves three CTAs an SM; whole prompts on both sides (us, staged up to
+// 200 KB, and so): 16 heads of 128, 4096 tokens 1450, 756, 512 tokens 150, 93; 8 heads of 96 286, 203 and 62, 58; 16 of 80 355, 313 and 59, 57; 8 of
+// 128 keys and 64 values 264, 188 and 60, 61.  64 x 64 is staged on both.
 __global__ void __launch_bounds__(RET_CHUNK_THREADS)
 retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const int* __restrict__ chunk_row0, const int* __restrict__ chunk_len,
                            const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0, const float* __restrict__ ws, int stage_s) {

@@ -31,7 +31,8 @@
 //                         the heads in shared memory and adds the values with the mixed weights.
 //   lp_window_attn_talk_tiles  the same for prompts, a CTA per tile of 4 consecutive rows of a request and all heads.
 //   lp_window_attn_tiles  the same for prompts, a CTA per tile of 2 or 4 consecutive rows of a request: the rows share every key and
-//                         value row the tile reads, each (row, key) pair masked by the row's own rule.
+//                         value row the tile reads, each (row, key) pair masked by the row's own rule.  Heads of 128 run on the matrix
+//                         instructions, a CTA per chunk of up to 32 rows, where such CTAs fill the chip.
 #include <cuda_pipeline.h>
 #include "lp_host.h"
 #include "../../include/leopard_b200.h"
@@ -742,10 +743,10 @@ window_attn_tile_kernel(WinArgs a, int n_chunks, const int* __restrict__ chunk_s
 // An infinity, a NaN and a number that rounds to infinity have no terms (their last one is NaN), and a weight of zero times one of them is NaN in
 // every row of the product, seen or not.  So a CTA with an output that is not finite starts again on wm_plain_chunk: fp32 multiply-adds, each
 // pair over the keys it sees, as window_attn_kernel does.
-// Bound by instruction issue at two warps a scheduler (Q, K and V planes fill shared memory): about 2,000 instructions beside the 384 products
-// of a warp's tile, so rows are looked up once a key (a lane each), chains start from zero in the instruction, masks run only on tiles that
+// Bound by instruction issue at two warps a scheduler (Q, K and V planes fill shared memory): about 1,800 instructions beside the 384 products
+// of a warp's tile (issue slots 35 %, tensor pipe 50 % busy), so rows are looked up once a key (a lane each), chains start from zero in the instruction, masks run only on tiles that
 // need them.  Measured (B200, 4096 tokens, 16 heads on 4, window 1024 + pooled blocks, capped): 0.90 ms a layer, without the cap and blocks 0.76;
-// fp32 multiply-adds (window_attn_tile_kernel, which keeps other head sizes) 1.90; the first form of this kernel 1.07.
+// fp32 multiply-adds (window_attn_tile_kernel, which keeps other head sizes and small launches) 1.90; the first form of this kernel 1.07.
 constexpr int WM_D = 128, WM_KT = 32, WM_ROWS = 32;
 template <int QH> constexpr size_t wm_smem_words() { return (size_t)3 * WM_ROWS * QH * WM_D / 2 + 2 * 3 * WM_KT * WM_D / 2 + 2 * WM_KT * WM_D; }
 
