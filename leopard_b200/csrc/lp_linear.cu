@@ -19,6 +19,7 @@
 //
 // The tcgen05 GEMM (lp_gemm_bf16) stays the matrix product of large bf16 problems; these kernels cover what it does not take:
 // fp32 operands, arbitrary shapes, few rows, and row-indexed groups whose sizes are only known on the device.
+#include <cuda_pipeline.h>
 #include "lp_host.h"
 #include "../../include/leopard_b200.h"
 
@@ -288,8 +289,8 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) linear_rows_kernel(LinArgs a)
 // out of the way.  So the weight tile is the 16-row operand of the warp's matrix instruction and up to MG groups of eight rows of A
 // are its other one: a CTA owns 16 NT output columns, its warps share out K in steps of 32 (a lane reads 16 bytes of each weight row and of its
 // row of A; the same permutation of k on both sides, which a sum does not see), 4 NT weight loads per lane (2 NT from 17 rows on, where registers
-// are short) are in flight before the first product, and the warps' sums meet in shared memory in a fixed order, what each addition rounds
-// off kept and added at the end.  The gated units take gate row n and up row n + N / 2 as rows g and g + 8 of one tile, so both halves of an
+// are short) are in flight before the first product, and the warps' sums meet in shared memory in a fixed order; up to 16 rows, and for pairs, what each
+// addition rounds off is kept and added at the end (one-row kernels did these before; with more rows it costs up to 8 % of short products).  The gated units take gate row n and up row n + N / 2 as rows g and g + 8 of one tile, so both halves of an
 // output end up in one lane.
 // fp32 rows of A are cut into three bf16 terms that add up to them exactly (8 + 8 + 8 bits): every product is still exact.  The
 // instruction cuts its running sum off instead of rounding it, a bias that grows with the chain.  So chains are short and added in fp32: 16
@@ -543,13 +544,21 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
       if (n >= n_out) continue;
       const int j = gated ? nl >> 3 : nl >> 4, r = gated ? nl & 7 : nl & 15;
       const int at = (((j * MG + (ml >> 3)) * 4 + (r >> 3) * 2 + (ml & 1)) * 32) + (r & 7) * 4 + ((ml & 7) >> 1);
-      float s = 0.f, s2 = 0.f, lost = 0.f, lost2 = 0.f;      // what the additions round off is added at the end
-      for (int w = 0; w < n_warps; ++w) {
-        lost += add_exactly(s, dyn_smem[w * SLOTS * 32 + at]);
-        if (gated) lost2 += add_exactly(s2, dyn_smem[w * SLOTS * 32 + at + 64]);
+      float s = 0.f, s2 = 0.f;
+      if (MG <= 2 || pairs) {      // what the additions round off is added at the end
+        float lost = 0.f, lost2 = 0.f;
+        for (int w = 0; w < n_warps; ++w) {
+          lost += add_exactly(s, dyn_smem[w * SLOTS * 32 + at]);
+          if (gated) lost2 += add_exactly(s2, dyn_smem[w * SLOTS * 32 + at + 64]);
+        }
+        if (s + lost == s + lost) s += lost;      // beside an infinity the rest is NaN
+        if (s2 + lost2 == s2 + lost2) s2 += lost2;
+      } else {
+        for (int w = 0; w < n_warps; ++w) {
+          s += dyn_smem[w * SLOTS * 32 + at];
+          if (gated) s2 += dyn_smem[w * SLOTS * 32 + at + 64];
+        }
       }
-      if (s + lost == s + lost) s += lost;      // beside an infinity the rest is NaN
-      if (s2 + lost2 == s2 + lost2) s2 += lost2;
       const int m = pairs ? pair_of[m0 + ml] : m0 + ml;
       if (a.row_scale != nullptr) {
         s *= a.row_scale[m];
@@ -602,8 +611,8 @@ static int dispatch_stream(const LinArgs& a, int a_fp32, int c_fp32, int batch, 
   const long long wide = problems * ((n_out + 2 * per - 1) / (2 * per));
   const int nt = (mg == 1 || a_fp32) && wide >= 2 * sm_count() && (a.seg_cols == 0 || a.seg_cols % (2 * per) == 0) ? 2 : 1;
   const long long ctas = problems * ((n_out + nt * per - 1) / (nt * per));
-  // a short K has no work for more warps; a grid of few CTAs wants more loads in flight in each (N = 2048, K = 8192: 15 us with 16 warps, 11 with 32)
-  int warps = a.K <= 256 ? 4 : !a_fp32 && mg * nt == 1 && ctas <= sm_count() && a.K >= 4096 ? 32 : ctas <= 2 * sm_count() && a.K >= 1024 && mg <= 4 ? 16 : 8;
+  // a short K has no work for more warps (up to eight rows 192 of them run 4.0 us with four, 3.2 with eight); a grid of few CTAs wants more loads in flight in each (N = 2048, K = 8192: 15 us with 16 warps, 11 with 32)
+  int warps = a.K <= (mg == 1 ? 128 : 256) ? 4 : !a_fp32 && mg * nt == 1 && ctas <= sm_count() && a.K >= 4096 ? 32 : ctas <= 2 * sm_count() && a.K >= 1024 && mg <= 4 ? 16 : 8;
   dim3 grid((n_out + nt * per - 1) / (nt * per), n_groups > 0 ? n_groups : 1, n_groups > 0 ? 1 : batch);
 #define LP_STREAM(MG)                                                                                                               \
   (a_fp32 ? (nt == 2 ? launch_stream<float, 2, MG>(a, c_fp32, grid, warps, n_pairs, stream) : launch_stream<float, 1, MG>(a, c_fp32, grid, warps, n_pairs, stream)) \
@@ -623,7 +632,15 @@ static int dispatch_stream(const LinArgs& a, int a_fp32, int c_fp32, int batch, 
 // Measured (B200, M = 4096, N = 8192, K = 2048): fp32 rows 1.47 ms = 93 TFLOP/s (three products each; 64 x 64 tiles on fp32 FMAs 5.4 ms, 25),
 // bf16 rows 0.72 ms; mma.sync alone reaches 520 TFLOP/s of bf16 products here, 450 with a sum of its own every few.  Error against 64 bits at
 // K = 1024 / 4096: 1.2e-7 / 2.1e-7 (FMA chains over K: 5.7e-7 / 1.1e-6).
+// What a product is added to (c_accum) and its gate are copied in (cp.async) while the products run: read where they are used, a load at a time, they
+// took 6 us of every CTA (65 rows, N = 64, K = 16 to 256: 15.0 to 21.4 us instead of 9.1 to 15.8).
 constexpr int MT_BM = LIN_BM, MT_BN = 128, MT_BK = 32, MT_LDC = MT_BN + 4, MT_THREADS = 256;
+// bytes of shared memory: the stages, then in their place the tile of sums, and after them a tile each of what it is added to and of the gate
+template <typename AT> constexpr size_t mt_smem() {
+  constexpr size_t stages = 2 * sizeof(uint32_t) * ((sizeof(AT) == 4 ? 3 : 1) * MT_BM * MT_BK / 2 + MT_BN * MT_BK / 2), tile = sizeof(float) * MT_BM * MT_LDC;
+  return stages > tile ? stages : tile;
+}
+constexpr size_t MT_SIDE = sizeof(float) * MT_BM * MT_BN;
 
 // the tile's sums in shared memory (a gated unit's halves eight columns apart), rows from m0 and output columns from n0 on
 template <typename AT>
@@ -642,7 +659,7 @@ __device__ __noinline__ void lin_mend_tile(float* tile, const AT* A, long long l
   __syncthreads();
 }
 
-template <typename AT>
+template <typename AT, bool SIDE>
 __global__ void __launch_bounds__(MT_THREADS, 2) linear_mma_kernel(LinArgs a, int gated, int c_fp32) {
   extern __shared__ float dyn_smem[];
   constexpr int PLANES = sizeof(AT) == 4 ? 3 : 1;
@@ -706,6 +723,19 @@ __global__ void __launch_bounds__(MT_THREADS, 2) linear_mma_kernel(LinArgs a, in
 #pragma unroll
     for (int i = 0; i < W_CHUNKS; ++i) *reinterpret_cast<uint4*>(st + PLANES * A_WORDS + (tid + i * THREADS) * 4) = rw[i];
   };
+  if constexpr (SIDE) {      // each thread fetches what it will use itself: no barrier
+    float* side = dyn_smem + mt_smem<AT>() / sizeof(float);
+#pragma unroll 1
+    for (int e = tid; e < BM * cols; e += THREADS) {
+      const int m = m0 + e / cols, n = n0 + e % cols;
+      if (m >= a.M || n >= n_out) continue;
+      if (a.c_accum && c_fp32)
+        __pipeline_memcpy_async(side + e, reinterpret_cast<const float*>(a.C) + (long long)z * a.c_batch + (long long)m * a.ldc + n, 4);
+      if (a.gate != nullptr)
+        __pipeline_memcpy_async(side + BM * MT_BN + e, a.gate + (long long)z * a.gate_batch + (long long)m * a.ldg + n, 4);
+    }
+    __pipeline_commit();
+  }
   const int wm = (warp / WARPS_N) * 32, wn = (warp % WARPS_N) * NI * 8;
   float acc[2][NI][4];
 #pragma unroll
@@ -761,6 +791,8 @@ __global__ void __launch_bounds__(MT_THREADS, 2) linear_mma_kernel(LinArgs a, in
   } else {
     __syncthreads();
   }
+  const float* side = dyn_smem + mt_smem<AT>() / sizeof(float);
+  if constexpr (SIDE) __pipeline_wait_prior(0);
 #pragma unroll 1
   for (int e = tid; e < BM * cols; e += THREADS) {
     const int ml = e / cols, nl = e % cols, m = m0 + ml, n = n0 + nl;
@@ -776,11 +808,11 @@ __global__ void __launch_bounds__(MT_THREADS, 2) linear_mma_kernel(LinArgs a, in
       if (gated) s2 += a.bias[n + n_out];
     }
     float v = gated ? lin_gate(a.epi, s, s2, a.e0, a.e1) : lin_epi(a.epi, s, a.e0, a.e1);
-    if (a.gate != nullptr) v /= 1.0f + expf(-a.gate[(long long)z * a.gate_batch + (long long)m * a.ldg + n]);
+    if (SIDE && a.gate != nullptr) v /= 1.0f + expf(-side[BM * MT_BN + e]);
     const long long at_c = (long long)z * a.c_batch + (long long)m * a.ldc + n;
     if (c_fp32) {
       float* C = reinterpret_cast<float*>(a.C) + at_c;
-      *C = a.c_accum ? fmaf(a.c_scale, v, *C) : v;
+      *C = SIDE && a.c_accum ? fmaf(a.c_scale, v, side[e]) : v;
     } else {
       bf16* C = reinterpret_cast<bf16*>(a.C) + at_c;
       *C = __float2bfloat16(a.c_accum ? fmaf(a.c_scale, v, __bfloat162float(*C)) : v);
@@ -788,17 +820,38 @@ __global__ void __launch_bounds__(MT_THREADS, 2) linear_mma_kernel(LinArgs a, in
   }
 }
 
-template <typename AT>
+template <typename AT, bool SIDE>
 static int launch_mma(const LinArgs& a, int c_fp32, int batch, int m_tiles, cudaStream_t stream) {
-  constexpr size_t stages = 2 * sizeof(uint32_t) * ((sizeof(AT) == 4 ? 3 : 1) * MT_BM * MT_BK / 2 + MT_BN * MT_BK / 2), tile = sizeof(float) * MT_BM * MT_LDC;
-  constexpr size_t smem = stages > tile ? stages : tile;
+  constexpr size_t smem = mt_smem<AT>() + (SIDE ? 2 * MT_SIDE : 0);
   const int cols = gated_epi(a.epi) ? MT_BN / 2 : MT_BN, n_out = gated_epi(a.epi) ? a.N / 2 : a.N;
-  if (smem > 48 * 1024) LP_CHECK_CUDA(cudaFuncSetAttribute(linear_mma_kernel<AT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024) LP_CHECK_CUDA(cudaFuncSetAttribute(linear_mma_kernel<AT, SIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid((n_out + cols - 1) / cols, m_tiles, batch);
-  linear_mma_kernel<AT><<<grid, MT_THREADS, smem, stream>>>(a, gated_epi(a.epi), c_fp32);
+  linear_mma_kernel<AT, SIDE><<<grid, MT_THREADS, smem, stream>>>(a, gated_epi(a.epi), c_fp32);
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
+}
+// A K of a few steps does not pay for the terms, the tile in shared memory and a K step of 32; columns for half a tile pay for a whole one.  Measured (us,
+// linear_tile_kernel and this one, fp32 rows): K = 16: 65 x 64 5.3, 9.1, 4096 x 8192 84, 133; K = 32: 300 x 512 7.0, 9.3, 4096 x 2048 34, 37; K = 64: 300 x 512
+// 9.2, 10.2, 300 x 2048 11.6, 10.3, 4096 x 2048 56, 42; 16 products of 4096 x 64 32, 42; K = 96: 300 x 512 11.0, 11.2, 300 x 2048 13.9, 11.3; K = 128: 65 x 64
+// 12.8, 11.8.  Gated: K = 16 300 x 8192 10.1, 13.2; K = 32 65 x 64 8.8, 7.6, 300 x 8192 14.0, 13.2.  Added to a stream: K = 128 300 x 512
+// 14.7, 15.7, 300 x 8192 40, 31; behind a gate: 15.2, 17.8, K = 192 19.5, 19.4.  bf16 rows cross at the same places.
+static bool mma_pays(const LinArgs& a, int batch, int m_tiles) {
+  if (gated_epi(a.epi)) return a.K >= 32;
+  const int lo = a.c_accum || a.gate != nullptr ? 96 : 40, hi = a.c_accum || a.gate != nullptr ? 192 : 128;      // two more tiles to bring in
+  if (a.K < lo || a.K >= hi) return a.K >= hi;
+  return a.N > MT_BN / 2 && 2LL * batch * m_tiles * ((a.N + MT_BN - 1) / MT_BN) > sm_count();
+}
+// The same for up to 64 rows: 33 x 512 5.4, 6.9 (fp32 rows, K = 8), 6.7, 7.1 (32), 8.5, 7.1 (64); 64 x 512 5.4, 8.7, 6.7, 8.7, 8.7, 8.7; bf16 rows 64 x 512 5.6, 6.9
+// (8), 6.4, 6.7 (32), 33 x 512 5.6, 5.2 (8); up to 32 rows the streaming kernel is ahead at every K.
+static bool stream_pays(const LinArgs& a, int a_fp32) {
+  return a.M <= (a_fp32 ? 32 : 48) || a.K > 32 || (gated_epi(a.epi) && a.K >= 16);
+}
+
+static int dispatch_mma(const LinArgs& a, int a_fp32, int c_fp32, int batch, int m_tiles, cudaStream_t stream) {
+  if ((a.c_accum && c_fp32) || a.gate != nullptr)
+    return a_fp32 ? launch_mma<float, true>(a, c_fp32, batch, m_tiles, stream) : launch_mma<bf16, true>(a, c_fp32, batch, m_tiles, stream);
+  return a_fp32 ? launch_mma<float, false>(a, c_fp32, batch, m_tiles, stream) : launch_mma<bf16, false>(a, c_fp32, batch, m_tiles, stream);
 }
 
 template <typename AT, typename CT, bool GATED>
@@ -856,13 +909,12 @@ extern "C" int lp_linear(const lp_linear_desc* d, void* stream_) {
   LP_REQUIRE(d->seg_cols == 0 || (d->seg_cols > 0 && d->n_segs >= 1 && d->seg_cols % (d->M <= ROWS_MAX ? ROWS_WARPS : LIN_BN) == 0),
              "lp_linear: column segments of %d do not fit the CTAs of a product of %d rows", d->seg_cols, d->M);
   LP_REQUIRE(d->seg_cols == 0 || !gated_epi(d->epi), "lp_linear: a gated unit has one operand");
-  if (d->M <= STREAM_MAX_ROWS && stream_ok(a, d->a_fp32, d->batch) && (d->seg_cols == 0 || d->seg_cols % 16 == 0))
+  if (d->M <= STREAM_MAX_ROWS && stream_ok(a, d->a_fp32, d->batch) && (d->seg_cols == 0 || d->seg_cols % 16 == 0) && stream_pays(a, d->a_fp32))
     return dispatch_stream(a, d->a_fp32, d->c_fp32, d->batch, d->M, 0, 0, stream);
   // the tile kernel on the matrix instructions; operands without 16-byte rows stay on fp32 FMAs
-  if (stream_ok(a, d->a_fp32, d->batch) && (d->seg_cols == 0 || d->seg_cols % MT_BN == 0) && d->M > STREAM_MAX_ROWS) {
-    const int m_tiles = (d->M + MT_BM - 1) / MT_BM;
-    return d->a_fp32 ? launch_mma<float>(a, d->c_fp32, d->batch, m_tiles, stream) : launch_mma<bf16>(a, d->c_fp32, d->batch, m_tiles, stream);
-  }
+  if (stream_ok(a, d->a_fp32, d->batch) && (d->seg_cols == 0 || d->seg_cols % MT_BN == 0) && d->M > STREAM_MAX_ROWS &&
+      mma_pays(a, d->batch, (d->M + MT_BM - 1) / MT_BM))
+    return dispatch_mma(a, d->a_fp32, d->c_fp32, d->batch, (d->M + MT_BM - 1) / MT_BM, stream);
   return dispatch_linear(a, d->a_fp32, d->c_fp32, d->batch, (d->M + LIN_BM - 1) / LIN_BM, true, stream);
 }
 
@@ -919,8 +971,7 @@ extern "C" int lp_linear_grouped(const lp_linear_desc* d, const int* tile_group,
   a.a_rows = a_rows; a.tile_group = tile_group; a.z_group = nullptr; a.a_div = 1;
   a.bias = d->bias; a.row_scale = d->row_scale; a.gate = d->gate; a.ldg = d->ldg; a.gate_batch = d->gate_batch;
   a.seg_cols = 0; a.n_segs = 0; a.a_seg = 0;
-  if (stream_ok(a, d->a_fp32, 1))
-    return d->a_fp32 ? launch_mma<float>(a, d->c_fp32, 1, n_tiles, stream) : launch_mma<bf16>(a, d->c_fp32, 1, n_tiles, stream);
+  if (stream_ok(a, d->a_fp32, 1) && mma_pays(a, 1, n_tiles)) return dispatch_mma(a, d->a_fp32, d->c_fp32, 1, n_tiles, stream);
   return dispatch_linear(a, d->a_fp32, d->c_fp32, 1, n_tiles, false, stream);
 }
 

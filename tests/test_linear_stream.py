@@ -42,7 +42,8 @@ def _data(M, N, K, dtype, device, seed=0):
 
 
 @pytest.mark.parametrize("dtype", [BF16, F32])
-@pytest.mark.parametrize("M,N,K", [(1, 1, 8), (8, 17, 40), (9, 33, 256), (16, 16, 264), (33, 48, 400), (64, 40, 72), (65, 130, 40), (129, 9, 72)])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 8), (8, 17, 40), (9, 33, 256), (16, 16, 264), (33, 48, 400), (64, 40, 72), (65, 130, 40), (129, 9, 72),
+                                   (33, 24, 16), (49, 24, 16), (64, 24, 32), (64, 24, 40), (65, 130, 32), (65, 130, 136), (129, 9, 136), (100, 300, 264)])
 def test_rows_columns_and_steps(backend, dtype, M, N, K):
     a, w, want, ad, wd = _data(M, N, K, dtype, backend[0])
     out = torch.empty(M, N, device=backend[0])
@@ -54,9 +55,9 @@ def test_rows_columns_and_steps(backend, dtype, M, N, K):
 
 
 @pytest.mark.parametrize("dtype", [BF16, F32])
-@pytest.mark.parametrize("M", [11, 70])
-def test_epilogues(backend, dtype, M):
-    N, K = 36, 64
+@pytest.mark.parametrize("M,K", [(11, 64), (70, 64), (70, 200)])
+def test_epilogues(backend, dtype, M, K):
+    N = 36
     a, w, z, ad, wd = _data(M, N, K, dtype, backend[0])
     g = torch.Generator().manual_seed(1)
     bias, scale, gate, x = torch.randn(N, generator=g), torch.rand(M, generator=g), torch.randn(M, N, generator=g), torch.randn(M, N, generator=g)
@@ -73,12 +74,22 @@ def test_epilogues(backend, dtype, M):
 
 def test_batches_and_segments(backend):
     g = torch.Generator().manual_seed(3)
-    for M in (10, 66):
-        heads, N, K = 3, 24, 40
-        a, w = torch.randn(M, heads * 48, generator=g), torch.randn(heads, N, K, generator=g).to(BF16)
+    for M, K in ((10, 40), (66, 200), (66, 40)):
+        heads, N = 3, 24
+        a, w = torch.randn(M, heads * (K + 8), generator=g), torch.randn(heads, N, K, generator=g).to(BF16)
+        ad, wd = a.to(backend[0]), w.to(backend[0])
         out = torch.empty(M, heads * N, device=backend[0])
-        _call(backend, a.to(backend[0]), w.to(backend[0]), out, M, batch=heads, a_batch=48, c_batch=N)
-        assert rel_err(out, torch.cat([a[:, 48 * h:48 * h + K].double() @ w[h].double().T for h in range(heads)], 1)) < 2e-6
+        _call(backend, ad, wd, out, M, batch=heads, a_batch=K + 8, c_batch=N)
+        want = torch.cat([a[:, (K + 8) * h:(K + 8) * h + K].double() @ w[h].double().T for h in range(heads)], 1)
+        assert rel_err(out, want) < 2e-6
+        gate, x = torch.randn(M, heads * N, generator=g), torch.randn(M, heads * N, generator=g)      # a gate per problem, added to what is there
+        out, gd = x.clone().to(backend[0]), gate.to(backend[0])
+        _call(backend, ad, wd, out, M, batch=heads, a_batch=K + 8, c_batch=N, gate=gd, ldg=heads * N, gate_batch=N, c_accum=1, c_scale=0.5)
+        assert rel_err(out, x.double() + 0.5 * want * torch.sigmoid(gate.double())) < 2e-6
+        out = torch.empty(M, heads * N, dtype=BF16, device=backend[0])
+        _call(backend, ad, wd, out, M, batch=heads, a_batch=K + 8, c_batch=N, gate=gd, ldg=heads * N, gate_batch=N)
+        assert rel_err(out, want * torch.sigmoid(gate.double())) < 3e-3
+    K = 40
     ops, w = torch.randn(2, 5, K, generator=g).to(BF16), torch.randn(40, K, generator=g).to(BF16)
     out = torch.empty(5, 40, device=backend[0])
     od, wd = ops.to(backend[0]), w.to(backend[0])
@@ -142,7 +153,7 @@ def test_unusual_numbers(backend):
 def test_infinite_weights(backend, dtype, M, kind):
     """an infinite weight makes its column's outputs infinite, with the sign of the product, in both halves of a gated unit too; NaN where it
     meets a zero, an infinity of the other sign or a NaN"""
-    N, K, dev = 24, 40, backend[0]
+    N, K, dev = 24, 136, backend[0]
     a, w, _, _, _ = _data(M, N, K, dtype, dev)
     a[0, 3], a[1, 5] = 0.0, float("nan")
     w[2, 3], w[5, 3], w[7, 11], w[7, 12], w[N // 2 + 3, 30] = float("inf"), -float("inf"), float("inf"), -float("inf"), float("inf")
@@ -173,10 +184,11 @@ def test_infinite_weights(backend, dtype, M, kind):
 
 
 @pytest.mark.parametrize("dtype", [BF16, F32])
-def test_row_tiles_of_groups(backend, dtype):
+@pytest.mark.parametrize("K", [24, 40, 136])
+def test_row_tiles_of_groups(backend, dtype, K):
     """tiles of 64 gathered rows, each on its group's weight; padding rows are zeros, a tile without a group is left alone"""
     g = torch.Generator().manual_seed(9)
-    N, K, T = 136, 40, 30
+    N, T = 136, 30
     a, w = torch.randn(T, K, generator=g).to(dtype), (torch.randn(3, N, K, generator=g) * K ** -0.5).to(BF16)
     groups, rows = torch.tensor([2, -1, 0], dtype=torch.int32), torch.randint(-1, T, (192,), generator=g).to(torch.int32)
     out = torch.full((192, N), 7.0)
