@@ -611,7 +611,7 @@ static int dispatch_stream(const LinArgs& a, int a_fp32, int c_fp32, int batch, 
   const long long wide = problems * ((n_out + 2 * per - 1) / (2 * per));
   const int nt = (mg == 1 || a_fp32) && wide >= 2 * sm_count() && (a.seg_cols == 0 || a.seg_cols % (2 * per) == 0) ? 2 : 1;
   const long long ctas = problems * ((n_out + nt * per - 1) / (nt * per));
-  // a short K has no work for more warps (up to eight rows 192 of them run 4.0 us with four, 3.2 with eight); a grid of few CTAs wants more loads in flight in each (N = 2048, K = 8192: 15 us with 16 warps, 11 with 32)
+  // a short K has no work for more warps (K = 192, one row: 4.0 us with four, 3.2 with eight); a grid of few CTAs wants more loads in flight in each (N = 2048, K = 8192: 15 us with 16 warps, 11 with 32)
   int warps = a.K <= (mg == 1 ? 128 : 256) ? 4 : !a_fp32 && mg * nt == 1 && ctas <= sm_count() && a.K >= 4096 ? 32 : ctas <= 2 * sm_count() && a.K >= 1024 && mg <= 4 ? 16 : 8;
   dim3 grid((n_out + nt * per - 1) / (nt * per), n_groups > 0 ? n_groups : 1, n_groups > 0 ? 1 : batch);
 #define LP_STREAM(MG)                                                                                                               \
