@@ -289,16 +289,16 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) linear_rows_kernel(LinArgs a)
 // out of the way.  So the weight tile is the 16-row operand of the warp's matrix instruction and up to MG groups of eight rows of A
 // are its other one: a CTA owns 16 NT output columns, its warps share out K in steps of 32 (a lane reads 16 bytes of each weight row and of its
 // row of A; the same permutation of k on both sides, which a sum does not see), 4 NT weight loads per lane (2 NT from 17 rows on, where registers
-// are short) are in flight before the first product, and the warps' sums meet in shared memory in a fixed order; up to 16 rows, and for pairs, what each
-// addition rounds off is kept and added at the end (one-row kernels did these before; with more rows it costs up to 8 % of short products).  The gated units take gate row n and up row n + N / 2 as rows g and g + 8 of one tile, so both halves of an
-// output end up in one lane.
+// are short) are in flight before the first product, and the warps' sums meet in shared memory in a fixed order; up to 16 rows, and for pairs,
+// what each addition rounds off is kept and added at the end (one-row kernels did these before; with more rows it costs up to 8 % of short
+// products).  The gated units take gate row n and up row n + N / 2 as rows g and g + 8 of one tile, so both halves of an output end up in one lane.
 // fp32 rows of A are cut into three bf16 terms that add up to them exactly (8 + 8 + 8 bits): every product is still exact.  The
 // instruction cuts its running sum off instead of rounding it, a bias that grows with the chain.  So chains are short and added in fp32: 16
 // products of bf16 rows, 3 x 16 of fp32 rows (small terms first), 256 of 33 to 64 bf16 rows, whose additions would cost more than the products.
 // Measured (B200, graph of launches, weights from HBM, M = 8): N = 8192, K = 2048 10.4 us (3.2 TB/s; a warp per column with fp32 FMAs: 67.6),
 // N = 32000, K = 4096 51 us (5.1 TB/s; 350), N = 2048, K = 2048 6.6 us (29.7), fp32 A 6.5 us (66).  Error against 64 bits at N = 2048, K = 2048 /
 // 8192, 1e-7 of the result: bf16 rows 0.58 / 0.70 (without what the sums of the warps round off 0.92 / 1.23; FMA chains of a lane, which this
-// kernel replaced, 0.80 / 1.24), fp32 rows 0.75 / 1.0 (1.6 / 2.9), 64 bf16 rows 2.3 / 2.3 (FMA chains over K 3.9 / 9.5).
+// kernel replaced, 0.80 / 1.24), fp32 rows 0.75 / 1.0 (1.6 / 2.9), 64 bf16 rows 2.3 / 2.4 (FMA chains over K 3.9 / 9.5).
 // Pairs (experts): the CTAs of weight group blockIdx.y gather the pairs that chose it and read the group's weights once for all of them.
 constexpr int STREAM_MAX_ROWS = 64, STREAM_MAX_PAIRS = 1024;
 
