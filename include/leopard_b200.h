@@ -702,6 +702,24 @@ int lp_latent_attend_tiles(const lp_latent_desc* desc, int R, const int* row_seq
                            const int* chunk_row0, const int* chunk_len, const float* q_abs, long long ldqa, void* out, long long ldo,
                            int out_fp32, void* stream);
 
+/* fp32 numbers as three planes of bf16 terms (upper, middle, lower bits of the mantissa: cut off, they add up to the number exactly), `plane`
+ * elements apart: rows [M, K] of `src` -> [M, K] of each plane, rows ldp elements apart.  K a multiple of 8, rows on 16-byte boundaries. */
+int lp_split_rows(const float* src, long long ld, int M, int K, void* planes, long long ldp, long long plane, void* stream);
+/* C[M, N] = A[M, K] W[N, K]^T (+ bias fp32 [N]) on the tcgen05 tensor cores with A in three planes and W bf16: an fp32 product, sums in fp32.
+ * out: 0 bf16, 1 fp32, 2 three planes c_plane elements apart.  K and N multiples of 8, rows on 16-byte boundaries. */
+int lp_gemm_split(const void* A, long long lda, long long a_plane, const void* W, long long ldw, void* C, long long ldc, long long c_plane,
+                  int out, int M, int N, int K, const float* bias, void* stream);
+/* Latent attention of prompts with every head's keys and values expanded, on the tensor cores: heads of 128 + 64 rotated channels, values of
+ * 128, kv_rank a multiple of 8.  desc as for lp_latent_prep, whose results (rotated queries, this step's cache rows) it reads; w_kv bf16
+ * [2 * heads * 128, kv_rank], rows ldw elements apart: the heads' key rows, then their value rows.  seq_row0 [n_seqs + 1], seq_pos0 [n_seqs]:
+ * the requests' rows of this step and the positions these start at; n_tiles = sum of ceil(rows / 128); n_keys = sum over requests of the positions from
+ * max(0, seq_pos0 - window + 1) (window <= 0: from 0) to the last.  out_gate (fp32 [rows, ldog] or NULL): every output is multiplied by its sigmoid.
+ * out [rows, heads * 128]. */
+size_t lp_latent_expanded_workspace_bytes(int R, int heads, int dim, int rot_dim, int kv_rank, int n_keys);
+int lp_latent_attend_expanded(const lp_latent_desc* desc, int R, int n_seqs, const int* seq_row0, const int* seq_pos0, int n_tiles, int n_keys,
+                              const void* w_kv, long long ldw, const float* out_gate, long long ldog, void* out, long long ldo, int out_fp32,
+                              void* ws, size_t ws_bytes, void* stream);
+
 /* Grouped-query attention over a paged cache of rows [keys (kv_heads x dim) | values (kv_heads x vdim)] fp32, with the visibility
  * rules and score options of sliding-window designs as parameters (csrc/lp_winattn.cu).  Query at position i of a request sees
  *   - tokens j with 0 <= i - j < window (window <= 0: every j <= i),

@@ -37,6 +37,10 @@ TENSOR_CORE_MIN_ROWS = 64
 # whose sums are cut off: 2.1e-6 of the result at K = 2048, 9.1e-6 at 8192, against 2.3e-7 streamed and 3.9e-7, 9.6e-7 of fp32 multiply-adds.  So
 # it has the products of 64 rows and more, as large prompts always had; at 64 rows only those above the crossing.
 STREAM_MAX_OUTPUTS = 170_000
+# Rows of prompts expand the visible latents into every head's keys and values (lp_latent_attend_expanded), unless many requests bring a few rows each:
+# its tiles are 128 rows of one request.  A layer of width 1024 with 8 heads (us, lp_latent_attend_tiles and this one): one request of 20 rows 64, 45, of
+# 500 297, 85; 32 requests of 12 rows 92, 81; 64 of 12 97, 120, of 24 132, 126; width 2048, 16 heads: 4096 rows 6,490, 530; 64 requests of 12 rows 225, 205.
+EXPAND_TILES, EXPAND_TILE_ROWS = 32, 24
 # Up to MOE_PAIRS_MAX (token, choice) pairs an expert's weights are streamed once for the pairs that chose it.  Both products of 16 experts,
 # width 2048, 1024 inside (us, bf16; fp32 rows), against sorted tiles: 128 pairs 66, 108; 85, 182.  256 pairs 93, 108; 138, 182.  512 pairs 161,
 # 108; 282, 182: with this few experts the sorted tiles are ahead from about 300 pairs, with 32 (width 4096) not yet at 512: 554, 683; 876, 1116.
@@ -322,6 +326,11 @@ FIRST_PRODUCT = {RetentionConfig: "w_qkvg", LatentAttentionConfig: "w_qdkv", Win
 WKV_MIXES = ("r", "k", "v", "g", "w")      # the order of a WKV mixer's operands and projections
 
 
+def expands(m: LatentAttentionConfig) -> bool:
+    """whether lp_latent_attend_expanded has kernels for these heads"""
+    return m.dim == 128 and m.vdim == 128 and m.rot_dim == 64 and m.kv_rank % 8 == 0
+
+
 def _pad_rows(t: torch.Tensor, n: int) -> torch.Tensor:
     """zero rows up to n (a projection of the same operand as its neighbours whose last columns nobody reads)"""
     return t if t.shape[0] >= n else torch.cat([t, torch.zeros(n - t.shape[0], t.shape[1], dtype=t.dtype, device=t.device)], 0)
@@ -561,6 +570,9 @@ class SeqLMWeights:
                     uk = w(i, pfx + "uk", (m.heads * m.dim, m.kv_rank))
                     mw["w_ukT"] = mat(uk.reshape(m.heads, m.dim, m.kv_rank).transpose(1, 2))       # [heads][kv_rank, dim]
                     mw["w_uv"] = mat(w(i, pfx + "uv", (m.heads * m.vdim, m.kv_rank)))                 # [heads][vdim, kv_rank]
+                    if expands(m) and dev.type == "cuda":      # prompts: both weights as rows, keys then values
+                        mw["w_kv"] = torch.cat([mat(uk), mw["w_uv"]], 0)
+                        mw["w_uv"] = mw["w_kv"][m.heads * m.dim:]
                     mw["w_o"] = mat(w(i, pfx + "o", (D, m.heads * m.vdim)))
                 return mw
 
@@ -694,6 +706,7 @@ class _Batch:
         self.decode = all(ln == 1 for ln in lens)
         self.longest_chunk = min(max(lens), _lib.RETENTION_CHUNK)
         pos0 = np.fromiter([s.length for s in seqs], np.int32, n)
+        self.starts = pos0
         slot = np.fromiter([s.slot for s in seqs], np.int32, n)
         if self.decode:      # one row a request: every per-row table is a per-request one
             row0 = np.arange(n + 1, dtype=np.int32)
@@ -1089,6 +1102,10 @@ class SeqLMEngine:
                             page_table=_lib.ptr(b.page_table), max_pages=b.max_pages, window=m.window or 0, scale=m.scale,
                             sink=_lib.ptr(lw.get("sink")), gate=_lib.ptr(head_gate), ldg=qd.stride(0) if head_gate is not None else 0)
         self._check(self.L.lp_latent_prep(C.byref(d), b.R, _lib.ptr(b.row_seq), _lib.ptr(b.row_pos), self._stream()), "lp_latent_prep")
+        if "w_kv" in lw and not b.decode and b.R > _lib.LATENT_SPLIT_ROWS and q.stride(0) % 4 == 0 and hasattr(self.L, "lp_latent_attend_expanded"):
+            tiles = sum(-(-ln // 128) for ln in b.lens)
+            if tiles <= EXPAND_TILES or b.R >= EXPAND_TILE_ROWS * tiles:
+                return self.linear(self._latent_expanded(m, lw, d, b, tiles, out_gate), lw["w_o"], F32, into=into)
         q_abs = self._empty((b.R, m.heads * m.kv_rank), F32)
         self.linear_heads(q, per, lw["w_ukT"], q_abs, m.kv_rank)
         lat = self._empty((b.R, m.heads * m.kv_rank), self.act)
@@ -1103,6 +1120,19 @@ class SeqLMEngine:
         o = self._empty((b.R, m.heads * m.vdim), self.act)
         self.linear_heads(lat, m.kv_rank, lw["w_uv"].view(m.heads, m.vdim, m.kv_rank), o, m.vdim, gate=out_gate)
         return self.linear(o, lw["w_o"], F32, into=into)
+
+    def _latent_expanded(self, m: LatentAttentionConfig, lw, d, b: _Batch, tiles: int, out_gate) -> torch.Tensor:
+        """rows of prompts [R, heads * vdim]: every head's keys and values are made from the visible latents"""
+        keys = sum(int(p) + ln - (max(0, int(p) - m.window + 1) if m.window else 0) for p, ln in zip(b.starts, b.lens))
+        o = self._empty((b.R, m.heads * m.vdim), self.act)
+        nbytes = int(self.L.lp_latent_expanded_workspace_bytes(b.R, m.heads, m.dim, m.rot_dim, m.kv_rank, keys))
+        ws = self._empty((nbytes,), torch.uint8)
+        w = lw["w_kv"]
+        rc = self.L.lp_latent_attend_expanded(C.byref(d), b.R, b.n, _lib.ptr(b.seq_row0), _lib.ptr(b.seq_pos0), tiles, keys, _lib.ptr(w), w.stride(0),
+                                              _lib.ptr(out_gate), out_gate.stride(0) if out_gate is not None else 0, _lib.ptr(o), o.stride(0),
+                                              int(o.dtype == F32), _lib.ptr(ws), nbytes, self._stream())
+        self._check(rc, "lp_latent_attend_expanded")
+        return o
 
     def _window_attention(self, li, m: WindowAttentionConfig, lw, h: torch.Tensor, b: _Batch, into=None, proj=None) -> torch.Tensor:
         o = self._empty((b.R, m.heads * m.vdim), self.act)

@@ -1,0 +1,67 @@
+// Test infrastructure: runs the kernels of leopard_b200/csrc/lp_split32.cu on the CPU under tests/emu/tc_emu.h.
+#define LP_EMULATE 1
+#include "../../leopard_b200/csrc/lp_split32.cu"
+
+using namespace lp;
+
+static CUtensorMap tmap3(const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t ld, uint64_t plane, uint32_t rows) {
+  CUtensorMap m;
+  m.base = reinterpret_cast<const uint8_t*>(base);
+  m.dims[0] = d0; m.dims[1] = d1; m.dims[2] = d2;
+  m.strides[0] = ld * 2; m.strides[1] = plane * 2;
+  m.box[0] = 64; m.box[1] = rows; m.box[2] = 1;
+  return m;
+}
+
+extern "C" void emu_split_rows(const float* src, long long ld, int M, int K, void* dst, long long ldd, long long plane) {
+  emu::launch(dim3((unsigned)(((long long)M * (K / 8) + 255) / 256)), dim3(256), [&] { split_rows_kernel(src, ld, M, K, (bf16*)dst, ldd, plane); });
+}
+
+extern "C" void emu_latent_gather(int n_seqs, int window, const int* row0, const int* pos0, int n_keys, const float* cache, int page_size,
+                                  const int* table, int max_pages, int width, void* dst, long long plane) {
+  Seqs32 q = {n_seqs, window, row0, pos0};
+  emu::launch(dim3((unsigned)(((long long)n_keys * (width / 8) + 255) / 256)), dim3(256),
+              [&] { latent_gather_kernel(q, n_keys, cache, page_size, table, max_pages, width, (bf16*)dst, plane); });
+}
+
+template <int BN>
+static void run_gemm(Gemm32Args& a, int ctas) {
+  a.n_tiles_m = (a.M + 127) / 128;
+  a.n_tiles_n = (a.N + BN - 1) / BN;
+  const CUtensorMap ta = tmap3(a.A, a.K, a.M, 3, a.lda, a.a_plane, 128), tw = tmap3(a.W, a.K, a.N, 1, a.ldw, 0, BN);
+  emu::g_block_hook = [] { emu_tc::reset(); };
+  emu::launch(dim3(ctas), dim3(G32_THREADS), [&] { gemm32_kernel<BN>(ta, tw, a); });
+  emu::g_block_hook = nullptr;
+}
+
+extern "C" void emu_gemm_split(const void* A, long long lda, long long a_plane, const void* W, long long ldw, void* C, long long ldc, long long c_plane,
+                               int out, int M, int N, int K, const float* bias, int bn, int ctas) {
+  Gemm32Args a = {};
+  a.M = M; a.N = N; a.K = K; a.bias = bias; a.C = C; a.ldc = ldc; a.c_plane = c_plane; a.out = out;
+  a.A = (const bf16*)A; a.lda = lda; a.a_plane = a_plane; a.W = (const bf16*)W; a.ldw = ldw;
+  if (bn == 256) run_gemm<256>(a, ctas);
+  else run_gemm<128>(a, ctas);
+}
+
+// q planes [3][R][heads * DQ], k and v planes [3][n_keys][heads * 128], kr planes [3][n_keys][64] or null
+extern "C" void emu_attn32(const void* q, const void* k, const void* kr, const void* v, int R, int heads, int n_seqs, int window, const int* row0,
+                           const int* pos0, int n_tiles, int n_keys, float scale, const float* sink, const float* gate, const float* out_gate, void* out,
+                           int out_fp32) {
+  const int dq = kr != nullptr ? 192 : 128;
+  Attn32Args a = {};
+  a.seqs = {n_seqs, window, row0, pos0};
+  a.heads = heads; a.scale = scale; a.sink = sink; a.gate = gate; a.ldg = heads; a.out_gate = out_gate; a.ldog = heads * 128;
+  a.out = out; a.ldo = heads * 128; a.out_fp32 = out_fp32;
+  a.q = (const bf16*)q; a.k = (const bf16*)k; a.kr = (const bf16*)kr; a.v = (const bf16*)v;
+  a.ldq = heads * dq; a.ldk = heads * 128; a.ldkr = 64;
+  a.q_plane = (long long)R * a.ldq; a.k_plane = (long long)n_keys * a.ldk; a.kr_plane = (long long)n_keys * 64;
+  const CUtensorMap tq = tmap3(q, a.ldq, R, 3, a.ldq, a.q_plane, 128), tk = tmap3(k, a.ldk, n_keys, 3, a.ldk, a.k_plane, 128);
+  const CUtensorMap tv = tmap3(v, a.ldk, n_keys, 3, a.ldk, a.k_plane, 64);
+  const CUtensorMap tr = kr != nullptr ? tmap3(kr, 64, n_keys, 3, 64, a.kr_plane, 128) : tk;
+  emu::g_block_hook = [] { emu_tc::reset(); };
+  emu::launch(dim3(heads, n_tiles), dim3(A32_THREADS), [&] {
+    if (kr != nullptr) attn32_kernel<1>(tq, tk, tr, tv, a);
+    else attn32_kernel<0>(tq, tk, tr, tv, a);
+  });
+  emu::g_block_hook = nullptr;
+}

@@ -1,0 +1,192 @@
+"""The SOURCE of leopard_b200/csrc/lp_split32.cu executed on the CPU (tests/emu/tc_emu.h): fp32 operands as three planes of bf16 terms, the
+product and the attention kernel on them, against float64.  Errors are those of fp32 sums: the terms add up to their number exactly, so a
+product of K terms differs from float64 by at most K roundings of 2^-24 of the sum of magnitudes, in practice far less."""
+import ctypes as C
+import math
+import subprocess
+from pathlib import Path
+
+import pytest
+import torch
+
+ROOT = Path(__file__).resolve().parents[1]
+F32, BF, F64 = torch.float32, torch.bfloat16, torch.float64
+
+
+@pytest.fixture(scope="module")
+def emu(tmp_path_factory):
+    out = tmp_path_factory.mktemp("emu_split32")
+    common = (ROOT / "leopard_b200/csrc/lp_common.cuh").read_text()
+    a = common.rindex("// ----", 0, common.index("// UMMA descriptors"))
+    (out / "emu_helpers.inc").write_text("namespace lp {\n" + common[a:common.rindex("}  // namespace lp")] + "\n}\n")
+    lib = out / "libsplit32.so"
+    r = subprocess.run(["g++", "-std=c++20", "-O2", "-pthread", "-shared", "-fPIC", "-I", str(out), "-I", str(ROOT / "tests/emu"),
+                        str(ROOT / "tests/emu/split32_emu.cpp"), "-o", str(lib)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-3000:]
+    return C.CDLL(str(lib))
+
+
+def P(t):
+    return C.c_void_p(t.data_ptr() if t is not None else None)
+
+
+def LL(n):
+    return C.c_longlong(n)
+
+
+def planes(emu, x):
+    """[3][rows][cols] of fp32 [rows, cols]"""
+    x = x.contiguous()
+    p = torch.empty((3, *x.shape), dtype=BF)
+    emu.emu_split_rows(P(x), LL(x.shape[1]), x.shape[0], x.shape[1], P(p), LL(x.shape[1]), LL(x.numel()))
+    return p
+
+
+def test_terms_add_up_exactly(emu):
+    g = torch.Generator().manual_seed(1)
+    x = torch.randn((37, 64), generator=g) * torch.exp(torch.randn((37, 64), generator=g) * 8)
+    x[0, :6] = torch.tensor([float("inf"), -float("inf"), float("nan"), 0.0, -0.0, 3.4028e38])
+    p = planes(emu, x).double()
+    total = p[0] + p[1] + p[2]
+    fin = torch.isfinite(x)
+    assert torch.equal(total[fin], x.double()[fin])
+    assert torch.equal(total[0, :2].float(), x[0, :2]) and bool(torch.isnan(total[0, 2]))
+
+
+@pytest.mark.parametrize("M,N,K,bn,ctas,out", [(130, 136, 72, 128, 2, 1), (40, 264, 200, 256, 1, 1), (128, 128, 64, 128, 1, 0), (257, 128, 328, 128, 3, 2),
+                                               (100, 392, 136, 256, 2, 2)])
+def test_product_of_three_planes(emu, M, N, K, bn, ctas, out):
+    g = torch.Generator().manual_seed(M + N)
+    x, w, bias = torch.randn((M, K), generator=g), torch.randn((N, K), generator=g).to(BF), torch.randn(N, generator=g)
+    p = planes(emu, x)
+    c = torch.full({0: (M, N), 1: (M, N), 2: (3, M, N)}[out], float("nan"), dtype=F32 if out == 1 else BF)
+    emu.emu_gemm_split(P(p), LL(K), LL(M * K), P(w), LL(K), P(c), LL(N), LL(M * N), out, M, N, K, P(bias), bn, ctas)
+    want = x.double() @ w.double().T + bias.double()
+    got = c.double().sum(0) if out == 2 else c.double()
+    assert float((got - want).norm() / want.norm()) < (4e-3 if out == 0 else 5e-7)
+
+
+def test_product_with_infinite_weight(emu):
+    """as fp32 multiply-adds: an infinite weight gives infinities, zero times it NaN"""
+    x, w = torch.randn((5, 64), generator=torch.Generator().manual_seed(3)), torch.ones((128, 64)).to(BF)
+    x[1, 7] = 0.0
+    w[9, 7] = float("inf")
+    p, c = planes(emu, x), torch.zeros((5, 128))
+    emu.emu_gemm_split(P(p), LL(64), LL(5 * 64), P(w), LL(64), P(c), LL(128), LL(0), 1, 5, 128, 64, P(None), 128, 1)
+    for r in range(5):
+        assert bool(torch.isnan(c[r, 9])) if r == 1 else float(c[r, 9]) == math.copysign(math.inf, float(x[r, 7]))
+    assert bool(torch.isfinite(c[:, :9]).all()) and bool(torch.isfinite(c[:, 10:]).all())
+
+
+def reference(q, k, kr, v, lens, pos0, window, scale, sink, gate, out_gate):
+    """float64; keys and values lie request by request from its first visible position on"""
+    R, H = q.shape[0], v.shape[1] // 128
+    dq = q.shape[1] // H
+    out, r, base = torch.zeros((R, H * 128), dtype=F64), 0, 0
+    for n, p0 in zip(lens, pos0):
+        lo = max(0, p0 - window + 1) if window else 0
+        for i in range(n):
+            pos = p0 + i
+            a, b = base + (max(lo, pos - window + 1) if window else lo) - lo, base + pos - lo + 1
+            for h in range(H):
+                kk = k[a:b, h * 128:(h + 1) * 128].double()
+                if kr is not None:
+                    kk = torch.cat([kk, kr[a:b].double()], 1)
+                s = kk @ q[r, h * dq:(h + 1) * dq].double() * scale
+                top = max(float(s.max()), float(sink[h]) if sink is not None else -math.inf)
+                e = torch.exp(s - top)
+                den = e.sum() + (math.exp(float(sink[h]) - top) if sink is not None else 0.0)
+                o = e @ v[a:b, h * 128:(h + 1) * 128].double() / den
+                if gate is not None:
+                    o = o * torch.sigmoid(gate[r, h].double())
+                out[r, h * 128:(h + 1) * 128] = o
+            r += 1
+        base += p0 + n - lo
+    return out * torch.sigmoid(out_gate.double()) if out_gate is not None else out
+
+
+@pytest.mark.parametrize("lens,pos0,window,rot,opts", [([130], [0], 0, True, ""), ([40, 129], [300, 0], 100, True, "sink"), ([257], [70], 150, False, "gates"),
+                                                       ([3, 1, 20], [0, 500, 127], 0, True, "")])
+def test_attention_of_three_planes(emu, lens, pos0, window, rot, opts):
+    H, R, dq = 2, sum(lens), 192 if rot else 128
+    g = torch.Generator().manual_seed(R)
+    n_keys = sum(p + n - (max(0, p - window + 1) if window else 0) for n, p in zip(lens, pos0))
+    q, k = 2 * torch.randn((R, H * dq), generator=g), torch.randn((n_keys, H * 128), generator=g)
+    kr, v = torch.randn((n_keys, 64), generator=g) if rot else None, torch.randn((n_keys, H * 128), generator=g)
+    sink = torch.randn(H, generator=g) if opts == "sink" else None
+    gate, og = (torch.randn((R, H), generator=g), torch.randn((R, H * 128), generator=g)) if opts == "gates" else (None, None)
+    row0 = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32)
+    p0 = torch.tensor(pos0, dtype=torch.int32)
+    out = torch.full((R, H * 128), float("nan"))
+    tiles = sum(-(-n // 128) for n in lens)
+
+    def run():
+        p = [planes(emu, x) if x is not None else None for x in (q, k, kr, v)]
+        emu.emu_attn32(*[P(x) for x in p], R, H, len(lens), window, P(row0), P(p0), tiles, n_keys, C.c_float(dq ** -0.5), P(sink), P(gate), P(og), P(out), 1)
+    run()
+    want = reference(q, k, kr, v, lens, pos0, window, dq ** -0.5, sink, gate, og)
+    assert float((out.double() - want).norm() / want.norm()) < 1e-6
+    if opts == "sink":      # a value that is not finite reaches only the rows that see it
+        v[n_keys - 1, 3] = float("inf")
+        run()
+        assert not bool(torch.isfinite(out[R - 1, 3])) and bool(torch.isfinite(out[: R - 1]).all()) and bool(torch.isfinite(out[R - 1, 4:128]).all())
+
+
+def test_gather_of_cache_rows(emu):
+    g = torch.Generator().manual_seed(4)
+    width, page, lens, pos0, window = 24, 4, [3, 5], [6, 0], 4
+    cache = torch.randn((8 * page, width), generator=g)
+    table = torch.tensor([[5, 1, 7], [2, 0, -1]], dtype=torch.int32)
+    row0, p0 = torch.tensor([0, 3, 8], dtype=torch.int32), torch.tensor(pos0, dtype=torch.int32)
+    rows = [(s, p) for s, (n, a) in enumerate(zip(lens, pos0)) for p in range(max(0, a - window + 1), a + n)]
+    got = torch.zeros((3, len(rows), width), dtype=BF)
+    emu.emu_latent_gather(2, window, P(row0), P(p0), len(rows), P(cache), page, P(table), 3, width, P(got), LL(len(rows) * width))
+    want = torch.stack([cache[int(table[s, p // page]) * page + p % page] for s, p in rows])
+    assert torch.equal(got.double().sum(0), want.double())
+
+
+# ------------------------------------------------------------------------------------------------------------------- on a GPU, through the engine
+def latent_engine(dtype, heads, rank, window, **options):
+    from leopard_b200 import _lib
+    from leopard_b200.seqlm import LatentAttentionConfig, LayerConfig, RotaryConfig, SeqLMConfig, SeqLMEngine, SeqLMWeights
+    D, O = 256, heads * 128
+    m = LatentAttentionConfig(heads=heads, dim=128, rot_dim=64, vdim=128, kv_rank=rank, scale=192 ** -0.5, rot=RotaryConfig(dims=64, base=1e4),
+                              window=window, **options)
+    cfg = SeqLMConfig(architecture="latent", vocab=64, width=D, eps=1e-6, layers=(LayerConfig(mixer=m, ff=None),), norm="pre")
+    shapes = {"embed": (64, D), "head": (64, D), "final.norm": (D,), "norm1": (D,), "mix.q": (heads * 192, D), "mix.dkv": (rank + 64, D),
+              "mix.dkv.norm": (rank,), "mix.uk": (heads * 128, rank), "mix.uv": (O, rank), "mix.o": (D, O), "mix.sink": (heads,),
+              "mix.g": (heads if options.get("head_gate") else O, D)}
+
+    def get(name):
+        shape = shapes[name]
+        x = torch.randn(shape, generator=torch.Generator().manual_seed(sum(map(ord, name))))
+        return x * (2 * shape[1] ** -0.5 if len(shape) == 2 else 0.1)
+    w = SeqLMWeights(cfg, get, lambda layer, key: key, "cuda")
+    return SeqLMEngine(cfg, w, dtype=dtype, max_tokens=2048, page_size=16, max_seqs=4, lib=_lib.stream32_lib()), m
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,heads,rank,window,options,lens", [
+    ("float32", 3, 136, None, {}, [(17, 130), (1, 300)]), ("float32", 2, 64, 100, {"sink": True}, [(129, 257), (40, 5)]),
+    ("float32", 2, 72, 128, {"out_gate": True}, [(256, 1), (128, 33)]), ("bfloat16", 4, 128, 50, {"head_gate": True}, [(300, 64), (20, 500)])])
+def test_expanded_latent_attention_in_the_engine(dtype, heads, rank, window, options, lens):
+    """prompts, and portions that continue them, as the general path computes them (fp32: both within a few roundings of float64)"""
+    from leopard_b200.seqlm import StepEntry, _Batch
+    eng, m = latent_engine(dtype, heads, rank, window, **options)
+    lw, kv = eng.w.layers[0], None
+    calls = []
+    inner = eng._latent_expanded
+    eng._latent_expanded = lambda *a: calls.append(1) or inner(*a)
+    for a, b in lens:
+        batch = _Batch(eng, [StepEntry("a", [1] * a, []), StepEntry("b", [2] * b, [])])
+        h = torch.randn((a + b, 256), device="cuda", generator=torch.Generator("cuda").manual_seed(a)).to(eng.act)
+        n = len(calls)
+        got = eng._latent(0, m, lw, h, batch).double()
+        assert len(calls) == n + 1
+        kv = lw.pop("w_kv")
+        want = eng._latent(0, m, lw, h, batch).double()
+        lw["w_kv"] = kv
+        assert float((got - want).norm() / want.norm()) < (3e-6 if dtype == "float32" else 1e-2)
+        for s, ln in zip(batch.seqs, batch.lens):
+            eng.cache.advance(s, ln)
+
