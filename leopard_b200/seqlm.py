@@ -37,6 +37,10 @@ TENSOR_CORE_MIN_ROWS = 64
 # whose sums are cut off: 2.1e-6 of the result at K = 2048, 9.1e-6 at 8192, against 2.3e-7 streamed and 3.9e-7, 9.6e-7 of fp32 multiply-adds.  So
 # it has the products of 64 rows and more, as large prompts always had; at 64 rows only those above the crossing.
 STREAM_MAX_OUTPUTS = 170_000
+# fp32 rows of more than 64 go to the tcgen05 product of three bf16 terms, a pass for the terms included (us, lp_linear and this one): 65 rows, K = 64,
+# 128 columns 8.5, 6.5; K = 1024, 4096 columns 36, 21; 4000 rows, K = 1024, 4096 columns 388, 105.  Up to 64 rows lp_linear streams the weights: 48 rows,
+# K = 128, 6.7, 7.3, K = 1024 12.5, 20.  (K of less than a k block and columns of less than a tile were not measured: they stay.)
+SPLIT_MIN_ROWS, SPLIT_MIN_K = 65, 64
 # Rows of prompts expand the visible latents into every head's keys and values (lp_latent_attend_expanded), unless many requests bring a few rows each:
 # its tiles are 128 rows of one request.  A layer of width 1024 with 8 heads (us, lp_latent_attend_tiles and this one): one request of 20 rows 64, 45, of
 # 500 297, 85; 32 requests of 12 rows 92, 81; 64 of 12 97, 120, of 24 132, 126; width 2048, 16 heads: 4096 rows 6,490, 530; 64 requests of 12 rows 225, 205.
@@ -884,6 +888,7 @@ class SeqLMEngine:
         self.tile_rows = int(self.L.lp_linear_tile_rows())
         # large bf16 products of the serving precision go to the tcgen05 GEMM when the library has it (the native ones do)
         self.tensor_core_rows = TENSOR_CORE_MIN_ROWS if dtype == "bfloat16" and hasattr(self.L, "lp_gemm_bf16") else None
+        self.split_rows = SPLIT_MIN_ROWS if hasattr(self.L, "lp_gemm_split") and self.device.type == "cuda" else None
         self.tap: Optional[Callable[[int, torch.Tensor], None]] = None   # called with (layer, residual stream) after every layer
         # decode steps are launch-bound: a batch layout (requests, page-table width) that comes back is captured into a CUDA graph on
         # its second appearance and replayed from then on; only the index tables change between replays (LEOPARD_DECODE_GRAPH=0: off)
@@ -915,6 +920,21 @@ class SeqLMEngine:
         return (a.dtype == BF16 and N >= 128 and K >= 64 and N % 8 == 0 and K % 8 == 0 and a.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
                 and a.stride(1) == 1 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
+    def _on_split(self, a: torch.Tensor, w: torch.Tensor) -> bool:
+        """Whether fp32 rows go to the tcgen05 product of three bf16 terms"""
+        (M, K), N = a.shape, w.shape[0]
+        return (self.split_rows is not None and M >= self.split_rows and a.dtype == F32 and N >= 128 and K >= SPLIT_MIN_K and N % 8 == 0 and K % 8 == 0
+                and a.stride(0) % 4 == 0 and w.stride(0) % 8 == 0 and a.stride(1) == 1 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+    def _split_product(self, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias) -> None:
+        M, K = a.shape
+        terms = self._empty((3, M, K), BF16)
+        rc = self.L.lp_split_rows(_lib.ptr(a), a.stride(0), M, K, _lib.ptr(terms), K, M * K, self._stream())
+        self._check(rc, "lp_split_rows")
+        rc = self.L.lp_gemm_split(_lib.ptr(terms), K, M * K, _lib.ptr(w), w.stride(0), _lib.ptr(out), out.stride(0), 0,
+                                  _lib.GEMM_SPLIT_F32 if out.dtype == F32 else _lib.GEMM_SPLIT_BF16, M, w.shape[0], K, _lib.ptr(bias), self._stream())
+        self._check(rc, "lp_gemm_split")
+
     def linear(self, a: torch.Tensor, w: torch.Tensor, out_dtype, epi=_lib.EPI_NONE, epi_a=0.0, epi_b=0.0, out=None, into=None, bias=None,
                row_scale=None):
         """out[M, N'] = epi(row_scale[m] * (a[M, K] @ w[N, K].T) + bias[N]) (bias, row_scale: fp32 device vectors or None).  With
@@ -923,7 +943,8 @@ class SeqLMEngine:
         N = w.shape[0]
         n_out = N // 2 if epi in _lib.GATED_EPIS else N
         # a row scale reaches the tensor-core path only through the activation kernel that follows the product
-        tc = self._on_gemm(a, w) and (row_scale is None or (epi != _lib.EPI_NONE and bias is None))
+        split = self._on_split(a, w)
+        tc = (split or self._on_gemm(a, w)) and (row_scale is None or (epi != _lib.EPI_NONE and bias is None))
         if into is not None:
             x, mult = into[0], into[1]
             gate = into[2] if len(into) > 2 else None
@@ -946,9 +967,12 @@ class SeqLMEngine:
             out = self._empty((M, n_out), out_dtype)
         if tc and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0:
             raw = out if epi == _lib.EPI_NONE else self._empty((M, N), F32)
-            rc = self.L.lp_gemm_bf16(_lib.ptr(a), a.stride(0), _lib.ptr(w), w.stride(0), _lib.ptr(raw), raw.stride(0), M, N, K, _lib.ptr(bias),
-                                     None, 0, 0, _lib.ACT_NONE, int(raw.dtype == F32), 0, self._stream())
-            self._check(rc, "lp_gemm_bf16")
+            if split:
+                self._split_product(a, w, raw, bias)
+            else:
+                rc = self.L.lp_gemm_bf16(_lib.ptr(a), a.stride(0), _lib.ptr(w), w.stride(0), _lib.ptr(raw), raw.stride(0), M, N, K, _lib.ptr(bias),
+                                         None, 0, 0, _lib.ACT_NONE, int(raw.dtype == F32), 0, self._stream())
+                self._check(rc, "lp_gemm_bf16")
             if epi != _lib.EPI_NONE:
                 rc = self.L.lp_glu_scaled_f32(_lib.ptr(raw), raw.stride(0), 1, _lib.ptr(out), out.stride(0), int(out.dtype == F32), M, n_out,
                                               epi, epi_a, epi_b, _lib.ptr(row_scale), self._stream())

@@ -190,3 +190,25 @@ def test_expanded_latent_attention_in_the_engine(dtype, heads, rank, window, opt
         for s, ln in zip(batch.seqs, batch.lens):
             eng.cache.advance(s, ln)
 
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(65, 128, 64), (129, 264, 72), (300, 1000, 200), (257, 4096, 136)])
+def test_products_of_fp32_rows_in_the_engine(M, N, K):
+    """the split product and its epilogues are no further from float64 than lp_linear's"""
+    from leopard_b200 import _lib
+    eng, _ = latent_engine("float32", 2, 64, None)
+    g = torch.Generator("cuda").manual_seed(M)
+    a, w = torch.randn((M, K + 4), device="cuda", generator=g)[:, :K], torch.randn((N, K), device="cuda", generator=g).to(BF)
+    bias, x = torch.randn(N, device="cuda", generator=g), torch.randn((M, N), device="cuda", generator=g)
+    want = a.double() @ w.double().T + bias.double()
+    for epi, ref in ((_lib.EPI_NONE, want), (_lib.EPI_RELU2, want.clamp_min(0) ** 2)):
+        err = []
+        for rows in (eng.split_rows, None):
+            saved, eng.split_rows = eng.split_rows, rows
+            assert eng._on_split(a, w) == (rows is not None)
+            y = eng.linear(a, w, F32, epi, bias=bias).double()
+            z = eng.linear(a, w, F32, epi, bias=bias, into=(x.clone(), 0.5)).double()
+            eng.split_rows = saved
+            err.append(float((y - ref).norm() / ref.norm()))
+            assert float((z - (x.double() + 0.5 * ref)).norm() / z.norm()) < 1e-6
+        assert err[0] < max(err[1] * 1.2, 2e-7)
