@@ -317,8 +317,15 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
   }
 }
 
-// decode: one new row per request.  Threads own state columns; with vdim < blockDim several thread groups split the dim rows.
-constexpr int RET_DEC_THREADS = 256;
+// decode: one new row per request.  Threads own V neighbouring state columns (V = 4 where rows and slots are whole 16-byte pieces), groups of them split
+// the dim rows, eight of which are in flight at a time: with a column a thread and a row read after the one before was written, the chain of
+// loads took 16 us (8 requests of 16 heads of 128 x 128) and 37 us (64 of 8), whose bytes take 2.6 and 10.
+constexpr int RET_DEC_THREADS = 256, RET_DEC_BATCH = 8;
+template <int V> struct RetVec;
+template <> struct RetVec<1> { float v[1]; };
+template <> struct alignas(16) RetVec<4> { float v[4]; };
+template <int V> __host__ __device__ inline int ret_dec_groups(int vdim) { return vdim / V >= RET_DEC_THREADS ? 1 : RET_DEC_THREADS / (vdim / V); }
+template <int V>
 __global__ void __launch_bounds__(RET_DEC_THREADS)
 retention_decode_kernel(RetArgs a, const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0, const int* __restrict__ seq_slot) {
   extern __shared__ float dyn_smem[];
@@ -340,21 +347,40 @@ retention_decode_kernel(RetArgs a, const int* __restrict__ seq_row0, const int* 
   const float dec = a.decay[h];
   const bool fresh = pos == 0;
   float* st = a.state + (long long)seq_slot[s] * a.slot_stride + (long long)h * a.dim * a.vdim;
-  const int groups = a.vdim >= (int)blockDim.x ? 1 : (int)blockDim.x / a.vdim;
-  const int g = tid / a.vdim;
-  const int per = (a.dim + groups - 1) / groups;
+  const int groups = ret_dec_groups<V>(a.vdim);
+  const int cols = a.vdim / V, g = tid / cols, per = (a.dim + groups - 1) / groups;
   if (g < groups) {
     const int d0 = g * per, d1 = min(a.dim, d0 + per);
-    for (int y = tid % a.vdim; y < a.vdim; y += blockDim.x) {
-      float acc = 0.f;
-#pragma unroll 8
-      for (int d = d0; d < d1; ++d) {
-        const float old = fresh ? 0.f : st[(long long)d * a.vdim + y];
-        const float S = fmaf(dec, old, ks[d] * vv[y]);
-        st[(long long)d * a.vdim + y] = S;
-        acc = fmaf(S, qs[d], acc);
+    for (int y = tid % cols * V; y < a.vdim; y += RET_DEC_THREADS * V) {
+      float acc[V], v[V];
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        acc[k] = 0.f;
+        v[k] = vv[y + k];
       }
-      part[g * a.vdim + y] = acc;
+      for (int b = d0; b < d1; b += RET_DEC_BATCH) {      // a batch of rows is read before the first of them is written
+        RetVec<V> old[RET_DEC_BATCH];
+#pragma unroll
+        for (int i = 0; i < RET_DEC_BATCH; ++i)
+          if (b + i < d1 && !fresh) old[i] = *reinterpret_cast<const RetVec<V>*>(st + (long long)(b + i) * a.vdim + y);
+          else
+#pragma unroll
+            for (int k = 0; k < V; ++k) old[i].v[k] = 0.f;
+#pragma unroll
+        for (int i = 0; i < RET_DEC_BATCH; ++i) {
+          if (b + i < d1) {
+            const float kd = ks[b + i], qd = qs[b + i];
+#pragma unroll
+            for (int k = 0; k < V; ++k) {
+              old[i].v[k] = fmaf(dec, old[i].v[k], kd * v[k]);
+              acc[k] = fmaf(old[i].v[k], qd, acc[k]);
+            }
+            *reinterpret_cast<RetVec<V>*>(st + (long long)(b + i) * a.vdim + y) = old[i];
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < V; ++k) part[g * a.vdim + y + k] = acc[k];
     }
   }
   __syncthreads();
@@ -444,17 +470,23 @@ latent_prep_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int*
   }
 }
 
-// One CTA per (row, head): its warps take every LAT_WARPS-th visible key with an online softmax of their own, then the partial
-// (maximum, denominator, weighted sum) triples are merged.  NR = ceil(kv_rank / 32) accumulators per lane.
-constexpr int LAT_WARPS = 16;
+// One CTA per (row, head): its W warps take every W-th visible key with an online softmax of their own, then the partial (maximum,
+// denominator, weighted sum) triples are merged.  A lane holds pieces of V channels, every 32nd (NP pieces of the latent; V = 4 where cache rows are whole
+// 16-byte pieces), and LAT_KEYS keys are in flight at a time: their score reductions overlap, one rescale of the running sums serves them all.
+// With a channel a load and two keys in flight 8 rows of 16 heads over 150 keys took 18.5 us, 64 rows of 8 heads over 40 keys (which had a warp a row and head) 34.
+constexpr int LAT_KEYS = 4;
 constexpr int LAT_SPLIT_MAX_RANK = 512;      // larger latents take the per-row kernel
 constexpr int LAT_MAX_RANK = 1024;
-template <int NR>
-__global__ void __launch_bounds__(LAT_WARPS * 32)
+template <int V> struct LatVec;
+template <> struct LatVec<1> { float v[1]; };
+template <> struct alignas(16) LatVec<4> { float v[4]; };
+template <int V, int NP, int W>
+__global__ void __launch_bounds__(W * 32)
 latent_attend_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos, const float* __restrict__ q_abs,
                      long long ldqa, void* __restrict__ out, long long ldo, int out_fp32) {
-  __shared__ float s_acc[LAT_WARPS][LAT_SPLIT_MAX_RANK];
-  __shared__ float s_mx[LAT_WARPS], s_den[LAT_WARPS];
+  __align__(16) __shared__ float s_acc[W][32 * V * NP];
+  __shared__ float s_mx[W], s_den[W];
+  constexpr int NR = V == 4 ? 1 : NP;      // pieces of the rotated part
   const int item = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (item >= R * a.heads) return;
@@ -462,57 +494,94 @@ latent_attend_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const in
   const int seq = row_seq[r], pos = row_pos[r];
   const float* qa = q_abs + (long long)r * ldqa + (long long)h * a.kv_rank;
   const float* qr = a.q + (long long)r * a.ldq + (long long)h * (a.dim + a.rot_dim) + a.dim;
-  float qv[NR], qrv[NR], acc[NR];
+  LatVec<V> qv[NP], qrv[NR], acc[NP];
 #pragma unroll
-  for (int i = 0; i < NR; ++i) {
-    const int c = lane + 32 * i;
-    qv[i] = c < a.kv_rank ? qa[c] : 0.f;
-    qrv[i] = c < a.rot_dim ? qr[c] : 0.f;      // rot_dim <= 32 * NR (checked by the host): lanes hold it strided as well
-    acc[i] = 0.f;
-  }
+  for (int i = 0; i < NP; ++i)
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      const int c = V * (lane + 32 * i) + k;
+      qv[i].v[k] = c < a.kv_rank ? qa[c] : 0.f;
+      acc[i].v[k] = 0.f;
+    }
+#pragma unroll
+  for (int i = 0; i < NR; ++i)
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      const int c = V * (lane + 32 * i) + k;
+      qrv[i].v[k] = c < a.rot_dim ? qr[c] : 0.f;      // rot_dim <= 32 V NR (checked by the host)
+    }
   const int lo = (a.window > 0 && pos - a.window + 1 > 0) ? pos - a.window + 1 : 0;
   // the sink is a key without a value whose score is sink_h as it stands: warp 0 starts from it
   const bool sunk = a.sink != nullptr && warp == 0;
   float mx = sunk ? a.sink[h] : -INFINITY, den = sunk ? 1.f : 0.f;
-  // two keys per turn: their score reductions overlap, one rescale of the running sums serves both
-  for (int j = lo + warp; j <= pos; j += 2 * LAT_WARPS) {
-    const bool two = j + LAT_WARPS <= pos;
-    const float* kv0 = lat_cache_row(a, seq, j);
-    const float* kv1 = two ? lat_cache_row(a, seq, j + LAT_WARPS) : kv0;
-    float cv0[NR], cv1[NR];
-    float sc0 = 0.f, sc1 = 0.f;
+  for (int j = lo + warp; j <= pos; j += LAT_KEYS * W) {
+    LatVec<V> cv[LAT_KEYS][NP];
+    float sc[LAT_KEYS];
+    const float* kv[LAT_KEYS];
 #pragma unroll
-    for (int i = 0; i < NR; ++i) {
-      const int c = lane + 32 * i;
-      cv0[i] = c < a.kv_rank ? kv0[c] : 0.f;
-      cv1[i] = c < a.kv_rank ? kv1[c] : 0.f;
-      sc0 = fmaf(qv[i], cv0[i], sc0);
-      sc1 = fmaf(qv[i], cv1[i], sc1);
-      if (c < a.rot_dim) {
-        sc0 = fmaf(qrv[i], kv0[a.kv_rank + c], sc0);
-        sc1 = fmaf(qrv[i], kv1[a.kv_rank + c], sc1);
+    for (int n = 0; n < LAT_KEYS; ++n) kv[n] = lat_cache_row(a, seq, j + n * W <= pos ? j + n * W : j);
+#pragma unroll
+    for (int n = 0; n < LAT_KEYS; ++n) {
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        const int c = V * (lane + 32 * i);
+        if (c < a.kv_rank) {
+          cv[n][i] = *reinterpret_cast<const LatVec<V>*>(kv[n] + c);
+        } else {
+#pragma unroll
+          for (int k = 0; k < V; ++k) cv[n][i].v[k] = 0.f;
+        }
       }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      sc0 += __shfl_xor_sync(0xffffffffu, sc0, o);
-      sc1 += __shfl_xor_sync(0xffffffffu, sc1, o);
-    }
-    sc0 *= a.scale;
-    sc1 = two ? sc1 * a.scale : -INFINITY;
-    const float mn = fmaxf(mx, fmaxf(sc0, sc1));
-    const float corr = expf(mx - mn);      // exp(-inf) = 0 on the first turn
-    const float p0 = expf(sc0 - mn), p1 = expf(sc1 - mn);
-    den = den * corr + p0 + p1;
+    for (int n = 0; n < LAT_KEYS; ++n) {
+      sc[n] = 0.f;
 #pragma unroll
-    for (int i = 0; i < NR; ++i) acc[i] = fmaf(p1, cv1[i], fmaf(p0, cv0[i], acc[i] * corr));
+      for (int i = 0; i < NR; ++i) {
+        const int c = V * (lane + 32 * i);
+        if (c < a.rot_dim) {
+          const LatVec<V> kr = *reinterpret_cast<const LatVec<V>*>(kv[n] + a.kv_rank + c);
+#pragma unroll
+          for (int k = 0; k < V; ++k) sc[n] = fmaf(qrv[i].v[k], kr.v[k], sc[n]);
+        }
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < LAT_KEYS; ++n)
+#pragma unroll
+      for (int i = 0; i < NP; ++i)
+#pragma unroll
+        for (int k = 0; k < V; ++k) sc[n] = fmaf(qv[i].v[k], cv[n][i].v[k], sc[n]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int n = 0; n < LAT_KEYS; ++n) sc[n] += __shfl_xor_sync(0xffffffffu, sc[n], o);
+    float mn = mx;
+#pragma unroll
+    for (int n = 0; n < LAT_KEYS; ++n) {
+      sc[n] = j + n * W <= pos ? sc[n] * a.scale : -INFINITY;
+      mn = fmaxf(mn, sc[n]);
+    }
+    const float corr = expf(mx - mn);      // exp(-inf) = 0 on the first turn
+    den *= corr;
+#pragma unroll
+    for (int i = 0; i < NP; ++i)
+#pragma unroll
+      for (int k = 0; k < V; ++k) acc[i].v[k] *= corr;
+#pragma unroll
+    for (int n = 0; n < LAT_KEYS; ++n) {
+      if (j + n * W > pos) break;
+      const float p = expf(sc[n] - mn);
+      den += p;
+#pragma unroll
+      for (int i = 0; i < NP; ++i)
+#pragma unroll
+        for (int k = 0; k < V; ++k) acc[i].v[k] = fmaf(p, cv[n][i].v[k], acc[i].v[k]);
+    }
     mx = mn;
   }
 #pragma unroll
-  for (int i = 0; i < NR; ++i) {
-    const int c = lane + 32 * i;
-    if (c < a.kv_rank) s_acc[warp][c] = acc[i];
-  }
+  for (int i = 0; i < NP; ++i) *reinterpret_cast<LatVec<V>*>(&s_acc[warp][V * (lane + 32 * i)]) = acc[i];
   if (lane == 0) {
     s_mx[warp] = mx;
     s_den[warp] = den;
@@ -520,10 +589,10 @@ latent_attend_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const in
   __syncthreads();
   float top = s_mx[0];
 #pragma unroll
-  for (int w = 1; w < LAT_WARPS; ++w) top = fmaxf(top, s_mx[w]);
-  float f[LAT_WARPS], total = 0.f;
+  for (int w = 1; w < W; ++w) top = fmaxf(top, s_mx[w]);
+  float f[W], total = 0.f;
 #pragma unroll
-  for (int w = 0; w < LAT_WARPS; ++w) {
+  for (int w = 0; w < W; ++w) {
     f[w] = s_den[w] > 0.f ? expf(s_mx[w] - top) : 0.f;      // a warp without keys contributes nothing
     total = fmaf(s_den[w], f[w], total);
   }
@@ -531,7 +600,7 @@ latent_attend_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const in
   for (int c = threadIdx.x; c < a.kv_rank; c += blockDim.x) {
     float v = 0.f;
 #pragma unroll
-    for (int w = 0; w < LAT_WARPS; ++w) v = fmaf(s_acc[w][c], f[w], v);
+    for (int w = 0; w < W; ++w) v = fmaf(s_acc[w][c], f[w], v);
     const long long o = (long long)r * ldo + (long long)h * a.kv_rank + c;
     if (out_fp32) reinterpret_cast<float*>(out)[o] = v * inv;
     else reinterpret_cast<bf16*>(out)[o] = __float2bfloat16(v * inv);
@@ -541,7 +610,7 @@ latent_attend_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const in
 // Many rows (prompts): one CTA per row and group of LAT_ROW_HEADS heads, one warp per head, every warp walks all visible keys.
 // The heads of a row read the same cache rows at about the same time, so the cache traffic of a row is paid once per CTA (L1), and
 // neighbouring rows overlap in all but one key (L2).
-constexpr int LAT_ROW_HEADS = 4;
+constexpr int LAT_ROW_HEADS = 4, LAT_SPLIT_ROWS = 128;
 template <int NR>
 __global__ void __launch_bounds__(LAT_ROW_HEADS * 32)
 latent_attend_rows_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos, const float* __restrict__ q_abs,
@@ -793,7 +862,7 @@ static cudaError_t ensure_smem(K kern, size_t bytes, size_t& have) {
   if (e == cudaSuccess) have = bytes;
   return e;
 }
-static size_t g_smem_chunk_state = 48 * 1024, g_smem_chunk_out = 48 * 1024, g_smem_ret_decode = 48 * 1024;
+static size_t g_smem_chunk_state = 48 * 1024, g_smem_chunk_out = 48 * 1024;
 
 static int fill_ret(RetArgs& a, const lp_retention_desc* d) {
   LP_REQUIRE(d != nullptr && d->qkvg != nullptr && d->decay != nullptr && d->state != nullptr && d->out != nullptr,
@@ -871,20 +940,26 @@ extern "C" int lp_retention_prefill(const lp_retention_desc* d, int n_seqs, int 
   return 0;
 }
 
+template <int V>
+static int launch_ret_decode(const RetArgs& a, int n_seqs, const int* seq_row0, const int* seq_pos0, const int* seq_slot, cudaStream_t stream) {
+  static size_t have = 48 * 1024;
+  const size_t smem = ((size_t)2 * a.dim + 2 * a.vdim + (size_t)ret_dec_groups<V>(a.vdim) * a.vdim) * sizeof(float);
+  LP_REQUIRE(smem <= 200 * 1024, "lp_retention_decode: dim=%d vdim=%d do not fit shared memory", a.dim, a.vdim);
+  LP_CHECK_CUDA(ensure_smem(retention_decode_kernel<V>, smem, have));
+  retention_decode_kernel<V><<<dim3(n_seqs, a.heads), RET_DEC_THREADS, smem, stream>>>(a, seq_row0, seq_pos0, seq_slot);
+  note_launch();
+  LP_CHECK_CUDA(cudaGetLastError());
+  return 0;
+}
+
 extern "C" int lp_retention_decode(const lp_retention_desc* d, int n_seqs, const int* seq_row0, const int* seq_pos0, const int* seq_slot,
                                    void* stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   RetArgs a;
   if (int rc = fill_ret(a, d)) return rc;
   if (n_seqs <= 0) return 0;
-  const int groups = d->vdim >= RET_DEC_THREADS ? 1 : RET_DEC_THREADS / d->vdim;
-  const size_t smem = ((size_t)2 * d->dim + 2 * d->vdim + (size_t)groups * d->vdim) * sizeof(float);
-  LP_REQUIRE(smem <= 200 * 1024, "lp_retention_decode: dim=%d vdim=%d do not fit shared memory", d->dim, d->vdim);
-  LP_CHECK_CUDA(ensure_smem(retention_decode_kernel, smem, g_smem_ret_decode));
-  retention_decode_kernel<<<dim3(n_seqs, d->heads), RET_DEC_THREADS, smem, stream>>>(a, seq_row0, seq_pos0, seq_slot);
-  note_launch();
-  LP_CHECK_CUDA(cudaGetLastError());
-  return 0;
+  const bool pieces = d->vdim % 4 == 0 && d->slot_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(d->state) & 15) == 0;
+  return pieces ? launch_ret_decode<4>(a, n_seqs, seq_row0, seq_pos0, seq_slot, stream) : launch_ret_decode<1>(a, n_seqs, seq_row0, seq_pos0, seq_slot, stream);
 }
 
 extern "C" int lp_latent_prep(const lp_latent_desc* d, int R, const int* row_seq, const int* row_pos, void* stream_) {
@@ -909,7 +984,7 @@ extern "C" int lp_latent_attend(const lp_latent_desc* d, int R, const int* row_s
              d->kv_rank, d->rot_dim, LAT_MAX_RANK);
   if (R <= 0) return 0;
   const int nr = ((d->kv_rank > d->rot_dim ? d->kv_rank : d->rot_dim) + 31) / 32;      // lanes hold both vectors strided by 32
-  if (R > LP_LATENT_SPLIT_ROWS || d->kv_rank > LAT_SPLIT_MAX_RANK) {      // prompts: a CTA per row, a warp per head
+  if (R > LAT_SPLIT_ROWS || d->kv_rank > LAT_SPLIT_MAX_RANK || d->rot_dim > LAT_SPLIT_MAX_RANK) {      // prompts: a CTA per row, a warp per head
     const dim3 grid(R, (d->heads + LAT_ROW_HEADS - 1) / LAT_ROW_HEADS);
     const int threads = (d->heads < LAT_ROW_HEADS ? d->heads : LAT_ROW_HEADS) * 32;
     if (nr <= 2) latent_attend_rows_kernel<2><<<grid, threads, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);
@@ -917,13 +992,24 @@ extern "C" int lp_latent_attend(const lp_latent_desc* d, int R, const int* row_s
     else if (nr <= 8) latent_attend_rows_kernel<8><<<grid, threads, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);
     else if (nr <= 16) latent_attend_rows_kernel<16><<<grid, threads, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);
     else latent_attend_rows_kernel<32><<<grid, threads, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);
-  } else {                             // few rows (decoding): a CTA per (row, head), its warps split the keys
-    const unsigned grid = (unsigned)((long long)R * d->heads);
-    if (nr <= 2) latent_attend_kernel<2><<<grid, LAT_WARPS * 32, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);
-    else if (nr <= 4) latent_attend_kernel<4><<<grid, LAT_WARPS * 32, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);
-    else if (nr <= 8) latent_attend_kernel<8><<<grid, LAT_WARPS * 32, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);
-    else if (nr <= 16) latent_attend_kernel<16><<<grid, LAT_WARPS * 32, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);
-    else latent_attend_kernel<32><<<grid, LAT_WARPS * 32, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);
+  } else {      // decoding: a CTA per (row, head), its warps split the keys
+    const long long ctas = (long long)R * d->heads;
+    const bool pieces = d->kv_rank % 4 == 0 && d->rot_dim % 4 == 0 && d->rot_dim <= 128 && (reinterpret_cast<uintptr_t>(d->cache) & 15) == 0;
+#define LP_LAT(V, NP)                                                                                                                       \
+  do {                                                                                                                                      \
+    if (ctas <= 2LL * sm_count()) latent_attend_kernel<V, NP, 16><<<(unsigned)ctas, 16 * 32, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);    \
+    else latent_attend_kernel<V, NP, 4><<<(unsigned)ctas, 4 * 32, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);     \
+  } while (0)
+    if (pieces) {
+      const int np = (d->kv_rank + 127) / 128;
+      if (np <= 1) LP_LAT(4, 1);
+      else if (np <= 2) LP_LAT(4, 2);
+      else LP_LAT(4, 4);
+    } else {
+      if (nr <= 4) LP_LAT(1, 4);
+      else LP_LAT(1, 16);
+    }
+#undef LP_LAT
   }
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
