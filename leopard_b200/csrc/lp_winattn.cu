@@ -297,8 +297,8 @@ window_attn_pool_kernel(WinArgs a, int n_seqs, const int* __restrict__ seq_row0,
   win_block_row(a, s, b)[c] = sum / (float)a.pool;
 }
 
-template <int QH, int NV, bool DIST>
-__global__ void __launch_bounds__(256)
+template <int QH, int NV, bool DIST, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 window_attn_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos, void* __restrict__ out, long long ldo,
                    int out_fp32) {
   extern __shared__ float dyn_smem[];
@@ -345,16 +345,19 @@ window_attn_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const int*
       // four lanes share a key: each reads every fourth 16-byte piece of the row, so one load instruction of the warp touches 8 rows
       // of 64 contiguous bytes instead of 32 rows; four passes cover the tile's 32 keys, the partial sums meet by two shuffles
       const int piece = lane & 3, kq = lane >> 2;
+      if (valid) my_row[lane] = win_visible_row(a, vis, seq, t);      // looked up once a key, a lane each
+      __syncwarp();
+#pragma unroll 1
       for (int i = 0; i < 4; ++i) {
         const int tk = t0 + i * 8 + kq;
         float part[QH];
 #pragma unroll
         for (int h = 0; h < QH; ++h) part[h] = 0.f;
         if (tk < vis.count) {
-          const float* row = win_visible_row(a, vis, seq, tk);
-          if (piece == 0) my_row[i * 8 + kq] = row;
+          const float* row = my_row[i * 8 + kq];
           const float* kp = row + g * a.dim + 4 * piece;
           const float* qp = q_s + 4 * piece;
+#pragma unroll 8
           for (int d = 0; d < a.dim; d += 16) {
             const float4 k4 = *reinterpret_cast<const float4*>(kp + d);
 #pragma unroll
@@ -427,7 +430,7 @@ window_attn_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const int*
     }
     __syncwarp();
     const int cnt = vis.count - t0 < 32 ? vis.count - t0 : 32;
-#pragma unroll 4
+#pragma unroll (THREADS > 256 ? 8 : 4)
     for (int jj = 0; jj < cnt; ++jj) {
       const float* vp = my_row[jj] + v_off;
       float pj[QH];
@@ -1492,15 +1495,29 @@ template <int QH, bool DIST>
 static int launch_window_attn(const WinArgs& a, int R, const int* row_seq, const int* row_pos, void* out, long long ldo, int out_fp32,
                               cudaStream_t stream) {
   int warps = R <= WIN_SPLIT_ROWS ? 8 : 4;
+  const dim3 grid(R, a.kv_heads * (a.heads / a.kv_heads / QH));
+  // where a head has a CTA and CTAs leave SMs idle, a CTA's chain over its keys is the time: 32 warps walk it.  One row of 32 heads over 516 keys: 22 us with 8.
+  const bool wide = QH == 1 && grid.x * grid.y <= (unsigned)sm_count() && win_smem_floats(1, 32, a.dim, a.vdim) * sizeof(float) <= 48 * 1024;
+  if (wide) warps = 32;
   while (warps > 1 && win_smem_floats(QH, warps, a.dim, a.vdim) * sizeof(float) > 48 * 1024) warps >>= 1;
   const size_t smem = win_smem_floats(QH, warps, a.dim, a.vdim) * sizeof(float);
   LP_REQUIRE(smem <= 48 * 1024, "lp_window_attn: dim=%d vdim=%d do not fit shared memory", a.dim, a.vdim);
-  const dim3 grid(R, a.kv_heads * (a.heads / a.kv_heads / QH));
   const int nv = (a.vdim + 31) / 32;
-  if (nv <= 1) window_attn_kernel<QH, 1, DIST><<<grid, warps * 32, smem, stream>>>(a, R, row_seq, row_pos, out, ldo, out_fp32);
-  else if (nv <= 2) window_attn_kernel<QH, 2, DIST><<<grid, warps * 32, smem, stream>>>(a, R, row_seq, row_pos, out, ldo, out_fp32);
-  else if (nv <= 4) window_attn_kernel<QH, 4, DIST><<<grid, warps * 32, smem, stream>>>(a, R, row_seq, row_pos, out, ldo, out_fp32);
-  else window_attn_kernel<QH, 8, DIST><<<grid, warps * 32, smem, stream>>>(a, R, row_seq, row_pos, out, ldo, out_fp32);
+#define LP_WAK(NV)                                                                                                                             \
+  do {                                                                                                                                         \
+    if constexpr (QH == 1) {                                                                                                                   \
+      if (wide) {                                                                                                                              \
+        window_attn_kernel<QH, NV, DIST, 1024><<<grid, warps * 32, smem, stream>>>(a, R, row_seq, row_pos, out, ldo, out_fp32);               \
+        break;                                                                                                                                 \
+      }                                                                                                                                        \
+    }                                                                                                                                          \
+    window_attn_kernel<QH, NV, DIST, 256><<<grid, warps * 32, smem, stream>>>(a, R, row_seq, row_pos, out, ldo, out_fp32);                    \
+  } while (0)
+  if (nv <= 1) LP_WAK(1);
+  else if (nv <= 2) LP_WAK(2);
+  else if (nv <= 4) LP_WAK(4);
+  else LP_WAK(8);
+#undef LP_WAK
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
