@@ -584,7 +584,7 @@ int lp_parity_softmax(float* scores, long long ld, int Tq, int Tk, float scale, 
 enum lp_linear_epi { LP_EPI_NONE = 0, LP_EPI_XIELU = 1, LP_EPI_SILU_GATE = 2, LP_EPI_RELU2 = 3, LP_EPI_CLAMP_GLU = 4, LP_EPI_GELU_GATE = 5 };
 enum lp_rot_layout { LP_ROT_HALF = 0, LP_ROT_INTERLEAVED = 1 };
 #define LP_RETENTION_CHUNK 32
-#define LP_LATENT_SPLIT_ROWS 16   /* lp_latent_attend: up to this many rows a CTA per (row, head) splits the keys over its warps */
+#define LP_LATENT_SPLIT_ROWS 16   /* lp_latent_attend_tiles: up to this many rows go to lp_latent_attend, a CTA per (row, head) */
 
 /* C[M, N'] = epi(A[M, K] W[N, K]^T), `batch` problems `*_batch` elements apart.  A: fp32 (a_fp32) or bf16; W: bf16; C: fp32 (c_fp32) or
  * bf16.  epi XIELU: a z^2 + z/2 (z > 0), b (exp(z) - 1 - z) + z/2 (z <= 0) with a = epi_a, b = epi_b.  epi SILU_GATE: W = [gate rows;
@@ -702,13 +702,18 @@ int lp_latent_attend_tiles(const lp_latent_desc* desc, int R, const int* row_seq
                            const int* chunk_row0, const int* chunk_len, const float* q_abs, long long ldqa, void* out, long long ldo,
                            int out_fp32, void* stream);
 
-/* fp32 numbers as three planes of bf16 terms (upper, middle, lower bits of the mantissa: cut off, they add up to the number exactly), `plane`
+/* fp32 numbers as three planes of bf16 terms that add up to them (each takes 8 bits of what the ones before left), `plane`
  * elements apart: rows [M, K] of `src` -> [M, K] of each plane, rows ldp elements apart.  K a multiple of 8, rows on 16-byte boundaries. */
 int lp_split_rows(const float* src, long long ld, int M, int K, void* planes, long long ldp, long long plane, void* stream);
 /* C[M, N] = A[M, K] W[N, K]^T (+ bias fp32 [N]) on the tcgen05 tensor cores with A in three planes and W bf16: an fp32 product, sums in fp32.
  * out: 0 bf16, 1 fp32, 2 three planes c_plane elements apart.  K and N multiples of 8, rows on 16-byte boundaries. */
 int lp_gemm_split(const void* A, long long lda, long long a_plane, const void* W, long long ldw, void* C, long long ldc, long long c_plane,
                   int out, int M, int N, int K, const float* bias, void* stream);
+/* The products of sorted (token, expert) rows on the tcgen05 tensor cores: rows of A (bf16, n_tiles * 128 of them) in tiles of 128 that belong to weight
+ * group tile_group[tile] (device, < 0: an empty tile, whose rows of C are not written; lp_moe_align with tile_rows = 128), group g's weight [N, K] at W + g w_group.
+ * gated != 0: W holds N / 2 rows of gates and as many others, C [rows, N / 2] = silu(row_scale * gate) * (row_scale * other); else C [rows, N]. */
+int lp_gemm_grouped(const void* A, long long lda, const void* W, long long ldw, long long w_group, int groups, const int* tile_group, int n_tiles,
+                    int gated, const float* row_scale, void* C, long long ldc, int out_fp32, int N, int K, void* stream);
 /* Latent attention of prompts with every head's keys and values expanded, on the tensor cores: heads of 128 + 64 rotated channels, values of
  * 128, kv_rank a multiple of 8.  desc as for lp_latent_prep, whose results (rotated queries, this step's cache rows) it reads; w_kv bf16
  * [2 * heads * 128, kv_rank], rows ldw elements apart: the heads' key rows, then their value rows.  seq_row0 [n_seqs + 1], seq_pos0 [n_seqs]:
@@ -787,6 +792,12 @@ int lp_window_attn_talk_tiles(const lp_window_attn_desc* desc, int R, const int*
  * lp_retention_prefill (at most LP_RETENTION_CHUNK rows a chunk, never across requests) say which rows belong together */
 int lp_window_attn_tiles(const lp_window_attn_desc* desc, int R, const int* row_seq, const int* row_pos, int n_chunks, const int* chunk_seq,
                          const int* chunk_row0, const int* chunk_len, void* out, long long ldo, int out_fp32, void* stream);
+/* the same result for the rows of prompts on the tensor cores, heads of 128 without distance bias or mixed heads: 128 rows of a request
+ * and a head a CTA (tables as for lp_latent_attend_expanded).  n_keys = sum over requests of the kept tokens and blocks that its last row sees
+ * and of its tokens from the first that its first row's window (or own block of positions) holds; row_floats: floats of a cache row. */
+size_t lp_window_prompt_workspace_bytes(int R, int heads, int row_floats, int n_keys);
+int lp_window_attn_prompt(const lp_window_attn_desc* desc, int R, int n_seqs, const int* seq_row0, const int* seq_pos0, int n_tiles, int n_keys,
+                          void* out, long long ldo, int out_fp32, void* ws, size_t ws_bytes, void* stream);
 
 /* minGRU: z = sigmoid(zxg[:, z_off + c] + z_bias[c]), u = zxg[:, x_off + c] + x_bias[c], candidate = u + 1/2 (u >= 0) or sigmoid(u)
  * (u < 0); S_t = (1 - z) S_(t-1) + z candidate per channel, out = S_t * silu(zxg[:, g_off + c]).  state fp32 [slots][width], carried

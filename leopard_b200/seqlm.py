@@ -45,6 +45,12 @@ SPLIT_MIN_ROWS, SPLIT_MIN_K = 65, 64
 # its tiles are 128 rows of one request.  A layer of width 1024 with 8 heads (us, lp_latent_attend_tiles and this one): one request of 20 rows 64, 45, of
 # 500 297, 85; 32 requests of 12 rows 92, 81; 64 of 12 97, 120, of 24 132, 126; width 2048, 16 heads: 4096 rows 6,490, 530; 64 requests of 12 rows 225, 205.
 EXPAND_TILES, EXPAND_TILE_ROWS = 32, 24
+# Window attention of prompts goes to lp_window_attn_prompt (128 rows of a request and a head a CTA) where its tiles are filled, or where there is one
+# CTA an SM at most.  A layer, preparation included (us, lp_window_attn_tiles and this one; heads on a quarter of key / value heads): one request of 20 rows,
+# 8 heads 29, 22; of 500 86, 45; of 4096, 16 heads 845, 302; 16 requests of 20, 8 heads 32, 29, 16 heads 35, 42; 16 of 40, 16 heads 40, 54; 32 of 12, 4 heads 27,
+# 32.  Capped scores and values turned back by position cost it more (a table, tanh, an exchange): one request of 128 rows, 16 heads 51, 58; of 500, 4 heads
+# 72, 74, 8 heads 102, 76; of 4096, 16 heads 1009, 417.
+WINDOW_TILE_ROWS, WINDOW_FEW_ROWS, WINDOW_CAP_ROWS, WINDOW_CAP_WORK = 64, 20, 300, 4000
 # Up to MOE_PAIRS_MAX (token, choice) pairs an expert's weights are streamed once for the pairs that chose it.  Both products of 16 experts,
 # width 2048, 1024 inside (us, bf16; fp32 rows), against sorted tiles: 128 pairs 66, 108; 85, 182.  256 pairs 93, 108; 138, 182.  512 pairs 161,
 # 108; 282, 182: with this few experts the sorted tiles are ahead from about 300 pairs, with 32 (width 4096) not yet at 512: 554, 683; 876, 1116.
@@ -888,6 +894,7 @@ class SeqLMEngine:
         self.tile_rows = int(self.L.lp_linear_tile_rows())
         # large bf16 products of the serving precision go to the tcgen05 GEMM when the library has it (the native ones do)
         self.tensor_core_rows = TENSOR_CORE_MIN_ROWS if dtype == "bfloat16" and hasattr(self.L, "lp_gemm_bf16") else None
+        self.sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count if self.device.type == "cuda" else 1
         self.split_rows = SPLIT_MIN_ROWS if hasattr(self.L, "lp_gemm_split") and self.device.type == "cuda" else None
         self.tap: Optional[Callable[[int, torch.Tensor], None]] = None   # called with (layer, residual stream) after every layer
         # decode steps are launch-bound: a batch layout (requests, page-table width) that comes back is captured into a CUDA graph on
@@ -1225,10 +1232,40 @@ class SeqLMEngine:
         elif b.decode:
             rc = self.L.lp_window_attn(C.byref(d), b.R, _lib.ptr(b.row_seq), _lib.ptr(b.row_pos), _lib.ptr(o), o.stride(0),
                                        int(o.dtype == F32), st)
+        elif self._window_prompt(m, d, qkv, b, o):
+            return
         else:      # prompts and portions: tiles of consecutive rows share the keys they read
             rc = self.L.lp_window_attn_tiles(C.byref(d), b.R, _lib.ptr(b.row_seq), _lib.ptr(b.row_pos), b.n_chunks, _lib.ptr(b.chunk_seq),
                                              _lib.ptr(b.chunk_row0), _lib.ptr(b.chunk_len), _lib.ptr(o), o.stride(0), int(o.dtype == F32), st)
         self._check(rc, "lp_window_attn")
+
+    def _window_prompt(self, m: WindowAttentionConfig, d, qkv: torch.Tensor, b: _Batch, o: torch.Tensor) -> bool:
+        """whether lp_window_attn_prompt has taken these rows"""
+        if (not hasattr(self.L, "lp_window_attn_prompt") or m.dim != 128 or m.vdim != 128 or m.distance_bias or m.distance_slope
+                or qkv.stride(0) % 4 or qkv.data_ptr() % 16 or o.data_ptr() % 16 or o.stride(0) % (4 if o.dtype == F32 else 8)):
+            return False
+        tiles = sum(-(-ln // 128) for ln in b.lens)
+        if d.softcap > 0 or d.v_inv_freq:
+            pays = b.R >= WINDOW_TILE_ROWS * tiles and b.R >= WINDOW_CAP_ROWS and b.R * m.heads >= WINDOW_CAP_WORK
+        else:
+            pays = b.R >= WINDOW_TILE_ROWS * tiles or (b.R >= WINDOW_FEW_ROWS * tiles and tiles * m.heads <= self.sm_count)
+        if not pays:
+            return False
+
+        def first(pos):      # the first token of its window, or of its own block of positions
+            lo = max(0, pos - d.window + 1) if d.window > 0 else 0
+            return max(lo, pos // d.chunk * d.chunk) if d.chunk else lo
+        keys = 0
+        for p, ln in zip(b.starts.tolist(), b.lens):
+            past = p + ln - d.window if d.window > 0 else 0      # positions wholly before the last row's window
+            keys += min(d.keep_first, first(p + ln - 1)) + (past // d.pool if d.pool and past > 0 else 0) + p + ln - first(p)
+        row = m.kv_heads * 128 * (1 if m.values_are_keys else 2)
+        nbytes = int(self.L.lp_window_prompt_workspace_bytes(b.R, m.heads, row, keys))
+        ws = self._empty((nbytes,), torch.uint8)
+        rc = self.L.lp_window_attn_prompt(C.byref(d), b.R, b.n, _lib.ptr(b.seq_row0), _lib.ptr(b.seq_pos0), tiles, keys, _lib.ptr(o), o.stride(0),
+                                          int(o.dtype == F32), _lib.ptr(ws), nbytes, self._stream())
+        self._check(rc, "lp_window_attn_prompt")
+        return True
 
     def _decay_rows(self, lw, t: torch.Tensor, tanh: bool) -> torch.Tensor:
         """the pre-activations of a decay, fp32 [R, heads * dim], from its low-rank vector t: a product that keeps its operand's 32 bits — as

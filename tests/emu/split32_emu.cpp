@@ -17,20 +17,20 @@ extern "C" void emu_split_rows(const float* src, long long ld, int M, int K, voi
   emu::launch(dim3((unsigned)(((long long)M * (K / 8) + 255) / 256)), dim3(256), [&] { split_rows_kernel(src, ld, M, K, (bf16*)dst, ldd, plane); });
 }
 
-extern "C" void emu_latent_gather(int n_seqs, int window, const int* row0, const int* pos0, int n_keys, const float* cache, int page_size,
-                                  const int* table, int max_pages, int width, void* dst, long long plane) {
-  Seqs32 q = {n_seqs, window, row0, pos0};
+extern "C" void emu_gather_keys(int n_seqs, int window, int keep_first, int pool, const int* row0, const int* pos0, int n_keys, const float* cache,
+                                int page_size, const int* table, int max_pages, const float* blocks, const int* block_table, int width, void* dst, long long plane) {
+  Seqs32 q = {n_seqs, window, row0, pos0, 0, keep_first, pool};
   emu::launch(dim3((unsigned)(((long long)n_keys * (width / 8) + 255) / 256)), dim3(256),
-              [&] { latent_gather_kernel(q, n_keys, cache, page_size, table, max_pages, width, (bf16*)dst, plane); });
+              [&] { gather_keys_kernel(q, n_keys, cache, page_size, table, max_pages, blocks, block_table, max_pages, width, (bf16*)dst, plane); });
 }
 
-template <int BN>
-static void run_gemm(Gemm32Args& a, int ctas) {
+template <int BN, int PLANES, bool GATED>
+static void run_gemm(Gemm32Args& a, int ctas, int groups, long long w_group) {
   a.n_tiles_m = (a.M + 127) / 128;
-  a.n_tiles_n = (a.N + BN - 1) / BN;
-  const CUtensorMap ta = tmap3(a.A, a.K, a.M, 3, a.lda, a.a_plane, 128), tw = tmap3(a.W, a.K, a.N, 1, a.ldw, 0, BN);
+  a.n_tiles_n = (GATED ? (a.N / 2 + BN / 2 - 1) / (BN / 2) : (a.N + BN - 1) / BN);
+  const CUtensorMap ta = tmap3(a.A, a.K, a.M, PLANES, a.lda, a.a_plane, 128), tw = tmap3(a.W, a.K, a.N, groups, a.ldw, w_group, GATED ? 64 : BN);
   emu::g_block_hook = [] { emu_tc::reset(); };
-  emu::launch(dim3(ctas), dim3(G32_THREADS), [&] { gemm32_kernel<BN>(ta, tw, a); });
+  emu::launch(dim3(ctas), dim3(G32_THREADS), [&] { gemm32_kernel<BN, PLANES, GATED>(ta, tw, a); });
   emu::g_block_hook = nullptr;
 }
 
@@ -39,25 +39,40 @@ extern "C" void emu_gemm_split(const void* A, long long lda, long long a_plane, 
   Gemm32Args a = {};
   a.M = M; a.N = N; a.K = K; a.bias = bias; a.C = C; a.ldc = ldc; a.c_plane = c_plane; a.out = out;
   a.A = (const bf16*)A; a.lda = lda; a.a_plane = a_plane; a.W = (const bf16*)W; a.ldw = ldw;
-  if (bn == 256) run_gemm<256>(a, ctas);
-  else run_gemm<128>(a, ctas);
+  if (bn == 256) run_gemm<256, 3, false>(a, ctas, 1, 0);
+  else run_gemm<128, 3, false>(a, ctas, 1, 0);
 }
 
-// q planes [3][R][heads * DQ], k and v planes [3][n_keys][heads * 128], kr planes [3][n_keys][64] or null
-extern "C" void emu_attn32(const void* q, const void* k, const void* kr, const void* v, int R, int heads, int n_seqs, int window, const int* row0,
-                           const int* pos0, int n_tiles, int n_keys, float scale, const float* sink, const float* gate, const float* out_gate, void* out,
-                           int out_fp32) {
+extern "C" void emu_gemm_grouped(const void* A, const void* W, int groups, const int* tile_group, int n_tiles, int gated, const float* row_scale, void* C,
+                                 int out_fp32, int N, int K, int ctas) {
+  Gemm32Args a = {};
+  a.M = n_tiles * 128; a.N = N; a.K = K; a.C = C; a.ldc = gated ? N / 2 : N; a.out = out_fp32;
+  a.A = (const bf16*)A; a.lda = K; a.W = (const bf16*)W; a.ldw = K; a.tile_group = tile_group; a.row_scale = row_scale;
+  if (gated) run_gemm<256, 1, true>(a, ctas, groups, (long long)N * K);
+  else run_gemm<256, 1, false>(a, ctas, groups, (long long)N * K);
+}
+
+// q planes [3][R][heads * DQ], k and v planes [3][n_keys][heads / ratio * 128], kr planes [3][n_keys][64] or null
+extern "C" void emu_attn32(const void* q, const void* k, const void* kr, const void* v, int R, int heads, int ratio, int n_seqs, int window, int chunk,
+                           int keep_first, int pool, const int* row0, const int* pos0, int n_tiles, int n_keys, float scale, float softcap, int sink_one,
+                           const float* sink, const float* gate, const float* out_gate, const float* v_inv_freq, int turn_half, int turn_interleaved,
+                           void* table, void* out, int out_fp32) {
   const int dq = kr != nullptr ? 192 : 128;
   Attn32Args a = {};
-  a.seqs = {n_seqs, window, row0, pos0};
-  a.heads = heads; a.scale = scale; a.sink = sink; a.gate = gate; a.ldg = heads; a.out_gate = out_gate; a.ldog = heads * 128;
+  a.seqs = {n_seqs, window, row0, pos0, chunk, keep_first, pool};
+  a.ratio = ratio; a.scale = scale; a.softcap = softcap; a.sink_one = sink_one; a.out_scale = 1.0f;
+  a.sink = sink; a.gate = gate; a.ldg = heads; a.out_gate = out_gate; a.ldog = heads * 128;
   a.out = out; a.ldo = heads * 128; a.out_fp32 = out_fp32;
   a.q = (const bf16*)q; a.k = (const bf16*)k; a.kr = (const bf16*)kr; a.v = (const bf16*)v;
-  a.ldq = heads * dq; a.ldk = heads * 128; a.ldkr = 64;
+  a.ldq = heads * dq; a.ldk = heads / ratio * 128; a.ldkr = 64;
   a.q_plane = (long long)R * a.ldq; a.k_plane = (long long)n_keys * a.ldk; a.kr_plane = (long long)n_keys * 64;
   const CUtensorMap tq = tmap3(q, a.ldq, R, 3, a.ldq, a.q_plane, 128), tk = tmap3(k, a.ldk, n_keys, 3, a.ldk, a.k_plane, 128);
   const CUtensorMap tv = tmap3(v, a.ldk, n_keys, 3, a.ldk, a.k_plane, 64);
   const CUtensorMap tr = kr != nullptr ? tmap3(kr, 64, n_keys, 3, 64, a.kr_plane, 128) : tk;
+  if (turn_half > 0) {
+    emu::launch(dim3((unsigned)((R * turn_half + 255) / 256)), dim3(256), [&] { turn_table_kernel(a.seqs, R, v_inv_freq, turn_half, (float2*)table); });
+    a.turn = (const float2*)table; a.turn_half = turn_half; a.turn_interleaved = turn_interleaved;
+  }
   emu::g_block_hook = [] { emu_tc::reset(); };
   emu::launch(dim3(heads, n_tiles), dim3(A32_THREADS), [&] {
     if (kr != nullptr) attn32_kernel<1>(tq, tk, tr, tv, a);

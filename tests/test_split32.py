@@ -66,6 +66,27 @@ def test_product_of_three_planes(emu, M, N, K, bn, ctas, out):
     assert float((got - want).norm() / want.norm()) < (4e-3 if out == 0 else 5e-7)
 
 
+@pytest.mark.parametrize("groups,tile_group,N,K,gated,out,ctas", [(3, [2, -1, 0], 272, 136, True, 0, 2), (2, [1, 1], 144, 72, False, 1, 3),
+                                                                  (2, [0, 1, -1], 304, 200, True, 1, 1), (4, [3], 256, 64, False, 0, 1)])
+def test_grouped_product(emu, groups, tile_group, N, K, gated, out, ctas):
+    g, rows = torch.Generator().manual_seed(N), 128 * len(tile_group)
+    a, w = torch.randn((rows, K), generator=g).to(BF), (torch.randn((groups, N, K), generator=g) / K ** 0.5).to(BF)
+    scale = torch.rand(rows, generator=g) if gated else None
+    c = torch.full((rows, N // 2 if gated else N), float("nan"), dtype=F32 if out else BF)
+    tg = torch.tensor(tile_group, dtype=torch.int32)
+    emu.emu_gemm_grouped(P(a), P(w), groups, P(tg), len(tile_group), int(gated), P(scale), P(c), out, N, K, ctas)
+    for t, e in enumerate(tile_group):
+        r = slice(128 * t, 128 * t + 128)
+        if e < 0:
+            assert bool(torch.isnan(c[r].float()).all())
+            continue
+        y = a[r].double() @ w[e].double().T
+        if gated:
+            y = y * scale[r, None].double()
+            y = torch.nn.functional.silu(y[:, :N // 2]) * y[:, N // 2:]
+        assert float((c[r].double() - y).norm() / y.norm()) < (1e-6 if out else 4e-3)
+
+
 def test_product_with_infinite_weight(emu):
     """as fp32 multiply-adds: an infinite weight gives infinities, zero times it NaN"""
     x, w = torch.randn((5, 64), generator=torch.Generator().manual_seed(3)), torch.ones((128, 64)).to(BF)
@@ -78,70 +99,112 @@ def test_product_with_infinite_weight(emu):
     assert bool(torch.isfinite(c[:, :9]).all()) and bool(torch.isfinite(c[:, 10:]).all())
 
 
-def reference(q, k, kr, v, lens, pos0, window, scale, sink, gate, out_gate):
-    """float64; keys and values lie request by request from its first visible position on"""
-    R, H = q.shape[0], v.shape[1] // 128
+def seen(pos, window, chunk=0, keep_first=0, pool=0):
+    """(kept tokens, blocks, first token) that a query at `pos` sees"""
+    lo = max(0, pos - window + 1) if window else 0
+    if chunk:
+        lo = max(lo, pos // chunk * chunk)
+    return min(keep_first, lo), ((pos - window + 1) // pool if pool and window and pos - window + 1 > 0 else 0), lo
+
+
+def run_keys(p0, n, *rule):
+    """the key rows of a request that brings n tokens from position p0 on"""
+    keep, blocks, _ = seen(p0 + n - 1, *rule)
+    return [("token", t) for t in range(keep)] + [("block", t) for t in range(blocks)] + [("token", t) for t in range(seen(p0, *rule)[2], p0 + n)]
+
+
+def reference(q, k, kr, v, lens, pos0, rule, scale, heads, softcap=0.0, sink=None, gate=None, out_gate=None, turn=None):
+    """float64; keys and values lie request by request as run_keys says; sink: a score per head that joins the denominator"""
+    R, H, kvh = q.shape[0], heads, v.shape[1] // 128
     dq = q.shape[1] // H
     out, r, base = torch.zeros((R, H * 128), dtype=F64), 0, 0
     for n, p0 in zip(lens, pos0):
-        lo = max(0, p0 - window + 1) if window else 0
+        run = run_keys(p0, n, *rule)
+        n_blocks, n_keep = sum(kind == "block" for kind, _ in run), seen(p0 + n - 1, *rule)[0]
         for i in range(n):
-            pos = p0 + i
-            a, b = base + (max(lo, pos - window + 1) if window else lo) - lo, base + pos - lo + 1
+            keep, blocks, lo = seen(p0 + i, *rule)
+            first = seen(p0, *rule)[2]
+            at = list(range(keep)) + list(range(n_keep, n_keep + blocks)) + [n_keep + n_blocks + t - first for t in range(lo, p0 + i + 1)]
+            at = torch.tensor(at) + base
             for h in range(H):
-                kk = k[a:b, h * 128:(h + 1) * 128].double()
+                c = slice(h // (H // kvh) * 128, h // (H // kvh) * 128 + 128)
+                kk = k[at][:, c].double()
                 if kr is not None:
-                    kk = torch.cat([kk, kr[a:b].double()], 1)
+                    kk = torch.cat([kk, kr[at].double()], 1)
                 s = kk @ q[r, h * dq:(h + 1) * dq].double() * scale
+                if softcap:
+                    s = softcap * torch.tanh(s / softcap)
                 top = max(float(s.max()), float(sink[h]) if sink is not None else -math.inf)
                 e = torch.exp(s - top)
                 den = e.sum() + (math.exp(float(sink[h]) - top) if sink is not None else 0.0)
-                o = e @ v[a:b, h * 128:(h + 1) * 128].double() / den
+                o = e @ v[at][:, c].double() / den
+                if turn is not None:      # frequencies and layout
+                    angle = (p0 + i) * turn[0].double()
+                    m = len(angle)
+                    u, w = (o[0:2 * m:2].clone(), o[1:2 * m:2].clone()) if turn[1] else (o[:m].clone(), o[m:2 * m].clone())
+                    u, w = u * torch.cos(angle) + w * torch.sin(angle), w * torch.cos(angle) - u * torch.sin(angle)
+                    if turn[1]:
+                        o[0:2 * m:2], o[1:2 * m:2] = u, w
+                    else:
+                        o[:m], o[m:2 * m] = u, w
                 if gate is not None:
                     o = o * torch.sigmoid(gate[r, h].double())
                 out[r, h * 128:(h + 1) * 128] = o
             r += 1
-        base += p0 + n - lo
+        base += len(run)
     return out * torch.sigmoid(out_gate.double()) if out_gate is not None else out
 
 
-@pytest.mark.parametrize("lens,pos0,window,rot,opts", [([130], [0], 0, True, ""), ([40, 129], [300, 0], 100, True, "sink"), ([257], [70], 150, False, "gates"),
-                                                       ([3, 1, 20], [0, 500, 127], 0, True, "")])
+@pytest.mark.parametrize("lens,pos0,window,rot,opts", [
+    ([130], [0], 0, True, {}), ([40, 129], [300, 0], 100, True, {"sink": True}), ([257], [70], 150, False, {"gates": True}),
+    ([3, 1, 20], [0, 500, 127], 0, True, {}), ([200], [0], 40, False, {"keep": 4, "ratio": 2}), ([150, 30], [100, 900], 64, False, {"pool": 8, "cap": 3.0}),
+    ([140], [20], 30, False, {"keep": 5, "pool": 3, "sink_one": True, "turn": (64, False)}), ([20], [9], 16, False, {"turn": (24, True), "pool": 2}),
+    ([160, 9], [50, 7], 90, False, {"chunk": 32})])
 def test_attention_of_three_planes(emu, lens, pos0, window, rot, opts):
-    H, R, dq = 2, sum(lens), 192 if rot else 128
+    H, R, dq, ratio = 2, sum(lens), 192 if rot else 128, opts.get("ratio", 1)
     g = torch.Generator().manual_seed(R)
-    n_keys = sum(p + n - (max(0, p - window + 1) if window else 0) for n, p in zip(lens, pos0))
-    q, k = 2 * torch.randn((R, H * dq), generator=g), torch.randn((n_keys, H * 128), generator=g)
-    kr, v = torch.randn((n_keys, 64), generator=g) if rot else None, torch.randn((n_keys, H * 128), generator=g)
-    sink = torch.randn(H, generator=g) if opts == "sink" else None
-    gate, og = (torch.randn((R, H), generator=g), torch.randn((R, H * 128), generator=g)) if opts == "gates" else (None, None)
+    rule = (window, opts.get("chunk", 0), opts.get("keep", 0), opts.get("pool", 0))
+    n_keys = sum(len(run_keys(p, n, *rule)) for n, p in zip(lens, pos0))
+    q, k = 2 * torch.randn((R, H * dq), generator=g), torch.randn((n_keys, H // ratio * 128), generator=g)
+    kr, v = torch.randn((n_keys, 64), generator=g) if rot else None, torch.randn((n_keys, H // ratio * 128), generator=g)
+    sink = torch.randn(H, generator=g) if "sink" in opts else None
+    gate, og = (torch.randn((R, H), generator=g), torch.randn((R, H * 128), generator=g)) if "gates" in opts else (None, None)
     row0 = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32)
     p0 = torch.tensor(pos0, dtype=torch.int32)
     out = torch.full((R, H * 128), float("nan"))
     tiles = sum(-(-n // 128) for n in lens)
+    half, inter = opts.get("turn", (0, False))
+    freq, table = 10.0 ** -torch.linspace(0, 2, max(half, 1)), torch.empty((R, max(half, 1), 2))
 
     def run():
         p = [planes(emu, x) if x is not None else None for x in (q, k, kr, v)]
-        emu.emu_attn32(*[P(x) for x in p], R, H, len(lens), window, P(row0), P(p0), tiles, n_keys, C.c_float(dq ** -0.5), P(sink), P(gate), P(og), P(out), 1)
+        emu.emu_attn32(*[P(x) for x in p], R, H, ratio, len(lens), *rule, P(row0), P(p0), tiles, n_keys, C.c_float(dq ** -0.5),
+                       C.c_float(opts.get("cap", 0.0)), int("sink_one" in opts), P(sink), P(gate), P(og), P(freq), half, int(inter), P(table),
+                       P(out), 1)
     run()
-    want = reference(q, k, kr, v, lens, pos0, window, dq ** -0.5, sink, gate, og)
+    want = reference(q, k, kr, v, lens, pos0, rule, dq ** -0.5, H, opts.get("cap", 0.0), torch.zeros(H) if "sink_one" in opts else sink, gate, og,
+                     (freq, inter) if half else None)
     assert float((out.double() - want).norm() / want.norm()) < 1e-6
-    if opts == "sink":      # a value that is not finite reaches only the rows that see it
+    if "sink" in opts or "pool" in opts:      # a value that is not finite reaches only the rows that see it
         v[n_keys - 1, 3] = float("inf")
         run()
-        assert not bool(torch.isfinite(out[R - 1, 3])) and bool(torch.isfinite(out[: R - 1]).all()) and bool(torch.isfinite(out[R - 1, 4:128]).all())
+        assert not bool(torch.isfinite(out[R - 1, 3])) and bool(torch.isfinite(out[: R - 1]).all())
+        assert half or bool(torch.isfinite(out[R - 1, 4:128]).all())
+        assert float((out[: R - 1].double() - want[: R - 1]).norm() / want.norm()) < 1e-6
 
 
 def test_gather_of_cache_rows(emu):
     g = torch.Generator().manual_seed(4)
-    width, page, lens, pos0, window = 24, 4, [3, 5], [6, 0], 4
-    cache = torch.randn((8 * page, width), generator=g)
-    table = torch.tensor([[5, 1, 7], [2, 0, -1]], dtype=torch.int32)
+    width, page, lens, pos0, rule = 24, 4, [3, 5], [6, 0], (4, 0, 2, 2)
+    cache, blocks = torch.randn((8 * page, width), generator=g), torch.randn((4 * page, width), generator=g)
+    table, block_table = torch.tensor([[5, 1, 7], [2, 0, -1]], dtype=torch.int32), torch.tensor([[3, 1, -1], [0, 2, -1]], dtype=torch.int32)
     row0, p0 = torch.tensor([0, 3, 8], dtype=torch.int32), torch.tensor(pos0, dtype=torch.int32)
-    rows = [(s, p) for s, (n, a) in enumerate(zip(lens, pos0)) for p in range(max(0, a - window + 1), a + n)]
+    rows = [(s, kind, t) for s, (n, a) in enumerate(zip(lens, pos0)) for kind, t in run_keys(a, n, *rule)]
     got = torch.zeros((3, len(rows), width), dtype=BF)
-    emu.emu_latent_gather(2, window, P(row0), P(p0), len(rows), P(cache), page, P(table), 3, width, P(got), LL(len(rows) * width))
-    want = torch.stack([cache[int(table[s, p // page]) * page + p % page] for s, p in rows])
+    emu.emu_gather_keys(2, rule[0], rule[2], rule[3], P(row0), P(p0), len(rows), P(cache), page, P(table), 3, P(blocks), P(block_table), width, P(got),
+                        LL(len(rows) * width))
+    want = torch.stack([(blocks if kind == "block" else cache)[int((block_table if kind == "block" else table)[s, t // page]) * page + t % page]
+                        for s, kind, t in rows])
     assert torch.equal(got.double().sum(0), want.double())
 
 
