@@ -447,8 +447,8 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[j][i][c] = run[LONG ? j : 0][LONG ? i : 0][c] = 0.f;
     int turn = 0;
-    for (int s = warp; s * 32 < a.K; s += U * n_warps) {
-      uint4 u0[U][NT], u1[U][NT];
+    const int stride = U * n_warps;
+    auto fetch = [&](int s, uint4 (&u0)[U][NT], uint4 (&u1)[U][NT]) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int k = (s + u * n_warps) * 32 + t * 8;
@@ -458,6 +458,8 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
           u1[u][j] = k < a.K && w1[j] != nullptr ? ldg_once(w1[j] + k) : none;
         }
       }
+    };
+    auto take = [&](int s, const uint4 (&u0)[U][NT], const uint4 (&u1)[U][NT]) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int k = (s + u * n_warps) * 32 + t * 8;
@@ -511,6 +513,25 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
                 run[j][i][c] = 0.f;
               }
         }
+      }
+    };
+    uint4 a0[U][NT], a1[U][NT];
+    // one tile of up to eight bf16 rows leaves registers free: the next steps' weights are asked for before these are used (K = N = 4096, one row: 10.6 us,
+    // 8.7 so; two tiles 26.6, 27.4, fp32 rows 4.6, 5.3: their registers cost CTAs)
+    if constexpr (MG == 1 && NT == 1 && sizeof(AT) == 2) {
+      uint4 b0[U][NT], b1[U][NT];
+      fetch(warp, a0, a1);
+      for (int s = warp; s * 32 < a.K; s += 2 * stride) {
+        fetch(s + stride, b0, b1);
+        take(s, a0, a1);
+        if ((s + stride) * 32 >= a.K) break;
+        fetch(s + 2 * stride, a0, a1);
+        take(s + stride, b0, b1);
+      }
+    } else {
+      for (int s = warp; s * 32 < a.K; s += stride) {
+        fetch(s, a0, a1);
+        take(s, a0, a1);
       }
     }
     if constexpr (LONG) {
