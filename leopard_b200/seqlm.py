@@ -58,6 +58,7 @@ WINDOW_TILE_ROWS, WINDOW_FEW_ROWS, WINDOW_CAP_ROWS, WINDOW_CAP_WORK = 64, 20, 30
 # faster (width 2044, 1020 inside, 16 experts: 64 pairs 481, 488; 128 pairs 936, 488).
 MOE_PAIRS_MAX = 512
 MOE_PAIRS_ALONE = 64
+GROUP_TILE_ROWS = 128          # rows of a tensor-core tile of sorted expert rows
 PAD_PROJECTION_ROWS = 128      # a projection narrower than a tensor-core tile is padded with zero rows beside ones that are at least this wide
 MAX_DECODE_GRAPHS = 32         # captured decode layouts kept at a time
 PAGE_TABLE_STEP = 16           # decode batches round their page-table width up to a multiple of this
@@ -1460,21 +1461,33 @@ class SeqLMEngine:
                                  K=f.expert_ff, batch=1, epi=_lib.EPI_NONE, epi_a=0.0, epi_b=0.0)
             self._check(L.lp_linear_group_pairs(C.byref(d2), _lib.ptr(idx), f.experts, 1, n_pairs, st), "lp_linear_group_pairs")
             return self._moe_combine(f, lw, h, y, self._pair_rows, None if on_input else wts, gate)
-        tiles = int(L.lp_moe_max_tiles(n_pairs, f.experts, self.tile_rows))
+        w_gu, w_dn = lw["w_gu"], lw["w_edown"]
+        # rows enough to fill tensor-core tiles in the serving precision: an expert's rows are gathered into tiles of its own and all experts' products are
+        # one launch, without a look at the tables on the host
+        grouped = (self.tensor_core_rows is not None and n_pairs >= f.experts * self.tensor_core_rows and h.dtype == BF16 and epi == _lib.EPI_SILU_GATE
+                   and hasattr(L, "lp_gemm_grouped") and D % 16 == 0 and f.expert_ff % 8 == 0 and all(t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (w_gu, w_dn)))
+        tile_rows = GROUP_TILE_ROWS if grouped else self.tile_rows
+        tiles = int(L.lp_moe_max_tiles(n_pairs, f.experts, tile_rows))
         tile_group = self._empty((tiles,), I32)
-        sorted_token = self._empty((tiles * self.tile_rows,), I32)
+        sorted_token = self._empty((tiles * tile_rows,), I32)
         pair_row = self._empty((n_pairs,), I32)
-        rc = L.lp_moe_align(_lib.ptr(idx), n_pairs, f.top, f.experts, self.tile_rows, tiles, _lib.ptr(tile_group), _lib.ptr(sorted_token),
+        rc = L.lp_moe_align(_lib.ptr(idx), n_pairs, f.top, f.experts, tile_rows, tiles, _lib.ptr(tile_group), _lib.ptr(sorted_token),
                             _lib.ptr(pair_row), st)
         self._check(rc, "lp_moe_align")
-        rows = tiles * self.tile_rows
+        rows = tiles * tile_rows
         scale = None
         if on_input:      # the pairs' weights in the sorted row space
             scale = torch.zeros((rows,), dtype=F32, device=self.device)      # padding rows of the sorted space stay zero
             self._check(L.lp_moe_sorted_weights(_lib.ptr(pair_row), _lib.ptr(wts), n_pairs, _lib.ptr(scale), st), "lp_moe_sorted_weights")
         h1 = self._empty((rows, f.expert_ff), self.act)
         y = self._empty((rows, D), F32)
-        w_gu, w_dn = lw["w_gu"], lw["w_edown"]
+        if grouped:
+            a_sorted = h.index_select(0, sorted_token.clamp_min(0))
+            for a, w, c, n, k, gated in ((a_sorted, w_gu, h1, 2 * f.expert_ff, D, 1), (h1, w_dn, y, D, f.expert_ff, 0)):
+                rc = L.lp_gemm_grouped(_lib.ptr(a), a.stride(0), _lib.ptr(w), w.stride(1), w.stride(0), f.experts, _lib.ptr(tile_group), tiles, gated,
+                                       _lib.ptr(scale) if gated else None, _lib.ptr(c), c.stride(0), int(c.dtype == F32), n, k, st)
+                self._check(rc, "lp_gemm_grouped")
+            return self._moe_combine(f, lw, h, y, pair_row, None if on_input else wts, gate)
         capturing = self.device.type == "cuda" and torch.cuda.is_current_stream_capturing()      # no host read inside a graph
         if self.tensor_core_rows is not None and n_pairs >= f.experts * self.tensor_core_rows and h.dtype == BF16 and not capturing:
             # prefill in the serving precision: enough rows per expert to fill tensor-core tiles.  The segment bounds come to the host

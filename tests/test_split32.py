@@ -275,3 +275,27 @@ def test_products_of_fp32_rows_in_the_engine(M, N, K):
             err.append(float((y - ref).norm() / ref.norm()))
             assert float((z - (x.double() + 0.5 * ref)).norm() / z.norm()) < 1e-6
         assert err[0] < max(err[1] * 1.2, 2e-7)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,width,ff,on_host", [(128, 80, 72, False), (127, 80, 72, None), (300, 64, 136, False), (300, 72, 64, True)])
+def test_expert_products_of_prompts_are_one_launch(T, width, ff, on_host):
+    """the fewest tokens that fill tiles, one fewer, an expert whose rows are several tiles, and a width that is no multiple of 16 (a product an expert)"""
+    from oracle import seqlm as O
+    from seqlm_common import TOL, make_engine, model, moe, rel_err, retention_layer
+    form = moe(experts=4, top=2, groups=2, keep=2, ff=ff, shared=16)
+    cfg = model([retention_layer(mlp=form)], width=width)
+    w = O.random_weights(cfg, seed=1)
+    eng = make_engine(cfg, w, ("cuda", None), "bfloat16")
+    h = torch.randn(T, width, generator=torch.Generator().manual_seed(T)).to(BF)
+    calls = []
+
+    class Spy:
+        def __getattr__(self, name):
+            f = getattr(lib, name)
+            return (lambda *a: calls.append(name) or f(*a)) if name in ("lp_gemm_grouped", "lp_moe_align") else f
+    lib, eng.L = eng.L, Spy()
+    got = eng._moe(eng.cfg.layers[0].ff, eng.w.layers[0], h.cuda())
+    want = O.feed_forward(h.double(), {k: v.to(BF).double() if v.ndim == 2 else v.double() for k, v in w.items()}, "l0.mlp.", form)
+    assert rel_err(got, want) < TOL["bfloat16"]
+    assert calls.count("lp_gemm_grouped") == (2 if on_host is False else 0) and calls.count("lp_moe_align") == (on_host is not None)
