@@ -71,6 +71,9 @@ struct RetArgs {
   int in_act, finish;
 };
 
+// floats between rows of keys and queries in shared memory: rows of 16-byte pieces whose neighbours lie four banks further, or rows an odd stride apart
+template <bool WIDE> __host__ __device__ inline int ret_dimp(int dim) { return WIDE ? dim + 4 : ((dim + 3) & ~3) + 1; }
+
 __device__ __forceinline__ float ret_silu(float z) { return z / (1.0f + expf(-z)); }
 // element d of one head's q or k: activation (when asked for), then rotation
 __device__ __forceinline__ float ret_qk(const RetArgs& a, const float* __restrict__ x, int d, int pos) {
@@ -79,8 +82,45 @@ __device__ __forceinline__ float ret_qk(const RetArgs& a, const float* __restric
 }
 __device__ __forceinline__ float ret_v(const RetArgs& a, float v) { return a.in_act ? ret_silu(v) : v; }
 
-// (1) U[chunk][head] = sum_j decay^(len-1-j) k_j v_j^T.  4 x 4 outputs per thread; a thread's four columns are vdim/4 apart, so that
-// the threads of a warp read consecutive shared-memory words.
+__device__ __forceinline__ float4 ret_ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float ret_at(const float4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+
+// one chunk's keys (and queries) of a head into shared memory, rows dimp apart: a thread takes a rotation pair, whose one sine and cosine serve all it
+// holds (an element a thread took an eighth of the kernels' time for them), or a dimension that is not rotated.  kw: a factor of each row's key, or null.
+__device__ __forceinline__ void ret_load_keys(const RetArgs& a, int row0, int len, int pos0, int h, int dimp, const float* kw, float* ks, float* qs) {
+  const int half = a.in_act ? 0 : min(a.rot_dims, a.dim) >> 1, per = a.dim - half;      // no rotation with an activation
+  for (int it = threadIdx.x; it < len * per; it += blockDim.x) {
+    const int j = it / per, e = it % per;
+    const float* base = a.qkvg + (long long)(row0 + j) * a.ld + h * a.dim;
+    const float w = kw != nullptr ? kw[j] : 1.f;
+    if (e < half) {
+      const int d0 = a.rot_layout == LP_ROT_INTERLEAVED ? 2 * e : e, d1 = a.rot_layout == LP_ROT_INTERLEAVED ? 2 * e + 1 : e + half;
+      float sn, cs;
+      sincosf((float)(pos0 + j) * a.inv_freq[e], &sn, &cs);
+      sn *= a.rot_mscale;
+      cs *= a.rot_mscale;
+      const float k0 = base[a.k_off + d0], k1 = base[a.k_off + d1];
+      ks[j * dimp + d0] = (k0 * cs - k1 * sn) * a.k_scale * w;
+      ks[j * dimp + d1] = (k1 * cs + k0 * sn) * a.k_scale * w;
+      if (qs != nullptr) {
+        const float q0 = base[a.q_off + d0], q1 = base[a.q_off + d1];
+        qs[j * dimp + d0] = q0 * cs - q1 * sn;
+        qs[j * dimp + d1] = q1 * cs + q0 * sn;
+      }
+    } else {
+      const int d = half + e;
+      const float k = base[a.k_off + d];
+      ks[j * dimp + d] = (a.in_act ? ret_silu(k) : k) * a.k_scale * w;
+      if (qs != nullptr) {
+        const float q = base[a.q_off + d];
+        qs[j * dimp + d] = a.in_act ? ret_silu(q) : q;
+      }
+    }
+  }
+}
+
+// (1) U[chunk][head] = sum_j decay^(len-1-j) k_j v_j^T.  4 x 4 outputs per thread (8 x 8 from 16-byte reads: 208 us for 162); a thread's four columns are vdim/4
+// apart, so that the threads of a warp read consecutive shared-memory words.
 __global__ void __launch_bounds__(RET_CHUNK_THREADS)
 retention_chunk_state_kernel(RetArgs a, const int* __restrict__ chunk_seq, const int* __restrict__ chunk_row0, const int* __restrict__ chunk_len,
                              const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0, float* __restrict__ ws) {
@@ -88,19 +128,14 @@ retention_chunk_state_kernel(RetArgs a, const int* __restrict__ chunk_seq, const
   const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
   const int s = chunk_seq[c], row0 = chunk_row0[c], len = chunk_len[c];
   const int pos0 = seq_pos0[s] + (row0 - seq_row0[s]);
-  const int dimp = ((a.dim + 3) & ~3) + 1, vdimp = (a.vdim + 3) & ~3;      // padded rows: whole 4-tiles, odd stride for k
+  const int dimp = ret_dimp<false>(a.dim), vdimp = (a.vdim + 3) & ~3;      // padded rows: whole 4-tiles
   float* kd = dyn_smem;                   // [RET_CHUNK][dimp]
   float* vv = kd + RET_CHUNK * dimp;      // [RET_CHUNK][vdimp]
-  const float dec = a.decay[h];
-  for (int i = tid; i < len * dimp; i += blockDim.x) {
-    const int j = i / dimp, d = i % dimp;
-    float v = 0.f;
-    if (d < a.dim) {
-      const float* kr = a.qkvg + (long long)(row0 + j) * a.ld + a.k_off + h * a.dim;
-      v = ret_qk(a, kr, d, pos0 + j) * a.k_scale * powf(dec, (float)(len - 1 - j));
-    }
-    kd[i] = v;
-  }
+  __shared__ float power[RET_CHUNK];
+  if (tid < len) power[tid] = powf(a.decay[h], (float)(len - 1 - tid));
+  __syncthreads();
+  for (int i = tid; i < len * (dimp - a.dim); i += blockDim.x) kd[i / (dimp - a.dim) * dimp + a.dim + i % (dimp - a.dim)] = 0.f;
+  ret_load_keys(a, row0, len, pos0, h, dimp, power, kd, nullptr);
   for (int i = tid; i < len * vdimp; i += blockDim.x) {
     const int j = i / vdimp, d = i % vdimp;
     vv[i] = d < a.vdim ? ret_v(a, a.qkvg[(long long)(row0 + j) * a.ld + a.v_off + h * a.vdim + d]) : 0.f;
@@ -137,35 +172,54 @@ retention_chunk_state_kernel(RetArgs a, const int* __restrict__ chunk_seq, const
   }
 }
 
-// (2) one thread per state element of a (request, head): ws[chunk] <- state at the chunk's start; the state after the last chunk goes
-// to the slot.  The chunks' own contributions are loaded eight at a time (independent loads) ahead of the dependent multiply-adds.
+// (2) V state elements of a (request, head) a thread: ws[chunk] <- state at the chunk's start; the state after the last chunk goes to the slot.  The
+// chunks' own contributions are loaded SCAN_BATCH at a time, the next ones while these are added up.
 constexpr int SCAN_THREADS = 256, SCAN_BATCH = 8;
+template <int V> struct RetVec;
+template <> struct RetVec<1> { float v[1]; };
+template <> struct alignas(16) RetVec<4> { float v[4]; };
+template <int V>
 __global__ void __launch_bounds__(SCAN_THREADS)
 retention_scan_kernel(RetArgs a, const int* __restrict__ seq_chunk0, const int* __restrict__ chunk_len, const int* __restrict__ seq_pos0,
                       const int* __restrict__ seq_slot, float* __restrict__ ws) {
   const int s = blockIdx.x, h = blockIdx.y;
   const long long hs = (long long)a.dim * a.vdim;
-  const long long i = (long long)blockIdx.z * SCAN_THREADS + threadIdx.x;
+  const long long i = ((long long)blockIdx.z * SCAN_THREADS + threadIdx.x) * V;
   if (i >= hs) return;
   const int c0 = seq_chunk0[s], c1 = seq_chunk0[s + 1];
   const float dec = a.decay[h];
   const float dec_full = powf(dec, (float)RET_CHUNK);
-  float* st = a.state + (long long)seq_slot[s] * a.slot_stride + h * hs + i;
-  float S = seq_pos0[s] == 0 ? 0.f : *st;
+  RetVec<V>* st = reinterpret_cast<RetVec<V>*>(a.state + (long long)seq_slot[s] * a.slot_stride + h * hs + i);
+  RetVec<V> S;
+  if (seq_pos0[s] == 0) {
+#pragma unroll
+    for (int e = 0; e < V; ++e) S.v[e] = 0.f;
+  } else {
+    S = *st;
+  }
   const long long stride = (long long)a.heads * hs;
   float* u = ws + ((long long)c0 * a.heads + h) * hs + i;
-  for (int c = c0; c < c1; c += SCAN_BATCH) {
-    float own[SCAN_BATCH];
+  RetVec<V> own[SCAN_BATCH], next[SCAN_BATCH];
+  auto fetch = [&](RetVec<V>* dst, const float* from, int c) {
 #pragma unroll
-    for (int k = 0; k < SCAN_BATCH; ++k) own[k] = c + k < c1 ? u[k * stride] : 0.f;
+    for (int k = 0; k < SCAN_BATCH; ++k)
+      if (c + k < c1) dst[k] = *reinterpret_cast<const RetVec<V>*>(from + k * stride);
+  };
+  fetch(own, u, c0);
+  for (int c = c0; c < c1; c += SCAN_BATCH) {
+    fetch(next, u + SCAN_BATCH * stride, c + SCAN_BATCH);
 #pragma unroll
     for (int k = 0; k < SCAN_BATCH; ++k) {
       if (c + k < c1) {
         const int len = chunk_len[c + k];
-        u[k * stride] = S;
-        S = fmaf(len == RET_CHUNK ? dec_full : powf(dec, (float)len), S, own[k]);
+        const float f = len == RET_CHUNK ? dec_full : powf(dec, (float)len);
+        *reinterpret_cast<RetVec<V>*>(u + k * stride) = S;
+#pragma unroll
+        for (int e = 0; e < V; ++e) S.v[e] = fmaf(f, S.v[e], own[k].v[e]);
       }
     }
+#pragma unroll
+    for (int k = 0; k < SCAN_BATCH; ++k) own[k] = next[k];
     u += SCAN_BATCH * stride;
   }
   *st = S;
@@ -176,7 +230,8 @@ retention_scan_kernel(RetArgs a, const int* __restrict__ seq_chunk0, const int* 
 // each other's phases took 1.23 ms (4096 tokens, 16 heads): read where it lies (L2, whole lines, eight loads in flight) three CTAs share an
 // SM and it takes 0.46 ms.  4 x 4 outputs per thread.  The line is what leaves three CTAs an SM; whole prompts on both sides (us, staged up to
 // 200 KB, and so): 16 heads of 128, 4096 tokens 1450, 756, 512 tokens 150, 93; 8 heads of 96 286, 203 and 62, 58; 16 of 80 355, 313 and 59, 57; 8 of
-// 128 keys and 64 values 264, 188 and 60, 61.  64 x 64 is staged on both.
+// 128 keys and 64 values 264, 188 and 60, 61.  64 x 64 is staged on both.  WIDE: the same sums in the same order from 16-byte reads, a quarter as many.
+template <bool WIDE>
 __global__ void __launch_bounds__(RET_CHUNK_THREADS)
 retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const int* __restrict__ chunk_row0, const int* __restrict__ chunk_len,
                            const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0, const float* __restrict__ ws, int stage_s) {
@@ -184,7 +239,7 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
   const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
   const int s = chunk_seq[c], row0 = chunk_row0[c], len = chunk_len[c];
   const int pos0 = seq_pos0[s] + (row0 - seq_row0[s]);
-  const int dimp = ((a.dim + 3) & ~3) + 1, vdimp = (a.vdim + 3) & ~3;
+  const int dimp = ret_dimp<WIDE>(a.dim), vdimp = (a.vdim + 3) & ~3;
   float* qs = dyn_smem;                        // [RET_CHUNK][dimp]
   float* ks = qs + RET_CHUNK * dimp;           // [RET_CHUNK][dimp]
   float* vv = ks + RET_CHUNK * dimp;           // [RET_CHUNK][vdimp]
@@ -193,17 +248,8 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
   float* rr = pp + RET_CHUNK * (RET_CHUNK + 1);   // [RET_CHUNK]
   float* Ss = rr + RET_CHUNK;                  // [dim][vdimp] when stage_s
   const float dec = a.decay[h];
-  for (int i = tid; i < RET_CHUNK * dimp; i += blockDim.x) {
-    const int j = i / dimp, d = i % dimp;
-    float qv = 0.f, kv = 0.f;
-    if (j < len && d < a.dim) {
-      const float* base = a.qkvg + (long long)(row0 + j) * a.ld + h * a.dim;
-      qv = ret_qk(a, base + a.q_off, d, pos0 + j);
-      kv = ret_qk(a, base + a.k_off, d, pos0 + j) * a.k_scale;
-    }
-    qs[i] = qv;
-    ks[i] = kv;
-  }
+  for (int i = len * dimp + tid; i < RET_CHUNK * dimp; i += blockDim.x) qs[i] = ks[i] = 0.f;
+  ret_load_keys(a, row0, len, pos0, h, dimp, nullptr, ks, qs);
   for (int i = tid; i < RET_CHUNK * vdimp; i += blockDim.x) {
     const int j = i / vdimp, d = i % vdimp;
     vv[i] = (j < len && d < a.vdim) ? ret_v(a, a.qkvg[(long long)(row0 + j) * a.ld + a.v_off + h * a.vdim + d]) : 0.f;
@@ -219,6 +265,20 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
   for (int tile = tid; tile < (RET_CHUNK / 2) * (RET_CHUNK / 2); tile += blockDim.x) {
     const int i0 = (tile / (RET_CHUNK / 2)) * 2, tj = tile % (RET_CHUNK / 2);
     float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+    if constexpr (WIDE) {
+#pragma unroll 2
+      for (int d = 0; d < a.dim; d += 4) {
+        const float4 qa = ret_ld4(qs + i0 * dimp + d), qb = ret_ld4(qs + (i0 + 1) * dimp + d), ka = ret_ld4(ks + tj * dimp + d),
+                     kb = ret_ld4(ks + (tj + RET_CHUNK / 2) * dimp + d);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          acc[0][0] = fmaf(ret_at(qa, e), ret_at(ka, e), acc[0][0]);
+          acc[0][1] = fmaf(ret_at(qa, e), ret_at(kb, e), acc[0][1]);
+          acc[1][0] = fmaf(ret_at(qb, e), ret_at(ka, e), acc[1][0]);
+          acc[1][1] = fmaf(ret_at(qb, e), ret_at(kb, e), acc[1][1]);
+        }
+      }
+    } else {
 #pragma unroll 8
     for (int d = 0; d < a.dim; ++d) {
       float q2[2], k2[2];
@@ -231,6 +291,7 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
       for (int p = 0; p < 2; ++p)
 #pragma unroll
         for (int q = 0; q < 2; ++q) acc[p][q] = fmaf(q2[p], k2[q], acc[p][q]);
+    }
     }
 #pragma unroll
     for (int p = 0; p < 2; ++p)
@@ -249,6 +310,23 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
     for (int p = 0; p < 4; ++p)
 #pragma unroll
       for (int q = 0; q < 4; ++q) acc[p][q] = 0.f;
+    if constexpr (WIDE) {      // four neighbouring columns a thread
+      const float* from = (stage_s ? Ss : S) + ty * 4;
+#pragma unroll 2
+      for (int d = 0; d < a.dim; d += 4) {
+        float4 q4[4], s4[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s4[e] = ret_ld4(from + (d + e) * a.vdim);
+#pragma unroll
+        for (int p = 0; p < 4; ++p) q4[p] = ret_ld4(qs + (i0 + p) * dimp + d);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int p = 0; p < 4; ++p)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[p][q] = fmaf(ret_at(q4[p], e), ret_at(s4[e], q), acc[p][q]);
+      }
+    } else {
 #pragma unroll 8
     for (int d = 0; d < a.dim; ++d) {
       float q4[4], s4[4];
@@ -263,6 +341,7 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
 #pragma unroll
         for (int q = 0; q < 4; ++q) acc[p][q] = fmaf(q4[p], s4[q], acc[p][q]);
     }
+    }
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
       const float sc = powf(dec, (float)(i0 + p + 1));
@@ -275,7 +354,11 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
 #pragma unroll
       for (int p = 0; p < 4; ++p) {
         p4[p] = pp[(i0 + p) * (RET_CHUNK + 1) + j];
-        v4[p] = vv[j * vdimp + ty + p * tiles_y];
+        if (!WIDE) v4[p] = vv[j * vdimp + ty + p * tiles_y];
+      }
+      if constexpr (WIDE) {
+        const float4 v = ret_ld4(vv + j * vdimp + ty * 4);
+        v4[0] = v.x; v4[1] = v.y; v4[2] = v.z; v4[3] = v.w;
       }
 #pragma unroll
       for (int p = 0; p < 4; ++p)
@@ -285,7 +368,7 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
 #pragma unroll
     for (int p = 0; p < 4; ++p)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) os[(i0 + p) * vdimp + ty + q * tiles_y] = acc[p][q];
+      for (int q = 0; q < 4; ++q) os[(i0 + p) * vdimp + (WIDE ? ty * 4 + q : ty + q * tiles_y)] = acc[p][q];
   }
   __syncthreads();
   if (a.finish == LP_RET_FINISH_RAW) {      // o itself: what follows it is another kernel's
@@ -321,9 +404,6 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
 // the dim rows, eight of which are in flight at a time: with a column a thread and a row read after the one before was written, the chain of
 // loads took 16 us (8 requests of 16 heads of 128 x 128) and 37 us (64 of 8), whose bytes take 2.6 and 10.
 constexpr int RET_DEC_THREADS = 256, RET_DEC_BATCH = 8;
-template <int V> struct RetVec;
-template <> struct RetVec<1> { float v[1]; };
-template <> struct alignas(16) RetVec<4> { float v[4]; };
 template <int V> __host__ __device__ inline int ret_dec_groups(int vdim) { return vdim / V >= RET_DEC_THREADS ? 1 : RET_DEC_THREADS / (vdim / V); }
 template <int V>
 __global__ void __launch_bounds__(RET_DEC_THREADS)
@@ -862,7 +942,6 @@ static cudaError_t ensure_smem(K kern, size_t bytes, size_t& have) {
   if (e == cudaSuccess) have = bytes;
   return e;
 }
-static size_t g_smem_chunk_state = 48 * 1024, g_smem_chunk_out = 48 * 1024;
 
 static int fill_ret(RetArgs& a, const lp_retention_desc* d) {
   LP_REQUIRE(d != nullptr && d->qkvg != nullptr && d->decay != nullptr && d->state != nullptr && d->out != nullptr,
@@ -909,6 +988,32 @@ extern "C" size_t lp_retention_workspace_bytes(int n_chunks, int heads, int dim,
   return (size_t)n_chunks * heads * dim * vdim * sizeof(float);
 }
 
+static size_t g_smem_chunk_state = 48 * 1024;
+template <bool WIDE>
+static int launch_ret_prefill(const RetArgs& a, int n_seqs, int n_chunks, const int* seq_row0, const int* seq_pos0, const int* seq_slot, const int* seq_chunk0,
+                              const int* chunk_seq, const int* chunk_row0, const int* chunk_len, float* w, cudaStream_t stream) {
+  static size_t have_out = 48 * 1024;
+  const size_t dimp = ret_dimp<WIDE>(a.dim), vdimp = (a.vdim + 3) & ~3;
+  const size_t smem1 = (size_t)RET_CHUNK * (ret_dimp<false>(a.dim) + vdimp) * sizeof(float);
+  size_t smem3 = ((size_t)RET_CHUNK * (2 * dimp + 2 * vdimp) + RET_CHUNK * (RET_CHUNK + 1) + RET_CHUNK) * sizeof(float);
+  LP_REQUIRE(smem3 <= 200 * 1024, "lp_retention_prefill: dim=%d vdim=%d do not fit the chunk kernel's shared memory", a.dim, a.vdim);
+  const int stage_s = smem3 + (size_t)a.dim * vdimp * sizeof(float) <= 64 * 1024;      // three CTAs an SM keep their operands and the chunk's start state
+  if (stage_s) smem3 += (size_t)a.dim * vdimp * sizeof(float);
+  LP_CHECK_CUDA(ensure_smem(retention_chunk_state_kernel, smem1, g_smem_chunk_state));
+  LP_CHECK_CUDA(ensure_smem(retention_chunk_out_kernel<WIDE>, smem3, have_out));
+  retention_chunk_state_kernel<<<dim3(n_chunks, a.heads), RET_CHUNK_THREADS, smem1, stream>>>(a, chunk_seq, chunk_row0, chunk_len, seq_row0, seq_pos0, w);
+  LP_CHECK_CUDA(cudaGetLastError());
+  constexpr int V = WIDE ? 4 : 1;
+  retention_scan_kernel<V><<<dim3(n_seqs, a.heads, (a.dim * a.vdim / V + SCAN_THREADS - 1) / SCAN_THREADS), SCAN_THREADS, 0, stream>>>(
+      a, seq_chunk0, chunk_len, seq_pos0, seq_slot, w);
+  LP_CHECK_CUDA(cudaGetLastError());
+  retention_chunk_out_kernel<WIDE><<<dim3(n_chunks, a.heads), RET_CHUNK_THREADS, smem3, stream>>>(a, chunk_seq, chunk_row0, chunk_len, seq_row0, seq_pos0, w,
+                                                                                                  stage_s);
+  LP_CHECK_CUDA(cudaGetLastError());
+  note_launch(3);
+  return 0;
+}
+
 extern "C" int lp_retention_prefill(const lp_retention_desc* d, int n_seqs, int n_chunks, const int* seq_row0, const int* seq_pos0,
                                     const int* seq_slot, const int* seq_chunk0, const int* chunk_seq, const int* chunk_row0,
                                     const int* chunk_len, void* ws, size_t ws_bytes, void* stream_) {
@@ -920,24 +1025,11 @@ extern "C" int lp_retention_prefill(const lp_retention_desc* d, int n_seqs, int 
   LP_REQUIRE(ws != nullptr && ws_bytes >= lp_retention_workspace_bytes(n_chunks, d->heads, d->dim, d->vdim),
              "lp_retention_prefill: workspace too small");
   float* w = reinterpret_cast<float*>(ws);
-  const size_t dimp = ((d->dim + 3) & ~3) + 1, vdimp = (d->vdim + 3) & ~3;
-  const size_t smem1 = (size_t)RET_CHUNK * (dimp + vdimp) * sizeof(float);
-  size_t smem3 = ((size_t)RET_CHUNK * (2 * dimp + 2 * vdimp) + RET_CHUNK * (RET_CHUNK + 1) + RET_CHUNK) * sizeof(float);
-  LP_REQUIRE(smem3 <= 200 * 1024, "lp_retention_prefill: dim=%d vdim=%d do not fit the chunk kernel's shared memory", d->dim, d->vdim);
-  const int stage_s = smem3 + (size_t)d->dim * vdimp * sizeof(float) <= 64 * 1024;      // three CTAs an SM keep their operands and the chunk's start state
-  if (stage_s) smem3 += (size_t)d->dim * vdimp * sizeof(float);
-  LP_CHECK_CUDA(ensure_smem(retention_chunk_state_kernel, smem1, g_smem_chunk_state));
-  LP_CHECK_CUDA(ensure_smem(retention_chunk_out_kernel, smem3, g_smem_chunk_out));
-  retention_chunk_state_kernel<<<dim3(n_chunks, d->heads), RET_CHUNK_THREADS, smem1, stream>>>(a, chunk_seq, chunk_row0, chunk_len, seq_row0, seq_pos0, w);
-  LP_CHECK_CUDA(cudaGetLastError());
-  retention_scan_kernel<<<dim3(n_seqs, d->heads, (d->dim * d->vdim + SCAN_THREADS - 1) / SCAN_THREADS), SCAN_THREADS, 0, stream>>>(
-      a, seq_chunk0, chunk_len, seq_pos0, seq_slot, w);
-  LP_CHECK_CUDA(cudaGetLastError());
-  retention_chunk_out_kernel<<<dim3(n_chunks, d->heads), RET_CHUNK_THREADS, smem3, stream>>>(a, chunk_seq, chunk_row0, chunk_len, seq_row0, seq_pos0, w,
-                                                                                stage_s);
-  LP_CHECK_CUDA(cudaGetLastError());
-  note_launch(3);
-  return 0;
+  // 16-byte pieces of the operands, the state and the workspace; the wider padding has to fit too
+  const bool wide = d->dim % 8 == 0 && d->vdim % 8 == 0 && d->slot_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(d->state) & 15) == 0 &&
+                    (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && ((size_t)RET_CHUNK * 2 * (d->dim + 4 + d->vdim) + RET_CHUNK * (RET_CHUNK + 2)) * sizeof(float) <= 200 * 1024;
+  return wide ? launch_ret_prefill<true>(a, n_seqs, n_chunks, seq_row0, seq_pos0, seq_slot, seq_chunk0, chunk_seq, chunk_row0, chunk_len, w, stream)
+              : launch_ret_prefill<false>(a, n_seqs, n_chunks, seq_row0, seq_pos0, seq_slot, seq_chunk0, chunk_seq, chunk_row0, chunk_len, w, stream);
 }
 
 template <int V>
