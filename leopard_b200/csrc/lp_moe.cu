@@ -39,6 +39,14 @@ template <typename HT> __device__ __forceinline__ float moe_ld(const HT* p);
 template <> __device__ __forceinline__ float moe_ld<float>(const float* p) { return *p; }
 template <> __device__ __forceinline__ float moe_ld<bf16>(const bf16* p) { return __bfloat162float(*p); }
 
+// eight of a row's values, 16-byte pieces
+__device__ __forceinline__ void moe_ld8(const bf16* p, float* f) { bf16x8_to_f32(*reinterpret_cast<const uint4*>(p), f); }
+__device__ __forceinline__ void moe_ld8(const float* p, float* f) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
+  f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+}
+
 // the largest value of the warp's candidates, the lower index among equals; a lane without a candidate brings index `none`
 __device__ __forceinline__ void warp_best(float& v, int& i, int none) {
 #pragma unroll
@@ -68,18 +76,20 @@ moe_route_kernel(const HT* __restrict__ h, long long ldh, int T, int D, const bf
   const int t = blockIdx.x;
   if (t >= T) return;
   const HT* hr = h + (long long)t * ldh;
-  const bool vec = (D % 8 == 0) && (ldw % 8 == 0) && ((reinterpret_cast<uintptr_t>(w_router) & 15) == 0) &&
+  const bool vec = (D % 8 == 0) && (ldw % 8 == 0) && (ldh % 8 == 0) && (((reinterpret_cast<uintptr_t>(w_router) | reinterpret_cast<uintptr_t>(h)) & 15) == 0) &&
                    (w_gate == nullptr || (reinterpret_cast<uintptr_t>(w_gate) & 15) == 0);
   for (int e = warp; e <= E; e += n_warps) {
     if (e == E && w_gate == nullptr) break;
     const bf16* wr = e < E ? w_router + (long long)e * ldw : w_gate;
     float acc = 0.f;
     if (vec) {
+#pragma unroll 4
       for (int c = lane * 8; c < D; c += 256) {
-        float f[8];
+        float f[8], x[8];
         bf16x8_to_f32(*reinterpret_cast<const uint4*>(wr + c), f);
+        moe_ld8(hr + c, x);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc = fmaf(moe_ld<HT>(hr + c + i), f[i], acc);
+        for (int i = 0; i < 8; ++i) acc = fmaf(x[i], f[i], acc);
       }
     } else {
       for (int c = lane; c < D; c += 32) acc = fmaf(moe_ld<HT>(hr + c), __bfloat162float(wr[c]), acc);

@@ -515,12 +515,24 @@ __device__ __forceinline__ float* lat_cache_row(const LatArgs& a, int seq, int p
   return a.cache + ((long long)page * a.page_size + pos % a.page_size) * (a.kv_rank + a.rot_dim);
 }
 
-__global__ void __launch_bounds__(128)
+// A CTA a row; the row's sines and cosines are taken once for all heads (four a pair and head before: one row of 16 heads 7.0 us).
+constexpr int LAT_PREP_THREADS = 128, LAT_PREP_WIDE = 512, LAT_PREP_ROWS = 296;      // few rows (decoding) take wide CTAs
+__global__ void __launch_bounds__(LAT_PREP_WIDE)
 latent_prep_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos) {
-  __shared__ float red[4];
+  extern __shared__ float dyn_smem[];
+  __shared__ float red[LAT_PREP_WIDE / 32];
   const int r = blockIdx.x, tid = threadIdx.x;
   if (r >= R) return;
-  const int pos = row_pos[r];
+  const int pos = row_pos[r], half = a.rot_dims >> 1;
+  float* s_sin = dyn_smem;             // [half]
+  float* s_cos = dyn_smem + half;      // [half]
+  for (int i = tid; i < half; i += blockDim.x) {
+    float sn, cs;
+    sincosf((float)pos * a.inv_freq[i], &sn, &cs);
+    s_sin[i] = sn * a.rot_mscale;
+    s_cos[i] = cs * a.rot_mscale;
+  }
+  __syncthreads();
   if (a.dkv != nullptr) {      // the layer brings latents of its own
     const float* src = a.dkv + (long long)r * a.lddkv;
     float ss = 0.f;
@@ -529,22 +541,32 @@ latent_prep_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int*
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if ((tid & 31) == 0) red[tid >> 5] = ss;
     __syncthreads();
-    const float inv = 1.0f / sqrtf((red[0] + red[1] + red[2] + red[3]) / (float)a.kv_rank + a.eps);
+    float total = 0.f;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) total += red[w];
+    const float inv = 1.0f / sqrtf(total / (float)a.kv_rank + a.eps);
     float* dst = lat_cache_row(a, row_seq[r], pos);
     for (int c = tid; c < a.kv_rank; c += blockDim.x) dst[c] = src[c] * inv * a.c_gain[c];
-    for (int d = tid; d < a.rot_dim; d += blockDim.x)
-      dst[a.kv_rank + d] = rot_elem(src + a.kv_rank, d, a.rot_dims, a.rot_layout, a.inv_freq, a.rot_mscale, pos);
+    const float* x = src + a.kv_rank;
+    float* y = dst + a.kv_rank;
+    for (int i = tid; i < a.rot_dim - half; i += blockDim.x) {      // a pair, or a dimension that is not rotated
+      if (i < half) {
+        const int d0 = a.rot_layout == LP_ROT_INTERLEAVED ? 2 * i : i, d1 = a.rot_layout == LP_ROT_INTERLEAVED ? 2 * i + 1 : i + half;
+        y[d0] = x[d0] * s_cos[i] - x[d1] * s_sin[i];
+        y[d1] = x[d1] * s_cos[i] + x[d0] * s_sin[i];
+      } else {
+        y[half + i] = x[half + i];
+      }
+    }
   }
-  // the rotated part of every head's query, in place: one thread per pair reads both members, then writes both
+  // the rotated part of every head's query, in place: one thread per pair
   float* q = a.q + (long long)r * a.ldq;
-  const int per = a.dim + a.rot_dim, half = a.rot_dims >> 1;
+  const int per = a.dim + a.rot_dim;
   for (int p = tid; p < a.heads * half; p += blockDim.x) {
     float* x = q + (p / half) * per + a.dim;
     const int i = p % half;
     const int d0 = a.rot_layout == LP_ROT_INTERLEAVED ? 2 * i : i;
     const int d1 = a.rot_layout == LP_ROT_INTERLEAVED ? 2 * i + 1 : i + half;
-    const float u = rot_elem(x, d0, a.rot_dims, a.rot_layout, a.inv_freq, a.rot_mscale, pos);
-    const float v = rot_elem(x, d1, a.rot_dims, a.rot_layout, a.inv_freq, a.rot_mscale, pos);
+    const float u = x[d0] * s_cos[i] - x[d1] * s_sin[i], v = x[d1] * s_cos[i] + x[d0] * s_sin[i];
     x[d0] = u;
     x[d1] = v;
   }
@@ -1060,7 +1082,8 @@ extern "C" int lp_latent_prep(const lp_latent_desc* d, int R, const int* row_seq
   if (int rc = fill_lat(a, d)) return rc;
   LP_REQUIRE((d->dkv == nullptr || d->c_gain != nullptr) && row_seq != nullptr && row_pos != nullptr, "lp_latent_prep: null operand");
   if (R <= 0) return 0;
-  latent_prep_kernel<<<R, 128, 0, stream>>>(a, R, row_seq, row_pos);
+  LP_REQUIRE(d->rot_dims <= 12 * 1024, "lp_latent_prep: rot_dims=%d", d->rot_dims);
+  latent_prep_kernel<<<R, R <= LAT_PREP_ROWS ? LAT_PREP_WIDE : LAT_PREP_THREADS, d->rot_dims * sizeof(float), stream>>>(a, R, row_seq, row_pos);
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
