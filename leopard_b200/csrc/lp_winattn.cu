@@ -151,17 +151,6 @@ window_attn_prep_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const
   if (r >= R) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, n_warps = blockDim.x >> 5;
   const int seq = row_seq[r], pos = row_pos[r];
-  // the row's sines and cosines, once for all heads: one a pair and head took half of the time (4096 rows of 16 heads on 4: 59 us)
-  const int half = a.rot_dims >> 1, vhalf = a.v_inv_freq != nullptr ? a.v_rot_dims >> 1 : 0;
-  float* s_rot = dyn_smem + a.heads + 2 * a.kv_heads + 2;      // [half] sines, [half] cosines, then the values'
-  for (int i = tid; i < half + vhalf; i += blockDim.x) {
-    const bool value = i >= half;
-    float sn, cs;
-    sincosf((float)pos * (value ? a.v_inv_freq[i - half] : a.inv_freq[i]), &sn, &cs);
-    s_rot[i] = value ? sn : sn * a.rot_mscale;
-    s_rot[half + vhalf + i] = value ? cs : cs * a.rot_mscale;
-  }
-  const float* s_cos = s_rot + half + vhalf;
   float* x = a.qkv + (long long)r * a.ld;
   const int kvh = a.kv_shared ? 0 : a.kv_heads;      // key / value heads this row brings (none: they are another layer's)
   const int units = a.heads + kvh;
@@ -215,25 +204,19 @@ window_attn_prep_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const
     }
     __syncthreads();
     if (a.norm_mode == LP_QKNORM_FULL) {
-      if (warp == 0) {
+      if (tid == 0) {
         float tq = 0.f, tk = 0.f;
-        for (int u = lane; u < units; u += 32) (u < a.heads ? tq : tk) += s_ss[u];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          tq += __shfl_xor_sync(0xffffffffu, tq, o);
-          tk += __shfl_xor_sync(0xffffffffu, tk, o);
-        }
-        if (lane == 0) {
-          s_ss[units] = tq;
-          s_ss[units + 1] = tk;
-        }
+        for (int u = 0; u < a.heads; ++u) tq += s_ss[u];
+        for (int u = a.heads; u < units; ++u) tk += s_ss[u];
+        s_ss[units] = tq;
+        s_ss[units + 1] = tk;
       }
       __syncthreads();
     }
   }
-  __syncthreads();      // the sines and cosines are there
   float* crow = win_token_row(a, seq, pos);
   // q and k: per head rot_dims / 2 pairs and dim - rot_dims single dimensions
+  const int half = a.rot_dims >> 1;
   const int per = a.dim - half;
   for (int it = tid; it < units * per; it += blockDim.x) {
     const int u = it / per, e = it % per;
@@ -260,7 +243,10 @@ window_attn_prep_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const
         u0 *= gain[d0];
         u1 *= gain[d1];
       }
-      const float s = s_rot[e], c = s_cos[e];
+      float s, c;
+      sincosf((float)pos * a.inv_freq[e], &s, &c);
+      s *= a.rot_mscale;
+      c *= a.rot_mscale;
       dst[d0] = u0 * c - u1 * s;
       dst[d1] = u1 * c + u0 * s;
     } else {
@@ -271,6 +257,7 @@ window_attn_prep_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const
     }
   }
   // values: rotated over v_rot_dims by their own position when a table is given
+  const int vhalf = a.v_inv_freq != nullptr ? a.v_rot_dims >> 1 : 0;
   const int vrot = 2 * vhalf;
   const int vper = a.vdim - vhalf;
   if (a.v_is_k) return;
@@ -282,7 +269,8 @@ window_attn_prep_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const
     if (e < vhalf) {
       int d0, d1;
       win_pair(a.v_rot_layout, vhalf, e, d0, d1);
-      const float s = s_rot[half + e], c = s_cos[half + e];
+      float s, c;
+      sincosf((float)pos * a.v_inv_freq[e], &s, &c);
       const float u0 = src[d0] * vinv, u1 = src[d1] * vinv;
       dst[d0] = u0 * c - u1 * s;
       dst[d1] = u1 * c + u0 * s;
@@ -1595,7 +1583,7 @@ extern "C" int lp_window_attn_prep(const lp_window_attn_desc* d, int R, const in
   if (int rc = fill_win(a, d, true)) return rc;
   LP_REQUIRE(row_seq != nullptr && row_pos != nullptr, "lp_window_attn_prep: null operand");
   if (R <= 0) return 0;
-  const size_t smem = (size_t)(d->heads + 2 * d->kv_heads + 2 + d->rot_dims + (d->v_inv_freq != nullptr ? d->v_rot_dims : 0)) * sizeof(float);
+  const size_t smem = (size_t)(d->heads + 2 * d->kv_heads + 2) * sizeof(float);
   LP_REQUIRE(smem <= 48 * 1024, "lp_window_attn_prep: too many heads");
   // one row is a CTA: with few rows it should not walk its elements 128 at a time
   const int wide = d->heads * d->dim >= WIN_PREP_WIDE ? WIN_PREP_WIDE : 256;
