@@ -386,6 +386,9 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
   __shared__ int pair_of[STREAM_MAX_PAIRS];
   __shared__ int pair_count[STREAM_MAX_PAIRS / 32];
   constexpr int U = MG >= 4 ? 1 : 2;      // k steps whose weights are in flight together
+  // a warp's steps are neighbours, whole 128-byte lines of the weight rows (one tile: 14.6 us a launch of ronelorn's one-request steps, 13.7 so), or lie n_warps
+  // apart (two tiles, 32.5, 33.4)
+  constexpr bool NEAR = NT == 1;
   constexpr int SLOTS = NT * MG * 4;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
   const int g = lane >> 2, t = lane & 3;
@@ -447,11 +450,10 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[j][i][c] = run[LONG ? j : 0][LONG ? i : 0][c] = 0.f;
     int turn = 0;
-    const int stride = U * n_warps;
     auto fetch = [&](int s, uint4 (&u0)[U][NT], uint4 (&u1)[U][NT]) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int k = (s + u * n_warps) * 32 + t * 8;
+        const int k = (NEAR ? s * U + u : s + u * n_warps) * 32 + t * 8;
 #pragma unroll
         for (int j = 0; j < NT; ++j) {
           u0[u][j] = k < a.K && w0[j] != nullptr ? ldg_once(w0[j] + k) : none;
@@ -462,7 +464,7 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
     auto take = [&](int s, const uint4 (&u0)[U][NT], const uint4 (&u1)[U][NT]) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int k = (s + u * n_warps) * 32 + t * 8;
+        const int k = (NEAR ? s * U + u : s + u * n_warps) * 32 + t * 8;
         if constexpr (sizeof(AT) == 2) {
           uint4 v[MG];
 #pragma unroll
@@ -518,18 +520,19 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
     uint4 a0[U][NT], a1[U][NT];
     // one tile of up to eight bf16 rows leaves registers free: the next steps' weights are asked for before these are used (K = N = 4096, one row: 10.6 us,
     // 8.7 so; two tiles 26.6, 27.4, fp32 rows 4.6, 5.3: their registers cost CTAs)
+    const int stride = NEAR ? n_warps : U * n_warps, steps = NEAR ? (a.K + 32 * U - 1) / (32 * U) : (a.K + 31) / 32;
     if constexpr (MG == 1 && NT == 1 && sizeof(AT) == 2) {
       uint4 b0[U][NT], b1[U][NT];
       fetch(warp, a0, a1);
-      for (int s = warp; s * 32 < a.K; s += 2 * stride) {
+      for (int s = warp; s < steps; s += 2 * stride) {
         fetch(s + stride, b0, b1);
         take(s, a0, a1);
-        if ((s + stride) * 32 >= a.K) break;
+        if (s + stride >= steps) break;
         fetch(s + 2 * stride, a0, a1);
         take(s + stride, b0, b1);
       }
     } else {
-      for (int s = warp; s * 32 < a.K; s += stride) {
+      for (int s = warp; s < steps; s += stride) {
         fetch(s, a0, a1);
         take(s, a0, a1);
       }
