@@ -709,11 +709,15 @@ int lp_split_rows(const float* src, long long ld, int M, int K, void* planes, lo
  * out: 0 bf16, 1 fp32, 2 three planes c_plane elements apart.  K and N multiples of 8, rows on 16-byte boundaries. */
 int lp_gemm_split(const void* A, long long lda, long long a_plane, const void* W, long long ldw, void* C, long long ldc, long long c_plane,
                   int out, int M, int N, int K, const float* bias, void* stream);
-/* The products of sorted (token, expert) rows on the tcgen05 tensor cores: rows of A (bf16, n_tiles * 128 of them) in tiles of 128 that belong to weight
- * group tile_group[tile] (device, < 0: an empty tile, whose rows of C are not written; lp_moe_align with tile_rows = 128), group g's weight [N, K] at W + g w_group.
- * gated != 0: W holds N / 2 rows of gates and as many others, C [rows, N / 2] = silu(row_scale * gate) * (row_scale * other); else C [rows, N]. */
-int lp_gemm_grouped(const void* A, long long lda, const void* W, long long ldw, long long w_group, int groups, const int* tile_group, int n_tiles,
-                    int gated, const float* row_scale, void* C, long long ldc, int out_fp32, int N, int K, void* stream);
+/* the same from fp32 rows; terms: room for 3 M K bf16 */
+int lp_linear_split(const float* A, long long lda, const void* W, long long ldw, void* C, long long ldc, int out, int M, int N, int K, const float* bias,
+                    void* terms, void* stream);
+/* The products of sorted (token, expert) rows on the tcgen05 tensor cores: rows of A (n_tiles * 128 of them; bf16, or with a_plane > 0 fp32 in three planes) in
+ * tiles of 128 that belong to weight group tile_group[tile] (device, < 0: an empty tile, whose rows of C are not written; lp_moe_align with tile_rows = 128), group
+ * g's weight [N, K] at W + g w_group.  gated != 0: W holds N / 2 rows of gates and as many others, C [rows, N / 2] = silu(row_scale * gate) * (row_scale * other);
+ * else C [rows, N].  out as for lp_gemm_split. */
+int lp_gemm_grouped(const void* A, long long lda, long long a_plane, const void* W, long long ldw, long long w_group, int groups, const int* tile_group,
+                    int n_tiles, int gated, const float* row_scale, void* C, long long ldc, long long c_plane, int out, int N, int K, void* stream);
 /* Latent attention of prompts with every head's keys and values expanded, on the tensor cores: heads of 128 + 64 rotated channels, values of
  * 128, kv_rank a multiple of 8.  desc as for lp_latent_prep, whose results (rotated queries, this step's cache rows) it reads; w_kv bf16
  * [2 * heads * 128, kv_rank], rows ldw elements apart: the heads' key rows, then their value rows.  seq_row0 [n_seqs + 1], seq_pos0 [n_seqs]:

@@ -149,23 +149,33 @@ struct Gemm32Args {
   long long lda, a_plane;
   const bf16* W;
   long long ldw;
+  long long w_group;          // between the weights of groups
   const int* tile_group;      // [n_tiles_m] weight group of each row tile (< 0: an empty tile), or null
   const float* row_scale;     // [M] multiplies a gated unit's products, or null
 };
 
 // An infinite weight times a term that is zero, or of the other sign, is a NaN that the product of the uncut number is not: outputs that came out NaN
 // are taken again in fp32 multiply-adds (by the thread that wrote them)
-__device__ __noinline__ void gemm32_mend(const Gemm32Args& a, int row, int col0, int cols) {
+__device__ float gemm32_plain(const Gemm32Args& a, int row, const bf16* w) {
+  const bf16* x = a.A + (long long)row * a.lda;
+  float s = 0.f;
 #pragma unroll 1
-  for (int c = col0; c < col0 + cols && c < a.N; ++c) {
+  for (int k = 0; k < a.K && s == s; ++k) s = fmaf(s32_value(x + k, a.a_plane), (float)w[k], s);
+  return s;
+}
+__device__ __forceinline__ float gemm32_gated(float z, float u, float rs) {
+  z *= rs;
+  return z / (1.0f + expf(-z)) * (u * rs);
+}
+__device__ __noinline__ void gemm32_mend(const Gemm32Args& a, int row, int group, int col0, int cols, int gated) {
+  const bf16* W = a.W + (long long)group * a.w_group;
+#pragma unroll 1
+  for (int c = col0; c < col0 + cols && c < (gated ? a.N / 2 : a.N); ++c) {
     const long long at = (long long)row * a.ldc + c;
     const float was = a.out == G32_OUT_F32 ? reinterpret_cast<const float*>(a.C)[at] : (float)reinterpret_cast<const bf16*>(a.C)[at];
     if (was == was) continue;
-    const bf16* x = a.A + (long long)row * a.lda;
-    const bf16* w = a.W + (long long)c * a.ldw;
-    float s = 0.f;
-#pragma unroll 1
-    for (int k = 0; k < a.K && s == s; ++k) s = fmaf(s32_value(x + k, a.a_plane), (float)w[k], s);
+    float s = gemm32_plain(a, row, W + (long long)c * a.ldw);
+    if (gated) s = gemm32_gated(s, gemm32_plain(a, row, W + (long long)(c + a.N / 2) * a.ldw), a.row_scale != nullptr ? a.row_scale[row] : 1.f);
     if (a.bias != nullptr) s += a.bias[c];
     if (a.out == G32_OUT_F32) {
       reinterpret_cast<float*>(a.C)[at] = s;
@@ -320,6 +330,7 @@ gemm32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
         mbar_arrive(acc_empty + b);
       }
       if (row < a.M) {
+        bool odd = false;
         if (GATED) {
           const float rs = a.row_scale != nullptr ? a.row_scale[row] : 1.f;
 #pragma unroll
@@ -329,8 +340,8 @@ gemm32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
               float v[8];
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
-                const float z = acc[g * 8 + i] * rs;
-                v[i] = z / (1.0f + expf(-z)) * (acc[COLS / 2 + g * 8 + i] * rs);
+                v[i] = gemm32_gated(acc[g * 8 + i], acc[COLS / 2 + g * 8 + i], rs);
+                if (PLANES == 3) odd |= v[i] != v[i];
               }
               const long long at = (long long)row * a.ldc + col;
               if (a.out == G32_OUT_F32) {
@@ -346,7 +357,6 @@ gemm32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
             }
           }
         } else {
-          bool odd = false;
 #pragma unroll
           for (int g = 0; g < BN / 16; ++g) {
             const int col = n0 + g * 8;
@@ -373,8 +383,8 @@ gemm32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
               }
             }
           }
-          if (PLANES == 3 && odd) gemm32_mend(a, row, n0, BN / 2);
         }
+        if (PLANES == 3 && odd) gemm32_mend(a, row, group_of(tile), n0, COLS / 2, GATED);
       }
     }
   }
@@ -956,6 +966,7 @@ static int launch_gemm32(Gemm32Args a, int groups, long long w_group, cudaStream
   if (int rc = make_tmap_bf16_3d(&tw, a.W, a.K, a.N, groups, a.ldw, w_group, 64, GATED ? 64 : BN, 1)) return rc;
   a.n_tiles_m = (a.M + 127) / 128;
   a.n_tiles_n = ((GATED ? a.N / 2 : a.N) + cols - 1) / cols;
+  a.w_group = w_group;
   const int tiles = a.n_tiles_m * a.n_tiles_n;
   kern<<<tiles < sm_count() ? tiles : sm_count(), G32_THREADS, S::TOTAL, stream>>>(ta, tw, a);
   note_launch();
@@ -986,6 +997,12 @@ extern "C" int lp_gemm_split(const void* A, long long lda, long long a_plane, co
   return gemm32(a, reinterpret_cast<cudaStream_t>(stream_));
 }
 
+extern "C" int lp_linear_split(const float* A, long long lda, const void* W, long long ldw, void* C, long long ldc, int out, int M, int N, int K,
+                               const float* bias, void* terms, void* stream) {
+  if (int rc = lp_split_rows(A, lda, M, K, terms, K, (long long)M * K, stream)) return rc;
+  return lp_gemm_split(terms, K, (long long)M * K, W, ldw, C, ldc, 0, out, M, N, K, bias, stream);
+}
+
 template <int NR>
 static int launch_attn32(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tr, const CUtensorMap& tv, const Attn32Args& a, int heads,
                          int n_tiles, cudaStream_t stream) {
@@ -1002,21 +1019,24 @@ static int launch_attn32(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
   return 0;
 }
 
-extern "C" int lp_gemm_grouped(const void* A, long long lda, const void* W, long long ldw, long long w_group, int groups, const int* tile_group, int n_tiles,
-                               int gated, const float* row_scale, void* C, long long ldc, int out_fp32, int N, int K, void* stream_) {
+extern "C" int lp_gemm_grouped(const void* A, long long lda, long long a_plane, const void* W, long long ldw, long long w_group, int groups,
+                               const int* tile_group, int n_tiles, int gated, const float* row_scale, void* C, long long ldc, long long c_plane, int out, int N,
+                               int K, void* stream_) {
   LP_REQUIRE(A != nullptr && W != nullptr && C != nullptr && tile_group != nullptr, "lp_gemm_grouped: null operand");
-  LP_REQUIRE(K >= 8 && K % 8 == 0 && N % 16 == 0 && groups > 0 && lda % 8 == 0 && ldw % 8 == 0 && w_group % 8 == 0 && ldc % (out_fp32 ? 4 : 8) == 0 &&
-                 aligned16(A) && aligned16(W) && aligned16(C),
+  LP_REQUIRE(out >= G32_OUT_BF16 && out <= G32_OUT_PLANES, "lp_gemm_grouped: unknown output form %d", out);
+  LP_REQUIRE(K >= 8 && K % 8 == 0 && N % 16 == 0 && groups > 0 && lda % 8 == 0 && a_plane % 8 == 0 && ldw % 8 == 0 && w_group % 8 == 0 &&
+                 ldc % (out == G32_OUT_F32 ? 4 : 8) == 0 && c_plane % 8 == 0 && aligned16(A) && aligned16(W) && aligned16(C),
              "lp_gemm_grouped: 16-byte rows of whole eights");
   LP_REQUIRE(gated || row_scale == nullptr, "lp_gemm_grouped: a row scale comes with a gated unit");
   if (n_tiles <= 0 || N <= 0) return 0;
   Gemm32Args a = {};
   a.M = n_tiles * 128; a.N = N; a.K = K;
-  a.C = C; a.ldc = ldc; a.out = out_fp32 ? G32_OUT_F32 : G32_OUT_BF16;
-  a.A = reinterpret_cast<const bf16*>(A); a.lda = lda;
+  a.C = C; a.ldc = ldc; a.c_plane = c_plane; a.out = out;
+  a.A = reinterpret_cast<const bf16*>(A); a.lda = lda; a.a_plane = a_plane;
   a.W = reinterpret_cast<const bf16*>(W); a.ldw = ldw;
   a.tile_group = tile_group; a.row_scale = row_scale;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  if (a_plane > 0) return gated ? launch_gemm32<256, 3, true>(a, groups, w_group, stream) : launch_gemm32<256, 3, false>(a, groups, w_group, stream);
   return gated ? launch_gemm32<256, 1, true>(a, groups, w_group, stream) : launch_gemm32<256, 1, false>(a, groups, w_group, stream);
 }
 

@@ -45,12 +45,12 @@ SPLIT_MIN_ROWS, SPLIT_MIN_K = 65, 64
 # its tiles are 128 rows of one request.  A layer of width 1024 with 8 heads (us, lp_latent_attend_tiles and this one): one request of 20 rows 64, 45, of
 # 500 297, 85; 32 requests of 12 rows 92, 81; 64 of 12 97, 120, of 24 132, 126; width 2048, 16 heads: 4096 rows 6,490, 530; 64 requests of 12 rows 225, 205.
 EXPAND_TILES, EXPAND_TILE_ROWS = 32, 24
-# Window attention of prompts goes to lp_window_attn_prompt (128 rows of a request and a head a CTA) where its tiles are filled, or where there is one
-# CTA an SM at most.  A layer, preparation included (us, lp_window_attn_tiles and this one; heads on a quarter of key / value heads): one request of 20 rows,
-# 8 heads 29, 22; of 500 86, 45; of 4096, 16 heads 845, 302; 16 requests of 20, 8 heads 32, 29, 16 heads 35, 42; 16 of 40, 16 heads 40, 54; 32 of 12, 4 heads 27,
-# 32.  Capped scores and values turned back by position cost it more (a table, tanh, an exchange): one request of 128 rows, 16 heads 51, 58; of 500, 4 heads
-# 72, 74, 8 heads 102, 76; of 4096, 16 heads 1009, 417.
-WINDOW_TILE_ROWS, WINDOW_FEW_ROWS, WINDOW_CAP_ROWS, WINDOW_CAP_WORK = 64, 20, 300, 4000
+# Window attention of prompts goes to lp_window_attn_prompt (128 rows of a request and a head a CTA) where its tiles are filled and it saves more than its launches
+# cost the host.  A layer, preparation included (us, lp_window_attn_tiles and this one; heads on a quarter of key / value heads): one request of 128 rows, 8
+# heads 34, 27; of 500 86, 45; of 4096, 16 heads 845, 302; 16 requests of 20, 16 heads 35, 42; of 40 40, 54.  Capped scores and values turned back
+# by position cost it more (a table, tanh, an exchange): one request of 128 rows, 16 heads 51, 58; of 500, 4 heads 72, 74, 8 heads 102, 76; of 4096, 16 heads 1009,
+# 417.
+WINDOW_TILE_ROWS, WINDOW_ROWS, WINDOW_CAP_WORK = 64, 200, 4000
 # Up to MOE_PAIRS_MAX (token, choice) pairs an expert's weights are streamed once for the pairs that chose it.  Both products of 16 experts,
 # width 2048, 1024 inside (us, bf16; fp32 rows), against sorted tiles: 128 pairs 66, 108; 85, 182.  256 pairs 93, 108; 138, 182.  512 pairs 161,
 # 108; 282, 182: with this few experts the sorted tiles are ahead from about 300 pairs, with 32 (width 4096) not yet at 512: 554, 683; 876, 1116.
@@ -895,8 +895,7 @@ class SeqLMEngine:
         self.tile_rows = int(self.L.lp_linear_tile_rows())
         # large bf16 products of the serving precision go to the tcgen05 GEMM when the library has it (the native ones do)
         self.tensor_core_rows = TENSOR_CORE_MIN_ROWS if dtype == "bfloat16" and hasattr(self.L, "lp_gemm_bf16") else None
-        self.sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count if self.device.type == "cuda" else 1
-        self.split_rows = SPLIT_MIN_ROWS if hasattr(self.L, "lp_gemm_split") and self.device.type == "cuda" else None
+        self.split_rows = SPLIT_MIN_ROWS if hasattr(self.L, "lp_linear_split") and self.device.type == "cuda" else None
         self.tap: Optional[Callable[[int, torch.Tensor], None]] = None   # called with (layer, residual stream) after every layer
         # decode steps are launch-bound: a batch layout (requests, page-table width) that comes back is captured into a CUDA graph on
         # its second appearance and replayed from then on; only the index tables change between replays (LEOPARD_DECODE_GRAPH=0: off)
@@ -937,11 +936,9 @@ class SeqLMEngine:
     def _split_product(self, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias) -> None:
         M, K = a.shape
         terms = self._empty((3, M, K), BF16)
-        rc = self.L.lp_split_rows(_lib.ptr(a), a.stride(0), M, K, _lib.ptr(terms), K, M * K, self._stream())
-        self._check(rc, "lp_split_rows")
-        rc = self.L.lp_gemm_split(_lib.ptr(terms), K, M * K, _lib.ptr(w), w.stride(0), _lib.ptr(out), out.stride(0), 0,
-                                  _lib.GEMM_SPLIT_F32 if out.dtype == F32 else _lib.GEMM_SPLIT_BF16, M, w.shape[0], K, _lib.ptr(bias), self._stream())
-        self._check(rc, "lp_gemm_split")
+        rc = self.L.lp_linear_split(_lib.ptr(a), a.stride(0), _lib.ptr(w), w.stride(0), _lib.ptr(out), out.stride(0),
+                                    _lib.GEMM_SPLIT_F32 if out.dtype == F32 else _lib.GEMM_SPLIT_BF16, M, w.shape[0], K, _lib.ptr(bias), _lib.ptr(terms), self._stream())
+        self._check(rc, "lp_linear_split")
 
     def linear(self, a: torch.Tensor, w: torch.Tensor, out_dtype, epi=_lib.EPI_NONE, epi_a=0.0, epi_b=0.0, out=None, into=None, bias=None,
                row_scale=None):
@@ -1246,10 +1243,7 @@ class SeqLMEngine:
                 or qkv.stride(0) % 4 or qkv.data_ptr() % 16 or o.data_ptr() % 16 or o.stride(0) % (4 if o.dtype == F32 else 8)):
             return False
         tiles = sum(-(-ln // 128) for ln in b.lens)
-        if d.softcap > 0 or d.v_inv_freq:
-            pays = b.R >= WINDOW_TILE_ROWS * tiles and b.R >= WINDOW_CAP_ROWS and b.R * m.heads >= WINDOW_CAP_WORK
-        else:
-            pays = b.R >= WINDOW_TILE_ROWS * tiles or (b.R >= WINDOW_FEW_ROWS * tiles and tiles * m.heads <= self.sm_count)
+        pays = b.R >= WINDOW_ROWS and b.R >= WINDOW_TILE_ROWS * tiles and ((d.softcap <= 0 and not d.v_inv_freq) or b.R * m.heads >= WINDOW_CAP_WORK)
         if not pays:
             return False
 
@@ -1464,7 +1458,7 @@ class SeqLMEngine:
         w_gu, w_dn = lw["w_gu"], lw["w_edown"]
         # rows enough to fill tensor-core tiles in the serving precision: an expert's rows are gathered into tiles of its own and all experts' products are
         # one launch, without a look at the tables on the host
-        grouped = (self.tensor_core_rows is not None and n_pairs >= f.experts * self.tensor_core_rows and h.dtype == BF16 and epi == _lib.EPI_SILU_GATE
+        grouped = (self.split_rows is not None and n_pairs >= f.experts * TENSOR_CORE_MIN_ROWS and epi == _lib.EPI_SILU_GATE
                    and hasattr(L, "lp_gemm_grouped") and D % 16 == 0 and f.expert_ff % 8 == 0 and all(t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (w_gu, w_dn)))
         tile_rows = GROUP_TILE_ROWS if grouped else self.tile_rows
         tiles = int(L.lp_moe_max_tiles(n_pairs, f.experts, tile_rows))
@@ -1479,14 +1473,21 @@ class SeqLMEngine:
         if on_input:      # the pairs' weights in the sorted row space
             scale = torch.zeros((rows,), dtype=F32, device=self.device)      # padding rows of the sorted space stay zero
             self._check(L.lp_moe_sorted_weights(_lib.ptr(pair_row), _lib.ptr(wts), n_pairs, _lib.ptr(scale), st), "lp_moe_sorted_weights")
-        h1 = self._empty((rows, f.expert_ff), self.act)
         y = self._empty((rows, D), F32)
+        if not grouped or h.dtype == BF16:
+            h1 = self._empty((rows, f.expert_ff), self.act)
         if grouped:
-            a_sorted = h.index_select(0, sorted_token.clamp_min(0))
-            for a, w, c, n, k, gated in ((a_sorted, w_gu, h1, 2 * f.expert_ff, D, 1), (h1, w_dn, y, D, f.expert_ff, 0)):
-                rc = L.lp_gemm_grouped(_lib.ptr(a), a.stride(0), _lib.ptr(w), w.stride(1), w.stride(0), f.experts, _lib.ptr(tile_group), tiles, gated,
-                                       _lib.ptr(scale) if gated else None, _lib.ptr(c), c.stride(0), int(c.dtype == F32), n, k, st)
-                self._check(rc, "lp_gemm_grouped")
+            a, plane, plane1, form = h.index_select(0, sorted_token.clamp_min(0)), 0, 0, _lib.GEMM_SPLIT_BF16
+            if h.dtype == F32:      # three bf16 terms each, the inner rows as the first product's store makes them
+                terms, plane, plane1, form = self._empty((3, rows, D), BF16), rows * D, rows * f.expert_ff, _lib.GEMM_SPLIT_PLANES
+                self._check(L.lp_split_rows(_lib.ptr(a), a.stride(0), rows, D, _lib.ptr(terms), D, plane, st), "lp_split_rows")
+                a, h1 = terms, self._empty((3, rows, f.expert_ff), BF16)
+            rc = L.lp_gemm_grouped(_lib.ptr(a), D, plane, _lib.ptr(w_gu), w_gu.stride(1), w_gu.stride(0), f.experts, _lib.ptr(tile_group), tiles, 1,
+                                   _lib.ptr(scale), _lib.ptr(h1), f.expert_ff, plane1, form, 2 * f.expert_ff, D, st)
+            self._check(rc, "lp_gemm_grouped")
+            rc = L.lp_gemm_grouped(_lib.ptr(h1), f.expert_ff, plane1, _lib.ptr(w_dn), w_dn.stride(1), w_dn.stride(0), f.experts, _lib.ptr(tile_group), tiles, 0,
+                                   None, _lib.ptr(y), D, 0, _lib.GEMM_SPLIT_F32, D, f.expert_ff, st)
+            self._check(rc, "lp_gemm_grouped")
             return self._moe_combine(f, lw, h, y, pair_row, None if on_input else wts, gate)
         capturing = self.device.type == "cuda" and torch.cuda.is_current_stream_capturing()      # no host read inside a graph
         if self.tensor_core_rows is not None and n_pairs >= f.experts * self.tensor_core_rows and h.dtype == BF16 and not capturing:

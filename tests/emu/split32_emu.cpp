@@ -43,13 +43,18 @@ extern "C" void emu_gemm_split(const void* A, long long lda, long long a_plane, 
   else run_gemm<128, 3, false>(a, ctas, 1, 0);
 }
 
-extern "C" void emu_gemm_grouped(const void* A, const void* W, int groups, const int* tile_group, int n_tiles, int gated, const float* row_scale, void* C,
-                                 int out_fp32, int N, int K, int ctas) {
+extern "C" void emu_gemm_grouped(const void* A, long long a_plane, const void* W, int groups, const int* tile_group, int n_tiles, int gated,
+                                 const float* row_scale, void* C, long long c_plane, int out, int N, int K, int ctas) {
   Gemm32Args a = {};
-  a.M = n_tiles * 128; a.N = N; a.K = K; a.C = C; a.ldc = gated ? N / 2 : N; a.out = out_fp32;
-  a.A = (const bf16*)A; a.lda = K; a.W = (const bf16*)W; a.ldw = K; a.tile_group = tile_group; a.row_scale = row_scale;
-  if (gated) run_gemm<256, 1, true>(a, ctas, groups, (long long)N * K);
-  else run_gemm<256, 1, false>(a, ctas, groups, (long long)N * K);
+  a.M = n_tiles * 128; a.N = N; a.K = K; a.C = C; a.ldc = gated ? N / 2 : N; a.out = out; a.c_plane = c_plane; a.w_group = (long long)N * K;
+  a.A = (const bf16*)A; a.lda = K; a.a_plane = a_plane; a.W = (const bf16*)W; a.ldw = K; a.tile_group = tile_group; a.row_scale = row_scale;
+  if (a_plane > 0) {
+    if (gated) run_gemm<256, 3, true>(a, ctas, groups, a.w_group);
+    else run_gemm<256, 3, false>(a, ctas, groups, a.w_group);
+  } else {
+    if (gated) run_gemm<256, 1, true>(a, ctas, groups, a.w_group);
+    else run_gemm<256, 1, false>(a, ctas, groups, a.w_group);
+  }
 }
 
 // q planes [3][R][heads * DQ], k and v planes [3][n_keys][heads / ratio * 128], kr planes [3][n_keys][64] or null
