@@ -89,34 +89,54 @@ __device__ __forceinline__ float ret_at(const float4& v, int i) { return i == 0 
 // holds (an element a thread took an eighth of the kernels' time for them), or a dimension that is not rotated.  kw: a factor of each row's key, or null.
 __device__ __forceinline__ void ret_load_keys(const RetArgs& a, int row0, int len, int pos0, int h, int dimp, const float* kw, float* ks, float* qs) {
   const int half = a.in_act ? 0 : min(a.rot_dims, a.dim) >> 1, per = a.dim - half;      // no rotation with an activation
-  for (int it = threadIdx.x; it < len * per; it += blockDim.x) {
-    const int j = it / per, e = it % per;
-    const float* base = a.qkvg + (long long)(row0 + j) * a.ld + h * a.dim;
-    const float w = kw != nullptr ? kw[j] : 1.f;
-    if (e < half) {
-      const int d0 = a.rot_layout == LP_ROT_INTERLEAVED ? 2 * e : e, d1 = a.rot_layout == LP_ROT_INTERLEAVED ? 2 * e + 1 : e + half;
-      float sn, cs;
-      sincosf((float)(pos0 + j) * a.inv_freq[e], &sn, &cs);
-      sn *= a.rot_mscale;
-      cs *= a.rot_mscale;
-      const float k0 = base[a.k_off + d0], k1 = base[a.k_off + d1];
-      ks[j * dimp + d0] = (k0 * cs - k1 * sn) * a.k_scale * w;
-      ks[j * dimp + d1] = (k1 * cs + k0 * sn) * a.k_scale * w;
-      if (qs != nullptr) {
-        const float q0 = base[a.q_off + d0], q1 = base[a.q_off + d1];
-        qs[j * dimp + d0] = q0 * cs - q1 * sn;
-        qs[j * dimp + d1] = q1 * cs + q0 * sn;
-      }
-    } else {
-      const int d = half + e;
-      const float k = base[a.k_off + d];
-      ks[j * dimp + d] = (a.in_act ? ret_silu(k) : k) * a.k_scale * w;
-      if (qs != nullptr) {
-        const float q = base[a.q_off + d];
-        qs[j * dimp + d] = a.in_act ? ret_silu(q) : q;
+  constexpr int BATCH = 4;      // what a batch reads is asked for before any of it is stored
+  for (int it0 = threadIdx.x; it0 < len * per; it0 += BATCH * blockDim.x) {
+    float k0[BATCH], k1[BATCH], q0[BATCH], q1[BATCH];
+#pragma unroll
+    for (int n = 0; n < BATCH; ++n) {
+      const int it = it0 + n * blockDim.x, j = it / per, e = it % per;
+      if (it >= len * per) break;
+      const float* base = a.qkvg + (long long)(row0 + j) * a.ld + h * a.dim;
+      const int d0 = e >= half ? half + e : a.rot_layout == LP_ROT_INTERLEAVED ? 2 * e : e, d1 = e >= half ? d0 : a.rot_layout == LP_ROT_INTERLEAVED ? 2 * e + 1 : e + half;
+      k0[n] = base[a.k_off + d0];
+      k1[n] = base[a.k_off + d1];
+      q0[n] = qs != nullptr ? base[a.q_off + d0] : 0.f;
+      q1[n] = qs != nullptr ? base[a.q_off + d1] : 0.f;
+    }
+#pragma unroll
+    for (int n = 0; n < BATCH; ++n) {
+      const int it = it0 + n * blockDim.x, j = it / per, e = it % per;
+      if (it >= len * per) break;
+      const float w = kw != nullptr ? kw[j] : 1.f;
+      if (e < half) {
+        const int d0 = a.rot_layout == LP_ROT_INTERLEAVED ? 2 * e : e, d1 = a.rot_layout == LP_ROT_INTERLEAVED ? 2 * e + 1 : e + half;
+        float sn, cs;
+        sincosf((float)(pos0 + j) * a.inv_freq[e], &sn, &cs);
+        sn *= a.rot_mscale;
+        cs *= a.rot_mscale;
+        ks[j * dimp + d0] = (k0[n] * cs - k1[n] * sn) * a.k_scale * w;
+        ks[j * dimp + d1] = (k1[n] * cs + k0[n] * sn) * a.k_scale * w;
+        if (qs != nullptr) {
+          qs[j * dimp + d0] = q0[n] * cs - q1[n] * sn;
+          qs[j * dimp + d1] = q1[n] * cs + q0[n] * sn;
+        }
+      } else {
+        ks[j * dimp + half + e] = (a.in_act ? ret_silu(k0[n]) : k0[n]) * a.k_scale * w;
+        if (qs != nullptr) qs[j * dimp + half + e] = a.in_act ? ret_silu(q0[n]) : q0[n];
       }
     }
   }
+}
+// `len` rows of vdim columns from column `off` of the projection on, rows ldd apart, copied while other work is done (the caller commits and waits);
+// false: rows are not whole 16-byte pieces, nothing was copied
+__device__ __forceinline__ bool ret_copy_rows(const RetArgs& a, int row0, int len, int off, float* dst, int ldd) {
+  if (((a.ld | off | a.vdim | ldd) & 3) != 0 || (reinterpret_cast<uintptr_t>(a.qkvg) & 15) != 0) return false;
+  const int per = a.vdim >> 2;
+  for (int i = threadIdx.x; i < len * per; i += blockDim.x) {
+    const int j = i / per, c = (i % per) * 4;
+    __pipeline_memcpy_async(dst + j * ldd + c, a.qkvg + (long long)(row0 + j) * a.ld + off + c, 16);
+  }
+  return true;
 }
 
 // (1) U[chunk][head] = sum_j decay^(len-1-j) k_j v_j^T.  4 x 4 outputs per thread (8 x 8 from 16-byte reads: 208 us for 162); a thread's four columns are vdim/4
@@ -134,12 +154,15 @@ retention_chunk_state_kernel(RetArgs a, const int* __restrict__ chunk_seq, const
   __shared__ float power[RET_CHUNK];
   if (tid < len) power[tid] = powf(a.decay[h], (float)(len - 1 - tid));
   __syncthreads();
+  const bool copied = !a.in_act && ret_copy_rows(a, row0, len, a.v_off + h * a.vdim, vv, vdimp);
+  __pipeline_commit();
   for (int i = tid; i < len * (dimp - a.dim); i += blockDim.x) kd[i / (dimp - a.dim) * dimp + a.dim + i % (dimp - a.dim)] = 0.f;
   ret_load_keys(a, row0, len, pos0, h, dimp, power, kd, nullptr);
-  for (int i = tid; i < len * vdimp; i += blockDim.x) {
+  for (int i = tid; !copied && i < len * vdimp; i += blockDim.x) {
     const int j = i / vdimp, d = i % vdimp;
     vv[i] = d < a.vdim ? ret_v(a, a.qkvg[(long long)(row0 + j) * a.ld + a.v_off + h * a.vdim + d]) : 0.f;
   }
+  __pipeline_wait_prior(0);
   __syncthreads();
   float* U = ws + ((long long)c * a.heads + h) * a.dim * a.vdim;
   const int tiles_y = vdimp >> 2, tiles_x = (a.dim + 3) >> 2;
@@ -248,9 +271,11 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
   float* rr = pp + RET_CHUNK * (RET_CHUNK + 1);   // [RET_CHUNK]
   float* Ss = rr + RET_CHUNK;                  // [dim][vdimp] when stage_s
   const float dec = a.decay[h];
+  const bool copied = !a.in_act && ret_copy_rows(a, row0, len, a.v_off + h * a.vdim, vv, vdimp);
+  __pipeline_commit();
   for (int i = len * dimp + tid; i < RET_CHUNK * dimp; i += blockDim.x) qs[i] = ks[i] = 0.f;
   ret_load_keys(a, row0, len, pos0, h, dimp, nullptr, ks, qs);
-  for (int i = tid; i < RET_CHUNK * vdimp; i += blockDim.x) {
+  for (int i = tid; !copied && i < RET_CHUNK * vdimp; i += blockDim.x) {
     const int j = i / vdimp, d = i % vdimp;
     vv[i] = (j < len && d < a.vdim) ? ret_v(a, a.qkvg[(long long)(row0 + j) * a.ld + a.v_off + h * a.vdim + d]) : 0.f;
   }
@@ -260,6 +285,7 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
       const int d = i / vdimp, y = i % vdimp;
       Ss[i] = y < a.vdim ? S[d * a.vdim + y] : 0.f;
     }
+  __pipeline_wait_prior(0);
   __syncthreads();
   // in-chunk scores, 2 x 2 per thread (rows i0, i0 + 1, columns tj, tj + 16): every thread has one
   for (int tile = tid; tile < (RET_CHUNK / 2) * (RET_CHUNK / 2); tile += blockDim.x) {
@@ -302,6 +328,9 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
       }
   }
   __syncthreads();
+  // nobody reads the keys any more: the gates come in their place while the outputs are taken
+  const bool gates = WIDE && a.finish != LP_RET_FINISH_RAW && a.vdim <= dimp && ret_copy_rows(a, row0, len, a.g_off + h * a.vdim, ks, dimp);
+  __pipeline_commit();
   const int tiles_y = vdimp >> 2, tiles_i = (len + 3) >> 2;
   for (int tile = tid; tile < tiles_i * tiles_y; tile += blockDim.x) {
     const int i0 = (tile / tiles_y) * 4, ty = tile % tiles_y;
@@ -389,10 +418,11 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if (lane == 0) rr[i] = 1.0f / sqrtf(ss / (float)a.vdim + a.eps);
   }
+  __pipeline_wait_prior(0);
   __syncthreads();
   for (int e = tid; e < len * a.vdim; e += blockDim.x) {
     const int i = e / a.vdim, y = e % a.vdim;
-    const float g = a.qkvg[(long long)(row0 + i) * a.ld + a.g_off + h * a.vdim + y];
+    const float g = gates ? ks[i * dimp + y] : a.qkvg[(long long)(row0 + i) * a.ld + a.g_off + h * a.vdim + y];
     const float v = os[i * vdimp + y] * rr[i] * (g / (1.0f + expf(-g)));
     const long long o = (long long)(row0 + i) * a.ldo + h * a.vdim + y;
     if (a.out_fp32) reinterpret_cast<float*>(a.out)[o] = v;
