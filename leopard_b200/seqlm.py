@@ -39,18 +39,19 @@ TENSOR_CORE_MIN_ROWS = 64
 STREAM_MAX_OUTPUTS = 170_000
 # fp32 rows of more than 64 go to the tcgen05 product of three bf16 terms, a pass for the terms included (us, lp_linear and this one): 65 rows, K = 64,
 # 128 columns 8.5, 6.5; K = 1024, 4096 columns 36, 21; 4000 rows, K = 1024, 4096 columns 388, 105.  Up to 64 rows lp_linear streams the weights: 48 rows,
-# K = 128, 6.7, 7.3, K = 1024 12.5, 20.  (K of less than a k block and columns of less than a tile were not measured: they stay.)
-SPLIT_MIN_ROWS, SPLIT_MIN_K = 65, 64
+# K = 128, 6.7, 7.3, K = 1024 12.5, 20.  (K of less than a k block and columns of less than a tile were not measured: they stay.)  Its second launch costs the
+# host 3 us, so short products of few outputs, which gain up to 8 us in steps that wait for the host, stay too.
+SPLIT_MIN_ROWS, SPLIT_MIN_K, SPLIT_LONG_K, SPLIT_OUTPUTS = 65, 64, 768, 1 << 20
 # Rows of prompts expand the visible latents into every head's keys and values (lp_latent_attend_expanded), unless many requests bring a few rows each:
 # its tiles are 128 rows of one request.  A layer of width 1024 with 8 heads (us, lp_latent_attend_tiles and this one): one request of 20 rows 64, 45, of
 # 500 297, 85; 32 requests of 12 rows 92, 81; 64 of 12 97, 120, of 24 132, 126; width 2048, 16 heads: 4096 rows 6,490, 530; 64 requests of 12 rows 225, 205.
 EXPAND_TILES, EXPAND_TILE_ROWS = 32, 24
-# Window attention of prompts goes to lp_window_attn_prompt (128 rows of a request and a head a CTA) where its tiles are filled and it saves more than its launches
-# cost the host.  A layer, preparation included (us, lp_window_attn_tiles and this one; heads on a quarter of key / value heads): one request of 128 rows, 8
-# heads 34, 27; of 500 86, 45; of 4096, 16 heads 845, 302; 16 requests of 20, 16 heads 35, 42; of 40 40, 54.  Capped scores and values turned back
-# by position cost it more (a table, tanh, an exchange): one request of 128 rows, 16 heads 51, 58; of 500, 4 heads 72, 74, 8 heads 102, 76; of 4096, 16 heads 1009,
-# 417.
-WINDOW_TILE_ROWS, WINDOW_ROWS, WINDOW_CAP_WORK = 64, 200, 4000
+# Window attention of prompts goes to lp_window_attn_prompt (128 rows of a request and a head a CTA) where its tiles are filled and there is enough work that the
+# device's time counts: its launches cost the host some 15 us a layer more, and steps of fewer rows wait for the host.  A layer, preparation
+# included (us on the device, lp_window_attn_tiles and this one; heads on a quarter of key / value heads): one request of 500 rows, 8 heads 86, 45, 16 heads 150, 55; of
+# 4096, 4 heads 101, 62, 16 heads 845, 302; 16 requests of 40, 16 heads 40, 54.  Capped scores and values turned back by position: of 500 rows, 8 heads 102, 76, of
+# 4096, 16 heads 1009, 417.  Whole prompts of three layers: 1,143 rows of 4 heads 764 us, 818 with this one; 4096 of 16 heads 2,927, 1,902.
+WINDOW_TILE_ROWS, WINDOW_WORK = 64, 8000
 # Up to MOE_PAIRS_MAX (token, choice) pairs an expert's weights are streamed once for the pairs that chose it.  Both products of 16 experts,
 # width 2048, 1024 inside (us, bf16; fp32 rows), against sorted tiles: 128 pairs 66, 108; 85, 182.  256 pairs 93, 108; 138, 182.  512 pairs 161,
 # 108; 282, 182: with this few experts the sorted tiles are ahead from about 300 pairs, with 32 (width 4096) not yet at 512: 554, 683; 876, 1116.
@@ -930,7 +931,7 @@ class SeqLMEngine:
     def _on_split(self, a: torch.Tensor, w: torch.Tensor) -> bool:
         """Whether fp32 rows go to the tcgen05 product of three bf16 terms"""
         (M, K), N = a.shape, w.shape[0]
-        return (self.split_rows is not None and M >= self.split_rows and a.dtype == F32 and N >= 128 and K >= SPLIT_MIN_K and N % 8 == 0 and K % 8 == 0
+        return (self.split_rows is not None and M >= self.split_rows and a.dtype == F32 and N >= 128 and K >= SPLIT_MIN_K and (K >= SPLIT_LONG_K or M * N >= SPLIT_OUTPUTS) and N % 8 == 0 and K % 8 == 0
                 and a.stride(0) % 4 == 0 and w.stride(0) % 8 == 0 and a.stride(1) == 1 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
     def _split_product(self, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias) -> None:
@@ -1243,8 +1244,7 @@ class SeqLMEngine:
                 or qkv.stride(0) % 4 or qkv.data_ptr() % 16 or o.data_ptr() % 16 or o.stride(0) % (4 if o.dtype == F32 else 8)):
             return False
         tiles = sum(-(-ln // 128) for ln in b.lens)
-        pays = b.R >= WINDOW_ROWS and b.R >= WINDOW_TILE_ROWS * tiles and ((d.softcap <= 0 and not d.v_inv_freq) or b.R * m.heads >= WINDOW_CAP_WORK)
-        if not pays:
+        if b.R < WINDOW_TILE_ROWS * tiles or b.R * m.heads < WINDOW_WORK:
             return False
 
         def first(pos):      # the first token of its window, or of its own block of positions

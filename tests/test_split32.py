@@ -268,7 +268,7 @@ def test_expanded_latent_attention_in_the_engine(dtype, heads, rank, window, opt
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("M,N,K", [(65, 128, 64), (129, 264, 72), (300, 1000, 200), (257, 4096, 136)])
+@pytest.mark.parametrize("M,N,K", [(65, 128, 768), (4100, 264, 72), (1100, 1000, 200), (257, 4096, 136)])
 def test_products_of_fp32_rows_in_the_engine(M, N, K):
     """the split product and its epilogues are no further from float64 than lp_linear's"""
     from leopard_b200 import _lib
