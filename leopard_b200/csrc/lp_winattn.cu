@@ -32,7 +32,8 @@
 //   lp_window_attn_talk_tiles  the same for prompts, a CTA per tile of 4 consecutive rows of a request and all heads.
 //   lp_window_attn_tiles  the same for prompts, a CTA per tile of 2 or 4 consecutive rows of a request: the rows share every key and
 //                         value row the tile reads, each (row, key) pair masked by the row's own rule.  Heads of 128 run on the matrix
-//                         instructions, a CTA per chunk of up to 32 rows, where such CTAs fill the chip.
+//                         instructions, a CTA per chunk of up to 32 rows, where such CTAs fill the chip (long prompts without a distance bias
+//                         take lp_window_attn_prompt instead, csrc/lp_split32.cu).
 #include <cuda_pipeline.h>
 #include "lp_host.h"
 #include "../../include/leopard_b200.h"
