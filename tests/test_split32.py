@@ -222,7 +222,7 @@ def test_gather_of_cache_rows(emu):
 
 
 # ------------------------------------------------------------------------------------------------------------------- on a GPU, through the engine
-def latent_engine(dtype, heads, rank, window, **options):
+def latent_engine(dtype, heads, rank, window, max_tokens=2048, **options):
     from leopard_b200 import _lib
     from leopard_b200.seqlm import LatentAttentionConfig, LayerConfig, RotaryConfig, SeqLMConfig, SeqLMEngine, SeqLMWeights
     D, O = 256, heads * 128
@@ -238,7 +238,7 @@ def latent_engine(dtype, heads, rank, window, **options):
         x = torch.randn(shape, generator=torch.Generator().manual_seed(sum(map(ord, name))))
         return x * (2 * shape[1] ** -0.5 if len(shape) == 2 else 0.1)
     w = SeqLMWeights(cfg, get, lambda layer, key: key, "cuda")
-    return SeqLMEngine(cfg, w, dtype=dtype, max_tokens=2048, page_size=16, max_seqs=4, lib=_lib.stream32_lib()), m
+    return SeqLMEngine(cfg, w, dtype=dtype, max_tokens=max_tokens, page_size=16, max_seqs=4, lib=_lib.stream32_lib()), m
 
 
 @pytest.mark.gpu
@@ -265,6 +265,24 @@ def test_expanded_latent_attention_in_the_engine(dtype, heads, rank, window, opt
         assert float((got - want).norm() / want.norm()) < (3e-6 if dtype == "float32" else 1e-2)
         for s, ln in zip(batch.seqs, batch.lens):
             eng.cache.advance(s, ln)
+
+
+@pytest.mark.gpu
+def test_expanded_heads_in_groups():
+    """more keys than all heads' expanded keys and values are held for at a time (512 MB): the heads run in groups, the last one smaller"""
+    from leopard_b200.seqlm import StepEntry, _Batch
+    eng, m = latent_engine("float32", 19, 64, None, max_tokens=20480)
+    lw, n = eng.w.layers[0], 19000
+    assert n * 1536 * 19 > 512 << 20
+    for ln in (n, 40):      # a prompt, then a portion over all of it
+        batch = _Batch(eng, [StepEntry("a", [1] * ln, [])])
+        h = torch.randn((ln, 256), device="cuda", generator=torch.Generator("cuda").manual_seed(ln))
+        got = eng._latent(0, m, lw, h, batch).double()
+        kv = lw.pop("w_kv")
+        want = eng._latent(0, m, lw, h, batch).double()
+        lw["w_kv"] = kv
+        assert float((got - want).norm() / want.norm()) < 3e-6
+        eng.cache.advance(batch.seqs[0], ln)
 
 
 @pytest.mark.gpu
