@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
   __shared__ int pair_count[STREAM_MAX_PAIRS / 32];
   constexpr int U = MG >= 4 ? 1 : 2;      // k steps whose weights are in flight together
   // a warp's steps are neighbours, whole 128-byte lines of the weight rows (one tile: 14.6 us a launch of ronelorn's one-request steps, 13.7 so), or lie n_warps
-  // apart (two tiles, 32.5, 33.4)
+  // apart (two tiles)
   constexpr bool NEAR = NT == 1;
   constexpr int SLOTS = NT * MG * 4;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
     };
     uint4 a0[U][NT], a1[U][NT];
     // one tile of up to eight bf16 rows leaves registers free: the next steps' weights are asked for before these are used (K = N = 4096, one row: 10.6 us,
-    // 8.7 so; two tiles 26.6, 27.4, fp32 rows 4.6, 5.3: their registers cost CTAs)
+    // 8.7 so; fp32 rows 4.6, 5.3: their registers cost CTAs)
     const int stride = NEAR ? n_warps : U * n_warps, steps = NEAR ? (a.K + 32 * U - 1) / (32 * U) : (a.K + 31) / 32;
     if constexpr (MG == 1 && NT == 1 && sizeof(AT) == 2) {
       uint4 b0[U][NT], b1[U][NT];
@@ -630,10 +630,11 @@ static int dispatch_stream(const LinArgs& a, int a_fp32, int c_fp32, int batch, 
   const int n_out = gated_epi(a.epi) ? a.N / 2 : a.N, per = gated_epi(a.epi) ? 8 : 16;
   const int mg = rows <= 8 ? 1 : rows <= 16 ? 2 : rows <= 32 ? 4 : 8;
   const long long problems = n_groups > 0 ? n_groups : batch;
-  // two tiles a CTA read A half as often (and cut it into terms once): taken once the grid still has two CTAs for every SM and where
-  // segments allow; with more than eight bf16 rows its registers cost more CTAs than it saves (N = 12288, K = 4096, M = 16: 35 us with one tile, 46 with two)
+  // fp32 rows: two tiles a CTA read A half as often and cut it into terms once, taken once the grid still has two CTAs for every SM and where segments
+  // allow.  bf16 rows take one: its registers leave room for the next steps' weights (one row, us, two tiles and one: K = 4096, N = 16384 28.1, 25.9, N =
+  // 32000 49.2, 46.1; eight rows of 14 experts, K = 2048, N = 2048 27.2, 24.1; with 16 rows, N = 12288, K = 4096, 46, 35)
   const long long wide = problems * ((n_out + 2 * per - 1) / (2 * per));
-  const int nt = (mg == 1 || a_fp32) && wide >= 2 * sm_count() && (a.seg_cols == 0 || a.seg_cols % (2 * per) == 0) ? 2 : 1;
+  const int nt = a_fp32 && wide >= 2 * sm_count() && (a.seg_cols == 0 || a.seg_cols % (2 * per) == 0) ? 2 : 1;
   const long long ctas = problems * ((n_out + nt * per - 1) / (nt * per));
   // a short K has no work for more warps (K = 192, one row: 4.0 us with four, 3.2 with eight); a grid of few CTAs wants more loads in flight in each (N = 2048, K = 8192: 15 us with 16 warps, 11 with 32)
   int warps = a.K <= (mg == 1 ? 128 : 256) ? 4 : !a_fp32 && mg * nt == 1 && ctas <= sm_count() && a.K >= 4096 ? 32 : ctas <= 2 * sm_count() && a.K >= 1024 && mg <= 4 ? 16 : 8;
@@ -641,7 +642,6 @@ static int dispatch_stream(const LinArgs& a, int a_fp32, int c_fp32, int batch, 
 #define LP_STREAM(MG)                                                                                                               \
   (a_fp32 ? (nt == 2 ? launch_stream<float, 2, MG>(a, c_fp32, grid, warps, n_pairs, stream) : launch_stream<float, 1, MG>(a, c_fp32, grid, warps, n_pairs, stream)) \
           : launch_stream<bf16, 1, MG>(a, c_fp32, grid, warps, n_pairs, stream))
-  if (!a_fp32 && nt == 2) return launch_stream<bf16, 2, 1>(a, c_fp32, grid, warps, n_pairs, stream);      // nt == 2 means mg == 1
   return mg == 1 ? LP_STREAM(1) : mg == 2 ? LP_STREAM(2) : mg == 4 ? LP_STREAM(4) : LP_STREAM(8);
 #undef LP_STREAM
 }
