@@ -281,7 +281,8 @@ def test_expanded_heads_in_groups():
         kv = lw.pop("w_kv")
         want = eng._latent(0, m, lw, h, batch).double()
         lw["w_kv"] = kv
-        assert float((got - want).norm() / want.norm()) < 3e-6
+        # a sum over n keys of either sign, one after the other, rounds off 2^-24 sqrt(n / 2) = 6e-6 of itself in the general path
+        assert float((got - want).norm() / want.norm()) < 2e-5
         eng.cache.advance(batch.seqs[0], ln)
 
 
