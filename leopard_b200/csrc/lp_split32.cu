@@ -28,9 +28,11 @@ inline void s32_wait(uint64_t* bar, uint32_t parity) { mbar_wait(bar, parity); }
 inline void s32_bar(int id, int n) { named_bar(id, n, true); }
 inline float s32_ex2(float x) { return exp2f(x); }
 inline uint32_t __byte_perm(uint32_t a, uint32_t b, uint32_t) { return (a >> 16) | (b & 0xffff0000u); }
-template <int N> inline void s32_more_regs() {}
-template <int N> inline void s32_fewer_regs() {}
+template <int N> inline void s32_more_regs() { emu_registers = N; }
+template <int N> inline void s32_fewer_regs() { emu_registers = N; }
+inline void s32_serial() { emu_serial(); }
 #else
+__device__ __forceinline__ void s32_serial() {}      // where results are taken again one by one: the emulated build looks at what the CTA is about then
 // as mbar_wait, without its message: a call in the loop of the one thread that issues the MMAs costs it registers, and its spills the tensor cores' time
 __device__ __forceinline__ void s32_wait(uint64_t* bar, uint32_t parity) {
   if (mbar_try_wait(bar, parity)) return;
@@ -520,9 +522,10 @@ __global__ void __launch_bounds__(256) turn_table_kernel(Seqs32 q, int R, const 
 // the rows of a tile again, each over the keys it sees, in fp32 multiply-adds: a warp a row, a lane a key and four channels
 template <int NR>
 __device__ __noinline__ void attn32_plain(const Attn32Args& a, int r0, int nrows, int pos0, int kbase, const Run32& run, int h, int kvl, float* p_s,
-                                          int n_warps) {
+                                          int warp, int n_warps) {
   constexpr int DQ = Attn32Smem<NR>::DQ;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31;
+  s32_serial();
   p_s += warp * 160;
   for (int x = warp; x < nrows; x += n_warps) {
     const int pos = pos0 + x;
@@ -607,6 +610,7 @@ attn32_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   uint64_t* pv_done = p_full + 1;         // [2]: the first sum of a tile, the second
   uint64_t* o_taken = pv_done + 2;
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(o_taken + 1);
+  uint32_t* odd_s = tmem_ptr + 1;         // outputs that are not finite
   float* top_s = reinterpret_cast<float*>(smem + S::TOP_OFF);      // [2][2][128]
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   // this tile's request and rows, and where its keys lie; later tiles see more keys: they start first
@@ -647,6 +651,7 @@ attn32_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     mbar_init(pv_done + 1, 1);
     mbar_init(o_taken, 256);
     fence_barrier_init();
+    *odd_s = 0;
   }
   if (warp == 0) {
     tmem_alloc(tmem_ptr, 512);
@@ -656,7 +661,6 @@ attn32_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = *tmem_ptr;
-  bool odd = false;
   if (warp < 4) {
     s32_fewer_regs<S32_FEW>();
     if (warp == 0) {
@@ -883,6 +887,7 @@ attn32_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     s32_bar(1 + lg, 64);
     den += ds[(hh ^ 1) * 128 + x];
     if (mine) {
+      bool odd = false;
       float f = den == 0.f && a.sink == nullptr && a.zero_empty ? 0.f : 1.0f / den;
       if (a.gate != nullptr) f *= 1.0f / (1.0f + expf(-a.gate[(long long)(r0 + x) * a.ldg + h]));
 #pragma unroll
@@ -890,6 +895,7 @@ attn32_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         odd |= !(fabsf(o[c]) <= 3.402823466e38f);
         o[c] *= f;
       }
+      if (odd) *odd_s = 1;
     }
     if (a.turn != nullptr) {      // the two threads of a row exchange their channels where the queries were: all products have run
       float* os = reinterpret_cast<float*>(smem) + x * 129;
@@ -922,15 +928,17 @@ attn32_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                             pack_bf16x2(o[8 * c + 6], o[8 * c + 7]));
       }
     }
+    // an infinity or a NaN among the keys or values: weights of zero times it are NaN in every row of the product, seen or not.  All products have run.
+    // The other warps have given up the registers that this may want: they stay out.
+    s32_bar(5, A32_THREADS - 128);
+    if (*odd_s != 0) attn32_plain<NR>(a, r0, nrows, pos0, kbase, run, h, kvl, reinterpret_cast<float*>(smem), warp - 4, A32_THREADS / 32 - 4);
   }
   tc_fence_before();
-  const int again = __syncthreads_or(odd);
+  __syncthreads();
   if (warp == 0) {
     __syncwarp();
     tmem_dealloc(tm, 512);
   }
-  // an infinity or a NaN among the keys or values: weights of zero times it are NaN in every row of the product, seen or not
-  if (again) attn32_plain<NR>(a, r0, nrows, pos0, kbase, run, h, kvl, reinterpret_cast<float*>(smem), A32_THREADS / 32);
 }
 
 }  // namespace lp

@@ -1,8 +1,27 @@
 // Test infrastructure: runs the kernels of leopard_b200/csrc/lp_split32.cu on the CPU under tests/emu/tc_emu.h.
 #define LP_EMULATE 1
+#include <atomic>
+// a thread's registers as the kernels split them, and what the CTA was about when results were first taken again one by one
+static thread_local int emu_registers = 0;
+static std::atomic<int> emu_fewest_registers{1 << 20};
+static std::atomic<long> emu_first_serial{-1};
+static void emu_serial();
 #include "../../leopard_b200/csrc/lp_split32.cu"
 
 using namespace lp;
+
+static void emu_serial() {
+  for (int had = emu_fewest_registers; emu_registers < had && !emu_fewest_registers.compare_exchange_weak(had, emu_registers);) {
+  }
+  long none = -1;
+  emu_first_serial.compare_exchange_strong(none, emu_tc::g_issued);
+}
+// since the last call: the fewest registers that a thread had when it took results again; MMAs that had been issued when the first one did (-1: none did), and in all
+extern "C" void emu_serial_stats(int* registers, long* at_first, long* in_all) {
+  *registers = emu_fewest_registers.exchange(1 << 20);
+  *at_first = emu_first_serial.exchange(-1);
+  *in_all = emu_tc::g_issued.exchange(0);
+}
 
 static CUtensorMap tmap3(const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t ld, uint64_t plane, uint32_t rows) {
   CUtensorMap m;

@@ -59,6 +59,7 @@ struct Cta {
   uint32_t rank = 0;
 };
 inline std::mutex g_mu;
+inline std::atomic<long> g_issued{0};   // MMAs, over all launches
 inline Cta g_cta[4];
 alignas(1024) inline uint8_t g_smem_peers[3][232448];
 inline uint32_t g_tmem_store[4][128][512];
@@ -310,6 +311,7 @@ inline void tmem_st(const uint32_t* regs, uint32_t taddr, int n) {
 // in CTA n / (N / 2); the descriptors name the same shared-memory offsets in both CTAs.
 inline void umma_exec(uint32_t tmem_d, bool a_in_tmem, uint32_t tmem_a, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                       uint32_t accumulate, bool pair) {
+  ++emu_tc::g_issued;
   const int M = (int)((idesc >> 24) & 0x1f) << 4, N = (int)((idesc >> 17) & 0x3f) << 3;
   const bool a_mn = (idesc >> 15) & 1, b_mn = (idesc >> 16) & 1;
   if (M != (pair ? 256 : 128) || (a_mn && a_in_tmem) || (pair && a_in_tmem)) {

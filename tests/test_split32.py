@@ -206,6 +206,35 @@ def test_attention_of_three_planes(emu, lens, pos0, window, rot, opts):
         assert float((out[: R - 1].double() - want[: R - 1]).norm() / want.norm()) < 1e-6
 
 
+def serial_stats(emu):
+    """(fewest registers of a thread that took results again, MMAs issued before the first one did or -1, MMAs) since the last call"""
+    regs, first, total = C.c_int(), C.c_long(), C.c_long()
+    emu.emu_serial_stats(C.byref(regs), C.byref(first), C.byref(total))
+    return regs.value, first.value, total.value
+
+
+@pytest.mark.parametrize("rot", [False, True])
+def test_rows_are_taken_again_by_warps_that_have_the_registers(emu, rot):
+    """the warps that load and multiply give registers up when they start: what takes rows again was compiled for as many as a thread starts with (168)"""
+    R, keys, dq = 40, 200, 192 if rot else 128
+    g = torch.Generator().manual_seed(R)
+    q, k, v = torch.randn((R, dq), generator=g), torch.randn((keys, 128), generator=g), torch.randn((keys, 128), generator=g)
+    kr = torch.randn((keys, 64), generator=g) if rot else None
+    row0, p0 = torch.tensor([0, R], dtype=torch.int32), torch.tensor([keys - R], dtype=torch.int32)
+    out = torch.empty((R, 128))
+    for bad in (False, True):
+        if bad:
+            v[keys - 3, 9] = math.inf
+        p = [planes(emu, x) if x is not None else None for x in (q, k, kr, v)]
+        serial_stats(emu)
+        emu.emu_attn32(*[P(x) for x in p], R, 1, 1, 1, 0, 0, 0, 0, P(row0), P(p0), 1, keys, C.c_float(dq ** -0.5), C.c_float(0.0), 0, P(None), P(None), P(None),
+                       P(None), 0, 0, P(None), P(out), 1)
+        regs, first, total = serial_stats(emu)
+        assert (first == total and regs >= 168) if bad else first == -1
+    want = reference(q, k, kr, v, [R], [keys - R], (0,), dq ** -0.5, 1)
+    assert torch.equal(out.isinf(), want.isinf()) and float((out[:-3].double() - want[:-3]).norm() / want[:-3].norm()) < 1e-6
+
+
 def test_gather_of_cache_rows(emu):
     g = torch.Generator().manual_seed(4)
     width, page, lens, pos0, rule = 24, 4, [3, 5], [6, 0], (4, 0, 2, 2)
@@ -265,6 +294,26 @@ def test_expanded_latent_attention_in_the_engine(dtype, heads, rank, window, opt
         assert float((got - want).norm() / want.norm()) < (3e-6 if dtype == "float32" else 1e-2)
         for s, ln in zip(batch.seqs, batch.lens):
             eng.cache.advance(s, ln)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bad", [math.inf, math.nan])
+def test_a_latent_that_is_not_finite_stays_with_the_rows_that_see_it(bad):
+    from leopard_b200.seqlm import StepEntry, _Batch
+    eng, m = latent_engine("float32", 3, 136, 100)
+    lw, got = eng.w.layers[0], None
+    for ln in (300, 150):
+        batch = _Batch(eng, [StepEntry("a", [1] * ln, [])])
+        if ln == 150:      # position 250: rows 300 .. 349 see it
+            eng.cache.pools[0][batch.seqs[0].pages[250 // 16], 250 % 16, 3] = bad
+        h = torch.randn((ln, 256), device="cuda", generator=torch.Generator("cuda").manual_seed(ln))
+        got = eng._latent(0, m, lw, h, batch)
+        eng.cache.advance(batch.seqs[0], ln) if ln == 300 else None
+    kv = lw.pop("w_kv")
+    want = eng._latent(0, m, lw, h, batch)
+    lw["w_kv"] = kv
+    assert not bool(want[:50].isfinite().any()) and not bool(got[:50].isfinite().any())
+    assert float((got[50:].double() - want[50:].double()).norm() / want[50:].double().norm()) < 3e-6      # the bound of the test above
 
 
 @pytest.mark.gpu
