@@ -157,7 +157,8 @@ struct Gemm32Args {
 };
 
 // An infinite weight times a term that is zero, or of the other sign, is a NaN that the product of the uncut number is not: outputs that came out NaN
-// are taken again in fp32 multiply-adds (by the thread that wrote them)
+// are taken again in fp32 multiply-adds (by the thread that wrote them, once its CTA's products have run: K steps an output are too long for other warps
+// to wait on)
 __device__ float gemm32_plain(const Gemm32Args& a, int row, const bf16* w) {
   const bf16* x = a.A + (long long)row * a.lda;
   float s = 0.f;
@@ -170,6 +171,7 @@ __device__ __forceinline__ float gemm32_gated(float z, float u, float rs) {
   return z / (1.0f + expf(-z)) * (u * rs);
 }
 __device__ __noinline__ void gemm32_mend(const Gemm32Args& a, int row, int group, int col0, int cols, int gated) {
+  s32_serial();
   const bf16* W = a.W + (long long)group * a.w_group;
 #pragma unroll 1
   for (int c = col0; c < col0 + cols && c < (gated ? a.N / 2 : a.N); ++c) {
@@ -310,7 +312,8 @@ gemm32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
     const uint32_t lane_addr = tm + ((uint32_t)(lg * 32) << 16) + half * (BN / 2);
     const int chains = (kb_n + CHAIN - 1) / CHAIN;
     int it = 0;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    uint32_t odd_turns = 0;      // bit t: a tile of turn t, t + 32, .. has a NaN
+    for (int tile = blockIdx.x, turn = 0; tile < tiles; tile += gridDim.x, ++turn) {
       if (group_of(tile) < 0) continue;
       const int row = tile_m(tile) * 128 + lg * 32 + lane, n0 = tile_n(tile) * COLS + half * (COLS / 2);
       float acc[BN / 2];
@@ -386,9 +389,14 @@ gemm32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
             }
           }
         }
-        if (PLANES == 3 && odd) gemm32_mend(a, row, group_of(tile), n0, COLS / 2, GATED);
+        if (PLANES == 3 && odd) odd_turns |= 1u << (turn & 31);
       }
     }
+    for (int tile = blockIdx.x, turn = 0; odd_turns != 0 && tile < tiles; tile += gridDim.x, ++turn)
+      if (odd_turns >> (turn & 31) & 1) {
+        const int row = tile_m(tile) * 128 + lg * 32 + lane;
+        if (group_of(tile) >= 0 && row < a.M) gemm32_mend(a, row, group_of(tile), tile_n(tile) * COLS + half * (COLS / 2), COLS / 2, GATED);
+      }
   }
   tc_fence_before();
   __syncthreads();

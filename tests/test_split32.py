@@ -235,6 +235,32 @@ def test_rows_are_taken_again_by_warps_that_have_the_registers(emu, rot):
     assert torch.equal(out.isinf(), want.isinf()) and float((out[:-3].double() - want[:-3]).norm() / want[:-3].norm()) < 1e-6
 
 
+@pytest.mark.parametrize("gated", [None, False, True])
+def test_products_are_taken_again_after_the_tiles(emu, gated):
+    """one CTA, more than 32 tiles: outputs that came out NaN are looked at again when all of its MMAs have been issued, so no warp waits meanwhile"""
+    M, N, K = 1408, 384, 64      # 33 tiles of 128 x 128; of groups 22 of 256 columns, 33 of a gated unit
+    g = torch.Generator().manual_seed(9)
+    x, w = torch.randn((M, K), generator=g), torch.ones((2 * N if gated else N, K)).to(BF)
+    w[5, 7] = math.inf
+    x[:, 7] = x[:, 7].abs() + 0.1
+    x[1300, 7] = 0.0
+    p, c = planes(emu, x), torch.zeros((M, N))
+    serial_stats(emu)
+    if gated is None:
+        emu.emu_gemm_split(P(p), LL(K), LL(M * K), P(w), LL(K), P(c), LL(N), LL(0), 1, M, N, K, P(None), 128, 1)
+    else:
+        groups = torch.zeros(M // 128, dtype=torch.int32)
+        groups[3] = -1
+        emu.emu_gemm_grouped(P(p), LL(M * K), P(w), 1, P(groups), M // 128, int(gated), P(None), P(c), LL(0), 1, w.shape[0], K, 1)
+    regs, first, total = serial_stats(emu)
+    assert first == total > 0 and regs >= 168
+    y = x.double() @ w.double().T
+    if gated:
+        y = torch.nn.functional.silu(y[:, :N]) * y[:, N:]
+    rows = torch.tensor([r for r in range(M) if gated is None or r // 128 != 3])
+    assert torch.equal(c.isnan()[rows], y.isnan()[rows]) and torch.equal(c.isinf()[rows], y.isinf()[rows]) and bool(c.isnan().any())
+
+
 def test_gather_of_cache_rows(emu):
     g = torch.Generator().manual_seed(4)
     width, page, lens, pos0, rule = 24, 4, [3, 5], [6, 0], (4, 0, 2, 2)
