@@ -574,9 +574,10 @@ __device__ __noinline__ void attn32_plain(const Attn32Args& a, int r0, int nrows
       }
       __syncwarp();
     }
-    float f = den == 0.f && a.sink == nullptr && a.zero_empty ? 0.f : 1.0f / den;
+    const bool empty = den == 0.f && a.sink == nullptr && a.zero_empty;
+    float f = 1.0f / den;
     if (a.gate != nullptr) f *= 1.0f / (1.0f + expf(-a.gate[(long long)(r0 + x) * a.ldg + h]));
-    for (int i = 0; i < 4; ++i) p_s[32 + lane + 32 * i] = f == 0.f ? 0.f : o[i] * f;
+    for (int i = 0; i < 4; ++i) p_s[32 + lane + 32 * i] = empty ? 0.f : o[i] * f;
     __syncwarp();
     for (int i = 0; i < 4; ++i) {
       const long long at = (long long)(r0 + x) * a.ldo + (long long)h * 128 + lane + 32 * i;

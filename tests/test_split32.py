@@ -235,6 +235,21 @@ def test_rows_are_taken_again_by_warps_that_have_the_registers(emu, rot):
     assert torch.equal(out.isinf(), want.isinf()) and float((out[:-3].double() - want[:-3]).norm() / want[:-3].norm()) < 1e-6
 
 
+def test_a_closed_gate_does_not_hide_a_nan(emu):
+    """zero times NaN is NaN: rows of a head whose gate's sigmoid is zero"""
+    R, H = 3, 2
+    g = torch.Generator().manual_seed(2)
+    q, k, kr, v = (torch.randn((R, n), generator=g) for n in (H * 192, H * 128, 64, H * 128))
+    v[1, 4] = math.nan
+    gate = torch.tensor([[0.0, -200.0], [-200.0, 0.0], [-200.0, -200.0]])
+    row0, p0, out = torch.tensor([0, R], dtype=torch.int32), torch.zeros(1, dtype=torch.int32), torch.empty((R, H * 128))
+    emu.emu_attn32(*[P(planes(emu, x)) for x in (q, k, kr, v)], R, H, 1, 1, 0, 0, 0, 0, P(row0), P(p0), 1, R, C.c_float(192 ** -0.5), C.c_float(0.0), 0, P(None),
+                   P(gate), P(None), P(None), 0, 0, P(None), P(out), 1)
+    nan = torch.zeros((R, H * 128), dtype=torch.bool)
+    nan[1:, 4] = True
+    assert torch.equal(out.isnan(), nan) and bool((out[2, 5:] == 0).all())
+
+
 @pytest.mark.parametrize("gated", [None, False, True])
 def test_products_are_taken_again_after_the_tiles(emu, gated):
     """one CTA, more than 32 tiles: outputs that came out NaN are looked at again when all of its MMAs have been issued, so no warp waits meanwhile"""
