@@ -243,7 +243,8 @@ def test_a_closed_gate_does_not_hide_a_nan(emu):
     v[1, 4] = math.nan
     gate = torch.tensor([[0.0, -200.0], [-200.0, 0.0], [-200.0, -200.0]])
     row0, p0, out = torch.tensor([0, R], dtype=torch.int32), torch.zeros(1, dtype=torch.int32), torch.empty((R, H * 128))
-    emu.emu_attn32(*[P(planes(emu, x)) for x in (q, k, kr, v)], R, H, 1, 1, 0, 0, 0, 0, P(row0), P(p0), 1, R, C.c_float(192 ** -0.5), C.c_float(0.0), 0, P(None),
+    p = [planes(emu, x) for x in (q, k, kr, v)]
+    emu.emu_attn32(*[P(x) for x in p], R, H, 1, 1, 0, 0, 0, 0, P(row0), P(p0), 1, R, C.c_float(192 ** -0.5), C.c_float(0.0), 0, P(None),
                    P(gate), P(None), P(None), 0, 0, P(None), P(out), 1)
     nan = torch.zeros((R, H * 128), dtype=torch.bool)
     nan[1:, 4] = True
