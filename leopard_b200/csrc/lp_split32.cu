@@ -117,9 +117,23 @@ __device__ __forceinline__ float s32_value(const bf16* p, long long plane) {
   return (__float_as_uint(h) & 0x7f800000u) == 0x7f800000u ? h : h + ((float)p[plane] + (float)p[2 * plane]);
 }
 
-// fp32 rows -> planes, eight columns a thread
+// a factor in two floats, so that its own rounding does not reach everything that it is applied to
+struct Factor32 {
+  float hi, lo;
+};
+inline Factor32 factor32(double f) {
+  const float hi = (float)f;
+  return {hi, (float)(f - (double)hi)};
+}
+// x times it; an infinity stays one
+__device__ __forceinline__ float times32(float x, const Factor32& f) {
+  const float y = x * f.hi;
+  return fabsf(y) < INFINITY ? fmaf(x, f.hi, x * f.lo) : y;
+}
+// fp32 rows (times a factor) -> planes, eight columns a thread
+template <bool SCALED>
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ src, long long ld, int M, int K, bf16* __restrict__ dst,
-                                                         long long ldd, long long plane) {
+                                                         long long ldd, long long plane, Factor32 factor) {
   const int per = K >> 3;
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= (long long)M * per) return;
@@ -127,7 +141,10 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
   const int c = (int)(i - r * per) * 8;
   const float* s = src + r * ld + c;
   const float4 a = *reinterpret_cast<const float4*>(s), b = *reinterpret_cast<const float4*>(s + 4);
-  const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    if (SCALED) v[i] = times32(v[i], factor);
   s32_store_terms(dst + r * ldd + c, plane, v);
 }
 
@@ -473,7 +490,7 @@ __global__ void __launch_bounds__(256) gather_keys_kernel(Seqs32 q, int n_keys, 
 struct Attn32Args {
   Seqs32 seqs;
   int head0, ratio;      // this launch has heads head0 .. head0 + gridDim.x - 1; `ratio` of them share a key / value head, which lie from head0's on
-  float scale, softcap;
+  float cap;             // scores are cap * tanh(query * key), or 0: query * key.  The queries' planes hold what makes that the score times log2(e): scale32
   const float* sink;     // [heads] or null
   int sink_one;          // 1 joins the denominator
   int zero_empty;        // a row whose scores are all -inf gives zeros (else NaN)
@@ -500,10 +517,19 @@ struct Attn32Smem {
   static constexpr int RING = 3 * NB * S32_BOX, BAR_OFF = RING + SLOTS * S32_BOX, TOP_OFF = BAR_OFF + 256, TOTAL = TOP_OFF + 2 * 2 * 128 * 4 + 1024;
 };
 
-__device__ __forceinline__ float score32(const Attn32Args& a, float s) {
-  s *= a.scale;
-  return a.softcap > 0.f ? a.softcap * tanhf(s / a.softcap) : s;
+constexpr float LOG2E = 1.4426950408889634f;
+// What cutting sums off instead of rounding them takes from a score (eight to twelve full-size steps) and from an output (chains of four), of itself and on
+// average: measured as the error's component along the score and along the output, 1.2e-7 to 1.4e-7 and 0.2e-7 to 1.0e-7 over 100 to 4096 rows, 128 and 192
+// channels, windows of 100 keys and none, scores of deviation 0.2 and 1, values around 0 and around 1
+constexpr double CUT_SCORE = 1.2e-7, CUT_OUT = 0.4e-7, TANH_OVER = 0.5e-7;      // (tanhf of a small number is the last so much too large)
+// the factor of the queries and the cap of the scores, both for scores times log2(e)
+inline Factor32 scale32(float scale, float softcap, float& cap) {
+  constexpr double log2e = 1.4426950408889634;
+  cap = softcap > 0.f ? (float)(softcap * log2e) : 0.f;
+  // small scores are query * key * cap: what rounding takes from the cap goes to the queries
+  return factor32((softcap > 0.f ? scale / (double)softcap * (softcap * log2e / cap) : scale * log2e) * (1.0 + CUT_SCORE - (softcap > 0.f ? TANH_OVER : 0.0)));
 }
+__device__ __forceinline__ float score32(const Attn32Args& a, float s) { return a.cap > 0.f ? a.cap * tanhf(s) : s; }
 __device__ __forceinline__ float out32(const Attn32Args& a, int row, int h, int c, float v) {
   if (a.out_gate != nullptr) v *= 1.0f / (1.0f + expf(-a.out_gate[(long long)row * a.ldog + h * 128 + c]));
   return v * a.out_scale;
@@ -544,7 +570,7 @@ __device__ __noinline__ void attn32_plain(const Attn32Args& a, int r0, int nrows
                                                                               : run.keep + run.blocks + see.lo - run.lo + t - see.keep - see.blocks);
     };
     const bf16* q = a.q + (long long)(r0 + x) * a.ldq + (long long)h * DQ;
-    float mx = a.sink != nullptr ? a.sink[h] : a.sink_one ? 0.f : -INFINITY, den = a.sink != nullptr || a.sink_one ? 1.f : 0.f;
+    float mx = a.sink != nullptr ? a.sink[h] * LOG2E : a.sink_one ? 0.f : -INFINITY, den = a.sink != nullptr || a.sink_one ? 1.f : 0.f;
     float o[4] = {0.f, 0.f, 0.f, 0.f};
     for (int t0 = 0; t0 < count; t0 += 32) {
       const int t = t0 + lane;
@@ -556,11 +582,11 @@ __device__ __noinline__ void attn32_plain(const Attn32Args& a, int r0, int nrows
           const float kv = d < 128 ? s32_value(a.k + kr * a.ldk + kvl * 128 + d, a.k_plane) : s32_value(a.kr + kr * a.ldkr + (d - 128), a.kr_plane);
           s = fmaf(s32_value(q + d, a.q_plane), kv, s);
         }
-        s = score32(a, s);
+        s = score32(a, s * (float)(1.0 - CUT_SCORE));      // nothing is cut off here
       }
       float top = s;
       for (int m = 16; m > 0; m >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, m));
-      const float mn = fmaxf(mx, top), ref = mn == -INFINITY ? 0.f : mn, corr = expf(mx - ref), p = t < count ? expf(s - ref) : 0.f;
+      const float mn = fmaxf(mx, top), ref = mn == -INFINITY ? 0.f : mn, corr = exp2f(mx - ref), p = t < count ? exp2f(s - ref) : 0.f;
       float sum = p;
       for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
       den = fmaf(den, corr, sum);
@@ -602,6 +628,10 @@ __device__ __noinline__ void attn32_plain(const Attn32Args& a, int r0, int nrows
 // instructions a warp and tile, two warps a scheduler) and outputs: tensor pipe 45 % active, the softmax warps mostly waiting for TMEM.
 // Measured (B200, 4096 tokens, 16 heads): latent attention over 1024 keys 240 us (fp32 multiply-adds over the latents themselves 6,125), window attention 205 to
 // 280 (window_attn_mma_kernel on mma.sync 760 to 930).  The MMA thread's spills and the softmax in expf with truncated terms had cost 100 us.
+// Error against 64 bits, 1e-7 of the output (window_attn_mma_kernel; this kernel before its queries carried the scale and what cutting off takes; now): 4096 rows
+// of 16 heads, window 1024, 4 kept 1.70, 1.97, 1.45; capped at 30, blocks of 64 1.79, 1.99, 1.56; 500 rows of 32 heads 1.33, 1.65, 1.23; 640 rows after 3000
+// 2.11, 2.39, 1.72; 200 rows of 64 heads 1.23, 1.48, 1.16; scores of deviation 3 over values of mean 1, beyond what layers make of normed queries and keys,
+// 1.94, 2.68, 2.15.  Latent attention, 4096 rows over 1024 keys (fp32 multiply-adds over the latents; before; now): 3.92, 1.72, 1.36.
 template <int NR>
 __global__ void __launch_bounds__(A32_THREADS, 1)
 attn32_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmKr,
@@ -797,9 +827,7 @@ attn32_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     const Seen32 see = seen32(a.seqs, pos0 + x);
     const int my_keep = mine ? see.keep : 0, my_blocks = mine ? run.keep + see.blocks : 0, my_lo = tok + see.lo, my_hi = mine ? tok + pos0 + x : -1;
     const int all_lo = tok + see1.lo, all_hi = tok + pos0;      // tokens that every row sees
-    // scores and their maxima are kept times log2(e)
-    constexpr float LOG2E = 1.4426950408889634f;
-    const float factor = a.softcap > 0.f ? a.scale / a.softcap : a.scale * LOG2E, cap = a.softcap * LOG2E;
+    const float cap = a.cap > 0.f ? a.cap : 1.f;
     float mx = a.sink != nullptr ? a.sink[h] * LOG2E : a.sink_one ? 0.f : -INFINITY, den = (a.sink != nullptr || a.sink_one) && hh == 0 ? 1.f : 0.f;
     float corr_before = 0.f;
     float o[64];
@@ -831,11 +859,9 @@ attn32_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       LP_TMEM_LD_32((v + 32), s_addr + 32);
       tmem_wait_ld();
       const int k0 = key_at(i) + hh * 64;
+      if (a.cap > 0.f) {
 #pragma unroll
-      for (int j = 0; j < 64; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * factor);
-      if (a.softcap > 0.f) {
-#pragma unroll
-        for (int j = 0; j < 64; ++j) v[j] = __float_as_uint(cap * tanhf(__uint_as_float(v[j])));
+        for (int j = 0; j < 64; ++j) v[j] = __float_as_uint(tanhf(__uint_as_float(v[j])));
       }
       if (i < n_a) {      // kept tokens, then blocks
 #pragma unroll
@@ -851,22 +877,23 @@ attn32_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       float top = -INFINITY;
 #pragma unroll
       for (int j = 0; j < 64; ++j) top = fmaxf(top, __uint_as_float(v[j]));
+      top *= cap;
       float* ts = top_s + (i & 1) * 256;
       ts[hh * 128 + x] = top;
       s32_bar(1 + lg, 64);
       if (i > 0) take_first(i - 1);
       const float mn = fmaxf(mx, fmaxf(top, ts[(hh ^ 1) * 128 + x])), ref = mn == -INFINITY ? 0.f : mn;      // -inf: nothing seen so far
       const float corr = s32_ex2(mx - ref);
-      float sum0 = 0.f, sum1 = 0.f;
+      float sums[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int j = 0; j < 64; j += 2) {
-        const float p0 = s32_ex2(__uint_as_float(v[j]) - ref), p1 = s32_ex2(__uint_as_float(v[j + 1]) - ref);      // 2^-inf = 0: not seen
+        const float p0 = s32_ex2(fmaf(__uint_as_float(v[j]), cap, -ref)), p1 = s32_ex2(fmaf(__uint_as_float(v[j + 1]), cap, -ref));      // 2^-inf = 0: not seen
         v[j] = __float_as_uint(p0);
         v[j + 1] = __float_as_uint(p1);
-        sum0 += p0;
-        sum1 += p1;
+        sums[j & 2] += p0;
+        sums[(j & 2) + 1] += p1;
       }
-      den = fmaf(den, corr, sum0 + sum1);
+      den = fmaf(den, corr, (sums[0] + sums[1]) + (sums[2] + sums[3]));
       mx = mn;
       if (i > 0) {      // all of P V of the tile before has run: its lower terms of P are no longer read
         s32_wait(pv_done + 1, (uint32_t)(i - 1) & 1);
@@ -897,12 +924,18 @@ attn32_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     den += ds[(hh ^ 1) * 128 + x];
     if (mine) {
       bool odd = false;
-      float f = den == 0.f && a.sink == nullptr && a.zero_empty ? 0.f : 1.0f / den;
-      if (a.gate != nullptr) f *= 1.0f / (1.0f + expf(-a.gate[(long long)(r0 + x) * a.ldg + h]));
+      const bool empty = den == 0.f && a.sink == nullptr && a.zero_empty;
+      Factor32 f = {empty ? 0.f : 1.0f / den, 0.f};
+      if (!empty) f.lo = fmaf(fmaf(-f.hi, den, 1.f), f.hi, (float)CUT_OUT * f.hi);
+      if (a.gate != nullptr) {
+        const float open = 1.0f / (1.0f + expf(-a.gate[(long long)(r0 + x) * a.ldg + h]));
+        f.hi *= open;
+        f.lo *= open;
+      }
 #pragma unroll
       for (int c = 0; c < 64; ++c) {
         odd |= !(fabsf(o[c]) <= 3.402823466e38f);
-        o[c] *= f;
+        o[c] = fmaf(o[c], f.hi, o[c] * f.lo);
       }
       if (odd) *odd_s = 1;
     }
@@ -957,15 +990,22 @@ using namespace lp;
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-extern "C" int lp_split_rows(const float* src, long long ld, int M, int K, void* planes, long long ldp, long long plane, void* stream_) {
+static int split_rows(const float* src, long long ld, int M, int K, void* planes, long long ldp, long long plane, const Factor32* factor, void* stream_) {
   LP_REQUIRE(src != nullptr && planes != nullptr, "lp_split_rows: null operand");
   LP_REQUIRE(K % 8 == 0 && ld % 4 == 0 && ldp % 8 == 0 && plane % 8 == 0 && aligned16(src) && aligned16(planes), "lp_split_rows: 16-byte rows of whole eights");
   if (M <= 0 || K <= 0) return 0;
   const long long pieces = (long long)M * (K >> 3);
-  split_rows_kernel<<<(unsigned)((pieces + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(src, ld, M, K, reinterpret_cast<bf16*>(planes), ldp, plane);
+  const unsigned grid = (unsigned)((pieces + 255) / 256);
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  bf16* dst = reinterpret_cast<bf16*>(planes);
+  if (factor != nullptr) split_rows_kernel<true><<<grid, 256, 0, stream>>>(src, ld, M, K, dst, ldp, plane, *factor);
+  else split_rows_kernel<false><<<grid, 256, 0, stream>>>(src, ld, M, K, dst, ldp, plane, Factor32{});
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
+}
+extern "C" int lp_split_rows(const float* src, long long ld, int M, int K, void* planes, long long ldp, long long plane, void* stream) {
+  return split_rows(src, ld, M, K, planes, ldp, plane, nullptr, stream);
 }
 
 template <int BN, int PLANES, bool GATED>
@@ -1090,7 +1130,9 @@ extern "C" int lp_latent_attend_expanded(const lp_latent_desc* d, int R, int n_s
   bf16* c_p = q_p + lx_round((size_t)6 * R * H * 192) / 2;
   bf16* kv_p = c_p + lx_round((size_t)6 * n_keys * width) / 2;
   const long long q_plane = (long long)R * H * 192, c_plane = (long long)n_keys * width;
-  if (int rc = lp_split_rows(d->q, d->ldq, R, H * 192, q_p, (long long)H * 192, q_plane, stream_)) return rc;
+  float cap;
+  const Factor32 factor = scale32(d->scale, 0.f, cap);
+  if (int rc = split_rows(d->q, d->ldq, R, H * 192, q_p, (long long)H * 192, q_plane, &factor, stream_)) return rc;
   const Seqs32 seqs = {n_seqs, d->window, seq_row0, seq_pos0, 0, 0, 0};
   const long long pieces = (long long)n_keys * (width >> 3);
   gather_keys_kernel<<<(unsigned)((pieces + 255) / 256), 256, 0, stream>>>(seqs, n_keys, d->cache, d->page_size, d->page_table, d->max_pages, nullptr, nullptr, 0,
@@ -1124,7 +1166,7 @@ extern "C" int lp_latent_attend_expanded(const lp_latent_desc* d, int R, int n_s
     if (int rc = make_tmap_bf16_3d(&tv, kv_p + 128 * g, 128ULL * g, n_keys, 3, ld, plane, 64, 64, 1)) return rc;
     Attn32Args a = {};
     a.seqs = seqs; a.head0 = h0; a.ratio = 1;
-    a.scale = d->scale; a.out_scale = 1.0f; a.sink = d->sink; a.gate = d->gate; a.ldg = d->ldg;
+    a.out_scale = 1.0f; a.sink = d->sink; a.gate = d->gate; a.ldg = d->ldg;
     a.out_gate = out_gate; a.ldog = ldog;
     a.out = out; a.ldo = ldo; a.out_fp32 = out_fp32;
     a.q = q_p; a.ldq = H * 192LL; a.q_plane = q_plane;
@@ -1164,7 +1206,9 @@ extern "C" int lp_window_attn_prompt(const lp_window_attn_desc* d, int R, int n_
   bf16* q_p = reinterpret_cast<bf16*>(ws);
   bf16* kv_p = q_p + lx_round((size_t)6 * R * H * 128) / 2;
   const long long q_plane = (long long)R * H * 128, plane = (long long)n_keys * row;
-  if (int rc = lp_split_rows(d->qkv + d->q_off, d->ld, R, H * 128, q_p, (long long)H * 128, q_plane, stream_)) return rc;
+  float cap;
+  const Factor32 factor = scale32(d->scale, d->softcap, cap);
+  if (int rc = split_rows(d->qkv + d->q_off, d->ld, R, H * 128, q_p, (long long)H * 128, q_plane, &factor, stream_)) return rc;
   const Seqs32 seqs = {n_seqs, d->window, seq_row0, seq_pos0, d->chunk, d->keep_first, d->pool};
   const long long pieces = (long long)n_keys * (row >> 3);
   gather_keys_kernel<<<(unsigned)((pieces + 255) / 256), 256, 0, stream>>>(seqs, n_keys, d->cache, d->page_size, d->page_table, d->max_pages, d->pooled,
@@ -1178,7 +1222,7 @@ extern "C" int lp_window_attn_prompt(const lp_window_attn_desc* d, int R, int n_
   if (int rc = make_tmap_bf16_3d(&tv, v_p, (uint64_t)d->kv_heads * 128, n_keys, 3, row, plane, 64, 64, 1)) return rc;
   Attn32Args a = {};
   a.seqs = seqs; a.ratio = H / d->kv_heads;
-  a.scale = d->scale; a.softcap = d->softcap; a.sink_one = d->sink != 0; a.zero_empty = 1;
+  a.cap = cap; a.sink_one = d->sink != 0; a.zero_empty = 1;
   a.out_gate = d->gate; a.ldog = d->ldg; a.out_scale = d->out_scale == 0.f ? 1.f : d->out_scale;
   a.out = out; a.ldo = ldo; a.out_fp32 = out_fp32;
   a.q = q_p; a.ldq = H * 128LL; a.q_plane = q_plane;

@@ -33,7 +33,7 @@ static CUtensorMap tmap3(const void* base, uint64_t d0, uint64_t d1, uint64_t d2
 }
 
 extern "C" void emu_split_rows(const float* src, long long ld, int M, int K, void* dst, long long ldd, long long plane) {
-  emu::launch(dim3((unsigned)(((long long)M * (K / 8) + 255) / 256)), dim3(256), [&] { split_rows_kernel(src, ld, M, K, (bf16*)dst, ldd, plane); });
+  emu::launch(dim3((unsigned)(((long long)M * (K / 8) + 255) / 256)), dim3(256), [&] { split_rows_kernel<false>(src, ld, M, K, (bf16*)dst, ldd, plane, Factor32{}); });
 }
 
 extern "C" void emu_gather_keys(int n_seqs, int window, int keep_first, int pool, const int* row0, const int* pos0, int n_keys, const float* cache,
@@ -84,7 +84,15 @@ extern "C" void emu_attn32(const void* q, const void* k, const void* kr, const v
   const int dq = kr != nullptr ? 192 : 128;
   Attn32Args a = {};
   a.seqs = {n_seqs, window, row0, pos0, chunk, keep_first, pool};
-  a.ratio = ratio; a.scale = scale; a.softcap = softcap; a.sink_one = sink_one; a.out_scale = 1.0f;
+  a.ratio = ratio; a.sink_one = sink_one; a.out_scale = 1.0f;
+  // the queries again as the host function has them cut: times their factor
+  const long long n = (long long)R * heads * dq;
+  std::vector<float> rows(n);
+  for (long long i = 0; i < n; ++i) rows[i] = s32_value((const bf16*)q + i, n);
+  std::vector<bf16> scaled(3 * n);
+  const Factor32 factor = scale32(scale, softcap, a.cap);
+  emu::launch(dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), [&] { split_rows_kernel<true>(rows.data(), heads * dq, R, heads * dq, scaled.data(), heads * dq, n, factor); });
+  q = scaled.data();
   a.sink = sink; a.gate = gate; a.ldg = heads; a.out_gate = out_gate; a.ldog = heads * 128;
   a.out = out; a.ldo = heads * 128; a.out_fp32 = out_fp32;
   a.q = (const bf16*)q; a.k = (const bf16*)k; a.kr = (const bf16*)kr; a.v = (const bf16*)v;
