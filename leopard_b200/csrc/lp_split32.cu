@@ -926,7 +926,7 @@ attn32_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       bool odd = false;
       const bool empty = den == 0.f && a.sink == nullptr && a.zero_empty;
       Factor32 f = {empty ? 0.f : 1.0f / den, 0.f};
-      if (!empty) f.lo = fmaf(fmaf(-f.hi, den, 1.f), f.hi, (float)CUT_OUT * f.hi);
+      if (!empty) f.lo = fmaf(fmaf(-f.hi, den, 1.f), f.hi, den > 1.f ? (float)CUT_OUT * f.hi : 0.f);      // (one key: its value as it is)
       if (a.gate != nullptr) {
         const float open = 1.0f / (1.0f + expf(-a.gate[(long long)(r0 + x) * a.ldg + h]));
         f.hi *= open;

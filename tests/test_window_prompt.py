@@ -116,6 +116,13 @@ def test_portions_of_two_requests(form, dtype, monkeypatch):
         assert -1 in eng.cache.get(0).pages
 
 
+def test_a_row_that_sees_one_key_has_its_value():
+    """exactly: its weight is one, and the value's three terms add up to it"""
+    eng, m = engine(64, 2, chunk=16)
+    got, _, want = portion(eng, m, (200,), 0)
+    assert torch.equal(got[::16], want[::16])
+
+
 @pytest.mark.parametrize("bad", [math.inf, math.nan])
 def test_a_value_that_is_not_finite_stays_with_the_rows_that_see_it(bad, monkeypatch):
     monkeypatch.setattr(seqlm, "WINDOW_TILE_ROWS", 0)
