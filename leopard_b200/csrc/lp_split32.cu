@@ -187,6 +187,9 @@ __device__ __forceinline__ float gemm32_gated(float z, float u, float rs) {
   z *= rs;
   return z / (1.0f + expf(-z)) * (u * rs);
 }
+// What cutting off takes on average from a gated unit of three-term products: 0.6e-7 from each of its sums at every K from 64 to 8192 (1.29e-7 to 1.40e-7 of
+// the result; without it both products of 8 experts, width and inside 512, were 2.42e-7 of the result off, with it 1.90, lp_linear_grouped 2.22; 1024 2.69, 2.19, 2.60)
+constexpr float CUT_GATED = 1.3e-7f;
 __device__ __noinline__ void gemm32_mend(const Gemm32Args& a, int row, int group, int col0, int cols, int gated) {
   s32_serial();
   const bf16* W = a.W + (long long)group * a.w_group;
@@ -363,7 +366,10 @@ gemm32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
                 v[i] = gemm32_gated(acc[g * 8 + i], acc[COLS / 2 + g * 8 + i], rs);
-                if (PLANES == 3) odd |= v[i] != v[i];
+                if (PLANES == 3) {
+                  v[i] = fmaf(v[i], CUT_GATED, v[i]);
+                  odd |= v[i] != v[i];
+                }
               }
               const long long at = (long long)row * a.ldc + col;
               if (a.out == G32_OUT_F32) {
