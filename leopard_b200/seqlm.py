@@ -37,11 +37,12 @@ TENSOR_CORE_MIN_ROWS = 64
 # whose sums are cut off: 2.1e-6 of the result at K = 2048, 9.1e-6 at 8192, against 2.3e-7 streamed and 3.9e-7, 9.6e-7 of fp32 multiply-adds.  So
 # it has the products of 64 rows and more, as large prompts always had; at 64 rows only those above the crossing.
 STREAM_MAX_OUTPUTS = 170_000
-# fp32 rows of more than 64 go to the tcgen05 product of three bf16 terms, a pass for the terms included (us, lp_linear and this one): 65 rows, K = 64,
-# 128 columns 8.5, 6.5; K = 1024, 4096 columns 36, 21; 4000 rows, K = 1024, 4096 columns 388, 105.  Up to 64 rows lp_linear streams the weights: 48 rows,
-# K = 128, 6.7, 7.3, K = 1024 12.5, 20.  (K of less than a k block and columns of less than a tile were not measured: they stay.)  Its second launch costs the
-# host 3 us, so short products of few outputs, which gain up to 8 us in steps that wait for the host, stay too.
-SPLIT_MIN_ROWS, SPLIT_MIN_K, SPLIT_LONG_K, SPLIT_OUTPUTS = 65, 64, 768, 1 << 20
+# fp32 rows of more than 64 go to the tcgen05 product of three bf16 terms where K is long, a pass for the terms included (us, lp_linear and this one): 65 rows,
+# K = 1024, 4096 columns 36, 21; 4000 rows, K = 1024, 4096 columns 388, 105.  Up to 64 rows lp_linear streams the weights: 48 rows, K = 1024 12.5, 20.  What the
+# tensor cores cut off does not depend on K while lp_linear's roundings grow with it, so a short K stays although it would be faster too (65 rows, K = 64, 128
+# columns 8.5, 6.5): error against 64 bits, 1e-7 of the result, K = 64 0.65, 0.77; 256 0.82, 0.88; 512 0.97, 0.96 (0.79, 0.81 where rows and weights have a mean); 768
+# 1.10, 1.03, but squared 1.89, 2.02; 1024 1.21, 1.09, a gated unit 2.04, 1.95; 4096 2.13, 1.66.  Columns of less than a tile were not measured: they stay.
+SPLIT_MIN_ROWS, SPLIT_MIN_K = 65, 1024
 # Rows of prompts expand the visible latents into every head's keys and values (lp_latent_attend_expanded), unless many requests bring a few rows each:
 # its tiles are 128 rows of one request.  A layer of width 1024 with 8 heads (us, lp_latent_attend_tiles and this one): one request of 20 rows 64, 45, of
 # 500 297, 85; 32 requests of 12 rows 92, 81; 64 of 12 97, 120, of 24 132, 126; width 2048, 16 heads: 4096 rows 6,490, 530; 64 requests of 12 rows 225, 205.
@@ -931,7 +932,7 @@ class SeqLMEngine:
     def _on_split(self, a: torch.Tensor, w: torch.Tensor) -> bool:
         """Whether fp32 rows go to the tcgen05 product of three bf16 terms"""
         (M, K), N = a.shape, w.shape[0]
-        return (self.split_rows is not None and M >= self.split_rows and a.dtype == F32 and N >= 128 and K >= SPLIT_MIN_K and (K >= SPLIT_LONG_K or M * N >= SPLIT_OUTPUTS) and N % 8 == 0 and K % 8 == 0
+        return (self.split_rows is not None and M >= self.split_rows and a.dtype == F32 and N >= 128 and K >= SPLIT_MIN_K and N % 8 == 0 and K % 8 == 0
                 and a.stride(0) % 4 == 0 and w.stride(0) % 8 == 0 and a.stride(1) == 1 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
     def _split_product(self, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias) -> None:
