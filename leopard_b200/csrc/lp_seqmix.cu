@@ -548,6 +548,7 @@ __device__ __forceinline__ float* lat_cache_row(const LatArgs& a, int seq, int p
 
 // A CTA a row; the row's sines and cosines are taken once for all heads (four a pair and head before: one row of 16 heads 7.0 us).
 constexpr int LAT_PREP_THREADS = 128, LAT_PREP_WIDE = 512, LAT_PREP_ROWS = 296;      // few rows (decoding) take wide CTAs
+constexpr int LAT_PREP_PAIRS = 4096;      // rotation pairs whose sines and cosines shared memory holds; with more of them each is taken where it is used
 __global__ void __launch_bounds__(LAT_PREP_WIDE)
 latent_prep_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos) {
   extern __shared__ float dyn_smem[];
@@ -555,14 +556,15 @@ latent_prep_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int*
   const int r = blockIdx.x, tid = threadIdx.x;
   if (r >= R) return;
   const int pos = row_pos[r], half = a.rot_dims >> 1;
-  float* s_sin = dyn_smem;             // [half]
-  float* s_cos = dyn_smem + half;      // [half]
-  for (int i = tid; i < half; i += blockDim.x) {
+  float2* s_turn = reinterpret_cast<float2*>(dyn_smem);      // [half] (cos, sin)
+  const bool table = half <= LAT_PREP_PAIRS;
+  auto make = [&](int i) {
     float sn, cs;
     sincosf((float)pos * a.inv_freq[i], &sn, &cs);
-    s_sin[i] = sn * a.rot_mscale;
-    s_cos[i] = cs * a.rot_mscale;
-  }
+    return make_float2(cs * a.rot_mscale, sn * a.rot_mscale);
+  };
+  auto turn = [&](int i) { return table ? s_turn[i] : make(i); };
+  for (int i = tid; table && i < half; i += blockDim.x) s_turn[i] = make(i);
   __syncthreads();
   if (a.dkv != nullptr) {      // the layer brings latents of its own
     const float* src = a.dkv + (long long)r * a.lddkv;
@@ -582,8 +584,9 @@ latent_prep_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int*
     for (int i = tid; i < a.rot_dim - half; i += blockDim.x) {      // a pair, or a dimension that is not rotated
       if (i < half) {
         const int d0 = a.rot_layout == LP_ROT_INTERLEAVED ? 2 * i : i, d1 = a.rot_layout == LP_ROT_INTERLEAVED ? 2 * i + 1 : i + half;
-        y[d0] = x[d0] * s_cos[i] - x[d1] * s_sin[i];
-        y[d1] = x[d1] * s_cos[i] + x[d0] * s_sin[i];
+        const float2 t = turn(i);
+        y[d0] = x[d0] * t.x - x[d1] * t.y;
+        y[d1] = x[d1] * t.x + x[d0] * t.y;
       } else {
         y[half + i] = x[half + i];
       }
@@ -597,7 +600,8 @@ latent_prep_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int*
     const int i = p % half;
     const int d0 = a.rot_layout == LP_ROT_INTERLEAVED ? 2 * i : i;
     const int d1 = a.rot_layout == LP_ROT_INTERLEAVED ? 2 * i + 1 : i + half;
-    const float u = x[d0] * s_cos[i] - x[d1] * s_sin[i], v = x[d1] * s_cos[i] + x[d0] * s_sin[i];
+    const float2 t = turn(i);
+    const float u = x[d0] * t.x - x[d1] * t.y, v = x[d1] * t.x + x[d0] * t.y;
     x[d0] = u;
     x[d1] = v;
   }
@@ -1113,8 +1117,8 @@ extern "C" int lp_latent_prep(const lp_latent_desc* d, int R, const int* row_seq
   if (int rc = fill_lat(a, d)) return rc;
   LP_REQUIRE((d->dkv == nullptr || d->c_gain != nullptr) && row_seq != nullptr && row_pos != nullptr, "lp_latent_prep: null operand");
   if (R <= 0) return 0;
-  LP_REQUIRE(d->rot_dims <= 12 * 1024, "lp_latent_prep: rot_dims=%d", d->rot_dims);
-  latent_prep_kernel<<<R, R <= LAT_PREP_ROWS ? LAT_PREP_WIDE : LAT_PREP_THREADS, d->rot_dims * sizeof(float), stream>>>(a, R, row_seq, row_pos);
+  const size_t smem = d->rot_dims / 2 <= LAT_PREP_PAIRS ? d->rot_dims / 2 * sizeof(float2) : 0;
+  latent_prep_kernel<<<R, R <= LAT_PREP_ROWS ? LAT_PREP_WIDE : LAT_PREP_THREADS, smem, stream>>>(a, R, row_seq, row_pos);
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
