@@ -43,10 +43,16 @@ STREAM_MAX_OUTPUTS = 170_000
 # columns 8.5, 6.5): error against 64 bits, 1e-7 of the result, K = 64 0.65, 0.77; 256 0.82, 0.88; 512 0.97, 0.96 (0.79, 0.81 where rows and weights have a mean); 768
 # 1.10, 1.03, but squared 1.89, 2.02; 1024 1.21, 1.09, a gated unit 2.04, 1.95; 4096 2.13, 1.66.  Columns of less than a tile were not measured: they stay.
 SPLIT_MIN_ROWS, SPLIT_MIN_K = 65, 1024
-# Rows of prompts expand the visible latents into every head's keys and values (lp_latent_attend_expanded), unless many requests bring a few rows each:
-# its tiles are 128 rows of one request.  A layer of width 1024 with 8 heads (us, lp_latent_attend_tiles and this one): one request of 20 rows 64, 45, of
-# 500 297, 85; 32 requests of 12 rows 92, 81; 64 of 12 97, 120, of 24 132, 126; width 2048, 16 heads: 4096 rows 6,490, 530; 64 requests of 12 rows 225, 205.
-EXPAND_TILES, EXPAND_TILE_ROWS = 32, 24
+# Rows of prompts expand the visible latents into every head's keys and values (lp_latent_attend_expanded) or attend over the latents themselves
+# (lp_latent_attend_tiles), whichever `latent_route` expects to be done first: the first pays 1.4 (rank 128) to 2 ns (512) for every visible key and
+# head, however few rows see it, the second about 80 GFMA/s a CTA of 64 (row, head) pairs over keys of 2 rank + 64.  Its figures are fitted to 366 steps of 4 to
+# 32 heads over latents of 128 to 512 (1 to 128 requests of 1 to 4096 rows behind 0 to 64,000 tokens, windows of 100 to 2048 keys and none, both precisions), of
+# which it picks the slower way 7 times, by 7 to 23 %.  Some of them (us, tiles and expanded), 16 heads of rank 512: one request of 17 rows 123, 99, behind 4000 tokens
+# 3,377, 382; a prompt of 20 rows beside 7 running requests of 2000 tokens 1,731, 562, beside 31 of 2000 1,744, 2,768, of 8000 6,670, 14,829; of 2000 rows beside 31
+# of 2000 4,526, 2,891; 64 requests of 4 rows behind 4000 tokens 3,422, 11,767, of 48 rows 20,478, 11,934.
+EXPAND_GROUP_BYTES = 512 << 20      # heads whose keys and values are held at a time (csrc/lp_split32.cu): each group of heads walks a request's keys anew
+# What planes of earlier tokens' keys may take; beyond that, and where the allocation fails, the kernels that read the cache itself have the rows
+SCRATCH_BYTES = 1 << 30
 # Window attention of prompts goes to lp_window_attn_prompt (128 rows of a request and a head a CTA) where its tiles are filled and there is enough work that the
 # device's time counts: its launches cost the host some 15 us a layer more, and steps of fewer rows wait for the host.  A layer, preparation
 # included (us on the device, lp_window_attn_tiles and this one; heads on a quarter of key / value heads): one request of 500 rows, 8 heads 86, 45, 16 heads 150, 55; of
@@ -342,6 +348,30 @@ WKV_MIXES = ("r", "k", "v", "g", "w")      # the order of a WKV mixer's operands
 def expands(m: LatentAttentionConfig) -> bool:
     """whether lp_latent_attend_expanded has kernels for these heads"""
     return m.dim == 128 and m.vdim == 128 and m.rot_dim == 64 and m.kv_rank % 8 == 0
+
+
+def latent_route(starts, lens, heads: int, rank: int, window: Optional[int], sms: int) -> Tuple[float, float, int, int]:
+    """(microseconds of lp_latent_attend_tiles with its two head products, of lp_latent_attend_expanded, tiles of 128 rows, visible keys) of one step"""
+    keys = tiles = ctas = 0
+    tile_keys = cta_keys = 0.0             # summed over tiles of 128 rows, and over CTAs of 64 (row, head) pairs of a chunk of 32
+    longest = longest_tile = 0
+    for p, n in zip(starts, lens):
+        def seen(block):                   # by the last and by the average `block` rows of this request
+            few = min(n, block)
+            last, mean = p + n, p + (n + few) / 2
+            return (min(last, window + few - 1), min(mean, window + few - 1)) if window else (last, mean)
+        last, mean = seen(128)
+        t = -(-n // 128)
+        tiles, tile_keys, longest_tile = tiles + t, tile_keys + t * mean, max(longest_tile, last)
+        last, mean = seen(_lib.RETENTION_CHUNK)
+        full, rest = divmod(n, _lib.RETENTION_CHUNK)
+        c = full * -(-_lib.RETENTION_CHUNK * heads // 64) + -(-rest * heads // 64)
+        ctas, cta_keys, longest = ctas + c, cta_keys + c * mean, max(longest, last)
+        keys += p + n - (max(0, p - window + 1) if window else 0)
+    groups = -(-heads // max(1, min(heads, EXPAND_GROUP_BYTES // (keys * 1536))))
+    by_tiles = 90 + 64 * (2 * rank + 64) * 1.21e-5 * max(longest, cta_keys / ctas * -(-ctas // sms)) + sum(lens) * heads * rank * 2.2e-5
+    expanded = 60 + keys * heads * max(0.0008, 0.0022 - 0.1 / rank) + max(groups * (17 + 0.055 * longest_tile), (17 * tiles + 0.055 * tile_keys) * heads / sms)
+    return by_tiles, expanded, tiles, keys
 
 
 def _pad_rows(t: torch.Tensor, n: int) -> torch.Tensor:
@@ -719,7 +749,8 @@ class _Batch:
         self.decode = all(ln == 1 for ln in lens)
         self.longest_chunk = min(max(lens), _lib.RETENTION_CHUNK)
         pos0 = np.fromiter([s.length for s in seqs], np.int32, n)
-        self.starts = pos0
+        self.starts = pos0.tolist()
+        self.latent_routes: Dict[tuple, tuple] = {}      # of this step's latent layers, by their sizes
         slot = np.fromiter([s.slot for s in seqs], np.int32, n)
         if self.decode:      # one row a request: every per-row table is a per-request one
             row0 = np.arange(n + 1, dtype=np.int32)
@@ -897,6 +928,7 @@ class SeqLMEngine:
         self.tile_rows = int(self.L.lp_linear_tile_rows())
         # large bf16 products of the serving precision go to the tcgen05 GEMM when the library has it (the native ones do)
         self.tensor_core_rows = TENSOR_CORE_MIN_ROWS if dtype == "bfloat16" and hasattr(self.L, "lp_gemm_bf16") else None
+        self.sms = torch.cuda.get_device_properties(self.device).multi_processor_count if self.device.type == "cuda" else 1
         self.split_rows = SPLIT_MIN_ROWS if hasattr(self.L, "lp_linear_split") and self.device.type == "cuda" else None
         self.tap: Optional[Callable[[int, torch.Tensor], None]] = None   # called with (layer, residual stream) after every layer
         # decode steps are launch-bound: a batch layout (requests, page-table width) that comes back is captured into a CUDA graph on
@@ -1134,9 +1166,9 @@ class SeqLMEngine:
                             sink=_lib.ptr(lw.get("sink")), gate=_lib.ptr(head_gate), ldg=qd.stride(0) if head_gate is not None else 0)
         self._check(self.L.lp_latent_prep(C.byref(d), b.R, _lib.ptr(b.row_seq), _lib.ptr(b.row_pos), self._stream()), "lp_latent_prep")
         if "w_kv" in lw and not b.decode and b.R > _lib.LATENT_SPLIT_ROWS and q.stride(0) % 4 == 0 and hasattr(self.L, "lp_latent_attend_expanded"):
-            tiles = sum(-(-ln // 128) for ln in b.lens)
-            if tiles <= EXPAND_TILES or b.R >= EXPAND_TILE_ROWS * tiles:
-                return self.linear(self._latent_expanded(m, lw, d, b, tiles, out_gate), lw["w_o"], F32, into=into)
+            room = self._room_to_expand(m, b)
+            if room is not None:
+                return self.linear(self._latent_expanded(m, lw, d, b, *room, out_gate), lw["w_o"], F32, into=into)
         q_abs = self._empty((b.R, m.heads * m.kv_rank), F32)
         self.linear_heads(q, per, lw["w_ukT"], q_abs, m.kv_rank)
         lat = self._empty((b.R, m.heads * m.kv_rank), self.act)
@@ -1152,16 +1184,33 @@ class SeqLMEngine:
         self.linear_heads(lat, m.kv_rank, lw["w_uv"].view(m.heads, m.vdim, m.kv_rank), o, m.vdim, gate=out_gate)
         return self.linear(o, lw["w_o"], F32, into=into)
 
-    def _latent_expanded(self, m: LatentAttentionConfig, lw, d, b: _Batch, tiles: int, out_gate) -> torch.Tensor:
-        """rows of prompts [R, heads * vdim]: every head's keys and values are made from the visible latents"""
-        keys = sum(int(p) + ln - (max(0, int(p) - m.window + 1) if m.window else 0) for p, ln in zip(b.starts, b.lens))
-        o = self._empty((b.R, m.heads * m.vdim), self.act)
+    def _scratch(self, nbytes: int) -> Optional[torch.Tensor]:
+        """room that a faster way wants, or None where the device has none left"""
+        try:
+            return self._empty((nbytes,), torch.uint8)
+        except torch.OutOfMemoryError:
+            return None
+
+    def _room_to_expand(self, m: LatentAttentionConfig, b: _Batch) -> Optional[Tuple[int, int, torch.Tensor]]:
+        """tiles, visible keys and scratch of lp_latent_attend_expanded; None where it is not the faster way for this step or its scratch is too large"""
+        sizes = (m.heads, m.kv_rank, m.window)
+        if sizes not in b.latent_routes:
+            b.latent_routes[sizes] = latent_route(b.starts, b.lens, *sizes, self.sms)
+        by_tiles, expanded, tiles, keys = b.latent_routes[sizes]
+        if by_tiles < expanded:
+            return None
         nbytes = int(self.L.lp_latent_expanded_workspace_bytes(b.R, m.heads, m.dim, m.rot_dim, m.kv_rank, keys))
-        ws = self._empty((nbytes,), torch.uint8)
+        # the other way holds a query and a sum of latents for every row and head
+        ws = self._scratch(nbytes) if nbytes <= max(SCRATCH_BYTES, b.R * m.heads * m.kv_rank * (4 + self.act.itemsize)) else None
+        return None if ws is None else (tiles, keys, ws)
+
+    def _latent_expanded(self, m: LatentAttentionConfig, lw, d, b: _Batch, tiles: int, keys: int, ws: torch.Tensor, out_gate) -> torch.Tensor:
+        """rows of prompts [R, heads * vdim]: every head's keys and values are made from the visible latents"""
+        o = self._empty((b.R, m.heads * m.vdim), self.act)
         w = lw["w_kv"]
         rc = self.L.lp_latent_attend_expanded(C.byref(d), b.R, b.n, _lib.ptr(b.seq_row0), _lib.ptr(b.seq_pos0), tiles, keys, _lib.ptr(w), w.stride(0),
                                               _lib.ptr(out_gate), out_gate.stride(0) if out_gate is not None else 0, _lib.ptr(o), o.stride(0),
-                                              int(o.dtype == F32), _lib.ptr(ws), nbytes, self._stream())
+                                              int(o.dtype == F32), _lib.ptr(ws), ws.numel(), self._stream())
         self._check(rc, "lp_latent_attend_expanded")
         return o
 
@@ -1252,7 +1301,7 @@ class SeqLMEngine:
             lo = max(0, pos - d.window + 1) if d.window > 0 else 0
             return max(lo, pos // d.chunk * d.chunk) if d.chunk else lo
         keys = 0
-        for p, ln in zip(b.starts.tolist(), b.lens):
+        for p, ln in zip(b.starts, b.lens):
             past = p + ln - d.window if d.window > 0 else 0      # positions wholly before the last row's window
             keys += min(d.keep_first, first(p + ln - 1)) + (past // d.pool if d.pool and past > 0 else 0) + p + ln - first(p)
         row = m.kv_heads * 128 * (1 if m.values_are_keys else 2)

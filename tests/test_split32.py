@@ -360,6 +360,46 @@ def test_a_latent_that_is_not_finite_stays_with_the_rows_that_see_it(bad):
     assert float((got[50:].double() - want[50:].double()).norm() / want[50:].double().norm()) < 3e-6      # the bound of the test above
 
 
+@pytest.mark.parametrize("reqs,heads,rank,window,expands", [
+    ([(0, 17)], 16, 512, None, True), ([(64000, 17)], 16, 512, None, True), ([(0, 4096)], 16, 512, 1024, True), ([(3000, 64)], 8, 256, 512, True),
+    ([(8000, 1)] * 31 + [(0, 20)], 16, 512, None, False), ([(8000, 1)] * 31 + [(0, 20)], 8, 256, None, False),
+    ([(2000, 1)] * 31 + [(0, 500)], 16, 512, None, False), ([(2000, 1)] * 31 + [(0, 2000)], 16, 512, None, True), ([(2000, 1)] * 7 + [(0, 20)], 16, 512, None, True),
+    ([(4000, 4)] * 64, 16, 512, None, False), ([(4000, 48)] * 64, 16, 512, None, True), ([(0, 12)] * 128, 8, 256, None, False), ([(0, 24)] * 64, 8, 256, 512, True),
+    ([(8000, 1)] * 31 + [(0, 20)], 4, 128, 256, True), ([(8000, 1)] * 31 + [(0, 20)], 16, 512, 100, False), ([(8000, 1)] * 31 + [(0, 20)], 32, 512, 2048, False),
+    ([(8000, 1)] * 7 + [(0, 300)], 32, 512, 2048, True), ([(0, 24)] * 64, 16, 128, None, False)])
+def test_which_steps_expand_their_latents(reqs, heads, rank, window, expands):
+    """by the work of either way, measured on both sides: running requests with a long past beside a short prompt do not, portions behind a long past do"""
+    from leopard_b200.seqlm import latent_route
+    by_tiles, expanded, tiles, keys = latent_route([p for p, _ in reqs], [n for _, n in reqs], heads, rank, window, 148)
+    assert (expanded <= by_tiles) == expands
+    assert tiles == sum(-(-n // 128) for _, n in reqs) and keys == sum(p + n - seen(p, window or 0)[2] for p, n in reqs)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("why", ["work", "limit", "full"])
+def test_latents_are_attended_as_they_are_where_expanding_does_not_pay_or_fit(why, monkeypatch):
+    from leopard_b200 import seqlm
+    eng, m = latent_engine("float32", 2, 64, None)
+    batch = seqlm._Batch(eng, [seqlm.StepEntry("a", [1] * 40, [])])
+    h = torch.randn((40, 256), device="cuda")
+    want = eng._latent(0, m, eng.w.layers[0], h, batch).double()
+    if why == "work":
+        batch.latent_routes[(2, 64, None)] = (1.0, 2.0, 1, 40)
+    elif why == "limit":
+        monkeypatch.setattr(seqlm, "SCRATCH_BYTES", 0)
+    else:
+        inner = eng._empty
+
+        def full(shape, dtype):
+            if dtype == torch.uint8:
+                raise torch.OutOfMemoryError("no room")
+            return inner(shape, dtype)
+        eng._empty = full
+    monkeypatch.setattr(eng, "_latent_expanded", None)
+    got = eng._latent(0, m, eng.w.layers[0], h, batch).double()
+    assert float((got - want).norm() / want.norm()) < 3e-6      # the bound of the test above
+
+
 @pytest.mark.gpu
 def test_expanded_heads_in_groups():
     """more keys than all heads' expanded keys and values are held for at a time (512 MB): the heads run in groups, the last one smaller"""
