@@ -51,7 +51,8 @@ SPLIT_MIN_ROWS, SPLIT_MIN_K = 65, 1024
 # 3,377, 382; a prompt of 20 rows beside 7 running requests of 2000 tokens 1,731, 562, beside 31 of 2000 1,744, 2,768, of 8000 6,670, 14,829; of 2000 rows beside 31
 # of 2000 4,526, 2,891; 64 requests of 4 rows behind 4000 tokens 3,422, 11,767, of 48 rows 20,478, 11,934.
 EXPAND_GROUP_BYTES = 512 << 20      # heads whose keys and values are held at a time (csrc/lp_split32.cu): each group of heads walks a request's keys anew
-# What planes of earlier tokens' keys may take; beyond that, and where the allocation fails, the kernels that read the cache itself have the rows
+# What the planes of keys may take that lp_latent_attend_expanded and lp_window_attn_prompt read: the kernels that read the cache itself need none, so they have
+# the rows where it would be more or the allocation fails.  32 requests of 8 key / value heads over 8000 tokens: 3 GB, 7.1 ms with the cache's rows and 4.5 so.
 SCRATCH_BYTES = 1 << 30
 # Window attention of prompts goes to lp_window_attn_prompt (128 rows of a request and a head a CTA) where its tiles are filled and there is enough work that the
 # device's time counts: its launches cost the host some 15 us a layer more, and steps of fewer rows wait for the host.  A layer, preparation
@@ -1306,7 +1307,9 @@ class SeqLMEngine:
             keys += min(d.keep_first, first(p + ln - 1)) + (past // d.pool if d.pool and past > 0 else 0) + p + ln - first(p)
         row = m.kv_heads * 128 * (1 if m.values_are_keys else 2)
         nbytes = int(self.L.lp_window_prompt_workspace_bytes(b.R, m.heads, row, keys))
-        ws = self._empty((nbytes,), torch.uint8)
+        ws = self._scratch(nbytes) if 6 * (keys - b.R) * row <= SCRATCH_BYTES else None      # planes of this step's own rows are of its projection's size
+        if ws is None:
+            return False
         rc = self.L.lp_window_attn_prompt(C.byref(d), b.R, b.n, _lib.ptr(b.seq_row0), _lib.ptr(b.seq_pos0), tiles, keys, _lib.ptr(o), o.stride(0),
                                           int(o.dtype == F32), _lib.ptr(ws), nbytes, self._stream())
         self._check(rc, "lp_window_attn_prompt")

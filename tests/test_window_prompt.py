@@ -64,12 +64,12 @@ def reference(eng, m, lw, batch, qkv):
     return out * torch.sigmoid(qkv[:, qkv.shape[1] - H * D:].double()) if m.out_gate else out
 
 
-def portion(eng, m, lens, seed, plant=None):
+def portion(eng, m, lens, seed, plant=None, expect=True):
     """one step of requests 0, 1, .. : its results by both kernels and in 64 bits"""
     lw, parts = eng.w.layers[0], m.heads + m.kv_heads * (1 if m.values_are_keys else 2) + (m.heads if m.out_gate else 0)
     batch = _Batch(eng, [StepEntry(i, [1] * n, []) for i, n in enumerate(lens)])
     raw = torch.randn((batch.R, parts * D), device="cuda", generator=torch.Generator("cuda").manual_seed(seed))
-    got, taken, inner = [], [], eng._window_prompt
+    got, taken, inner = [], [], eng._window_prompt      # `taken`: whether lp_window_attn_prompt has had them
     if plant is not None:
         plant(batch)
     for take in (True, False):
@@ -78,7 +78,7 @@ def portion(eng, m, lens, seed, plant=None):
         eng._window_heads(0, m, lw, raw, batch, o, qkv)
         got.append(o.double())
     eng._window_prompt = inner
-    assert taken == [True, False]
+    assert taken == [expect, False]
     want = reference(eng, m, lw, batch, qkv)
     for s, n in zip(batch.seqs, batch.lens):
         eng.cache.advance(s, n)
@@ -168,3 +168,21 @@ def test_both_sides_of_the_rule(heads, lens, taken):
     eng.L = Spy()
     eng._window_heads(0, m, eng.w.layers[0], qkv, batch, torch.empty((batch.R, heads * D), device="cuda"), qkv)
     assert calls[-1] == ("lp_window_attn_prompt" if taken else "lp_window_attn_tiles")
+
+
+def test_rows_that_leave_no_room_for_planes(monkeypatch):
+    """earlier tokens' planes beyond the limit, or an allocation that fails: lp_window_attn_tiles has the rows; this step's own planes have no limit"""
+    monkeypatch.setattr(seqlm, "SCRATCH_BYTES", 6 * 299 * 2 * D)
+    eng, m = engine(64, 1)
+    for seed, (n, expect) in enumerate([(299, True), (130, True), (130, False)]):      # behind 0, 299 and 429 tokens
+        got, tiles, want = portion(eng, m, (n,), seed, expect=expect)
+        assert error(got, want) < 4e-7 and (expect or torch.equal(got, tiles))
+    inner = eng._empty
+
+    def full(shape, dtype):
+        if dtype == torch.uint8:
+            raise torch.OutOfMemoryError("no room")
+        return inner(shape, dtype)
+    monkeypatch.setattr(seqlm, "SCRATCH_BYTES", 1 << 30)
+    eng._empty = full
+    portion(eng, m, (130,), 9, expect=False)
