@@ -1166,7 +1166,7 @@ class SeqLMEngine:
                             page_table=_lib.ptr(b.page_table), max_pages=b.max_pages, window=m.window or 0, scale=m.scale,
                             sink=_lib.ptr(lw.get("sink")), gate=_lib.ptr(head_gate), ldg=qd.stride(0) if head_gate is not None else 0)
         self._check(self.L.lp_latent_prep(C.byref(d), b.R, _lib.ptr(b.row_seq), _lib.ptr(b.row_pos), self._stream()), "lp_latent_prep")
-        if "w_kv" in lw and not b.decode and b.R > _lib.LATENT_SPLIT_ROWS and q.stride(0) % 4 == 0 and hasattr(self.L, "lp_latent_attend_expanded"):
+        if "w_kv" in lw and not b.decode and b.R > _lib.LATENT_SPLIT_ROWS and q.stride(0) % 4 == 0 and q.data_ptr() % 16 == 0 and hasattr(self.L, "lp_latent_attend_expanded"):
             room = self._room_to_expand(m, b)
             if room is not None:
                 return self.linear(self._latent_expanded(m, lw, d, b, *room, out_gate), lw["w_o"], F32, into=into)

@@ -401,6 +401,19 @@ def test_latents_are_attended_as_they_are_where_expanding_does_not_pay_or_fit(wh
 
 
 @pytest.mark.gpu
+def test_queries_off_16_byte_boundaries_are_attended_too():
+    """columns of a wider product at an odd offset: the expanded keys' kernel reads 16 bytes at a time, the other one takes them as they are"""
+    from leopard_b200.seqlm import StepEntry, _Batch
+    eng, m = latent_engine("float32", 2, 64, None)
+    batch = _Batch(eng, [StepEntry("a", [1] * 40, [])])
+    qd = torch.randn((40, 2 * 192 + 128), device="cuda")
+    shifted = torch.empty((40, qd.shape[1] + 4), device="cuda")[:, 1:1 + qd.shape[1]].copy_(qd)
+    want = eng._latent(0, m, eng.w.layers[0], None, batch, proj=qd).double()
+    got = eng._latent(0, m, eng.w.layers[0], None, batch, proj=shifted).double()
+    assert float((got - want).norm() / want.norm()) < 3e-6      # the bound of the test above
+
+
+@pytest.mark.gpu
 def test_expanded_heads_in_groups():
     """more keys than all heads' expanded keys and values are held for at a time (512 MB): the heads run in groups, the last one smaller"""
     from leopard_b200.seqlm import StepEntry, _Batch
