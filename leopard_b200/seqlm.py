@@ -1509,9 +1509,10 @@ class SeqLMEngine:
             self._check(L.lp_linear_group_pairs(C.byref(d2), _lib.ptr(idx), f.experts, 1, n_pairs, st), "lp_linear_group_pairs")
             return self._moe_combine(f, lw, h, y, self._pair_rows, None if on_input else wts, gate)
         w_gu, w_dn = lw["w_gu"], lw["w_edown"]
-        # rows enough to fill tensor-core tiles in the serving precision: an expert's rows are gathered into tiles of its own and all experts' products are
-        # one launch, without a look at the tables on the host
-        grouped = (self.split_rows is not None and n_pairs >= f.experts * TENSOR_CORE_MIN_ROWS and epi == _lib.EPI_SILU_GATE
+        # rows enough to fill tensor-core tiles: an expert's rows are gathered into tiles of its own and all experts' products are one launch, without a look at
+        # the tables on the host
+        on_tensor_cores = self.tensor_core_rows if h.dtype == BF16 else self.split_rows
+        grouped = (on_tensor_cores is not None and n_pairs >= f.experts * TENSOR_CORE_MIN_ROWS and epi == _lib.EPI_SILU_GATE
                    and hasattr(L, "lp_gemm_grouped") and D % 16 == 0 and f.expert_ff % 8 == 0 and all(t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (w_gu, w_dn)))
         tile_rows = GROUP_TILE_ROWS if grouped else self.tile_rows
         tiles = int(L.lp_moe_max_tiles(n_pairs, f.experts, tile_rows))

@@ -505,3 +505,28 @@ def test_fp32_experts_are_no_further_from_float64_than_sorted_tiles(T, width, ex
         eng.split_rows = rows
         err.append(rel_err(eng._moe(eng.cfg.layers[0].ff, eng.w.layers[0], h.cuda()), want))
     assert err[0] < err[1], err
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+def test_experts_of_an_engine_without_tensor_core_rows(dtype):
+    """`tensor_core_rows` = None keeps bf16 rows off the tcgen05 products, `split_rows` = None fp32 rows, each only its own"""
+    from oracle import seqlm as O
+    from seqlm_common import make_engine, model, moe, retention_layer
+    cfg = model([retention_layer(mlp=moe(experts=4, top=2, groups=2, keep=2, ff=72, shared=16))], width=80)
+    eng = make_engine(cfg, O.random_weights(cfg, seed=1), ("cuda", None), dtype)
+    calls, lib = [], eng.L
+
+    class Spy:
+        def __getattr__(self, name):
+            f = getattr(lib, name)
+            return (lambda *a: calls.append(name) or f(*a)) if name in ("lp_gemm_grouped", "lp_linear_grouped") else f
+    eng.L = Spy()
+    h, own = torch.randn((1000, 80), device="cuda").to(eng.act), "tensor_core_rows" if dtype == "bfloat16" else "split_rows"
+    for name in ("tensor_core_rows", "split_rows"):
+        saved = getattr(eng, name)
+        setattr(eng, name, None)
+        calls.clear()
+        eng._moe(eng.cfg.layers[0].ff, eng.w.layers[0], h)
+        setattr(eng, name, saved)
+        assert calls == 2 * (["lp_linear_grouped"] if name == own else ["lp_gemm_grouped"])
