@@ -42,6 +42,23 @@ def test_prompts_portions_and_steps(backend, layer, n):
             done[i] += 1
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("layer", [latent_layer(heads=8, dim=4, rot_dim=8, vdim=4, kv_rank=136, window=20), latent_layer(heads=8, dim=4, rot_dim=6, vdim=4, kv_rank=132, window=7),
+                                   latent_layer(heads=8, dim=4, rot_dim=4, vdim=4, kv_rank=512, window=None), latent_layer(heads=8, dim=4, rot_dim=4, vdim=4, kv_rank=20, window=9)],
+                         ids=["rank136", "rank132-rot6", "rank512", "rank20"])
+@pytest.mark.parametrize("n", [37, 38])
+def test_latent_steps_of_more_pairs_than_two_a_processor(layer, n):
+    """8 heads of 37 requests are 296 (row, head) pairs, two an SM, of 38 more: 16 warps a pair, then four"""
+    cfg = model([layer])
+    w = O.random_weights(cfg, seed=1)
+    eng = make_engine(cfg, w, ("cuda", None), max_tokens=1024, max_seqs=n)
+    toks = _prompts(n, cfg["vocab"], [23 - i % 17 for i in range(n)])
+    eng.step([StepEntry(i, t[:-2], [0]) for i, t in enumerate(toks)])
+    for k in (2, 1):
+        got = eng.step([StepEntry(i, [t[-k]], [0]) for i, t in enumerate(toks)])
+        assert rel_err(got, torch.stack([O.forward(cfg, w, t)[-k] for t in toks])) < TOL["float32"]
+
+
 @pytest.mark.parametrize("rot_dims,rot_dim,interleaved", [(8192, 8192, 0), (8194, 8200, 1), (12280, 12280, 0), (12290, 12300, 1)])
 def test_rotation_of_many_dimensions(backend, rot_dims, rot_dim, interleaved):
     """as many pairs as shared memory holds sines and cosines for, one more, and sizes at which such a table would not fit a launch.  Sums of two products of

@@ -415,21 +415,32 @@ def test_queries_off_16_byte_boundaries_are_attended_too():
 
 @pytest.mark.gpu
 def test_expanded_heads_in_groups():
-    """more keys than all heads' expanded keys and values are held for at a time (512 MB): the heads run in groups, the last one smaller"""
-    from leopard_b200.seqlm import StepEntry, _Batch
-    eng, m = latent_engine("float32", 19, 64, None, max_tokens=20480)
-    lw, n = eng.w.layers[0], 19000
-    assert n * 1536 * 19 > 512 << 20
+    """more keys than all heads' expanded keys and values are held for at a time: the heads run in groups, the last one smaller; every 500th row against float64.
+    Scores, their exponentials and 148 tiles of keys are each a few roundings of 2^-24, and the output's product sums 2,432 of them: 1e-6"""
+    from leopard_b200.seqlm import EXPAND_GROUP_BYTES, StepEntry, _Batch
+    H, rank, n = 19, 64, 19000
+    eng, m = latent_engine("float32", H, rank, None, max_tokens=20480)
+    lw, calls, inner = eng.w.layers[0], [], eng._latent_expanded
+    eng._latent_expanded = lambda *a: calls.append(1) or inner(*a)
+    assert n * 1536 * H > EXPAND_GROUP_BYTES
+    w_kv, w_o = lw["w_kv"].double(), lw["w_o"].double()
     for ln in (n, 40):      # a prompt, then a portion over all of it
         batch = _Batch(eng, [StepEntry("a", [1] * ln, [])])
-        h = torch.randn((ln, 256), device="cuda", generator=torch.Generator("cuda").manual_seed(ln))
-        got = eng._latent(0, m, lw, h, batch).double()
-        kv = lw.pop("w_kv")
-        want = eng._latent(0, m, lw, h, batch).double()
-        lw["w_kv"] = kv
-        # a sum over n keys of either sign, one after the other, rounds off 2^-24 sqrt(n / 2) = 6e-6 of itself in the general path
-        assert float((got - want).norm() / want.norm()) < 2e-5
+        qd = torch.randn((ln, H * 192 + rank + 64), device="cuda", generator=torch.Generator("cuda").manual_seed(ln))
+        got = eng._latent(0, m, lw, None, batch, proj=qd)      # queries are turned in place
+        first = batch.seqs[0].length
+        cache = eng.cache.pools[0][torch.tensor(batch.seqs[0].pages, device="cuda")].flatten(0, 1)[:first + ln].double()
+        rows = torch.arange(ln - 1, -1, -500, device="cuda")
+        unseen = torch.arange(first + ln, device="cuda")[None] > first + rows[:, None]
+        heads = []
+        for h in range(H):
+            keys = torch.cat([cache[:, :rank] @ w_kv[h * 128:h * 128 + 128].T, cache[:, rank:]], 1)
+            weights = torch.softmax((qd[rows, h * 192:h * 192 + 192].double() @ keys.T * 192 ** -0.5).masked_fill(unseen, -math.inf), 1)
+            heads.append(weights @ (cache[:, :rank] @ w_kv[(H + h) * 128:(H + h) * 128 + 128].T))
+        want = torch.cat(heads, 1) @ w_o.T
+        assert float((got[rows].double() - want).norm() / want.norm()) < 1e-6
         eng.cache.advance(batch.seqs[0], ln)
+    assert len(calls) == 2
 
 
 @pytest.mark.gpu
