@@ -54,12 +54,15 @@ EXPAND_GROUP_BYTES = 512 << 20      # heads whose keys and values are held at a 
 # What the planes of keys may take that lp_latent_attend_expanded and lp_window_attn_prompt read: the kernels that read the cache itself need none, so they have
 # the rows where it would be more or the allocation fails.  32 requests of 8 key / value heads over 8000 tokens: 3 GB, 7.1 ms with the cache's rows and 4.5 so.
 SCRATCH_BYTES = 1 << 30
-# Window attention of prompts goes to lp_window_attn_prompt (128 rows of a request and a head a CTA) where its tiles are filled and there is enough work that the
-# device's time counts: its launches cost the host some 15 us a layer more, and steps of fewer rows wait for the host.  A layer, preparation
-# included (us on the device, lp_window_attn_tiles and this one; heads on a quarter of key / value heads): one request of 500 rows, 8 heads 86, 45, 16 heads 150, 55; of
-# 4096, 4 heads 101, 62, 16 heads 845, 302; 16 requests of 40, 16 heads 40, 54.  Capped scores and values turned back by position: of 500 rows, 8 heads 102, 76, of
-# 4096, 16 heads 1009, 417.  Whole prompts of three layers: 1,143 rows of 4 heads 764 us, 818 with this one; 4096 of 16 heads 2,927, 1,902.
-WINDOW_TILE_ROWS, WINDOW_WORK = 64, 8000
+# Window attention of prompts goes to lp_window_attn_prompt (128 rows of a request and a head a CTA) where its tiles are filled and the step has enough work that the
+# device's time counts: its launches cost the host 10 to 23 us a layer more, and steps of less work wait for the host.  A layer, preparation included (us on the
+# device, lp_window_attn_tiles and this one; heads on a quarter of key / value heads): one request of 500 rows, 8 heads 89, 54, 16 heads 149, 64; of 4096, 8 heads 487,
+# 188, 16 heads 828, 299; behind 32,000 tokens 512 rows of 16 heads 10,682, 1,469; 32 requests of 70, 16 heads 114, 121.
+# Work is rows x heads x width, what the step's products grow with.  Whole prompts of two windowed layers and a recurrence (us between steps; rows, heads = width / 128),
+# bf16: 2000, 8 (16 M) 484, 504, on a box of slower host 794, 841; 500, 16 (16 M) 450, 460; 550, 16 (18 M) 505, 464; 260, 24 (19 M) 450, 466; 330, 24 (24 M) 504, 466; 3000, 8 (24 M)
+# 679, 537; 8000, 4 (16 M) 643, 666; 12000, 4 (24 M) 867, 777; one windowed layer, 800, 16 (26 M) 326, 331, 1000, 16 (33 M) 600, 573, 6000, 8 (49 M) 613, 522.  Fp32 rows,
+# whose products take longer: 130, 24 (10 M) 674, 683; 200, 24 (15 M) 713, 692; 300, 16 (10 M) 587, 550; 999, 8 (8 M) 931, 847, one windowed layer 597, 601.
+WINDOW_TILE_ROWS, WINDOW_WORK, WINDOW_WORK_F32 = 64, 25_000_000, 10_000_000
 # Up to MOE_PAIRS_MAX (token, choice) pairs an expert's weights are streamed once for the pairs that chose it.  Both products of 16 experts,
 # width 2048, 1024 inside (us, bf16; fp32 rows), against sorted tiles: 128 pairs 66, 108; 85, 182.  256 pairs 93, 108; 138, 182.  512 pairs 161,
 # 108; 282, 182: with this few experts the sorted tiles are ahead from about 300 pairs, with 32 (width 4096) not yet at 512: 554, 683; 876, 1116.
@@ -1295,7 +1298,7 @@ class SeqLMEngine:
                 or qkv.stride(0) % 4 or qkv.data_ptr() % 16 or o.data_ptr() % 16 or o.stride(0) % (4 if o.dtype == F32 else 8)):
             return False
         tiles = sum(-(-ln // 128) for ln in b.lens)
-        if b.R < WINDOW_TILE_ROWS * tiles or b.R * m.heads < WINDOW_WORK:
+        if b.R < WINDOW_TILE_ROWS * tiles or b.R * m.heads * self.cfg.width < (WINDOW_WORK if self.act == BF16 else WINDOW_WORK_F32):
             return False
 
         def first(pos):      # the first token of its window, or of its own block of positions
@@ -1510,7 +1513,9 @@ class SeqLMEngine:
             return self._moe_combine(f, lw, h, y, self._pair_rows, None if on_input else wts, gate)
         w_gu, w_dn = lw["w_gu"], lw["w_edown"]
         # rows enough to fill tensor-core tiles: an expert's rows are gathered into tiles of its own and all experts' products are one launch, without a look at
-        # the tables on the host
+        # the tables on the host.  The line is where a product an expert (bf16) ran on the tensor cores before.  Both products of 64 and of 256 pairs an expert (us,
+        # without and with; 8 experts, width and inside 1024): bf16 600, 97 and 534, 100, fp32 124, 110 and 213, 138; 16 experts, width 2048 859, 104 and 970, 173,
+        # fp32 295, 145 and 701, 307; the nearest fp32 rows: 8 experts of 80 pairs 130, 139, width 512 99, 108
         on_tensor_cores = self.tensor_core_rows if h.dtype == BF16 else self.split_rows
         grouped = (on_tensor_cores is not None and n_pairs >= f.experts * TENSOR_CORE_MIN_ROWS and epi == _lib.EPI_SILU_GATE
                    and hasattr(L, "lp_gemm_grouped") and D % 16 == 0 and f.expert_ff % 8 == 0 and all(t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (w_gu, w_dn)))
