@@ -42,7 +42,10 @@ STREAM_MAX_OUTPUTS = 170_000
 # tensor cores cut off does not depend on K while lp_linear's roundings grow with it, so a short K stays although it would be faster too (65 rows, K = 64, 128
 # columns 8.5, 6.5): error against 64 bits, 1e-7 of the result, K = 64 0.65, 0.77; 256 0.82, 0.88; 512 0.97, 0.96 (0.79, 0.81 where rows and weights have a mean); 768
 # 1.10, 1.03, but squared 1.89, 2.02; 1024 1.21, 1.09, a gated unit 2.04, 1.95; 4096 2.13, 1.66.  Columns of less than a tile were not measured: they stay.
-SPLIT_MIN_ROWS, SPLIT_MIN_K = 65, 1024
+# Its two launches, three where the result is added to the stream, are the host's time in steps that wait for it: whole prompts of small models, whose products of up
+# to a million weights are too short for the device's time to count (us between steps, lp_linear and this one: width 512, 70 rows 578, 619, 600 rows of 20 requests 682,
+# 739, 1500 511, 530; width 1024, whose larger products gain, 70 rows 854, 734), have them from 2^31 multiplications on.
+SPLIT_MIN_ROWS, SPLIT_MIN_K, SPLIT_MIN_WEIGHTS, SPLIT_WORK = 65, 1024, 1 << 21, 1 << 31
 # Rows of prompts expand the visible latents into every head's keys and values (lp_latent_attend_expanded) or attend over the latents themselves
 # (lp_latent_attend_tiles), whichever `latent_route` expects to be done first: the first pays 1.4 (rank 128) to 2 ns (512) for every visible key and
 # head, however few rows see it, the second about 80 GFMA/s a CTA of 64 (row, head) pairs over keys of 2 rank + 64.  Its figures are fitted to 366 steps of 4 to
@@ -968,8 +971,8 @@ class SeqLMEngine:
     def _on_split(self, a: torch.Tensor, w: torch.Tensor) -> bool:
         """Whether fp32 rows go to the tcgen05 product of three bf16 terms"""
         (M, K), N = a.shape, w.shape[0]
-        return (self.split_rows is not None and M >= self.split_rows and a.dtype == F32 and N >= 128 and K >= SPLIT_MIN_K and N % 8 == 0 and K % 8 == 0
-                and a.stride(0) % 4 == 0 and w.stride(0) % 8 == 0 and a.stride(1) == 1 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+        return (self.split_rows is not None and M >= self.split_rows and a.dtype == F32 and N >= 128 and K >= SPLIT_MIN_K and (N * K >= SPLIT_MIN_WEIGHTS or M * N * K >= SPLIT_WORK)
+                and N % 8 == 0 and K % 8 == 0 and a.stride(0) % 4 == 0 and w.stride(0) % 8 == 0 and a.stride(1) == 1 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
     def _split_product(self, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias) -> None:
         M, K = a.shape
@@ -986,8 +989,8 @@ class SeqLMEngine:
         N = w.shape[0]
         n_out = N // 2 if epi in _lib.GATED_EPIS else N
         # a row scale reaches the tensor-core path only through the activation kernel that follows the product
-        split = self._on_split(a, w)
-        tc = (split or self._on_gemm(a, w)) and (row_scale is None or (epi != _lib.EPI_NONE and bias is None))
+        split = a.dtype == F32 and self._on_split(a, w)
+        tc = (split or (a.dtype == BF16 and self._on_gemm(a, w))) and (row_scale is None or (epi != _lib.EPI_NONE and bias is None))
         if into is not None:
             x, mult = into[0], into[1]
             gate = into[2] if len(into) > 2 else None

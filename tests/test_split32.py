@@ -445,9 +445,10 @@ def test_expanded_heads_in_groups():
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("M,N,K", [(65, 128, 1024), (4100, 264, 1032), (1100, 1000, 1400), (257, 4096, 3000)])
-def test_products_of_fp32_rows_in_the_engine(M, N, K):
-    """the split product and its epilogues are no further from float64 than lp_linear's"""
-    from leopard_b200 import _lib
+def test_products_of_fp32_rows_in_the_engine(M, N, K, monkeypatch):
+    """the split product and its epilogues are no further from float64 than lp_linear's (few weights too)"""
+    from leopard_b200 import _lib, seqlm
+    monkeypatch.setattr(seqlm, "SPLIT_MIN_WEIGHTS", 0)
     eng, _ = latent_engine("float32", 2, 64, None)
     g = torch.Generator("cuda").manual_seed(M)
     a, w = torch.randn((M, K + 4), device="cuda", generator=g)[:, :K], torch.randn((N, K), device="cuda", generator=g).to(BF)
@@ -467,9 +468,10 @@ def test_products_of_fp32_rows_in_the_engine(M, N, K):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("M,N,K,split", [(65, 128, 1024, True), (64, 128, 1024, False), (65, 120, 1024, False), (5000, 512, 1016, False), (65, 132, 1024, False)])
+@pytest.mark.parametrize("M,N,K,split", [(65, 2048, 1024, True), (64, 2048, 1024, False), (65, 2040, 1024, False), (65, 2052, 1024, False), (5000, 4096, 1016, False),
+                                         (65, 120, 20000, False), (65, 128, 16384, True), (2048, 1024, 1024, True), (2047, 1024, 1024, False)])
 def test_which_fp32_products_are_split(M, N, K, split):
-    """65 rows, 128 columns, K = 1024 and more: below that lp_linear's sums are the more precise ones (or the faster)"""
+    """65 rows, 128 columns, K = 1024, and 2^21 weights or 2^31 multiplications: below that lp_linear's sums are the more precise ones, or its one launch the faster"""
     eng, _ = latent_engine("float32", 2, 64, None)
     assert eng._on_split(torch.empty((M, K), device="cuda"), torch.empty((N, K), device="cuda", dtype=BF)) == split
 
