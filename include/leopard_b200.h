@@ -724,6 +724,9 @@ int lp_gemm_grouped(const void* A, long long lda, long long a_plane, const void*
  * the requests' rows of this step and the positions these start at; n_tiles = sum of ceil(rows / 128); n_keys = sum over requests of the positions from
  * max(0, seq_pos0 - window + 1) (window <= 0: from 0) to the last.  out_gate (fp32 [rows, ldog] or NULL): every output is multiplied by its sigmoid.
  * out [rows, heads * 128]. */
+/* From the requests' tables on the HOST: whether lp_latent_attend_expanded is expected to be done before lp_latent_attend_tiles and its two head products (1) or not
+ * (0), and the step's n_tiles and n_keys. */
+int lp_latent_route(const int* seq_row0, const int* seq_pos0, int n_seqs, int heads, int kv_rank, int window, int* n_tiles, int* n_keys);
 size_t lp_latent_expanded_workspace_bytes(int R, int heads, int dim, int rot_dim, int kv_rank, int n_keys);
 int lp_latent_attend_expanded(const lp_latent_desc* desc, int R, int n_seqs, const int* seq_row0, const int* seq_pos0, int n_tiles, int n_keys,
                               const void* w_kv, long long ldw, const float* out_gate, long long ldog, void* out, long long ldo, int out_fp32,
@@ -799,6 +802,7 @@ int lp_window_attn_tiles(const lp_window_attn_desc* desc, int R, const int* row_
 /* the same result for the rows of prompts on the tensor cores, heads of 128 without distance bias or mixed heads: 128 rows of a request
  * and a head a CTA (tables as for lp_latent_attend_expanded).  n_keys = sum over requests of the kept tokens and blocks that its last row sees
  * and of its tokens from the first that its first row's window (or own block of positions) holds; row_floats: floats of a cache row. */
+int lp_window_prompt_count(const lp_window_attn_desc* desc, const int* seq_row0, const int* seq_pos0, int n_seqs, int* n_tiles, int* n_keys);      /* from tables on the host */
 size_t lp_window_prompt_workspace_bytes(int R, int heads, int row_floats, int n_keys);
 int lp_window_attn_prompt(const lp_window_attn_desc* desc, int R, int n_seqs, const int* seq_row0, const int* seq_pos0, int n_tiles, int n_keys,
                           void* out, long long ldo, int out_fp32, void* ws, size_t ws_bytes, void* stream);

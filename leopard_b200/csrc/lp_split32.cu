@@ -444,7 +444,7 @@ struct Seqs32 {
 struct Seen32 {
   int keep, blocks, lo;
 };
-__device__ __forceinline__ Seen32 seen32(const Seqs32& q, int pos) {
+__host__ __device__ __forceinline__ Seen32 seen32(const Seqs32& q, int pos) {
   Seen32 v;
   v.lo = q.window > 0 && pos - q.window + 1 > 0 ? pos - q.window + 1 : 0;
   if (q.chunk > 0 && pos / q.chunk * q.chunk > v.lo) v.lo = pos / q.chunk * q.chunk;
@@ -457,7 +457,7 @@ __device__ __forceinline__ Seen32 seen32(const Seqs32& q, int pos) {
 struct Run32 {
   int keep, blocks, lo, count;
 };
-__device__ __forceinline__ Run32 run32(const Seqs32& q, int pos0, int len) {
+__host__ __device__ __forceinline__ Run32 run32(const Seqs32& q, int pos0, int len) {
   const Seen32 last = seen32(q, pos0 + len - 1);
   Run32 r;
   r.keep = last.keep;
@@ -1112,6 +1112,58 @@ static int lx_group(int heads, int n_keys) {
 }
 static size_t lx_round(size_t b) { return (b + 255) & ~(size_t)255; }
 
+// tiles of 128 rows and key rows of a step, from the requests' tables as they lie on the host
+static void count32(const Seqs32& q, int* n_tiles, int* n_keys) {
+  int tiles = 0, keys = 0;
+  for (int s = 0; s < q.n; ++s) {
+    const int len = q.row0[s + 1] - q.row0[s];
+    tiles += (len + 127) / 128;
+    keys += run32(q, q.pos0[s], len).count;
+  }
+  *n_tiles = tiles;
+  *n_keys = keys;
+}
+// Whether a step's latents are expected to be attended sooner with every head's keys and values expanded (1) or as they are (0).  Expanding pays 1.4 ns (rank 128)
+// to 2 ns (512) for every visible key and head, however few rows see it, and then a tile's chain of 55 ns a key; lp_latent_attend_tiles about 80 GFMA/s a CTA of
+// 64 (row, head) pairs of a chunk over keys of 2 rank + 64, one CTA an SM, and its two head products.  The figures (us) are fitted to 366 steps of 4 to 32 heads over
+// latents of 128 to 512 (1 to 128 requests of 1 to 4096 rows behind 0 to 64,000 tokens, windows of 100 to 2048 keys and none, both precisions), of which this picks the
+// slower way 7 times, by 7 to 23 %.  Some of them (tiles and expanded), 16 heads of rank 512: one request of 17 rows 123, 99, behind 4000 tokens 3,377, 382; a prompt of
+// 20 rows beside 7 running requests of 2000 tokens 1,731, 562, beside 31 of 2000 1,744, 2,768, of 8000 6,670, 14,829; of 2000 rows beside 31 of 2000 4,526, 2,891;
+// 64 requests of 4 rows behind 4000 tokens 3,422, 11,767, of 48 rows 20,478, 11,934.
+extern "C" int lp_latent_route(const int* seq_row0, const int* seq_pos0, int n_seqs, int heads, int kv_rank, int window, int* n_tiles, int* n_keys) {
+  const Seqs32 q = {n_seqs, window, seq_row0, seq_pos0, 0, 0, 0};
+  count32(q, n_tiles, n_keys);
+  const int sms = sm_count();
+  double ctas = 0, cta_keys = 0, longest = 0, tile_keys = 0, longest_tile = 0;
+  for (int s = 0; s < n_seqs; ++s) {
+    const double pos0 = seq_pos0[s];
+    const int len = seq_row0[s + 1] - seq_row0[s];
+    auto seen = [&](int block, double& last, double& mean) {      // keys of the last and of the average `block` rows
+      const int few = len < block ? len : block;
+      last = pos0 + len;
+      mean = pos0 + (len + few) / 2.0;
+      if (window > 0 && last > window + few - 1) last = window + few - 1;
+      if (window > 0 && mean > window + few - 1) mean = window + few - 1;
+    };
+    double last, mean;
+    seen(128, last, mean);
+    tile_keys += (len + 127) / 128 * mean;
+    longest_tile = last > longest_tile ? last : longest_tile;
+    seen(LP_RETENTION_CHUNK, last, mean);
+    const double c = (double)(len / LP_RETENTION_CHUNK) * ((LP_RETENTION_CHUNK * heads + 63) / 64) + (len % LP_RETENTION_CHUNK * heads + 63) / 64;
+    ctas += c;
+    cta_keys += c * mean;
+    longest = last > longest ? last : longest;
+  }
+  if (ctas == 0) return 0;
+  const double waves = cta_keys / ctas * (double)(((long long)ctas + sms - 1) / sms);
+  const double tiles_us = 90 + 64.0 * (2 * kv_rank + 64) * 1.21e-5 * (waves > longest ? waves : longest) + (double)seq_row0[n_seqs] * heads * kv_rank * 2.2e-5;
+  const int groups = (heads + lx_group(heads, *n_keys) - 1) / lx_group(heads, *n_keys);      // each walks a request's keys anew
+  const double chain = groups * (17 + 0.055 * longest_tile), all = (17.0 * *n_tiles + 0.055 * tile_keys) * heads / sms, a_key = 0.0022 - 0.1 / kv_rank;
+  const double expanded_us = 60 + (double)*n_keys * heads * (a_key > 0.0008 ? a_key : 0.0008) + (chain > all ? chain : all);
+  return expanded_us <= tiles_us;
+}
+
 extern "C" size_t lp_latent_expanded_workspace_bytes(int R, int heads, int dim, int rot_dim, int kv_rank, int n_keys) {
   return lx_round((size_t)6 * R * heads * (dim + rot_dim)) + lx_round((size_t)6 * n_keys * (kv_rank + rot_dim)) +
          lx_round((size_t)6 * n_keys * lx_group(heads, n_keys) * 256);
@@ -1185,6 +1237,11 @@ extern "C" int lp_latent_attend_expanded(const lp_latent_desc* d, int R, int n_s
 
 // ---- window attention of prompts
 static int window_row(const lp_window_attn_desc* d) { return d->kv_heads * 128 * (d->v_is_k ? 1 : 2); }
+extern "C" int lp_window_prompt_count(const lp_window_attn_desc* d, const int* seq_row0, const int* seq_pos0, int n_seqs, int* n_tiles, int* n_keys) {
+  LP_REQUIRE(d != nullptr && seq_row0 != nullptr && seq_pos0 != nullptr && n_tiles != nullptr && n_keys != nullptr, "lp_window_prompt_count: null operand");
+  count32({n_seqs, d->window, seq_row0, seq_pos0, d->chunk, d->keep_first, d->pool}, n_tiles, n_keys);
+  return 0;
+}
 extern "C" size_t lp_window_prompt_workspace_bytes(int R, int heads, int row_floats, int n_keys) {
   return lx_round((size_t)6 * R * heads * 128) + lx_round((size_t)6 * n_keys * row_floats) + lx_round((size_t)8 * R * 64);
 }

@@ -46,14 +46,6 @@ STREAM_MAX_OUTPUTS = 170_000
 # to a million weights are too short for the device's time to count (us between steps, lp_linear and this one: width 512, 70 rows 578, 619, 600 rows of 20 requests 682,
 # 739, 1500 511, 530; width 1024, whose larger products gain, 70 rows 854, 734), have them from 2^31 multiplications on.
 SPLIT_MIN_ROWS, SPLIT_MIN_K, SPLIT_MIN_WEIGHTS, SPLIT_WORK = 65, 1024, 1 << 21, 1 << 31
-# Rows of prompts expand the visible latents into every head's keys and values (lp_latent_attend_expanded) or attend over the latents themselves
-# (lp_latent_attend_tiles), whichever `latent_route` expects to be done first: the first pays 1.4 (rank 128) to 2 ns (512) for every visible key and
-# head, however few rows see it, the second about 80 GFMA/s a CTA of 64 (row, head) pairs over keys of 2 rank + 64.  Its figures are fitted to 366 steps of 4 to
-# 32 heads over latents of 128 to 512 (1 to 128 requests of 1 to 4096 rows behind 0 to 64,000 tokens, windows of 100 to 2048 keys and none, both precisions), of
-# which it picks the slower way 7 times, by 7 to 23 %.  Some of them (us, tiles and expanded), 16 heads of rank 512: one request of 17 rows 123, 99, behind 4000 tokens
-# 3,377, 382; a prompt of 20 rows beside 7 running requests of 2000 tokens 1,731, 562, beside 31 of 2000 1,744, 2,768, of 8000 6,670, 14,829; of 2000 rows beside 31
-# of 2000 4,526, 2,891; 64 requests of 4 rows behind 4000 tokens 3,422, 11,767, of 48 rows 20,478, 11,934.
-EXPAND_GROUP_BYTES = 512 << 20      # heads whose keys and values are held at a time (csrc/lp_split32.cu): each group of heads walks a request's keys anew
 # What the planes of keys may take that lp_latent_attend_expanded and lp_window_attn_prompt read: the kernels that read the cache itself need none, so they have
 # the rows where it would be more or the allocation fails.  32 requests of 8 key / value heads over 8000 tokens: 3 GB, 7.1 ms with the cache's rows and 4.5 so.
 SCRATCH_BYTES = 1 << 30
@@ -65,7 +57,9 @@ SCRATCH_BYTES = 1 << 30
 # bf16: 2000, 8 (16 M) 484, 504, on a box of slower host 794, 841; 500, 16 (16 M) 450, 460; 550, 16 (18 M) 505, 464; 260, 24 (19 M) 450, 466; 330, 24 (24 M) 504, 466; 3000, 8 (24 M)
 # 679, 537; 8000, 4 (16 M) 643, 666; 12000, 4 (24 M) 867, 777; one windowed layer, 800, 16 (26 M) 326, 331, 1000, 16 (33 M) 600, 573, 6000, 8 (49 M) 613, 522.  Fp32 rows,
 # whose products take longer: 130, 24 (10 M) 674, 683; 200, 24 (15 M) 713, 692; 300, 16 (10 M) 587, 550; 999, 8 (8 M) 931, 847, one windowed layer 597, 601.
-WINDOW_TILE_ROWS, WINDOW_WORK, WINDOW_WORK_F32 = 64, 25_000_000, 10_000_000
+# Tiles of 128 rows: filled ones, or where the keys are many beside the rows half filled ones.  5 requests of 200 rows, 16 heads of width 2048 in bf16 754, 811; 32 of 70
+# rows 114, 121 a layer, behind 2000 tokens each 1,384, 636; a prompt of 2048 beside 15 running requests of 500 tokens 640, 231.
+WINDOW_FULL_ROWS, WINDOW_TILE_ROWS, WINDOW_PAST, WINDOW_WORK, WINDOW_WORK_F32 = 112, 64, 4, 25_000_000, 10_000_000
 # Up to MOE_PAIRS_MAX (token, choice) pairs an expert's weights are streamed once for the pairs that chose it.  Both products of 16 experts,
 # width 2048, 1024 inside (us, bf16; fp32 rows), against sorted tiles: 128 pairs 66, 108; 85, 182.  256 pairs 93, 108; 138, 182.  512 pairs 161,
 # 108; 282, 182: with this few experts the sorted tiles are ahead from about 300 pairs, with 32 (width 4096) not yet at 512: 554, 683; 876, 1116.
@@ -355,30 +349,6 @@ WKV_MIXES = ("r", "k", "v", "g", "w")      # the order of a WKV mixer's operands
 def expands(m: LatentAttentionConfig) -> bool:
     """whether lp_latent_attend_expanded has kernels for these heads"""
     return m.dim == 128 and m.vdim == 128 and m.rot_dim == 64 and m.kv_rank % 8 == 0
-
-
-def latent_route(starts, lens, heads: int, rank: int, window: Optional[int], sms: int) -> Tuple[float, float, int, int]:
-    """(microseconds of lp_latent_attend_tiles with its two head products, of lp_latent_attend_expanded, tiles of 128 rows, visible keys) of one step"""
-    keys = tiles = ctas = 0
-    tile_keys = cta_keys = 0.0             # summed over tiles of 128 rows, and over CTAs of 64 (row, head) pairs of a chunk of 32
-    longest = longest_tile = 0
-    for p, n in zip(starts, lens):
-        def seen(block):                   # by the last and by the average `block` rows of this request
-            few = min(n, block)
-            last, mean = p + n, p + (n + few) / 2
-            return (min(last, window + few - 1), min(mean, window + few - 1)) if window else (last, mean)
-        last, mean = seen(128)
-        t = -(-n // 128)
-        tiles, tile_keys, longest_tile = tiles + t, tile_keys + t * mean, max(longest_tile, last)
-        last, mean = seen(_lib.RETENTION_CHUNK)
-        full, rest = divmod(n, _lib.RETENTION_CHUNK)
-        c = full * -(-_lib.RETENTION_CHUNK * heads // 64) + -(-rest * heads // 64)
-        ctas, cta_keys, longest = ctas + c, cta_keys + c * mean, max(longest, last)
-        keys += p + n - (max(0, p - window + 1) if window else 0)
-    groups = -(-heads // max(1, min(heads, EXPAND_GROUP_BYTES // (keys * 1536))))
-    by_tiles = 90 + 64 * (2 * rank + 64) * 1.21e-5 * max(longest, cta_keys / ctas * -(-ctas // sms)) + sum(lens) * heads * rank * 2.2e-5
-    expanded = 60 + keys * heads * max(0.0008, 0.0022 - 0.1 / rank) + max(groups * (17 + 0.055 * longest_tile), (17 * tiles + 0.055 * tile_keys) * heads / sms)
-    return by_tiles, expanded, tiles, keys
 
 
 def _pad_rows(t: torch.Tensor, n: int) -> torch.Tensor:
@@ -756,8 +726,8 @@ class _Batch:
         self.decode = all(ln == 1 for ln in lens)
         self.longest_chunk = min(max(lens), _lib.RETENTION_CHUNK)
         pos0 = np.fromiter([s.length for s in seqs], np.int32, n)
-        self.starts = pos0.tolist()
-        self.latent_routes: Dict[tuple, tuple] = {}      # of this step's latent layers, by their sizes
+        self.host_pos0 = pos0
+        self.counts: Dict[tuple, tuple] = {}      # tiles, visible keys (and, of latents, the way) of this step's rows, by what a layer sees
         slot = np.fromiter([s.slot for s in seqs], np.int32, n)
         if self.decode:      # one row a request: every per-row table is a per-request one
             row0 = np.arange(n + 1, dtype=np.int32)
@@ -769,6 +739,7 @@ class _Batch:
             row_seq = np.repeat(np.arange(n, dtype=np.int32), lens)
             row_pos = np.concatenate([np.arange(p, p + ln, dtype=np.int32) for p, ln in zip(pos0, lens)])
             tokens = np.concatenate([np.asarray(e.tokens, np.int64) for e in entries])
+        self.host_row0 = row0
         if tokens.min() < 0 or tokens.max() >= eng.cfg.vocab:
             raise ValueError("token id outside the vocabulary")
 
@@ -935,7 +906,6 @@ class SeqLMEngine:
         self.tile_rows = int(self.L.lp_linear_tile_rows())
         # large bf16 products of the serving precision go to the tcgen05 GEMM when the library has it (the native ones do)
         self.tensor_core_rows = TENSOR_CORE_MIN_ROWS if dtype == "bfloat16" and hasattr(self.L, "lp_gemm_bf16") else None
-        self.sms = torch.cuda.get_device_properties(self.device).multi_processor_count if self.device.type == "cuda" else 1
         self.split_rows = SPLIT_MIN_ROWS if hasattr(self.L, "lp_linear_split") and self.device.type == "cuda" else None
         self.tap: Optional[Callable[[int, torch.Tensor], None]] = None   # called with (layer, residual stream) after every layer
         # decode steps are launch-bound: a batch layout (requests, page-table width) that comes back is captured into a CUDA graph on
@@ -1200,11 +1170,13 @@ class SeqLMEngine:
 
     def _room_to_expand(self, m: LatentAttentionConfig, b: _Batch) -> Optional[Tuple[int, int, torch.Tensor]]:
         """tiles, visible keys and scratch of lp_latent_attend_expanded; None where it is not the faster way for this step or its scratch is too large"""
-        sizes = (m.heads, m.kv_rank, m.window)
-        if sizes not in b.latent_routes:
-            b.latent_routes[sizes] = latent_route(b.starts, b.lens, *sizes, self.sms)
-        by_tiles, expanded, tiles, keys = b.latent_routes[sizes]
-        if by_tiles < expanded:
+        seen = (m.heads, m.kv_rank, m.window)
+        if seen not in b.counts:
+            tiles, keys = C.c_int(), C.c_int()
+            pays = self.L.lp_latent_route(b.host_row0.ctypes.data, b.host_pos0.ctypes.data, b.n, m.heads, m.kv_rank, m.window or 0, C.byref(tiles), C.byref(keys))
+            b.counts[seen] = (pays, tiles.value, keys.value)
+        pays, tiles, keys = b.counts[seen]
+        if not pays:
             return None
         nbytes = int(self.L.lp_latent_expanded_workspace_bytes(b.R, m.heads, m.dim, m.rot_dim, m.kv_rank, keys))
         # the other way holds a query and a sum of latents for every row and head
@@ -1300,17 +1272,16 @@ class SeqLMEngine:
         if (not hasattr(self.L, "lp_window_attn_prompt") or m.dim != 128 or m.vdim != 128 or m.distance_bias or m.distance_slope
                 or qkv.stride(0) % 4 or qkv.data_ptr() % 16 or o.data_ptr() % 16 or o.stride(0) % (4 if o.dtype == F32 else 8)):
             return False
-        tiles = sum(-(-ln // 128) for ln in b.lens)
-        if b.R < WINDOW_TILE_ROWS * tiles or b.R * m.heads * self.cfg.width < (WINDOW_WORK if self.act == BF16 else WINDOW_WORK_F32):
+        if b.R * m.heads * self.cfg.width < (WINDOW_WORK if self.act == BF16 else WINDOW_WORK_F32):
             return False
-
-        def first(pos):      # the first token of its window, or of its own block of positions
-            lo = max(0, pos - d.window + 1) if d.window > 0 else 0
-            return max(lo, pos // d.chunk * d.chunk) if d.chunk else lo
-        keys = 0
-        for p, ln in zip(b.starts, b.lens):
-            past = p + ln - d.window if d.window > 0 else 0      # positions wholly before the last row's window
-            keys += min(d.keep_first, first(p + ln - 1)) + (past // d.pool if d.pool and past > 0 else 0) + p + ln - first(p)
+        seen = (d.window, d.keep_first, d.pool, d.chunk)
+        if seen not in b.counts:
+            tiles, keys = C.c_int(), C.c_int()
+            self._check(self.L.lp_window_prompt_count(C.byref(d), b.host_row0.ctypes.data, b.host_pos0.ctypes.data, b.n, C.byref(tiles), C.byref(keys)), "lp_window_prompt_count")
+            b.counts[seen] = (tiles.value, keys.value)
+        tiles, keys = b.counts[seen]
+        if b.R < (WINDOW_TILE_ROWS if keys >= WINDOW_PAST * b.R else WINDOW_FULL_ROWS) * tiles:
+            return False
         row = m.kv_heads * 128 * (1 if m.values_are_keys else 2)
         nbytes = int(self.L.lp_window_prompt_workspace_bytes(b.R, m.heads, row, keys))
         ws = self._scratch(nbytes) if 6 * (keys - b.R) * row <= SCRATCH_BYTES else None      # planes of this step's own rows are of its projection's size

@@ -367,12 +367,24 @@ def test_a_latent_that_is_not_finite_stays_with_the_rows_that_see_it(bad):
     ([(4000, 4)] * 64, 16, 512, None, False), ([(4000, 48)] * 64, 16, 512, None, True), ([(0, 12)] * 128, 8, 256, None, False), ([(0, 24)] * 64, 8, 256, 512, True),
     ([(8000, 1)] * 31 + [(0, 20)], 4, 128, 256, True), ([(8000, 1)] * 31 + [(0, 20)], 16, 512, 100, False), ([(8000, 1)] * 31 + [(0, 20)], 32, 512, 2048, False),
     ([(8000, 1)] * 7 + [(0, 300)], 32, 512, 2048, True), ([(0, 24)] * 64, 16, 128, None, False)])
-def test_which_steps_expand_their_latents(reqs, heads, rank, window, expands):
+def test_which_steps_expand_their_latents(native_lib, reqs, heads, rank, window, expands):
     """by the work of either way, measured on both sides: running requests with a long past beside a short prompt do not, portions behind a long past do"""
-    from leopard_b200.seqlm import latent_route
-    by_tiles, expanded, tiles, keys = latent_route([p for p, _ in reqs], [n for _, n in reqs], heads, rank, window, 148)
-    assert (expanded <= by_tiles) == expands
-    assert tiles == sum(-(-n // 128) for _, n in reqs) and keys == sum(p + n - seen(p, window or 0)[2] for p, n in reqs)
+    row0, pos0 = torch.tensor([0] + [n for _, n in reqs]).cumsum(0).int(), torch.tensor([p for p, _ in reqs], dtype=torch.int32)
+    tiles, keys = C.c_int(), C.c_int()
+    assert native_lib.lp_latent_route(row0.data_ptr(), pos0.data_ptr(), len(reqs), heads, rank, window or 0, C.byref(tiles), C.byref(keys)) == expands
+    assert tiles.value == sum(-(-n // 128) for _, n in reqs) and keys.value == sum(p + n - seen(p, window or 0)[2] for p, n in reqs)
+
+
+@pytest.mark.parametrize("rule", [(0,), (40, 0, 3), (48, 0, 0, 8), (0, 48), (33, 0, 7, 5), (30, 64)])
+def test_key_rows_of_a_step(native_lib, rule):
+    """window, own block, kept tokens, pooled blocks: what the host counts is what the kernels walk"""
+    from leopard_b200._lib import WindowAttnDesc
+    reqs = [(0, 1), (0, 200), (47, 1), (48, 100), (500, 3), (129, 300)]
+    row0, pos0 = torch.tensor([0] + [n for _, n in reqs]).cumsum(0).int(), torch.tensor([p for p, _ in reqs], dtype=torch.int32)
+    window, chunk, keep, pool = (*rule, 0, 0, 0)[:4]
+    d, tiles, keys = WindowAttnDesc(window=window, chunk=chunk, keep_first=keep, pool=pool), C.c_int(), C.c_int()
+    assert native_lib.lp_window_prompt_count(C.byref(d), row0.data_ptr(), pos0.data_ptr(), len(reqs), C.byref(tiles), C.byref(keys)) == 0
+    assert tiles.value == sum(-(-n // 128) for _, n in reqs) and keys.value == sum(len(run_keys(p, n, *rule)) for p, n in reqs)
 
 
 @pytest.mark.gpu
@@ -384,7 +396,7 @@ def test_latents_are_attended_as_they_are_where_expanding_does_not_pay_or_fit(wh
     h = torch.randn((40, 256), device="cuda")
     want = eng._latent(0, m, eng.w.layers[0], h, batch).double()
     if why == "work":
-        batch.latent_routes[(2, 64, None)] = (1.0, 2.0, 1, 40)
+        batch.counts[(2, 64, None)] = (0, 1, 40)
     elif why == "limit":
         monkeypatch.setattr(seqlm, "SCRATCH_BYTES", 0)
     else:
@@ -417,12 +429,12 @@ def test_queries_off_16_byte_boundaries_are_attended_too():
 def test_expanded_heads_in_groups():
     """more keys than all heads' expanded keys and values are held for at a time: the heads run in groups, the last one smaller; every 500th row against float64.
     Scores, their exponentials and 148 tiles of keys are each a few roundings of 2^-24, and the output's product sums 2,432 of them: 1e-6"""
-    from leopard_b200.seqlm import EXPAND_GROUP_BYTES, StepEntry, _Batch
+    from leopard_b200.seqlm import StepEntry, _Batch
     H, rank, n = 19, 64, 19000
     eng, m = latent_engine("float32", H, rank, None, max_tokens=20480)
     lw, calls, inner = eng.w.layers[0], [], eng._latent_expanded
     eng._latent_expanded = lambda *a: calls.append(1) or inner(*a)
-    assert n * 1536 * H > EXPAND_GROUP_BYTES
+    assert n * 1536 * H > 512 << 20
     w_kv, w_o = lw["w_kv"].double(), lw["w_o"].double()
     for ln in (n, 40):      # a prompt, then a portion over all of it
         batch = _Batch(eng, [StepEntry("a", [1] * ln, [])])

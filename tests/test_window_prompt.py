@@ -20,7 +20,7 @@ BOUND = 2.5e-7
 def every_size(request, monkeypatch):
     """the tensor-core kernel has rows of any number here, but where the rule is what is tested"""
     if "rule" not in request.node.name:
-        for name in ("WINDOW_TILE_ROWS", "WINDOW_WORK", "WINDOW_WORK_F32"):
+        for name in ("WINDOW_FULL_ROWS", "WINDOW_TILE_ROWS", "WINDOW_WORK", "WINDOW_WORK_F32"):
             monkeypatch.setattr(seqlm, name, 0)
 
 
@@ -156,12 +156,18 @@ def test_errors_are_no_larger_than_those_of_the_tiles(heads, kv_heads, options, 
 
 
 @pytest.mark.parametrize("dtype,width,heads,lens,taken", [
-    ("float32", 1000, 16, (625,), True), ("float32", 1000, 16, (624,), False), ("bfloat16", 2000, 16, (782,), True), ("bfloat16", 2000, 16, (781,), False),
-    ("float32", 4000, 64, (64, 64), True), ("float32", 4000, 64, (64, 63), False), ("float32", 4000, 63, (129,), True), ("float32", 4000, 63, (65, 65, 60), False)])
+    ("float32", 1000, 16, (625,), True), ("float32", 1000, 16, (624,), False), ("bfloat16", 1744, 16, (896,), True), ("bfloat16", 1736, 16, (896,), False),
+    ("float32", 4000, 64, (112, 112), True), ("float32", 4000, 64, (112, 111), False), ("float32", 4000, 63, (224,), True), ("float32", 4000, 63, (129,), False),
+    ("float32", 4000, 64, (64, 64), False), ("float32", 4000, 64, ((200, 64), (184, 64)), True), ("float32", 4000, 64, ((200, 64), (183, 64)), False),
+    ("float32", 4000, 64, ((200, 64), (400, 63)), False)])
 def test_both_sides_of_the_rule(dtype, width, heads, lens, taken):
-    """rows x heads x width of 10 million in fp32, 25 million in bf16, and 64 rows a tile of 128"""
-    eng, m = engine(heads, 1, dtype, width=width, window=50)
-    batch = _Batch(eng, [StepEntry(i, [1] * n, []) for i, n in enumerate(lens)])
+    """rows x heads x width of 10 million in fp32, 25 million in bf16; 112 rows a tile of 128, or 64 where the keys are four times the rows (here: (past, rows))"""
+    eng, m = engine(heads, 1, dtype, width=width)
+    for i, n in enumerate(lens):
+        if isinstance(n, tuple):
+            eng.cache.reserve(eng.cache.open(i), n[0])
+            eng.cache.advance(eng.cache.get(i), n[0])
+    batch = _Batch(eng, [StepEntry(i, [1] * (n[1] if isinstance(n, tuple) else n), []) for i, n in enumerate(lens)])
     calls, L = [], eng.L
 
     class Spy:
