@@ -705,6 +705,9 @@ int lp_latent_attend_tiles(const lp_latent_desc* desc, int R, const int* row_seq
 /* fp32 numbers as three planes of bf16 terms that add up to them (each takes 8 bits of what the ones before left), `plane`
  * elements apart: rows [M, K] of `src` -> [M, K] of each plane, rows ldp elements apart.  K a multiple of 8, rows on 16-byte boundaries. */
 int lp_split_rows(const float* src, long long ld, int M, int K, void* planes, long long ldp, long long plane, void* stream);
+/* rows row_of[0 .. rows) of src, K columns each (row_of on the device; a negative index: zeros) -> dst [rows, K]: bf16 as they are, fp32 as three planes `plane`
+ * elements apart.  K a multiple of 8, rows on 16-byte boundaries. */
+int lp_gather_rows(const void* src, long long ld, int src_fp32, const int* row_of, int rows, int K, void* dst, long long plane, void* stream);
 /* C[M, N] = A[M, K] W[N, K]^T (+ bias fp32 [N]) on the tcgen05 tensor cores with A in three planes and W bf16: an fp32 product, sums in fp32.
  * out: 0 bf16, 1 fp32, 2 three planes c_plane elements apart.  K and N multiples of 8, rows on 16-byte boundaries. */
 int lp_gemm_split(const void* A, long long lda, long long a_plane, const void* W, long long ldw, void* C, long long ldc, long long c_plane,

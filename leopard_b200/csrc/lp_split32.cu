@@ -148,6 +148,30 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
   s32_store_terms(dst + r * ldd + c, plane, v);
 }
 
+// rows of src by an index (a negative one: zeros), eight columns a thread: bf16 as they are, or fp32 -> planes
+template <bool SPLIT>
+__global__ void __launch_bounds__(256) gather_rows_kernel(const void* __restrict__ src, long long ld, const int* __restrict__ row_of, int rows, int K,
+                                                          bf16* __restrict__ dst, long long plane) {
+  const int per = K >> 3;
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i >= (long long)rows * per) return;
+  const long long r = i / per;
+  const int c = (int)(i - r * per) * 8, from = row_of[r];
+  bf16* to = dst + r * K + c;
+  if (SPLIT) {
+    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (from >= 0) {
+      const float* s = reinterpret_cast<const float*>(src) + from * ld + c;
+      const float4 a = *reinterpret_cast<const float4*>(s), b = *reinterpret_cast<const float4*>(s + 4);
+      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+      v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    }
+    s32_store_terms(to, plane, v);
+  } else {
+    *reinterpret_cast<uint4*>(to) = from >= 0 ? *reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(src) + from * ld + c) : make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+
 // ---------------------------------------------------------------------------------------------------------------------------------
 // C[M, N] = A W^T (+ bias).  Persistent CTAs (one an SM) walk 128 x BN tiles; a k block of 64 is W's box(es) and A's three boxes, each with a
 // barrier pair of its own so that a term's box is refilled as soon as its product has run.  Every k block is a chain of its own in one of two
@@ -1012,6 +1036,19 @@ static int split_rows(const float* src, long long ld, int M, int K, void* planes
 }
 extern "C" int lp_split_rows(const float* src, long long ld, int M, int K, void* planes, long long ldp, long long plane, void* stream) {
   return split_rows(src, ld, M, K, planes, ldp, plane, nullptr, stream);
+}
+
+extern "C" int lp_gather_rows(const void* src, long long ld, int src_fp32, const int* row_of, int rows, int K, void* dst, long long plane, void* stream_) {
+  LP_REQUIRE(src != nullptr && row_of != nullptr && dst != nullptr, "lp_gather_rows: null operand");
+  LP_REQUIRE(K % 8 == 0 && ld % (src_fp32 ? 4 : 8) == 0 && plane % 8 == 0 && aligned16(src) && aligned16(dst), "lp_gather_rows: 16-byte rows of whole eights");
+  if (rows <= 0 || K <= 0) return 0;
+  const unsigned grid = (unsigned)(((long long)rows * (K >> 3) + 255) / 256);
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  if (src_fp32) gather_rows_kernel<true><<<grid, 256, 0, stream>>>(src, ld, row_of, rows, K, reinterpret_cast<bf16*>(dst), plane);
+  else gather_rows_kernel<false><<<grid, 256, 0, stream>>>(src, ld, row_of, rows, K, reinterpret_cast<bf16*>(dst), plane);
+  note_launch();
+  LP_CHECK_CUDA(cudaGetLastError());
+  return 0;
 }
 
 template <int BN, int PLANES, bool GATED>

@@ -1492,7 +1492,8 @@ class SeqLMEngine:
         # fp32 295, 145 and 701, 307; the nearest fp32 rows: 8 experts of 80 pairs 130, 139, width 512 99, 108
         on_tensor_cores = self.tensor_core_rows if h.dtype == BF16 else self.split_rows
         grouped = (on_tensor_cores is not None and n_pairs >= f.experts * TENSOR_CORE_MIN_ROWS and epi == _lib.EPI_SILU_GATE
-                   and hasattr(L, "lp_gemm_grouped") and D % 16 == 0 and f.expert_ff % 8 == 0 and all(t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (w_gu, w_dn)))
+                   and hasattr(L, "lp_gemm_grouped") and D % 16 == 0 and f.expert_ff % 8 == 0 and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0
+                   and all(t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (w_gu, w_dn)))
         tile_rows = GROUP_TILE_ROWS if grouped else self.tile_rows
         tiles = int(L.lp_moe_max_tiles(n_pairs, f.experts, tile_rows))
         tile_group = self._empty((tiles,), I32)
@@ -1510,11 +1511,11 @@ class SeqLMEngine:
         if not grouped or h.dtype == BF16:
             h1 = self._empty((rows, f.expert_ff), self.act)
         if grouped:
-            a, plane, plane1, form = h.index_select(0, sorted_token.clamp_min(0)), 0, 0, _lib.GEMM_SPLIT_BF16
+            plane, plane1, form = 0, 0, _lib.GEMM_SPLIT_BF16
             if h.dtype == F32:      # three bf16 terms each, the inner rows as the first product's store makes them
-                terms, plane, plane1, form = self._empty((3, rows, D), BF16), rows * D, rows * f.expert_ff, _lib.GEMM_SPLIT_PLANES
-                self._check(L.lp_split_rows(_lib.ptr(a), a.stride(0), rows, D, _lib.ptr(terms), D, plane, st), "lp_split_rows")
-                a, h1 = terms, self._empty((3, rows, f.expert_ff), BF16)
+                plane, plane1, form, h1 = rows * D, rows * f.expert_ff, _lib.GEMM_SPLIT_PLANES, self._empty((3, rows, f.expert_ff), BF16)
+            a = self._empty((3 if plane else 1, rows, D), BF16)
+            self._check(L.lp_gather_rows(_lib.ptr(h), h.stride(0), int(h.dtype == F32), _lib.ptr(sorted_token), rows, D, _lib.ptr(a), plane, st), "lp_gather_rows")
             rc = L.lp_gemm_grouped(_lib.ptr(a), D, plane, _lib.ptr(w_gu), w_gu.stride(1), w_gu.stride(0), f.experts, _lib.ptr(tile_group), tiles, 1,
                                    _lib.ptr(scale), _lib.ptr(h1), f.expert_ff, plane1, form, 2 * f.expert_ff, D, st)
             self._check(rc, "lp_gemm_grouped")

@@ -36,6 +36,13 @@ extern "C" void emu_split_rows(const float* src, long long ld, int M, int K, voi
   emu::launch(dim3((unsigned)(((long long)M * (K / 8) + 255) / 256)), dim3(256), [&] { split_rows_kernel<false>(src, ld, M, K, (bf16*)dst, ldd, plane, Factor32{}); });
 }
 
+extern "C" void emu_gather_rows(const void* src, long long ld, int src_fp32, const int* row_of, int rows, int K, void* dst, long long plane) {
+  emu::launch(dim3((unsigned)(((long long)rows * (K / 8) + 255) / 256)), dim3(256), [&] {
+    if (src_fp32) gather_rows_kernel<true>(src, ld, row_of, rows, K, (bf16*)dst, plane);
+    else gather_rows_kernel<false>(src, ld, row_of, rows, K, (bf16*)dst, plane);
+  });
+}
+
 extern "C" void emu_gather_keys(int n_seqs, int window, int keep_first, int pool, const int* row0, const int* pos0, int n_keys, const float* cache,
                                 int page_size, const int* table, int max_pages, const float* blocks, const int* block_table, int width, void* dst, long long plane) {
   Seqs32 q = {n_seqs, window, row0, pos0, 0, keep_first, pool};

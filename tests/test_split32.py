@@ -292,6 +292,18 @@ def test_gather_of_cache_rows(emu):
     assert torch.equal(got.double().sum(0), want.double())
 
 
+@pytest.mark.parametrize("rows,K,dtype", [(1, 8, F32), (37, 72, F32), (130, 16, BF), (9, 264, BF)])
+def test_gather_of_rows(emu, rows, K, dtype):
+    """by an index, rows that stand apart, a negative index zeros"""
+    g = torch.Generator().manual_seed(rows)
+    src = torch.randn((11, K + 8), generator=g).to(dtype)
+    index = torch.randint(-1, 11, (rows,), generator=g).int()
+    got = torch.full((3 if dtype == F32 else 1, rows, K), float("nan"), dtype=BF)
+    emu.emu_gather_rows(P(src), LL(K + 8), int(dtype == F32), P(index), rows, K, P(got), LL(rows * K))
+    want = torch.where(index[:, None] < 0, torch.zeros((), dtype=F64), src[index.clamp_min(0).long()][:, :K].double())
+    assert torch.equal(got.double().sum(0), want)
+
+
 # ------------------------------------------------------------------------------------------------------------------- on a GPU, through the engine
 def latent_engine(dtype, heads, rank, window, max_tokens=2048, **options):
     from leopard_b200 import _lib
