@@ -305,21 +305,22 @@ window_attn_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const int*
   extern __shared__ float dyn_smem[];
   const int r = blockIdx.x;
   if (r >= R) return;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, W = blockDim.x >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, all = blockDim.x >> 5;
   const int ratio = a.heads / a.kv_heads, per_g = ratio / QH;
   const int g = blockIdx.y / per_g, h0 = g * ratio + (blockIdx.y % per_g) * QH;
   const float** row_s = reinterpret_cast<const float**>(dyn_smem);      // [W][32] cache row of each key of a warp's current tile
-  float* q_s = dyn_smem + 2 * W * 32;       // [QH][dim]
+  float* q_s = dyn_smem + 2 * all * 32;       // [QH][dim]
   float* p_s = q_s + QH * a.dim;            // [W][QH][32] softmax weights of a warp's current tile
-  float* m_s = p_s + W * QH * 32;           // [W][QH]
-  float* d_s = m_s + W * QH;                // [W][QH]
-  float* o_s = d_s + W * QH;                // [W][QH][vdim]
-  float* f_s = o_s + W * QH * a.vdim;       // [QH][vdim] merged output before it is turned back
+  float* m_s = p_s + all * QH * 32;           // [W][QH]
+  float* d_s = m_s + all * QH;                // [W][QH]
+  float* o_s = d_s + all * QH;                // [W][QH][vdim]
+  float* f_s = o_s + all * QH * a.vdim;       // [QH][vdim] merged output before it is turned back
   const int seq = row_seq[r], pos = row_pos[r];
   const float* q = a.qkv + (long long)r * a.ld + a.q_off + (long long)h0 * a.dim;
   for (int i = tid; i < QH * a.dim; i += blockDim.x) q_s[i] = q[i];
   __syncthreads();
   const WinVisible vis = win_visible(a, pos);
+  const int W = min((int)blockDim.x >> 5, (vis.count + 31) >> 5);      // warps that have keys
   const int v_off = a.v_base + g * a.vdim;
   const bool vec = (a.dim % 4 == 0) && (a.vdim % 4 == 0);      // rows and head offsets are then 16-byte aligned
   const bool quads = vec && (a.dim % 16 == 0);
@@ -348,7 +349,9 @@ window_attn_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const int*
       const int piece = lane & 3, kq = lane >> 2;
       if (valid) my_row[lane] = win_visible_row(a, vis, seq, t);      // looked up once a key, a lane each
       __syncwarp();
-#pragma unroll 1
+      // loads in flight (one head a CTA of 8 warps: two passes of four; with one of eight the compiler has them wait for each other, 64 rows of 4 heads over 1500 keys
+      // 360 us instead of 146)
+#pragma unroll (QH == 1 && THREADS == 256 ? 2 : 1)
       for (int i = 0; i < 4; ++i) {
         const int tk = t0 + i * 8 + kq;
         float part[QH];
@@ -358,7 +361,7 @@ window_attn_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const int*
           const float* row = my_row[i * 8 + kq];
           const float* kp = row + g * a.dim + 4 * piece;
           const float* qp = q_s + 4 * piece;
-#pragma unroll 8
+#pragma unroll (QH == 1 && THREADS == 256 ? 4 : 8)
           for (int d = 0; d < a.dim; d += 16) {
             const float4 k4 = *reinterpret_cast<const float4*>(kp + d);
 #pragma unroll
@@ -450,7 +453,7 @@ window_attn_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const int*
     __syncwarp();
   }
 #pragma unroll
-  for (int h = 0; h < QH; ++h) {
+  for (int h = 0; h < QH && warp < W; ++h) {
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int c = lane + 32 * i;
@@ -1497,8 +1500,11 @@ static int launch_window_attn(const WinArgs& a, int R, const int* row_seq, const
                               cudaStream_t stream) {
   int warps = R <= WIN_SPLIT_ROWS ? 8 : 4;
   const dim3 grid(R, a.kv_heads * (a.heads / a.kv_heads / QH));
-  // where a head has a CTA and CTAs leave SMs idle, a CTA's chain over its keys is the time: 32 warps walk it.  One row of 32 heads over 516 keys: 22 us with 8.
-  const bool wide = QH == 1 && grid.x * grid.y <= (unsigned)sm_count() && win_smem_floats(1, 32, a.dim, a.vdim) * sizeof(float) <= 48 * 1024;
+  // where a head has a CTA and CTAs leave SMs idle, a CTA's chain over its keys is the time: 32 warps walk it, if there may be more keys than eight warps
+  // take at once.  One row of 32 heads, us with 8 and 32 warps: 200 keys 10.0, 11.2; 300 16.3, 11.5; 600 23.1, 13.4; 1500 43.3, 24.9.  (Merging the 21 to 31 warps
+  // without keys as well, 200 keys took 12.9.)
+  const long long may_see = (a.window > 0 ? (long long)a.window + a.keep_first : (long long)a.max_pages * a.page_size) + (a.pool > 0 ? (long long)a.max_pooled_pages * a.page_size : 0);
+  const bool wide = QH == 1 && may_see > 256 && grid.x * grid.y <= (unsigned)sm_count() && win_smem_floats(1, 32, a.dim, a.vdim) * sizeof(float) <= 48 * 1024;
   if (wide) warps = 32;
   while (warps > 1 && win_smem_floats(QH, warps, a.dim, a.vdim) * sizeof(float) > 48 * 1024) warps >>= 1;
   const size_t smem = win_smem_floats(QH, warps, a.dim, a.vdim) * sizeof(float);

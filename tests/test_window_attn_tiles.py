@@ -188,3 +188,10 @@ def test_one_row_steps_with_and_without_shared_rows(backend, heads, kv_heads, ro
     a CTA, the others share"""
     _, row_wise = _run(backend, "kept", heads, kv_heads, [9] * rows, [1] * rows, rule=True)
     assert row_wise < 4e-6
+
+
+@pytest.mark.parametrize("heads,kv_heads,pos", [(4, 1, 255), (4, 1, 256), (2, 2, 700), (4, 1, 1100)])
+def test_one_row_over_many_keys(backend, heads, kv_heads, pos):
+    """a head a CTA: pages for 256 keys, which eight warps take at once, and for more, which up to 32 warps walk"""
+    _, row_wise = _run(backend, "all", heads, kv_heads, [pos], [1], rule=True)
+    assert row_wise < 4e-6
