@@ -307,18 +307,18 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
       }
     } else {
 #pragma unroll 8
-    for (int d = 0; d < a.dim; ++d) {
-      float q2[2], k2[2];
+      for (int d = 0; d < a.dim; ++d) {
+        float q2[2], k2[2];
 #pragma unroll
-      for (int p = 0; p < 2; ++p) {
-        q2[p] = qs[(i0 + p) * dimp + d];
-        k2[p] = ks[(tj + p * (RET_CHUNK / 2)) * dimp + d];
+        for (int p = 0; p < 2; ++p) {
+          q2[p] = qs[(i0 + p) * dimp + d];
+          k2[p] = ks[(tj + p * (RET_CHUNK / 2)) * dimp + d];
+        }
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) acc[p][q] = fmaf(q2[p], k2[q], acc[p][q]);
       }
-#pragma unroll
-      for (int p = 0; p < 2; ++p)
-#pragma unroll
-        for (int q = 0; q < 2; ++q) acc[p][q] = fmaf(q2[p], k2[q], acc[p][q]);
-    }
     }
 #pragma unroll
     for (int p = 0; p < 2; ++p)
@@ -358,19 +358,19 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
       }
     } else {
 #pragma unroll 8
-    for (int d = 0; d < a.dim; ++d) {
-      float q4[4], s4[4];
+      for (int d = 0; d < a.dim; ++d) {
+        float q4[4], s4[4];
 #pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        q4[p] = qs[(i0 + p) * dimp + d];
-        const int y = ty + p * tiles_y;
-        s4[p] = stage_s ? Ss[d * vdimp + y] : (y < a.vdim ? S[d * a.vdim + y] : 0.f);
+        for (int p = 0; p < 4; ++p) {
+          q4[p] = qs[(i0 + p) * dimp + d];
+          const int y = ty + p * tiles_y;
+          s4[p] = stage_s ? Ss[d * vdimp + y] : (y < a.vdim ? S[d * a.vdim + y] : 0.f);
+        }
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) acc[p][q] = fmaf(q4[p], s4[q], acc[p][q]);
       }
-#pragma unroll
-      for (int p = 0; p < 4; ++p)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[p][q] = fmaf(q4[p], s4[q], acc[p][q]);
-    }
     }
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
@@ -547,7 +547,7 @@ __device__ __forceinline__ float* lat_cache_row(const LatArgs& a, int seq, int p
 }
 
 // A CTA a row; the row's sines and cosines are taken once for all heads (four a pair and head before: one row of 16 heads 7.0 us).
-constexpr int LAT_PREP_THREADS = 128, LAT_PREP_WIDE = 512, LAT_PREP_ROWS = 296;      // few rows (decoding) take wide CTAs
+constexpr int LAT_PREP_THREADS = 128, LAT_PREP_WIDE = 512;      // up to two rows an SM (decoding) take wide CTAs
 constexpr int LAT_PREP_PAIRS = 4096;      // rotation pairs whose sines and cosines shared memory holds; with more of them each is taken where it is used
 __global__ void __launch_bounds__(LAT_PREP_WIDE)
 latent_prep_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos) {
@@ -747,6 +747,8 @@ latent_attend_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const in
 // Many rows (prompts): one CTA per row and group of LAT_ROW_HEADS heads, one warp per head, every warp walks all visible keys.
 // The heads of a row read the same cache rows at about the same time, so the cache traffic of a row is paid once per CTA (L1), and
 // neighbouring rows overlap in all but one key (L2).
+// Up to LAT_SPLIT_ROWS rows latent_attend_kernel splits a row's keys over warps (us, this kernel and that one): 17 rows of 8 heads over 40 keys 37, 10; 128 over 40 38, 21, over
+// 300 233, 80; 16 heads 39, 37 and 225, 164.  Beyond it that one is ahead as well (192 rows of 8 heads over 300 keys 238, 88; 512 over 40 44, 45): the line was not moved.
 constexpr int LAT_ROW_HEADS = 4, LAT_SPLIT_ROWS = 128;
 template <int NR>
 __global__ void __launch_bounds__(LAT_ROW_HEADS * 32)
@@ -1118,7 +1120,7 @@ extern "C" int lp_latent_prep(const lp_latent_desc* d, int R, const int* row_seq
   LP_REQUIRE((d->dkv == nullptr || d->c_gain != nullptr) && row_seq != nullptr && row_pos != nullptr, "lp_latent_prep: null operand");
   if (R <= 0) return 0;
   const size_t smem = d->rot_dims / 2 <= LAT_PREP_PAIRS ? d->rot_dims / 2 * sizeof(float2) : 0;
-  latent_prep_kernel<<<R, R <= LAT_PREP_ROWS ? LAT_PREP_WIDE : LAT_PREP_THREADS, smem, stream>>>(a, R, row_seq, row_pos);
+  latent_prep_kernel<<<R, R <= 2 * sm_count() ? LAT_PREP_WIDE : LAT_PREP_THREADS, smem, stream>>>(a, R, row_seq, row_pos);
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;

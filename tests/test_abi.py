@@ -53,6 +53,13 @@ def test_struct_layouts_match_header(tmp_path):
             assert int(got[f"{cname}.{fname}"]) == getattr(ct, fname).offset, f"{cname}.{fname}"
 
 
+def test_constants_match_header():
+    from leopard_b200 import _lib
+    txt = (ROOT / "include" / "leopard_b200.h").read_text()
+    for name in ("RETENTION_CHUNK", "LATENT_SPLIT_ROWS"):
+        assert getattr(_lib, name) == int(re.search(rf"#define LP_{name} (\d+)", txt)[1]), name
+
+
 def test_argument_errors_are_status_codes(native_lib):
     rc = native_lib.lp_gemm_bf16(None, 8, None, 8, None, 8, 0, 8, 8, None, None, 0, 0, 0, 0, 0, None)
     assert rc == -1 and b"empty problem" in native_lib.lp_last_error()
