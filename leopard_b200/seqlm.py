@@ -54,7 +54,7 @@ SCRATCH_BYTES = 1 << 30
 # device, lp_window_attn_tiles and this one; heads on a quarter of key / value heads): one request of 500 rows, 8 heads 89, 54, 16 heads 149, 64; of 4096, 8 heads 487,
 # 188, 16 heads 828, 299; behind 32,000 tokens 512 rows of 16 heads 10,682, 1,469; 32 requests of 70, 16 heads 114, 121.
 # Work is rows x heads x width, what the step's products grow with.  Whole prompts of two windowed layers and a recurrence (us between steps; rows, heads = width / 128),
-# bf16: 2000, 8 (16 M) 484, 504, on a box of slower host 794, 841; 500, 16 (16 M) 450, 460; 550, 16 (18 M) 505, 464; 260, 24 (19 M) 450, 466; 330, 24 (24 M) 504, 466; 3000, 8 (24 M)
+# bf16: 2000, 8 (16 M) 484, 504, with a slower host 794, 841; 500, 16 (16 M) 450, 460; 550, 16 (18 M) 505, 464; 260, 24 (19 M) 450, 466; 330, 24 (24 M) 504, 466; 3000, 8 (24 M)
 # 679, 537; 8000, 4 (16 M) 643, 666; 12000, 4 (24 M) 867, 777; one windowed layer, 800, 16 (26 M) 326, 331, 1000, 16 (33 M) 600, 573, 6000, 8 (49 M) 613, 522.  Fp32 rows,
 # whose products take longer: 130, 24 (10 M) 674, 683; 200, 24 (15 M) 713, 692; 300, 16 (10 M) 587, 550; 999, 8 (8 M) 931, 847, one windowed layer 597, 601.
 # Tiles of 128 rows: filled ones, or where the keys are many beside the rows half filled ones.  5 requests of 200 rows, 16 heads of width 2048 in bf16 754, 811; 32 of 70
@@ -1488,8 +1488,8 @@ class SeqLMEngine:
         w_gu, w_dn = lw["w_gu"], lw["w_edown"]
         # rows enough to fill tensor-core tiles: an expert's rows are gathered into tiles of its own and all experts' products are one launch, without a look at
         # the tables on the host.  The line is where a product an expert (bf16) ran on the tensor cores before.  Both products of 64 and of 256 pairs an expert (us,
-        # without and with; 8 experts, width and inside 1024): bf16 600, 97 and 534, 100, fp32 124, 110 and 213, 138; 16 experts, width 2048 859, 104 and 970, 173,
-        # fp32 295, 145 and 701, 307; the nearest fp32 rows: 8 experts of 80 pairs 130, 139, width 512 99, 108
+        # without and with; 8 experts, width and inside 1024): bf16 596, 82 and 510, 100, fp32 126, 93 and 214, 139; 16 experts, width 2048 787, 106 and 932, 184,
+        # fp32 294, 134 and 704, 305; 8 experts of width 512, fp32 98, 85 and 138, 105
         on_tensor_cores = self.tensor_core_rows if h.dtype == BF16 else self.split_rows
         grouped = (on_tensor_cores is not None and n_pairs >= f.experts * TENSOR_CORE_MIN_ROWS and epi == _lib.EPI_SILU_GATE
                    and hasattr(L, "lp_gemm_grouped") and D % 16 == 0 and f.expert_ff % 8 == 0 and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0
