@@ -94,7 +94,7 @@ class LinearDesc(C.Structure):
     _fields_ = [("A", _vp), ("lda", _ll), ("a_batch", _ll), ("a_fp32", _i), ("W", _vp), ("ldw", _ll), ("w_batch", _ll), ("C", _vp),
                 ("ldc", _ll), ("c_batch", _ll), ("c_fp32", _i), ("M", _i), ("N", _i), ("K", _i), ("batch", _i), ("epi", _i),
                 ("epi_a", _f), ("epi_b", _f), ("c_accum", _i), ("c_scale", _f), ("bias", _vp), ("row_scale", _vp), ("gate", _vp), ("ldg", _ll),
-                ("gate_batch", _ll), ("seg_cols", _i), ("n_segs", _i), ("a_seg", _ll)]
+                ("gate_batch", _ll), ("seg_cols", _i), ("n_segs", _i), ("a_seg", _ll), ("w_constant", _i)]
 
 
 class WindowAttnDesc(C.Structure):

@@ -116,6 +116,11 @@ int make_tmap_bf16_3d(CUtensorMap* map, const void* base, uint64_t d0, uint64_t 
   cuuint32_t box[3] = {b0, b1, b2};
   return encode(map, base, 3, dims, strides, box);
 }
+int make_tmap_bf16_4d(CUtensorMap* map, const void* base, const uint64_t* dims, const uint64_t* strides_elems, const uint32_t* box) {
+  cuuint64_t d[4] = {dims[0], dims[1], dims[2], dims[3]}, s[3] = {strides_elems[0] * 2, strides_elems[1] * 2, strides_elems[2] * 2};
+  cuuint32_t b[4] = {box[0], box[1], box[2], box[3]};
+  return encode(map, base, 4, d, s, b);
+}
 
 }  // namespace lp
 

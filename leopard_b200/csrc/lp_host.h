@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
+#include "lp_pdl.cuh"
 
 namespace lp {
 
@@ -115,6 +116,14 @@ inline cudaError_t launch_ex(void (*kern)(KArgs...), dim3 grid, dim3 block, size
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
+// The next kernel of a step: where it is small (decoding), its CTAs may be placed while the kernel before it still drains, when that one has asked for it; it
+// waits (pdl_wait) before it touches memory.  Pointers to what earlier kernels wrote are not __restrict__ there: a read-only load could be moved
+// before the wait.  Kernels of many CTAs gain nothing (prompts of 4,096 rows: 0.5 % slower with all of them launched so).
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_next(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  return launch_ex(kern, grid, block, smem, stream, 1, (long long)grid.x * grid.y * grid.z <= 4LL * sm_count(), args...);
+}
+
 // launch accounting + optional per-launch CUDA-event timing (off by default; see lp_profile_* in the public header)
 void note_launch(int n = 1);
 struct ProfScope {
@@ -155,5 +164,6 @@ int make_tmap_2d(CUtensorMap* map, const void* base, int elem_bytes, uint64_t in
                  uint32_t box_inner, uint32_t box_outer, int swizzle_bytes);
 int make_tmap_bf16_3d(CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t ld1_elems,
                       uint64_t ld2_elems, uint32_t b0, uint32_t b1, uint32_t b2);
+int make_tmap_bf16_4d(CUtensorMap* map, const void* base, const uint64_t* dims, const uint64_t* strides_elems, const uint32_t* box);
 
 }  // namespace lp

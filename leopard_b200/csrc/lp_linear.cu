@@ -20,6 +20,7 @@
 // The tcgen05 GEMM (lp_gemm_bf16) stays the matrix product of large bf16 problems; these kernels cover what it does not take:
 // fp32 operands, arbitrary shapes, few rows, and row-indexed groups whose sizes are only known on the device.
 #include <cuda_pipeline.h>
+#include "lp_common.cuh"
 #include "lp_host.h"
 #include "../../include/leopard_b200.h"
 
@@ -43,6 +44,7 @@ struct LinArgs {
   const float* bias;      // [N] added to the accumulators before the epilogue, or NULL
   const float* row_scale; // [rows of C] multiplies the accumulators before the bias, or NULL
   int seg_cols, n_segs; long long a_seg;   // seg_cols > 0: output columns [i seg_cols, (i + 1) seg_cols) read A + i a_seg (the last of n_segs: all that follow)
+  int w_constant;         // W is not written by launches that may still run: its first pieces are asked for before they have ended
   const float* gate; long long ldg, gate_batch;   // [rows of C, N'] pre-activations: the result is multiplied by sigmoid(gate), or NULL
 };
 
@@ -303,6 +305,9 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) linear_rows_kernel(LinArgs a)
 constexpr int STREAM_MAX_ROWS = 64, STREAM_MAX_PAIRS = 1024;
 
 struct Bf16Terms { uint4 hi, mid, lo; };
+__device__ __forceinline__ float4 as_floats(const uint4& u) {
+  return make_float4(__uint_as_float(u.x), __uint_as_float(u.y), __uint_as_float(u.z), __uint_as_float(u.w));
+}
 __device__ __forceinline__ uint32_t pack_upper(float x, float y) { return (__float_as_uint(x) >> 16) | (__float_as_uint(y) & 0xffff0000u); }
 __device__ __forceinline__ uint32_t take_upper(float& x, float& y) {      // what is left of x and y stays behind
   const uint32_t r = pack_upper(x, y);
@@ -352,6 +357,8 @@ __device__ float lin_plain_dot(const AT* x, const bf16* w, int K) {
   for (int k = 0; k < K && s == s; ++k) s = fmaf(lin_load(x + k), lin_load(w + k), s);
   return s;
 }
+template <typename AT>
+__device__ __noinline__ float lin_plain_sum(const AT* x, const bf16* w, int K) { return lin_plain_dot(x, w, K); }
 // linear_stream_kernel: `here` rows from m0 on, the first warp's share takes the new sum
 template <typename AT, int NT, int MG>
 __device__ __noinline__ void lin_mend_sums(float* sums, const AT* A, long long lda, const int* pair_of, int a_div, const bf16* W, long long ldw, int K,
@@ -382,6 +389,7 @@ __device__ __forceinline__ void mma_step(float* d, float* e, const uint4& w0, co
 
 template <typename AT, int NT, int MG>
 __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) linear_stream_kernel(LinArgs a, int gated, int c_fp32, int n_pairs) {
+  pdl_wait();
   extern __shared__ float dyn_smem[];      // [warps][NT MG 4][32] partial sums
   __shared__ int pair_of[STREAM_MAX_PAIRS];
   __shared__ int pair_count[STREAM_MAX_PAIRS / 32];
@@ -606,13 +614,368 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
   }
 }
 
+// ---------------------------------------------------------------------------------------------------------------------------------
+// The same product for up to 16 rows as one stream of weights: a CTA an SM walks its tiles of 16 or 32 weight rows, and one thread keeps a ring of pieces
+// of them full by TMA, so that DRAM sees whole kilobytes and the next pieces are under way while the sums of a tile are
+// stored.  Eight warps take the products of a piece, four others add up their sums and store the tile before: nothing in the stream waits for
+// an epilogue.  Where no launch before this one writes the weights (w_constant), the ring is filled before that launch has ended.
+// What bounds it is DRAM from about 30 MB of weights on (K = 4096, N = 32000: 39 us, 6.7 TB/s; the kernel above 46 at one row and 62 at 16; N = 16384 21.3 and
+// 24.7), below that the latency of a launch (K = N = 2048 3.7 us, 4.9).  A piece has to be large: at half of these sizes the waits between
+// pieces took the issue slots (39 -> 49 us), and bulk copies of a row each cost 110 cycles of a warp.  190 KB under way an SM: with 96 KB the same took 50 us.
+// The weights leave the L2 first: left to its usual order, they threw out the caches and states of the small kernels around them (window attention of one row 13 ->
+// 23 us).  Sums: 16 products a chain, which the instruction cuts off, then exactly; error against 64 bits, 1e-7 of the result: 0.5 for bf16 rows, 0.7 for fp32
+// rows at every K (above: 0.5 to 1.2 and 0.7 to 1.2).
+constexpr int RING_TAKERS = 8, RING_STORERS = 4, RING_WARPS = 2 + RING_TAKERS + RING_STORERS, RING_MAX_STAGES = 8, RING_MAX_GROUPS = 256;
+constexpr int RING_BYTES = 208 * 1024;      // of pieces and sums
+// A piece is KC columns of 16 NT weight rows and of the rows of A, boxes of 8 rows x 128 bytes one after another: a warp takes KC / 32 / 8 steps of it between two waits.
+template <typename AT> constexpr int ring_kc() { return sizeof(AT) == 2 ? 1024 : 512; }
+template <typename AT, int NT> constexpr int ring_w() { return NT * 16 * ring_kc<AT>() * 2; }
+// the rows of pairs lie apart and come by a bulk copy each: bytes from one to the next (four lanes' pieces of two rows are in banks of their own)
+template <typename AT> constexpr int ring_pair_row() { return ring_kc<AT>() * (int)sizeof(AT) + (sizeof(AT) == 2 ? 64 : 16); }
+template <typename AT, int NT, int MG, bool PAIRS> constexpr int ring_piece() {
+  return ring_w<AT, NT>() + (PAIRS ? (8 * MG * ring_pair_row<AT>() + 1023) / 1024 * 1024 : 8 * MG * ring_kc<AT>() * (int)sizeof(AT));
+}
+template <int NT, int MG> constexpr int ring_sums() { return 2 * RING_TAKERS * NT * MG * 4 * 32 * (int)sizeof(float); }
+template <typename AT, int NT, int MG, bool PAIRS> constexpr int ring_stages() {
+  constexpr int n = (RING_BYTES - ring_sums<NT, MG>()) / ring_piece<AT, NT, MG, PAIRS>();
+  return n < RING_MAX_STAGES ? n : RING_MAX_STAGES;
+}
+
+template <typename AT, int NT, int MG, bool PAIRS>
+__global__ void __launch_bounds__(RING_WARPS * 32, 1) linear_ring_kernel(const __grid_constant__ CUtensorMap tw, const __grid_constant__ CUtensorMap ta, LinArgs a,
+                                                                         int gated, int c_fp32, int batch, int n_pairs, int n_groups) {
+  extern __shared__ float dyn_smem[];      // (from the next multiple of 1024 bytes) [stages] pieces, then [2][takers][MG 4][32] sums
+  __shared__ uint64_t full[RING_MAX_STAGES], empty[RING_MAX_STAGES], sums_full[2], sums_empty[2];
+  __shared__ int pair_of[PAIRS ? STREAM_MAX_PAIRS : 1];      // the pairs, a group's together
+  __shared__ int count[PAIRS ? RING_MAX_GROUPS : 1];
+  __shared__ int2 block_of[PAIRS ? RING_MAX_GROUPS + STREAM_MAX_PAIRS / 8 : 1];      // {group, place of its first pair, number of pairs << 16} of up to 8 MG of a group's pairs
+  __shared__ int n_blocks;
+  constexpr int KC = ring_kc<AT>(), STEPS = KC / 32 / RING_TAKERS, SLOTS = NT * MG * 4, PIECE = ring_piece<AT, NT, MG, PAIRS>(), STAGES = ring_stages<AT, NT, MG, PAIRS>();
+  constexpr int HALF = 8 * KC * 2;      // eight weight rows
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int n_out = gated ? a.N / 2 : a.N, cols = gated ? 8 * NT : 16 * NT, tiles = (n_out + cols - 1) / cols;
+  uint8_t* const ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn_smem) + 1023) & ~(uintptr_t)1023);
+  float* const sums = reinterpret_cast<float*>(ring + STAGES * PIECE);
+  const int pieces = (a.K + KC - 1) / KC;
+  const bool ahead = !PAIRS && a.w_constant != 0;
+  pdl_launch_dependents();
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < STAGES; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], RING_TAKERS);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&sums_full[i], RING_TAKERS);
+      mbar_init(&sums_empty[i], RING_STORERS);
+    }
+    fence_barrier_init();
+  }
+  if constexpr (PAIRS) {      // the pairs of each group, in order: counts, places, blocks of up to 8 MG
+    pdl_wait();
+    const int spans = (n_pairs + 31) / 32;
+    for (int e = warp; e < n_groups; e += RING_WARPS) {
+      int c = 0;
+      for (int q = 0; q < spans; ++q) c += __popc(__ballot_sync(0xffffffffu, q * 32 + lane < n_pairs && a.z_group[q * 32 + lane] == e));
+      if (lane == 0) count[e] = c;
+    }
+    __syncthreads();
+    for (int e = warp; e < n_groups; e += RING_WARPS) {
+      if (count[e] == 0) continue;
+      int place = 0, block = 0;
+      for (int i = 0; i < e; ++i) {
+        place += count[i];
+        block += (count[i] + 8 * MG - 1) / (8 * MG);
+      }
+      for (int i = lane; i * 8 * MG < count[e]; i += 32) block_of[block + i] = make_int2(e, (place + i * 8 * MG) | (min(8 * MG, count[e] - i * 8 * MG) << 16));
+      for (int q = 0; q < spans; ++q) {
+        const bool mine = q * 32 + lane < n_pairs && a.z_group[q * 32 + lane] == e;
+        const unsigned m = __ballot_sync(0xffffffffu, mine);
+        if (mine) pair_of[place + __popc(m & ((1u << lane) - 1u))] = q * 32 + lane;
+        place += __popc(m);
+      }
+    }
+    if (threadIdx.x == 0) {
+      int n = 0;
+      for (int i = 0; i < n_groups; ++i) n += (count[i] + 8 * MG - 1) / (8 * MG);
+      n_blocks = n;
+    }
+  }
+  __syncthreads();
+  const int units = tiles * (PAIRS ? n_blocks : batch);
+  struct Unit { int n0, z, first, here; };      // its first output column, its problem or group, its rows (PAIRS: from place `first` on)
+  auto unit_at = [&](int u) {
+    Unit r;
+    const int b = u / tiles;
+    r.n0 = (u - b * tiles) * cols;
+    if constexpr (PAIRS) {
+      const int2 v = block_of[b];
+      r.z = v.x;
+      r.first = v.y & 0xffff;
+      r.here = v.y >> 16;
+    } else {
+      r.z = b;
+      r.first = 0;
+      r.here = a.M;
+    }
+    return r;
+  };
+  auto row_of = [&](const Unit& u, int m) {      // row m of a unit's operand
+    const AT* A = reinterpret_cast<const AT*>(a.A);
+    if constexpr (PAIRS) return A + (long long)(pair_of[u.first + m] / a.a_div) * a.lda;
+    return A + (long long)u.z * a.a_batch + lin_seg(a, u.n0) + (long long)m * a.lda;
+  };
+  if (warp == 0) {
+    // ---------------------------------------------------------------- copies
+    const uint64_t once = read_once_policy();
+    struct At { int u, piece; Unit unit; };      // a place in the stream of this CTA's pieces
+    auto next = [&](At& p) {
+      if (++p.piece < pieces) return;
+      p.piece = 0;
+      p.u += gridDim.x;
+      if (p.u < units) p.unit = unit_at(p.u);
+    };
+    auto load_w = [&](const At& p, int stage) {
+      if (lane != 0) return;
+      const int kc = min(KC, a.K - p.piece * KC);
+      mbar_arrive_expect_tx(&full[stage], (uint32_t)(ring_w<AT, NT>() + (PAIRS ? p.unit.here * kc : 8 * MG * KC) * (int)sizeof(AT)));
+#pragma unroll
+      for (int h = 0; h < 2 * NT; ++h) {
+        const int n = gated ? p.unit.n0 + (h >> 1) * 8 + (h & 1) * n_out : p.unit.n0 + h * 8;
+        tma_load_4d_once(ring + stage * PIECE + h * HALF, &tw, &full[stage], 0, n, p.piece * (KC / 64), p.unit.z, once);
+      }
+    };
+    auto load_a = [&](const At& p, int stage) {
+      if (PAIRS || lane != 0) return;
+      const int z = a.seg_cols > 0 ? min(p.unit.n0 / a.seg_cols, a.n_segs - 1) : p.unit.z;
+#pragma unroll
+      for (int i = 0; i < MG; ++i)
+        tma_load_4d(ring + stage * PIECE + ring_w<AT, NT>() + i * 8 * KC * (int)sizeof(AT), &ta, &full[stage], 0, 8 * i, p.piece * (KC * (int)sizeof(AT) / 128), z);
+    };
+    At w{(int)blockIdx.x, 0, {}};
+    if (w.u < units) w.unit = unit_at(w.u);
+    int stage = 0;
+    uint32_t phase = 0;
+    if (ahead) {
+      At x = w;
+      for (; stage < STAGES && w.u < units; ++stage) {
+        load_w(w, stage);
+        next(w);
+      }
+      pdl_wait();
+      for (int i = 0; i < stage; ++i) {
+        load_a(x, i);
+        next(x);
+      }
+      if (stage == STAGES) { stage = 0; phase = 1; }
+    } else {
+      pdl_wait();
+    }
+    for (; w.u < units; next(w)) {
+      mbar_wait(&empty[stage], phase ^ 1);
+      load_w(w, stage);
+      load_a(w, stage);
+      if (++stage == STAGES) { stage = 0; phase ^= 1; }
+    }
+  } else if (warp <= RING_TAKERS) {
+    // ---------------------------------------------------------------- products: STEPS steps of 32 columns of every piece are this warp's
+    const int cw = warp - 1;
+    // row g of a box lies where four lanes' pieces of two rows are in banks of their own
+    const int at_row = (g >> 1) | ((g & 1) << 2), x_row = sizeof(AT) == 2 ? at_row : g;
+    constexpr int XV = sizeof(AT) == 2 ? 1 : 2;      // 16-byte pieces of eight values of a row
+    // this lane's piece of a step in the lower half of a 128-byte line; the upper half's is 64 bytes away, either way
+    const int w_at = at_row * 128 + (t ^ at_row) * 16;
+    const int x_at = PAIRS ? g * ring_pair_row<AT>() + t * 8 * (int)sizeof(AT) : sizeof(AT) == 2 ? w_at : x_row * 128;
+    int stage = 0, turn = 0;
+    uint32_t phase = 0;
+    pdl_wait();
+    for (int u = blockIdx.x; u < units; u += gridDim.x, ++turn) {
+      float acc[NT][MG][4], rest[NT][MG][4];      // rest: what adding the steps' sums rounded off
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int i = 0; i < MG; ++i)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[j][i][c] = rest[j][i][c] = 0.f;
+#pragma unroll 1
+      for (int piece = 0; piece < pieces; ++piece) {
+        mbar_wait(&full[stage], phase);
+        const uint8_t* const base = ring + stage * PIECE;
+        uint4 u0[STEPS][NT], u1[STEPS][NT], v[STEPS][MG][XV];
+#pragma unroll
+        for (int q = 0; q < STEPS; ++q) {
+          const int step = STEPS * cw + q;      // STEPS is even: which half of the line is known here
+#pragma unroll
+          for (int j = 0; j < NT; ++j) {
+            const uint8_t* const w = base + j * 2 * HALF + (step >> 1) * 1024 + (w_at ^ ((q & 1) * 64));
+            u0[q][j] = *reinterpret_cast<const uint4*>(w);
+            u1[q][j] = *reinterpret_cast<const uint4*>(w + HALF);
+          }
+#pragma unroll
+          for (int i = 0; i < MG; ++i)
+#pragma unroll
+            for (int p = 0; p < XV; ++p) {
+              const uint8_t* x = base + ring_w<AT, NT>();
+              if constexpr (PAIRS) x += 8 * i * ring_pair_row<AT>() + step * 32 * (int)sizeof(AT) + x_at + 16 * p;
+              else if constexpr (sizeof(AT) == 2) x += i * 8 * KC * 2 + (step >> 1) * 1024 + (x_at ^ ((q & 1) * 64));
+              else x += i * 8 * KC * 4 + step * 1024 + x_at + ((2 * t + p) ^ x_row) * 16;
+              v[q][i][p] = *reinterpret_cast<const uint4*>(x);
+            }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[stage]);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        if (piece * KC + STEPS * cw * 32 >= a.K) continue;      // the columns from K on of a piece are zeros
+#pragma unroll
+        for (int i = 0; i < MG; ++i) {
+          float sum[NT][STEPS][4];
+#pragma unroll
+          for (int q = 0; q < STEPS; ++q) {
+            Bf16Terms y;
+            if constexpr (sizeof(AT) == 4) y = split3(as_floats(v[q][i][0]), as_floats(v[q][i][XV - 1]));
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+              float d[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
+              if constexpr (sizeof(AT) == 2) {
+                mma_step(d, e, u0[q][j], u1[q][j], v[q][i][0]);
+              } else {      // the small terms first
+                mma_step(d, e, u0[q][j], u1[q][j], y.lo);
+                mma_step(d, e, u0[q][j], u1[q][j], y.mid);
+                mma_step(d, e, u0[q][j], u1[q][j], y.hi);
+              }
+#pragma unroll
+              for (int c = 0; c < 4; ++c) sum[j][q][c] = d[c] + e[c];
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+              for (int q = 0; q < STEPS; ++q) rest[j][i][c] += add_exactly(acc[j][i][c], sum[j][q][c]);
+        }
+      }
+      const int buf = turn & 1;
+      mbar_wait(&sums_empty[buf], ((turn >> 1) & 1) ^ 1);
+      float* mine = sums + (buf * RING_TAKERS + cw) * SLOTS * 32 + lane;
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int i = 0; i < MG; ++i)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const float s = acc[j][i][c] + rest[j][i][c];
+            mine[((j * MG + i) * 4 + c) * 32] = s == s ? s : acc[j][i][c];      // beside an infinity the rest is NaN
+          }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sums_full[buf]);
+    }
+  } else if (warp == RING_WARPS - 1) {
+    // ---------------------------------------------------------------- the rows of pairs, which lie apart: a lane each
+    if constexpr (PAIRS) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int at = blockIdx.x; at < units; at += gridDim.x) {
+        const Unit u = unit_at(at);
+        const AT* const x = lane < u.here ? row_of(u, lane) : nullptr;
+        for (int piece = 0; piece < pieces; ++piece) {
+          mbar_wait(&empty[stage], phase ^ 1);
+          if (x != nullptr)
+            bulk_load(ring + stage * PIECE + ring_w<AT, NT>() + lane * ring_pair_row<AT>(), x + piece * KC,
+                      (uint32_t)(min(KC, a.K - piece * KC) * (int)sizeof(AT)), &full[stage]);
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+  } else {
+    // ---------------------------------------------------------------- the takers' sums in a fixed order, what the additions round off kept; the epilogue
+    const int et = threadIdx.x - (1 + RING_TAKERS) * 32;
+    int turn = 0;
+    pdl_wait();
+    for (int at = blockIdx.x; at < units; at += gridDim.x, ++turn) {
+      const Unit u = unit_at(at);
+      const int buf = turn & 1;
+      mbar_wait(&sums_full[buf], (turn >> 1) & 1);
+      const float* part = sums + buf * RING_TAKERS * SLOTS * 32;
+      for (int e = et; e < cols * u.here; e += RING_STORERS * 32) {
+        const int nl = e & (cols - 1), ml = e / cols, n = u.n0 + nl;
+        if (n >= n_out) continue;
+        const int j = gated ? nl >> 3 : nl >> 4, r = gated ? nl & 7 : nl & 15;
+        const int lane_row = ((r & 3) << 1) | ((r & 7) >> 2);      // the lanes' g whose weight row this is
+        const int mc = sizeof(AT) == 2 && !PAIRS ? ((ml & 3) << 1) | ((ml & 7) >> 2) : ml & 7;      // and whose row of A
+        const int slot = ((j * MG + (ml >> 3)) * 4 + (r >> 3) * 2 + (mc & 1)) * 32 + lane_row * 4 + (mc >> 1);
+        float s = 0.f, s2 = 0.f, lost = 0.f, lost2 = 0.f;
+#pragma unroll
+        for (int w = 0; w < RING_TAKERS; ++w) {
+          lost += add_exactly(s, part[w * SLOTS * 32 + slot]);
+          if (gated) lost2 += add_exactly(s2, part[w * SLOTS * 32 + slot + 64]);
+        }
+        if (s + lost == s + lost) s += lost;      // beside an infinity the rest is NaN
+        if (s2 + lost2 == s2 + lost2) s2 += lost2;
+        if constexpr (sizeof(AT) == 4) {      // terms of what is not finite: the sum in plain multiply-adds
+          const bf16* W = a.W + (long long)u.z * a.w_batch;
+          if (s != s) s = lin_plain_sum(row_of(u, ml), W + (long long)n * a.ldw, a.K);
+          if (s2 != s2) s2 = lin_plain_sum(row_of(u, ml), W + (long long)(n + n_out) * a.ldw, a.K);
+        }
+        const int m = PAIRS ? pair_of[u.first + ml] : ml;
+        if (a.row_scale != nullptr) {
+          s *= a.row_scale[m];
+          s2 *= a.row_scale[m];
+        }
+        if (a.bias != nullptr) {
+          s += a.bias[n];
+          if (gated) s2 += a.bias[n + n_out];
+        }
+        float v = gated ? lin_gate(a.epi, s, s2, a.e0, a.e1) : lin_epi(a.epi, s, a.e0, a.e1);
+        const int z = PAIRS ? 0 : u.z;
+        if (a.gate != nullptr) v /= 1.0f + expf(-a.gate[(long long)z * a.gate_batch + (long long)m * a.ldg + n]);
+        const long long at_c = (long long)z * a.c_batch + (long long)m * a.ldc + n;
+        if (c_fp32) {
+          float* C = reinterpret_cast<float*>(a.C) + at_c;
+          *C = a.c_accum ? fmaf(a.c_scale, v, *C) : v;
+        } else {
+          bf16* C = reinterpret_cast<bf16*>(a.C) + at_c;
+          *C = __float2bfloat16(a.c_accum ? fmaf(a.c_scale, v, __bfloat162float(*C)) : v);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sums_empty[buf]);
+    }
+  }
+}
+
 static bool gated_epi(int epi) { return epi == LP_EPI_SILU_GATE || epi == LP_EPI_CLAMP_GLU || epi == LP_EPI_GELU_GATE; }
 
 template <typename AT, int NT, int MG>
 static int launch_stream(const LinArgs& a, int c_fp32, dim3 grid, int warps, int n_pairs, cudaStream_t stream) {
   const size_t smem = (size_t)warps * NT * MG * 4 * 32 * sizeof(float);
   if (smem > 40 * 1024) LP_CHECK_CUDA(cudaFuncSetAttribute(linear_stream_kernel<AT, NT, MG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536));
-  linear_stream_kernel<AT, NT, MG><<<grid, warps * 32, smem, stream>>>(a, gated_epi(a.epi), c_fp32, n_pairs);
+  LP_CHECK_CUDA((launch_next(linear_stream_kernel<AT, NT, MG>, grid, dim3(warps * 32), smem, stream, a, gated_epi(a.epi), c_fp32, n_pairs)));
+  note_launch();
+  LP_CHECK_CUDA(cudaGetLastError());
+  return 0;
+}
+
+template <typename AT, int NT, int MG, bool PAIRS>
+static int launch_ring(const LinArgs& a, int c_fp32, int batch, int n_pairs, int n_groups, cudaStream_t stream) {
+  constexpr int KC = ring_kc<AT>(), halves = sizeof(AT) / 2;
+  const int n_out = gated_epi(a.epi) ? a.N / 2 : a.N, per = (gated_epi(a.epi) ? 8 : 16) * NT, problems = PAIRS ? n_groups : batch;
+  const long long units = (long long)problems * ((n_out + per - 1) / per);
+  // 64 columns of 16 bits, the rows, the blocks of 64, the problems (of A: the segments)
+  CUtensorMap tw, ta = {};
+  const uint64_t w_dims[4] = {64, (uint64_t)a.N, (uint64_t)(a.K / 64), (uint64_t)problems}, w_strides[3] = {(uint64_t)(a.N > 1 ? a.ldw : 64), 64, (uint64_t)(problems > 1 ? a.w_batch : 64)};
+  const uint32_t w_box[4] = {64, 8, KC / 64, 1};
+  if (const int rc = make_tmap_bf16_4d(&tw, a.W, w_dims, w_strides, w_box)) return rc;
+  if (!PAIRS) {
+    const uint64_t many = a.seg_cols > 0 ? a.n_segs : batch, far = a.seg_cols > 0 ? a.a_seg : a.a_batch;
+    const uint64_t dims[4] = {64, (uint64_t)a.M, (uint64_t)(a.K * halves / 64), many}, strides[3] = {(uint64_t)(a.M > 1 ? a.lda * halves : 64), 64, many > 1 ? far * halves : 64};
+    const uint32_t box[4] = {64, 8, KC * halves / 64, 1};
+    if (const int rc = make_tmap_bf16_4d(&ta, a.A, dims, strides, box)) return rc;
+  }
+  constexpr int smem = 1024 + ring_stages<AT, NT, MG, PAIRS>() * ring_piece<AT, NT, MG, PAIRS>() + ring_sums<NT, MG>();
+  LP_CHECK_CUDA((cudaFuncSetAttribute(linear_ring_kernel<AT, NT, MG, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)));
+  LP_CHECK_CUDA((launch_next(linear_ring_kernel<AT, NT, MG, PAIRS>, dim3((unsigned)(units < sm_count() ? units : sm_count())), dim3(RING_WARPS * 32), smem, stream, tw, ta, a,
+                             (int)gated_epi(a.epi), c_fp32, batch, n_pairs, n_groups)));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
@@ -630,6 +993,27 @@ static int dispatch_stream(const LinArgs& a, int a_fp32, int c_fp32, int batch, 
   const int n_out = gated_epi(a.epi) ? a.N / 2 : a.N, per = gated_epi(a.epi) ? 8 : 16;
   const int mg = rows <= 8 ? 1 : rows <= 16 ? 2 : rows <= 32 ? 4 : 8;
   const long long problems = n_groups > 0 ? n_groups : batch;
+  const long long ring_units = problems * ((n_out + per - 1) / per);
+  const long long ring_pairs = (ring_units + 1) / 2;      // units of two tiles
+  // Both sides (us, the kernel below and the ring, us a launch in a graph; K, N, rows): bf16 512, 512, 1 2.5, 2.3; 2048, 2048, 8 5.0, 3.6; 4096, 6144, 8 12.1, 9.1; 16384, 4096, 8
+  // 24.2, 21.3; 4096, 32000, 16 62, 44; but 128, 16 x 512, 16 4.3, 6.5 (tiles of one short piece).  fp32 rows are cut into terms for every tile: two tiles a piece where there
+  // is more than one a CTA (2048, 8192, 4 13.0, 10.2 with one and two), and not where the last round of these would be mostly empty (4096, 6144, 4 14.8, 15.7) or
+  // 9 to 16 rows fill the issue slots (4096, 16384, 16 47, 55; 2048, 2048, 16 7.3, 7.5; but 4096, 6144, 16 34, 29).  Pairs: 16 groups of 2048 x 1024, 12 pairs 13.4, 11.7; 32 of
+  // 2048 x 4096, 32 pairs 67, 59; 8 of 1024 x 1024, 16 pairs 6.1, 7.1 (the sorting of the pairs is not hidden).
+  const bool fp32_pays = !a_fp32 || (mg == 1 ? ring_pairs <= sm_count() || 2 * ring_pairs > 3 * sm_count() : ring_units > sm_count() && ring_units <= 4 * sm_count());
+  const bool ring_pays = n_groups > 0 ? n_pairs <= 4 || (long long)(n_pairs < n_groups ? n_pairs : n_groups) * a.N * a.K >= (1 << 24) : a.K >= (mg == 1 ? 512 : 2048) || ring_units <= sm_count();
+  // rows, operands and problems lie at increasing addresses: what a tensor map can say
+  const bool ring_reads = (a.N == 1 || a.ldw > 0) && (a.M == 1 || a.lda > 0) && (problems == 1 || a.w_batch > 0) && (batch == 1 || a.a_batch > 0) &&
+                          (a.seg_cols == 0 || a.n_segs == 1 || a.a_seg > 0);
+  if (mg <= 2 && ring_reads && ring_pays && (n_groups > 0 || fp32_pays) && n_groups <= RING_MAX_GROUPS && a.K % 64 == 0 && ring_units < (1LL << 31)) {
+    const bool two = a_fp32 && ring_units > sm_count() && (a.seg_cols == 0 || a.seg_cols % (2 * per) == 0);
+#define LP_RING(MG, PAIRS)                                                                                                 \
+  (!a_fp32 ? launch_ring<bf16, 1, MG, PAIRS>(a, c_fp32, batch, n_pairs, n_groups, stream)                                  \
+           : two ? launch_ring<float, 2, MG, PAIRS>(a, c_fp32, batch, n_pairs, n_groups, stream) : launch_ring<float, 1, MG, PAIRS>(a, c_fp32, batch, n_pairs, n_groups, stream))
+    if (n_groups > 0) return mg == 1 ? LP_RING(1, true) : LP_RING(2, true);
+    return mg == 1 ? LP_RING(1, false) : LP_RING(2, false);
+#undef LP_RING
+  }
   // fp32 rows: two tiles a CTA read A half as often and cut it into terms once, taken once the grid still has two CTAs for every SM and where segments
   // allow.  bf16 rows take one: its registers leave room for the next steps' weights (one row, us, two tiles and one: K = 4096, N = 16384 28.1, 25.9, N =
   // 32000 49.2, 46.1; eight rows of 14 experts, K = 2048, N = 2048 27.2, 24.1; with 16 rows, N = 12288, K = 4096, 46, 35)
@@ -928,6 +1312,7 @@ extern "C" int lp_linear(const lp_linear_desc* d, void* stream_) {
   a.a_rows = nullptr; a.tile_group = nullptr; a.z_group = nullptr; a.a_div = 1;
   a.bias = d->bias; a.row_scale = d->row_scale; a.gate = d->gate; a.ldg = d->ldg; a.gate_batch = d->gate_batch;
   a.seg_cols = d->seg_cols; a.n_segs = d->n_segs; a.a_seg = d->a_seg;
+  a.w_constant = d->w_constant;
   LP_REQUIRE(d->batch == 1 || (d->bias == nullptr && d->row_scale == nullptr), "lp_linear: bias and row scale are for one problem");
   // a CTA's columns read one operand: 8 columns for few rows, a tile otherwise
   LP_REQUIRE(d->seg_cols == 0 || (d->seg_cols > 0 && d->n_segs >= 1 && d->seg_cols % (d->M <= ROWS_MAX ? ROWS_WARPS : LIN_BN) == 0),
@@ -958,7 +1343,7 @@ static int linear_pairs(const lp_linear_desc* d, const int* pair_group, int n_gr
   a.epi = d->epi; a.e0 = d->epi_a; a.e1 = d->epi_b; a.c_accum = d->c_accum; a.c_scale = d->c_scale;
   a.a_rows = nullptr; a.tile_group = nullptr; a.z_group = pair_group; a.a_div = a_div;
   a.bias = d->bias; a.row_scale = d->row_scale; a.gate = d->gate; a.ldg = d->ldg; a.gate_batch = d->gate_batch;
-  a.seg_cols = 0; a.n_segs = 0; a.a_seg = 0;
+  a.seg_cols = 0; a.n_segs = 0; a.a_seg = 0; a.w_constant = d->w_constant;
   // with the number of groups a group's weights are read once for all of its pairs
   if (n_groups > 0 && n_pairs <= STREAM_MAX_PAIRS && stream_ok(a, d->a_fp32, 1))
     return dispatch_stream(a, d->a_fp32, d->c_fp32, 1, 2 * ((n_pairs + n_groups - 1) / n_groups), n_groups, n_pairs, stream);
@@ -994,7 +1379,7 @@ extern "C" int lp_linear_grouped(const lp_linear_desc* d, const int* tile_group,
   a.epi = d->epi; a.e0 = d->epi_a; a.e1 = d->epi_b; a.c_accum = d->c_accum; a.c_scale = d->c_scale;
   a.a_rows = a_rows; a.tile_group = tile_group; a.z_group = nullptr; a.a_div = 1;
   a.bias = d->bias; a.row_scale = d->row_scale; a.gate = d->gate; a.ldg = d->ldg; a.gate_batch = d->gate_batch;
-  a.seg_cols = 0; a.n_segs = 0; a.a_seg = 0;
+  a.seg_cols = 0; a.n_segs = 0; a.a_seg = 0; a.w_constant = d->w_constant;
   if (stream_ok(a, d->a_fp32, 1) && mma_pays(a, 1, n_tiles)) return dispatch_mma(a, d->a_fp32, d->c_fp32, 1, n_tiles, stream);
   return dispatch_linear(a, d->a_fp32, d->c_fp32, 1, n_tiles, false, stream);
 }

@@ -42,6 +42,8 @@ constexpr int GRU_THREADS = 128;
 
 __global__ void __launch_bounds__(GRU_THREADS)
 mingru_chunk_kernel(GruArgs a, const int* __restrict__ chunk_row0, const int* __restrict__ chunk_len, float* __restrict__ ws, int n_chunks) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int c = blockIdx.x, ch = blockIdx.y * GRU_THREADS + threadIdx.x;
   if (ch >= a.width) return;
   const int row0 = chunk_row0[c], len = chunk_len[c];
@@ -61,7 +63,9 @@ mingru_chunk_kernel(GruArgs a, const int* __restrict__ chunk_row0, const int* __
 
 __global__ void __launch_bounds__(GRU_THREADS)
 mingru_scan_kernel(GruArgs a, const int* __restrict__ seq_chunk0, const int* __restrict__ seq_pos0, const int* __restrict__ seq_slot,
-                   float* __restrict__ ws, int n_chunks) {
+                   float* ws, int n_chunks) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int s = blockIdx.x, ch = blockIdx.y * GRU_THREADS + threadIdx.x;
   if (ch >= a.width) return;
   float S = seq_pos0[s] == 0 ? 0.f : a.state[(long long)seq_slot[s] * a.slot_stride + ch];
@@ -74,7 +78,9 @@ mingru_scan_kernel(GruArgs a, const int* __restrict__ seq_chunk0, const int* __r
 
 __global__ void __launch_bounds__(GRU_THREADS)
 mingru_out_kernel(GruArgs a, const int* __restrict__ chunk_seq, const int* __restrict__ chunk_row0, const int* __restrict__ chunk_len,
-                  const int* __restrict__ seq_chunk0, const int* __restrict__ seq_slot, const float* __restrict__ ws) {
+                  const int* __restrict__ seq_chunk0, const int* __restrict__ seq_slot, const float* ws) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int c = blockIdx.x, ch = blockIdx.y * GRU_THREADS + threadIdx.x;
   if (ch >= a.width) return;
   const int row0 = chunk_row0[c], len = chunk_len[c], s = chunk_seq[c];
@@ -90,6 +96,8 @@ mingru_out_kernel(GruArgs a, const int* __restrict__ chunk_seq, const int* __res
 
 __global__ void __launch_bounds__(GRU_THREADS)
 mingru_decode_kernel(GruArgs a, const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0, const int* __restrict__ seq_slot) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int s = blockIdx.x, ch = blockIdx.y * GRU_THREADS + threadIdx.x;
   if (ch >= a.width) return;
   const long long row = seq_row0[s];
@@ -131,11 +139,11 @@ extern "C" int lp_mingru_prefill(const lp_mingru_desc* d, int n_seqs, int n_chun
   LP_REQUIRE(ws != nullptr && ws_bytes >= lp_mingru_workspace_bytes(n_chunks, d->width), "lp_mingru_prefill: workspace too small");
   float* w = reinterpret_cast<float*>(ws);
   const int cy = (d->width + GRU_THREADS - 1) / GRU_THREADS;
-  mingru_chunk_kernel<<<dim3(n_chunks, cy), GRU_THREADS, 0, stream>>>(a, chunk_row0, chunk_len, w, n_chunks);
+  LP_CHECK_CUDA(launch_next(mingru_chunk_kernel, dim3(n_chunks, cy), dim3(GRU_THREADS), 0, stream, a, chunk_row0, chunk_len, w, n_chunks));
   LP_CHECK_CUDA(cudaGetLastError());
-  mingru_scan_kernel<<<dim3(n_seqs, cy), GRU_THREADS, 0, stream>>>(a, seq_chunk0, seq_pos0, seq_slot, w, n_chunks);
+  LP_CHECK_CUDA(launch_next(mingru_scan_kernel, dim3(n_seqs, cy), dim3(GRU_THREADS), 0, stream, a, seq_chunk0, seq_pos0, seq_slot, w, n_chunks));
   LP_CHECK_CUDA(cudaGetLastError());
-  mingru_out_kernel<<<dim3(n_chunks, cy), GRU_THREADS, 0, stream>>>(a, chunk_seq, chunk_row0, chunk_len, seq_chunk0, seq_slot, w);
+  LP_CHECK_CUDA(launch_next(mingru_out_kernel, dim3(n_chunks, cy), dim3(GRU_THREADS), 0, stream, a, chunk_seq, chunk_row0, chunk_len, seq_chunk0, seq_slot, w));
   LP_CHECK_CUDA(cudaGetLastError());
   note_launch(3);
   return 0;
@@ -148,7 +156,7 @@ extern "C" int lp_mingru_decode(const lp_mingru_desc* d, int n_seqs, const int* 
   if (int rc = fill_gru(a, d)) return rc;
   LP_REQUIRE(seq_row0 != nullptr && seq_pos0 != nullptr && seq_slot != nullptr, "lp_mingru_decode: null table");
   if (n_seqs <= 0) return 0;
-  mingru_decode_kernel<<<dim3(n_seqs, (d->width + GRU_THREADS - 1) / GRU_THREADS), GRU_THREADS, 0, stream>>>(a, seq_row0, seq_pos0, seq_slot);
+  LP_CHECK_CUDA(launch_next(mingru_decode_kernel, dim3(n_seqs, (d->width + GRU_THREADS - 1) / GRU_THREADS), dim3(GRU_THREADS), 0, stream, a, seq_row0, seq_pos0, seq_slot));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;

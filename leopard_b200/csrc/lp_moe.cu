@@ -64,10 +64,12 @@ __device__ __forceinline__ void warp_best(float& v, int& i, int none) {
 // allows; then one warp makes the choice among the E scores.
 template <typename HT>
 __global__ void __launch_bounds__(ROUTE_WARPS_WIDE * 32)
-moe_route_kernel(const HT* __restrict__ h, long long ldh, int T, int D, const bf16* __restrict__ w_router, long long ldw, int E,
+moe_route_kernel(const HT* h, long long ldh, int T, int D, const bf16* __restrict__ w_router, long long ldw, int E,
                  const float* __restrict__ correction, int n_groups, int keep_groups, int top, const bf16* __restrict__ w_gate,
                  int* __restrict__ idx_out, float* __restrict__ w_out, float* __restrict__ gate_out, int softmax_mode,
                  const float* __restrict__ logit_bias, float w_scale) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float sc[MOE_MAX_EXPERTS];   // sigmoid scores
   __shared__ float ch[MOE_MAX_EXPERTS];   // choice scores (minus infinity once taken or not eligible)
   __shared__ float gsc[MOE_MAX_GROUPS];   // group scores
@@ -180,8 +182,10 @@ __global__ void moe_sorted_weights_kernel(const int* __restrict__ pair_row, cons
 // one CTA: counts, padded offsets, scatter
 constexpr int ALIGN_THREADS = 1024;
 __global__ void __launch_bounds__(ALIGN_THREADS)
-moe_align_kernel(const int* __restrict__ idx, int n_pairs, int top, int E, int tile_rows, int max_tiles, int* __restrict__ tile_group,
+moe_align_kernel(const int* idx, int n_pairs, int top, int E, int tile_rows, int max_tiles, int* __restrict__ tile_group,
                  int* __restrict__ sorted_token, int* __restrict__ pair_row) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ unsigned cnt[MOE_MAX_EXPERTS];
   __shared__ int off[MOE_MAX_EXPERTS + 1];
   const int tid = threadIdx.x;
@@ -209,9 +213,11 @@ moe_align_kernel(const int* __restrict__ idx, int n_pairs, int top, int E, int t
   }
 }
 
-__global__ void moe_combine_kernel(const float* __restrict__ y, long long ldy, const int* __restrict__ pair_row, const float* __restrict__ w,
-                                   int top, const float* __restrict__ shared, long long lds, const float* __restrict__ gate,
+__global__ void moe_combine_kernel(const float* y, long long ldy, const int* pair_row, const float* w,
+                                   int top, const float* shared, long long lds, const float* gate,
                                    float* __restrict__ out, long long ldo, int T, int D) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int t = blockIdx.x;
   if (t >= T) return;
   for (int c = threadIdx.x; c < D; c += blockDim.x) {
@@ -244,13 +250,13 @@ extern "C" int lp_moe_route(const void* h, long long ldh, int h_fp32, int T, int
   if (T <= 0) return 0;
   const unsigned grid = (unsigned)T;
   if (h_fp32)
-    moe_route_kernel<float><<<grid, route_threads(T, E), 0, stream>>>(reinterpret_cast<const float*>(h), ldh, T, D,
+    LP_CHECK_CUDA(launch_next(moe_route_kernel<float>, grid, dim3(route_threads(T, E)), 0, stream, reinterpret_cast<const float*>(h), ldh, T, D,
         reinterpret_cast<const bf16*>(w_router), ldw, E, correction, n_groups, keep_groups, top, reinterpret_cast<const bf16*>(w_gate),
-        idx_out, w_out, gate_out, 0, nullptr, 1.0f);
+        idx_out, w_out, gate_out, 0, nullptr, 1.0f));
   else
-    moe_route_kernel<bf16><<<grid, route_threads(T, E), 0, stream>>>(reinterpret_cast<const bf16*>(h), ldh, T, D,
+    LP_CHECK_CUDA(launch_next(moe_route_kernel<bf16>, grid, dim3(route_threads(T, E)), 0, stream, reinterpret_cast<const bf16*>(h), ldh, T, D,
         reinterpret_cast<const bf16*>(w_router), ldw, E, correction, n_groups, keep_groups, top, reinterpret_cast<const bf16*>(w_gate),
-        idx_out, w_out, gate_out, 0, nullptr, 1.0f);
+        idx_out, w_out, gate_out, 0, nullptr, 1.0f));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
@@ -265,11 +271,11 @@ extern "C" int lp_moe_route_softmax(const void* h, long long ldh, int h_fp32, in
   if (T <= 0) return 0;
   const unsigned grid = (unsigned)T;
   if (h_fp32)
-    moe_route_kernel<float><<<grid, route_threads(T, E), 0, stream>>>(reinterpret_cast<const float*>(h), ldh, T, D,
-        reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, 1, 1, top, nullptr, idx_out, w_out, nullptr, 1, logit_bias, 1.0f);
+    LP_CHECK_CUDA(launch_next(moe_route_kernel<float>, grid, dim3(route_threads(T, E)), 0, stream, reinterpret_cast<const float*>(h), ldh, T, D,
+        reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, 1, 1, top, nullptr, idx_out, w_out, nullptr, 1, logit_bias, 1.0f));
   else
-    moe_route_kernel<bf16><<<grid, route_threads(T, E), 0, stream>>>(reinterpret_cast<const bf16*>(h), ldh, T, D,
-        reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, 1, 1, top, nullptr, idx_out, w_out, nullptr, 1, logit_bias, 1.0f);
+    LP_CHECK_CUDA(launch_next(moe_route_kernel<bf16>, grid, dim3(route_threads(T, E)), 0, stream, reinterpret_cast<const bf16*>(h), ldh, T, D,
+        reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, 1, 1, top, nullptr, idx_out, w_out, nullptr, 1, logit_bias, 1.0f));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
@@ -284,11 +290,11 @@ extern "C" int lp_moe_route_sigmoid(const void* h, long long ldh, int h_fp32, in
   if (T <= 0) return 0;
   const unsigned grid = (unsigned)T;
   if (h_fp32)
-    moe_route_kernel<float><<<grid, route_threads(T, E), 0, stream>>>(reinterpret_cast<const float*>(h), ldh, T, D,
-        reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, 1, 1, top, nullptr, idx_out, w_out, nullptr, 2, nullptr, 1.0f);
+    LP_CHECK_CUDA(launch_next(moe_route_kernel<float>, grid, dim3(route_threads(T, E)), 0, stream, reinterpret_cast<const float*>(h), ldh, T, D,
+        reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, 1, 1, top, nullptr, idx_out, w_out, nullptr, 2, nullptr, 1.0f));
   else
-    moe_route_kernel<bf16><<<grid, route_threads(T, E), 0, stream>>>(reinterpret_cast<const bf16*>(h), ldh, T, D,
-        reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, 1, 1, top, nullptr, idx_out, w_out, nullptr, 2, nullptr, 1.0f);
+    LP_CHECK_CUDA(launch_next(moe_route_kernel<bf16>, grid, dim3(route_threads(T, E)), 0, stream, reinterpret_cast<const bf16*>(h), ldh, T, D,
+        reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, 1, 1, top, nullptr, idx_out, w_out, nullptr, 2, nullptr, 1.0f));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
@@ -308,11 +314,11 @@ extern "C" int lp_moe_route_group_softmax(const void* h, long long ldh, int h_fp
   if (T <= 0) return 0;
   const unsigned grid = (unsigned)T;
   if (h_fp32)
-    moe_route_kernel<float><<<grid, route_threads(T, E), 0, stream>>>(reinterpret_cast<const float*>(h), ldh, T, D,
-        reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, n_groups, keep_groups, top, nullptr, idx_out, w_out, nullptr, 3, nullptr, w_scale);
+    LP_CHECK_CUDA(launch_next(moe_route_kernel<float>, grid, dim3(route_threads(T, E)), 0, stream, reinterpret_cast<const float*>(h), ldh, T, D,
+        reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, n_groups, keep_groups, top, nullptr, idx_out, w_out, nullptr, 3, nullptr, w_scale));
   else
-    moe_route_kernel<bf16><<<grid, route_threads(T, E), 0, stream>>>(reinterpret_cast<const bf16*>(h), ldh, T, D,
-        reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, n_groups, keep_groups, top, nullptr, idx_out, w_out, nullptr, 3, nullptr, w_scale);
+    LP_CHECK_CUDA(launch_next(moe_route_kernel<bf16>, grid, dim3(route_threads(T, E)), 0, stream, reinterpret_cast<const bf16*>(h), ldh, T, D,
+        reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, n_groups, keep_groups, top, nullptr, idx_out, w_out, nullptr, 3, nullptr, w_scale));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
@@ -340,7 +346,7 @@ extern "C" int lp_moe_align(const int* idx, int n_pairs, int top, int E, int til
   LP_REQUIRE(E > 0 && E <= MOE_MAX_EXPERTS && top > 0 && tile_rows > 0, "lp_moe_align: bad sizes");
   LP_REQUIRE(max_tiles >= lp_moe_max_tiles(n_pairs, E, tile_rows), "lp_moe_align: max_tiles=%d is too small for %d pairs", max_tiles, n_pairs);
   if (n_pairs <= 0) return 0;
-  moe_align_kernel<<<1, ALIGN_THREADS, 0, stream>>>(idx, n_pairs, top, E, tile_rows, max_tiles, tile_group, sorted_token, pair_row);
+  LP_CHECK_CUDA(launch_next(moe_align_kernel, dim3(1), dim3(ALIGN_THREADS), 0, stream, idx, n_pairs, top, E, tile_rows, max_tiles, tile_group, sorted_token, pair_row));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
@@ -352,7 +358,7 @@ extern "C" int lp_moe_combine(const float* y, long long ldy, const int* pair_row
   LP_REQUIRE(y != nullptr && pair_row != nullptr && out != nullptr, "lp_moe_combine: null operand");
   if (T <= 0) return 0;
   const int threads = T > MOE_FEW_TOKENS || D < 512 ? 128 : D < 1024 ? 256 : 1024;
-  moe_combine_kernel<<<T, threads, 0, stream>>>(y, ldy, pair_row, w, top, shared, lds, gate, out, ldo, T, D);
+  LP_CHECK_CUDA(launch_next(moe_combine_kernel, dim3(T), dim3(threads), 0, stream, y, ldy, pair_row, w, top, shared, lds, gate, out, ldo, T, D));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;

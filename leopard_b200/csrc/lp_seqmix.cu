@@ -144,6 +144,8 @@ __device__ __forceinline__ bool ret_copy_rows(const RetArgs& a, int row0, int le
 __global__ void __launch_bounds__(RET_CHUNK_THREADS)
 retention_chunk_state_kernel(RetArgs a, const int* __restrict__ chunk_seq, const int* __restrict__ chunk_row0, const int* __restrict__ chunk_len,
                              const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0, float* __restrict__ ws) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float dyn_smem[];
   const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
   const int s = chunk_seq[c], row0 = chunk_row0[c], len = chunk_len[c];
@@ -204,7 +206,9 @@ template <> struct alignas(16) RetVec<4> { float v[4]; };
 template <int V>
 __global__ void __launch_bounds__(SCAN_THREADS)
 retention_scan_kernel(RetArgs a, const int* __restrict__ seq_chunk0, const int* __restrict__ chunk_len, const int* __restrict__ seq_pos0,
-                      const int* __restrict__ seq_slot, float* __restrict__ ws) {
+                      const int* __restrict__ seq_slot, float* ws) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int s = blockIdx.x, h = blockIdx.y;
   const long long hs = (long long)a.dim * a.vdim;
   const long long i = ((long long)blockIdx.z * SCAN_THREADS + threadIdx.x) * V;
@@ -258,7 +262,9 @@ retention_scan_kernel(RetArgs a, const int* __restrict__ seq_chunk0, const int* 
 template <bool WIDE>
 __global__ void __launch_bounds__(RET_CHUNK_THREADS)
 retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const int* __restrict__ chunk_row0, const int* __restrict__ chunk_len,
-                           const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0, const float* __restrict__ ws, int stage_s) {
+                           const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0, const float* ws, int stage_s) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float dyn_smem[];
   const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
   const int s = chunk_seq[c], row0 = chunk_row0[c], len = chunk_len[c];
@@ -439,6 +445,8 @@ template <int V> __host__ __device__ inline int ret_dec_groups(int vdim) { retur
 template <int V>
 __global__ void __launch_bounds__(RET_DEC_THREADS)
 retention_decode_kernel(RetArgs a, const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0, const int* __restrict__ seq_slot) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float dyn_smem[];
   const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
   const int row = seq_row0[s], pos = seq_pos0[s];
@@ -551,6 +559,8 @@ constexpr int LAT_PREP_THREADS = 128, LAT_PREP_WIDE = 512;      // up to two row
 constexpr int LAT_PREP_PAIRS = 4096;      // rotation pairs whose sines and cosines shared memory holds; with more of them each is taken where it is used
 __global__ void __launch_bounds__(LAT_PREP_WIDE)
 latent_prep_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float dyn_smem[];
   __shared__ float red[LAT_PREP_WIDE / 32];
   const int r = blockIdx.x, tid = threadIdx.x;
@@ -619,8 +629,10 @@ template <> struct LatVec<1> { float v[1]; };
 template <> struct alignas(16) LatVec<4> { float v[4]; };
 template <int V, int NP, int W>
 __global__ void __launch_bounds__(W * 32)
-latent_attend_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos, const float* __restrict__ q_abs,
+latent_attend_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos, const float* q_abs,
                      long long ldqa, void* __restrict__ out, long long ldo, int out_fp32) {
+  pdl_launch_dependents();
+  pdl_wait();
   __align__(16) __shared__ float s_acc[W][32 * V * NP];
   __shared__ float s_mx[W], s_den[W];
   constexpr int NR = V == 4 ? 1 : NP;      // pieces of the rotated part
@@ -752,8 +764,10 @@ latent_attend_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const in
 constexpr int LAT_ROW_HEADS = 4, LAT_SPLIT_ROWS = 128;
 template <int NR>
 __global__ void __launch_bounds__(LAT_ROW_HEADS * 32)
-latent_attend_rows_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos, const float* __restrict__ q_abs,
+latent_attend_rows_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos, const float* q_abs,
                           long long ldqa, void* __restrict__ out, long long ldo, int out_fp32) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int r = blockIdx.x;
   const int h = blockIdx.y * LAT_ROW_HEADS + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -1060,14 +1074,14 @@ static int launch_ret_prefill(const RetArgs& a, int n_seqs, int n_chunks, const 
   if (stage_s) smem3 += (size_t)a.dim * vdimp * sizeof(float);
   LP_CHECK_CUDA(ensure_smem(retention_chunk_state_kernel, smem1, g_smem_chunk_state));
   LP_CHECK_CUDA(ensure_smem(retention_chunk_out_kernel<WIDE>, smem3, have_out));
-  retention_chunk_state_kernel<<<dim3(n_chunks, a.heads), RET_CHUNK_THREADS, smem1, stream>>>(a, chunk_seq, chunk_row0, chunk_len, seq_row0, seq_pos0, w);
+  LP_CHECK_CUDA(launch_next(retention_chunk_state_kernel, dim3(n_chunks, a.heads), dim3(RET_CHUNK_THREADS), smem1, stream, a, chunk_seq, chunk_row0, chunk_len, seq_row0, seq_pos0, w));
   LP_CHECK_CUDA(cudaGetLastError());
   constexpr int V = WIDE ? 4 : 1;
-  retention_scan_kernel<V><<<dim3(n_seqs, a.heads, (a.dim * a.vdim / V + SCAN_THREADS - 1) / SCAN_THREADS), SCAN_THREADS, 0, stream>>>(
-      a, seq_chunk0, chunk_len, seq_pos0, seq_slot, w);
+  LP_CHECK_CUDA(launch_next(retention_scan_kernel<V>, dim3(n_seqs, a.heads, (a.dim * a.vdim / V + SCAN_THREADS - 1) / SCAN_THREADS), dim3(SCAN_THREADS), 0, stream, 
+      a, seq_chunk0, chunk_len, seq_pos0, seq_slot, w));
   LP_CHECK_CUDA(cudaGetLastError());
-  retention_chunk_out_kernel<WIDE><<<dim3(n_chunks, a.heads), RET_CHUNK_THREADS, smem3, stream>>>(a, chunk_seq, chunk_row0, chunk_len, seq_row0, seq_pos0, w,
-                                                                                                  stage_s);
+  LP_CHECK_CUDA(launch_next(retention_chunk_out_kernel<WIDE>, dim3(n_chunks, a.heads), dim3(RET_CHUNK_THREADS), smem3, stream, a, chunk_seq, chunk_row0, chunk_len, seq_row0, seq_pos0, w,
+                                                                                                  stage_s));
   LP_CHECK_CUDA(cudaGetLastError());
   note_launch(3);
   return 0;
@@ -1097,7 +1111,7 @@ static int launch_ret_decode(const RetArgs& a, int n_seqs, const int* seq_row0, 
   const size_t smem = ((size_t)2 * a.dim + 2 * a.vdim + (size_t)ret_dec_groups<V>(a.vdim) * a.vdim) * sizeof(float);
   LP_REQUIRE(smem <= 200 * 1024, "lp_retention_decode: dim=%d vdim=%d do not fit shared memory", a.dim, a.vdim);
   LP_CHECK_CUDA(ensure_smem(retention_decode_kernel<V>, smem, have));
-  retention_decode_kernel<V><<<dim3(n_seqs, a.heads), RET_DEC_THREADS, smem, stream>>>(a, seq_row0, seq_pos0, seq_slot);
+  LP_CHECK_CUDA(launch_next(retention_decode_kernel<V>, dim3(n_seqs, a.heads), dim3(RET_DEC_THREADS), smem, stream, a, seq_row0, seq_pos0, seq_slot));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
@@ -1120,7 +1134,7 @@ extern "C" int lp_latent_prep(const lp_latent_desc* d, int R, const int* row_seq
   LP_REQUIRE((d->dkv == nullptr || d->c_gain != nullptr) && row_seq != nullptr && row_pos != nullptr, "lp_latent_prep: null operand");
   if (R <= 0) return 0;
   const size_t smem = d->rot_dims / 2 <= LAT_PREP_PAIRS ? d->rot_dims / 2 * sizeof(float2) : 0;
-  latent_prep_kernel<<<R, R <= 2 * sm_count() ? LAT_PREP_WIDE : LAT_PREP_THREADS, smem, stream>>>(a, R, row_seq, row_pos);
+  LP_CHECK_CUDA(launch_next(latent_prep_kernel, dim3(R), dim3(R <= 2 * sm_count() ? LAT_PREP_WIDE : LAT_PREP_THREADS), smem, stream, a, R, row_seq, row_pos));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
@@ -1139,18 +1153,18 @@ extern "C" int lp_latent_attend(const lp_latent_desc* d, int R, const int* row_s
   if (R > LAT_SPLIT_ROWS || d->kv_rank > LAT_SPLIT_MAX_RANK || d->rot_dim > LAT_SPLIT_MAX_RANK) {      // prompts: a CTA per row, a warp per head
     const dim3 grid(R, (d->heads + LAT_ROW_HEADS - 1) / LAT_ROW_HEADS);
     const int threads = (d->heads < LAT_ROW_HEADS ? d->heads : LAT_ROW_HEADS) * 32;
-    if (nr <= 2) latent_attend_rows_kernel<2><<<grid, threads, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);
-    else if (nr <= 4) latent_attend_rows_kernel<4><<<grid, threads, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);
-    else if (nr <= 8) latent_attend_rows_kernel<8><<<grid, threads, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);
-    else if (nr <= 16) latent_attend_rows_kernel<16><<<grid, threads, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);
-    else latent_attend_rows_kernel<32><<<grid, threads, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);
+    if (nr <= 2) LP_CHECK_CUDA(launch_next(latent_attend_rows_kernel<2>, grid, dim3(threads), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32));
+    else if (nr <= 4) LP_CHECK_CUDA(launch_next(latent_attend_rows_kernel<4>, grid, dim3(threads), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32));
+    else if (nr <= 8) LP_CHECK_CUDA(launch_next(latent_attend_rows_kernel<8>, grid, dim3(threads), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32));
+    else if (nr <= 16) LP_CHECK_CUDA(launch_next(latent_attend_rows_kernel<16>, grid, dim3(threads), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32));
+    else LP_CHECK_CUDA(launch_next(latent_attend_rows_kernel<32>, grid, dim3(threads), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32));
   } else {      // decoding: a CTA per (row, head), its warps split the keys
     const long long ctas = (long long)R * d->heads;
     const bool pieces = d->kv_rank % 4 == 0 && d->rot_dim % 4 == 0 && d->rot_dim <= 128 && (reinterpret_cast<uintptr_t>(d->cache) & 15) == 0;
 #define LP_LAT(V, NP)                                                                                                                       \
   do {                                                                                                                                      \
-    if (ctas <= 2LL * sm_count()) latent_attend_kernel<V, NP, 16><<<(unsigned)ctas, 16 * 32, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);    \
-    else latent_attend_kernel<V, NP, 4><<<(unsigned)ctas, 4 * 32, 0, stream>>>(a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32);     \
+    if (ctas <= 2LL * sm_count()) LP_CHECK_CUDA((launch_next(latent_attend_kernel<V, NP, 16>, dim3((unsigned)ctas), dim3(16 * 32), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32)));    \
+    else LP_CHECK_CUDA((launch_next(latent_attend_kernel<V, NP, 4>, dim3((unsigned)ctas), dim3(4 * 32), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32)));     \
   } while (0)
     if (pieces) {
       const int np = (d->kv_rank + 127) / 128;

@@ -40,8 +40,10 @@ namespace lp {
 
 typedef __nv_bfloat16 bf16;
 
-__global__ void embed_rows_f32_kernel(const int* __restrict__ ids, int R, const bf16* __restrict__ table, long long ldt, int vocab,
+__global__ void embed_rows_f32_kernel(const int* ids, int R, const bf16* __restrict__ table, long long ldt, int vocab,
                                       float scale, float* __restrict__ out, long long ldo, int D) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int r = blockIdx.x;
   if (r >= R) return;
   int id = ids[r];
@@ -129,9 +131,11 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 }
 template <int VN>
 __global__ void __launch_bounds__(1024)
-rmsnorm_row_kernel(const float* __restrict__ x, long long ldx, int D, float gain_scalar, const float* __restrict__ gain_vec, float eps,
-                   float* __restrict__ out_f32, bf16* __restrict__ out_bf16, long long ldo, float* __restrict__ accum, long long lda,
+rmsnorm_row_kernel(const float* x, long long ldx, int D, float gain_scalar, const float* __restrict__ gain_vec, float eps,
+                   float* __restrict__ out_f32, bf16* __restrict__ out_bf16, long long ldo, float* accum, long long lda,
                    NormNext next) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[2][32];
   const long long row = blockIdx.x;
   f32vec<4> v[VN], y[VN];
@@ -224,8 +228,10 @@ __device__ __forceinline__ float glu_one(int mode, float z, float u, float a, fl
 // clamped gated unit of lp_linear on (in[m, n], in[m, n + N]) with limit a and slope b.  row_scale multiplies what is read.
 // Bound by its bytes: 4096 x 8192 fp32 -> bf16 130 us with a column a thread (and a 64-bit division each), 41 us = 4.9 TB/s with four (relu2).
 template <typename IT, typename OT, int V>
-__global__ void glu_kernel(const IT* __restrict__ in, long long ldi, OT* __restrict__ out, long long ldo, int M, int N, int mode, float a,
-                           float b, const float* __restrict__ row_scale) {
+__global__ void glu_kernel(const IT* in, long long ldi, OT* __restrict__ out, long long ldo, int M, int N, int mode, float a,
+                           float b, const float* row_scale) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int n = (int)(blockIdx.x * blockDim.x + threadIdx.x) * V;
   if (n >= N) return;
   const bool pair = mode == LP_EPI_SILU_GATE || mode == LP_EPI_GELU_GATE || mode == LP_EPI_CLAMP_GLU;
@@ -363,7 +369,9 @@ static bool vec4_ok(int N, std::initializer_list<const void*> bases, std::initia
 static dim3 rows_grid(int groups, int M) { return dim3((unsigned)((groups + 255) / 256), (unsigned)(M < 65535 ? M : 65535)); }
 
 template <int V>
-__global__ void axpy_f32_kernel(float* __restrict__ y, long long ldy, const float* __restrict__ x, long long ldx, float alpha, int M, int N) {
+__global__ void axpy_f32_kernel(float* y, long long ldy, const float* x, long long ldx, float alpha, int M, int N) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int n = (int)(blockIdx.x * blockDim.x + threadIdx.x) * V;
   if (n >= N) return;
   for (int m = blockIdx.y; m < M; m += gridDim.y) {
@@ -996,7 +1004,7 @@ extern "C" int lp_embed_rows_f32(const int* ids, int R, const void* table, long 
   if (R == 0) return 0;
   // four columns a thread: as many threads as a row has work for (2048 rows of 512 columns: 512 threads 4.7 us, 128 3.7)
   const int threads = D >= 2048 ? 512 : D > 512 ? 256 : 128;
-  embed_rows_f32_kernel<<<R, threads, 0, stream>>>(ids, R, reinterpret_cast<const bf16*>(table), ldt, vocab, scale, out, ldo, D);
+  LP_CHECK_CUDA(launch_next(embed_rows_f32_kernel, dim3(R), dim3(threads), 0, stream, ids, R, reinterpret_cast<const bf16*>(table), ldt, vocab, scale, out, ldo, D));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
@@ -1013,9 +1021,9 @@ static int launch_rmsnorm(const float* x, long long ldx, int M, int D, float gai
     // 2048 3.1, 3.5, 592 4.1, 4.0, 1024 5.8, 4.9, 4096 16.4, 13.8; 592 rows of 1024 3.3, 3.7, of 4096 6.3, 5.0)
     const int groups = D / 4;
     if (groups <= 1024 && M <= 4 * sm_count())
-      rmsnorm_row_kernel<1><<<M, (groups + 31) / 32 * 32, 0, stream>>>(x, ldx, D, gain_scalar, gain_vec, eps, of, ob, ldo, accum, ld_accum, next);
+      LP_CHECK_CUDA(launch_next(rmsnorm_row_kernel<1>, dim3(M), dim3((groups + 31) / 32 * 32), 0, stream, x, ldx, D, gain_scalar, gain_vec, eps, of, ob, ldo, accum, ld_accum, next));
     else
-      rmsnorm_row_kernel<2><<<M, (groups + 63) / 64 * 32, 0, stream>>>(x, ldx, D, gain_scalar, gain_vec, eps, of, ob, ldo, accum, ld_accum, next);
+      LP_CHECK_CUDA(launch_next(rmsnorm_row_kernel<2>, dim3(M), dim3((groups + 63) / 64 * 32), 0, stream, x, ldx, D, gain_scalar, gain_vec, eps, of, ob, ldo, accum, ld_accum, next));
     note_launch();
     LP_CHECK_CUDA(cudaGetLastError());
     return 0;
@@ -1069,8 +1077,8 @@ extern "C" int lp_glu_scaled_f32(const void* in, long long ldi, int in_fp32, voi
   const dim3 grid = rows_grid(v4 ? N / 4 : N, M);
 #define LP_GLU(IT, OT)                                                                                                                        \
   do {                                                                                                                                        \
-    if (v4) glu_kernel<IT, OT, 4><<<grid, 256, 0, stream>>>(reinterpret_cast<const IT*>(in), ldi, reinterpret_cast<OT*>(out), ldo, M, N, mode, a, b, row_scale); \
-    else glu_kernel<IT, OT, 1><<<grid, 256, 0, stream>>>(reinterpret_cast<const IT*>(in), ldi, reinterpret_cast<OT*>(out), ldo, M, N, mode, a, b, row_scale);    \
+    if (v4) LP_CHECK_CUDA((launch_next(glu_kernel<IT, OT, 4>, grid, dim3(256), 0, stream, reinterpret_cast<const IT*>(in), ldi, reinterpret_cast<OT*>(out), ldo, M, N, mode, a, b, row_scale))); \
+    else LP_CHECK_CUDA((launch_next(glu_kernel<IT, OT, 1>, grid, dim3(256), 0, stream, reinterpret_cast<const IT*>(in), ldi, reinterpret_cast<OT*>(out), ldo, M, N, mode, a, b, row_scale)));    \
   } while (0)
   if (in_fp32 && out_fp32) LP_GLU(float, float);
   else if (in_fp32) LP_GLU(float, bf16);
@@ -1165,8 +1173,8 @@ extern "C" int lp_axpy_f32(float* y, long long ldy, const float* x, long long ld
   if (M == 0) return 0;
   const bool v4 = vec4_ok(N, {y, x}, {ldy, ldx});
   const dim3 grid = rows_grid(v4 ? N / 4 : N, M);
-  if (v4) axpy_f32_kernel<4><<<grid, 256, 0, stream>>>(y, ldy, x, ldx, alpha, M, N);
-  else axpy_f32_kernel<1><<<grid, 256, 0, stream>>>(y, ldy, x, ldx, alpha, M, N);
+  if (v4) LP_CHECK_CUDA(launch_next(axpy_f32_kernel<4>, grid, dim3(256), 0, stream, y, ldy, x, ldx, alpha, M, N));
+  else LP_CHECK_CUDA(launch_next(axpy_f32_kernel<1>, grid, dim3(256), 0, stream, y, ldy, x, ldx, alpha, M, N));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;

@@ -146,6 +146,8 @@ __device__ __forceinline__ const float* win_visible_row(const WinArgs& a, const 
 constexpr int WIN_PREP_THREADS = 128, WIN_PREP_WIDE = 1024;      // few rows (decoding) take the wide CTA
 __global__ void __launch_bounds__(WIN_PREP_WIDE)
 window_attn_prep_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float dyn_smem[];
   float* s_ss = dyn_smem;      // [heads + kv_heads] sums of squares, then the two totals
   const int r = blockIdx.x;
@@ -285,6 +287,8 @@ window_attn_prep_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const
 constexpr int WIN_POOL_THREADS = 128;
 __global__ void __launch_bounds__(WIN_POOL_THREADS)
 window_attn_pool_kernel(WinArgs a, int n_seqs, const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int s = blockIdx.x;
   if (s >= n_seqs) return;
   const int pos0 = seq_pos0[s], len = seq_row0[s + 1] - seq_row0[s];
@@ -302,6 +306,8 @@ template <int QH, int NV, bool DIST, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 window_attn_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos, void* __restrict__ out, long long ldo,
                    int out_fp32) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float dyn_smem[];
   const int r = blockIdx.x;
   if (r >= R) return;
@@ -1514,11 +1520,11 @@ static int launch_window_attn(const WinArgs& a, int R, const int* row_seq, const
   do {                                                                                                                                         \
     if constexpr (QH == 1) {                                                                                                                   \
       if (wide) {                                                                                                                              \
-        window_attn_kernel<QH, NV, DIST, 1024><<<grid, warps * 32, smem, stream>>>(a, R, row_seq, row_pos, out, ldo, out_fp32);               \
+        LP_CHECK_CUDA((launch_next(window_attn_kernel<QH, NV, DIST, 1024>, grid, dim3(warps * 32), smem, stream, a, R, row_seq, row_pos, out, ldo, out_fp32)));               \
         break;                                                                                                                                 \
       }                                                                                                                                        \
     }                                                                                                                                          \
-    window_attn_kernel<QH, NV, DIST, 256><<<grid, warps * 32, smem, stream>>>(a, R, row_seq, row_pos, out, ldo, out_fp32);                    \
+    LP_CHECK_CUDA((launch_next(window_attn_kernel<QH, NV, DIST, 256>, grid, dim3(warps * 32), smem, stream, a, R, row_seq, row_pos, out, ldo, out_fp32)));                    \
   } while (0)
   if (nv <= 1) LP_WAK(1);
   else if (nv <= 2) LP_WAK(2);
@@ -1594,7 +1600,7 @@ extern "C" int lp_window_attn_prep(const lp_window_attn_desc* d, int R, const in
   LP_REQUIRE(smem <= 48 * 1024, "lp_window_attn_prep: too many heads");
   // one row is a CTA: with few rows it should not walk its elements 128 at a time
   const int wide = d->heads * d->dim >= WIN_PREP_WIDE ? WIN_PREP_WIDE : 256;
-  window_attn_prep_kernel<<<R, R <= WIN_PREP_ROWS ? wide : WIN_PREP_THREADS, smem, stream>>>(a, R, row_seq, row_pos);
+  LP_CHECK_CUDA(launch_next(window_attn_prep_kernel, dim3(R), dim3(R <= WIN_PREP_ROWS ? wide : WIN_PREP_THREADS), smem, stream, a, R, row_seq, row_pos));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
@@ -1609,8 +1615,8 @@ extern "C" int lp_window_attn_pool(const lp_window_attn_desc* d, int n_seqs, con
   if (n_seqs <= 0 || max_new_blocks <= 0) return 0;
   LP_REQUIRE(max_new_blocks <= 65535, "lp_window_attn_pool: %d blocks per request in one step", max_new_blocks);
   const int roww = a.roww;
-  window_attn_pool_kernel<<<dim3(n_seqs, max_new_blocks, (roww + WIN_POOL_THREADS - 1) / WIN_POOL_THREADS), WIN_POOL_THREADS, 0, stream>>>(
-      a, n_seqs, seq_row0, seq_pos0);
+  LP_CHECK_CUDA(launch_next(window_attn_pool_kernel, dim3(n_seqs, max_new_blocks, (roww + WIN_POOL_THREADS - 1) / WIN_POOL_THREADS), dim3(WIN_POOL_THREADS), 0, stream, 
+      a, n_seqs, seq_row0, seq_pos0));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;

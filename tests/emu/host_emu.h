@@ -97,6 +97,11 @@ inline void set_error(const char* fmt, ...) {
 inline void note_launch(int = 1) {}
 inline void pdl_wait() {}
 inline void pdl_launch_dependents() {}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_next(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t, cudaStream_t, Args... args) {
+  emu::launch(grid, block, [&] { kern(static_cast<KArgs>(args)...); });
+  return cudaSuccess;
+}
 inline int g_emu_sms = 4;      // emu_set_sm_count: rules that count CTAs per SM
 inline int sm_count() { return g_emu_sms; }
 inline float2 fma2(float2 a, float2 b, float2 c) { return {std::fma(a.x, b.x, c.x), std::fma(a.y, b.y, c.y)}; }
@@ -139,6 +144,61 @@ inline void cut3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
 }
 inline bool not_finite(float v) { return !std::isfinite(v); }
 inline uint32_t smem_u32(const void* p) { return (uint32_t)(uintptr_t)p; }
+#ifdef EMU_FIBERS
+#define __grid_constant__
+// mbarriers (an arrival count, bytes that are still to come, a phase) and bulk copies, which complete at once
+struct EmuMbar { int16_t pending; uint8_t count, phase; int32_t bytes; };
+static_assert(sizeof(EmuMbar) == sizeof(uint64_t));
+inline EmuMbar& emu_mbar(uint64_t* b) { return *reinterpret_cast<EmuMbar*>(b); }
+inline void emu_mbar_turn(EmuMbar& m) {
+  ++emu::g_sched->progress;
+  if (m.pending < 0) { std::fprintf(stderr, "emu: mbarrier over-arrival\n"); std::abort(); }
+  if (m.pending > 0 || m.bytes != 0) return;
+  m.pending = m.count;
+  m.phase ^= 1;
+}
+inline void mbar_init(uint64_t* b, uint32_t count) { emu_mbar(b) = {(int16_t)count, (uint8_t)count, 0, 0}; }
+inline void fence_barrier_init() {}
+inline void mbar_arrive(uint64_t* b) { --emu_mbar(b).pending; emu_mbar_turn(emu_mbar(b)); }
+inline void mbar_arrive_expect_tx(uint64_t* b, uint32_t bytes) { emu_mbar(b).bytes += (int32_t)bytes; mbar_arrive(b); }
+inline void mbar_wait(uint64_t* b, uint32_t parity) { while (emu_mbar(b).phase == parity) emu::give_way(); }
+inline void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* b) {
+  if (((uintptr_t)src & 15) || ((uintptr_t)dst & 15) || bytes % 16) { std::fprintf(stderr, "emu: bulk copy off 16-byte boundaries\n"); std::abort(); }
+  std::memcpy(dst, src, bytes);
+  emu_mbar(b).bytes -= (int32_t)bytes;
+  emu_mbar_turn(emu_mbar(b));
+}
+// tiled copies of bf16 boxes with the 128-byte swizzle: 16-byte pieces of each 128-byte line are exchanged by its number in the box
+struct CUtensorMap { const uint8_t* base; uint64_t dims[4], strides[4]; uint32_t box[4]; };
+inline int make_tmap_bf16_4d(CUtensorMap* m, const void* base, const uint64_t* dims, const uint64_t* strides, const uint32_t* box) {
+  m->base = (const uint8_t*)base;
+  for (int i = 0; i < 4; ++i) {
+    m->dims[i] = dims[i];
+    m->box[i] = box[i];
+    m->strides[i] = i == 0 ? 2 : strides[i - 1] * 2;
+    if (i > 0 && m->strides[i] % 16) { set_error("tensor map stride"); return -1; }
+  }
+  return 0;
+}
+inline void tma_load_4d(void* dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2, int c3) {
+  if ((uintptr_t)dst % 1024 || m->box[0] != 64 || c0 % 8) { std::fprintf(stderr, "emu: box off its boundary\n"); std::abort(); }
+  const int64_t c[4] = {c0, c1, c2, c3};
+  uint32_t line = 0;
+  for (uint32_t i3 = 0; i3 < m->box[3]; ++i3)
+    for (uint32_t i2 = 0; i2 < m->box[2]; ++i2)
+      for (uint32_t i1 = 0; i1 < m->box[1]; ++i1, ++line)
+        for (uint32_t p = 0; p < 8; ++p) {
+          uint8_t* to = (uint8_t*)dst + line * 128 + ((p ^ (line & 7)) * 16);
+          const bool in = c[0] + p * 8 < (int64_t)m->dims[0] && c[1] + i1 < (int64_t)m->dims[1] && c[2] + i2 < (int64_t)m->dims[2] && c[3] + i3 < (int64_t)m->dims[3];
+          if (in) std::memcpy(to, m->base + (c[0] + p * 8) * 2 + (c[1] + i1) * m->strides[1] + (c[2] + i2) * m->strides[2] + (c[3] + i3) * m->strides[3], 16);
+          else std::memset(to, 0, 16);
+        }
+  emu_mbar(bar).bytes -= (int32_t)(line * 128);
+  emu_mbar_turn(emu_mbar(bar));
+}
+inline uint64_t read_once_policy() { return 0; }
+inline void tma_load_4d_once(void* dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2, int c3, uint64_t) { tma_load_4d(dst, m, bar, c0, c1, c2, c3); }
+#endif
 struct ProfScope { ProfScope(int, int, int, int, cudaStream_t) {} };
 }  // namespace lp
 

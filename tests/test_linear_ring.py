@@ -1,0 +1,102 @@
+"""The product of up to 16 rows as one stream of weights through a ring of TMA pieces (lp_linear, lp_linear_group_pairs with K a multiple of 64) against a
+float64 product: pieces that end within K, tiles that end within N, more tiles than CTAs and more pieces than the ring has places, both operand types, batches,
+segments, gated units, groups whose pairs fill several tiles; weights that may be read early and weights that may not.
+
+Error bounds: as for the weight-streaming kernel, products are exact and K / 16 fp32 sums follow, less than 2e-6 of the result's size for K <= 1600."""
+import ctypes as C
+
+import pytest
+import torch
+
+from leopard_b200 import _lib
+from seqlm_common import backend, emu_lib, rel_err  # noqa: F401
+from test_linear_stream import _call, _data
+
+F32, BF16 = torch.float32, torch.bfloat16
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 64), (1, 200, 1088), (3, 40, 576), (5, 130, 512), (8, 16, 1600), (8, 300, 64), (9, 33, 640), (16, 130, 448)])
+@pytest.mark.parametrize("constant", [0, 1])
+def test_rows_tiles_and_pieces(backend, dtype, M, N, K, constant):
+    a, w, want, ad, wd = _data(M, N, K, dtype, backend[0])
+    out = torch.empty(M, N, device=backend[0])
+    _call(backend, ad, wd, out, M, w_constant=constant)
+    assert rel_err(out, want) < 2e-6
+    again = torch.empty(M, N, device=backend[0])
+    _call(backend, ad, wd, again, M, w_constant=1 - constant)
+    assert torch.equal(out, again)
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("M", [3, 12])
+def test_gated_and_added(backend, dtype, M):
+    N, K = 76, 704
+    a, w, z, ad, wd = _data(M, N, K, dtype, backend[0])
+    half = torch.empty(M, N // 2, device=backend[0])
+    _call(backend, ad, wd, half, M, epi=_lib.EPI_SILU_GATE, w_constant=1)
+    p, q = z[:, : N // 2], z[:, N // 2:]
+    assert rel_err(half, p * torch.sigmoid(p) * q) < 5e-6      # the unit's slope is below 1.1, its factors carry one error each
+    g = torch.Generator().manual_seed(1)
+    bias, scale, gate, x = torch.randn(N, generator=g), torch.rand(M, generator=g), torch.randn(M, N, generator=g), torch.randn(M, N, generator=g)
+    out = x.clone().to(backend[0])
+    _call(backend, ad, wd, out, M, bias=bias.to(backend[0]), row_scale=scale.to(backend[0]), gate=gate.to(backend[0]), ldg=N, epi=_lib.EPI_RELU2,
+          c_accum=1, c_scale=0.5, w_constant=1)
+    v = torch.relu(z * scale.double()[:, None] + bias.double()) ** 2 * torch.sigmoid(gate.double())
+    assert rel_err(out, x.double() + 0.5 * v) < 2e-6
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("M", [2, 11])
+def test_batches_and_segments(backend, dtype, M):
+    g = torch.Generator().manual_seed(M)
+    heads, N, K = 5, 40, 576
+    a, w = torch.randn(M, heads * (K + 8), generator=g).to(dtype), torch.randn(heads, N, K, generator=g).to(BF16)
+    ad, wd = a.to(backend[0]), w.to(backend[0])
+    out = torch.empty(M, heads * N, device=backend[0])
+    _call(backend, ad, wd, out, M, batch=heads, a_batch=K + 8, c_batch=N, w_constant=1)
+    want = torch.cat([a[:, h * (K + 8): h * (K + 8) + K].double() @ w[h].double().T for h in range(heads)], 1)
+    assert rel_err(out, want) < 2e-6
+    _call(backend, ad, wd, out, M, batch=heads, a_batch=0, c_batch=N, w_constant=1)      # one operand for all problems: not a tensor map's stride
+    want = torch.cat([a[:, :K].double() @ w[h].double().T for h in range(heads)], 1)
+    assert rel_err(out, want) < 2e-6
+    segs, seg, N = 3, 64, 200
+    a, w = torch.randn(segs, M, K, generator=g).to(dtype), torch.randn(N, K, generator=g).to(BF16)
+    ad, wd = a.to(backend[0]), w.to(backend[0])
+    out = torch.empty(M, N, device=backend[0])
+    _call(backend, ad, wd, out, M, seg_cols=seg, n_segs=segs, a_seg=M * K, w_constant=1)
+    which = [min(n // seg, segs - 1) for n in range(N)]
+    want = torch.stack([a[i].double() @ w[n].double() for n, i in enumerate(which)], 1)
+    assert rel_err(out, want) < 2e-6
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("n_pairs,groups,a_div", [(1, 4, 1), (10, 3, 2), (37, 9, 1), (64, 33, 4), (70, 200, 2)])
+def test_pairs(backend, dtype, n_pairs, groups, a_div):
+    g = torch.Generator().manual_seed(n_pairs)
+    N, K = 44, 1088
+    a, w = torch.randn((n_pairs + a_div - 1) // a_div, K, generator=g).to(dtype), torch.randn(groups, N, K, generator=g).to(BF16)
+    of = torch.randint(0, groups, (n_pairs,), generator=g)
+    of[: n_pairs // 2] = groups - 1      # more than a tile's rows in one group, groups without pairs
+    ad, wd = a.to(backend[0]), w.to(backend[0])
+    out = torch.full((n_pairs, N), 7.0, device=backend[0])
+    _call(backend, ad, wd, out, 1, pairs=of.to(torch.int32).to(backend[0]), groups=groups, a_div=a_div, w_constant=1)
+    want = torch.stack([a[z // a_div].double() @ w[int(of[z])].double().T for z in range(n_pairs)])
+    assert rel_err(out, want) < 2e-6
+
+
+def test_numbers_that_are_not_finite(backend):
+    """an fp32 row with an infinity: its products are those of the uncut number; rows and columns beside it keep theirs"""
+    M, N, K = 5, 40, 640
+    a, w, want, ad, wd = _data(M, N, K, F32, "cpu")
+    a = a.clone()
+    a[2, 600] = float("inf")
+    a[4, 3] = float("nan")
+    w[7, 600] = 0.0
+    want = a.double() @ w.double().T
+    out = torch.empty(M, N, device=backend[0])
+    _call(backend, a.to(backend[0]), w.to(backend[0]), out, M, w_constant=1)
+    out = out.cpu().double()
+    fine = torch.isfinite(want)
+    assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(out[torch.isinf(want)], want[torch.isinf(want)])
+    assert rel_err(out[fine], want[fine]) < 2e-6
