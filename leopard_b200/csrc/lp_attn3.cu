@@ -220,7 +220,8 @@ attn3_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const AttnArgs args)
     // ------------------------------------------------------------------ MMA issuer of tile q
     const int q = warp - 1;
     const int n_q = q ? nB : nA;
-    if (lane == 0 && n_q > 0) {
+    if (n_q > 0) {
+      const bool issue = elect_one();
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64, 0, 0);
       constexpr uint32_t idesc_o = umma_idesc_bf16(128, DH, 0, 1);
       const uint32_t q_addr = smem_u32(smem + Q_OFF + q * HEAD_BYTES);
@@ -229,55 +230,59 @@ attn3_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const AttnArgs args)
       int t_pv = 0;  // P·V halves issued so far
       auto issue_S = [&](int j, int h) {  // S_q(j).h = Q_q K_j[64h .. 64h+63]^T
         const uint32_t k_addr = smem_u32(smem + K_OFF + (j & 1) * HEAD_BYTES) + (uint32_t)h * 64 * 128;
+        if (issue) {
 #pragma unroll
-        for (int ks = 0; ks < KS_QK; ++ks) {
-          const uint32_t off = (ks >> 2) * A3_BOX + (ks & 3) * 32;
-          umma_ss(s_tm + (uint32_t)h * 64, umma_desc_sw128(q_addr + off, 0, 1024),
-                  umma_desc_sw128(k_addr + off, 0, 1024), idesc_s, ks > 0 ? 1u : 0u);
+          for (int ks = 0; ks < KS_QK; ++ks) {
+            const uint32_t off = (ks >> 2) * A3_BOX + (ks & 3) * 32;
+            umma_ss(s_tm + (uint32_t)h * 64, umma_desc_sw128(q_addr + off, 0, 1024),
+                    umma_desc_sw128(k_addr + off, 0, 1024), idesc_s, ks > 0 ? 1u : 0u);
+          }
+          umma_commit(&s_full[q * 2 + h]);
         }
-        umma_commit(&s_full[q * 2 + h]);
         A3_TRACE(14 + h);
       };
       auto issue_PV = [&](int j, int h) {  // O_q += P_q(j).h V_j[64h .. 64h+63]
         const uint32_t v_addr = smem_u32(smem + V_OFF + (j & 1) * HEAD_BYTES);
         A3_TRACE(10 + h);
-        mbar_wait(&p_full[q * 2 + h], j & 1);
+        mbar_wait_warp(&p_full[q * 2 + h], j & 1);
         A3_TRACE(12 + h);
         tc_fence_after();
+        if (issue) {
 #pragma unroll
-        for (int k4 = 0; k4 < 4; ++k4) {
-          const int ks = h * 4 + k4;
-          const uint64_t vdesc = umma_desc_sw128(v_addr + ks * 2048, A3_BOX, 1024);
-          umma_ts(d_o, s_tm + (uint32_t)h * 64 + k4 * 8, vdesc, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
+          for (int k4 = 0; k4 < 4; ++k4) {
+            const int ks = h * 4 + k4;
+            const uint64_t vdesc = umma_desc_sw128(v_addr + ks * 2048, A3_BOX, 1024);
+            umma_ts(d_o, s_tm + (uint32_t)h * 64 + k4 * 8, vdesc, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
+          }
+          umma_commit(&pv_done[q * 2 + (t_pv & 1)]);
         }
-        umma_commit(&pv_done[q * 2 + (t_pv & 1)]);
         ++t_pv;
       };
-      mbar_wait(&q_full[q], 0);
-      mbar_wait(&k_full[0], 0);
+      mbar_wait_warp(&q_full[q], 0);
+      mbar_wait_warp(&k_full[0], 0);
       tc_fence_after();
       issue_S(0, 0);
       const bool hi0 = 64 < T;
       if (hi0) issue_S(0, 1);
-      umma_commit(&k_empty[q * 2 + 0]);
+      if (issue) umma_commit(&k_empty[q * 2 + 0]);
       for (int j = 0; j < n_q; ++j) {
         const bool hi = j * 128 + 64 < T;            // second half of this tile holds real keys
         const bool more = j + 1 < n_q;
         const bool hi_next = more && ((j + 1) * 128 + 64 < T);
-        mbar_wait(&v_full[j & 1], (j >> 1) & 1);
+        mbar_wait_warp(&v_full[j & 1], (j >> 1) & 1);
         issue_PV(j, 0);
         if (more) {
-          mbar_wait(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1);
+          mbar_wait_warp(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1);
           tc_fence_after();
           issue_S(j + 1, 0);
         }
         if (hi) issue_PV(j, 1);
-        umma_commit(&v_empty[q * 2 + (j & 1)]);
+        if (issue) umma_commit(&v_empty[q * 2 + (j & 1)]);
         if (more) {
           if (hi_next) issue_S(j + 1, 1);
-          umma_commit(&k_empty[q * 2 + ((j + 1) & 1)]);
+          if (issue) umma_commit(&k_empty[q * 2 + ((j + 1) & 1)]);
         }
-        if (!more) umma_commit(&o_done[q]);
+        if (!more && issue) umma_commit(&o_done[q]);
       }
     }
   } else if (warp >= 4) {

@@ -170,7 +170,8 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const AttnArgs args,
   } else if (warp == 1 || warp == 2) {
     // ------------------------------------------------------------------ MMA issuer of tile q
     const int q = warp - 1;
-    if (lane == 0) {
+    {
+      const bool issue = elect_one();
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64, 0, 0);
       constexpr uint32_t idesc_o = umma_idesc_bf16(128, DH, 0, 1);
       const uint32_t q_addr = smem_u32(smem + Q_OFF + q * HEAD_BYTES);
@@ -183,59 +184,63 @@ attn5_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const AttnArgs args,
         const int c_lo = it_n * n_total, c_hi = it_n * n_hi;   // completed phases of the lo / hi barriers before this item
         auto issue_S = [&](int j, int h) {  // S_q(j).h = Q_q K_j[64h .. 64h+63]^T
           const uint32_t k_addr = smem_u32(smem + K_OFF + ((g0 + j) & 1) * HEAD_BYTES) + (uint32_t)h * 64 * 128;
+          if (issue) {
 #pragma unroll
-          for (int ks = 0; ks < KS_QK; ++ks) {
-            const uint32_t off = (ks >> 2) * A5_BOX + (ks & 3) * 32;
-            umma_ss(s_tm + (uint32_t)h * 64, umma_desc_sw128(q_addr + off, 0, 1024),
-                    umma_desc_sw128(k_addr + off, 0, 1024), idesc_s, ks > 0 ? 1u : 0u);
+            for (int ks = 0; ks < KS_QK; ++ks) {
+              const uint32_t off = (ks >> 2) * A5_BOX + (ks & 3) * 32;
+              umma_ss(s_tm + (uint32_t)h * 64, umma_desc_sw128(q_addr + off, 0, 1024),
+                      umma_desc_sw128(k_addr + off, 0, 1024), idesc_s, ks > 0 ? 1u : 0u);
+            }
+            umma_commit(&s_full[q * 2 + h]);
           }
-          umma_commit(&s_full[q * 2 + h]);
         };
         auto issue_PV = [&](int j, int h) {  // O_q += P_q(j).h V_j[64h .. 64h+63]
           const uint32_t v_addr = smem_u32(smem + V_OFF + ((g0 + j) & 1) * HEAD_BYTES);
-          mbar_wait(&p_full[q * 2 + h], ((h ? c_hi : c_lo) + j) & 1);
+          mbar_wait_warp(&p_full[q * 2 + h], ((h ? c_hi : c_lo) + j) & 1);
           tc_fence_after();
+          if (issue) {
 #pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4) {
-            const int ks = h * 4 + k4;
-            const uint64_t vdesc = umma_desc_sw128(v_addr + ks * 2048, A5_BOX, 1024);
-            umma_ts(d_o, s_tm + (uint32_t)h * 64 + k4 * 8, vdesc, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
+            for (int k4 = 0; k4 < 4; ++k4) {
+              const int ks = h * 4 + k4;
+              const uint64_t vdesc = umma_desc_sw128(v_addr + ks * 2048, A5_BOX, 1024);
+              umma_ts(d_o, s_tm + (uint32_t)h * 64 + k4 * 8, vdesc, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
+            }
+            umma_commit(&pv_done[q * 2 + (t_pv & 1)]);
           }
-          umma_commit(&pv_done[q * 2 + (t_pv & 1)]);
           ++t_pv;
         };
-        mbar_wait(&q_full[q], it_n & 1);
-        mbar_wait(&k_full[g0 & 1], (g0 >> 1) & 1);
+        mbar_wait_warp(&q_full[q], it_n & 1);
+        mbar_wait_warp(&k_full[g0 & 1], (g0 >> 1) & 1);
         tc_fence_after();
         issue_S(0, 0);
         if (0 < n_hi) issue_S(0, 1);
-        umma_commit(&k_empty[q * 2 + (g0 & 1)]);
-        if (n_total == 1) umma_commit(&q_empty[q]);
+        if (issue) umma_commit(&k_empty[q * 2 + (g0 & 1)]);
+        if (n_total == 1 && issue) umma_commit(&q_empty[q]);
         for (int j = 0; j < n_total; ++j) {
           const bool hi = j < n_hi;                  // second half of this tile holds real keys
           const bool more = j + 1 < n_total;
           const bool hi_next = more && (j + 1 < n_hi);
           const int g = g0 + j;
-          mbar_wait(&v_full[g & 1], (g >> 1) & 1);
+          mbar_wait_warp(&v_full[g & 1], (g >> 1) & 1);
           if (j == 0 && it_n > 0) {
             // the first P·V of an item overwrites O: the softmax warpgroup must have read the previous item's result
-            mbar_wait(&o_free[q], (it_n - 1) & 1);
+            mbar_wait_warp(&o_free[q], (it_n - 1) & 1);
             tc_fence_after();
           }
           issue_PV(j, 0);
           if (more) {
-            mbar_wait(&k_full[(g + 1) & 1], ((g + 1) >> 1) & 1);
+            mbar_wait_warp(&k_full[(g + 1) & 1], ((g + 1) >> 1) & 1);
             tc_fence_after();
             issue_S(j + 1, 0);
           }
           if (hi) issue_PV(j, 1);
-          umma_commit(&v_empty[q * 2 + (g & 1)]);
+          if (issue) umma_commit(&v_empty[q * 2 + (g & 1)]);
           if (more) {
             if (hi_next) issue_S(j + 1, 1);
-            umma_commit(&k_empty[q * 2 + ((g + 1) & 1)]);
-            if (j + 2 == n_total) umma_commit(&q_empty[q]);  // the item's last S MMAs are in flight: Q may be replaced once they retire
+            if (issue) umma_commit(&k_empty[q * 2 + ((g + 1) & 1)]);
+            if (j + 2 == n_total && issue) umma_commit(&q_empty[q]);  // the item's last S MMAs are in flight: Q may be replaced once they retire
           }
-          if (!more) umma_commit(&o_done[q]);
+          if (!more && issue) umma_commit(&o_done[q]);
         }
       }
     }

@@ -210,42 +210,49 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    {
+      const bool issue = elect_one();
       const uint32_t q_addr = smem_u32(smem + Q_OFF), do_addr = smem_u32(smem + DO_OFF);
-      mbar_wait(q_full, 0);
+      mbar_wait_warp(q_full, 0);
       int kt = 0;
       // pass 1: S_j = Q K_j^T into the two S buffers (columns 0 and 128), for the row statistics
       for (int j = 0; j < n_kv; ++j, ++kt) {
         const int st = kt & 1;
-        mbar_wait(&k_full[st], (kt >> 1) & 1);
-        if (j >= 2) mbar_wait(&s_done[j & 1], ((j - 2) >> 1) & 1);
+        mbar_wait_warp(&k_full[st], (kt >> 1) & 1);
+        if (j >= 2) mbar_wait_warp(&s_done[j & 1], ((j - 2) >> 1) & 1);
         tc_fence_after();
-        mma_ss_kmajor<DH>(tmem_base + (uint32_t)(j & 1) * 128, q_addr, smem_u32(smem + K_OFF + st * AB_HEAD));
-        umma_commit(&k_empty[st]);
-        umma_commit(&s_full[j & 1]);
+        if (issue) {
+          mma_ss_kmajor<DH>(tmem_base + (uint32_t)(j & 1) * 128, q_addr, smem_u32(smem + K_OFF + st * AB_HEAD));
+          umma_commit(&k_empty[st]);
+          umma_commit(&s_full[j & 1]);
+        }
       }
       // both buffers must have been read before pass 2 reuses their columns
       for (int b = 0; b < 2; ++b) {
         const int cnt = (n_kv + 1 - b) >> 1;   // tiles that used buffer b
-        if (cnt >= 1) mbar_wait(&s_done[b], (cnt - 1) & 1);
+        if (cnt >= 1) mbar_wait_warp(&s_done[b], (cnt - 1) & 1);
       }
       tc_fence_after();
       // pass 2
       for (int j = 0; j < n_kv; ++j, ++kt) {
         const int st = kt & 1, vs = j & 1;
-        mbar_wait(&k_full[st], (kt >> 1) & 1);
-        mbar_wait(&v_full[vs], (j >> 1) & 1);
+        mbar_wait_warp(&k_full[st], (kt >> 1) & 1);
+        mbar_wait_warp(&v_full[vs], (j >> 1) & 1);
         tc_fence_after();
         const uint32_t k_addr = smem_u32(smem + K_OFF + st * AB_HEAD);
-        mma_ss_kmajor<DH>(tmem_base + TM_S, q_addr, k_addr);                                   // S_j  = Q  K_j^T
-        mma_ss_kmajor<DH>(tmem_base + TM_DP, do_addr, smem_u32(smem + V_OFF + vs * AB_HEAD));  // dP_j = dO V_j^T
-        umma_commit(sdp_full);
-        mbar_wait(ds_full, j & 1);
+        if (issue) {
+          mma_ss_kmajor<DH>(tmem_base + TM_S, q_addr, k_addr);                                   // S_j  = Q  K_j^T
+          mma_ss_kmajor<DH>(tmem_base + TM_DP, do_addr, smem_u32(smem + V_OFF + vs * AB_HEAD));  // dP_j = dO V_j^T
+          umma_commit(sdp_full);
+        }
+        mbar_wait_warp(ds_full, j & 1);
         tc_fence_after();
-        mma_ts_mnmajor<DH>(tmem_base + TM_DQ, tmem_base + TM_S, k_addr, j > 0);                // dQ += dS_j K_j
-        umma_commit(&k_empty[st]);
-        umma_commit(&v_empty[vs]);
-        umma_commit(dq_done);
+        if (issue) {
+          mma_ts_mnmajor<DH>(tmem_base + TM_DQ, tmem_base + TM_S, k_addr, j > 0);                // dQ += dS_j K_j
+          umma_commit(&k_empty[st]);
+          umma_commit(&v_empty[vs]);
+          umma_commit(dq_done);
+        }
       }
     }
   } else {
@@ -432,23 +439,28 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    {
+      const bool issue = elect_one();
       const uint32_t k_addr = smem_u32(smem + K_OFF), v_addr = smem_u32(smem + V_OFF);
-      mbar_wait(kv_full, 0);
+      mbar_wait_warp(kv_full, 0);
       for (int t = 0; t < n_steps; ++t) {
         const int st = t & 1;
-        mbar_wait(&qd_full[st], (t >> 1) & 1);
+        mbar_wait_warp(&qd_full[st], (t >> 1) & 1);
         tc_fence_after();
         const uint32_t q_addr = smem_u32(smem + Q_OFF + st * AB_HEAD), do_addr = smem_u32(smem + DO_OFF + st * AB_HEAD);
-        mma_ss_kmajor<DH>(tmem_base + TM_ST, k_addr, q_addr);      // S^T  = K  Q^T   (kv rows on the lanes)
-        mma_ss_kmajor<DH>(tmem_base + TM_DPT, v_addr, do_addr);    // dP^T = V dO^T
-        umma_commit(st_full);
-        mbar_wait(pd_full, t & 1);
+        if (issue) {
+          mma_ss_kmajor<DH>(tmem_base + TM_ST, k_addr, q_addr);      // S^T  = K  Q^T   (kv rows on the lanes)
+          mma_ss_kmajor<DH>(tmem_base + TM_DPT, v_addr, do_addr);    // dP^T = V dO^T
+          umma_commit(st_full);
+        }
+        mbar_wait_warp(pd_full, t & 1);
         tc_fence_after();
-        mma_ts_mnmajor<DH>(tmem_base + TM_DV, tmem_base + TM_ST, do_addr, t > 0);   // dV += P^T  dO
-        mma_ts_mnmajor<DH>(tmem_base + TM_DK, tmem_base + TM_DPT, q_addr, t > 0);   // dK += dS^T Q
-        umma_commit(&qd_empty[st]);
-        umma_commit(acc_done);
+        if (issue) {
+          mma_ts_mnmajor<DH>(tmem_base + TM_DV, tmem_base + TM_ST, do_addr, t > 0);   // dV += P^T  dO
+          mma_ts_mnmajor<DH>(tmem_base + TM_DK, tmem_base + TM_DPT, q_addr, t > 0);   // dK += dS^T Q
+          umma_commit(&qd_empty[st]);
+          umma_commit(acc_done);
+        }
       }
     }
   } else {

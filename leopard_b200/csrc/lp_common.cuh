@@ -34,6 +34,9 @@ __device__ __forceinline__ void sts_u4(void* p, uint4 v) {
   asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(smem_u32(p)), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
+// One lane of a converged warp.  The loops that issue MMAs run with the whole warp and only the instructions are this lane's: addresses and descriptors are then
+// known to be the same in all lanes.  As a branch of one lane the loop took 72 ns an MMA, since each operand had to be moved to the uniform registers on its
+// own: more than a 128 x 128 x 16 product itself (34 ns).
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(
@@ -107,6 +110,11 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
       __trap();
     }
   }
+}
+// ... of a warp that stays together: no lane runs ahead to let the barrier go through another phase before the others have seen this one
+__device__ __forceinline__ void mbar_wait_warp(uint64_t* bar, uint32_t parity) {
+  mbar_wait(bar, parity);
+  __syncwarp();
 }
 
 // Wait that is expected to be LONG (an epilogue warp waiting for a whole k loop): between probes the warp sleeps `ns` nanoseconds

@@ -179,7 +179,8 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && leader) {
+    if (leader) {
+      const bool issue = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       int as = 0;
@@ -192,31 +193,35 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         const uint32_t idesc = umma_idesc_bf16(BMT, (A_MN || B_MN) ? BN : min(BN, ((args.N - n_blk * BN) + 31) & ~31), A_MN ? 1 : 0,
                                                B_MN ? 1 : 0);
         G_TRACE(20);
-        mbar_wait(&tempty_bar[as], aphase ^ 1);
+        mbar_wait_warp(&tempty_bar[as], aphase ^ 1);
         G_TRACE(21);
         const bool resume = w.kind == GEMM_ITEM_END;   // the accumulator continues another unit's partial sums
-        if (resume) mbar_wait(tpre_bar, 0);
+        if (resume) mbar_wait_warp(tpre_bar, 0);
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + as * BN;
         for (int kb = w.kb0; kb < w.kb1; ++kb) {
-          mbar_wait(&full_bar[stage], phase);
+          mbar_wait_warp(&full_bar[stage], phase);
           tc_fence_after();
           const uint32_t a_addr = smem_u32(smem + stage * L::STAGE_BYTES);
           const uint64_t adesc = umma_desc_sw128(a_addr, A_MN ? 8192 : 0, 1024);
           const uint64_t bdesc = umma_desc_sw128(a_addr + L::A_BYTES, B_MN ? 8192 : 0, 1024);
           constexpr uint32_t a_step = A_MN ? 128 : 2, b_step = B_MN ? 128 : 2;   // descriptor units of 16 B per K = 16 step
+          if (issue) {
 #pragma unroll
-          for (int k = 0; k < GEMM_BK / 16; ++k) {  // +32 B per K=16 step inside the 128 B swizzle row
-            const uint32_t acc = (resume || kb > w.kb0 || k > 0) ? 1u : 0u;
-            if (CTA2) umma_ss_pair(d_tmem, adesc + a_step * k, bdesc + b_step * k, idesc, acc);
-            else umma_ss(d_tmem, adesc + a_step * k, bdesc + b_step * k, idesc, acc);
+            for (int k = 0; k < GEMM_BK / 16; ++k) {  // +32 B per K=16 step inside the 128 B swizzle row
+              const uint32_t acc = (resume || kb > w.kb0 || k > 0) ? 1u : 0u;
+              if (CTA2) umma_ss_pair(d_tmem, adesc + a_step * k, bdesc + b_step * k, idesc, acc);
+              else umma_ss(d_tmem, adesc + a_step * k, bdesc + b_step * k, idesc, acc);
+            }
+            // smem slot reusable once these MMAs retire (in both CTAs of a pair)
+            if (CTA2) umma_commit_pair(&empty_bar[stage]); else umma_commit(&empty_bar[stage]);
           }
-          // smem slot reusable once these MMAs retire (in both CTAs of a pair)
-          if (CTA2) umma_commit_pair(&empty_bar[stage]); else umma_commit(&empty_bar[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         // accumulator complete -> epilogue (of both CTAs)
-        if (CTA2) umma_commit_pair(&tfull_bar[as]); else umma_commit(&tfull_bar[as]);
+        if (issue) {
+          if (CTA2) umma_commit_pair(&tfull_bar[as]); else umma_commit(&tfull_bar[as]);
+        }
         G_TRACE(22);
         as ^= 1;
         if (as == 0) aphase ^= 1;

@@ -117,7 +117,8 @@ gemm_chain_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constan
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA)
-    if (lane == 0 && leader) {
+    if (leader) {
+      const bool issue = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       int as = 0;
@@ -126,21 +127,23 @@ gemm_chain_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constan
         int layer, m_blk, n_blk;
         coords(t, layer, m_blk, n_blk);
         const uint32_t idesc = umma_idesc_bf16(BMT, min(BN, ((args.N[layer] - n_blk * BN) + 31) & ~31), 0, 0);
-        mbar_wait(&tempty_bar[as], aphase ^ 1);
+        mbar_wait_warp(&tempty_bar[as], aphase ^ 1);
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + as * BN;
         for (int kb = 0; kb < args.num_k_blk[layer]; ++kb) {
-          mbar_wait(&full_bar[stage], phase);
+          mbar_wait_warp(&full_bar[stage], phase);
           tc_fence_after();
           const uint32_t a_addr = smem_u32(smem + stage * L::STAGE_BYTES);
           const uint64_t adesc = umma_desc_sw128(a_addr, 0, 1024);
           const uint64_t bdesc = umma_desc_sw128(a_addr + L::A_BYTES, 0, 1024);
+          if (issue) {
 #pragma unroll
-          for (int k = 0; k < GEMM_BK / 16; ++k) umma_ss_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
-          umma_commit_pair(&empty_bar[stage]);
+            for (int k = 0; k < GEMM_BK / 16; ++k) umma_ss_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+            umma_commit_pair(&empty_bar[stage]);
+          }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-        umma_commit_pair(&tfull_bar[as]);
+        if (issue) umma_commit_pair(&tfull_bar[as]);
         as ^= 1;
         if (as == 0) aphase ^= 1;
       }

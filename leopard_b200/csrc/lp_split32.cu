@@ -25,6 +25,7 @@ constexpr int S32_FEW = 104, S32_MANY = 200;
 
 #ifdef LP_EMULATE
 inline void s32_wait(uint64_t* bar, uint32_t parity) { mbar_wait(bar, parity); }
+inline void s32_wait_warp(uint64_t* bar, uint32_t parity) { mbar_wait_warp(bar, parity); }
 inline void s32_bar(int id, int n) { named_bar(id, n, true); }
 inline float s32_ex2(float x) { return exp2f(x); }
 inline uint32_t __byte_perm(uint32_t a, uint32_t b, uint32_t) { return (a >> 16) | (b & 0xffff0000u); }
@@ -33,12 +34,16 @@ template <int N> inline void s32_fewer_regs() { emu_registers = N; }
 inline void s32_serial() { emu_serial(); }
 #else
 __device__ __forceinline__ void s32_serial() {}      // where results are taken again one by one: the emulated build looks at what the CTA is about then
-// as mbar_wait, without its message: a call in the loop of the one thread that issues the MMAs costs it registers, and its spills the tensor cores' time
+// as mbar_wait, without its message: a call in the loop of the warp that issues the MMAs costs it registers, and its spills the tensor cores' time
 __device__ __forceinline__ void s32_wait(uint64_t* bar, uint32_t parity) {
   if (mbar_try_wait(bar, parity)) return;
   const long long t0 = clock64();
   while (!mbar_try_wait(bar, parity))
     if (clock64() - t0 > LP_WATCHDOG_CYCLES) __trap();
+}
+__device__ __forceinline__ void s32_wait_warp(uint64_t* bar, uint32_t parity) {      // as mbar_wait_warp
+  s32_wait(bar, parity);
+  __syncwarp();
 }
 __device__ __forceinline__ float s32_ex2(float x) {
   float y;
@@ -318,7 +323,8 @@ gemm32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
         }
       }
     } else if (warp == 1) {
-      if (lane == 0) {
+      {
+        const bool issue = elect_one();
         constexpr uint32_t idesc = umma_idesc_bf16(128, BN, 0, 0);
         const uint32_t first = smem_u32(smem) >> 4;
         Ring32<STAGES> ring;
@@ -329,21 +335,23 @@ gemm32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
             const int st = ring.at, b = chain & 1;
             const uint32_t base = first + st * (S::STAGE >> 4);
             const bool starts = kb % CHAIN == 0;
-            if (starts && chain >= 2) s32_wait(acc_empty + b, ((uint32_t)(chain >> 1) & 1) ^ 1);
-            s32_wait(full + st * PARTS, ring.round);
+            if (starts && chain >= 2) s32_wait_warp(acc_empty + b, ((uint32_t)(chain >> 1) & 1) ^ 1);
+            s32_wait_warp(full + st * PARTS, ring.round);
 #pragma unroll
             for (int p = 1; p < PARTS; ++p) {      // the small terms first
-              s32_wait(full + st * PARTS + p, ring.round);
+              s32_wait_warp(full + st * PARTS + p, ring.round);
               tc_fence_after();
+              if (issue) {
 #pragma unroll
-              for (int ks = 0; ks < 4; ++ks)
-                umma_ss(tm + (uint32_t)b * BN, s32_desc(base + ((S::W_BYTES + (p - 1) * S32_BOX) >> 4) + ks * 2), s32_desc(base + ks * 2), idesc,
-                        (p > 1 || ks > 0 || !starts) ? 1u : 0u);
-              umma_commit(empty + st * PARTS + p);
+                for (int ks = 0; ks < 4; ++ks)
+                  umma_ss(tm + (uint32_t)b * BN, s32_desc(base + ((S::W_BYTES + (p - 1) * S32_BOX) >> 4) + ks * 2), s32_desc(base + ks * 2), idesc,
+                          (p > 1 || ks > 0 || !starts) ? 1u : 0u);
+                umma_commit(empty + st * PARTS + p);
+              }
             }
-            umma_commit(empty + st * PARTS);
+            if (issue) umma_commit(empty + st * PARTS);
             if (kb % CHAIN == CHAIN - 1 || kb == kb_n - 1) {
-              umma_commit(acc_full + b);
+              if (issue) umma_commit(acc_full + b);
               ++chain;
             }
           }
@@ -778,18 +786,19 @@ attn32_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         }
       }
     } else if (warp == 1) {
-      if (lane == 0) {
+      {
+        const bool issue = elect_one();
         constexpr uint32_t idesc_o = umma_idesc_bf16(128, 128, 0, 1);
         const uint32_t q_at = smem_u32(smem) >> 4, ring_at = smem_u32(smem + S::RING) >> 4;
         constexpr uint32_t BOX = S32_BOX >> 4;
         Ring32<SLOTS> ring;
         auto box = [&]() {
-          s32_wait(full + ring.at, ring.round);
+          s32_wait_warp(full + ring.at, ring.round);
           tc_fence_after();
           return ring_at + ring.at * BOX;
         };
         auto done = [&]() {
-          umma_commit(empty + ring.at);
+          if (issue) umma_commit(empty + ring.at);
           ring.next();
         };
         // a box of keys and the terms of the queries that it meets
@@ -800,15 +809,17 @@ attn32_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 #pragma unroll
             for (int b = 0; b < NB; ++b) {
               const uint32_t k_at = box();
+              if (issue) {
 #pragma unroll
-              for (int q = g == 1 ? 1 : g == 2 ? 2 : 0; q >= (g == 2 ? 1 : 0); --q)
+                for (int q = g == 1 ? 1 : g == 2 ? 2 : 0; q >= (g == 2 ? 1 : 0); --q)
 #pragma unroll
-                for (int ks = 0; ks < 4; ++ks)
-                  umma_ss(d, s32_desc(q_at + (q * NB + b) * BOX + ks * 2), s32_desc(k_at + ks * 2), idesc_s, g + b + ks > 0 ? 1u : 0u);
+                  for (int ks = 0; ks < 4; ++ks)
+                    umma_ss(d, s32_desc(q_at + (q * NB + b) * BOX + ks * 2), s32_desc(k_at + ks * 2), idesc_s, g + b + ks > 0 ? 1u : 0u);
+              }
               done();
             }
           }
-          umma_commit(s_full + (i & 1));
+          if (issue) umma_commit(s_full + (i & 1));
         };
         // the output of a tile as two sums, one after the other in the same columns: full-size products of the first 64 keys; then all smaller
         // ones and after them the full-size ones of the other keys.  One chain of eight full-size steps lost 1.4e-7 of the output.
@@ -820,30 +831,32 @@ attn32_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             const int kh = g == 7 || (g > 0 && (g & 1) == 0);
             if (kh * 4 < steps) {
               const uint32_t v_at = box() | (S32_BOX / 2 >> 4) << 16;
+              if (issue) {
 #pragma unroll
-              for (int q = g == 3 || g == 4 ? 1 : g == 5 || g == 6 ? 2 : 0; q >= (g == 5 || g == 6 ? 1 : 0); --q)
+                for (int q = g == 3 || g == 4 ? 1 : g == 5 || g == 6 ? 2 : 0; q >= (g == 5 || g == 6 ? 1 : 0); --q)
 #pragma unroll
-                for (int k4 = 0; k4 < 4; ++k4) {
-                  const int ks = kh * 4 + k4;      // 16 keys: upper and middle terms lie side by side, 32 keys at a time
-                  if (ks < steps)
-                    umma_ts(tm + TM_O, q == 2 ? tm + TM_X + ks * 8 : p + (ks >> 1) * 32 + (ks & 1) * 8 + q * 16, s32_desc(v_at + k4 * 128), idesc_o,
-                            g > 1 || k4 > 0 ? 1u : 0u);
-                }
+                  for (int k4 = 0; k4 < 4; ++k4) {
+                    const int ks = kh * 4 + k4;      // 16 keys: upper and middle terms lie side by side, 32 keys at a time
+                    if (ks < steps)
+                      umma_ts(tm + TM_O, q == 2 ? tm + TM_X + ks * 8 : p + (ks >> 1) * 32 + (ks & 1) * 8 + q * 16, s32_desc(v_at + k4 * 128), idesc_o,
+                              g > 1 || k4 > 0 ? 1u : 0u);
+                  }
+              }
               done();
             }
             if (g == 0) {
-              umma_commit(pv_done);
-              s32_wait(o_taken, i & 1);
+              if (issue) umma_commit(pv_done);
+              s32_wait_warp(o_taken, i & 1);
               tc_fence_after();
             }
           }
-          umma_commit(pv_done + 1);
+          if (issue) umma_commit(pv_done + 1);
         };
-        s32_wait(q_full, 0);
+        s32_wait_warp(q_full, 0);
         scores(0);
         for (int i = 0; i < n; ++i) {
           if (i + 1 < n) scores(i + 1);
-          s32_wait(p_full, i & 1);
+          s32_wait_warp(p_full, i & 1);
           tc_fence_after();
           outputs(i);
         }

@@ -234,6 +234,8 @@ inline void named_bar(int id, int n, bool wait) {
     }
   }
 }
+inline void mbar_wait_warp(uint64_t* bar, uint32_t parity) { mbar_wait(bar, parity); __syncwarp(); }
+inline bool elect_one() { return (emu::linear_tid() & 31) == 0; }
 inline void pdl_wait() {}
 inline void pdl_launch_dependents() {}
 
