@@ -389,7 +389,9 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         stat_row = row;
       }
       const int row_base = m0 + lg * 32;
-      const int c_begin_n = wg == 0 ? 0 : (NC + 1) / 2, c_end_n = wg == 0 ? (NC + 1) / 2 : NC;   // this warp's 32-column chunks
+      // this warp's 32-column chunks
+      const bool one_wg = BN == 128 && args.stat_parts > 0;
+      const int c_begin_n = wg == 0 ? 0 : one_wg ? NC : (NC + 1) / 2, c_end_n = wg == 0 && !one_wg ? (NC + 1) / 2 : NC;
       auto res_issue = [&](uint32_t g, int col0) {      // lane 0: residual tile of chunk g -> ring buffer g % 3
         mbar_arrive_expect_tx(&rbar[g % 3], 2048);
         tma_load_2d(ring + (g % 3) * 2048, &tmR, &rbar[g % 3], col0, row_base);
@@ -398,7 +400,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         // the first two residual chunks of the tile are requested before the accumulator is even complete; buffers g % 3 and
         // (g + 1) % 3 were last read by the stores of chunks g - 3 and g - 2: at most the newest store may still be reading
         tma_store_wait_read<1>();
-        if (n0 + c_begin_n * 32 < args.N) res_issue(rg, n0 + c_begin_n * 32);
+        if (c_begin_n < c_end_n && n0 + c_begin_n * 32 < args.N) res_issue(rg, n0 + c_begin_n * 32);
         if (c_begin_n + 1 < c_end_n && n0 + (c_begin_n + 1) * 32 < args.N) res_issue(rg + 1, n0 + (c_begin_n + 1) * 32);
       }
       epi_named_barrier();   // bias / column sums of this item (written during the previous item) are visible
@@ -416,15 +418,17 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       float2 ostat = make_float2(0.f, 0.f);
       float2* ostat_p = args.stats_out != nullptr ? &ostat : nullptr;
       if (!swiglu) {
-        const int c_begin = wg == 0 ? 0 : (NC + 1) / 2, c_end = wg == 0 ? (NC + 1) / 2 : NC;
-        // RoPE tiles (BN = 256): each warpgroup owns one 128-column head = chunks c_begin .. c_begin + 3; column i pairs with i + 64
-        const bool rope_tile = BN == 256 && args.rope_heads > 0 && ((n0 >> 7) + wg) < args.rope_heads;
+        const int c_begin = c_begin_n, c_end = c_end_n;
+        // RoPE tiles: column i of a 128-column head pairs with i + 64.  BN = 256: each warpgroup owns a head = chunks c_begin .. c_begin + 3; BN = 128: the tile is a
+        // head, each warpgroup takes one of its two pairs of chunks
+        const bool rope_tile = (BN == 256 || BN == 128) && args.rope_heads > 0 && ((n0 >> 7) + (BN == 256 ? wg : 0)) < args.rope_heads;
         if (rope_tile) {
+          const int head0 = BN == 256 ? c_begin : 0;
 #pragma unroll 1
-          for (int p = 0; p < 2; ++p) {
+          for (int p = BN == 256 ? 0 : wg; p < (BN == 256 ? 2 : wg + 1); ++p) {
             uint32_t rl[32], rh[32];
-            LP_TMEM_LD_32(rl, taddr0 + (c_begin + p) * 32);
-            LP_TMEM_LD_32(rh, taddr0 + (c_begin + p + 2) * 32);
+            LP_TMEM_LD_32(rl, taddr0 + (head0 + p) * 32);
+            LP_TMEM_LD_32(rh, taddr0 + (head0 + p + 2) * 32);
             tmem_wait_ld();
             float lo[32], hi[32];
             const float* cp = args.rope_cos + (long long)(row_ok ? row : 0) * 64 + p * 32;
@@ -442,8 +446,8 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
               LP_ROPE_PAIR(0, c4.x, s4.x) LP_ROPE_PAIR(1, c4.y, s4.y) LP_ROPE_PAIR(2, c4.z, s4.z) LP_ROPE_PAIR(3, c4.w, s4.w)
 #undef LP_ROPE_PAIR
             }
-            staged_store_chunk(args, tmc, stage, lo, nullptr, row_base - st_shift, n0 + (c_begin + p) * 32, lane, ostat_p);
-            staged_store_chunk(args, tmc, stage, hi, nullptr, row_base - st_shift, n0 + (c_begin + p + 2) * 32, lane, ostat_p);
+            staged_store_chunk(args, tmc, stage, lo, nullptr, row_base - st_shift, n0 + (head0 + p) * 32, lane, ostat_p);
+            staged_store_chunk(args, tmc, stage, hi, nullptr, row_base - st_shift, n0 + (head0 + p + 2) * 32, lane, ostat_p);
           }
         } else if (TMARES) {
           uint32_t done = 0;
@@ -477,7 +481,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
           rg += done;
         } else {
         ResidualRegs rr;
-        if (has_res && !args.out_fp32 && n0 + c_begin * 32 < args.N)
+        if (has_res && !args.out_fp32 && c_begin < c_end && n0 + c_begin * 32 < args.N)
           residual_fetch(args, rr, row_base, n0 + c_begin * 32, args.N, lane);
 #pragma unroll 1
         for (int c = c_begin; c < c_end; ++c) {
@@ -531,8 +535,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
           staged_store_chunk(args, tmc, stage, v, has_res ? &cur : nullptr, row_base - st_shift, col0 / 2, lane);
         }
       }
-      if (args.stats_out != nullptr && row_ok)
-        args.stats_out[(long long)row * (2 * args.num_n_blk) + 2 * n_blk + wg] = ostat;
+      if (args.stats_out != nullptr && row_ok) {
+        if (!one_wg) args.stats_out[(long long)row * (2 * args.num_n_blk) + 2 * n_blk + wg] = ostat;
+        else if (wg == 0 || (n_blk == args.num_n_blk - 1 && n_blk + 1 < args.stat_parts)) args.stats_out[(long long)row * args.stat_parts + n_blk + wg] = ostat;
+      }
       if (prefetch_cols && col_thread) {   // the other buffer: last read during item it - 1, which every warp has left (barrier above)
         bias_smem[(as ^ 1) * BN + et] = nbv;
         colsum_smem[(as ^ 1) * BN + et] = ncv;
@@ -775,13 +781,34 @@ extern "C" int lp_gemm_bf16_ex(const lp_gemm_desc* d, void* stream_) {
   args.norm_inv_k = 1.0f / (float)K;
   args.stats_out = reinterpret_cast<float2*>(d->stats_out);
   args.rope_cos = d->rope_cos; args.rope_sin = d->rope_sin; args.rope_heads = d->rope_heads;
+  const int parts_256 = 2 * ((N + 255) / 256);
   if (pair && (block_n == 160 || mb * ((N + block_n - 1) / block_n) < units)) pair = false;
+  // A problem of fewer 256-row tiles than CTA pairs is bound by what each CTA brings from the L2 a k-block: 128 rows of A and block_n rows of W, or half of these
+  // as one of a pair, 1.02 ns a row (62 bytes a clock), more where over 105 CTAs share the L2.  So it takes the shape that brings least; a pair costs 1 us more
+  // to start, which a K below 3072 does not give back.  M = 201, us (CTAs of 256, of 128, pairs of 128): N = 4096, K = 4096 28.5, 18.9, 18.7; N = 1152, K = 4304
+  // 31.0, 20.9, 18.6; N = K = 1152 11.5, 8.2, 9.0; N = K = 2048 16.5, 10.9, 11.8; M = 1000, N = 6144, K = 4096 50.8, 41.4, 38.2.  Launches of rotated heads or row statistics
+  // have 256-wide tiles unless this narrows them.
+  if (g_gemm_pair_mode != 0 && !pair && !d->a_t && !d->b_t && (d->block_n == 0 || block_n == 256) &&
+      (long long)((M + 255) / 256) * ((N + block_n - 1) / block_n) < sms / 2) {
+    auto cost = [&](bool pairs, int bn) {      // rows a CTA brings, wave after wave
+      const long long tiles = ((M + (pairs ? 255 : 127)) / (pairs ? 256 : 128)) * (long long)((N + bn - 1) / bn), room = pairs ? sms / 2 : sms;
+      const long long waves = (tiles + room - 1) / room, ctas = (pairs ? 2 : 1) * (tiles < room ? tiles : room);
+      return (double)waves * (128 + (pairs ? bn / 2 : bn)) * (ctas > 105 ? ctas / 105.0 : 1.0);
+    };
+    const bool long_k = K >= 3072;
+    double best = 0.95 * cost(false, block_n);
+    int narrow = block_n;
+    if (long_k && block_n != 160 && cost(true, block_n) < best) { best = cost(true, block_n); pair = true; }
+    if ((long_k || block_n == 256) && cost(long_k, 128) < best) { narrow = 128; pair = long_k; }
+    if (narrow != block_n && d->stats_out != nullptr) args.stat_parts = parts_256;
+    block_n = narrow;
+  }
   args.num_m_blk = pair ? (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM) : (M + GEMM_BM - 1) / GEMM_BM;
   args.num_n_blk = (N + block_n - 1) / block_n;
   args.num_k_blk = (K + GEMM_BK - 1) / GEMM_BK;
-  LP_REQUIRE(d->stats_out == nullptr || d->stats_out_parts == 2 * args.num_n_blk,
+  LP_REQUIRE(d->stats_out == nullptr || d->stats_out_parts == (args.stat_parts > 0 ? args.stat_parts : 2 * args.num_n_blk),
              "lp_gemm_bf16_ex: stats_out_parts=%d, this launch writes %d per row (2 x column blocks of %d)", d->stats_out_parts,
-             2 * args.num_n_blk, block_n);
+             args.stat_parts > 0 ? args.stat_parts : 2 * args.num_n_blk, args.stat_parts > 0 ? 256 : block_n);
   {
     // L2-aware rasterisation: keep the operand that fits L2 resident, stream the other from HBM once
     const double l2_budget = 56e6;

@@ -38,7 +38,10 @@ struct GemmArgs {
   // ---- producer side: per-row (sum, sum of squares) of the bf16-ROUNDED outputs of this GEMM, one pair per (column block,
   // epilogue warpgroup): stats_out[row * 2 * num_n_blk + 2 * n_blk + wg]; summed in index order by the consumer (deterministic)
   float2* stats_out;
-  // ---- rotate-half RoPE on the first `rope_heads` 128-column heads (decoder QKV; tables [M, 64] fp32; BN = 256 only)
+  // 128-wide tiles that write the statistics of 256-wide ones, a pair per 128 columns added up by one warpgroup in the same order: stats_out[row *
+  // stat_parts + n_blk] (the second half of a last block that has none is written as zeros); 0: the tile's own two halves
+  int stat_parts;
+  // ---- rotate-half RoPE on the first `rope_heads` 128-column heads (decoder QKV; tables [M, 64] fp32; BN = 256 or 128)
   const float* rope_cos;
   const float* rope_sin;
   int rope_heads;

@@ -56,6 +56,10 @@ static int g_sk_pure = 0;     // pure stream-K over a column-block-fastest raste
 extern "C" void emu_gemm_set_streamk(void* ws) { g_sk_ws = ws; }
 extern "C" void emu_gemm_set_streamk_pure(int on) { g_sk_pure = on; }
 
+// 128-wide tiles that write the row statistics of 256-wide ones
+static int g_stat_256 = 0;
+extern "C" void emu_gemm_set_stat_256(int on) { g_stat_256 = on; }
+
 extern "C" void emu_gemm_ex(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc, int M, int N, int K,
                             const float* bias, const void* residual, long long ldr, int res_row_mod, int act, int out_fp32,
                             int block_n, int pair, int group_m, int ctas, const EmuFusions* fx) {
@@ -67,6 +71,7 @@ extern "C" void emu_gemm_ex(const void* A, long long lda, const void* W, long lo
     args.stats_out = reinterpret_cast<float2*>(fx->stats_out);
     args.rope_cos = fx->rope_cos; args.rope_sin = fx->rope_sin; args.rope_heads = fx->rope_heads;
   }
+  if (g_stat_256 && block_n == 128 && args.stats_out != nullptr) args.stat_parts = 2 * ((N + 255) / 256);
   args.M = M; args.N = N; args.K = K;
   args.C = C; args.ldc = ldc; args.out_fp32 = out_fp32;
   args.bias = bias;
