@@ -715,6 +715,9 @@ int lp_gather_rows(const void* src, long long ld, int src_fp32, const int* row_o
 int lp_gemm_split(const void* A, long long lda, long long a_plane, const void* W, long long ldw, void* C, long long ldc, long long c_plane,
                   int out, int M, int N, int K, const float* bias, void* stream);
 /* the same from fp32 rows; terms: room for 3 M K bf16 */
+/* The products of lp_linear's descriptor that the tcgen05 GEMM ends itself (bf16 A, one problem; the alignments of lp_gemm_bf16): c_accum with epi NONE and fp32 C,
+ * C <- C + c_scale * (A W^T + bias), or bf16 C = relu2 / xielu(A W^T + bias). */
+int lp_gemm_linear(const lp_linear_desc* desc, void* stream);
 int lp_linear_split(const float* A, long long lda, const void* W, long long ldw, void* C, long long ldc, int out, int M, int N, int K, const float* bias,
                     void* terms, void* stream);
 /* The products of sorted (token, expert) rows on the tcgen05 tensor cores: rows of A (n_tiles * 128 of them; bf16, or with a_plane > 0 fp32 in three planes) in

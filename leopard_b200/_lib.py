@@ -294,6 +294,7 @@ _SIGS = {
     "lp_gather_rows": (_i, [_vp, _ll, _i, _vp, _i, _i, _vp, _ll, _vp]),
     "lp_latent_route": (_i, [_vp, _vp, _i, _i, _i, _i, C.POINTER(_i), C.POINTER(_i)]),
     "lp_window_prompt_count": (_i, [C.POINTER(WindowAttnDesc), _vp, _vp, _i, C.POINTER(_i), C.POINTER(_i)]),
+    "lp_gemm_linear": (_i, [C.POINTER(LinearDesc), _vp]),
     "lp_linear_split": (_i, [_vp, _ll, _vp, _ll, _vp, _ll, _i, _i, _i, _i, _vp, _vp, _vp]),
     "lp_gemm_grouped": (_i, [_vp, _ll, _ll, _vp, _ll, _ll, _i, _vp, _i, _i, _vp, _vp, _ll, _ll, _i, _i, _i, _vp]),
     "lp_window_prompt_workspace_bytes": (C.c_size_t, [_i, _i, _i, _i]),
@@ -357,7 +358,7 @@ STREAM32_SYMBOLS = ("lp_last_error", "lp_abi_version", "lp_launch_count", "lp_li
                     "lp_moe_route_group_softmax")
 STREAM32_OPTIONAL = ("lp_gemm_bf16", "lp_split_rows", "lp_gemm_split", "lp_latent_expanded_workspace_bytes", "lp_latent_attend_expanded",
                      "lp_latent_route", "lp_window_prompt_count", "lp_gather_rows",
-                     "lp_window_prompt_workspace_bytes", "lp_window_attn_prompt", "lp_gemm_grouped", "lp_linear_split")      # present in the native libraries, absent from the CPU-emulated build
+                     "lp_window_prompt_workspace_bytes", "lp_window_attn_prompt", "lp_gemm_grouped", "lp_linear_split", "lp_gemm_linear")      # present in the native libraries, absent from the CPU-emulated build
 _stream32 = None
 
 

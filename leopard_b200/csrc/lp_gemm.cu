@@ -495,10 +495,14 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
           apply_row_norm(args, v, cs + c * 32, rs, nmu);
-          if (args.out_fp32) {
+          if (RES == 3 && args.end == GEMM_END_ADD) {
+            apply_bias_act(args, v, bs + c * 32);
+            end_add_chunk(args, v, row, row_ok, col0, args.N);
+          } else if (RES != 3 && args.out_fp32) {
             epilogue_store_chunk(args, v, bs + c * 32, row, rrow, row_ok, col0, args.N);
           } else {
             apply_bias_act(args, v, bs + c * 32);
+            if (RES == 3) apply_end_act(args, v);
             ResidualRegs cur = rr;
             if (has_res && c + 1 < c_end && col0 + 32 < args.N)  // prefetch the next chunk's residual
               residual_fetch(args, rr, row_base, col0 + 32, args.N, lane);
@@ -604,6 +608,14 @@ gemm_bf16_lres_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   gemm_body<BN, STAGES, CTA2, false, 1>(tmA, tmB, tmC, nullptr, tmC, args);
 }
 
+// the ends of the 32-bit stream's products: kernels of their own, since the activations' code would cost the others instruction misses
+template <int BN, int STAGES, bool CTA2>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+gemm_bf16_end_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                     const __grid_constant__ CUtensorMap tmC, const GemmArgs args) {
+  gemm_body<BN, STAGES, CTA2, false, 3>(tmA, tmB, tmC, nullptr, tmC, args);
+}
+
 // residual launches of the layer loops: residual tile by TMA (tmR; equal to tmC for the in-place residual stream)
 template <int BN, int STAGES, bool CTA2>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
@@ -623,11 +635,13 @@ template <int BN, int STAGES, bool CTA2>
 static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const GemmArgs& args,
                        cudaStream_t stream) {
   using L = GemmSmem<BN, STAGES, CTA2>;
-  auto kern = args.residual != nullptr ? gemm_bf16_lres_kernel<BN, STAGES, CTA2> : gemm_bf16_kernel<BN, STAGES, CTA2>;
+  auto kern = args.end != GEMM_END_NONE ? gemm_bf16_end_kernel<BN, STAGES, CTA2>
+              : args.residual != nullptr ? gemm_bf16_lres_kernel<BN, STAGES, CTA2> : gemm_bf16_kernel<BN, STAGES, CTA2>;
   static bool configured = false;
   if (!configured) {
     LP_CHECK_CUDA(cudaFuncSetAttribute(gemm_bf16_kernel<BN, STAGES, CTA2>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
     LP_CHECK_CUDA(cudaFuncSetAttribute(gemm_bf16_lres_kernel<BN, STAGES, CTA2>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
+    LP_CHECK_CUDA(cudaFuncSetAttribute(gemm_bf16_end_kernel<BN, STAGES, CTA2>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
     configured = true;
   }
   const int tiles = args.num_m_blk * args.num_n_blk;
@@ -722,7 +736,8 @@ extern "C" int lp_gemm_pick_block_n(int M, int N, int act) {
   return pick_block_n(M, N, act, g_gemm_pair_mode != 0 && M > GEMM_BM, sm_count());
 }
 
-extern "C" int lp_gemm_bf16_ex(const lp_gemm_desc* d, void* stream_) {
+struct GemmEnd { int end; float a, b, scale; };
+static int gemm_run(const lp_gemm_desc* d, const GemmEnd& end, void* stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LP_REQUIRE(d != nullptr, "lp_gemm_bf16_ex: null descriptor");
   const void* A = d->A; const void* W = d->W; void* C = d->C;
@@ -772,6 +787,7 @@ extern "C" int lp_gemm_bf16_ex(const lp_gemm_desc* d, void* stream_) {
   args.residual = reinterpret_cast<const bf16*>(residual);
   args.ldr = ldr; args.res_row_mod = res_row_mod;
   args.act = act;
+  args.end = end.end; args.end_a = end.a; args.end_b = end.b; args.end_scale = end.scale;
   args.epi_sleep_ns = g_gemm_epi_sleep_ns;
   args.norm_mode = d->norm_mode;
   args.stats_in = reinterpret_cast<const float2*>(d->stats_in);
@@ -922,6 +938,22 @@ extern "C" int lp_gemm_bf16_ex(const lp_gemm_desc* d, void* stream_) {
     case 160: return launch_gemm<160, 5, false>(tmA, tmB, tmC, args, stream);
     default: return launch_gemm<128, 6, false>(tmA, tmB, tmC, args, stream);
   }
+}
+
+extern "C" int lp_gemm_bf16_ex(const lp_gemm_desc* d, void* stream) { return gemm_run(d, GemmEnd{GEMM_END_NONE, 0.f, 0.f, 0.f}, stream); }
+
+// Products of the 32-bit residual stream in one launch: bf16 squared relu or xIELU of the sums (4,096 rows, N = 8192, K = 2048: 110 us and 42 or 68 for the
+// activation's kernel over the fp32 sums; as one 84 and 148), or x <- x + m * sums (N = 2048, K = 8192: 97 and 12.7, as one 103).
+extern "C" int lp_gemm_linear(const lp_linear_desc* d, void* stream) {
+  LP_REQUIRE(d != nullptr && !d->a_fp32 && d->batch == 1 && d->gate == nullptr && d->row_scale == nullptr && d->seg_cols == 0,
+             "lp_gemm_linear: one product of bf16 rows without gates, row scales or segments");
+  const bool add = d->c_accum != 0;
+  LP_REQUIRE(add ? d->epi == LP_EPI_NONE && d->c_fp32 : (d->epi == LP_EPI_RELU2 || d->epi == LP_EPI_XIELU) && !d->c_fp32,
+             "lp_gemm_linear: fp32 C += m * A W^T, or bf16 C = the squared relu or xIELU of A W^T");
+  lp_gemm_desc g = {};
+  g.A = d->A; g.lda = d->lda; g.W = d->W; g.ldw = d->ldw; g.C = d->C; g.ldc = d->ldc;
+  g.M = d->M; g.N = d->N; g.K = d->K; g.bias = d->bias; g.out_fp32 = add;
+  return gemm_run(&g, GemmEnd{add ? GEMM_END_ADD : d->epi == LP_EPI_RELU2 ? GEMM_END_RELU2 : GEMM_END_XIELU, d->epi_a, d->epi_b, d->c_scale}, stream);
 }
 
 extern "C" int lp_gemm_bf16(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc, int M,

@@ -13,6 +13,7 @@ constexpr int GEMM_BK = 64;
 constexpr int GEMM_THREADS = 320;
 constexpr int GEMM_EPI_THREADS = 256;
 
+enum { GEMM_END_NONE = 0, GEMM_END_RELU2 = 1, GEMM_END_XIELU = 2, GEMM_END_ADD = 3 };
 struct GemmArgs {
   int M, N, K;
   void* C;
@@ -38,6 +39,9 @@ struct GemmArgs {
   // ---- producer side: per-row (sum, sum of squares) of the bf16-ROUNDED outputs of this GEMM, one pair per (column block,
   // epilogue warpgroup): stats_out[row * 2 * num_n_blk + 2 * n_blk + wg]; summed in index order by the consumer (deterministic)
   float2* stats_out;
+  // ---- ends of the 32-bit stream's products (gemm_bf16_end_kernel): an activation of the fp32 sums before a bf16 store, or fp32 C <- C + end_scale * sums
+  int end;                       // GEMM_END_*
+  float end_a, end_b, end_scale;
   // 128-wide tiles that write the statistics of 256-wide ones, a pair per 128 columns added up by one warpgroup in the same order: stats_out[row *
   // stat_parts + n_blk] (the second half of a last block that has none is written as zeros); 0: the tile's own two halves
   int stat_parts;
@@ -191,6 +195,32 @@ __device__ __forceinline__ int tile_row0(const GemmArgs& a, int m_blk, int rows_
 }
 
 
+
+// the squared relu and xIELU of 32 sums
+__device__ __forceinline__ void apply_end_act(const GemmArgs& args, float* v) {
+  if (args.end == GEMM_END_RELU2) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f) * fmaxf(v[j], 0.f);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      v[j] = v[j] > 0.f ? args.end_a * v[j] * v[j] + 0.5f * v[j] : args.end_b * (expm1f(v[j]) - v[j]) + 0.5f * v[j];
+  }
+}
+// 32 columns of one row of C <- C + end_scale * sums
+__device__ __forceinline__ void end_add_chunk(const GemmArgs& args, const float* v, int row, bool row_ok, int col0, int n_limit) {
+  if (!row_ok) return;
+  float* cp = reinterpret_cast<float*>(args.C) + (long long)row * args.ldc + col0;
+  float4 c[8];
+#pragma unroll
+  for (int g = 0; g < 8; ++g)
+    if (col0 + g * 4 < n_limit) c[g] = *reinterpret_cast<const float4*>(cp + g * 4);
+#pragma unroll
+  for (int g = 0; g < 8; ++g)
+    if (col0 + g * 4 < n_limit)
+      *reinterpret_cast<float4*>(cp + g * 4) = make_float4(fmaf(args.end_scale, v[g * 4], c[g].x), fmaf(args.end_scale, v[g * 4 + 1], c[g].y),
+                                                           fmaf(args.end_scale, v[g * 4 + 2], c[g].z), fmaf(args.end_scale, v[g * 4 + 3], c[g].w));
+}
 
 // applies bias/activation/residual to 32 accumulator columns of one row and stores them
 __device__ __forceinline__ void epilogue_store_chunk(const GemmArgs& args, float* v, const float* bias_s, int row,

@@ -37,6 +37,9 @@ TENSOR_CORE_MIN_ROWS = 64
 # whose sums are cut off: 2.1e-6 of the result at K = 2048, 9.1e-6 at 8192, against 2.3e-7 streamed and 3.9e-7, 9.6e-7 of fp32 multiply-adds.  So
 # it has the products of 64 rows and more, as large prompts always had; at 64 rows only those above the crossing.
 STREAM_MAX_OUTPUTS = 170_000
+# xIELU in the store of the product: its code is long, and with a tile or two a CTA reading it costs more than a kernel of its own (64 x 4096 outputs 21.7 us, as two
+# launches 12.0; 4,096 x 8,192 148 us and 108 + 68)
+XIELU_END_OUTPUTS = 1 << 23
 # fp32 rows of more than 64 go to the tcgen05 product of three bf16 terms where K is long, a pass for the terms included (us, lp_linear and this one): 65 rows,
 # K = 1024, 4096 columns 36, 21; 4000 rows, K = 1024, 4096 columns 388, 105.  Up to 64 rows lp_linear streams the weights: 48 rows, K = 1024 12.5, 20.  What the
 # tensor cores cut off does not depend on K while lp_linear's roundings grow with it, so a short K stays although it would be faster too (65 rows, K = 64, 128
@@ -964,6 +967,11 @@ class SeqLMEngine:
         if into is not None:
             x, mult = into[0], into[1]
             gate = into[2] if len(into) > 2 else None
+            if tc and not split and epi == _lib.EPI_NONE and gate is None and row_scale is None and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0:
+                d = _lib.LinearDesc(A=_lib.ptr(a), lda=a.stride(0), W=_lib.ptr(w), ldw=w.stride(0), C=_lib.ptr(x), ldc=x.stride(0), c_fp32=1, M=M, N=N, K=K,
+                                    batch=1, epi=epi, c_accum=1, c_scale=float(mult), bias=_lib.ptr(bias))
+                self._check(self.L.lp_gemm_linear(C.byref(d), self._stream()), "lp_gemm_linear")
+                return x
             if tc:
                 y = self.linear(a, w, F32, epi, epi_a, epi_b, bias=bias, row_scale=row_scale)
                 if gate is None:
@@ -982,6 +990,11 @@ class SeqLMEngine:
         if out is None:
             out = self._empty((M, n_out), out_dtype)
         if tc and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0:
+            if not split and out.dtype == BF16 and row_scale is None and (epi == _lib.EPI_RELU2 or (epi == _lib.EPI_XIELU and M * N >= XIELU_END_OUTPUTS)):
+                d = _lib.LinearDesc(A=_lib.ptr(a), lda=a.stride(0), W=_lib.ptr(w), ldw=w.stride(0), C=_lib.ptr(out), ldc=out.stride(0), M=M, N=N, K=K, batch=1,
+                                    epi=epi, epi_a=epi_a, epi_b=epi_b, bias=_lib.ptr(bias))
+                self._check(self.L.lp_gemm_linear(C.byref(d), self._stream()), "lp_gemm_linear")
+                return out
             raw = out if epi == _lib.EPI_NONE else self._empty((M, N), F32)
             if split:
                 self._split_product(a, w, raw, bias)
