@@ -615,7 +615,7 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
 }
 
 // ---------------------------------------------------------------------------------------------------------------------------------
-// The same product for up to 16 rows as one stream of weights: a CTA an SM walks its tiles of 16 or 32 weight rows, and one thread keeps a ring of pieces
+// The same product as one stream of weights: a CTA an SM walks its tiles of 16 or 32 weight rows, and one thread keeps a ring of pieces
 // of them full by TMA, so that DRAM sees whole kilobytes and the next pieces are under way while the sums of a tile are
 // stored.  Eight warps take the products of a piece, four others add up their sums and store the tile before: nothing in the stream waits for
 // an epilogue.  Where no launch before this one writes the weights (w_constant), the ring is filled before that launch has ended.
@@ -624,18 +624,20 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
 // pieces took the issue slots (39 -> 49 us), and bulk copies of a row each cost 110 cycles of a warp.  190 KB under way an SM: with 96 KB the same took 50 us.
 // The weights leave the L2 first: left to its usual order, they threw out the caches and states of the small kernels around them (window attention of one row 13 ->
 // 23 us).  Sums: 16 products a chain, which the instruction cuts off, then exactly; error against 64 bits, 1e-7 of the result: 0.5 for bf16 rows, 0.7 for fp32
-// rows at every K (above: 0.5 to 1.2 and 0.7 to 1.2).
+// rows at every K (above: 0.5 to 1.2 and 0.7 to 1.2); more than 16 rows are added up plainly, 0.6 and 0.75 at K = 1024 (above: 0.9 to 1.3 and 0.9 to 1.0).
 constexpr int RING_TAKERS = 8, RING_STORERS = 4, RING_WARPS = 2 + RING_TAKERS + RING_STORERS, RING_MAX_STAGES = 8, RING_MAX_GROUPS = 256;
 constexpr int RING_BYTES = 208 * 1024;      // of pieces and sums
 // A piece is KC columns of 16 NT weight rows and of the rows of A, boxes of 8 rows x 128 bytes one after another: a warp takes KC / 32 / 8 steps of it between two waits.
-template <typename AT> constexpr int ring_kc() { return sizeof(AT) == 2 ? 1024 : 512; }
-template <typename AT, int NT> constexpr int ring_w() { return NT * 16 * ring_kc<AT>() * 2; }
+// More rows of A take more of the ring: fewer columns of them.
+template <typename AT, int MG> constexpr int ring_kc() { return MG == 8 ? 256 : MG == 4 ? (sizeof(AT) == 2 ? 512 : 256) : sizeof(AT) == 2 ? 1024 : 512; }
+template <typename AT, int NT, int MG> constexpr int ring_w() { return NT * 16 * ring_kc<AT, MG>() * 2; }
 // the rows of pairs lie apart and come by a bulk copy each: bytes from one to the next (four lanes' pieces of two rows are in banks of their own)
-template <typename AT> constexpr int ring_pair_row() { return ring_kc<AT>() * (int)sizeof(AT) + (sizeof(AT) == 2 ? 64 : 16); }
+template <typename AT, int MG> constexpr int ring_pair_row() { return ring_kc<AT, MG>() * (int)sizeof(AT) + (sizeof(AT) == 2 ? 64 : 16); }
 template <typename AT, int NT, int MG, bool PAIRS> constexpr int ring_piece() {
-  return ring_w<AT, NT>() + (PAIRS ? (8 * MG * ring_pair_row<AT>() + 1023) / 1024 * 1024 : 8 * MG * ring_kc<AT>() * (int)sizeof(AT));
+  return ring_w<AT, NT, MG>() + (PAIRS ? (8 * MG * ring_pair_row<AT, MG>() + 1023) / 1024 * 1024 : 8 * MG * ring_kc<AT, MG>() * (int)sizeof(AT));
 }
-template <int NT, int MG> constexpr int ring_sums() { return 2 * RING_TAKERS * NT * MG * 4 * 32 * (int)sizeof(float); }
+template <int MG> constexpr int ring_bufs() { return MG <= 2 ? 2 : 1; }      // tiles of sums: more rows leave room for one
+template <int NT, int MG> constexpr int ring_sums() { return ring_bufs<MG>() * RING_TAKERS * NT * MG * 4 * 32 * (int)sizeof(float); }
 template <typename AT, int NT, int MG, bool PAIRS> constexpr int ring_stages() {
   constexpr int n = (RING_BYTES - ring_sums<NT, MG>()) / ring_piece<AT, NT, MG, PAIRS>();
   return n < RING_MAX_STAGES ? n : RING_MAX_STAGES;
@@ -644,14 +646,16 @@ template <typename AT, int NT, int MG, bool PAIRS> constexpr int ring_stages() {
 template <typename AT, int NT, int MG, bool PAIRS>
 __global__ void __launch_bounds__(RING_WARPS * 32, 1) linear_ring_kernel(const __grid_constant__ CUtensorMap tw, const __grid_constant__ CUtensorMap ta, LinArgs a,
                                                                          int gated, int c_fp32, int batch, int n_pairs, int n_groups) {
-  extern __shared__ float dyn_smem[];      // (from the next multiple of 1024 bytes) [stages] pieces, then [2][takers][MG 4][32] sums
+  extern __shared__ float dyn_smem[];      // (from the next multiple of 1024 bytes) [stages] pieces, then [BUFS][takers][NT MG 4][32] sums
   __shared__ uint64_t full[RING_MAX_STAGES], empty[RING_MAX_STAGES], sums_full[2], sums_empty[2];
   __shared__ int pair_of[PAIRS ? STREAM_MAX_PAIRS : 1];      // the pairs, a group's together
   __shared__ int count[PAIRS ? RING_MAX_GROUPS : 1];
   __shared__ int2 block_of[PAIRS ? RING_MAX_GROUPS + STREAM_MAX_PAIRS / 8 : 1];      // {group, place of its first pair, number of pairs << 16} of up to 8 MG of a group's pairs
   __shared__ int n_blocks;
-  constexpr int KC = ring_kc<AT>(), STEPS = KC / 32 / RING_TAKERS, SLOTS = NT * MG * 4, PIECE = ring_piece<AT, NT, MG, PAIRS>(), STAGES = ring_stages<AT, NT, MG, PAIRS>();
+  constexpr int KC = ring_kc<AT, MG>(), STEPS = KC / 32 / RING_TAKERS, SLOTS = NT * MG * 4, PIECE = ring_piece<AT, NT, MG, PAIRS>(), STAGES = ring_stages<AT, NT, MG, PAIRS>();
   constexpr int HALF = 8 * KC * 2;      // eight weight rows
+  constexpr int BUFS = ring_bufs<MG>();
+  constexpr bool EXACT = MG <= 2;      // what the additions round off is kept; the kernel above has longer chains with more rows
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const int n_out = gated ? a.N / 2 : a.N, cols = gated ? 8 * NT : 16 * NT, tiles = (n_out + cols - 1) / cols;
@@ -738,7 +742,7 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 1) linear_ring_kernel(const _
     auto load_w = [&](const At& p, int stage) {
       if (lane != 0) return;
       const int kc = min(KC, a.K - p.piece * KC);
-      mbar_arrive_expect_tx(&full[stage], (uint32_t)(ring_w<AT, NT>() + (PAIRS ? p.unit.here * kc : 8 * MG * KC) * (int)sizeof(AT)));
+      mbar_arrive_expect_tx(&full[stage], (uint32_t)(ring_w<AT, NT, MG>() + (PAIRS ? p.unit.here * kc : 8 * MG * KC) * (int)sizeof(AT)));
 #pragma unroll
       for (int h = 0; h < 2 * NT; ++h) {
         const int n = gated ? p.unit.n0 + (h >> 1) * 8 + (h & 1) * n_out : p.unit.n0 + h * 8;
@@ -750,7 +754,7 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 1) linear_ring_kernel(const _
       const int z = a.seg_cols > 0 ? min(p.unit.n0 / a.seg_cols, a.n_segs - 1) : p.unit.z;
 #pragma unroll
       for (int i = 0; i < MG; ++i)
-        tma_load_4d(ring + stage * PIECE + ring_w<AT, NT>() + i * 8 * KC * (int)sizeof(AT), &ta, &full[stage], 0, 8 * i, p.piece * (KC * (int)sizeof(AT) / 128), z);
+        tma_load_4d(ring + stage * PIECE + ring_w<AT, NT, MG>() + i * 8 * KC * (int)sizeof(AT), &ta, &full[stage], 0, 8 * i, p.piece * (KC * (int)sizeof(AT) / 128), z);
     };
     At w{(int)blockIdx.x, 0, {}};
     if (w.u < units) w.unit = unit_at(w.u);
@@ -785,18 +789,18 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 1) linear_ring_kernel(const _
     constexpr int XV = sizeof(AT) == 2 ? 1 : 2;      // 16-byte pieces of eight values of a row
     // this lane's piece of a step in the lower half of a 128-byte line; the upper half's is 64 bytes away, either way
     const int w_at = at_row * 128 + (t ^ at_row) * 16;
-    const int x_at = PAIRS ? g * ring_pair_row<AT>() + t * 8 * (int)sizeof(AT) : sizeof(AT) == 2 ? w_at : x_row * 128;
+    const int x_at = PAIRS ? g * ring_pair_row<AT, MG>() + t * 8 * (int)sizeof(AT) : sizeof(AT) == 2 ? w_at : x_row * 128;
     int stage = 0, turn = 0;
     uint32_t phase = 0;
     pdl_wait();
     for (int u = blockIdx.x; u < units; u += gridDim.x, ++turn) {
-      float acc[NT][MG][4], rest[NT][MG][4];      // rest: what adding the steps' sums rounded off
+      float acc[NT][MG][4], rest[EXACT ? NT : 1][EXACT ? MG : 1][4];      // rest: what adding the steps' sums rounded off
 #pragma unroll
       for (int j = 0; j < NT; ++j)
 #pragma unroll
         for (int i = 0; i < MG; ++i)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) acc[j][i][c] = rest[j][i][c] = 0.f;
+          for (int c = 0; c < 4; ++c) acc[j][i][c] = rest[EXACT ? j : 0][EXACT ? i : 0][c] = 0.f;
 #pragma unroll 1
       for (int piece = 0; piece < pieces; ++piece) {
         mbar_wait(&full[stage], phase);
@@ -804,10 +808,10 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 1) linear_ring_kernel(const _
         uint4 u0[STEPS][NT], u1[STEPS][NT], v[STEPS][MG][XV];
 #pragma unroll
         for (int q = 0; q < STEPS; ++q) {
-          const int step = STEPS * cw + q;      // STEPS is even: which half of the line is known here
+          const int step = STEPS * cw + q, upper = ((STEPS == 1 ? cw : q) & 1) * 64;      // the half of the line
 #pragma unroll
           for (int j = 0; j < NT; ++j) {
-            const uint8_t* const w = base + j * 2 * HALF + (step >> 1) * 1024 + (w_at ^ ((q & 1) * 64));
+            const uint8_t* const w = base + j * 2 * HALF + (step >> 1) * 1024 + (w_at ^ upper);
             u0[q][j] = *reinterpret_cast<const uint4*>(w);
             u1[q][j] = *reinterpret_cast<const uint4*>(w + HALF);
           }
@@ -815,9 +819,9 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 1) linear_ring_kernel(const _
           for (int i = 0; i < MG; ++i)
 #pragma unroll
             for (int p = 0; p < XV; ++p) {
-              const uint8_t* x = base + ring_w<AT, NT>();
-              if constexpr (PAIRS) x += 8 * i * ring_pair_row<AT>() + step * 32 * (int)sizeof(AT) + x_at + 16 * p;
-              else if constexpr (sizeof(AT) == 2) x += i * 8 * KC * 2 + (step >> 1) * 1024 + (x_at ^ ((q & 1) * 64));
+              const uint8_t* x = base + ring_w<AT, NT, MG>();
+              if constexpr (PAIRS) x += 8 * i * ring_pair_row<AT, MG>() + step * 32 * (int)sizeof(AT) + x_at + 16 * p;
+              else if constexpr (sizeof(AT) == 2) x += i * 8 * KC * 2 + (step >> 1) * 1024 + (x_at ^ upper);
               else x += i * 8 * KC * 4 + step * 1024 + x_at + ((2 * t + p) ^ x_row) * 16;
               v[q][i][p] = *reinterpret_cast<const uint4*>(x);
             }
@@ -852,11 +856,14 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 1) linear_ring_kernel(const _
 #pragma unroll
             for (int c = 0; c < 4; ++c)
 #pragma unroll
-              for (int q = 0; q < STEPS; ++q) rest[j][i][c] += add_exactly(acc[j][i][c], sum[j][q][c]);
+              for (int q = 0; q < STEPS; ++q) {
+                if constexpr (EXACT) rest[j][i][c] += add_exactly(acc[j][i][c], sum[j][q][c]);
+                else acc[j][i][c] += sum[j][q][c];
+              }
         }
       }
-      const int buf = turn & 1;
-      mbar_wait(&sums_empty[buf], ((turn >> 1) & 1) ^ 1);
+      const int buf = turn % BUFS;
+      mbar_wait(&sums_empty[buf], ((turn / BUFS) & 1) ^ 1);
       float* mine = sums + (buf * RING_TAKERS + cw) * SLOTS * 32 + lane;
 #pragma unroll
       for (int j = 0; j < NT; ++j)
@@ -864,7 +871,7 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 1) linear_ring_kernel(const _
         for (int i = 0; i < MG; ++i)
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            const float s = acc[j][i][c] + rest[j][i][c];
+            const float s = EXACT ? acc[j][i][c] + rest[EXACT ? j : 0][EXACT ? i : 0][c] : acc[j][i][c];
             mine[((j * MG + i) * 4 + c) * 32] = s == s ? s : acc[j][i][c];      // beside an infinity the rest is NaN
           }
       __syncwarp();
@@ -881,7 +888,7 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 1) linear_ring_kernel(const _
         for (int piece = 0; piece < pieces; ++piece) {
           mbar_wait(&empty[stage], phase ^ 1);
           if (x != nullptr)
-            bulk_load(ring + stage * PIECE + ring_w<AT, NT>() + lane * ring_pair_row<AT>(), x + piece * KC,
+            bulk_load(ring + stage * PIECE + ring_w<AT, NT, MG>() + lane * ring_pair_row<AT, MG>(), x + piece * KC,
                       (uint32_t)(min(KC, a.K - piece * KC) * (int)sizeof(AT)), &full[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -894,8 +901,8 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 1) linear_ring_kernel(const _
     pdl_wait();
     for (int at = blockIdx.x; at < units; at += gridDim.x, ++turn) {
       const Unit u = unit_at(at);
-      const int buf = turn & 1;
-      mbar_wait(&sums_full[buf], (turn >> 1) & 1);
+      const int buf = turn % BUFS;
+      mbar_wait(&sums_full[buf], (turn / BUFS) & 1);
       const float* part = sums + buf * RING_TAKERS * SLOTS * 32;
       for (int e = et; e < cols * u.here; e += RING_STORERS * 32) {
         const int nl = e & (cols - 1), ml = e / cols, n = u.n0 + nl;
@@ -958,7 +965,7 @@ static int launch_stream(const LinArgs& a, int c_fp32, dim3 grid, int warps, int
 
 template <typename AT, int NT, int MG, bool PAIRS>
 static int launch_ring(const LinArgs& a, int c_fp32, int batch, int n_pairs, int n_groups, cudaStream_t stream) {
-  constexpr int KC = ring_kc<AT>(), halves = sizeof(AT) / 2;
+  constexpr int KC = ring_kc<AT, MG>(), halves = sizeof(AT) / 2;
   const int n_out = gated_epi(a.epi) ? a.N / 2 : a.N, per = (gated_epi(a.epi) ? 8 : 16) * NT, problems = PAIRS ? n_groups : batch;
   const long long units = (long long)problems * ((n_out + per - 1) / per);
   // 64 columns of 16 bits, the rows, the blocks of 64, the problems (of A: the segments)
@@ -1005,11 +1012,19 @@ static int dispatch_stream(const LinArgs& a, int a_fp32, int c_fp32, int batch, 
   // rows, operands and problems lie at increasing addresses: what a tensor map can say
   const bool ring_reads = (a.N == 1 || a.ldw > 0) && (a.M == 1 || a.lda > 0) && (problems == 1 || a.w_batch > 0) && (batch == 1 || a.a_batch > 0) &&
                           (a.seg_cols == 0 || a.n_segs == 1 || a.a_seg > 0);
-  if (mg <= 2 && ring_reads && ring_pays && (n_groups > 0 || fp32_pays) && n_groups <= RING_MAX_GROUPS && a.K % 64 == 0 && ring_units < (1LL << 31)) {
+  // 17 to 64 rows: a CTA's rows of A are most of what it brings, so a tile a CTA, or a K long enough (64 rows: K = 1024, N = 1024 9.2, 6.9; K = 4096, N = 1024 24.6, 15.4; K = 2048,
+  // N = 6144, 33 rows 23.9, 21.1; K = 1024, N = 8192 15.6, 16.2; fp32 K = 1024, N = 2048 14.9, 12.7, N = 4096 17.7, 20.8; 32 bf16 rows N = 4096 7.8, 7.1)
+  const bool rows_pay = n_groups == 0 && (ring_units <= sm_count() || (ring_units <= 4 * sm_count() && a.K >= 2048) || (mg == 4 && ring_units <= 2 * sm_count() && a.K >= 1024));
+  if (ring_reads && (mg > 2 ? rows_pay : ring_pays && (n_groups > 0 || fp32_pays)) && n_groups <= RING_MAX_GROUPS && a.K % 64 == 0 && ring_units < (1LL << 31)) {
     const bool two = a_fp32 && ring_units > sm_count() && (a.seg_cols == 0 || a.seg_cols % (2 * per) == 0);
 #define LP_RING(MG, PAIRS)                                                                                                 \
   (!a_fp32 ? launch_ring<bf16, 1, MG, PAIRS>(a, c_fp32, batch, n_pairs, n_groups, stream)                                  \
            : two ? launch_ring<float, 2, MG, PAIRS>(a, c_fp32, batch, n_pairs, n_groups, stream) : launch_ring<float, 1, MG, PAIRS>(a, c_fp32, batch, n_pairs, n_groups, stream))
+    if (mg > 2) {
+#define LP_RING1(MG) (a_fp32 ? launch_ring<float, 1, MG, false>(a, c_fp32, batch, 0, 0, stream) : launch_ring<bf16, 1, MG, false>(a, c_fp32, batch, 0, 0, stream))
+      return mg == 4 ? LP_RING1(4) : LP_RING1(8);
+#undef LP_RING1
+    }
     if (n_groups > 0) return mg == 1 ? LP_RING(1, true) : LP_RING(2, true);
     return mg == 1 ? LP_RING(1, false) : LP_RING(2, false);
 #undef LP_RING

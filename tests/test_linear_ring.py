@@ -1,4 +1,4 @@
-"""The product of up to 16 rows as one stream of weights through a ring of TMA pieces (lp_linear, lp_linear_group_pairs with K a multiple of 64) against a
+"""The product of up to 64 rows as one stream of weights through a ring of TMA pieces (lp_linear, lp_linear_group_pairs with K a multiple of 64) against a
 float64 product: pieces that end within K, tiles that end within N, more tiles than CTAs and more pieces than the ring has places, both operand types, batches,
 segments, gated units, groups whose pairs fill several tiles; weights that may be read early and weights that may not.
 
@@ -16,7 +16,7 @@ F32, BF16 = torch.float32, torch.bfloat16
 
 
 @pytest.mark.parametrize("dtype", [BF16, F32])
-@pytest.mark.parametrize("M,N,K", [(1, 1, 64), (1, 200, 1088), (3, 40, 576), (5, 130, 512), (8, 16, 1600), (8, 300, 64), (9, 33, 640), (16, 130, 448)])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 64), (1, 200, 1088), (3, 40, 576), (5, 130, 512), (8, 16, 1600), (8, 300, 64), (9, 33, 640), (16, 130, 448), (17, 40, 320), (32, 130, 576), (33, 72, 256), (64, 130, 832)])
 @pytest.mark.parametrize("constant", [0, 1])
 def test_rows_tiles_and_pieces(backend, dtype, M, N, K, constant):
     a, w, want, ad, wd = _data(M, N, K, dtype, backend[0])
@@ -29,7 +29,7 @@ def test_rows_tiles_and_pieces(backend, dtype, M, N, K, constant):
 
 
 @pytest.mark.parametrize("dtype", [BF16, F32])
-@pytest.mark.parametrize("M", [3, 12])
+@pytest.mark.parametrize("M", [3, 12, 20, 50])
 def test_gated_and_added(backend, dtype, M):
     N, K = 76, 704
     a, w, z, ad, wd = _data(M, N, K, dtype, backend[0])
@@ -47,7 +47,7 @@ def test_gated_and_added(backend, dtype, M):
 
 
 @pytest.mark.parametrize("dtype", [BF16, F32])
-@pytest.mark.parametrize("M", [2, 11])
+@pytest.mark.parametrize("M", [2, 11, 30, 41])
 def test_batches_and_segments(backend, dtype, M):
     g = torch.Generator().manual_seed(M)
     heads, N, K = 5, 40, 576
