@@ -73,6 +73,8 @@ struct RetArgs {
 
 // floats between rows of keys and queries in shared memory: rows of 16-byte pieces whose neighbours lie four banks further, or rows an odd stride apart
 template <bool WIDE> __host__ __device__ inline int ret_dimp(int dim) { return WIDE ? dim + 4 : ((dim + 3) & ~3) + 1; }
+// the same where the output kernel's products are matrix instructions: four 16-byte pieces of each of two rows lie in different banks
+__host__ __device__ inline int ret_mm_dimp(int dim) { return dim + 16; }
 
 __device__ __forceinline__ float ret_silu(float z) { return z / (1.0f + expf(-z)); }
 // element d of one head's q or k: activation (when asked for), then rotation
@@ -87,9 +89,53 @@ __device__ __forceinline__ float ret_at(const float4& v, int i) { return i == 0 
 
 // one chunk's keys (and queries) of a head into shared memory, rows dimp apart: a thread takes a rotation pair, whose one sine and cosine serve all it
 // holds (an element a thread took an eighth of the kernels' time for them), or a dimension that is not rotated.  kw: a factor of each row's key, or null.
+// MM (heads of whole RET_MM dimensions): a lane keeps its pairs from row to row, no divisions.
+template <bool MM>
 __device__ __forceinline__ void ret_load_keys(const RetArgs& a, int row0, int len, int pos0, int h, int dimp, const float* kw, float* ks, float* qs) {
   const int half = a.in_act ? 0 : min(a.rot_dims, a.dim) >> 1, per = a.dim - half;      // no rotation with an activation
   constexpr int BATCH = 4;      // what a batch reads is asked for before any of it is stored
+  if constexpr (MM) {
+    constexpr int WARPS = RET_CHUNK_THREADS / 32;
+    static_assert(RET_CHUNK == BATCH * WARPS, "a warp's rows are one batch");
+    const int warp = threadIdx.x >> 5;
+    for (int e = threadIdx.x & 31; e < per; e += 32) {
+      const bool turn = e < half;
+      const int d0 = !turn ? half + e : a.rot_layout == LP_ROT_INTERLEAVED ? 2 * e : e, d1 = !turn ? d0 : a.rot_layout == LP_ROT_INTERLEAVED ? 2 * e + 1 : e + half;
+      const float freq = turn ? a.inv_freq[e] : 0.f;
+      float k0[BATCH], k1[BATCH], q0[BATCH], q1[BATCH];
+#pragma unroll
+      for (int n = 0; n < BATCH; ++n) {
+        const int j = warp + n * WARPS;
+        const float* base = a.qkvg + (long long)(row0 + j) * a.ld + h * a.dim;
+        k0[n] = j < len ? base[a.k_off + d0] : 0.f;
+        k1[n] = j < len ? base[a.k_off + d1] : 0.f;
+        q0[n] = j < len && qs != nullptr ? base[a.q_off + d0] : 0.f;
+        q1[n] = j < len && qs != nullptr ? base[a.q_off + d1] : 0.f;
+      }
+#pragma unroll
+      for (int n = 0; n < BATCH; ++n) {
+        const int j = warp + n * WARPS;
+        if (j >= len) break;
+        const float w = kw != nullptr ? kw[j] : 1.f;
+        if (turn) {
+          float sn, cs;
+          sincosf((float)(pos0 + j) * freq, &sn, &cs);
+          sn *= a.rot_mscale;
+          cs *= a.rot_mscale;
+          ks[j * dimp + d0] = (k0[n] * cs - k1[n] * sn) * a.k_scale * w;
+          ks[j * dimp + d1] = (k1[n] * cs + k0[n] * sn) * a.k_scale * w;
+          if (qs != nullptr) {
+            qs[j * dimp + d0] = q0[n] * cs - q1[n] * sn;
+            qs[j * dimp + d1] = q1[n] * cs + q0[n] * sn;
+          }
+        } else {
+          ks[j * dimp + d0] = (a.in_act ? ret_silu(k0[n]) : k0[n]) * a.k_scale * w;
+          if (qs != nullptr) qs[j * dimp + d0] = a.in_act ? ret_silu(q0[n]) : q0[n];
+        }
+      }
+    }
+    return;
+  }
   for (int it0 = threadIdx.x; it0 < len * per; it0 += BATCH * blockDim.x) {
     float k0[BATCH], k1[BATCH], q0[BATCH], q1[BATCH];
 #pragma unroll
@@ -129,9 +175,15 @@ __device__ __forceinline__ void ret_load_keys(const RetArgs& a, int row0, int le
 }
 // `len` rows of vdim columns from column `off` of the projection on, rows ldd apart, copied while other work is done (the caller commits and waits);
 // false: rows are not whole 16-byte pieces, nothing was copied
+template <bool MM>
 __device__ __forceinline__ bool ret_copy_rows(const RetArgs& a, int row0, int len, int off, float* dst, int ldd) {
   if (((a.ld | off | a.vdim | ldd) & 3) != 0 || (reinterpret_cast<uintptr_t>(a.qkvg) & 15) != 0) return false;
   const int per = a.vdim >> 2;
+  if constexpr (MM) {      // a warp a row
+    for (int j = threadIdx.x >> 5; j < len; j += RET_CHUNK_THREADS / 32)
+      for (int c = (threadIdx.x & 31) * 4; c < a.vdim; c += 128) __pipeline_memcpy_async(dst + j * ldd + c, a.qkvg + (long long)(row0 + j) * a.ld + off + c, 16);
+    return true;
+  }
   for (int i = threadIdx.x; i < len * per; i += blockDim.x) {
     const int j = i / per, c = (i % per) * 4;
     __pipeline_memcpy_async(dst + j * ldd + c, a.qkvg + (long long)(row0 + j) * a.ld + off + c, 16);
@@ -139,9 +191,44 @@ __device__ __forceinline__ bool ret_copy_rows(const RetArgs& a, int row0, int le
   return true;
 }
 
+// Heads whose keys and values both have a multiple of RET_MM dimensions take the matrix instruction for the three products of a chunk: both operands
+// in three bf16 terms each (cut3), the six products of weight above 2^-26 with the small ones first, 16 terms of a sum at a time and these added in
+// fp32.  The order of k within such a step is free as long as both sides agree: where a lane's four k are neighbours, it reads them at once.
+// 4,096 rows of 16 heads of 128 x 128 (us, fp32 sums from shared memory and so): the chunks' states 116, 74, the outputs 237, 138; errors against
+// 64 bits 1.2e-7 of the outputs for 2.3e-7.  Both are bound by instructions now (65 % of the issue slots; cutting the operands is a third of them).
+constexpr int RET_MM = 128;
+struct RetRows { uint32_t hi[4], mid[4], lo[4]; };      // 16 x 16: rows g and g + 8 at this lane's four k
+__device__ __forceinline__ RetRows ret_cut_rows(const float4& x, const float4& y) {
+  RetRows r;
+  cut3(x.x, x.y, r.hi[0], r.mid[0], r.lo[0]);
+  cut3(y.x, y.y, r.hi[1], r.mid[1], r.lo[1]);
+  cut3(x.z, x.w, r.hi[2], r.mid[2], r.lo[2]);
+  cut3(y.z, y.w, r.hi[3], r.mid[3], r.lo[3]);
+  return r;
+}
+struct RetColumn { uint32_t hi[2], mid[2], lo[2]; };      // 16 x 8: column g at this lane's four k
+__device__ __forceinline__ RetColumn ret_cut_column(float k0, float k1, float k2, float k3) {
+  RetColumn r;
+  cut3(k0, k1, r.hi[0], r.mid[0], r.lo[0]);
+  cut3(k2, k3, r.hi[1], r.mid[1], r.lo[1]);
+  return r;
+}
+__device__ __forceinline__ void ret_mma(float (&acc)[4], const RetRows& a, const RetColumn& b) {
+  float d[4];
+  mma_bf16_first(d, a.lo[0], a.lo[1], a.lo[2], a.lo[3], b.hi[0], b.hi[1]);
+  mma_bf16(d, a.hi[0], a.hi[1], a.hi[2], a.hi[3], b.lo[0], b.lo[1]);
+  mma_bf16(d, a.mid[0], a.mid[1], a.mid[2], a.mid[3], b.mid[0], b.mid[1]);
+  mma_bf16(d, a.mid[0], a.mid[1], a.mid[2], a.mid[3], b.hi[0], b.hi[1]);
+  mma_bf16(d, a.hi[0], a.hi[1], a.hi[2], a.hi[3], b.mid[0], b.mid[1]);
+  mma_bf16(d, a.hi[0], a.hi[1], a.hi[2], a.hi[3], b.hi[0], b.hi[1]);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) acc[c] += d[c];
+}
+
 // (1) U[chunk][head] = sum_j decay^(len-1-j) k_j v_j^T.  4 x 4 outputs per thread (8 x 8 from 16-byte reads: 208 us for 162); a thread's four columns are vdim/4
-// apart, so that the threads of a warp read consecutive shared-memory words.
-__global__ void __launch_bounds__(RET_CHUNK_THREADS)
+// apart, so that the threads of a warp read consecutive shared-memory words.  MM: two CTAs an SM (three, at 80 registers, spill: 78 us for 74).
+template <bool MM>
+__global__ void __launch_bounds__(RET_CHUNK_THREADS, MM ? 2 : 1)
 retention_chunk_state_kernel(RetArgs a, const int* __restrict__ chunk_seq, const int* __restrict__ chunk_row0, const int* __restrict__ chunk_len,
                              const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0, float* __restrict__ ws) {
   pdl_launch_dependents();
@@ -150,24 +237,69 @@ retention_chunk_state_kernel(RetArgs a, const int* __restrict__ chunk_seq, const
   const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
   const int s = chunk_seq[c], row0 = chunk_row0[c], len = chunk_len[c];
   const int pos0 = seq_pos0[s] + (row0 - seq_row0[s]);
-  const int dimp = ret_dimp<false>(a.dim), vdimp = (a.vdim + 3) & ~3;      // padded rows: whole 4-tiles
+  // padded rows: whole 4-tiles; MM: neighbouring rows eight banks further
+  const int dimp = MM ? a.dim + 8 : ret_dimp<false>(a.dim), vdimp = MM ? a.vdim + 8 : (a.vdim + 3) & ~3;
   float* kd = dyn_smem;                   // [RET_CHUNK][dimp]
   float* vv = kd + RET_CHUNK * dimp;      // [RET_CHUNK][vdimp]
   __shared__ float power[RET_CHUNK];
   if (tid < len) power[tid] = powf(a.decay[h], (float)(len - 1 - tid));
   __syncthreads();
-  const bool copied = !a.in_act && ret_copy_rows(a, row0, len, a.v_off + h * a.vdim, vv, vdimp);
+  const bool copied = !a.in_act && ret_copy_rows<MM>(a, row0, len, a.v_off + h * a.vdim, vv, vdimp);
   __pipeline_commit();
-  for (int i = tid; i < len * (dimp - a.dim); i += blockDim.x) kd[i / (dimp - a.dim) * dimp + a.dim + i % (dimp - a.dim)] = 0.f;
-  ret_load_keys(a, row0, len, pos0, h, dimp, power, kd, nullptr);
+  for (int i = tid; !MM && i < len * (dimp - a.dim); i += blockDim.x) kd[i / (dimp - a.dim) * dimp + a.dim + i % (dimp - a.dim)] = 0.f;
+  ret_load_keys<MM>(a, row0, len, pos0, h, dimp, power, kd, nullptr);
   for (int i = tid; !copied && i < len * vdimp; i += blockDim.x) {
     const int j = i / vdimp, d = i % vdimp;
     vv[i] = d < a.vdim ? ret_v(a, a.qkvg[(long long)(row0 + j) * a.ld + a.v_off + h * a.vdim + d]) : 0.f;
   }
+  if constexpr (MM) {      // rows that the chunk does not have are zeros
+    for (int i = len * dimp + tid; i < RET_CHUNK * dimp; i += blockDim.x) kd[i] = 0.f;
+    for (int i = len * vdimp + tid; i < RET_CHUNK * vdimp; i += blockDim.x) vv[i] = 0.f;
+  }
   __pipeline_wait_prior(0);
   __syncthreads();
   float* U = ws + ((long long)c * a.heads + h) * a.dim * a.vdim;
-  const int tiles_y = vdimp >> 2, tiles_x = (a.dim + 3) >> 2;
+  if constexpr (MM) {      // a warp: 64 dimensions of the keys x 32 columns, whose terms it keeps
+    const int lane = tid & 31, g = lane >> 2, t = lane & 3, halves = a.dim >> 6;
+    bool odd = false;
+    for (int tile = tid >> 5; tile < halves * (a.vdim >> 5); tile += RET_CHUNK_THREADS / 32) {
+      const int x0 = tile % halves * 64, y0 = tile / halves * 32;
+      RetColumn b[RET_CHUNK / 16][4];
+#pragma unroll
+      for (int kb = 0; kb < RET_CHUNK / 16; ++kb) {
+        float4 v[4];
+#pragma unroll
+        for (int n = 0; n < 4; ++n) v[n] = ret_ld4(vv + (kb * 16 + 4 * n + t) * vdimp + y0 + 4 * g);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) b[kb][j] = ret_cut_column(ret_at(v[0], j), ret_at(v[1], j), ret_at(v[2], j), ret_at(v[3], j));
+      }
+#pragma unroll 1
+      for (int i = 0; i < 4; ++i) {
+        float acc[4][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
+#pragma unroll
+        for (int kb = 0; kb < RET_CHUNK / 16; ++kb) {
+          const float* k = kd + (kb * 16 + t) * dimp + x0 + 16 * i + g;
+          const RetRows ka = ret_cut_rows(make_float4(k[0], k[4 * dimp], k[8 * dimp], k[12 * dimp]),
+                                          make_float4(k[8], k[4 * dimp + 8], k[8 * dimp + 8], k[12 * dimp + 8]));
+#pragma unroll
+          for (int j = 0; j < 4; ++j) ret_mma(acc[j], ka, b[kb][j]);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {      // row g or g + 8, column 2 t or 2 t + 1 of the four tiles
+          float* to = U + (long long)(x0 + 16 * i + g + (e >> 1) * 8) * a.vdim + y0 + 8 * t + (e & 1) * 4;
+          *reinterpret_cast<float4*>(to) = make_float4(acc[0][e], acc[1][e], acc[2][e], acc[3][e]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) odd |= not_finite(acc[j][e]);
+        }
+      }
+    }
+    if (!__syncthreads_or(odd)) return;      // the terms of an infinity do not add up to it: such a chunk is taken again below
+  }
+  const int tiles_y = (a.vdim + 3) >> 2, tiles_x = (a.dim + 3) >> 2;
   for (int tile = tid; tile < tiles_x * tiles_y; tile += blockDim.x) {
     const int x0 = (tile / tiles_y) * 4, ty = tile % tiles_y;
     float acc[4][4];
@@ -258,9 +390,9 @@ retention_scan_kernel(RetArgs a, const int* __restrict__ seq_chunk0, const int* 
 // SM and it takes 0.46 ms.  4 x 4 outputs per thread.  The line is what leaves three CTAs an SM; whole prompts on both sides (us, staged up to
 // 200 KB, and so): 16 heads of 128, 4096 tokens 1450, 756, 512 tokens 150, 93; 8 heads of 96 286, 203 and 62, 58; 16 of 80 355, 313 and 59, 57; 8 of
 // 128 keys and 64 values 264, 188 and 60, 61.  64 x 64 is staged on both.  WIDE: the same sums in the same order from 16-byte reads,
-// a quarter as many, values and gates copied in meanwhile: 0.46 -> 0.24 ms.
-template <bool WIDE>
-__global__ void __launch_bounds__(RET_CHUNK_THREADS)
+// a quarter as many, values and gates copied in meanwhile: 0.46 -> 0.24 ms.  MM: matrix instructions, 0.14 ms; the state's terms are cut once.
+template <bool WIDE, bool MM>
+__global__ void __launch_bounds__(RET_CHUNK_THREADS, MM ? 3 : 1)
 retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const int* __restrict__ chunk_row0, const int* __restrict__ chunk_len,
                            const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0, const float* ws, int stage_s) {
   pdl_launch_dependents();
@@ -269,19 +401,22 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
   const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
   const int s = chunk_seq[c], row0 = chunk_row0[c], len = chunk_len[c];
   const int pos0 = seq_pos0[s] + (row0 - seq_row0[s]);
-  const int dimp = ret_dimp<WIDE>(a.dim), vdimp = (a.vdim + 3) & ~3;
+  const int dimp = MM ? ret_mm_dimp(a.dim) : ret_dimp<WIDE>(a.dim), vdimp = (a.vdim + 3) & ~3;
   float* qs = dyn_smem;                        // [RET_CHUNK][dimp]
   float* ks = qs + RET_CHUNK * dimp;           // [RET_CHUNK][dimp]
   float* vv = ks + RET_CHUNK * dimp;           // [RET_CHUNK][vdimp]
   float* os = vv + RET_CHUNK * vdimp;          // [RET_CHUNK][vdimp]
   float* pp = os + RET_CHUNK * vdimp;          // [RET_CHUNK][RET_CHUNK + 1]
-  float* rr = pp + RET_CHUNK * (RET_CHUNK + 1);   // [RET_CHUNK]
-  float* Ss = rr + RET_CHUNK;                  // [dim][vdimp] when stage_s
+  float* power = pp + RET_CHUNK * (RET_CHUNK + 1);   // [RET_CHUNK]: decay^(i + 1)
+  float* Ss = power + RET_CHUNK;               // [dim][vdimp] when stage_s
   const float dec = a.decay[h];
-  const bool copied = !a.in_act && ret_copy_rows(a, row0, len, a.v_off + h * a.vdim, vv, vdimp);
+  if (tid < RET_CHUNK) power[tid] = powf(dec, (float)(tid + 1));
+  const bool copied = !a.in_act && ret_copy_rows<MM>(a, row0, len, a.v_off + h * a.vdim, vv, vdimp);
   __pipeline_commit();
   for (int i = len * dimp + tid; i < RET_CHUNK * dimp; i += blockDim.x) qs[i] = ks[i] = 0.f;
-  ret_load_keys(a, row0, len, pos0, h, dimp, nullptr, ks, qs);
+  if constexpr (MM)
+    for (int i = len * vdimp + tid; i < RET_CHUNK * vdimp; i += blockDim.x) vv[i] = 0.f;
+  ret_load_keys<MM>(a, row0, len, pos0, h, dimp, nullptr, ks, qs);
   for (int i = tid; !copied && i < RET_CHUNK * vdimp; i += blockDim.x) {
     const int j = i / vdimp, d = i % vdimp;
     vv[i] = (j < len && d < a.vdim) ? ret_v(a, a.qkvg[(long long)(row0 + j) * a.ld + a.v_off + h * a.vdim + d]) : 0.f;
@@ -294,8 +429,30 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
     }
   __pipeline_wait_prior(0);
   __syncthreads();
+  bool scored = false;
+  if constexpr (MM) {      // in-chunk scores, a warp: 16 rows x 8 keys
+    const int lane = tid & 31, g = lane >> 2, t = lane & 3, r0 = (tid >> 5 & 1) * 16, j0 = (tid >> 6) * 8;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    if (j0 < r0 + 16) {
+      const float* q = qs + (r0 + g) * dimp + 4 * t;
+      const float* k = ks + (j0 + g) * dimp + 4 * t;
+#pragma unroll 2
+      for (int d = 0; d < a.dim; d += 16) {
+        const float4 kv = ret_ld4(k + d);
+        ret_mma(acc, ret_cut_rows(ret_ld4(q + d), ret_ld4(q + 8 * dimp + d)), ret_cut_column(kv.x, kv.y, kv.z, kv.w));
+      }
+    }
+    bool odd = false;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = r0 + g + (e >> 1) * 8, j = j0 + 2 * t + (e & 1);
+      odd |= not_finite(acc[e]);
+      pp[i * (RET_CHUNK + 1) + j] = (j <= i && i < len) ? acc[e] * (i == j ? 1.f : power[i - j - 1]) : 0.f;
+    }
+    scored = !__syncthreads_or(odd);      // the terms of an infinity do not add up to it: such scores are taken again
+  }
   // in-chunk scores, 2 x 2 per thread (rows i0, i0 + 1, columns tj, tj + 16): every thread has one
-  for (int tile = tid; tile < (RET_CHUNK / 2) * (RET_CHUNK / 2); tile += blockDim.x) {
+  for (int tile = scored ? (RET_CHUNK / 2) * (RET_CHUNK / 2) : tid; tile < (RET_CHUNK / 2) * (RET_CHUNK / 2); tile += blockDim.x) {
     const int i0 = (tile / (RET_CHUNK / 2)) * 2, tj = tile % (RET_CHUNK / 2);
     float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
     if constexpr (WIDE) {
@@ -331,15 +488,80 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
         const int i = i0 + p, j = tj + q * (RET_CHUNK / 2);
-        pp[i * (RET_CHUNK + 1) + j] = (j <= i && i < len) ? acc[p][q] * powf(dec, (float)(i - j)) : 0.f;
+        pp[i * (RET_CHUNK + 1) + j] = (j <= i && i < len) ? acc[p][q] * (i == j ? 1.f : power[i - j - 1]) : 0.f;
       }
   }
   __syncthreads();
   // nobody reads the keys any more: the gates come in their place while the outputs are taken
-  const bool gates = WIDE && a.finish != LP_RET_FINISH_RAW && a.vdim <= dimp && ret_copy_rows(a, row0, len, a.g_off + h * a.vdim, ks, dimp);
+  const bool gates = WIDE && a.finish != LP_RET_FINISH_RAW && a.vdim <= dimp && ret_copy_rows<MM>(a, row0, len, a.g_off + h * a.vdim, ks, dimp);
   __pipeline_commit();
+  bool taken = false;
+  if constexpr (MM) {      // a warp: the chunk's 32 rows x 16 columns, so that the state is read once
+    const int lane = tid & 31, g = lane >> 2, t = lane & 3;
+    bool odd = false;
+    for (int y0 = (tid >> 5) * 16; y0 < a.vdim; y0 += RET_CHUNK_THREADS / 2) {
+      float acc[2][2][4];      // rows 16 i + .., columns 2 c + j of the 16
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
+      const float* from = S + (long long)(4 * t) * a.vdim + y0 + 2 * g;
+      const float* q = qs + g * dimp + 4 * t;
+#pragma unroll 2
+      for (int d = 0; d < a.dim; d += 16) {
+        float2 s2[4];
+#pragma unroll
+        for (int n = 0; n < 4; ++n) s2[n] = *reinterpret_cast<const float2*>(from + (long long)(d + n) * a.vdim);
+        const RetColumn b0 = ret_cut_column(s2[0].x, s2[1].x, s2[2].x, s2[3].x), b1 = ret_cut_column(s2[0].y, s2[1].y, s2[2].y, s2[3].y);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const RetRows w = ret_cut_rows(ret_ld4(q + 16 * i * dimp + d), ret_ld4(q + (16 * i + 8) * dimp + d));
+          ret_mma(acc[i][0], w, b0);
+          ret_mma(acc[i][1], w, b1);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float lo = power[16 * i + g], hi = power[16 * i + g + 8];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          acc[i][j][0] *= lo;
+          acc[i][j][1] *= lo;
+          acc[i][j][2] *= hi;
+          acc[i][j][3] *= hi;
+        }
+      }
+#pragma unroll
+      for (int kb = 0; kb < RET_CHUNK / 16; ++kb) {
+        float2 v2[4];
+#pragma unroll
+        for (int n = 0; n < 4; ++n) v2[n] = *reinterpret_cast<const float2*>(vv + (kb * 16 + 4 * t + n) * vdimp + y0 + 2 * g);
+        const RetColumn b0 = ret_cut_column(v2[0].x, v2[1].x, v2[2].x, v2[3].x), b1 = ret_cut_column(v2[0].y, v2[1].y, v2[2].y, v2[3].y);
+#pragma unroll
+        for (int i = kb; i < 2; ++i) {      // the second half's keys are none of the first half's rows'
+          const float* p = pp + (16 * i + g) * (RET_CHUNK + 1) + kb * 16 + 4 * t;
+          const float* p8 = p + 8 * (RET_CHUNK + 1);
+          const RetRows w = ret_cut_rows(make_float4(p[0], p[1], p[2], p[3]), make_float4(p8[0], p8[1], p8[2], p8[3]));
+          ret_mma(acc[i][0], w, b0);
+          ret_mma(acc[i][1], w, b1);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; e += 2) {      // columns 2 t and 2 t + 1 of both tiles
+          *reinterpret_cast<float4*>(os + (16 * i + g + (e >> 1) * 8) * vdimp + y0 + 4 * t) =
+              make_float4(acc[i][0][e], acc[i][1][e], acc[i][0][e + 1], acc[i][1][e + 1]);
+#pragma unroll
+          for (int j = 0; j < 2; ++j) odd |= not_finite(acc[i][j][e]) || not_finite(acc[i][j][e + 1]);
+        }
+    }
+    taken = !__syncthreads_or(odd);      // as above
+  }
   const int tiles_y = vdimp >> 2, tiles_i = (len + 3) >> 2;
-  for (int tile = tid; tile < tiles_i * tiles_y; tile += blockDim.x) {
+  for (int tile = taken ? tiles_i * tiles_y : tid; tile < tiles_i * tiles_y; tile += blockDim.x) {
     const int i0 = (tile / tiles_y) * 4, ty = tile % tiles_y;
     float acc[4][4];
 #pragma unroll
@@ -380,7 +602,7 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
     }
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
-      const float sc = powf(dec, (float)(i0 + p + 1));
+      const float sc = power[i0 + p];
 #pragma unroll
       for (int q = 0; q < 4; ++q) acc[p][q] *= sc;
     }
@@ -406,34 +628,30 @@ retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const i
 #pragma unroll
       for (int q = 0; q < 4; ++q) os[(i0 + p) * vdimp + (WIDE ? ty * 4 + q : ty + q * tiles_y)] = acc[p][q];
   }
-  __syncthreads();
-  if (a.finish == LP_RET_FINISH_RAW) {      // o itself: what follows it is another kernel's
-    for (int e = tid; e < len * a.vdim; e += blockDim.x) {
-      const int i = e / a.vdim, y = e % a.vdim;
-      const long long o = (long long)(row0 + i) * a.ldo + h * a.vdim + y;
-      if (a.out_fp32) reinterpret_cast<float*>(a.out)[o] = os[i * vdimp + y];
-      else reinterpret_cast<bf16*>(a.out)[o] = __float2bfloat16(os[i * vdimp + y]);
-    }
-    return;
-  }
-  // one warp per row: root mean square over the head's vdim outputs
-  const int warp = tid >> 5, lane = tid & 31, nwarp = blockDim.x >> 5;
-  for (int i = warp; i < len; i += nwarp) {
-    float ss = 0.f;
-    for (int y = lane; y < a.vdim; y += 32) ss = fmaf(os[i * vdimp + y], os[i * vdimp + y], ss);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (lane == 0) rr[i] = 1.0f / sqrtf(ss / (float)a.vdim + a.eps);
-  }
   __pipeline_wait_prior(0);
   __syncthreads();
-  for (int e = tid; e < len * a.vdim; e += blockDim.x) {
-    const int i = e / a.vdim, y = e % a.vdim;
-    const float g = gates ? ks[i * dimp + y] : a.qkvg[(long long)(row0 + i) * a.ld + a.g_off + h * a.vdim + y];
-    const float v = os[i * vdimp + y] * rr[i] * (g / (1.0f + expf(-g)));
-    const long long o = (long long)(row0 + i) * a.ldo + h * a.vdim + y;
-    if (a.out_fp32) reinterpret_cast<float*>(a.out)[o] = v;
-    else reinterpret_cast<bf16*>(a.out)[o] = __float2bfloat16(v);
+  // a warp a row: o itself (what follows it is another kernel's), or over the root mean square of the head's vdim outputs and gated
+  const int warp = tid >> 5, lane = tid & 31;
+  for (int i = warp; i < len; i += RET_CHUNK_THREADS / 32) {
+    const long long o = (long long)(row0 + i) * a.ldo + h * a.vdim;
+    float inv = 1.f;
+    if (a.finish != LP_RET_FINISH_RAW) {
+      float ss = 0.f;
+      for (int y = lane; y < a.vdim; y += 32) ss = fmaf(os[i * vdimp + y], os[i * vdimp + y], ss);
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+      inv = 1.0f / sqrtf(ss / (float)a.vdim + a.eps);
+    }
+#pragma unroll 4
+    for (int y = lane; y < a.vdim; y += 32) {
+      float v = os[i * vdimp + y];
+      if (a.finish != LP_RET_FINISH_RAW) {
+        const float g = gates ? ks[i * dimp + y] : a.qkvg[(long long)(row0 + i) * a.ld + a.g_off + h * a.vdim + y];
+        v = v * inv * (g / (1.0f + expf(-g)));
+      }
+      if (a.out_fp32) reinterpret_cast<float*>(a.out)[o + y] = v;
+      else reinterpret_cast<bf16*>(a.out)[o + y] = __float2bfloat16(v);
+    }
   }
 }
 
@@ -1061,27 +1279,26 @@ extern "C" size_t lp_retention_workspace_bytes(int n_chunks, int heads, int dim,
   return (size_t)n_chunks * heads * dim * vdim * sizeof(float);
 }
 
-static size_t g_smem_chunk_state = 48 * 1024;
-template <bool WIDE>
+template <bool WIDE, bool MM>
 static int launch_ret_prefill(const RetArgs& a, int n_seqs, int n_chunks, const int* seq_row0, const int* seq_pos0, const int* seq_slot, const int* seq_chunk0,
                               const int* chunk_seq, const int* chunk_row0, const int* chunk_len, float* w, cudaStream_t stream) {
-  static size_t have_out = 48 * 1024;
-  const size_t dimp = ret_dimp<WIDE>(a.dim), vdimp = (a.vdim + 3) & ~3;
-  const size_t smem1 = (size_t)RET_CHUNK * (ret_dimp<false>(a.dim) + vdimp) * sizeof(float);
+  static size_t have_out = 48 * 1024, have_state = 48 * 1024;
+  const size_t dimp = MM ? ret_mm_dimp(a.dim) : ret_dimp<WIDE>(a.dim), vdimp = (a.vdim + 3) & ~3;
+  const size_t smem1 = (size_t)RET_CHUNK * (MM ? a.dim + a.vdim + 16 : ret_dimp<false>(a.dim) + vdimp) * sizeof(float);
   size_t smem3 = ((size_t)RET_CHUNK * (2 * dimp + 2 * vdimp) + RET_CHUNK * (RET_CHUNK + 1) + RET_CHUNK) * sizeof(float);
   LP_REQUIRE(smem3 <= 200 * 1024, "lp_retention_prefill: dim=%d vdim=%d do not fit the chunk kernel's shared memory", a.dim, a.vdim);
   const int stage_s = smem3 + (size_t)a.dim * vdimp * sizeof(float) <= 64 * 1024;      // three CTAs an SM keep their operands and the chunk's start state
   if (stage_s) smem3 += (size_t)a.dim * vdimp * sizeof(float);
-  LP_CHECK_CUDA(ensure_smem(retention_chunk_state_kernel, smem1, g_smem_chunk_state));
-  LP_CHECK_CUDA(ensure_smem(retention_chunk_out_kernel<WIDE>, smem3, have_out));
-  LP_CHECK_CUDA(launch_next(retention_chunk_state_kernel, dim3(n_chunks, a.heads), dim3(RET_CHUNK_THREADS), smem1, stream, a, chunk_seq, chunk_row0, chunk_len, seq_row0, seq_pos0, w));
+  LP_CHECK_CUDA(ensure_smem(retention_chunk_state_kernel<MM>, smem1, have_state));
+  LP_CHECK_CUDA((ensure_smem(retention_chunk_out_kernel<WIDE, MM>, smem3, have_out)));
+  LP_CHECK_CUDA(launch_next(retention_chunk_state_kernel<MM>, dim3(n_chunks, a.heads), dim3(RET_CHUNK_THREADS), smem1, stream, a, chunk_seq, chunk_row0, chunk_len, seq_row0, seq_pos0, w));
   LP_CHECK_CUDA(cudaGetLastError());
   constexpr int V = WIDE ? 4 : 1;
   LP_CHECK_CUDA(launch_next(retention_scan_kernel<V>, dim3(n_seqs, a.heads, (a.dim * a.vdim / V + SCAN_THREADS - 1) / SCAN_THREADS), dim3(SCAN_THREADS), 0, stream, 
       a, seq_chunk0, chunk_len, seq_pos0, seq_slot, w));
   LP_CHECK_CUDA(cudaGetLastError());
-  LP_CHECK_CUDA(launch_next(retention_chunk_out_kernel<WIDE>, dim3(n_chunks, a.heads), dim3(RET_CHUNK_THREADS), smem3, stream, a, chunk_seq, chunk_row0, chunk_len, seq_row0, seq_pos0, w,
-                                                                                                  stage_s));
+  LP_CHECK_CUDA((launch_next(retention_chunk_out_kernel<WIDE, MM>, dim3(n_chunks, a.heads), dim3(RET_CHUNK_THREADS), smem3, stream, a, chunk_seq, chunk_row0, chunk_len, seq_row0,
+                             seq_pos0, w, stage_s)));
   LP_CHECK_CUDA(cudaGetLastError());
   note_launch(3);
   return 0;
@@ -1101,8 +1318,13 @@ extern "C" int lp_retention_prefill(const lp_retention_desc* d, int n_seqs, int 
   // 16-byte pieces of the operands, the state and the workspace; the wider padding has to fit too
   const bool wide = d->dim % 8 == 0 && d->vdim % 8 == 0 && d->slot_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(d->state) & 15) == 0 &&
                     (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && ((size_t)RET_CHUNK * 2 * (d->dim + 4 + d->vdim) + RET_CHUNK * (RET_CHUNK + 2)) * sizeof(float) <= 200 * 1024;
-  return wide ? launch_ret_prefill<true>(a, n_seqs, n_chunks, seq_row0, seq_pos0, seq_slot, seq_chunk0, chunk_seq, chunk_row0, chunk_len, w, stream)
-              : launch_ret_prefill<false>(a, n_seqs, n_chunks, seq_row0, seq_pos0, seq_slot, seq_chunk0, chunk_seq, chunk_row0, chunk_len, w, stream);
+  // whole 128s: every warp of both kernels has a tile; narrower heads would leave half of them without (and stay on the fp32 sums)
+  const bool mm = wide && d->dim % RET_MM == 0 && d->vdim % RET_MM == 0 &&
+                  ((size_t)RET_CHUNK * 2 * (ret_mm_dimp(d->dim) + d->vdim) + RET_CHUNK * (RET_CHUNK + 2)) * sizeof(float) <= 200 * 1024;
+  if (mm)
+    return launch_ret_prefill<true, true>(a, n_seqs, n_chunks, seq_row0, seq_pos0, seq_slot, seq_chunk0, chunk_seq, chunk_row0, chunk_len, w, stream);
+  return wide ? launch_ret_prefill<true, false>(a, n_seqs, n_chunks, seq_row0, seq_pos0, seq_slot, seq_chunk0, chunk_seq, chunk_row0, chunk_len, w, stream)
+              : launch_ret_prefill<false, false>(a, n_seqs, n_chunks, seq_row0, seq_pos0, seq_slot, seq_chunk0, chunk_seq, chunk_row0, chunk_len, w, stream);
 }
 
 template <int V>
