@@ -785,7 +785,7 @@ class _Batch:
         parts = [tokens.astype(np.int32), row_seq, row_pos, row0, pos0, slot, table.reshape(-1), np.asarray(c_seq, np.int32),
                  np.asarray(c_row0, np.int32), np.asarray(c_len, np.int32), np.asarray(seq_c0, np.int32)] + sum_tables
         tables = torch.from_numpy(np.concatenate(parts).astype(np.int32, copy=False))
-        want_t = torch.from_numpy(np.asarray(want, np.int32))
+        self._want, self._device = torch.from_numpy(np.asarray(want, np.int32)), eng.device
         self.layout = (n, max_pages, *self.summary_width) if self.decode else None      # fixes the size of every table of a decode batch
         if eng.device.type == "cuda":
             host = tables.pin_memory()
@@ -796,8 +796,6 @@ class _Batch:
                 tables.copy_(host, non_blocking=True)
             else:
                 tables = host.to(eng.device, non_blocking=True)
-            if len(want):
-                want_t = want_t.pin_memory().to(eng.device, non_blocking=True)
         views, o = [], 0
         for p in parts:
             views.append(tables[o:o + len(p)])
@@ -805,8 +803,13 @@ class _Batch:
         (self.tokens, self.row_seq, self.row_pos, self.seq_row0, self.seq_pos0, self.seq_slot, self.page_table, self.chunk_seq,
          self.chunk_row0, self.chunk_len, self.seq_chunk0) = views[:11]
         self.summary_table = views[11:]
-        self.want_rows = want_t
         self._tables = tables
+
+    @property
+    def want_rows(self) -> torch.Tensor:
+        """the wanted rows on the device: copied when asked for, since a replayed step that wants every row does without (a copy and the gap
+        behind it are 4 us of its 170)"""
+        return self._want.pin_memory().to(self._device, non_blocking=True) if self._device.type == "cuda" else self._want
 
 
 # ---------------------------------------------------------------------------------------------------------------- engine
