@@ -46,6 +46,20 @@ def test_a_tile_is_a_head(emu):
     assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("M", [1, 32, 97, 129, 201, 224])
+@pytest.mark.parametrize("pair", [False, True])
+def test_gated_rows_of_a_ragged_block(emu, M, pair):
+    """the rows that are there have the bits they have in a whole block, beside warps and lanes without a row"""
+    g = torch.Generator().manual_seed(M)
+    x, w = torch.randn((256, 72), generator=g).to(BF), (torch.randn((320, 72), generator=g) * 0.1).to(BF)
+    x[M - 1, :] = 0      # a row of zeros that is there
+    seen = []
+    for rows in (256, M):
+        seen.append(torch.full((256, 160), float("nan"), dtype=BF))
+        _gemm_ex(emu, x[:rows], w, seen[-1][:rows], act=3, bn=256, pair=pair, ctas=4)
+    assert torch.equal(seen[0][:M], seen[1][:M]) and bool(seen[1][M:].isnan().all()) and not bool(seen[0].isnan().any())
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("M", [1, 33, 128, 129, 201, 256, 300, 513, 676, 1000])
 @pytest.mark.parametrize("N,K,what", [(4096, 512, "stats"), (1152, 1160, "stats"), (6144, 256, "rope"), (512, 4304, "plain"), (1152, 256, "modulo")])
