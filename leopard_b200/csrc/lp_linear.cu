@@ -9,8 +9,8 @@
 //                      sigmoid(gate[m, n]) (a gated residual branch closes in the store of its last product).
 //                      seg_cols: groups of output columns that read operands of their own (a mixer whose projections see different
 //                      mixes of the stream) in one launch.  `batch` independent problems with element strides (per-head products of latent attention).
-//                      Operands whose rows are whole 16-byte pieces run on the matrix instructions, a weight-streaming kernel for up to 64
-//                      rows and 64 x 128 tiles for more; fp32 rows as three bf16 terms that add up to them exactly.  The others run on
+//                      Operands whose rows are whole 16-byte pieces run on the matrix instructions, weight-streaming kernels for up to 64
+//                      rows (through a TMA ring where rows and sizes allow) and 64 x 128 tiles for more; fp32 rows as three bf16 terms that add up to them exactly.  The others run on
 //                      two fp32-FMA kernels: a 64 x 64 x 16 shared-memory tile kernel, and one with one warp
 //                      per output column for M <= 8 rows (decode: every weight byte is read once, 16-byte loads).
 //   lp_linear_grouped  the same tile kernel over row tiles that each belong to one group (expert): tile t multiplies rows
