@@ -789,6 +789,9 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 1) linear_ring_kernel(const _
     constexpr int XV = sizeof(AT) == 2 ? 1 : 2;      // 16-byte pieces of eight values of a row
     // this lane's piece of a step in the lower half of a 128-byte line; the upper half's is 64 bytes away, either way
     const int w_at = at_row * 128 + (t ^ at_row) * 16;
+    // The columns from K on of a piece are zeros, but for rows of pairs: a bulk copy ends at K and leaves there what was there, maybe a NaN.  K is a multiple of 64, so
+    // where a warp takes more columns its last steps are looked at one by one.
+    constexpr bool ENDS_WITHIN = PAIRS && STEPS * 32 > 64;
     const int x_at = PAIRS ? g * ring_pair_row<AT, MG>() + t * 8 * (int)sizeof(AT) : sizeof(AT) == 2 ? w_at : x_row * 128;
     int stage = 0, turn = 0;
     uint32_t phase = 0;
@@ -823,13 +826,13 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 1) linear_ring_kernel(const _
               if constexpr (PAIRS) x += 8 * i * ring_pair_row<AT, MG>() + step * 32 * (int)sizeof(AT) + x_at + 16 * p;
               else if constexpr (sizeof(AT) == 2) x += i * 8 * KC * 2 + (step >> 1) * 1024 + (x_at ^ upper);
               else x += i * 8 * KC * 4 + step * 1024 + x_at + ((2 * t + p) ^ x_row) * 16;
-              v[q][i][p] = *reinterpret_cast<const uint4*>(x);
+              v[q][i][p] = !ENDS_WITHIN || piece * KC + step * 32 < a.K ? *reinterpret_cast<const uint4*>(x) : make_uint4(0u, 0u, 0u, 0u);
             }
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[stage]);
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
-        if (piece * KC + STEPS * cw * 32 >= a.K) continue;      // the columns from K on of a piece are zeros
+        if (piece * KC + STEPS * cw * 32 >= a.K) continue;      // no column of this warp's
 #pragma unroll
         for (int i = 0; i < MG; ++i) {
           float sum[NT][STEPS][4];

@@ -134,6 +134,13 @@ struct BlockCtx {
 };
 inline BlockCtx* t_ctx = nullptr;
 inline std::function<void()>* g_body = nullptr;
+inline unsigned long long g_block = 0;      // blocks so far
+// what a block finds in its dynamic shared memory is anybody's: NaNs here, whether read as floats or as bf16 (`of`: the block that was last shown them)
+inline void unwritten(void* smem, size_t bytes, unsigned long long& of) {
+  if (of == g_block) return;
+  std::memset(smem, 0xff, bytes);
+  of = g_block;
+}
 inline void fiber_main() {
   (*g_body)();
   t_ctx->block_bar->arrive_and_drop();      // a thread that has returned no longer takes part in __syncthreads
@@ -157,6 +164,7 @@ void launch(dim3 grid, dim3 block, F&& body) {
   gridDim = grid;
   for (unsigned long long b = 0; b < n_blocks; ++b) {
     BlockCtx ctx;
+    ++g_block;
     ctx.block_bar = std::make_unique<Barrier>((int)n);
     for (unsigned w = 0; w < n_warps; ++w) ctx.warp_bar.push_back(std::make_unique<Barrier>((int)std::min(32u, n - w * 32)));
     ctx.warp_buf.assign(n_warps * 32, 0.f);

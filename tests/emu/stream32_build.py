@@ -1,6 +1,6 @@
 """Test infrastructure: builds the 32-bit residual-stream kernel files (lp_linear.cu, lp_stream32.cu, lp_seqmix.cu, lp_winattn.cu, lp_mingru.cu, lp_mlstm.cu, lp_gla.cu, lp_moe.cu — kernels
-AND their host entry points) for the CPU emulator: includes dropped, dynamic shared memory turned into a static buffer, launches
-rewritten (launch_rewrite.py), runtime names from host_emu.h.  The result exports the same C symbols as the native library."""
+AND their host entry points) for the CPU emulator: includes dropped, dynamic shared memory turned into a static buffer that every block
+finds full of NaNs, launches rewritten (launch_rewrite.py), runtime names from host_emu.h.  The result exports the same C symbols as the native library."""
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
@@ -21,7 +21,8 @@ def build_emulated(out: Path) -> Path:
         for line in ('#include "lp_host.h"\n', '#include "../../include/leopard_b200.h"\n'):
             assert line in src, (name, line)
             src = src.replace(line, "")
-        src = src.replace("  extern __shared__ float dyn_smem[];", "  static float dyn_smem[1 << 16];")
+        src = src.replace("  extern __shared__ float dyn_smem[];", "  static float dyn_smem[1 << 16];\n  static unsigned long long dyn_smem_of;\n"
+                          "  emu::unwritten(dyn_smem, sizeof(dyn_smem), dyn_smem_of);")
         assert "extern __shared__" not in src and "asm" not in src, name
         src = rewrite_launches(src)
         assert "<<<" not in src, name

@@ -15,6 +15,14 @@ from test_linear_stream import _call, _data
 F32, BF16 = torch.float32, torch.bfloat16
 
 
+def _leave_nans(backend):
+    """shared memory as a product of NaNs leaves it (the emulated kernels find NaNs in any case)"""
+    if backend[0] == "cuda":
+        a, w = torch.full((64, 1664), float("nan"), dtype=BF16, device="cuda"), torch.full((3200, 1664), float("nan"), dtype=BF16, device="cuda")
+        _call(backend, a, w, torch.empty(64, 3200, device="cuda"), 64)
+        _call(backend, a, w, torch.empty(8, 3200, device="cuda"), 8)
+
+
 @pytest.mark.parametrize("dtype", [BF16, F32])
 @pytest.mark.parametrize("M,N,K", [(1, 1, 64), (1, 200, 1088), (3, 40, 576), (5, 130, 512), (8, 16, 1600), (8, 300, 64), (9, 33, 640), (16, 130, 448), (17, 40, 320), (32, 130, 576), (33, 72, 256), (64, 130, 832)])
 @pytest.mark.parametrize("constant", [0, 1])
@@ -83,6 +91,71 @@ def test_pairs(backend, dtype, n_pairs, groups, a_div):
     _call(backend, ad, wd, out, 1, pairs=of.to(torch.int32).to(backend[0]), groups=groups, a_div=a_div, w_constant=1)
     want = torch.stack([a[z // a_div].double() @ w[int(of[z])].double().T for z in range(n_pairs)])
     assert rel_err(out, want) < 2e-6
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("n_pairs", [1, 4])
+@pytest.mark.parametrize("K", [64, 192, 704, 1088])
+def test_few_pairs_of_any_whole_piece(backend, dtype, n_pairs, K):
+    """up to four pairs take the ring whatever their size: K of odd multiples of 64 ends within what a warp takes of a piece"""
+    g = torch.Generator().manual_seed(K + n_pairs)
+    N, groups = 40, 6
+    a, w = torch.randn(n_pairs, K, generator=g).to(dtype), torch.randn(groups, N, K, generator=g).to(BF16)
+    of = torch.tensor([4, 1, 4, 5], dtype=torch.int32)[:n_pairs]
+    ad, wd = a.to(backend[0]), w.to(backend[0])
+    _leave_nans(backend)
+    out = torch.full((n_pairs, N), 7.0, device=backend[0])
+    _call(backend, ad, wd, out, 1, pairs=of.to(backend[0]), groups=groups)
+    want = torch.stack([a[z].double() @ w[int(of[z])].double().T for z in range(n_pairs)])
+    assert rel_err(out, want) < 2e-6
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("n_pairs,groups,N,K,a_div", [(12, 4, 6000, 704, 1), (24, 4, 6000, 704, 2), (20, 4, 3860, 1088, 4)])
+def test_pairs_in_blocks(backend, dtype, n_pairs, groups, N, K, a_div):
+    """enough weights for the ring: groups of more than 8 and more than 16 pairs (blocks of 8 or of 16 rows each) and groups without any"""
+    assert min(n_pairs, groups) * N * K >= 1 << 24      # the dispatch's line
+    g = torch.Generator().manual_seed(n_pairs)
+    a, w = torch.randn((n_pairs + a_div - 1) // a_div, K, generator=g).to(dtype), torch.randn(groups, N, K, generator=g).to(BF16)
+    of = torch.full((n_pairs,), groups - 1)
+    of[1::7] = 1
+    ad, wd = a.to(backend[0]), w.to(backend[0])
+    _leave_nans(backend)
+    out = torch.full((n_pairs, N), 7.0, device=backend[0])
+    _call(backend, ad, wd, out, 1, pairs=of.to(torch.int32).to(backend[0]), groups=groups, a_div=a_div)
+    want = torch.stack([a[z // a_div].double() @ w[int(of[z])].double().T for z in range(n_pairs)])
+    assert rel_err(out, want) < 2e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("M,N,K", [(1, 2600, 8256), (8, 3200, 5184), (16, 2500, 8256), (13, 5000, 2112), (30, 2400, 5184), (64, 2400, 4160)])
+def test_more_tiles_than_sms_and_more_pieces_than_stages(dtype, M, N, K):
+    """the ring goes round several times within a tile and from tile to tile; fp32 rows with two tiles a piece (149 to 592 tiles).  K / 16 sums that are kept
+    exactly, or for more than 16 rows rounded: below 3e-6 of the result for K <= 8256."""
+    backend = "cuda", None
+    a, w, want, ad, wd = _data(M, N, K, dtype, "cuda")
+    out, again = torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
+    _call(backend, ad, wd, out, M, w_constant=1)
+    assert rel_err(out, want) < 3e-6
+    _call(backend, ad, wd, again, M)
+    assert torch.equal(out, again)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("n_pairs,groups,N,K", [(16, 8, 1000, 5824), (40, 8, 2100, 5824), (100, 50, 712, 1344)])
+def test_pairs_of_many_tiles(dtype, n_pairs, groups, N, K):
+    backend = "cuda", None
+    g = torch.Generator().manual_seed(n_pairs)
+    a, w = torch.randn(n_pairs, K, generator=g).to(dtype), torch.randn(groups, N, K, generator=g).to(BF16)
+    of = torch.randint(0, groups, (n_pairs,), generator=g)
+    ad, wd = a.cuda(), w.cuda()
+    _leave_nans(backend)
+    out = torch.full((n_pairs, N), 7.0, device="cuda")
+    _call(backend, ad, wd, out, 1, pairs=of.to(torch.int32).cuda(), groups=groups)
+    want = torch.stack([a[z].double() @ w[int(of[z])].double().T for z in range(n_pairs)])
+    assert rel_err(out, want) < 3e-6
 
 
 def test_numbers_that_are_not_finite(backend):
