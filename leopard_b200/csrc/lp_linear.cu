@@ -776,7 +776,7 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 1) linear_ring_kernel(const _
       pdl_wait();
     }
     for (; w.u < units; next(w)) {
-      mbar_wait(&empty[stage], phase ^ 1);
+      mbar_wait_warp(&empty[stage], phase ^ 1);      // one lane's copies let the ring go on
       load_w(w, stage);
       load_a(w, stage);
       if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -889,7 +889,7 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 1) linear_ring_kernel(const _
         const Unit u = unit_at(at);
         const AT* const x = lane < u.here ? row_of(u, lane) : nullptr;
         for (int piece = 0; piece < pieces; ++piece) {
-          mbar_wait(&empty[stage], phase ^ 1);
+          mbar_wait_warp(&empty[stage], phase ^ 1);      // as many lanes as there are rows let the ring go on
           if (x != nullptr)
             bulk_load(ring + stage * PIECE + ring_w<AT, NT, MG>() + lane * ring_pair_row<AT, MG>(), x + piece * KC,
                       (uint32_t)(min(KC, a.K - piece * KC) * (int)sizeof(AT)), &full[stage]);

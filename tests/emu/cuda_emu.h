@@ -135,6 +135,7 @@ struct BlockCtx {
 inline BlockCtx* t_ctx = nullptr;
 inline std::function<void()>* g_body = nullptr;
 inline unsigned long long g_block = 0;      // blocks so far
+inline unsigned g_lag_warp = ~0u, g_lag_lane = 0;      // lanes from g_lag_lane on of this warp take a turn only when no other thread of the block gets further
 // what a block finds in its dynamic shared memory is anybody's: NaNs here, whether read as floats or as bf16 (`of`: the block that was last shown them)
 inline void unwritten(void* smem, size_t bytes, unsigned long long& of) {
   if (of == g_block) return;
@@ -172,11 +173,12 @@ void launch(dim3 grid, dim3 block, F&& body) {
     blockIdx = {(unsigned)(b % grid.x), (unsigned)((b / grid.x) % grid.y), (unsigned)(b / ((unsigned long long)grid.x * grid.y))};
     for (auto& f : sched.fibers) f.entered = f.done = false;
     volatile unsigned left = n;
+    volatile bool all = g_lag_warp >= n_warps;
     while (left) {
       const unsigned long long before = sched.progress;
       for (volatile unsigned t = 0; t < n; t = t + 1) {
         Fiber& f = sched.fibers[t];
-        if (f.done) continue;
+        if (f.done || (!all && t >> 5 == g_lag_warp && (t & 31) >= g_lag_lane)) continue;
         sched.current = t;
         threadIdx = {t % block.x, (t / block.x) % block.y, t / (block.x * block.y)};
         if (_setjmp(sched.home) == 0) {
@@ -191,7 +193,10 @@ void launch(dim3 grid, dim3 block, F&& body) {
         }
         if (sched.fibers[t].done) left = left - 1;
       }
-      if (left && sched.progress == before) {
+      const bool stuck = left && sched.progress == before;
+      if (!all || !stuck) {
+        all = g_lag_warp >= n_warps || stuck;
+      } else {
         std::fprintf(stderr, "emu: every remaining thread of a block waits at a barrier that cannot fill\n");
         std::abort();
       }

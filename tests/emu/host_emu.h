@@ -162,6 +162,7 @@ inline void fence_barrier_init() {}
 inline void mbar_arrive(uint64_t* b) { --emu_mbar(b).pending; emu_mbar_turn(emu_mbar(b)); }
 inline void mbar_arrive_expect_tx(uint64_t* b, uint32_t bytes) { emu_mbar(b).bytes += (int32_t)bytes; mbar_arrive(b); }
 inline void mbar_wait(uint64_t* b, uint32_t parity) { while (emu_mbar(b).phase == parity) emu::give_way(); }
+inline void mbar_wait_warp(uint64_t* b, uint32_t parity) { mbar_wait(b, parity); __syncwarp(); }
 inline void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* b) {
   if (((uintptr_t)src & 15) || ((uintptr_t)dst & 15) || bytes % 16) { std::fprintf(stderr, "emu: bulk copy off 16-byte boundaries\n"); std::abort(); }
   std::memcpy(dst, src, bytes);

@@ -4,6 +4,10 @@ segments, gated units, groups whose pairs fill several tiles; weights that may b
 
 Error bounds: as for the weight-streaming kernel, products are exact and K / 16 fp32 sums follow, less than 2e-6 of the result's size for K <= 1600."""
 import ctypes as C
+import os
+import subprocess
+import sys
+from pathlib import Path
 
 import pytest
 import torch
@@ -156,6 +160,24 @@ def test_pairs_of_many_tiles(dtype, n_pairs, groups, N, K):
     _call(backend, ad, wd, out, 1, pairs=of.to(torch.int32).cuda(), groups=groups)
     want = torch.stack([a[z].double() @ w[int(of[z])].double().T for z in range(n_pairs)])
     assert rel_err(out, want) < 3e-6
+
+
+@pytest.mark.parametrize("warp,pairs", [(0, False), (0, True), (13, True), (1, False), (9, False)])
+def test_lanes_that_lag_behind(emu_lib, warp, pairs):
+    """the warps that fill the ring, take the products and add them up: lanes that only look on may run as late as they like (a block that gets stuck ends the process, so it is another one)"""
+    r = subprocess.run([sys.executable, "-c", f"import test_linear_ring as t; t.product_with_lagging_lanes({emu_lib._name!r}, {warp}, {pairs})"],
+                       cwd=Path(__file__).parent, env={**os.environ, "PYTHONPATH": str(Path(__file__).resolve().parents[1])}, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+def product_with_lagging_lanes(path, warp, pairs):
+    """one row, pieces for two rounds of the ring in every CTA"""
+    lib = _lib.bind_stream32(C.CDLL(path))
+    lib.emu_set_lagging(warp, 1)
+    a, w, want, ad, wd = _data(1, 256, 2048, BF16, "cpu")
+    out = torch.empty(1, 256)
+    _call(("cpu", lib), ad, wd[None] if pairs else wd, out, 1, **({"pairs": torch.zeros(1, dtype=torch.int32), "groups": 1} if pairs else {}))
+    assert rel_err(out, want) < 2e-6
 
 
 def test_numbers_that_are_not_finite(backend):
