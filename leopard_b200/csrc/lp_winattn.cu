@@ -289,16 +289,13 @@ window_attn_prep_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const
 // before (an element a thread, with its own division, root and sine): 4,096 rows of 16 + 4 + 4 heads 63 us, now 29 (100 MB).  One row of 32 + 8 + 8 heads beside a stream of weights 7.6, 6.3.
 constexpr int PREP_HEADS = 4, PREP_MAX_WARPS = 16;
 __device__ __forceinline__ float4 win_ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-struct WinTurn { float c[4], s[4]; };      // of a lane's four dimensions; 1 and 0 outside of the rotated ones
+struct WinTurn { float c[4], s[4]; };      // of a lane's four dimensions
 // dimension d + i turns with its partner: x cos + partner sin (the sine of the first of a pair is negative)
 __device__ __forceinline__ WinTurn win_turn(const float* inv_freq, int rot_dims, int layout, float mscale, int pos, int d) {
   WinTurn t;
   const int half = rot_dims >> 1;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    t.c[i] = 1.f;
-    t.s[i] = 0.f;
-  }
+  for (int i = 0; i < 4; ++i) t.c[i] = t.s[i] = 0.f;
   if (d >= rot_dims) return t;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -315,7 +312,7 @@ __device__ __forceinline__ WinTurn win_turn(const float* inv_freq, int rot_dims,
   }
   return t;
 }
-__device__ __forceinline__ float4 win_turned(const WinTurn& t, const float4& x, int rot_dims, int layout) {
+__device__ __forceinline__ float4 win_turned(const WinTurn& t, const float4& x, int rot_dims, int layout, int d) {
   float4 p = make_float4(x.y, x.x, x.w, x.z);
   if (layout != LP_ROT_INTERLEAVED && rot_dims > 0) {      // all lanes of the warp take part
     const int away = rot_dims >> 3;
@@ -324,6 +321,7 @@ __device__ __forceinline__ float4 win_turned(const WinTurn& t, const float4& x, 
     p.z = __shfl_xor_sync(0xffffffffu, x.z, away);
     p.w = __shfl_xor_sync(0xffffffffu, x.w, away);
   }
+  if (d >= rot_dims) return x;      // not turned, whatever the others hold
   return make_float4(fmaf(p.x, t.s[0], x.x * t.c[0]), fmaf(p.y, t.s[1], x.y * t.c[1]), fmaf(p.z, t.s[2], x.z * t.c[2]), fmaf(p.w, t.s[3], x.w * t.c[3]));
 }
 __device__ __forceinline__ float win_head_sum(const float4& v) {
@@ -386,7 +384,7 @@ window_attn_prep_heads_kernel(WinArgs a, int R, const int* __restrict__ row_seq,
       const float4 gn = win_ld4(gain + d);
       y = make_float4(y.x * gn.x, y.y * gn.y, y.z * gn.z, y.w * gn.w);
     }
-    *reinterpret_cast<float4*>((is_q ? x + a.q_off + hl * 128 : crow + hl * 128) + d) = win_turned(turn, y, a.rot_dims, a.rot_layout);
+    *reinterpret_cast<float4*>((is_q ? x + a.q_off + hl * 128 : crow + hl * 128) + d) = win_turned(turn, y, a.rot_dims, a.rot_layout, d);
   }
   if (a.v_is_k) return;
   const int vrot = a.v_inv_freq != nullptr ? a.v_rot_dims : 0;
@@ -396,7 +394,7 @@ window_attn_prep_heads_kernel(WinArgs a, int R, const int* __restrict__ row_seq,
       const float vinv = 1.0f / sqrtf(win_head_sum(y) / 128.0f + a.eps);
       y = make_float4(y.x * vinv, y.y * vinv, y.z * vinv, y.w * vinv);
     }
-    if (vrot > 0) y = win_turned(win_turn(a.v_inv_freq, vrot, a.v_rot_layout, 1.f, pos, d), y, vrot, a.v_rot_layout);
+    if (vrot > 0) y = win_turned(win_turn(a.v_inv_freq, vrot, a.v_rot_layout, 1.f, pos, d), y, vrot, a.v_rot_layout, d);
     *reinterpret_cast<float4*>(crow + a.v_base + g * 128 + d) = y;
   }
 }

@@ -91,3 +91,33 @@ def test_both_kernels(backend, form, R):
             if not f.get("v_is_k"):
                 assert rel_err(rows[:, G * D:], v.flatten(1)) < 2e-6
         assert float((cache == 7.0).float().mean()) >= 1 - (R * roww if kvh else 0) / cache.numel() - 1e-6 and math.isfinite(float(cache.sum()))
+
+
+@pytest.mark.parametrize("layout,rot,value_rot", [(0, 64, 32), (0, 0, 8), (1, 24, 20)])
+def test_dimensions_that_are_not_turned_stay_apart(backend, layout, rot, value_rot):
+    """an infinity or a NaN in one of them is nobody's partner: all others are what they are in the general kernel (the same fp32 products; 1e-6 of the result)"""
+    H, G, R, dev, lib = 4, 2, 2, backend[0], backend[1]
+    L = lib if lib is not None else _lib.stream32_lib()
+    width = (H + 2 * G) * D
+    raw = torch.randn(R, width, generator=torch.Generator().manual_seed(rot))
+    for at, odd in ((100, float("inf")), (D + 127, float("nan")), (H * D + 90, float("-inf")), ((H + G) * D + 120, float("nan")), ((H + G + 1) * D + 33, float("inf"))):
+        raw[1, at] = odd
+    freq, vfreq = (torch.rand(max(n // 2, 1)).to(dev) for n in (rot, value_rot))
+    table, seqs, posd = torch.arange(R, dtype=I32).to(dev), torch.arange(R, dtype=I32).to(dev), torch.full((R,), 5, dtype=I32).to(dev)
+    seen = []
+    for shift in (0, 1):
+        flat = torch.zeros(R * width + 4, dtype=F32)
+        flat[shift: shift + R * width] = raw.flatten()
+        flat, cache = flat.to(dev), torch.zeros(R * 8, 2 * G * D, device=dev)
+        d = _lib.WindowAttnDesc(qkv=flat.data_ptr() + 4 * shift, ld=width, q_off=0, k_off=H * D, v_off=(H + G) * D, heads=H, kv_heads=G, dim=D, vdim=D,
+                                eps=1e-5, inv_freq=_lib.ptr(freq), rot_dims=rot, rot_layout=layout, rot_mscale=1.0, v_inv_freq=_lib.ptr(vfreq),
+                                v_rot_dims=value_rot, v_rot_layout=layout, cache=_lib.ptr(cache), page_size=8, page_table=_lib.ptr(table), max_pages=1, scale=1.0,
+                                out_scale=1.0)
+        stream = C.c_void_p(torch.cuda.current_stream().cuda_stream) if dev != "cpu" else None
+        assert L.lp_window_attn_prep(C.byref(d), R, _lib.ptr(seqs), _lib.ptr(posd), stream) == 0, L.lp_last_error()
+        seen.append(torch.cat([flat.cpu()[shift: shift + R * width], cache.cpu().flatten()]))
+    new, old = seen
+    fine = torch.isfinite(old)
+    assert int((~fine).sum()) == 8      # the five, of which three are in the cache too
+    assert torch.equal(new[~fine].nan_to_num(7.0), old[~fine].nan_to_num(7.0)) and torch.isfinite(new[fine]).all()
+    assert rel_err(new[fine], old[fine].double()) < 1e-6
