@@ -596,7 +596,9 @@ enum lp_rot_layout { LP_ROT_HALF = 0, LP_ROT_INTERLEAVED = 1 };
  * the pair; one problem only).  gate (fp32 [rows of C, ldg], or NULL): the epilogue's result is multiplied by sigmoid(gate[m, n]);
  * problem z of a batch reads gate + z * gate_batch.  seg_cols > 0: output columns [i seg_cols, (i + 1) seg_cols) multiply the operand at
  * A + i * a_seg, the columns from (n_segs - 1) seg_cols on that of the last segment (seg_cols a multiple of 8 for M <= 8 rows, else of 64).
- * w_constant != 0: no call of this library that is still queued on the stream writes W, so that its first pieces may be read before those calls have ended. */
+ * epi | LP_LINEAR_W_CONSTANT (lp_linear only): nothing that is on the stream before this call, and may still run, writes W; its first pieces may be read before
+ * that has ended. */
+#define LP_LINEAR_W_CONSTANT 0x100
 typedef struct lp_linear_desc {
   const void* A; long long lda; long long a_batch; int a_fp32;
   const void* W; long long ldw; long long w_batch;
@@ -607,7 +609,6 @@ typedef struct lp_linear_desc {
   const float* bias; const float* row_scale;
   const float* gate; long long ldg; long long gate_batch;
   int seg_cols, n_segs; long long a_seg;
-  int w_constant;
 } lp_linear_desc;
 int lp_linear(const lp_linear_desc* desc, void* stream);
 /* row tiles of lp_linear_tile_rows() rows, each multiplied by the weight of group tile_group[tile] (w_batch elements apart; < 0: the

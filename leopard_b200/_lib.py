@@ -86,6 +86,7 @@ ROT_HALF, ROT_INTERLEAVED = 0, 1
 RETENTION_CHUNK = 32
 LATENT_SPLIT_ROWS = 16
 GEMM_SPLIT_BF16, GEMM_SPLIT_F32, GEMM_SPLIT_PLANES = 0, 1, 2
+LINEAR_W_CONSTANT = 0x100      # lp_linear: with an epilogue, for weights that nothing on the stream writes
 LINEAR_ROWS_MAX, LINEAR_ROWS_COLS = 8, 8      # lp_linear: up to this many rows stream the weights, a CTA to so many columns
 
 
@@ -94,7 +95,7 @@ class LinearDesc(C.Structure):
     _fields_ = [("A", _vp), ("lda", _ll), ("a_batch", _ll), ("a_fp32", _i), ("W", _vp), ("ldw", _ll), ("w_batch", _ll), ("C", _vp),
                 ("ldc", _ll), ("c_batch", _ll), ("c_fp32", _i), ("M", _i), ("N", _i), ("K", _i), ("batch", _i), ("epi", _i),
                 ("epi_a", _f), ("epi_b", _f), ("c_accum", _i), ("c_scale", _f), ("bias", _vp), ("row_scale", _vp), ("gate", _vp), ("ldg", _ll),
-                ("gate_batch", _ll), ("seg_cols", _i), ("n_segs", _i), ("a_seg", _ll), ("w_constant", _i)]
+                ("gate_batch", _ll), ("seg_cols", _i), ("n_segs", _i), ("a_seg", _ll)]
 
 
 class WindowAttnDesc(C.Structure):

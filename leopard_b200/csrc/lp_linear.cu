@@ -44,7 +44,7 @@ struct LinArgs {
   const float* bias;      // [N] added to the accumulators before the epilogue, or NULL
   const float* row_scale; // [rows of C] multiplies the accumulators before the bias, or NULL
   int seg_cols, n_segs; long long a_seg;   // seg_cols > 0: output columns [i seg_cols, (i + 1) seg_cols) read A + i a_seg (the last of n_segs: all that follow)
-  int w_constant;         // W is not written by launches that may still run: its first pieces are asked for before they have ended
+  int w_constant;         // nothing that may still run writes W (LP_LINEAR_W_CONSTANT): its first pieces are asked for before the launch before has ended
   const float* gate; long long ldg, gate_batch;   // [rows of C, N'] pre-activations: the result is multiplied by sigmoid(gate), or NULL
 };
 
@@ -1318,24 +1318,25 @@ extern "C" int lp_linear(const lp_linear_desc* d, void* stream_) {
   LP_REQUIRE(d != nullptr && d->A != nullptr && d->W != nullptr && d->C != nullptr, "lp_linear: null operand");
   LP_REQUIRE(d->M >= 0 && d->N > 0 && d->K > 0 && d->batch >= 1, "lp_linear: bad problem M=%d N=%d K=%d batch=%d", d->M, d->N, d->K,
              d->batch);
-  LP_REQUIRE(d->epi >= LP_EPI_NONE && d->epi <= LP_EPI_GELU_GATE, "lp_linear: bad epilogue %d", d->epi);
-  LP_REQUIRE(!gated_epi(d->epi) || d->N % 2 == 0, "lp_linear: the gated epilogue needs an even N (gate rows, then up rows)");
+  const int epi = d->epi & ~LP_LINEAR_W_CONSTANT;
+  LP_REQUIRE(epi >= LP_EPI_NONE && epi <= LP_EPI_GELU_GATE, "lp_linear: bad epilogue %d", d->epi);
+  LP_REQUIRE(!gated_epi(epi) || d->N % 2 == 0, "lp_linear: the gated epilogue needs an even N (gate rows, then up rows)");
   if (d->M == 0) return 0;
   LinArgs a;
   a.A = d->A; a.lda = d->lda; a.a_batch = d->a_batch;
   a.W = reinterpret_cast<const bf16*>(d->W); a.ldw = d->ldw; a.w_batch = d->w_batch;
   a.C = d->C; a.ldc = d->ldc; a.c_batch = d->c_batch;
   a.M = d->M; a.N = d->N; a.K = d->K;
-  a.epi = d->epi; a.e0 = d->epi_a; a.e1 = d->epi_b; a.c_accum = d->c_accum; a.c_scale = d->c_scale;
+  a.epi = epi; a.e0 = d->epi_a; a.e1 = d->epi_b; a.c_accum = d->c_accum; a.c_scale = d->c_scale;
   a.a_rows = nullptr; a.tile_group = nullptr; a.z_group = nullptr; a.a_div = 1;
   a.bias = d->bias; a.row_scale = d->row_scale; a.gate = d->gate; a.ldg = d->ldg; a.gate_batch = d->gate_batch;
   a.seg_cols = d->seg_cols; a.n_segs = d->n_segs; a.a_seg = d->a_seg;
-  a.w_constant = d->w_constant;
+  a.w_constant = d->epi & LP_LINEAR_W_CONSTANT;
   LP_REQUIRE(d->batch == 1 || (d->bias == nullptr && d->row_scale == nullptr), "lp_linear: bias and row scale are for one problem");
   // a CTA's columns read one operand: 8 columns for few rows, a tile otherwise
   LP_REQUIRE(d->seg_cols == 0 || (d->seg_cols > 0 && d->n_segs >= 1 && d->seg_cols % (d->M <= ROWS_MAX ? ROWS_WARPS : LIN_BN) == 0),
              "lp_linear: column segments of %d do not fit the CTAs of a product of %d rows", d->seg_cols, d->M);
-  LP_REQUIRE(d->seg_cols == 0 || !gated_epi(d->epi), "lp_linear: a gated unit has one operand");
+  LP_REQUIRE(d->seg_cols == 0 || !gated_epi(epi), "lp_linear: a gated unit has one operand");
   if (d->M <= STREAM_MAX_ROWS && stream_ok(a, d->a_fp32, d->batch) && (d->seg_cols == 0 || d->seg_cols % 16 == 0) && stream_pays(a, d->a_fp32))
     return dispatch_stream(a, d->a_fp32, d->c_fp32, d->batch, d->M, 0, 0, stream);
   // the tile kernel on the matrix instructions; operands without 16-byte rows stay on fp32 FMAs
@@ -1361,7 +1362,7 @@ static int linear_pairs(const lp_linear_desc* d, const int* pair_group, int n_gr
   a.epi = d->epi; a.e0 = d->epi_a; a.e1 = d->epi_b; a.c_accum = d->c_accum; a.c_scale = d->c_scale;
   a.a_rows = nullptr; a.tile_group = nullptr; a.z_group = pair_group; a.a_div = a_div;
   a.bias = d->bias; a.row_scale = d->row_scale; a.gate = d->gate; a.ldg = d->ldg; a.gate_batch = d->gate_batch;
-  a.seg_cols = 0; a.n_segs = 0; a.a_seg = 0; a.w_constant = d->w_constant;
+  a.seg_cols = 0; a.n_segs = 0; a.a_seg = 0; a.w_constant = 0;
   // with the number of groups a group's weights are read once for all of its pairs
   if (n_groups > 0 && n_pairs <= STREAM_MAX_PAIRS && stream_ok(a, d->a_fp32, 1))
     return dispatch_stream(a, d->a_fp32, d->c_fp32, 1, 2 * ((n_pairs + n_groups - 1) / n_groups), n_groups, n_pairs, stream);
@@ -1397,7 +1398,7 @@ extern "C" int lp_linear_grouped(const lp_linear_desc* d, const int* tile_group,
   a.epi = d->epi; a.e0 = d->epi_a; a.e1 = d->epi_b; a.c_accum = d->c_accum; a.c_scale = d->c_scale;
   a.a_rows = a_rows; a.tile_group = tile_group; a.z_group = nullptr; a.a_div = 1;
   a.bias = d->bias; a.row_scale = d->row_scale; a.gate = d->gate; a.ldg = d->ldg; a.gate_batch = d->gate_batch;
-  a.seg_cols = 0; a.n_segs = 0; a.a_seg = 0; a.w_constant = d->w_constant;
+  a.seg_cols = 0; a.n_segs = 0; a.a_seg = 0; a.w_constant = 0;
   if (stream_ok(a, d->a_fp32, 1) && mma_pays(a, 1, n_tiles)) return dispatch_mma(a, d->a_fp32, d->c_fp32, 1, n_tiles, stream);
   return dispatch_linear(a, d->a_fp32, d->c_fp32, 1, n_tiles, false, stream);
 }

@@ -985,9 +985,9 @@ class SeqLMEngine:
                 self._check(rc, "lp_axpy_f32")
                 return x
             d = _lib.LinearDesc(A=_lib.ptr(a), lda=a.stride(0), a_batch=0, a_fp32=int(a.dtype == F32), W=_lib.ptr(w), ldw=w.stride(0),
-                                w_batch=0, C=_lib.ptr(x), ldc=x.stride(0), c_batch=0, c_fp32=1, M=M, N=N, K=K, batch=1, epi=epi,
+                                w_batch=0, C=_lib.ptr(x), ldc=x.stride(0), c_batch=0, c_fp32=1, M=M, N=N, K=K, batch=1, epi=epi | _lib.LINEAR_W_CONSTANT,
                                 epi_a=epi_a, epi_b=epi_b, c_accum=1, c_scale=float(mult), bias=_lib.ptr(bias), row_scale=_lib.ptr(row_scale),
-                                gate=_lib.ptr(gate), ldg=gate.stride(0) if gate is not None else 0, w_constant=1)
+                                gate=_lib.ptr(gate), ldg=gate.stride(0) if gate is not None else 0)
             self._check(self.L.lp_linear(C.byref(d), self._stream()), "lp_linear")
             return x
         if out is None:
@@ -1012,7 +1012,7 @@ class SeqLMEngine:
             return out
         d = _lib.LinearDesc(A=_lib.ptr(a), lda=a.stride(0), a_batch=0, a_fp32=int(a.dtype == F32), W=_lib.ptr(w), ldw=w.stride(0),
                             w_batch=0, C=_lib.ptr(out), ldc=out.stride(0), c_batch=0, c_fp32=int(out.dtype == F32), M=M, N=N, K=K,
-                            batch=1, epi=epi, epi_a=epi_a, epi_b=epi_b, bias=_lib.ptr(bias), row_scale=_lib.ptr(row_scale), w_constant=1)
+                            batch=1, epi=epi | _lib.LINEAR_W_CONSTANT, epi_a=epi_a, epi_b=epi_b, bias=_lib.ptr(bias), row_scale=_lib.ptr(row_scale))
         self._check(self.L.lp_linear(C.byref(d), self._stream()), "lp_linear")
         return out
 
@@ -1040,8 +1040,8 @@ class SeqLMEngine:
         heads, N, K = w.shape
         d = _lib.LinearDesc(A=_lib.ptr(a), lda=a.stride(0), a_batch=a_head, a_fp32=int(a.dtype == F32), W=_lib.ptr(w), ldw=w.stride(1),
                             w_batch=w.stride(0), C=_lib.ptr(out), ldc=out.stride(0), c_batch=out_head, c_fp32=int(out.dtype == F32),
-                            M=a.shape[0], N=N, K=K, batch=heads, epi=_lib.EPI_NONE, epi_a=0.0, epi_b=0.0, gate=_lib.ptr(gate),
-                            ldg=gate.stride(0) if gate is not None else 0, gate_batch=N, w_constant=1)
+                            M=a.shape[0], N=N, K=K, batch=heads, epi=_lib.EPI_NONE | _lib.LINEAR_W_CONSTANT, epi_a=0.0, epi_b=0.0, gate=_lib.ptr(gate),
+                            ldg=gate.stride(0) if gate is not None else 0, gate_batch=N)
         self._check(self.L.lp_linear(C.byref(d), self._stream()), "lp_linear")
         return out
 

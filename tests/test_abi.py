@@ -53,11 +53,17 @@ def test_struct_layouts_match_header(tmp_path):
             assert int(got[f"{cname}.{fname}"]) == getattr(ct, fname).offset, f"{cname}.{fname}"
 
 
+def test_descriptors_that_callers_were_built_with():
+    """a caller of version 3 passes the linear descriptor as it was: it ends with the distance of the column segments, 176 bytes in all"""
+    from leopard_b200 import _lib
+    assert _lib.LinearDesc._fields_[-1][0] == "a_seg" and C.sizeof(_lib.LinearDesc) == 176
+
+
 def test_constants_match_header():
     from leopard_b200 import _lib
     txt = (ROOT / "include" / "leopard_b200.h").read_text()
-    for name in ("RETENTION_CHUNK", "LATENT_SPLIT_ROWS"):
-        assert getattr(_lib, name) == int(re.search(rf"#define LP_{name} (\d+)", txt)[1]), name
+    for name in ("RETENTION_CHUNK", "LATENT_SPLIT_ROWS", "LINEAR_W_CONSTANT"):
+        assert getattr(_lib, name) == int(re.search(rf"#define LP_{name} (\w+)", txt)[1], 0), name
 
 
 def test_argument_errors_are_status_codes(native_lib):

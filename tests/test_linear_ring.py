@@ -33,10 +33,10 @@ def _leave_nans(backend):
 def test_rows_tiles_and_pieces(backend, dtype, M, N, K, constant):
     a, w, want, ad, wd = _data(M, N, K, dtype, backend[0])
     out = torch.empty(M, N, device=backend[0])
-    _call(backend, ad, wd, out, M, w_constant=constant)
+    _call(backend, ad, wd, out, M, constant=constant)
     assert rel_err(out, want) < 2e-6
     again = torch.empty(M, N, device=backend[0])
-    _call(backend, ad, wd, again, M, w_constant=1 - constant)
+    _call(backend, ad, wd, again, M, constant=1 - constant)
     assert torch.equal(out, again)
 
 
@@ -46,14 +46,14 @@ def test_gated_and_added(backend, dtype, M):
     N, K = 76, 704
     a, w, z, ad, wd = _data(M, N, K, dtype, backend[0])
     half = torch.empty(M, N // 2, device=backend[0])
-    _call(backend, ad, wd, half, M, epi=_lib.EPI_SILU_GATE, w_constant=1)
+    _call(backend, ad, wd, half, M, epi=_lib.EPI_SILU_GATE, constant=1)
     p, q = z[:, : N // 2], z[:, N // 2:]
     assert rel_err(half, p * torch.sigmoid(p) * q) < 5e-6      # the unit's slope is below 1.1, its factors carry one error each
     g = torch.Generator().manual_seed(1)
     bias, scale, gate, x = torch.randn(N, generator=g), torch.rand(M, generator=g), torch.randn(M, N, generator=g), torch.randn(M, N, generator=g)
     out = x.clone().to(backend[0])
     _call(backend, ad, wd, out, M, bias=bias.to(backend[0]), row_scale=scale.to(backend[0]), gate=gate.to(backend[0]), ldg=N, epi=_lib.EPI_RELU2,
-          c_accum=1, c_scale=0.5, w_constant=1)
+          c_accum=1, c_scale=0.5, constant=1)
     v = torch.relu(z * scale.double()[:, None] + bias.double()) ** 2 * torch.sigmoid(gate.double())
     assert rel_err(out, x.double() + 0.5 * v) < 2e-6
 
@@ -66,17 +66,17 @@ def test_batches_and_segments(backend, dtype, M):
     a, w = torch.randn(M, heads * (K + 8), generator=g).to(dtype), torch.randn(heads, N, K, generator=g).to(BF16)
     ad, wd = a.to(backend[0]), w.to(backend[0])
     out = torch.empty(M, heads * N, device=backend[0])
-    _call(backend, ad, wd, out, M, batch=heads, a_batch=K + 8, c_batch=N, w_constant=1)
+    _call(backend, ad, wd, out, M, batch=heads, a_batch=K + 8, c_batch=N, constant=1)
     want = torch.cat([a[:, h * (K + 8): h * (K + 8) + K].double() @ w[h].double().T for h in range(heads)], 1)
     assert rel_err(out, want) < 2e-6
-    _call(backend, ad, wd, out, M, batch=heads, a_batch=0, c_batch=N, w_constant=1)      # one operand for all problems: not a tensor map's stride
+    _call(backend, ad, wd, out, M, batch=heads, a_batch=0, c_batch=N, constant=1)      # one operand for all problems: not a tensor map's stride
     want = torch.cat([a[:, :K].double() @ w[h].double().T for h in range(heads)], 1)
     assert rel_err(out, want) < 2e-6
     segs, seg, N = 3, 64, 200
     a, w = torch.randn(segs, M, K, generator=g).to(dtype), torch.randn(N, K, generator=g).to(BF16)
     ad, wd = a.to(backend[0]), w.to(backend[0])
     out = torch.empty(M, N, device=backend[0])
-    _call(backend, ad, wd, out, M, seg_cols=seg, n_segs=segs, a_seg=M * K, w_constant=1)
+    _call(backend, ad, wd, out, M, seg_cols=seg, n_segs=segs, a_seg=M * K, constant=1)
     which = [min(n // seg, segs - 1) for n in range(N)]
     want = torch.stack([a[i].double() @ w[n].double() for n, i in enumerate(which)], 1)
     assert rel_err(out, want) < 2e-6
@@ -92,7 +92,7 @@ def test_pairs(backend, dtype, n_pairs, groups, a_div):
     of[: n_pairs // 2] = groups - 1      # more than a tile's rows in one group, groups without pairs
     ad, wd = a.to(backend[0]), w.to(backend[0])
     out = torch.full((n_pairs, N), 7.0, device=backend[0])
-    _call(backend, ad, wd, out, 1, pairs=of.to(torch.int32).to(backend[0]), groups=groups, a_div=a_div, w_constant=1)
+    _call(backend, ad, wd, out, 1, pairs=of.to(torch.int32).to(backend[0]), groups=groups, a_div=a_div)
     want = torch.stack([a[z // a_div].double() @ w[int(of[z])].double().T for z in range(n_pairs)])
     assert rel_err(out, want) < 2e-6
 
@@ -140,7 +140,7 @@ def test_more_tiles_than_sms_and_more_pieces_than_stages(dtype, M, N, K):
     backend = "cuda", None
     a, w, want, ad, wd = _data(M, N, K, dtype, "cuda")
     out, again = torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
-    _call(backend, ad, wd, out, M, w_constant=1)
+    _call(backend, ad, wd, out, M, constant=1)
     assert rel_err(out, want) < 3e-6
     _call(backend, ad, wd, again, M)
     assert torch.equal(out, again)
@@ -190,7 +190,7 @@ def test_numbers_that_are_not_finite(backend):
     w[7, 600] = 0.0
     want = a.double() @ w.double().T
     out = torch.empty(M, N, device=backend[0])
-    _call(backend, a.to(backend[0]), w.to(backend[0]), out, M, w_constant=1)
+    _call(backend, a.to(backend[0]), w.to(backend[0]), out, M, constant=1)
     out = out.cpu().double()
     fine = torch.isfinite(want)
     assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(out[torch.isinf(want)], want[torch.isinf(want)])

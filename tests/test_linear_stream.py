@@ -19,12 +19,14 @@ def _lib_of(backend):
     return backend[1] if backend[1] is not None else _lib.stream32_lib()
 
 
-def _call(backend, a, w, out, M, batch=1, pairs=None, groups=None, a_div=1, **kw):
+def _call(backend, a, w, out, M, batch=1, pairs=None, groups=None, a_div=1, constant=0, **kw):
     L = _lib_of(backend)
     stream = C.c_void_p(torch.cuda.current_stream().cuda_stream) if a.is_cuda else None
     d = _lib.LinearDesc(A=_lib.ptr(a), lda=a.stride(-2), a_batch=kw.pop("a_batch", 0), a_fp32=int(a.dtype == F32), W=_lib.ptr(w), ldw=w.stride(-2),
                         w_batch=w.stride(0) if w.dim() == 3 else 0, C=_lib.ptr(out), ldc=out.stride(0), c_batch=kw.pop("c_batch", 0),
                         c_fp32=int(out.dtype == F32), M=M, N=w.shape[-2], K=w.shape[-1], batch=batch, **{k: _lib.ptr(v) if isinstance(v, torch.Tensor) else v for k, v in kw.items()})
+    if constant:
+        d.epi |= _lib.LINEAR_W_CONSTANT
     if pairs is None:
         rc = L.lp_linear(C.byref(d), stream)
     elif groups is None:
