@@ -42,8 +42,9 @@ typedef __nv_bfloat16 bf16;
 
 __global__ void embed_rows_f32_kernel(const int* ids, int R, const bf16* __restrict__ table, long long ldt, int vocab,
                                       float scale, float* __restrict__ out, long long ldo, int D) {
-  pdl_launch_dependents();
+  // a step's first launch: the products after it read their weights before they wait, so none of them starts before all that wrote weights has ended
   pdl_wait();
+  pdl_launch_dependents();
   const int r = blockIdx.x;
   if (r >= R) return;
   int id = ids[r];
