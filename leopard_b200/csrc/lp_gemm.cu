@@ -420,12 +420,12 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       if (!swiglu) {
         const int c_begin = c_begin_n, c_end = c_end_n;
         // RoPE tiles: column i of a 128-column head pairs with i + 64.  BN = 256: each warpgroup owns a head = chunks c_begin .. c_begin + 3; BN = 128: the tile is a
-        // head, each warpgroup takes one of its two pairs of chunks
+        // head, each warpgroup takes one of its two pairs of chunks, or the first both where it adds up the row's statistics
         const bool rope_tile = (BN == 256 || BN == 128) && args.rope_heads > 0 && ((n0 >> 7) + (BN == 256 ? wg : 0)) < args.rope_heads;
         if (rope_tile) {
           const int head0 = BN == 256 ? c_begin : 0;
 #pragma unroll 1
-          for (int p = BN == 256 ? 0 : wg; p < (BN == 256 ? 2 : wg + 1); ++p) {
+          for (int p = BN == 256 || one_wg ? 0 : wg; p < (BN == 256 ? 2 : one_wg ? 2 - 2 * wg : wg + 1); ++p) {
             uint32_t rl[32], rh[32];
             LP_TMEM_LD_32(rl, taddr0 + (head0 + p) * 32);
             LP_TMEM_LD_32(rh, taddr0 + (head0 + p + 2) * 32);

@@ -46,6 +46,27 @@ def test_a_tile_is_a_head(emu):
     assert torch.equal(outs[0], outs[1])
 
 
+def test_statistics_of_rotated_heads(emu):
+    """row statistics of heads that are rotated, and of those that are not"""
+    M, K, heads, rot = 140, 72, 5, 3
+    g = torch.Generator().manual_seed(6)
+    x = torch.randn((M, K), generator=g).to(BF)
+    w = (torch.randn((heads * 128, K), generator=g) * K ** -0.5).to(BF)
+    ang = torch.rand((M, 64), generator=g) * 6.28
+    cos, sin, parts, seen = ang.cos().contiguous(), ang.sin().contiguous(), 6, []
+    for bn, pair in ((256, False), (128, True), (128, False)):
+        out, st = torch.full((M, heads * 128), float("nan"), dtype=BF), torch.full((M, parts, 2), float("nan"))
+        emu.emu_gemm_set_stat_256(1)
+        try:
+            _gemm_ex(emu, x, w, out, bn=bn, pair=pair, ctas=4, fx=_Fx(stats_out=st.data_ptr(), rope_cos=cos.data_ptr(), rope_sin=sin.data_ptr(), rope_heads=rot))
+        finally:
+            emu.emu_gemm_set_stat_256(0)
+        seen.append((out, st))
+    assert all(torch.equal(o, seen[0][0]) and torch.equal(s, seen[0][1]) for o, s in seen)
+    y = seen[0][0].float().view(M, heads, 128)
+    assert torch.allclose(seen[0][1][:, :heads, 0], y.sum(2), atol=1e-3) and torch.allclose(seen[0][1][:, :heads, 1], (y * y).sum(2), rtol=1e-5)      # 128 fp32 additions
+
+
 @pytest.mark.parametrize("M", [1, 32, 97, 129, 201, 224])
 @pytest.mark.parametrize("pair", [False, True])
 def test_gated_rows_of_a_ragged_block(emu, M, pair):
@@ -62,7 +83,7 @@ def test_gated_rows_of_a_ragged_block(emu, M, pair):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("M", [1, 33, 128, 129, 201, 256, 300, 513, 676, 1000])
-@pytest.mark.parametrize("N,K,what", [(4096, 512, "stats"), (1152, 1160, "stats"), (6144, 256, "rope"), (512, 4304, "plain"), (1152, 256, "modulo")])
+@pytest.mark.parametrize("N,K,what", [(4096, 512, "stats"), (1152, 1160, "stats"), (6144, 256, "rope"), (512, 4304, "plain"), (1152, 256, "modulo"), (1408, 256, "rope, stats")])
 def test_dispatch_keeps_the_bits(native_lib, M, N, K, what):
     from leopard_b200 import _lib
     L = _lib.lib()
@@ -79,7 +100,9 @@ def test_dispatch_keeps_the_bits(native_lib, M, N, K, what):
         if what in ("stats", "modulo"):
             d.residual, d.ldr, d.block_n, d.stats_out, d.stats_out_parts = r.data_ptr(), N, 256, st.data_ptr(), parts
             d.res_row_mod = 17 if what == "modulo" else 0
-        if what == "rope":
+        if what == "rope, stats":
+            d.stats_out, d.stats_out_parts = st.data_ptr(), parts
+        if what[:4] == "rope":
             d.rope_cos, d.rope_sin, d.rope_heads = cos.data_ptr(), sin.data_ptr(), N // 128 - 8
         old = L.lp_gemm_set_pair_mode(mode)
         try:
@@ -88,7 +111,7 @@ def test_dispatch_keeps_the_bits(native_lib, M, N, K, what):
             L.lp_gemm_set_pair_mode(old)
         seen.append((out, st))
     assert torch.equal(seen[0][0], seen[1][0]) and not bool(torch.isnan(seen[1][0].float()).any())
-    if what in ("stats", "modulo"):
+    if "stats" in what or what == "modulo":
         assert torch.equal(seen[0][1], seen[1][1])
     if what == "plain":
         want = a.float() @ w.float().T
