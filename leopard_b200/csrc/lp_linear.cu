@@ -1012,9 +1012,10 @@ static int dispatch_stream(const LinArgs& a, int a_fp32, int c_fp32, int batch, 
   // 2048 x 4096, 32 pairs 67, 59; 8 of 1024 x 1024, 16 pairs 6.1, 7.1 (the sorting of the pairs is not hidden).
   const bool fp32_pays = !a_fp32 || (mg == 1 ? ring_pairs <= sm_count() || 2 * ring_pairs > 3 * sm_count() : ring_units > sm_count() && ring_units <= 4 * sm_count());
   const bool ring_pays = n_groups > 0 ? n_pairs <= 4 || (long long)(n_pairs < n_groups ? n_pairs : n_groups) * a.N * a.K >= (1 << 24) : a.K >= (mg == 1 ? 512 : 2048) || ring_units <= sm_count();
-  // rows, operands and problems lie at increasing addresses: what a tensor map can say
-  const bool ring_reads = (a.N == 1 || a.ldw > 0) && (a.M == 1 || a.lda > 0) && (problems == 1 || a.w_batch > 0) && (batch == 1 || a.a_batch > 0) &&
-                          (a.seg_cols == 0 || a.n_segs == 1 || a.a_seg > 0);
+  // rows, operands and problems lie at increasing addresses less than 2^40 bytes apart: what a tensor map can say
+  auto follows = [](long long count, long long elements) { return count == 1 || (elements > 0 && elements < (1LL << 38)); };
+  const bool ring_reads = follows(a.N, a.ldw) && follows(a.M, a.lda) && follows(problems, a.w_batch) && follows(batch, a.a_batch) &&
+                          (a.seg_cols == 0 || follows(a.n_segs, a.a_seg));
   // 17 to 64 rows: a CTA's rows of A are most of what it brings, so a tile a CTA, or a K long enough (64 rows: K = 1024, N = 1024 9.2, 6.9; K = 4096, N = 1024 24.6, 15.4; K = 2048,
   // N = 6144, 33 rows 23.9, 21.1; K = 1024, N = 8192 15.6, 16.2; fp32 K = 1024, N = 2048 14.9, 12.7, N = 4096 17.7, 20.8; 32 bf16 rows N = 4096 7.8, 7.1)
   const bool rows_pay = n_groups == 0 && (ring_units <= sm_count() || (ring_units <= 4 * sm_count() && a.K >= 2048) || (mg == 4 && ring_units <= 2 * sm_count() && a.K >= 1024));

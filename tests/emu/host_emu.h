@@ -177,7 +177,7 @@ inline int make_tmap_bf16_4d(CUtensorMap* m, const void* base, const uint64_t* d
     m->dims[i] = dims[i];
     m->box[i] = box[i];
     m->strides[i] = i == 0 ? 2 : strides[i - 1] * 2;
-    if (i > 0 && m->strides[i] % 16) { set_error("tensor map stride"); return -1; }
+    if (i > 0 && (m->strides[i] % 16 || m->strides[i] >= 1ULL << 40)) { set_error("tensor map stride"); return -1; }
   }
   return 0;
 }

@@ -162,6 +162,24 @@ def test_pairs_of_many_tiles(dtype, n_pairs, groups, N, K):
     assert rel_err(out, want) < 3e-6
 
 
+def test_operands_that_lie_far_apart(emu_lib):
+    """the operands of two problems, 32 TiB of addresses from one to the other: more than a tensor map's stride can be"""
+    libc = C.CDLL(None, use_errno=True)
+    libc.mmap.restype, libc.mmap.argtypes = C.c_void_p, [C.c_void_p, C.c_size_t, C.c_int, C.c_int, C.c_int, C.c_long]
+    M, N, K, far = 2, 24, 576, 1 << 45
+    a = torch.randn(2, M, K, generator=torch.Generator().manual_seed(1))
+    base = 1 << 44
+    for z in range(2):
+        at = libc.mmap(base + z * far, 1 << 16, 3, 0x100022, -1, 0)      # private and anonymous, at this address or nowhere
+        assert at == base + z * far
+        C.memmove(at, a[z].data_ptr(), 4 * M * K)
+    w = torch.randn(2, N, K, generator=torch.Generator().manual_seed(2)).to(BF16)
+    out = torch.empty(M, 2 * N)
+    d = _lib.LinearDesc(A=base, lda=K, a_batch=far // 4, a_fp32=1, W=_lib.ptr(w), ldw=K, w_batch=N * K, C=_lib.ptr(out), ldc=2 * N, c_batch=N, c_fp32=1, M=M, N=N, K=K, batch=2)
+    assert emu_lib.lp_linear(C.byref(d), None) == 0, emu_lib.lp_last_error()
+    assert rel_err(out, torch.cat([a[z].double() @ w[z].double().T for z in range(2)], 1)) < 2e-6
+
+
 @pytest.mark.parametrize("warp,pairs", [(0, False), (0, True), (13, True), (1, False), (9, False)])
 def test_lanes_that_lag_behind(emu_lib, warp, pairs):
     """the warps that fill the ring, take the products and add them up: lanes that only look on may run as late as they like (a block that gets stuck ends the process, so it is another one)"""
