@@ -1016,10 +1016,13 @@ static int dispatch_stream(const LinArgs& a, int a_fp32, int c_fp32, int batch, 
   auto follows = [](long long count, long long elements) { return count == 1 || (elements > 0 && elements < (1LL << 38)); };
   const bool ring_reads = follows(a.N, a.ldw) && follows(a.M, a.lda) && follows(problems, a.w_batch) && follows(batch, a.a_batch) &&
                           (a.seg_cols == 0 || follows(a.n_segs, a.a_seg));
+  // The ring waits while a thread takes sums of fp32 rows again that are not finite: up to 8 of them, 76 ns a product (64 rows, K = 16384, infinite weights: 10 ms for
+  // 0.12).  0.6 s at this K; the waits give up after two.
+  const bool ring_mends = !a_fp32 || a.K <= (1 << 20);
   // 17 to 64 rows: a CTA's rows of A are most of what it brings, so a tile a CTA, or a K long enough (64 rows: K = 1024, N = 1024 9.2, 6.9; K = 4096, N = 1024 24.6, 15.4; K = 2048,
   // N = 6144, 33 rows 23.9, 21.1; K = 1024, N = 8192 15.6, 16.2; fp32 K = 1024, N = 2048 14.9, 12.7, N = 4096 17.7, 20.8; 32 bf16 rows N = 4096 7.8, 7.1)
   const bool rows_pay = n_groups == 0 && (ring_units <= sm_count() || (ring_units <= 4 * sm_count() && a.K >= 2048) || (mg == 4 && ring_units <= 2 * sm_count() && a.K >= 1024));
-  if (ring_reads && (mg > 2 ? rows_pay : ring_pays && (n_groups > 0 || fp32_pays)) && n_groups <= RING_MAX_GROUPS && a.K % 64 == 0 && ring_units < (1LL << 31)) {
+  if (ring_reads && (mg > 2 ? rows_pay : ring_pays && (n_groups > 0 || fp32_pays)) && n_groups <= RING_MAX_GROUPS && a.K % 64 == 0 && ring_units < (1LL << 31) && ring_mends) {
     const bool two = a_fp32 && ring_units > sm_count() && (a.seg_cols == 0 || a.seg_cols % (2 * per) == 0);
 #define LP_RING(MG, PAIRS)                                                                                                 \
   (!a_fp32 ? launch_ring<bf16, 1, MG, PAIRS>(a, c_fp32, batch, n_pairs, n_groups, stream)                                  \

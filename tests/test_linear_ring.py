@@ -213,3 +213,19 @@ def test_numbers_that_are_not_finite(backend):
     fine = torch.isfinite(want)
     assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(out[torch.isinf(want)], want[torch.isinf(want)])
     assert rel_err(out[fine], want[fine]) < 2e-6
+
+
+@pytest.mark.parametrize("M", [3, 12, 20])
+def test_weights_that_are_not_finite(backend, M):
+    """infinite weights times fp32 rows whose terms differ in sign: each such sum is taken again, and is infinite or a NaN as the uncut product's is"""
+    N, K = 40, 640
+    a, w, _, _, _ = _data(M, N, K, F32, "cpu")
+    a, w = a.to(BF16).float(), w.clone()      # two terms that are zero
+    w[:, 77] = float("inf")
+    w[5, 600] = float("-inf")
+    a[1, 77] = 0.0
+    want = a.double() @ w.double().T
+    out = torch.empty(M, N, device=backend[0])
+    _call(backend, a.to(backend[0]), w.to(backend[0]), out, M, constant=1)
+    out = out.cpu().double()
+    assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(out[torch.isinf(want)], want[torch.isinf(want)])
