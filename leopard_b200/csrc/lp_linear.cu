@@ -998,20 +998,58 @@ static bool stream_ok(const LinArgs& a, int a_fp32, int batch) {
          (a.seg_cols == 0 || a.a_seg % q == 0) && (reinterpret_cast<uintptr_t>(a.A) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.W) & 15) == 0;
 }
 
+// Where the ring is ahead of the kernel without it (both on 9,000 random sizes, us a launch in a graph, that kernel and the ring).  It brings whole pieces of a tile through one
+// CTA an SM, so it wants a K of several pieces, and full rounds of tiles: 8 rows of bf16, K = 512, N = 7168 3.8, 5.3; K = 640, N = 7808 4.6, 5.9; K = 2048, N = 2048
+// 5.0, 3.6; K = 4096, N = 6144 12.1, 9.1; 16 rows, K = 4096, N = 32000 62, 44; but one row, K = 13376, N = 3072 (192 tiles on 148 SMs) 17.3, 18.9.  A few
+// columns over a very long K: all of it comes through a few CTAs (one row, K = 13312, N = 16 7.1, 7.9; fp32 K = 8256, N = 96 10.0, 12.2).
+// Weights that may be read early come while the small kernel before it runs, as in a decode step, and the lines are drawn for these: after a row norm of 2 us, 111 to 148 tiles of
+// K = 512 took 0.89 of that kernel's time (alone 1.05), two rounds of K = 640 to 1024 0.93 (1.0), 64 rows of 111 to 148 tiles of K = 512 0.92 (1.03).
+// fp32 rows are cut into terms for every tile: two tiles a piece where there is more than one a CTA (4 rows, K = 2048, N = 8192 13.0, 10.2 with one and
+// two tiles); 9 to 16 of them fill the issue slots up to one tile a CTA (K = N = 2048 7.3, 7.5; but N = 6144, K = 4096 34, 29).
+// 17 to 64 rows: A is most of what a CTA brings (64 rows, K = 4096, N = 1024 24.6, 15.4; fp32 K = 1024, N = 2048 14.9, 12.7), and up to 32 its plain sums are the cheaper
+// ones at most sizes; more are ahead up to a tile a CTA, and in a third round (K = 2048, N = 6144, 33 rows 23.9, 21.1) that is nearly full, not in a
+// second or a fourth (35 rows, K = 16192, N = 2752 72, 93; 58 gated rows, K = 5120, N = 2864 28.8, 32.5).
+static bool ring_pays_rows(int a_fp32, int mg, long long tiles, int K) {
+  const long long sms = sm_count();
+  const bool one = tiles <= sms, few = 4 * tiles <= sms;      // one tile a CTA; a quarter of the SMs at most
+  if (mg == 8) {
+    if (!one) return tiles > 2 * sms && tiles <= 3 * sms && K >= 2048;
+    return K <= 256 || (K <= 512 ? !few : a_fp32 || tiles > 8);
+  }
+  if (mg == 4) {
+    if (one) return !a_fp32 || K < 1024 || (K >= 2048 && !few) || (K > 4096 && tiles > 8);
+    return K >= (tiles <= 2 * sms ? 1024 : 2048) && tiles <= 4 * sms;
+  }
+  const bool half = !one && 2 * tiles <= 3 * sms;      // a second round of half the SMs at most
+  if (mg == 2) {
+    if (a_fp32) return !one && tiles <= 4 * sms && K >= 2048;
+    return one ? K > 512 : !half && K >= (tiles > 3 * sms && tiles <= 4 * sms ? 4096 : 2048);
+  }
+  if (a_fp32) {
+    if (one) return few ? K <= 1536 : K > 128;
+    return K >= 512 && (tiles <= 2 * sms || tiles > 3 * sms);
+  }
+  if (one) return K > 256 && (tiles > 8 || K <= 8192);
+  if (!one && 5 * tiles <= 8 * sms && K > 4096) return false;
+  return K >= 2048 || (K > 512 && tiles <= 2 * sms) || (K >= 1024 && tiles > 4 * sms);
+}
+// The same for pairs.  Its CTAs sort all pairs, 0.75 ns a group that has some and group (200 groups of 512 x 512, 188 pairs 35.8, 58.4); that kernel has CTAs for the groups
+// without pairs too (256 groups of 512 x 512: 18 us for two pairs, 13).  So: few groups to sort, or weights that take eight times as long, and then either many CTAs there, or
+// enough weights and tiles (16 groups of 2048 x 1024, 12 pairs 13.4, 11.7; 32 of 2048 x 4096, 32 pairs 67, 59; 8 of 1024 x 1024, 16 pairs 6.1, 7.1).  Two short steps a
+// tile, or more than 8 rows a group, are that kernel's (128 x 1544, 4 pairs 3.8, 5.8; 52 pairs in 8 groups of 2048 x 2304 4.9, 12.5).
+static bool ring_pays_pairs(const LinArgs& a, int a_fp32, long long tiles, int n_groups, int n_pairs) {
+  const long long used = n_pairs < n_groups ? n_pairs : n_groups, weights = used * a.N * a.K, sorting = used * n_groups;
+  if (sorting > 4000 && weights < 8000 * sorting) return false;
+  if (tiles >= 40LL * sm_count() && a.K >= (n_pairs <= 12 ? 192 : 512)) return true;
+  return weights >= (1 << 24) && n_groups * (n_pairs > 32 ? n_pairs : 32) <= 1024 && tiles / n_groups * used >= 4 * sm_count() && a.K >= (a_fp32 ? 512 : 1024);
+}
+
 // n_groups > 0: pairs, of which a group has up to about `rows` (more run in further rounds over its weights); else one problem of `rows` rows per batch entry
 static int dispatch_stream(const LinArgs& a, int a_fp32, int c_fp32, int batch, int rows, int n_groups, int n_pairs, cudaStream_t stream) {
   const int n_out = gated_epi(a.epi) ? a.N / 2 : a.N, per = gated_epi(a.epi) ? 8 : 16;
   const int mg = rows <= 8 ? 1 : rows <= 16 ? 2 : rows <= 32 ? 4 : 8;
   const long long problems = n_groups > 0 ? n_groups : batch;
   const long long ring_units = problems * ((n_out + per - 1) / per);
-  const long long ring_pairs = (ring_units + 1) / 2;      // units of two tiles
-  // Both sides (us, the kernel below and the ring, us a launch in a graph; K, N, rows): bf16 512, 512, 1 2.5, 2.3; 2048, 2048, 8 5.0, 3.6; 4096, 6144, 8 12.1, 9.1; 16384, 4096, 8
-  // 24.2, 21.3; 4096, 32000, 16 62, 44; but 128, 16 x 512, 16 4.3, 6.5 (tiles of one short piece).  fp32 rows are cut into terms for every tile: two tiles a piece where there
-  // is more than one a CTA (2048, 8192, 4 13.0, 10.2 with one and two), and not where the last round of these would be mostly empty (4096, 6144, 4 14.8, 15.7) or
-  // 9 to 16 rows fill the issue slots (4096, 16384, 16 47, 55; 2048, 2048, 16 7.3, 7.5; but 4096, 6144, 16 34, 29).  Pairs: 16 groups of 2048 x 1024, 12 pairs 13.4, 11.7; 32 of
-  // 2048 x 4096, 32 pairs 67, 59; 8 of 1024 x 1024, 16 pairs 6.1, 7.1 (the sorting of the pairs is not hidden).
-  const bool fp32_pays = !a_fp32 || (mg == 1 ? ring_pairs <= sm_count() || 2 * ring_pairs > 3 * sm_count() : ring_units > sm_count() && ring_units <= 4 * sm_count());
-  const bool ring_pays = n_groups > 0 ? n_pairs <= 4 || (long long)(n_pairs < n_groups ? n_pairs : n_groups) * a.N * a.K >= (1 << 24) : a.K >= (mg == 1 ? 512 : 2048) || ring_units <= sm_count();
   // rows, operands and problems lie at increasing addresses less than 2^40 bytes apart: what a tensor map can say
   auto follows = [](long long count, long long elements) { return count == 1 || (elements > 0 && elements < (1LL << 38)); };
   const bool ring_reads = follows(a.N, a.ldw) && follows(a.M, a.lda) && follows(problems, a.w_batch) && follows(batch, a.a_batch) &&
@@ -1019,21 +1057,14 @@ static int dispatch_stream(const LinArgs& a, int a_fp32, int c_fp32, int batch, 
   // The ring waits while a thread takes sums of fp32 rows again that are not finite: up to 8 of them, 76 ns a product (64 rows, K = 16384, infinite weights: 10 ms for
   // 0.12).  0.6 s at this K; the waits give up after two.
   const bool ring_mends = !a_fp32 || a.K <= (1 << 20);
-  // 17 to 64 rows: a CTA's rows of A are most of what it brings, so a tile a CTA, or a K long enough (64 rows: K = 1024, N = 1024 9.2, 6.9; K = 4096, N = 1024 24.6, 15.4; K = 2048,
-  // N = 6144, 33 rows 23.9, 21.1; K = 1024, N = 8192 15.6, 16.2; fp32 K = 1024, N = 2048 14.9, 12.7, N = 4096 17.7, 20.8; 32 bf16 rows N = 4096 7.8, 7.1)
-  const bool rows_pay = n_groups == 0 && (ring_units <= sm_count() || (ring_units <= 4 * sm_count() && a.K >= 2048) || (mg == 4 && ring_units <= 2 * sm_count() && a.K >= 1024));
-  if (ring_reads && (mg > 2 ? rows_pay : ring_pays && (n_groups > 0 || fp32_pays)) && n_groups <= RING_MAX_GROUPS && a.K % 64 == 0 && ring_units < (1LL << 31) && ring_mends) {
+  const bool ring_pays = n_groups > 0 ? mg == 1 && ring_pays_pairs(a, a_fp32, ring_units, n_groups, n_pairs) : ring_pays_rows(a_fp32, mg, ring_units, a.K);
+  if (ring_reads && ring_pays && n_groups <= RING_MAX_GROUPS && a.K % 64 == 0 && ring_units < (1LL << 31) && ring_mends) {
     const bool two = a_fp32 && ring_units > sm_count() && (a.seg_cols == 0 || a.seg_cols % (2 * per) == 0);
-#define LP_RING(MG, PAIRS)                                                                                                 \
-  (!a_fp32 ? launch_ring<bf16, 1, MG, PAIRS>(a, c_fp32, batch, n_pairs, n_groups, stream)                                  \
-           : two ? launch_ring<float, 2, MG, PAIRS>(a, c_fp32, batch, n_pairs, n_groups, stream) : launch_ring<float, 1, MG, PAIRS>(a, c_fp32, batch, n_pairs, n_groups, stream))
-    if (mg > 2) {
-#define LP_RING1(MG) (a_fp32 ? launch_ring<float, 1, MG, false>(a, c_fp32, batch, 0, 0, stream) : launch_ring<bf16, 1, MG, false>(a, c_fp32, batch, 0, 0, stream))
-      return mg == 4 ? LP_RING1(4) : LP_RING1(8);
-#undef LP_RING1
-    }
-    if (n_groups > 0) return mg == 1 ? LP_RING(1, true) : LP_RING(2, true);
-    return mg == 1 ? LP_RING(1, false) : LP_RING(2, false);
+#define LP_RING(NT, MG, PAIRS) (a_fp32 ? launch_ring<float, NT, MG, PAIRS>(a, c_fp32, batch, n_pairs, n_groups, stream) : launch_ring<bf16, 1, MG, PAIRS>(a, c_fp32, batch, n_pairs, n_groups, stream))
+    if (n_groups > 0) return LP_RING(2, 1, true);
+    if (mg == 1) return two ? LP_RING(2, 1, false) : LP_RING(1, 1, false);
+    if (mg == 2) return two ? LP_RING(2, 2, false) : LP_RING(1, 2, false);
+    return mg == 4 ? LP_RING(1, 4, false) : LP_RING(1, 8, false);
 #undef LP_RING
   }
   // fp32 rows: two tiles a CTA read A half as often and cut it into terms once, taken once the grid still has two CTAs for every SM and where segments

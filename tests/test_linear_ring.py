@@ -1,8 +1,9 @@
 """The product of up to 64 rows as one stream of weights through a ring of TMA pieces (lp_linear, lp_linear_group_pairs with K a multiple of 64) against a
 float64 product: pieces that end within K, tiles that end within N, more tiles than CTAs and more pieces than the ring has places, both operand types, batches,
-segments, gated units, groups whose pairs fill several tiles; weights that may be read early and weights that may not.
+segments, gated units, groups whose pairs fill several blocks; weights that may be read early and weights that may not.  The dispatch takes the ring where it is the
+faster kernel, by tiles per SM and K; the sizes lie on both sides of its lines, on the emulator's four or sixteen SMs and on the GPU's.
 
-Error bounds: as for the weight-streaming kernel, products are exact and K / 16 fp32 sums follow, less than 2e-6 of the result's size for K <= 1600."""
+Error bounds: as for the weight-streaming kernel, products are exact and K / 16 fp32 sums follow, less than 2e-6 of the result's size for K <= 2112."""
 import ctypes as C
 import os
 import subprocess
@@ -28,7 +29,7 @@ def _leave_nans(backend):
 
 
 @pytest.mark.parametrize("dtype", [BF16, F32])
-@pytest.mark.parametrize("M,N,K", [(1, 1, 64), (1, 200, 1088), (3, 40, 576), (5, 130, 512), (8, 16, 1600), (8, 300, 64), (9, 33, 640), (16, 130, 448), (17, 40, 320), (32, 130, 576), (33, 72, 256), (64, 130, 832)])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 64), (1, 1, 576), (1, 200, 2112), (3, 40, 576), (5, 90, 832), (5, 130, 512), (8, 16, 1600), (8, 300, 64), (8, 300, 576), (9, 33, 640), (16, 130, 448), (17, 40, 320), (32, 130, 576), (33, 72, 256), (64, 130, 832), (12, 200, 2112), (20, 100, 1088), (33, 64, 576), (64, 160, 2112)])
 @pytest.mark.parametrize("constant", [0, 1])
 def test_rows_tiles_and_pieces(backend, dtype, M, N, K, constant):
     a, w, want, ad, wd = _data(M, N, K, dtype, backend[0])
@@ -40,6 +41,17 @@ def test_rows_tiles_and_pieces(backend, dtype, M, N, K, constant):
     assert torch.equal(out, again)
 
 
+@pytest.fixture
+def sixteen_sms(backend):
+    """products of a tile an SM take the ring at a shorter K than those of several rounds"""
+    if backend[1] is not None:
+        backend[1].emu_set_sm_count(16)
+    yield
+    if backend[1] is not None:
+        backend[1].emu_set_sm_count(4)
+
+
+@pytest.mark.usefixtures("sixteen_sms")
 @pytest.mark.parametrize("dtype", [BF16, F32])
 @pytest.mark.parametrize("M", [3, 12, 20, 50])
 def test_gated_and_added(backend, dtype, M):
@@ -58,6 +70,7 @@ def test_gated_and_added(backend, dtype, M):
     assert rel_err(out, x.double() + 0.5 * v) < 2e-6
 
 
+@pytest.mark.usefixtures("sixteen_sms")
 @pytest.mark.parametrize("dtype", [BF16, F32])
 @pytest.mark.parametrize("M", [2, 11, 30, 41])
 def test_batches_and_segments(backend, dtype, M):
@@ -98,27 +111,26 @@ def test_pairs(backend, dtype, n_pairs, groups, a_div):
 
 
 @pytest.mark.parametrize("dtype", [BF16, F32])
-@pytest.mark.parametrize("n_pairs", [1, 4])
-@pytest.mark.parametrize("K", [64, 192, 704, 1088])
-def test_few_pairs_of_any_whole_piece(backend, dtype, n_pairs, K):
-    """up to four pairs take the ring whatever their size: K of odd multiples of 64 ends within what a warp takes of a piece"""
-    g = torch.Generator().manual_seed(K + n_pairs)
-    N, groups = 40, 6
-    a, w = torch.randn(n_pairs, K, generator=g).to(dtype), torch.randn(groups, N, K, generator=g).to(BF16)
-    of = torch.tensor([4, 1, 4, 5], dtype=torch.int32)[:n_pairs]
+@pytest.mark.parametrize("of", [[4], [4, 1, 4, 5], [0] * 7 + [2] * 3, [3] * 12])
+@pytest.mark.parametrize("K", [192, 704, 1088])
+def test_few_pairs_of_many_tiles(backend, dtype, of, K):
+    """forty tiles an SM, of which most belong to groups without pairs: K of odd multiples of 64 ends within what a warp takes of a piece; more than 8 pairs in a group"""
+    g = torch.Generator().manual_seed(K + len(of))
+    N, groups = (432, 6) if backend[0] == "cpu" else (7904, 12)
+    assert groups * (N // 16) >= 40 * (4 if backend[0] == "cpu" else 148)      # the dispatch's line
+    a, w = torch.randn(len(of), K, generator=g).to(dtype), torch.randn(groups, N, K, generator=g).to(BF16)
     ad, wd = a.to(backend[0]), w.to(backend[0])
     _leave_nans(backend)
-    out = torch.full((n_pairs, N), 7.0, device=backend[0])
-    _call(backend, ad, wd, out, 1, pairs=of.to(backend[0]), groups=groups)
-    want = torch.stack([a[z].double() @ w[int(of[z])].double().T for z in range(n_pairs)])
+    out = torch.full((len(of), N), 7.0, device=backend[0])
+    _call(backend, ad, wd, out, 1, pairs=torch.tensor(of, dtype=torch.int32).to(backend[0]), groups=groups)
+    want = torch.stack([ad[z].double() @ wd[of[z]].double().T for z in range(len(of))])
     assert rel_err(out, want) < 2e-6
 
 
 @pytest.mark.parametrize("dtype", [BF16, F32])
-@pytest.mark.parametrize("n_pairs,groups,N,K,a_div", [(12, 4, 6000, 704, 1), (24, 4, 6000, 704, 2), (20, 4, 3860, 1088, 4)])
+@pytest.mark.parametrize("n_pairs,groups,N,K,a_div", [(12, 4, 4096, 1088, 1), (30, 8, 2064, 1088, 4), (32, 8, 432, 704, 1)])
 def test_pairs_in_blocks(backend, dtype, n_pairs, groups, N, K, a_div):
-    """enough weights for the ring: groups of more than 8 and more than 16 pairs (blocks of 8 or of 16 rows each) and groups without any"""
-    assert min(n_pairs, groups) * N * K >= 1 << 24      # the dispatch's line
+    """enough weights for the ring, or tiles (on the emulator's four SMs): groups of more than 8 and more than 16 pairs, a block of 8 after the other, and groups without any"""
     g = torch.Generator().manual_seed(n_pairs)
     a, w = torch.randn((n_pairs + a_div - 1) // a_div, K, generator=g).to(dtype), torch.randn(groups, N, K, generator=g).to(BF16)
     of = torch.full((n_pairs,), groups - 1)
@@ -133,9 +145,9 @@ def test_pairs_in_blocks(backend, dtype, n_pairs, groups, N, K, a_div):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [BF16, F32])
-@pytest.mark.parametrize("M,N,K", [(1, 2600, 8256), (8, 3200, 5184), (16, 2500, 8256), (13, 5000, 2112), (30, 2400, 5184), (64, 2400, 4160)])
+@pytest.mark.parametrize("M,N,K", [(1, 3600, 8256), (8, 3200, 3136), (8, 11200, 5184), (16, 2500, 8256), (13, 5000, 2112), (30, 2400, 5184), (64, 4800, 4160)])
 def test_more_tiles_than_sms_and_more_pieces_than_stages(dtype, M, N, K):
-    """the ring goes round several times within a tile and from tile to tile; fp32 rows with two tiles a piece (149 to 592 tiles).  K / 16 sums that are kept
+    """the ring goes round several times within a tile and from tile to tile; fp32 rows with two tiles a piece (149 to 222 tiles, and more than 592).  K / 16 sums that are kept
     exactly, or for more than 16 rows rounded: below 3e-6 of the result for K <= 8256."""
     backend = "cuda", None
     a, w, want, ad, wd = _data(M, N, K, dtype, "cuda")
@@ -148,7 +160,7 @@ def test_more_tiles_than_sms_and_more_pieces_than_stages(dtype, M, N, K):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [BF16, F32])
-@pytest.mark.parametrize("n_pairs,groups,N,K", [(16, 8, 1000, 5824), (40, 8, 2100, 5824), (100, 50, 712, 1344)])
+@pytest.mark.parametrize("n_pairs,groups,N,K", [(16, 8, 1216, 5824), (30, 8, 2104, 5824), (100, 50, 1944, 1344)])
 def test_pairs_of_many_tiles(dtype, n_pairs, groups, N, K):
     backend = "cuda", None
     g = torch.Generator().manual_seed(n_pairs)
@@ -189,11 +201,12 @@ def test_lanes_that_lag_behind(emu_lib, warp, pairs):
 
 
 def product_with_lagging_lanes(path, warp, pairs):
-    """one row, pieces for two rounds of the ring in every CTA"""
+    """one row, pieces for two rounds of the ring and more in every CTA"""
     lib = _lib.bind_stream32(C.CDLL(path))
     lib.emu_set_lagging(warp, 1)
-    a, w, want, ad, wd = _data(1, 256, 2048, BF16, "cpu")
-    out = torch.empty(1, 256)
+    N, K = (2560, 192) if pairs else (256, 2048)
+    a, w, want, ad, wd = _data(1, N, K, BF16, "cpu")
+    out = torch.empty(1, N)
     _call(("cpu", lib), ad, wd[None] if pairs else wd, out, 1, **({"pairs": torch.zeros(1, dtype=torch.int32), "groups": 1} if pairs else {}))
     assert rel_err(out, want) < 2e-6
 
