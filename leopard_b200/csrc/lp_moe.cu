@@ -213,12 +213,9 @@ moe_align_kernel(const int* idx, int n_pairs, int top, int E, int tile_rows, int
   }
 }
 
-// A CTA per token, V neighbouring columns a thread, four of the token's rows in flight (4096 tokens of 2048 columns, two experts and a shared one, us: a
+// A CTA per token, four neighbouring columns a thread, four of the token's rows in flight (4096 tokens of 2048 columns, two experts and a shared one, us: a
 // column a thread and a row at a time 53, so 35; 300 tokens 25, 12; launches included).
-template <int V> struct MoeVec;
-template <> struct MoeVec<1> { float v[1]; };
-template <> struct alignas(16) MoeVec<4> { float v[4]; };
-template <int V>
+struct alignas(16) MoeVec { float v[4]; };
 __global__ void moe_combine_kernel(const float* y, long long ldy, const int* pair_row, const float* w,
                                    int top, const float* shared, long long lds, const float* gate,
                                    float* __restrict__ out, long long ldo, int T, int D) {
@@ -229,23 +226,38 @@ __global__ void moe_combine_kernel(const float* y, long long ldy, const int* pai
   const int* row = pair_row + (long long)t * top;
   const float* weight = w != nullptr ? w + (long long)t * top : nullptr;
   const float g = shared != nullptr && gate != nullptr ? gate[t] : 1.0f;
-  for (int c = threadIdx.x * V; c < D; c += blockDim.x * V) {
-    MoeVec<V> acc, own;
+  for (int c = threadIdx.x * 4; c < D; c += blockDim.x * 4) {
+    MoeVec acc, own;
 #pragma unroll
-    for (int i = 0; i < V; ++i) acc.v[i] = 0.f;
-    if (shared != nullptr) own = *reinterpret_cast<const MoeVec<V>*>(shared + (long long)t * lds + c);
+    for (int i = 0; i < 4; ++i) acc.v[i] = 0.f;
+    if (shared != nullptr) own = *reinterpret_cast<const MoeVec*>(shared + (long long)t * lds + c);
 #pragma unroll 4
     for (int k = 0; k < top; ++k) {
-      const MoeVec<V> x = *reinterpret_cast<const MoeVec<V>*>(y + (long long)row[k] * ldy + c);
+      const MoeVec x = *reinterpret_cast<const MoeVec*>(y + (long long)row[k] * ldy + c);
       const float f = weight != nullptr ? weight[k] : 1.0f;
 #pragma unroll
-      for (int i = 0; i < V; ++i) acc.v[i] = fmaf(f, x.v[i], acc.v[i]);
+      for (int i = 0; i < 4; ++i) acc.v[i] = fmaf(f, x.v[i], acc.v[i]);
     }
     if (shared != nullptr) {
 #pragma unroll
-      for (int i = 0; i < V; ++i) acc.v[i] = fmaf(g, own.v[i], acc.v[i]);
+      for (int i = 0; i < 4; ++i) acc.v[i] = fmaf(g, own.v[i], acc.v[i]);
     }
-    *reinterpret_cast<MoeVec<V>*>(out + (long long)t * ldo + c) = acc;
+    *reinterpret_cast<MoeVec*>(out + (long long)t * ldo + c) = acc;
+  }
+}
+// a column a thread: rows that are not whole 16-byte pieces, and narrow rows of many tokens, which leave three warps of four idle above (330 tokens of 4053 columns, two
+// experts, four columns' loop with one 16.6 us, so 12.0; 3,980 of 108, one expert and a shared one, above 5.0, so 4.1).  Nothing it reads is written beside it.
+__global__ void moe_combine_columns_kernel(const float* __restrict__ y, long long ldy, const int* __restrict__ pair_row, const float* __restrict__ w,
+                                           int top, const float* __restrict__ shared, long long lds, const float* __restrict__ gate,
+                                           float* __restrict__ out, long long ldo, int T, int D) {
+  const int t = blockIdx.x;
+  if (t >= T) return;
+  for (int c = threadIdx.x; c < D; c += blockDim.x) {
+    float acc = 0.f;
+    for (int k = 0; k < top; ++k)
+      acc = fmaf(w != nullptr ? w[(long long)t * top + k] : 1.0f, y[(long long)pair_row[(long long)t * top + k] * ldy + c], acc);
+    if (shared != nullptr) acc = fmaf(gate != nullptr ? gate[t] : 1.0f, shared[(long long)t * lds + c], acc);
+    out[(long long)t * ldo + c] = acc;
   }
 }
 
@@ -377,12 +389,16 @@ extern "C" int lp_moe_combine(const float* y, long long ldy, const int* pair_row
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   LP_REQUIRE(y != nullptr && pair_row != nullptr && out != nullptr, "lp_moe_combine: null operand");
   if (T <= 0) return 0;
-  // rows of 16-byte pieces: four columns a thread; few tokens: as many threads as that takes
-  const bool vec = ((D | ldy | ldo | (shared != nullptr ? lds : 0)) & 3) == 0 &&
-                   ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(shared) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-  const int units = vec ? D / 4 : D, threads = T > MOE_FEW_TOKENS || units < 256 ? 128 : units < 1024 ? (units + 31) / 32 * 32 : 1024;
-  LP_CHECK_CUDA(vec ? launch_next(moe_combine_kernel<4>, dim3(T), dim3(threads), 0, stream, y, ldy, pair_row, w, top, shared, lds, gate, out, ldo, T, D)
-                    : launch_next(moe_combine_kernel<1>, dim3(T), dim3(threads), 0, stream, y, ldy, pair_row, w, top, shared, lds, gate, out, ldo, T, D));
+  // rows of 16-byte pieces: four columns a thread, of few tokens as many threads as that takes
+  const bool pieces = ((D | ldy | ldo | (shared != nullptr ? lds : 0)) & 3) == 0 &&
+                      ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(shared) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  const bool many = T > MOE_FEW_TOKENS;
+  if (pieces && (!many || D >= 512)) {
+    const int threads = many || D < 1024 ? 128 : D < 4096 ? (D / 4 + 31) / 32 * 32 : 1024;
+    LP_CHECK_CUDA(launch_next(moe_combine_kernel, dim3(T), dim3(threads), 0, stream, y, ldy, pair_row, w, top, shared, lds, gate, out, ldo, T, D));
+  } else {
+    moe_combine_columns_kernel<<<T, many || D < 512 ? 128 : D < 1024 ? 256 : 1024, 0, stream>>>(y, ldy, pair_row, w, top, shared, lds, gate, out, ldo, T, D);
+  }
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;

@@ -15,7 +15,7 @@ def _of(backend):
         C.c_void_p(torch.cuda.current_stream().cuda_stream) if backend[0] != "cpu" else None
 
 
-@pytest.mark.parametrize("T,D,top", [(3, 520, 2), (FEW + 1, 36, 5), (2, 4100, 1), (5, 33, 9)])
+@pytest.mark.parametrize("T,D,top", [(3, 520, 2), (FEW + 1, 36, 5), (FEW + 1, 516, 2), (2, 4100, 1), (5, 33, 9)])
 @pytest.mark.parametrize("extras", [True, False])
 def test_columns_together_and_alone(backend, T, D, top, extras):
     dev, L, stream = _of(backend)
