@@ -225,13 +225,14 @@ __device__ __forceinline__ void ret_mma(float (&acc)[4], const RetRows& a, const
   for (int c = 0; c < 4; ++c) acc[c] += d[c];
 }
 
+// The three kernels of a prompt wait as programmatic launches do, but none lets the next one start early: its CTAs, placed beside the running ones, took a third of
+// the time more than the launch gaps that they save (us a prompt of 887 rows of 4 heads of 96 x 256: early 74, so 51, plain launches 52; 5 rows of 16 heads of 128 x 128 32, 22, 23).
 // (1) U[chunk][head] = sum_j decay^(len-1-j) k_j v_j^T.  4 x 4 outputs per thread (8 x 8 from 16-byte reads: 208 us for 162); a thread's four columns are vdim/4
 // apart, so that the threads of a warp read consecutive shared-memory words.  MM: two CTAs an SM (three, at 80 registers, spill: 78 us for 74).
 template <bool MM>
 __global__ void __launch_bounds__(RET_CHUNK_THREADS, MM ? 2 : 1)
 retention_chunk_state_kernel(RetArgs a, const int* __restrict__ chunk_seq, const int* __restrict__ chunk_row0, const int* __restrict__ chunk_len,
                              const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0, float* __restrict__ ws) {
-  pdl_launch_dependents();
   pdl_wait();
   extern __shared__ float dyn_smem[];
   const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
@@ -339,7 +340,6 @@ template <int V>
 __global__ void __launch_bounds__(SCAN_THREADS)
 retention_scan_kernel(RetArgs a, const int* __restrict__ seq_chunk0, const int* __restrict__ chunk_len, const int* __restrict__ seq_pos0,
                       const int* __restrict__ seq_slot, float* ws) {
-  pdl_launch_dependents();
   pdl_wait();
   const int s = blockIdx.x, h = blockIdx.y;
   const long long hs = (long long)a.dim * a.vdim;
@@ -395,7 +395,6 @@ template <bool WIDE, bool MM>
 __global__ void __launch_bounds__(RET_CHUNK_THREADS, MM ? 3 : 1)
 retention_chunk_out_kernel(RetArgs a, const int* __restrict__ chunk_seq, const int* __restrict__ chunk_row0, const int* __restrict__ chunk_len,
                            const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0, const float* ws, int stage_s) {
-  pdl_launch_dependents();
   pdl_wait();
   extern __shared__ float dyn_smem[];
   const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
