@@ -124,6 +124,14 @@ inline cudaError_t launch_next(void (*kern)(KArgs...), dim3 grid, dim3 block, si
   return launch_ex(kern, grid, block, smem, stream, 1, (long long)grid.x * grid.y * grid.z <= 4LL * sm_count(), args...);
 }
 
+// Attention of a step over the past, `work` = rows x heads x keys at most: where it runs for long, CTAs that were placed beside the launch before, on the SMs that this one left empty,
+// make it longer (us a step, early and not: 32 requests of 900 tokens, window 512, 8 heads 287, 275; 48 of 1,400, 8 heads of latents 287, 276, now and then 335; 8 of 1,500, window
+// 1024, 16 heads 198, 188; one of 3,000, window 2048, 32 heads 304, 297; but one of 530 283, 284.5).
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_attention(long long work, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  return work < 50000 ? launch_next(kern, grid, block, smem, stream, args...) : launch_ex(kern, grid, block, smem, stream, 1, false, args...);
+}
+
 // launch accounting + optional per-launch CUDA-event timing (off by default; see lp_profile_* in the public header)
 void note_launch(int n = 1);
 struct ProfScope {

@@ -40,9 +40,10 @@ __device__ __forceinline__ void gru_store(const GruArgs& a, long long row, int c
 
 constexpr int GRU_THREADS = 128;
 
+// The kernels of a prompt do not let one another start early: waiting CTAs beside the running ones cost more than the launch gaps (630 rows of 2,846 channels 54 us, so 41; with
+// plain launches 41).
 __global__ void __launch_bounds__(GRU_THREADS)
 mingru_chunk_kernel(GruArgs a, const int* __restrict__ chunk_row0, const int* __restrict__ chunk_len, float* __restrict__ ws, int n_chunks) {
-  pdl_launch_dependents();
   pdl_wait();
   const int c = blockIdx.x, ch = blockIdx.y * GRU_THREADS + threadIdx.x;
   if (ch >= a.width) return;
@@ -64,7 +65,6 @@ mingru_chunk_kernel(GruArgs a, const int* __restrict__ chunk_row0, const int* __
 __global__ void __launch_bounds__(GRU_THREADS)
 mingru_scan_kernel(GruArgs a, const int* __restrict__ seq_chunk0, const int* __restrict__ seq_pos0, const int* __restrict__ seq_slot,
                    float* ws, int n_chunks) {
-  pdl_launch_dependents();
   pdl_wait();
   const int s = blockIdx.x, ch = blockIdx.y * GRU_THREADS + threadIdx.x;
   if (ch >= a.width) return;
@@ -79,7 +79,6 @@ mingru_scan_kernel(GruArgs a, const int* __restrict__ seq_chunk0, const int* __r
 __global__ void __launch_bounds__(GRU_THREADS)
 mingru_out_kernel(GruArgs a, const int* __restrict__ chunk_seq, const int* __restrict__ chunk_row0, const int* __restrict__ chunk_len,
                   const int* __restrict__ seq_chunk0, const int* __restrict__ seq_slot, const float* ws) {
-  pdl_launch_dependents();
   pdl_wait();
   const int c = blockIdx.x, ch = blockIdx.y * GRU_THREADS + threadIdx.x;
   if (ch >= a.width) return;
@@ -96,7 +95,7 @@ mingru_out_kernel(GruArgs a, const int* __restrict__ chunk_seq, const int* __res
 
 __global__ void __launch_bounds__(GRU_THREADS)
 mingru_decode_kernel(GruArgs a, const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0, const int* __restrict__ seq_slot) {
-  pdl_launch_dependents();
+  pdl_launch_next();
   pdl_wait();
   const int s = blockIdx.x, ch = blockIdx.y * GRU_THREADS + threadIdx.x;
   if (ch >= a.width) return;

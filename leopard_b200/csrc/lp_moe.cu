@@ -68,7 +68,7 @@ moe_route_kernel(const HT* h, long long ldh, int T, int D, const bf16* __restric
                  const float* __restrict__ correction, int n_groups, int keep_groups, int top, const bf16* __restrict__ w_gate,
                  int* __restrict__ idx_out, float* __restrict__ w_out, float* __restrict__ gate_out, int softmax_mode,
                  const float* __restrict__ logit_bias, float w_scale) {
-  pdl_launch_dependents();
+  pdl_launch_next();
   pdl_wait();
   __shared__ float sc[MOE_MAX_EXPERTS];   // sigmoid scores
   __shared__ float ch[MOE_MAX_EXPERTS];   // choice scores (minus infinity once taken or not eligible)
@@ -184,7 +184,7 @@ constexpr int ALIGN_THREADS = 1024;
 __global__ void __launch_bounds__(ALIGN_THREADS)
 moe_align_kernel(const int* idx, int n_pairs, int top, int E, int tile_rows, int max_tiles, int* __restrict__ tile_group,
                  int* __restrict__ sorted_token, int* __restrict__ pair_row) {
-  pdl_launch_dependents();
+  pdl_launch_next();
   pdl_wait();
   __shared__ unsigned cnt[MOE_MAX_EXPERTS];
   __shared__ int off[MOE_MAX_EXPERTS + 1];
@@ -219,7 +219,7 @@ struct alignas(16) MoeVec { float v[4]; };
 __global__ void moe_combine_kernel(const float* y, long long ldy, const int* pair_row, const float* w,
                                    int top, const float* shared, long long lds, const float* gate,
                                    float* __restrict__ out, long long ldo, int T, int D) {
-  pdl_launch_dependents();
+  pdl_launch_next();
   pdl_wait();
   const int t = blockIdx.x;
   if (t >= T) return;

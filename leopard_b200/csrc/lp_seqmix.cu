@@ -662,7 +662,7 @@ template <int V> __host__ __device__ inline int ret_dec_groups(int vdim) { retur
 template <int V>
 __global__ void __launch_bounds__(RET_DEC_THREADS)
 retention_decode_kernel(RetArgs a, const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0, const int* __restrict__ seq_slot) {
-  pdl_launch_dependents();
+  pdl_launch_next();
   pdl_wait();
   extern __shared__ float dyn_smem[];
   const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
@@ -776,7 +776,7 @@ constexpr int LAT_PREP_THREADS = 128, LAT_PREP_WIDE = 512;      // up to two row
 constexpr int LAT_PREP_PAIRS = 4096;      // rotation pairs whose sines and cosines shared memory holds; with more of them each is taken where it is used
 __global__ void __launch_bounds__(LAT_PREP_WIDE)
 latent_prep_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos) {
-  pdl_launch_dependents();
+  pdl_launch_next();
   pdl_wait();
   extern __shared__ float dyn_smem[];
   __shared__ float red[LAT_PREP_WIDE / 32];
@@ -848,7 +848,7 @@ template <int V, int NP, int W>
 __global__ void __launch_bounds__(W * 32)
 latent_attend_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos, const float* q_abs,
                      long long ldqa, void* __restrict__ out, long long ldo, int out_fp32) {
-  pdl_launch_dependents();
+  pdl_launch_next();
   pdl_wait();
   __align__(16) __shared__ float s_acc[W][32 * V * NP];
   __shared__ float s_mx[W], s_den[W];
@@ -983,7 +983,7 @@ template <int NR>
 __global__ void __launch_bounds__(LAT_ROW_HEADS * 32)
 latent_attend_rows_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos, const float* q_abs,
                           long long ldqa, void* __restrict__ out, long long ldo, int out_fp32) {
-  pdl_launch_dependents();
+  pdl_launch_next();
   pdl_wait();
   const int r = blockIdx.x;
   const int h = blockIdx.y * LAT_ROW_HEADS + (threadIdx.x >> 5);
@@ -1332,7 +1332,9 @@ static int launch_ret_decode(const RetArgs& a, int n_seqs, const int* seq_row0, 
   const size_t smem = ((size_t)2 * a.dim + 2 * a.vdim + (size_t)ret_dec_groups<V>(a.vdim) * a.vdim) * sizeof(float);
   LP_REQUIRE(smem <= 200 * 1024, "lp_retention_decode: dim=%d vdim=%d do not fit shared memory", a.dim, a.vdim);
   LP_CHECK_CUDA(ensure_smem(retention_decode_kernel<V>, smem, have));
-  LP_CHECK_CUDA(launch_next(retention_decode_kernel<V>, dim3(n_seqs, a.heads), dim3(RET_DEC_THREADS), smem, stream, a, seq_row0, seq_pos0, seq_slot));
+  // not before the launch before has ended: CTAs that are placed beside it lie on fewer SMs, whose loads then take longer (a step of 8 requests of 16 heads 1.3 % of its time;
+  // 18 requests of 8 heads, launch after launch, 6.7 us, so 5.4)
+  LP_CHECK_CUDA(launch_ex(retention_decode_kernel<V>, dim3(n_seqs, a.heads), dim3(RET_DEC_THREADS), smem, stream, 1, false, a, seq_row0, seq_pos0, seq_slot));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
   return 0;
@@ -1370,22 +1372,23 @@ extern "C" int lp_latent_attend(const lp_latent_desc* d, int R, const int* row_s
   LP_REQUIRE(d->kv_rank <= LAT_MAX_RANK && d->rot_dim <= LAT_MAX_RANK, "lp_latent_attend: kv_rank=%d / rot_dim=%d > %d is not instantiated",
              d->kv_rank, d->rot_dim, LAT_MAX_RANK);
   if (R <= 0) return 0;
+  const long long pages = (long long)d->max_pages * d->page_size, work = (long long)R * d->heads * (d->window > 0 && d->window < pages ? d->window : pages);
   const int nr = ((d->kv_rank > d->rot_dim ? d->kv_rank : d->rot_dim) + 31) / 32;      // lanes hold both vectors strided by 32
   if (R > LAT_SPLIT_ROWS || d->kv_rank > LAT_SPLIT_MAX_RANK || d->rot_dim > LAT_SPLIT_MAX_RANK) {      // prompts: a CTA per row, a warp per head
     const dim3 grid(R, (d->heads + LAT_ROW_HEADS - 1) / LAT_ROW_HEADS);
     const int threads = (d->heads < LAT_ROW_HEADS ? d->heads : LAT_ROW_HEADS) * 32;
-    if (nr <= 2) LP_CHECK_CUDA(launch_next(latent_attend_rows_kernel<2>, grid, dim3(threads), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32));
-    else if (nr <= 4) LP_CHECK_CUDA(launch_next(latent_attend_rows_kernel<4>, grid, dim3(threads), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32));
-    else if (nr <= 8) LP_CHECK_CUDA(launch_next(latent_attend_rows_kernel<8>, grid, dim3(threads), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32));
-    else if (nr <= 16) LP_CHECK_CUDA(launch_next(latent_attend_rows_kernel<16>, grid, dim3(threads), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32));
-    else LP_CHECK_CUDA(launch_next(latent_attend_rows_kernel<32>, grid, dim3(threads), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32));
+    if (nr <= 2) LP_CHECK_CUDA(launch_attention(work, latent_attend_rows_kernel<2>, grid, dim3(threads), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32));
+    else if (nr <= 4) LP_CHECK_CUDA(launch_attention(work, latent_attend_rows_kernel<4>, grid, dim3(threads), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32));
+    else if (nr <= 8) LP_CHECK_CUDA(launch_attention(work, latent_attend_rows_kernel<8>, grid, dim3(threads), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32));
+    else if (nr <= 16) LP_CHECK_CUDA(launch_attention(work, latent_attend_rows_kernel<16>, grid, dim3(threads), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32));
+    else LP_CHECK_CUDA(launch_attention(work, latent_attend_rows_kernel<32>, grid, dim3(threads), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32));
   } else {      // decoding: a CTA per (row, head), its warps split the keys
     const long long ctas = (long long)R * d->heads;
     const bool pieces = d->kv_rank % 4 == 0 && d->rot_dim % 4 == 0 && d->rot_dim <= 128 && (reinterpret_cast<uintptr_t>(d->cache) & 15) == 0;
 #define LP_LAT(V, NP)                                                                                                                       \
   do {                                                                                                                                      \
-    if (ctas <= 2LL * sm_count()) LP_CHECK_CUDA((launch_next(latent_attend_kernel<V, NP, 16>, dim3((unsigned)ctas), dim3(16 * 32), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32)));    \
-    else LP_CHECK_CUDA((launch_next(latent_attend_kernel<V, NP, 4>, dim3((unsigned)ctas), dim3(4 * 32), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32)));     \
+    if (ctas <= 2LL * sm_count()) LP_CHECK_CUDA((launch_attention(work, latent_attend_kernel<V, NP, 16>, dim3((unsigned)ctas), dim3(16 * 32), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32)));    \
+    else LP_CHECK_CUDA((launch_attention(work, latent_attend_kernel<V, NP, 4>, dim3((unsigned)ctas), dim3(4 * 32), 0, stream, a, R, row_seq, row_pos, q_abs, ldqa, out, ldo, out_fp32)));     \
   } while (0)
     if (pieces) {
       const int np = (d->kv_rank + 127) / 128;

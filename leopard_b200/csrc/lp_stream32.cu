@@ -44,7 +44,7 @@ __global__ void embed_rows_f32_kernel(const int* ids, int R, const bf16* __restr
                                       float scale, float* __restrict__ out, long long ldo, int D) {
   // a step's first launch: the products after it read their weights before they wait, so none of them starts before all that wrote weights has ended
   pdl_wait();
-  pdl_launch_dependents();
+  pdl_launch_next();
   const int r = blockIdx.x;
   if (r >= R) return;
   int id = ids[r];
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(1024)
 rmsnorm_row_kernel(const float* x, long long ldx, int D, float gain_scalar, const float* __restrict__ gain_vec, float eps,
                    float* __restrict__ out_f32, bf16* __restrict__ out_bf16, long long ldo, float* accum, long long lda,
                    NormNext next) {
-  pdl_launch_dependents();
+  pdl_launch_next();
   pdl_wait();
   __shared__ float red[2][32];
   const long long row = blockIdx.x;
@@ -231,7 +231,7 @@ __device__ __forceinline__ float glu_one(int mode, float z, float u, float a, fl
 template <typename IT, typename OT, int V>
 __global__ void glu_kernel(const IT* in, long long ldi, OT* __restrict__ out, long long ldo, int M, int N, int mode, float a,
                            float b, const float* row_scale) {
-  pdl_launch_dependents();
+  pdl_launch_next();
   pdl_wait();
   const int n = (int)(blockIdx.x * blockDim.x + threadIdx.x) * V;
   if (n >= N) return;
@@ -371,7 +371,7 @@ static dim3 rows_grid(int groups, int M) { return dim3((unsigned)((groups + 255)
 
 template <int V>
 __global__ void axpy_f32_kernel(float* y, long long ldy, const float* x, long long ldx, float alpha, int M, int N) {
-  pdl_launch_dependents();
+  pdl_launch_next();
   pdl_wait();
   const int n = (int)(blockIdx.x * blockDim.x + threadIdx.x) * V;
   if (n >= N) return;

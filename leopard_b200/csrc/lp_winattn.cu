@@ -146,7 +146,7 @@ __device__ __forceinline__ const float* win_visible_row(const WinArgs& a, const 
 constexpr int WIN_PREP_THREADS = 128, WIN_PREP_WIDE = 1024;      // few rows (decoding) take the wide CTA
 __global__ void __launch_bounds__(WIN_PREP_WIDE)
 window_attn_prep_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos) {
-  pdl_launch_dependents();
+  pdl_launch_next();
   pdl_wait();
   extern __shared__ float dyn_smem[];
   float* s_ss = dyn_smem;      // [heads + kv_heads] sums of squares, then the two totals
@@ -332,7 +332,7 @@ __device__ __forceinline__ float win_head_sum(const float4& v) {
 }
 __global__ void __launch_bounds__(PREP_MAX_WARPS * 32)
 window_attn_prep_heads_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos) {
-  pdl_launch_dependents();
+  pdl_launch_next();
   pdl_wait();
   __shared__ float s_ss[PREP_HEADS * PREP_MAX_WARPS];
   const int r = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5, d = lane * 4;
@@ -412,7 +412,7 @@ static bool prep_heads_ok(const WinArgs& a, int dim, int vdim) {
 constexpr int WIN_POOL_THREADS = 128;
 __global__ void __launch_bounds__(WIN_POOL_THREADS)
 window_attn_pool_kernel(WinArgs a, int n_seqs, const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0) {
-  pdl_launch_dependents();
+  pdl_launch_next();
   pdl_wait();
   const int s = blockIdx.x;
   if (s >= n_seqs) return;
@@ -431,7 +431,7 @@ template <int QH, int NV, bool DIST, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 window_attn_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos, void* __restrict__ out, long long ldo,
                    int out_fp32) {
-  pdl_launch_dependents();
+  pdl_launch_next();
   pdl_wait();
   extern __shared__ float dyn_smem[];
   const int r = blockIdx.x;
@@ -1637,6 +1637,7 @@ static int launch_window_attn(const WinArgs& a, int R, const int* row_seq, const
   const long long may_see = (a.window > 0 ? (long long)a.window + a.keep_first : (long long)a.max_pages * a.page_size) + (a.pool > 0 ? (long long)a.max_pooled_pages * a.page_size : 0);
   const bool wide = QH == 1 && may_see > 256 && grid.x * grid.y <= (unsigned)sm_count() && win_smem_floats(1, 32, a.dim, a.vdim) * sizeof(float) <= 48 * 1024;
   if (wide) warps = 32;
+  const long long pages = (long long)a.max_pages * a.page_size, work = (long long)R * a.heads * (may_see < pages || a.pool > 0 ? may_see : pages);
   while (warps > 1 && win_smem_floats(QH, warps, a.dim, a.vdim) * sizeof(float) > 48 * 1024) warps >>= 1;
   const size_t smem = win_smem_floats(QH, warps, a.dim, a.vdim) * sizeof(float);
   LP_REQUIRE(smem <= 48 * 1024, "lp_window_attn: dim=%d vdim=%d do not fit shared memory", a.dim, a.vdim);
@@ -1645,11 +1646,11 @@ static int launch_window_attn(const WinArgs& a, int R, const int* row_seq, const
   do {                                                                                                                                         \
     if constexpr (QH == 1) {                                                                                                                   \
       if (wide) {                                                                                                                              \
-        LP_CHECK_CUDA((launch_next(window_attn_kernel<QH, NV, DIST, 1024>, grid, dim3(warps * 32), smem, stream, a, R, row_seq, row_pos, out, ldo, out_fp32)));               \
+        LP_CHECK_CUDA((launch_attention(work, window_attn_kernel<QH, NV, DIST, 1024>, grid, dim3(warps * 32), smem, stream, a, R, row_seq, row_pos, out, ldo, out_fp32)));               \
         break;                                                                                                                                 \
       }                                                                                                                                        \
     }                                                                                                                                          \
-    LP_CHECK_CUDA((launch_next(window_attn_kernel<QH, NV, DIST, 256>, grid, dim3(warps * 32), smem, stream, a, R, row_seq, row_pos, out, ldo, out_fp32)));                    \
+    LP_CHECK_CUDA((launch_attention(work, window_attn_kernel<QH, NV, DIST, 256>, grid, dim3(warps * 32), smem, stream, a, R, row_seq, row_pos, out, ldo, out_fp32)));                    \
   } while (0)
   if (nv <= 1) LP_WAK(1);
   else if (nv <= 2) LP_WAK(2);

@@ -97,10 +97,19 @@ inline void set_error(const char* fmt, ...) {
 inline void note_launch(int = 1) {}
 inline void pdl_wait() {}
 inline void pdl_launch_dependents() {}
+inline void pdl_launch_next() {}
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_next(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t, cudaStream_t, Args... args) {
   emu::launch(grid, block, [&] { kern(static_cast<KArgs>(args)...); });
   return cudaSuccess;
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_attention(long long, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  return launch_next(kern, grid, block, smem, stream, args...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_ex(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int, int, Args... args) {
+  return launch_next(kern, grid, block, smem, stream, args...);
 }
 inline int g_emu_sms = 4;      // emu_set_sm_count: rules that count CTAs per SM
 inline int sm_count() { return g_emu_sms; }
