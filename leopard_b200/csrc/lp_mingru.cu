@@ -40,11 +40,8 @@ __device__ __forceinline__ void gru_store(const GruArgs& a, long long row, int c
 
 constexpr int GRU_THREADS = 128;
 
-// The kernels of a prompt do not let one another start early: waiting CTAs beside the running ones cost more than the launch gaps (630 rows of 2,846 channels 54 us, so 41; with
-// plain launches 41).
 __global__ void __launch_bounds__(GRU_THREADS)
 mingru_chunk_kernel(GruArgs a, const int* __restrict__ chunk_row0, const int* __restrict__ chunk_len, float* __restrict__ ws, int n_chunks) {
-  pdl_wait();
   const int c = blockIdx.x, ch = blockIdx.y * GRU_THREADS + threadIdx.x;
   if (ch >= a.width) return;
   const int row0 = chunk_row0[c], len = chunk_len[c];
@@ -64,8 +61,7 @@ mingru_chunk_kernel(GruArgs a, const int* __restrict__ chunk_row0, const int* __
 
 __global__ void __launch_bounds__(GRU_THREADS)
 mingru_scan_kernel(GruArgs a, const int* __restrict__ seq_chunk0, const int* __restrict__ seq_pos0, const int* __restrict__ seq_slot,
-                   float* ws, int n_chunks) {
-  pdl_wait();
+                   float* __restrict__ ws, int n_chunks) {
   const int s = blockIdx.x, ch = blockIdx.y * GRU_THREADS + threadIdx.x;
   if (ch >= a.width) return;
   float S = seq_pos0[s] == 0 ? 0.f : a.state[(long long)seq_slot[s] * a.slot_stride + ch];
@@ -78,8 +74,7 @@ mingru_scan_kernel(GruArgs a, const int* __restrict__ seq_chunk0, const int* __r
 
 __global__ void __launch_bounds__(GRU_THREADS)
 mingru_out_kernel(GruArgs a, const int* __restrict__ chunk_seq, const int* __restrict__ chunk_row0, const int* __restrict__ chunk_len,
-                  const int* __restrict__ seq_chunk0, const int* __restrict__ seq_slot, const float* ws) {
-  pdl_wait();
+                  const int* __restrict__ seq_chunk0, const int* __restrict__ seq_slot, const float* __restrict__ ws) {
   const int c = blockIdx.x, ch = blockIdx.y * GRU_THREADS + threadIdx.x;
   if (ch >= a.width) return;
   const int row0 = chunk_row0[c], len = chunk_len[c], s = chunk_seq[c];
@@ -138,11 +133,11 @@ extern "C" int lp_mingru_prefill(const lp_mingru_desc* d, int n_seqs, int n_chun
   LP_REQUIRE(ws != nullptr && ws_bytes >= lp_mingru_workspace_bytes(n_chunks, d->width), "lp_mingru_prefill: workspace too small");
   float* w = reinterpret_cast<float*>(ws);
   const int cy = (d->width + GRU_THREADS - 1) / GRU_THREADS;
-  LP_CHECK_CUDA(launch_next(mingru_chunk_kernel, dim3(n_chunks, cy), dim3(GRU_THREADS), 0, stream, a, chunk_row0, chunk_len, w, n_chunks));
+  mingru_chunk_kernel<<<dim3(n_chunks, cy), GRU_THREADS, 0, stream>>>(a, chunk_row0, chunk_len, w, n_chunks);
   LP_CHECK_CUDA(cudaGetLastError());
-  LP_CHECK_CUDA(launch_next(mingru_scan_kernel, dim3(n_seqs, cy), dim3(GRU_THREADS), 0, stream, a, seq_chunk0, seq_pos0, seq_slot, w, n_chunks));
+  mingru_scan_kernel<<<dim3(n_seqs, cy), GRU_THREADS, 0, stream>>>(a, seq_chunk0, seq_pos0, seq_slot, w, n_chunks);
   LP_CHECK_CUDA(cudaGetLastError());
-  LP_CHECK_CUDA(launch_next(mingru_out_kernel, dim3(n_chunks, cy), dim3(GRU_THREADS), 0, stream, a, chunk_seq, chunk_row0, chunk_len, seq_chunk0, seq_slot, w));
+  mingru_out_kernel<<<dim3(n_chunks, cy), GRU_THREADS, 0, stream>>>(a, chunk_seq, chunk_row0, chunk_len, seq_chunk0, seq_slot, w);
   LP_CHECK_CUDA(cudaGetLastError());
   note_launch(3);
   return 0;

@@ -60,6 +60,8 @@ __device__ __forceinline__ void warp_best(float& v, int& i, int none) {
   }
 }
 
+// Launched when the launch before has ended: placed beside it, on the SMs that it leaves empty, its CTAs took up to half as long again (norm, router of 128 experts and the rest of a
+// routing of 400 tokens of 1,024 columns 82 us, so 57, before such launches 64).
 // One CTA per token: the warps share out the router rows (and the gate row), 16-byte loads of the bf16 weights when the width
 // allows; then one warp makes the choice among the E scores.
 template <typename HT>
@@ -282,11 +284,11 @@ extern "C" int lp_moe_route(const void* h, long long ldh, int h_fp32, int T, int
   if (T <= 0) return 0;
   const unsigned grid = (unsigned)T;
   if (h_fp32)
-    LP_CHECK_CUDA(launch_next(moe_route_kernel<float>, grid, dim3(route_threads(T, E)), 0, stream, reinterpret_cast<const float*>(h), ldh, T, D,
+    LP_CHECK_CUDA(launch_ex(moe_route_kernel<float>, dim3(grid), dim3(route_threads(T, E)), 0, stream, 1, false, reinterpret_cast<const float*>(h), ldh, T, D,
         reinterpret_cast<const bf16*>(w_router), ldw, E, correction, n_groups, keep_groups, top, reinterpret_cast<const bf16*>(w_gate),
         idx_out, w_out, gate_out, 0, nullptr, 1.0f));
   else
-    LP_CHECK_CUDA(launch_next(moe_route_kernel<bf16>, grid, dim3(route_threads(T, E)), 0, stream, reinterpret_cast<const bf16*>(h), ldh, T, D,
+    LP_CHECK_CUDA(launch_ex(moe_route_kernel<bf16>, dim3(grid), dim3(route_threads(T, E)), 0, stream, 1, false, reinterpret_cast<const bf16*>(h), ldh, T, D,
         reinterpret_cast<const bf16*>(w_router), ldw, E, correction, n_groups, keep_groups, top, reinterpret_cast<const bf16*>(w_gate),
         idx_out, w_out, gate_out, 0, nullptr, 1.0f));
   note_launch();
@@ -303,10 +305,10 @@ extern "C" int lp_moe_route_softmax(const void* h, long long ldh, int h_fp32, in
   if (T <= 0) return 0;
   const unsigned grid = (unsigned)T;
   if (h_fp32)
-    LP_CHECK_CUDA(launch_next(moe_route_kernel<float>, grid, dim3(route_threads(T, E)), 0, stream, reinterpret_cast<const float*>(h), ldh, T, D,
+    LP_CHECK_CUDA(launch_ex(moe_route_kernel<float>, dim3(grid), dim3(route_threads(T, E)), 0, stream, 1, false, reinterpret_cast<const float*>(h), ldh, T, D,
         reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, 1, 1, top, nullptr, idx_out, w_out, nullptr, 1, logit_bias, 1.0f));
   else
-    LP_CHECK_CUDA(launch_next(moe_route_kernel<bf16>, grid, dim3(route_threads(T, E)), 0, stream, reinterpret_cast<const bf16*>(h), ldh, T, D,
+    LP_CHECK_CUDA(launch_ex(moe_route_kernel<bf16>, dim3(grid), dim3(route_threads(T, E)), 0, stream, 1, false, reinterpret_cast<const bf16*>(h), ldh, T, D,
         reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, 1, 1, top, nullptr, idx_out, w_out, nullptr, 1, logit_bias, 1.0f));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
@@ -322,10 +324,10 @@ extern "C" int lp_moe_route_sigmoid(const void* h, long long ldh, int h_fp32, in
   if (T <= 0) return 0;
   const unsigned grid = (unsigned)T;
   if (h_fp32)
-    LP_CHECK_CUDA(launch_next(moe_route_kernel<float>, grid, dim3(route_threads(T, E)), 0, stream, reinterpret_cast<const float*>(h), ldh, T, D,
+    LP_CHECK_CUDA(launch_ex(moe_route_kernel<float>, dim3(grid), dim3(route_threads(T, E)), 0, stream, 1, false, reinterpret_cast<const float*>(h), ldh, T, D,
         reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, 1, 1, top, nullptr, idx_out, w_out, nullptr, 2, nullptr, 1.0f));
   else
-    LP_CHECK_CUDA(launch_next(moe_route_kernel<bf16>, grid, dim3(route_threads(T, E)), 0, stream, reinterpret_cast<const bf16*>(h), ldh, T, D,
+    LP_CHECK_CUDA(launch_ex(moe_route_kernel<bf16>, dim3(grid), dim3(route_threads(T, E)), 0, stream, 1, false, reinterpret_cast<const bf16*>(h), ldh, T, D,
         reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, 1, 1, top, nullptr, idx_out, w_out, nullptr, 2, nullptr, 1.0f));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());
@@ -346,10 +348,10 @@ extern "C" int lp_moe_route_group_softmax(const void* h, long long ldh, int h_fp
   if (T <= 0) return 0;
   const unsigned grid = (unsigned)T;
   if (h_fp32)
-    LP_CHECK_CUDA(launch_next(moe_route_kernel<float>, grid, dim3(route_threads(T, E)), 0, stream, reinterpret_cast<const float*>(h), ldh, T, D,
+    LP_CHECK_CUDA(launch_ex(moe_route_kernel<float>, dim3(grid), dim3(route_threads(T, E)), 0, stream, 1, false, reinterpret_cast<const float*>(h), ldh, T, D,
         reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, n_groups, keep_groups, top, nullptr, idx_out, w_out, nullptr, 3, nullptr, w_scale));
   else
-    LP_CHECK_CUDA(launch_next(moe_route_kernel<bf16>, grid, dim3(route_threads(T, E)), 0, stream, reinterpret_cast<const bf16*>(h), ldh, T, D,
+    LP_CHECK_CUDA(launch_ex(moe_route_kernel<bf16>, dim3(grid), dim3(route_threads(T, E)), 0, stream, 1, false, reinterpret_cast<const bf16*>(h), ldh, T, D,
         reinterpret_cast<const bf16*>(w_router), ldw, E, nullptr, n_groups, keep_groups, top, nullptr, idx_out, w_out, nullptr, 3, nullptr, w_scale));
   note_launch();
   LP_CHECK_CUDA(cudaGetLastError());

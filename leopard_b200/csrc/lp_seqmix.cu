@@ -662,7 +662,7 @@ template <int V> __host__ __device__ inline int ret_dec_groups(int vdim) { retur
 template <int V>
 __global__ void __launch_bounds__(RET_DEC_THREADS)
 retention_decode_kernel(RetArgs a, const int* __restrict__ seq_row0, const int* __restrict__ seq_pos0, const int* __restrict__ seq_slot) {
-  pdl_launch_next();
+  pdl_launch_next_of_few();
   pdl_wait();
   extern __shared__ float dyn_smem[];
   const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
@@ -848,7 +848,7 @@ template <int V, int NP, int W>
 __global__ void __launch_bounds__(W * 32)
 latent_attend_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos, const float* q_abs,
                      long long ldqa, void* __restrict__ out, long long ldo, int out_fp32) {
-  pdl_launch_next();
+  pdl_launch_next_of_few();
   pdl_wait();
   __align__(16) __shared__ float s_acc[W][32 * V * NP];
   __shared__ float s_mx[W], s_den[W];
@@ -983,7 +983,7 @@ template <int NR>
 __global__ void __launch_bounds__(LAT_ROW_HEADS * 32)
 latent_attend_rows_kernel(LatArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos, const float* q_abs,
                           long long ldqa, void* __restrict__ out, long long ldo, int out_fp32) {
-  pdl_launch_next();
+  pdl_launch_next_of_few();
   pdl_wait();
   const int r = blockIdx.x;
   const int h = blockIdx.y * LAT_ROW_HEADS + (threadIdx.x >> 5);

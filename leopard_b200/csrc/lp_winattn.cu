@@ -431,7 +431,7 @@ template <int QH, int NV, bool DIST, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 window_attn_kernel(WinArgs a, int R, const int* __restrict__ row_seq, const int* __restrict__ row_pos, void* __restrict__ out, long long ldo,
                    int out_fp32) {
-  pdl_launch_next();
+  pdl_launch_next_of_few();
   pdl_wait();
   extern __shared__ float dyn_smem[];
   const int r = blockIdx.x;

@@ -98,6 +98,7 @@ inline void note_launch(int = 1) {}
 inline void pdl_wait() {}
 inline void pdl_launch_dependents() {}
 inline void pdl_launch_next() {}
+inline void pdl_launch_next_of_few() {}
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_next(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t, cudaStream_t, Args... args) {
   emu::launch(grid, block, [&] { kern(static_cast<KArgs>(args)...); });
