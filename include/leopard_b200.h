@@ -160,7 +160,8 @@ int lp_gemm_set_epilogue_sleep(int ns);
 /* Launch the hot prefill kernels (GEMM, attention v3, norms, RoPE) with programmatic dependent launch: the next kernel's
  * CTAs are scheduled as SMs free up and run their prologue (barrier init, TMEM allocation, descriptor prefetch) while the
  * previous kernel drains; each kernel executes griddepcontrol.wait before its first dependent global access.  Results
- * are unchanged.  Returns the previous setting (default set by the library). */
+ * are unchanged.  Returns the previous setting (default set by the library).  The kernels of the 32-bit residual stream are not among them: theirs are launched so
+ * wherever that was measured to pay, whatever this is. */
 int lp_set_prefill_pdl(int enable);
 
 /* O[b,t,h,:] = softmax(scale * Q K^T (+causal)) V          (tcgen05 flash attention, fp32 softmax, bf16 in/out)
@@ -715,10 +716,10 @@ int lp_gather_rows(const void* src, long long ld, int src_fp32, const int* row_o
  * out: 0 bf16, 1 fp32, 2 three planes c_plane elements apart.  K and N multiples of 8, rows on 16-byte boundaries. */
 int lp_gemm_split(const void* A, long long lda, long long a_plane, const void* W, long long ldw, void* C, long long ldc, long long c_plane,
                   int out, int M, int N, int K, const float* bias, void* stream);
-/* the same from fp32 rows; terms: room for 3 M K bf16 */
 /* The products of lp_linear's descriptor that the tcgen05 GEMM ends itself (bf16 A, one problem; the alignments of lp_gemm_bf16): c_accum with epi NONE and fp32 C,
  * C <- C + c_scale * (A W^T + bias), or bf16 C = relu2 / xielu(A W^T + bias). */
 int lp_gemm_linear(const lp_linear_desc* desc, void* stream);
+/* lp_gemm_split from fp32 rows; terms: room for 3 M K bf16 */
 int lp_linear_split(const float* A, long long lda, const void* W, long long ldw, void* C, long long ldc, int out, int M, int N, int K, const float* bias,
                     void* terms, void* stream);
 /* The products of sorted (token, expert) rows on the tcgen05 tensor cores: rows of A (n_tiles * 128 of them; bf16, or with a_plane > 0 fp32 in three planes) in

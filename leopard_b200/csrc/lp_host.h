@@ -118,7 +118,8 @@ inline cudaError_t launch_ex(void (*kern)(KArgs...), dim3 grid, dim3 block, size
 
 // The next kernel of a step: where it is small (decoding), its CTAs may be placed while the kernel before it still drains, when that one has asked for it; it
 // waits (pdl_wait) before it touches memory.  Pointers to what earlier kernels wrote are not __restrict__ there: a read-only load could be moved
-// before the wait.  Kernels of many CTAs gain nothing (prompts of 4,096 rows: 0.5 % slower with all of them launched so).
+// before the wait.  Kernels of many CTAs gain nothing (prompts of 4,096 rows: 0.5 % slower with all of them launched so).  For short kernels only: CTAs that are placed early lie
+// on the SMs that the launch before leaves empty, where long ones then take longer (attention below; retention's decode step, MinGRU's prompts and the router are launched plainly).
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_next(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
   return launch_ex(kern, grid, block, smem, stream, 1, (long long)grid.x * grid.y * grid.z <= 4LL * sm_count(), args...);

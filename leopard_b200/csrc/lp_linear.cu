@@ -621,7 +621,8 @@ __global__ void __launch_bounds__(MG * NT == 1 && sizeof(AT) == 2 ? 1024 : 512) 
 // an epilogue.  Where no launch before this one writes the weights (w_constant), the ring is filled before that launch has ended.
 // What bounds it is DRAM from about 30 MB of weights on (K = 4096, N = 32000: 39 us, 6.7 TB/s; the kernel above 46 at one row and 62 at 16; N = 16384 21.3 and
 // 24.7), below that the latency of a launch (K = N = 2048 3.7 us, 4.9).  A piece has to be large: at half of these sizes the waits between
-// pieces took the issue slots (39 -> 49 us), and bulk copies of a row each cost 110 cycles of a warp.  190 KB under way an SM: with 96 KB the same took 50 us.
+// pieces took the issue slots (39 -> 49 us), and bulk copies of a row each cost 110 cycles of a warp.  192 KB of pieces under way an SM (one to eight bf16 rows: 128 KB of them weights, which
+// alone are asked for before the wait): with 96 KB the same took 50 us.
 // The weights leave the L2 first: left to its usual order, they threw out the caches and states of the small kernels around them (window attention of one row 13 ->
 // 23 us).  Sums: 16 products a chain, which the instruction cuts off, then exactly; error against 64 bits, 1e-7 of the result: 0.5 for bf16 rows, 0.7 for fp32
 // rows at every K (above: 0.5 to 1.2 and 0.7 to 1.2); more than 16 rows are added up plainly, 0.6 and 0.75 at K = 1024 (above: 0.9 to 1.3 and 0.9 to 1.0).
@@ -1000,38 +1001,37 @@ static bool stream_ok(const LinArgs& a, int a_fp32, int batch) {
 
 // Where the ring is ahead of the kernel without it (both on 9,000 random sizes, us a launch in a graph, that kernel and the ring).  It brings whole pieces of a tile through one
 // CTA an SM, so it wants a K of several pieces, and full rounds of tiles: 8 rows of bf16, K = 512, N = 7168 3.8, 5.3; K = 640, N = 7808 4.6, 5.9; K = 2048, N = 2048
-// 5.0, 3.6; K = 4096, N = 6144 12.1, 9.1; 16 rows, K = 4096, N = 32000 62, 44; but one row, K = 13376, N = 3072 (192 tiles on 148 SMs) 17.3, 18.9.  A few
-// columns over a very long K: all of it comes through a few CTAs (one row, K = 13312, N = 16 7.1, 7.9; fp32 K = 8256, N = 96 10.0, 12.2).
-// Weights that may be read early come while the small kernel before it runs, as in a decode step, and the lines are drawn for these: after a row norm of 2 us, 111 to 148 tiles of
-// K = 512 took 0.89 of that kernel's time (alone 1.05), two rounds of K = 640 to 1024 0.93 (1.0), 64 rows of 111 to 148 tiles of K = 512 0.92 (1.03).
+// 5.0, 3.6; K = 4096, N = 6144 12.1, 9.1; 16 rows, K = 4096, N = 32000 62, 44.  A few columns over a very long K: all of it comes through a few CTAs (one row, K = 13312, N = 16 7.1,
+// 7.9; fp32 K = 8256, N = 96 10.0, 12.2).
+// The lines are those of whole decode steps, where weights that may be read early come while the small kernel before it runs and what others keep in the L2 stays there: after a
+// row norm of 2 us, 111 to 148 tiles of K = 512 took 0.89 of that kernel's time (alone 1.05), two rounds of K = 640 to 1024 0.93 (1.0).  Launches alone put K = 12288, N = 3072 (192 tiles
+// on 148 SMs; 17.3, 18.9) and K = 1536, N = 6144 (4.7, 4.9) on the other side; steps with these took 221 us so for 203, and 132 for 126.
 // fp32 rows are cut into terms for every tile: two tiles a piece where there is more than one a CTA (4 rows, K = 2048, N = 8192 13.0, 10.2 with one and
 // two tiles); 9 to 16 of them fill the issue slots up to one tile a CTA (K = N = 2048 7.3, 7.5; but N = 6144, K = 4096 34, 29).
 // 17 to 64 rows: A is most of what a CTA brings (64 rows, K = 4096, N = 1024 24.6, 15.4; fp32 K = 1024, N = 2048 14.9, 12.7), and up to 32 its plain sums are the cheaper
-// ones at most sizes; more are ahead up to a tile a CTA, and in a third round (K = 2048, N = 6144, 33 rows 23.9, 21.1) that is nearly full, not in a
+// ones at most sizes; more are ahead up to a tile a CTA (a step of 64 requests of width 512 176 us without K = 512, so 172), and in a third round (K = 2048, N = 6144, 33 rows 23.9, 21.1) that is nearly full, not in a
 // second or a fourth (35 rows, K = 16192, N = 2752 72, 93; 58 gated rows, K = 5120, N = 2864 28.8, 32.5).
 static bool ring_pays_rows(int a_fp32, int mg, long long tiles, int K) {
   const long long sms = sm_count();
   const bool one = tiles <= sms, few = 4 * tiles <= sms;      // one tile a CTA; a quarter of the SMs at most
   if (mg == 8) {
     if (!one) return tiles > 2 * sms && tiles <= 3 * sms && K >= 2048;
-    return K <= 256 || (K <= 512 ? !few : a_fp32 || tiles > 8);
+    return a_fp32 || tiles > 8 || K <= 2048;
   }
   if (mg == 4) {
     if (one) return !a_fp32 || K < 1024 || (K >= 2048 && !few) || (K > 4096 && tiles > 8);
     return K >= (tiles <= 2 * sms ? 1024 : 2048) && tiles <= 4 * sms;
   }
-  const bool half = !one && 2 * tiles <= 3 * sms;      // a second round of half the SMs at most
   if (mg == 2) {
     if (a_fp32) return !one && tiles <= 4 * sms && K >= 2048;
-    return one ? K > 512 : !half && K >= (tiles > 3 * sms && tiles <= 4 * sms ? 4096 : 2048);
+    return K > (one ? 512 : 2047);
   }
   if (a_fp32) {
     if (one) return few ? K <= 1536 : K > 128;
-    return K >= 512 && (tiles <= 2 * sms || tiles > 3 * sms);
+    return K >= 1024 || (K >= 512 && (tiles <= 2 * sms || tiles > 3 * sms));
   }
   if (one) return K > 256 && (tiles > 8 || K <= 8192);
-  if (!one && 5 * tiles <= 8 * sms && K > 4096) return false;
-  return K >= 2048 || (K > 512 && tiles <= 2 * sms) || (K >= 1024 && tiles > 4 * sms);
+  return K >= 1024 || (K > 512 && tiles <= 2 * sms);
 }
 // The same for pairs.  Its CTAs sort all pairs, 0.75 ns a group that has some and group (200 groups of 512 x 512, 188 pairs 35.8, 58.4); that kernel has CTAs for the groups
 // without pairs too (256 groups of 512 x 512: 18 us for two pairs, 13).  So: few groups to sort, or weights that take eight times as long, and then either many CTAs there, or
